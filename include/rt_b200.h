@@ -290,6 +290,19 @@ rt_status rt_relu_max_pool2x2_backward_from_output(rt_ctx* ctx, const float* y, 
  * the transposes. */
 rt_status rt_gemm(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a,
                   int64_t lda, const float* b, int64_t ldb, float* c, int64_t ldc, int accumulate);
+/* c[M,N] = act(a[M,K] * b[K,N] + bias[N]): a linear layer with its activation in the product's epilogue (the reference runs
+ * matmul, add and the activation one after the other, examples/train_mnist_cpu.rs:46-62).  bias may be NULL. */
+enum { RT_ACT_NONE = 0, RT_ACT_RELU = 1, RT_ACT_TANH = 2, RT_ACT_SIGMOID = 3 };
+rt_status rt_gemm_bias_act(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb,
+                           const float* bias, int act, float* c, int64_t ldc);
+/* The same for `count` pairs a_i, c_i (contiguous) with one b: a layer applied to every timestep, in one launch. */
+rt_status rt_gemm_bias_act_list(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k, const float* b,
+                                const float* bias, int act);
+/* c[K,N] += sum over i < count of a_i[M,K]^T * g_i[M,N] (contiguous a_i, g_i): the gradient of a weight that is used `count`
+ * times (recurrent layers), as one product with the reduction running over all uses.  Host arrays of device pointers. */
+rt_status rt_gemm_sum_products(rt_ctx* ctx, int count, const float* const* a, const float* const* g, int64_t m, int64_t k, int64_t n, float* c);
+/* out[c] += sum over i < count and rows r of x_i[rows, cols][r, c]: the same for a bias. */
+rt_status rt_sum_rows_accumulate_list(rt_ctx* ctx, int count, const float* const* x, int64_t rows, int64_t cols, float* out);
 /* da[M,K] = g * b^T, db[K,N] = a^T * g   (matmul_backward mod.rs:324); NULL skips one. */
 rt_status rt_matmul_backward(rt_ctx* ctx, const float* a, const float* b, const float* g, int64_t m, int64_t k,
                              int64_t n, float* da, float* db);

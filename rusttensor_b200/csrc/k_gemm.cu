@@ -19,6 +19,12 @@ rt_status rt_sum_axis_internal(rt_ctx* ctx, const float* x, int64_t outer, int64
 rt_status rt_gemm_tc_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a,
                               int64_t lda, const float* b, int64_t ldb, float* c, int64_t ldc, int accumulate);
 
+rt_status rt_gemm_small_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
+                                 const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
+rt_status rt_gemm_small_list_internal(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k,
+                                      const float* b, const float* bias, int act);
+rt_status rt_gemm_list_tc_internal(rt_ctx* ctx, int count, const float* const* a, const float* const* g, int64_t m, int64_t k, int64_t n,
+                                   float* out);
 rt_status rt_conv_forward_tc_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g,
                                       float* y);
 rt_status rt_conv_gather_tc_internal(rt_ctx* ctx, const float* y, const float* w, const float* bias, const ConvGeom& g,
@@ -571,8 +577,142 @@ rt_status channel_sum(rt_ctx* ctx, const float* t, int64_t nb, int64_t c, int64_
 
 }  // namespace
 
+namespace {
+// c = act(c + bias) in place, for the products whose kernel has no epilogue of its own
+__global__ void __launch_bounds__(256) bias_act_kernel(float* __restrict__ c, const float* __restrict__ bias, int64_t m, int n, int64_t ldc,
+                                                       int act) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m * n; i += (int64_t)gridDim.x * blockDim.x) {
+    float* q = c + i / n * ldc + i % n;
+    float v = *q + (bias ? __ldg(bias + i % n) : 0.f);
+    if (act == RT_ACT_RELU) v = fmaxf(v, 0.f);
+    else if (act == RT_ACT_TANH) v = tanhf(v);
+    else if (act == RT_ACT_SIGMOID) v = 1.f / (1.f + expf(-v));
+    *q = v;
+  }
+}
+// out[c] += column sums of a stack of [rows, cols] matrices: 32 row lanes per column, one block per 32 columns, so that nothing has
+// to be handed over between blocks and the order of the sums is fixed
+constexpr int kRowListTerms = 256;
+struct RowList {
+  const float* x[kRowListTerms];
+  FastDiv d_rows;
+  int count;
+};
+__global__ void __launch_bounds__(1024) col_sum_list_kernel(const RowList l, int64_t total, int64_t cols, float* __restrict__ out) {
+  __shared__ float red[32][33];
+  const int64_t c = (int64_t)blockIdx.x * 32 + threadIdx.x;
+  float acc = 0.f;
+  if (c < cols) {
+#pragma unroll 8
+    for (int64_t r = threadIdx.y; r < total; r += 32) {
+      uint32_t t, q;
+      l.d_rows.divmod((uint32_t)r, t, q);
+      acc += __ldg(l.x[t] + (int64_t)q * cols + c);
+    }
+  }
+  red[threadIdx.y][threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < cols) {
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) s += red[j][threadIdx.x];
+    out[c] += s;
+  }
+}
+}  // namespace
+
 extern "C" {
 
+// Products for the one-launch fp32 kernel (k_gemm_small.cu).  Above 32 M multiply-adds the tensor cores win (64 x 577 x 2048: 9.5 against
+// 11.8 us; 90 x 1000 x 100: 6.5 against 9.4), and a reduction of more than 8 x 256 leaves each CTA of the cluster a serial walk that the
+// tensor-core kernel splits over the whole chip.
+static bool small_product(int64_t m, int64_t n, int64_t k) {
+  return k > 0 && k <= 2048 && m * n * k <= (32ll << 20);
+}
+rt_status rt_gemm_bias_act(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb,
+                           const float* bias, int act, float* c, int64_t ldc) {
+  RT_CHECK_CTX(ctx);
+  if (act < RT_ACT_NONE || act > RT_ACT_SIGMOID) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_gemm_bias_act: unknown activation %d", act);
+  if (m <= 0 || n <= 0 || k <= 0 || lda < k || ldb < n || ldc < n) RT_FAIL(ctx, RT_ERR_SHAPE_MISMATCH, "rt_gemm_bias_act: bad extents");
+  RT_CHECK_PTR(ctx, a);
+  RT_CHECK_PTR(ctx, b);
+  RT_CHECK_PTR(ctx, c);
+  if (small_product(m, n, k)) {
+    rt_status st = rt_gemm_small_internal(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, bias, act, 0);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
+  rt_status st = rt_gemm(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, 0);
+  if (st != RT_OK || (!bias && act == RT_ACT_NONE)) return st;
+  bias_act_kernel<<<rt_grid_for(ctx, m * n, 256), 256, 0, ctx->stream>>>(c, bias, m, (int)n, ldc, act);
+  RT_LAUNCHED(ctx);
+  return RT_OK;
+}
+rt_status rt_gemm_bias_act_list(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k, const float* b,
+                                const float* bias, int act) {
+  RT_CHECK_CTX(ctx);
+  if (count <= 0) return RT_OK;
+  RT_CHECK_PTR(ctx, a);
+  RT_CHECK_PTR(ctx, c);
+  RT_CHECK_PTR(ctx, b);
+  if (act < RT_ACT_NONE || act > RT_ACT_SIGMOID) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_gemm_bias_act_list: unknown activation %d", act);
+  if (m <= 0 || n <= 0 || k <= 0) RT_FAIL(ctx, RT_ERR_SHAPE_MISMATCH, "rt_gemm_bias_act_list: bad extents");
+  if (small_product(m, n, k)) {
+    rt_status st = rt_gemm_small_list_internal(ctx, count, a, c, m, n, k, b, bias, act);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
+  for (int i = 0; i < count; ++i) {
+    rt_status st = rt_gemm_bias_act(ctx, m, n, k, a[i], k, b, n, bias, act, c[i], n);
+    if (st != RT_OK) return st;
+  }
+  return RT_OK;
+}
+rt_status rt_gemm_sum_products(rt_ctx* ctx, int count, const float* const* a, const float* const* g, int64_t m, int64_t k, int64_t n, float* c) {
+  RT_CHECK_CTX(ctx);
+  if (count < 0 || m < 0 || k < 0 || n < 0) RT_FAIL(ctx, RT_ERR_INVALID_INDEX, "rt_gemm_sum_products: negative extent");
+  if (count == 0 || m == 0 || k == 0 || n == 0) return RT_OK;
+  RT_CHECK_PTR(ctx, a);
+  RT_CHECK_PTR(ctx, g);
+  RT_CHECK_PTR(ctx, c);
+  if (ctx->use_tensor_cores && k >= 32 && n >= 16 && count > 1 && m * count < (1ll << 31) && m * n * k * count >= (1ll << 20)) {
+    RtScratch sum(ctx);
+    rt_status st = sum.alloc(sizeof(float) * (size_t)(k * n));
+    if (st != RT_OK) return st;
+    const int64_t shape[1] = {k * n};
+    for (int i = 0; i < count; i += 256) {
+      st = rt_gemm_list_tc_internal(ctx, count - i < 256 ? count - i : 256, a + i, g + i, m, k, n, sum.as<float>());
+      if (st == RT_OK) st = rt_binary(ctx, RT_ADD, c, shape, 1, sum.as<float>(), shape, 1, c);
+      if (st != RT_OK) return st;
+    }
+    return RT_OK;
+  }
+  for (int i = 0; i < count; ++i) {
+    rt_status st = rt_gemm(ctx, 1, 0, k, n, m, a[i], k, g[i], n, c, n, 1);
+    if (st != RT_OK) return st;
+  }
+  return RT_OK;
+}
+rt_status rt_sum_rows_accumulate_list(rt_ctx* ctx, int count, const float* const* x, int64_t rows, int64_t cols, float* out) {
+  RT_CHECK_CTX(ctx);
+  if (count <= 0 || rows <= 0 || cols <= 0) return RT_OK;
+  RT_CHECK_PTR(ctx, x);
+  RT_CHECK_PTR(ctx, out);
+  if (rows >= (1 << 22)) {
+    for (int i = 0; i < count; ++i) {
+      rt_status st = rt_sum_rows_accumulate(ctx, x[i], rows, cols, out);
+      if (st != RT_OK) return st;
+    }
+    return RT_OK;
+  }
+  for (int i = 0; i < count; i += kRowListTerms) {
+    RowList l{};
+    l.count = count - i < kRowListTerms ? count - i : kRowListTerms;
+    for (int j = 0; j < l.count; ++j) l.x[j] = x[i + j];
+    l.d_rows.init((uint32_t)rows);
+    col_sum_list_kernel<<<(unsigned)((cols + 31) / 32), dim3(32, 32), 0, ctx->stream>>>(l, rows * l.count, cols, out);
+    RT_LAUNCHED(ctx);
+  }
+  return RT_OK;
+}
 rt_status rt_gemm(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
                   const float* b, int64_t ldb, float* c, int64_t ldc, int accumulate) {
   RT_CHECK_CTX(ctx);
@@ -588,6 +728,10 @@ rt_status rt_gemm(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, i
   bool acc = accumulate != 0;
   if (ctx->use_tensor_cores) {  // narrow products: dedicated FP32 kernels
     rt_status st = gemm_narrow(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, accumulate);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
+  if (small_product(m, n, k)) {
+    rt_status st = rt_gemm_small_internal(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, nullptr, RT_ACT_NONE, accumulate);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   if (ctx->use_tensor_cores && k >= 32 && m >= 32 && n >= 16 && m * n * k >= (1ll << 20)) {

@@ -1,0 +1,290 @@
+// Small and narrow products in exact fp32: C[M,N] = act(op(A) op(B) + bias) (+ C).
+//
+// What bounds them: with a few dozen output tiles a product of this size occupies a fraction of the chip for as long as one tile
+// walks its reduction, and a second launch that adds split-K partial sums costs as much as the product.  So
+//  * 32 x 64 tiles, and the reduction of a tile is split over the CTAs of a cluster (1, 2, 4 or 8), so that about one to two
+//    CTAs land on every SM; their partial tiles meet in distributed shared memory and each CTA finishes a slice of the rows:
+//    bias, activation and accumulation included, one launch in all, sums in a fixed order;
+//  * inside a CTA two groups of four warps take alternate halves of every 64-deep K-block (4 x 4 outputs a thread);
+//  * operands arrive by cp.async, three K-blocks in flight, 16 bytes at a time where the rows allow it, else 4.
+// fp32 FMAs rather than tensor cores: below a few hundred MFLOP the splitting of operands into TF32 parts and the tensor-memory
+// set-up cost more than the arithmetic.
+#include <cooperative_groups.h>
+
+#include "rt_internal.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+constexpr int kBM = 32, kBN = 64, kBK = 64, kStages = 3, kThreads = 256;
+constexpr int kPad = 4;
+
+struct SmallGemm {
+  const float *a, *b, *bias;
+  float* c;
+  int64_t lda, ldb, ldc;
+  int m, n, k, k_per_split, act;
+  bool a16, b16, accumulate;
+};
+
+__device__ __forceinline__ void async_copy(float* dst, const float* src, int bytes, bool wide) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+// A ROWS x COLS piece of a row-major matrix (COLS contiguous) to shared memory with row stride COLS + kPad, zeros outside
+// [row_end) x [col_end).
+template <int ROWS, int COLS>
+__device__ __forceinline__ void load_piece(float* s, const float* g, int64_t ld, int row0, int row_end, int col0, int col_end, bool wide) {
+  if (wide) {
+    constexpr int kChunks = ROWS * COLS / 4;
+#pragma unroll
+    for (int i = threadIdx.x; i < kChunks; i += kThreads) {
+      const int r = i / (COLS / 4), c = i % (COLS / 4) * 4;
+      int left = (col_end - (col0 + c)) * 4;
+      left = row0 + r < row_end ? (left > 16 ? 16 : (left < 0 ? 0 : left)) : 0;
+      async_copy(s + r * (COLS + kPad) + c, left ? g + (int64_t)(row0 + r) * ld + col0 + c : g, left, true);
+    }
+  } else {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < ROWS * COLS; i += kThreads) {
+      const int r = i / COLS, c = i % COLS;
+      const bool in = row0 + r < row_end && col0 + c < col_end;
+      async_copy(s + r * (COLS + kPad) + c, in ? g + (int64_t)(row0 + r) * ld + col0 + c : g, in ? 4 : 0, false);
+    }
+  }
+}
+
+__device__ __forceinline__ float activate(float v, int act) {
+  switch (act) {
+    case RT_ACT_RELU: return fmaxf(v, 0.f);
+    case RT_ACT_TANH: return tanhf(v);
+    case RT_ACT_SIGMOID: return 1.f / (1.f + expf(-v));
+    default: return v;
+  }
+}
+
+template <bool TA, bool TB>
+struct Shape {
+  static constexpr int a_floats = TA ? kBK * (kBM + kPad) : kBM * (kBK + kPad);
+  static constexpr int b_floats = TB ? kBN * (kBK + kPad) : kBK * (kBN + kPad);
+  static constexpr size_t bytes = sizeof(float) * kStages * (a_floats + b_floats);
+  static_assert(kBM * (kBN + kPad) <= kStages * (a_floats + b_floats), "the partial tile reuses the stages");
+};
+
+// Several left operands and results for one right operand: the row tiles of item i follow those of item i - 1.
+constexpr int kListTerms = 256;
+struct SmallList {
+  const float* a[kListTerms];
+  float* c[kListTerms];
+  int row_tiles;
+};
+struct NoList {};
+
+template <bool TA, bool TB, class List>
+__global__ void __launch_bounds__(kThreads, 3) small_gemm_kernel(const SmallGemm args, const List list) {
+  extern __shared__ __align__(16) float smem[];
+  using S = Shape<TA, TB>;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int splits = cluster.num_blocks(), rank = cluster.block_rank();
+  SmallGemm p = args;
+  int row_tile = blockIdx.y;
+  if constexpr (sizeof(List) > sizeof(NoList)) {
+    const int item = row_tile / list.row_tiles;
+    row_tile -= item * list.row_tiles;
+    p.a = list.a[item];
+    p.c = list.c[item];
+  }
+  const int m0 = row_tile * kBM, n0 = (int)(blockIdx.x / splits) * kBN;
+  const int kbeg = rank * p.k_per_split, kend = min(p.k, kbeg + p.k_per_split);
+  const int blocks = kend > kbeg ? (kend - kbeg + kBK - 1) / kBK : 0;
+  const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const int tm = (lane >> 3) + 4 * (warp & 1), tn = (lane & 7) + 8 * (warp >> 1);  // 8 x 16 threads
+
+  auto fetch = [&](int i) {
+    if (i < blocks) {
+      float* sa = smem + (i % kStages) * (S::a_floats + S::b_floats);
+      float* sb = sa + S::a_floats;
+      const int k0 = kbeg + i * kBK;
+      if (TA) load_piece<kBK, kBM>(sa, p.a, p.lda, k0, kend, m0, p.m, p.a16);
+      else load_piece<kBM, kBK>(sa, p.a, p.lda, m0, p.m, k0, kend, p.a16);
+      if (TB) load_piece<kBN, kBK>(sb, p.b, p.ldb, n0, p.n, k0, kend, p.b16);
+      else load_piece<kBK, kBN>(sb, p.b, p.ldb, k0, kend, n0, p.n, p.b16);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+
+#pragma unroll
+  for (int i = 0; i < kStages - 1; ++i) fetch(i);
+  for (int it = 0; it < blocks; ++it) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();
+    fetch(it + kStages - 1);
+    const float* sa = smem + (it % kStages) * (S::a_floats + S::b_floats);
+    const float* sb = sa + S::a_floats;
+#pragma unroll
+    for (int q = 0; q < kBK / 2; q += 4) {
+      const int k = group * (kBK / 2) + q;
+      float av[4][4], bv[4][4];  // [row or column][k]
+      if (TA) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const float4 t = *reinterpret_cast<const float4*>(sa + (k + kk) * (kBM + kPad) + 4 * tm);
+          av[0][kk] = t.x; av[1][kk] = t.y; av[2][kk] = t.z; av[3][kk] = t.w;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 t = *reinterpret_cast<const float4*>(sa + (tm + 8 * i) * (kBK + kPad) + k);
+          av[i][0] = t.x; av[i][1] = t.y; av[i][2] = t.z; av[i][3] = t.w;
+        }
+      }
+      if (TB) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 t = *reinterpret_cast<const float4*>(sb + (tn + 16 * j) * (kBK + kPad) + k);
+          bv[j][0] = t.x; bv[j][1] = t.y; bv[j][2] = t.z; bv[j][3] = t.w;
+        }
+      } else {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const float4 t = *reinterpret_cast<const float4*>(sb + (k + kk) * (kBN + kPad) + 4 * tn);
+          bv[0][kk] = t.x; bv[1][kk] = t.y; bv[2][kk] = t.z; bv[3][kk] = t.w;
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i][kk], bv[j][kk], acc[i][j]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  // the two groups' sums, then the cluster's
+  float* part = smem;  // [kBM][kBN + kPad]
+  auto row_of = [&](int i) { return TA ? 4 * tm + i : tm + 8 * i; };
+  auto col_of = [&](int j) { return TB ? tn + 16 * j : 4 * tn + j; };
+  if (group == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[row_of(i) * (kBN + kPad) + col_of(j)] = acc[i][j];
+  }
+  __syncthreads();
+  if (group == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[row_of(i) * (kBN + kPad) + col_of(j)] += acc[i][j];
+  }
+  if (splits > 1) cluster.sync();
+  else __syncthreads();
+  const int rows = kBM / splits;
+  for (int idx = threadIdx.x; idx < rows * (kBN / 4); idx += kThreads) {
+    const int r = rank * rows + idx / (kBN / 4), c = idx % (kBN / 4) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < splits; ++s) {
+      const float* q = splits > 1 ? cluster.map_shared_rank(part, s) : part;
+      const float4 t = *reinterpret_cast<const float4*>(q + r * (kBN + kPad) + c);
+      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+    }
+    const int m = m0 + r, n = n0 + c;
+    if (m < p.m) {
+      float* out = p.c + (int64_t)m * p.ldc + n;
+      const float e[4] = {v.x, v.y, v.z, v.w};
+      float o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        o[j] = e[j];
+        if (n + j < p.n) {
+          if (p.bias) o[j] += __ldg(p.bias + n + j);
+          o[j] = activate(o[j], p.act);
+          if (p.accumulate) o[j] += out[j];
+        }
+      }
+      if (n + 3 < p.n && rt_aligned16(out)) {
+        *reinterpret_cast<float4*>(out) = make_float4(o[0], o[1], o[2], o[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (n + j < p.n) out[j] = o[j];
+      }
+    }
+  }
+  if (splits > 1) cluster.sync();  // nobody leaves while its partial tile may still be read
+}
+
+template <bool TA, bool TB, class List = NoList>
+rt_status launch_small(rt_ctx* ctx, const SmallGemm& p, int splits, const List& list = List{}, int items = 1) {
+  auto kern = small_gemm_kernel<TA, TB, List>;
+  using S = Shape<TA, TB>;
+  static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes);
+  if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "small product: %s", cudaGetErrorString(set));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((p.n + kBN - 1) / kBN * splits), (unsigned)((p.m + kBM - 1) / kBM * items), 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = S::bytes;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)splits;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  RT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, p, list));
+  RT_LAUNCHED(ctx);
+  return RT_OK;
+}
+
+}  // namespace
+
+rt_status rt_gemm_small_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
+                                 const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
+  const int64_t tiles = ((m + kBM - 1) / kBM) * ((n + kBN - 1) / kBN);
+  if (m >= (1 << 20) || n >= (1 << 20) || k >= (1 << 28) || (m + kBM - 1) / kBM > 65535) return RT_ERR_UNIMPLEMENTED;
+  // as many splits as put a CTA and a half on every SM, at least one K-block each
+  int splits = 1;
+  while (splits < 8 && tiles * splits * 2 <= (int64_t)ctx->sm_count * 2 && k > (int64_t)kBK * splits) splits *= 2;
+  int64_t per = (k + splits - 1) / splits;
+  per = (per + kBK - 1) / kBK * kBK;
+  SmallGemm p{a, b, bias, c, lda, ldb, ldc, (int)m, (int)n, (int)k, (int)per, act, rt_aligned16(a) && lda % 4 == 0, rt_aligned16(b) && ldb % 4 == 0,
+              accumulate != 0};
+  if (!trans_a && !trans_b) return launch_small<false, false>(ctx, p, splits);
+  if (!trans_a && trans_b) return launch_small<false, true>(ctx, p, splits);
+  if (trans_a && !trans_b) return launch_small<true, false>(ctx, p, splits);
+  return launch_small<true, true>(ctx, p, splits);
+}
+
+rt_status rt_gemm_small_list_internal(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k,
+                                      const float* b, const float* bias, int act) {
+  const int64_t row_tiles = (m + kBM - 1) / kBM, tiles = row_tiles * ((n + kBN - 1) / kBN) * (count < kListTerms ? count : kListTerms);
+  if (m >= (1 << 20) || n >= (1 << 20) || k >= (1 << 28) || row_tiles * kListTerms > 65535) return RT_ERR_UNIMPLEMENTED;
+  int splits = 1;
+  while (splits < 8 && tiles * splits * 2 <= (int64_t)ctx->sm_count * 2 && k > (int64_t)kBK * splits) splits *= 2;
+  int64_t per = (k + splits - 1) / splits;
+  per = (per + kBK - 1) / kBK * kBK;
+  for (int q = 0; q < count; q += kListTerms) {
+    const int items = count - q < kListTerms ? count - q : kListTerms;
+    SmallList l{};
+    l.row_tiles = (int)row_tiles;
+    bool a16 = k % 4 == 0;
+    for (int i = 0; i < items; ++i) {
+      l.a[i] = a[q + i];
+      l.c[i] = c[q + i];
+      a16 = a16 && rt_aligned16(a[q + i]);
+    }
+    SmallGemm p{nullptr, b, bias, nullptr, k, n, n, (int)m, (int)n, (int)k, (int)per, act, a16, rt_aligned16(b) && n % 4 == 0, false};
+    rt_status st = launch_small<false, false>(ctx, p, splits, l, items);
+    if (st != RT_OK) return st;
+  }
+  return RT_OK;
+}

@@ -91,6 +91,35 @@ struct MatMN {  // element(row, k) = p[k * ld + row]
   }
 };
 
+// Several [m, ld] matrices below one another, the row index of the stack as the reduction: element(row, k) =
+// p[k / m][(k % m) * ld + row].
+constexpr int kListTerms = 256;
+struct ListMN {
+  static constexpr int kKind = 1;
+  const float* p[kListTerms];
+  FastDiv d_m;
+  int64_t ld;
+  int rows;
+  bool vec;
+  struct State { int r0; };
+  __device__ __forceinline__ State prep_quad(int r0) const { return State{r0}; }
+  __device__ __forceinline__ void fetch_r4(const State& s, int k, int kend, float (&v)[4]) const {
+    v[0] = v[1] = v[2] = v[3] = 0.f;
+    if (k >= kend || s.r0 >= rows) return;
+    uint32_t t, r;
+    d_m.divmod((uint32_t)k, t, r);
+    const float* q = p[t] + (int64_t)r * ld + s.r0;
+    if (vec && s.r0 + 3 < rows) {
+      float4 u = __ldg(reinterpret_cast<const float4*>(q));
+      v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (s.r0 + i < rows) v[i] = __ldg(q + i);
+    }
+  }
+};
+
 // ---- implicit-GEMM views of a convolution -----------------------------------------------------
 // Geometry (conv_geom.cuh): wide tensor X[Nb,Cx,Hx,Wx], narrow tensor Y[Nb,Cy,Hy,Wy],
 // y(b,cy,yo,xo) touches x(b,cx,yo*sh-ph+ky,xo*sw-pw+kx).  All element offsets fit in 31 bits
@@ -1241,4 +1270,23 @@ rt_status rt_conv_weight_grad_tc_internal(rt_ctx* ctx, const float* x, const flo
   st = dispatch_bn(ctx, la, lb, epi, (int)M, (int)N, (int)K, splits, kps);
   if (st != RT_OK) return st;
   return rt_sum_axis_internal(ctx, ws.as<float>(), 1, splits, M * N, dw, 1.f);
+}
+
+// out[M,N] = sum over the terms of a_i^T g_i, M = columns of a_i, N = columns of g_i, the stacked rows as the reduction.
+rt_status rt_gemm_list_tc_internal(rt_ctx* ctx, int count, const float* const* a, const float* const* g, int64_t m, int64_t k, int64_t n,
+                                   float* out) {
+  using namespace tc;
+  if (count > kListTerms) return RT_ERR_UNIMPLEMENTED;
+  ListMN la{}, lb{};
+  la.ld = k; la.rows = (int)k; la.vec = k % 4 == 0;
+  lb.ld = n; lb.rows = (int)n; lb.vec = n % 4 == 0;
+  for (int i = 0; i < count; ++i) {
+    la.p[i] = a[i];
+    lb.p[i] = g[i];
+    la.vec = la.vec && al16(a[i]);
+    lb.vec = lb.vec && al16(g[i]);
+  }
+  la.d_m.init((uint32_t)m);
+  lb.d_m.init((uint32_t)m);
+  return gemm_plain(ctx, la, lb, out, n, k, n, m * count, false);
 }
