@@ -251,6 +251,18 @@ rt_status rt_softmax_cross_entropy(rt_ctx* ctx, const float* logits, const float
 rt_status rt_softmax_cross_entropy_backward(rt_ctx* ctx, const float* logits, const float* targets, const float* g,
                                             int64_t rows, int64_t classes, float* dlogits, float* dtargets);
 
+/* loss[0] = scale / divisor * sum over rows and classes of targets * log_softmax(logits), and
+ * dlogits = c * (targets - softmax(logits) * sum_k targets) for the upstream gradient c * targets of log_softmax: the chains
+ * log_softmax -> mul -> sum -> mul -> mean (src/ops/mod.rs:1356-1424) and their backward with the constants known. */
+rt_status rt_softmax_nll_scaled(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes, float scale,
+                                float divisor, float* loss);
+rt_status rt_softmax_nll_scaled_backward(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes, float c,
+                                         float* dlogits);
+
+/* loss[0] = the sum of `count` such losses (logits_i, targets_i) and of n_more scalars: the loss of a sequence. */
+rt_status rt_softmax_nll_list(rt_ctx* ctx, int count, const float* const* logits, const float* const* targets, int64_t rows, int64_t classes,
+                              float scale, float divisor, int n_more, const float* const* more, float* loss);
+
 /* out[outer, inner] = sum over the middle axis of x[outer, len, inner], like rt_reduce(RT_RED_SUM), but the
  * call allocates nothing: the partial sums of a split reduction go to a fixed 1 MiB array in device memory
  * (one per device) instead of a block from the context's allocator.  No counterpart in the reference; it

@@ -1093,7 +1093,7 @@ __device__ __forceinline__ void row_max_lse(const float* __restrict__ x, int cla
 }
 
 __global__ void __launch_bounds__(kThreads) sce_forward_kernel(const float* __restrict__ logits, const float* __restrict__ targets,
-                                                               float* __restrict__ loss, int64_t rows, int classes) {
+                                                               float* __restrict__ loss, int64_t rows, int classes, float scale, float divisor) {
   __shared__ float smem[kThreads / 32];
   float acc = 0.f;
   for (int64_t r = threadIdx.x; r < rows; r += kThreads) {
@@ -1106,14 +1106,14 @@ __global__ void __launch_bounds__(kThreads) sce_forward_kernel(const float* __re
     acc += e;
   }
   acc = block_reduce<RT_RED_SUM>(acc, smem);
-  if (threadIdx.x == 0) loss[0] = (acc / (float)rows) * -1.0f;
+  if (threadIdx.x == 0) loss[0] = (acc / divisor) * scale;
 }
 
 // dlogits = -(g/rows) * (t - softmax * sum_k t);  dtargets (optional) = -(g/rows) * log_softmax
 __global__ void __launch_bounds__(kThreads) sce_backward_kernel(const float* __restrict__ logits, const float* __restrict__ targets,
-                                                                const float* __restrict__ g, float* __restrict__ dlogits,
+                                                                const float* __restrict__ g, float c, float* __restrict__ dlogits,
                                                                 float* __restrict__ dtargets, int64_t rows, int classes) {
-  const float scale = -__ldg(g) / (float)rows;
+  const float scale = g ? -__ldg(g) / (float)rows : c;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
     const float* x = logits + r * classes;
     const float* t = targets + r * classes;
@@ -1153,7 +1153,7 @@ constexpr int kSceWarpBlock = 1024;
 // part[block] = sum over the block's rows of sum_k log_softmax * t; with `final` the single block writes the loss itself.
 __global__ void __launch_bounds__(kSceWarpBlock) sce_forward_warp_kernel(const float* __restrict__ logits,
                                                                          const float* __restrict__ targets, float* __restrict__ out,
-                                                                         int64_t rows, int classes, int final) {
+                                                                         int64_t rows, int classes, int final, float scale, float divisor) {
   __shared__ float smem[kSceWarpBlock / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int nw = kSceWarpBlock / 32;
@@ -1172,21 +1172,21 @@ __global__ void __launch_bounds__(kSceWarpBlock) sce_forward_warp_kernel(const f
   if (threadIdx.x == 0) {
     float total = 0.f;
     for (int w = 0; w < nw; ++w) total += smem[w];
-    out[blockIdx.x] = final ? (total / (float)rows) * -1.0f : total;
+    out[blockIdx.x] = final ? (total / divisor) * scale : total;
   }
 }
 
-__global__ void __launch_bounds__(32) sce_finish_kernel(const float* __restrict__ part, int n, float* __restrict__ loss, int64_t rows) {
+__global__ void __launch_bounds__(32) sce_finish_kernel(const float* __restrict__ part, int n, float* __restrict__ loss, float scale, float divisor) {
   float v = 0.f;
   for (int i = threadIdx.x; i < n; i += 32) v += part[i];
   v = warp_sum_all(v);
-  if (threadIdx.x == 0) loss[0] = (v / (float)rows) * -1.0f;
+  if (threadIdx.x == 0) loss[0] = (v / divisor) * scale;
 }
 
 __global__ void __launch_bounds__(kThreads) sce_backward_warp_kernel(const float* __restrict__ logits, const float* __restrict__ targets,
-                                                                     const float* __restrict__ g, float* __restrict__ dlogits,
+                                                                     const float* __restrict__ g, float c, float* __restrict__ dlogits,
                                                                      float* __restrict__ dtargets, int64_t rows, int classes) {
-  const float scale = -__ldg(g) / (float)rows;
+  const float scale = g ? -__ldg(g) / (float)rows : c;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int nw = kThreads / 32;
   for (int64_t r = (int64_t)blockIdx.x * nw + warp; r < rows; r += (int64_t)gridDim.x * nw) {
@@ -1207,23 +1207,23 @@ __global__ void __launch_bounds__(kThreads) sce_backward_warp_kernel(const float
 
 }  // namespace
 
-extern "C" rt_status rt_softmax_cross_entropy(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes,
-                                              float* loss) {
+extern "C" rt_status rt_softmax_nll_scaled(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes,
+                                           float scale, float divisor, float* loss) {
   RT_CHECK_CTX(ctx);
-  if (rows <= 0 || classes <= 0) RT_FAIL(ctx, RT_ERR_EMPTY_TENSOR, "rt_softmax_cross_entropy: empty input");
+  if (rows <= 0 || classes <= 0) RT_FAIL(ctx, RT_ERR_EMPTY_TENSOR, "rt_softmax_nll: empty input");
   if (classes > 4096 || rows > (int64_t(1) << 24))
-    RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_softmax_cross_entropy: at most 4096 classes and 2^24 rows");
+    RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_softmax_nll: at most 4096 classes and 2^24 rows");
   RT_CHECK_PTR(ctx, logits);
   RT_CHECK_PTR(ctx, targets);
   RT_CHECK_PTR(ctx, loss);
   if (classes <= 16) {  // a thread per row
-    sce_forward_kernel<<<1, kThreads, 0, ctx->stream>>>(logits, targets, loss, rows, (int)classes);
+    sce_forward_kernel<<<1, kThreads, 0, ctx->stream>>>(logits, targets, loss, rows, (int)classes, scale, divisor);
     RT_LAUNCHED(ctx);
     return RT_OK;
   }
   constexpr int rows_per_block = kSceWarpBlock / 32;
   if (rows <= 8 * rows_per_block) {
-    sce_forward_warp_kernel<<<1, kSceWarpBlock, 0, ctx->stream>>>(logits, targets, loss, rows, (int)classes, 1);
+    sce_forward_warp_kernel<<<1, kSceWarpBlock, 0, ctx->stream>>>(logits, targets, loss, rows, (int)classes, 1, scale, divisor);
     RT_LAUNCHED(ctx);
     return RT_OK;
   }
@@ -1232,28 +1232,125 @@ extern "C" rt_status rt_softmax_cross_entropy(rt_ctx* ctx, const float* logits, 
   RtScratch part(ctx);
   rt_status st = part.alloc(sizeof(float) * (size_t)grid);
   if (st != RT_OK) return st;
-  sce_forward_warp_kernel<<<grid, kSceWarpBlock, 0, ctx->stream>>>(logits, targets, part.as<float>(), rows, (int)classes, 0);
+  sce_forward_warp_kernel<<<grid, kSceWarpBlock, 0, ctx->stream>>>(logits, targets, part.as<float>(), rows, (int)classes, 0, scale, divisor);
   RT_LAUNCHED(ctx);
-  sce_finish_kernel<<<1, 32, 0, ctx->stream>>>(part.as<float>(), grid, loss, rows);
+  sce_finish_kernel<<<1, 32, 0, ctx->stream>>>(part.as<float>(), grid, loss, scale, divisor);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }
 
-extern "C" rt_status rt_softmax_cross_entropy_backward(rt_ctx* ctx, const float* logits, const float* targets, const float* g,
-                                                       int64_t rows, int64_t classes, float* dlogits, float* dtargets) {
+extern "C" rt_status rt_softmax_cross_entropy(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes,
+                                              float* loss) {
+  return rt_softmax_nll_scaled(ctx, logits, targets, rows, classes, -1.f, (float)rows, loss);
+}
+
+static rt_status softmax_nll_backward(rt_ctx* ctx, const float* logits, const float* targets, const float* g, float c, int64_t rows,
+                                      int64_t classes, float* dlogits, float* dtargets) {
   RT_CHECK_CTX(ctx);
   if (rows <= 0 || classes <= 0) return RT_OK;
   if (classes > 4096) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_softmax_cross_entropy_backward: at most 4096 classes");
   RT_CHECK_PTR(ctx, logits);
   RT_CHECK_PTR(ctx, targets);
-  RT_CHECK_PTR(ctx, g);
   if (!dlogits && !dtargets) return RT_OK;
   if (classes <= 16)
-    sce_backward_kernel<<<rt_grid_for(ctx, rows, kThreads), kThreads, 0, ctx->stream>>>(logits, targets, g, dlogits, dtargets, rows,
+    sce_backward_kernel<<<rt_grid_for(ctx, rows, kThreads), kThreads, 0, ctx->stream>>>(logits, targets, g, c, dlogits, dtargets, rows,
                                                                                        (int)classes);
   else
-    sce_backward_warp_kernel<<<rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, ctx->stream>>>(logits, targets, g, dlogits,
+    sce_backward_warp_kernel<<<rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, ctx->stream>>>(logits, targets, g, c, dlogits,
                                                                                                  dtargets, rows, (int)classes);
+  RT_LAUNCHED(ctx);
+  return RT_OK;
+}
+extern "C" rt_status rt_softmax_cross_entropy_backward(rt_ctx* ctx, const float* logits, const float* targets, const float* g,
+                                                       int64_t rows, int64_t classes, float* dlogits, float* dtargets) {
+  RT_CHECK_CTX(ctx);
+  if (rows > 0 && classes > 0) RT_CHECK_PTR(ctx, g);
+  return softmax_nll_backward(ctx, logits, targets, g, 0.f, rows, classes, dlogits, dtargets);
+}
+extern "C" rt_status rt_softmax_nll_scaled_backward(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes,
+                                                    float c, float* dlogits) {
+  return softmax_nll_backward(ctx, logits, targets, nullptr, c, rows, classes, dlogits, nullptr);
+}
+
+// ---- the losses of a sequence: a stack of (logits, targets) pairs of one shape in two launches -----------------------------
+namespace {
+constexpr int kNllTerms = 200, kNllMore = 16;
+struct NllList {
+  const float *x[kNllTerms], *t[kNllTerms];
+  int64_t rows;
+  int count, classes;
+};
+// part[block] = sum over the block's rows of sum_k log_softmax * t; a warp per row
+__global__ void __launch_bounds__(kThreads) nll_list_kernel(const NllList l, float* __restrict__ part) {
+  __shared__ float smem[kThreads / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float acc = 0.f;
+  for (int64_t r = (int64_t)blockIdx.x * (kThreads / 32) + warp; r < l.rows * l.count; r += (int64_t)gridDim.x * (kThreads / 32)) {
+    const int i = (int)(r / l.rows);
+    const int64_t off = (r - i * l.rows) * l.classes;
+    const float *x = l.x[i] + off, *t = l.t[i] + off;
+    float m, lse;
+    row_max_lse_warp(x, l.classes, lane, m, lse);
+    float e = 0.f;
+    for (int k = lane; k < l.classes; k += 32) e += ((__ldg(x + k) - m) - lse) * __ldg(t + k);
+    acc += warp_sum_all(e);
+  }
+  if (lane == 0) smem[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float total = 0.f;
+    for (int w = 0; w < kThreads / 32; ++w) total += smem[w];
+    part[blockIdx.x] = total;
+  }
+}
+struct Scalars {
+  const float* p[kNllMore];
+  int n;
+};
+__global__ void __launch_bounds__(32) nll_list_finish_kernel(const float* __restrict__ part, int n, const Scalars more, float* __restrict__ loss,
+                                                             float scale, float divisor) {
+  float v = 0.f;
+  for (int i = threadIdx.x; i < n; i += 32) v += part[i];
+  v = warp_sum_all(v);
+  if (threadIdx.x == 0) {
+    v = (v / divisor) * scale;
+    for (int i = 0; i < more.n; ++i) v += *more.p[i];
+    loss[0] = v;
+  }
+}
+}  // namespace
+
+extern "C" rt_status rt_softmax_nll_list(rt_ctx* ctx, int count, const float* const* logits, const float* const* targets, int64_t rows,
+                                         int64_t classes, float scale, float divisor, int n_more, const float* const* more, float* loss) {
+  RT_CHECK_CTX(ctx);
+  if (count < 1 || rows <= 0 || classes <= 0) RT_FAIL(ctx, RT_ERR_EMPTY_TENSOR, "rt_softmax_nll_list: empty input");
+  if (classes > 4096 || rows > (int64_t(1) << 22) || n_more < 0 || n_more > kNllMore)
+    RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_softmax_nll_list: at most 4096 classes, 2^22 rows and %d scalars", kNllMore);
+  RT_CHECK_PTR(ctx, logits);
+  RT_CHECK_PTR(ctx, targets);
+  RT_CHECK_PTR(ctx, loss);
+  const int lists = (count + kNllTerms - 1) / kNllTerms;
+  const int64_t per_list = (rows * (count < kNllTerms ? count : kNllTerms) + kThreads / 32 - 1) / (kThreads / 32);
+  const int grid = (int)(per_list < 4ll * ctx->sm_count ? per_list : 4ll * ctx->sm_count);
+  RtScratch part(ctx);
+  rt_status st = part.alloc(sizeof(float) * (size_t)grid * lists);
+  if (st != RT_OK) return st;
+  for (int q = 0; q < lists; ++q) {
+    NllList l{};
+    l.rows = rows;
+    l.classes = (int)classes;
+    l.count = count - q * kNllTerms < kNllTerms ? count - q * kNllTerms : kNllTerms;
+    for (int i = 0; i < l.count; ++i) {
+      l.x[i] = logits[q * kNllTerms + i];
+      l.t[i] = targets[q * kNllTerms + i];
+    }
+    nll_list_kernel<<<grid, kThreads, 0, ctx->stream>>>(l, part.as<float>() + (size_t)q * grid);
+    RT_LAUNCHED(ctx);
+  }
+  Scalars s{};
+  s.n = n_more;
+  for (int i = 0; i < n_more; ++i) s.p[i] = more[i];
+  nll_list_finish_kernel<<<1, 32, 0, ctx->stream>>>(part.as<float>(), grid * lists, s, loss, scale, divisor);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }
