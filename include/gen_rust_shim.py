@@ -25,7 +25,7 @@ C2RUST = {
     "uint32_t": "u32", "uint64_t": "u64", "uint64_t*": "*mut u64", "size_t": "usize", "float": "f32", "float*": "*mut f32", "const float*": "*const f32",
     "double*": "*mut f64", "float* const*": "*const *mut f32", "const float* const*": "*const *const f32",
     "void*": "*mut c_void", "void**": "*mut *mut c_void", "const void*": "*const c_void", "void* const*": "*const *mut c_void",
-    "rt_upload* const*": "*const *mut RtUpload",
+    "rt_upload* const*": "*const *mut RtUpload", "const rt_fused_program*": "*const RtFusedProgram",
     "const uint8_t*": "*const u8", "uint8_t*": "*mut u8", "rt_status": "RtStatus", "const char*": "*const c_char", "void": "()",
 }
 
@@ -123,6 +123,7 @@ pub mod ffi {
     #[repr(C)] pub struct RtCtx { _p: [u8; 0] }
     #[repr(C)] pub struct RtGraph { _p: [u8; 0] }
     #[repr(C)] pub struct RtUpload { _p: [u8; 0] }
+    #[repr(C)] pub struct RtFusedProgram { _p: [u8; 0] }
     #[repr(C)] pub struct RtEvent { _p: [u8; 0] }
     pub type RtStatus = i32;
 @ENUMS@

@@ -200,6 +200,62 @@ rt_status rt_slice_assign(rt_ctx* ctx, float* dst, const int64_t* dst_shape, int
 rt_status rt_slice(rt_ctx* ctx, const float* x, const int64_t* x_shape, int ndim, const int64_t* starts,
                    const int64_t* out_shape, float* out);
 
+/* ---- one kernel for a chain of elementwise ops -------------------------------------------------------------------
+ * An expression over tensors is given as a short program that one kernel runs for every element of an iteration space of
+ * up to RT_FUSED_MAX_DIMS dimensions (row-major, outermost first).  A host that builds elementwise ops lazily (no
+ * counterpart in the reference, which launches one kernel per op) hands whole chains over in this form; every op computes
+ * exactly what its rt_unary / rt_binary entry computes.
+ *
+ * The machine has an accumulator and RT_FUSED_REGS registers per element.  Operands 0 .. n_preload-1 are loaded into
+ * registers 0 .. n_preload-1 before the first instruction (their loads are then in flight together).  An instruction
+ * computes acc = op(acc [, B]) and then, unless dst = RT_FUSED_NONE, copies acc to register dst.  B is register `src`, or the
+ * immediate when src = RT_FUSED_IMM; with `swap` set the operands of a binary op change places.
+ *   RT_F_LOAD: acc = operand src     RT_F_REG: acc = B     RT_F_OUT: out[src] = acc
+ *   RT_F_SELECT: acc = inside region `swap` ? acc : B
+ * Operands are addressed as ptr[sum of coordinate * stride]; with region != RT_FUSED_NONE an operand is only read inside
+ * that box of iteration coordinates and is 0 outside.  Outputs are contiguous over the iteration space. */
+#define RT_FUSED_MAX_DIMS 4
+#define RT_FUSED_MAX_OPERANDS 16
+#define RT_FUSED_MAX_REGIONS 8
+#define RT_FUSED_MAX_OUTPUTS 12
+#define RT_FUSED_MAX_CODE 96
+#define RT_FUSED_REGS 8
+#define RT_FUSED_PRELOAD 5 /* most operands that can be loaded up front */
+#define RT_FUSED_NONE 255
+#define RT_FUSED_IMM 254
+enum {
+  RT_F_LOAD = 0, RT_F_OUT, RT_F_SELECT, RT_F_REG,
+  /* unary */
+  RT_F_RELU, RT_F_STEP /* x > 0 */, RT_F_EXP, RT_F_LN, RT_F_SIN, RT_F_COS, RT_F_TAN, RT_F_TANH, RT_F_SIGMOID, RT_F_SOFTPLUS, RT_F_SQRT,
+  RT_F_ABS, RT_F_SIGN, RT_F_NEG, RT_F_RECIP, RT_F_ONE_MINUS_SQUARE /* 1 - x*x */, RT_F_LOGISTIC_SLOPE /* x * (1 - x) */,
+  RT_F_HALF_RSQRT /* 0.5 / sqrt(x) */, RT_F_RECIP_SQUARE /* 1 / (x*x) */, RT_F_SQUARE,
+  RT_F_ELU /* imm = alpha */, RT_F_ELU_SLOPE,
+  /* binary */
+  RT_F_ADD, RT_F_SUB, RT_F_MUL, RT_F_DIV, RT_F_POWF, RT_F_MAX, RT_F_MIN, RT_F_EQ, RT_F_NE, RT_F_GT, RT_F_GE, RT_F_LT, RT_F_LE,
+  RT_F_COUNT
+};
+typedef struct {
+  uint8_t op, src, dst, swap;
+  float imm;
+} rt_fused_instr;
+typedef struct {
+  const float* ptr;
+  int32_t stride[RT_FUSED_MAX_DIMS];
+  int32_t region;
+} rt_fused_operand;
+typedef struct {
+  int32_t lo[RT_FUSED_MAX_DIMS], hi[RT_FUSED_MAX_DIMS]; /* lo <= coordinate < hi */
+} rt_fused_region;
+typedef struct {
+  int32_t nd, n_operands, n_preload, n_regions, n_outputs, n_code;
+  int32_t shape[RT_FUSED_MAX_DIMS];
+  rt_fused_operand operand[RT_FUSED_MAX_OPERANDS];
+  rt_fused_region region[RT_FUSED_MAX_REGIONS];
+  float* out[RT_FUSED_MAX_OUTPUTS];
+  rt_fused_instr code[RT_FUSED_MAX_CODE];
+} rt_fused_program;
+rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* program);
+
 /* out[i, :] = src[idx[i], :] (idx: n_idx int32 row numbers in DEVICE memory): the row gather of data::get_random_batch
  * (src/data.rs:125-209), done on the device instead of through a host copy of the whole data set. */
 rt_status rt_gather_rows(rt_ctx* ctx, const float* src, int64_t rows, int64_t row_len, const int32_t* idx, int64_t n_idx, float* out);

@@ -162,6 +162,12 @@ struct HasAccumulatingMatmul : std::false_type {};
 template <class B>
 struct HasAccumulatingMatmul<B, std::void_t<decltype(&B::matmul_backward_accumulate)>> : std::true_type {};
 
+// Backends whose backward functions can use the forward result (kept on the Op at no cost: buffers are shared).
+template <class B, class = void>
+struct KeepsOutputs : std::false_type {};
+template <class B>
+struct KeepsOutputs<B, std::void_t<decltype(&B::relu_max_pool2d)>> : std::true_type {};
+
 template <class B>
 class Tensor {
  public:
@@ -212,6 +218,10 @@ class Tensor {
     Shape ds = B::shape(inner->data), gs = B::shape(g);
     if (ds != gs) throw Error::incompatible("add_grad on Tensor ID " + std::to_string(id()), ds, gs);
     if (inner->grad) {
+      if constexpr (KeepsOutputs<B>::value) {  // a backend that defers work may join this contribution to earlier ones
+        inner->grad = B::accumulate(std::move(*inner->grad), g);
+        return;
+      }
       Storage existing = *inner->grad;
       inner->grad = B::add(existing, g);
     } else {
@@ -479,6 +489,7 @@ Tensor<B> max_pool2d(const Tensor<B>& input, Pair kernel, Pair stride, Pair padd
       St<B> gi = B::max_pool2d_backward(op, g);
       return Grads<B>{std::move(gi), B::unused_grad(B::shape(op.inputs[1].data()))};
     }));
+    if constexpr (KeepsOutputs<B>::value) t.inner->op->cached_outputs = t.data();
   }
   return t;
 }
@@ -516,6 +527,10 @@ RT_BINARY_OP(minimum, minimum, minimum_backward, Minimum)  // src/ops/mod.rs:124
       t.set_op(Op<B>(OpType(OpType::KIND), {x}, [](const Op<B>& op, const St<B>& g) {        \
         return Grads<B>{B::bwd(op, g)};                                                      \
       }));                                                                                   \
+      if constexpr (KeepsOutputs<B>::value &&                                                \
+                    (OpType::KIND == OpType::Relu || OpType::KIND == OpType::Sigmoid ||      \
+                     OpType::KIND == OpType::Tanh || OpType::KIND == OpType::Exp))           \
+        t.inner->op->cached_outputs = t.data();                                              \
     }                                                                                        \
     return t;                                                                                \
   }
@@ -962,6 +977,7 @@ Tensor<B> fused_lstm_cell_c(const Tensor<B>& gates, const Tensor<B>& c_prev) {
         auto p = B::lstm_cell_c_backward(op, g);
         return Grads<B>{std::move(p.first), std::move(p.second)};
       }));
+      t.inner->op->cached_outputs = t.data();
     }
     return t;
   }
@@ -986,6 +1002,7 @@ Tensor<B> fused_lstm_cell_h(const Tensor<B>& gates, const Tensor<B>& c) {
         auto p = B::lstm_cell_h_backward(op, g);
         return Grads<B>{std::move(p.first), std::move(p.second)};
       }));
+      t.inner->op->cached_outputs = t.data();
     }
     return t;
   }
@@ -1061,6 +1078,21 @@ std::vector<std::pair<size_t, typename B::Storage>> collect_updates(const std::v
   return ups;
 }
 
+// All updates of a step through the backend's multi-tensor entry.
+template <class B>
+void step_all(int kind, const std::vector<Tensor<B>>& params, std::vector<typename B::Storage>* s1, std::vector<typename B::Storage>* s2, float lr,
+              float b1, float b2, float eps, float momentum, size_t t) {
+  std::vector<typename B::Storage*> p, a, b;
+  std::vector<typename B::Storage> g;
+  for (auto& u : collect_updates(params)) {
+    p.push_back(&params[u.first].data_mut());
+    g.push_back(u.second);
+    a.push_back(s1 ? &(*s1)[u.first] : nullptr);
+    b.push_back(s2 ? &(*s2)[u.first] : nullptr);
+  }
+  B::step_all(kind, p, g, a, b, lr, b1, b2, eps, momentum, t);
+}
+
 template <class B>
 void zero_grad_all(const std::vector<Tensor<B>>& params) {
   for (auto& p : params)
@@ -1074,6 +1106,7 @@ struct Sgd {
   float learning_rate;
   Sgd(std::vector<Tensor<B>> p, float lr) : parameters(std::move(p)), learning_rate(lr) {}
   void step() {
+    if constexpr (KeepsOutputs<B>::value) return step_all<B>(0, parameters, nullptr, nullptr, learning_rate, 0.f, 0.f, 0.f, 0.f, 0);
     for (auto& u : collect_updates(parameters))
       B::sgd_step(parameters[u.first].data_mut(), u.second, learning_rate);
   }
@@ -1096,6 +1129,7 @@ struct Adam {
   }
   void step() {
     t += 1;
+    if constexpr (KeepsOutputs<B>::value) return step_all<B>(1, parameters, &m_states, &v_states, learning_rate, beta1, beta2, epsilon, 0.f, t);
     for (auto& u : collect_updates(parameters))
       B::adam_step(parameters[u.first].data_mut(), u.second, m_states[u.first], v_states[u.first],
                    learning_rate, beta1, beta2, epsilon, t);
@@ -1114,6 +1148,7 @@ struct MomentumSGD {
     for (auto& x : parameters) velocities.push_back(B::zeros(x.shape()));
   }
   void step() {
+    if constexpr (KeepsOutputs<B>::value) return step_all<B>(2, parameters, &velocities, nullptr, learning_rate, 0.f, 0.f, 0.f, momentum, 0);
     for (auto& u : collect_updates(parameters))
       B::momentum_sgd_step(parameters[u.first].data_mut(), u.second, velocities[u.first], learning_rate,
                            momentum);
@@ -1132,6 +1167,7 @@ struct AdaGrad {
     for (auto& x : parameters) accumulated_sq_grad.push_back(B::zeros(x.shape()));
   }
   void step() {
+    if constexpr (KeepsOutputs<B>::value) return step_all<B>(3, parameters, &accumulated_sq_grad, nullptr, learning_rate, 0.f, 0.f, epsilon, 0.f, 0);
     for (auto& u : collect_updates(parameters))
       B::adagrad_step(parameters[u.first].data_mut(), u.second, accumulated_sq_grad[u.first], learning_rate,
                       epsilon);

@@ -9,6 +9,7 @@
 // copy the reference's `Clone` performs; the in-place mutators (optimizer steps,
 // update_from_host) first make the buffer unique.
 #pragma once
+#include <algorithm>
 #include <memory>
 #include <cmath>
 #include <optional>
@@ -18,25 +19,14 @@
 
 #include "../../../include/rt_b200.h"
 #include "autograd.hpp"
+#include "lazy.hpp"
 
 namespace rt {
-
-struct DeviceBuffer {
-  rt_ctx* ctx;
-  float* ptr;
-  size_t numel;
-  DeviceBuffer(rt_ctx* c, float* p, size_t n) : ctx(c), ptr(p), numel(n) {}
-  DeviceBuffer(const DeviceBuffer&) = delete;
-  DeviceBuffer& operator=(const DeviceBuffer&) = delete;
-  ~DeviceBuffer() {
-    if (ptr) rt_free(ctx, ptr);
-  }
-};
 
 struct DeviceStorage {
   std::shared_ptr<DeviceBuffer> buf;
   Shape shape;
-  float* ptr() const { return buf ? buf->ptr : nullptr; }
+  float* ptr() const { return buf ? buf->data() : nullptr; }  // evaluates a deferred expression
   size_t numel() const { return shape_numel(shape); }
 };
 
@@ -63,16 +53,133 @@ struct B200Backend {
     check(rt_malloc(ctx(), sizeof(float) * std::max<size_t>(n, 1), &p));
     return Storage{std::make_shared<DeviceBuffer>(ctx(), (float*)p, n), s};
   }
+  // Before a buffer is changed in place: deferred expressions that read it are evaluated, and a buffer that somebody else
+  // holds too is replaced by a copy.
   static void make_unique(Storage& s) {
-    if (s.buf && s.buf.use_count() > 1) {
+    if (!s.buf) return;
+    s.buf->data();
+    bool costly = false;  // a product or convolution that nobody has asked for yet: keep its operand instead of computing it
+    if (!s.buf->escaped)
+      for (auto* r : s.buf->readers) costly = costly || r->node->kind == lazy::Kind::Opaque;
+    if (!costly) s.buf->flush_readers();
+    if (s.buf.use_count() > 1 || s.buf->owner) {
       Storage c = alloc(s.shape);
       check(rt_memcpy_d2d(ctx(), c.ptr(), s.ptr(), sizeof(float) * s.numel()));
       s.buf = std::move(c.buf);
     }
+    s.buf->id = DeviceBuffer::next_id();
+  }
+
+  // ---- deferred elementwise ops (lazy.hpp) --------------------------------------------------------------------------
+  static bool deferrable(const Shape& s) {
+    const size_t n = shape_numel(s);
+    return n > 0 && n < ((size_t)1 << 31) && s.size() <= (size_t)lazy::kMaxRawDims;
+  }
+  static Storage defer(lazy::Node n, const Shape& shape) {
+    n.shape = shape;
+    bool now = false;
+    for (auto& i : n.in) {
+      if (i.buf->node) {
+        n.depth = std::max(n.depth, i.buf->node->depth + 1);
+        n.weight += i.buf->node->weight;
+      }
+      now = now || (i.buf->escaped && !lazy::capturing());
+    }
+    const bool scalar_sum = n.kind == lazy::Kind::Binary && n.op == RT_F_ADD && shape_numel(shape) == 1;
+    now = now || n.depth >= (scalar_sum ? lazy::kMaxChain : lazy::kMaxDepth);
+    n.weight = std::min(n.weight, 1 << 20);
+    Storage s{std::make_shared<DeviceBuffer>(ctx(), std::make_unique<lazy::Node>(std::move(n)), shape_numel(shape)), shape};
+    if (now) s.buf->data();
+    return s;
+  }
+  static lazy::Input input(const Storage& x) { return lazy::Input{x.buf, x.shape}; }
+  static bool is_const(const Storage& x) { return x.buf && x.buf->node && x.buf->node->kind == lazy::Kind::Const; }
+  static Storage lz_unary(uint8_t op, const Storage& x, float imm = 0.f) {
+    lazy::Node n{lazy::Kind::Unary};
+    n.op = op;
+    n.imm = imm;
+    n.weight = lazy::op_weight(op);
+    n.in.push_back(input(x));
+    Storage y = defer(std::move(n), x.shape);
+    y.buf->made_from = x.buf->id;
+    return y;
+  }
+  static Storage lz_imm(uint8_t op, const Storage& x, float imm, bool swap = false) {
+    if (is_const(x)) {  // both operands known: the same IEEE operation here (a loss gradient starts as a chain of these)
+      const float c = x.buf->node->imm;
+      if (op == RT_F_MUL) return filled(x.shape, c * imm);
+      if (op == RT_F_DIV && !swap) return filled(x.shape, c / imm);
+    }
+    lazy::Node n{lazy::Kind::BinaryImm};
+    n.op = op;
+    n.imm = imm;
+    n.swap = swap;
+    n.weight = lazy::op_weight(op);
+    n.in.push_back(input(x));
+    return defer(std::move(n), x.shape);
+  }
+  static Storage lz_binary(uint8_t op, const Storage& a, const Storage& b, const Shape& shape) {
+    if (is_const(a) && is_const(b) && op == RT_F_MUL) return filled(shape, a.buf->node->imm * b.buf->node->imm);
+    lazy::Node n{lazy::Kind::Binary};
+    n.op = op;
+    n.weight = lazy::op_weight(op);
+    n.in.push_back(input(a));
+    n.in.push_back(input(b));
+    return defer(std::move(n), shape);
+  }
+  static Storage lz_mul(const Storage& a, const Storage& b) { return lz_binary(RT_F_MUL, a, b, a.shape); }
+  static Storage lz_box(lazy::Kind kind, const Storage& x, const Shape& shape, Shape starts) {
+    if (kind == lazy::Kind::Broadcast && is_const(x)) return filled(shape, x.buf->node->imm);
+    lazy::Node n{kind};
+    n.starts = std::move(starts);
+    n.in.push_back(input(x));
+    return defer(std::move(n), shape);
+  }
+  // A result with a kernel of its own.  `run` gets the node and the block to fill.
+  template <class F>
+  static Storage lz_opaque(lazy::Tag tag, std::vector<int64_t> geo, std::vector<lazy::Input> in, const Shape& shape, F run) {
+    lazy::Node n{lazy::Kind::Opaque};
+    n.tag = tag;
+    n.geo = std::move(geo);
+    n.in = std::move(in);
+    n.weight = 1 << 10;
+    n.run = [run](lazy::Node& nd, DeviceBuffer* b) {
+      float* out = lazy::new_block(b->ctx, b->numel);
+      const rt_status st = run(nd, out);
+      if (st != RT_OK) {
+        rt_free(b->ctx, out);
+        check(st);
+      }
+      b->ptr = out;
+    };
+    return defer(std::move(n), shape);
+  }
+  // The address of a tensor's values for use outside the engine: whoever has it may write there at any time.
+  static float* escape(const Storage& s) {
+    if (!s.buf) return nullptr;
+    s.buf->flush_readers();
+    float* p = s.buf->data();
+    s.buf->escaped = true;
+    if (s.buf->owner) s.buf->owner->escaped = true;
+    return p;
+  }
+  static void begin_capture() {
+    lazy::flush_all();  // what was asked for before the capture must not become part of the graph
+    check(rt_graph_begin(ctx()));
+    lazy::capturing() = true;
+  }
+  static void end_capture(rt_graph** out) {
+    lazy::capturing() = false;
+    check(rt_graph_end(ctx(), out));
   }
 
   // ---- factories / access (mod.rs:44-88, 248-252) --------------------------------------
   static Storage filled(const Shape& s, float v) {
+    if (deferrable(s)) {
+      lazy::Node n{lazy::Kind::Const};
+      n.imm = v;
+      return defer(std::move(n), s);
+    }
     Storage r = alloc(s);
     check(rt_fill(ctx(), r.ptr(), v, (int64_t)r.numel()));
     return r;
@@ -165,6 +272,10 @@ struct B200Backend {
     check(rt_memcpy_h2d(ctx(), s.ptr(), d.data(), sizeof(float) * d.size()));
   }
   static void set_data(Storage& s, Storage d) { s = std::move(d); }
+  static Storage reshaped(Storage s, const Shape& shape) {
+    set_shape(s, shape);
+    return s;
+  }
   static void set_shape(Storage& s, const Shape& shape) {
     if (shape_numel(shape) != s.numel()) throw Error::shape_mismatch(shape, s.shape);
     s.shape = shape;
@@ -175,6 +286,27 @@ struct B200Backend {
 
   // ---- elementwise -----------------------------------------------------------------------
   static Storage unary(int op, const Storage& x, float p0 = 0.f, float p1 = 0.f) {
+    if (deferrable(x.shape)) {
+      switch (op) {
+        case RT_RELU: return lz_unary(RT_F_RELU, x);
+        case RT_ELU: return lz_unary(RT_F_ELU, x, p0);
+        case RT_EXP: return lz_unary(RT_F_EXP, x);
+        case RT_LN: return lz_unary(RT_F_LN, x);
+        case RT_SIN: return lz_unary(RT_F_SIN, x);
+        case RT_COS: return lz_unary(RT_F_COS, x);
+        case RT_TAN: return lz_unary(RT_F_TAN, x);
+        case RT_TANH: return lz_unary(RT_F_TANH, x);
+        case RT_SIGMOID: return lz_unary(RT_F_SIGMOID, x);
+        case RT_SOFTPLUS: return lz_unary(RT_F_SOFTPLUS, x);
+        case RT_SQUARE: return lz_unary(RT_F_SQUARE, x);
+        case RT_SQRT: return lz_unary(RT_F_SQRT, x);
+        case RT_ABS: return lz_unary(RT_F_ABS, x);
+        case RT_CLIP: return lz_imm(RT_F_MIN, lz_imm(RT_F_MAX, x, p0), p1);
+        case RT_MUL_SCALAR: return lz_imm(RT_F_MUL, x, p0);
+        case RT_DIV_SCALAR: return lz_imm(RT_F_DIV, x, p0);
+        default: break;
+      }
+    }
     Storage y = alloc(x.shape);
     check(rt_unary(ctx(), op, x.ptr(), y.ptr(), (int64_t)x.numel(), p0, p1));
     return y;
@@ -183,6 +315,36 @@ struct B200Backend {
     if (o.inputs.empty()) throw Error::invalid_op("backward requires 1 input");
     const Storage& x = o.inputs[0].data();
     if (x.shape != g.shape) throw Error::shape_mismatch(x.shape, g.shape);
+    if (deferrable(x.shape)) {  // g * f'(x), each f' in the form of the stand-alone kernel
+      // where f' follows from f(x), which the forward pass has (unless x has been changed since)
+      if (o.cached_outputs && o.cached_outputs->buf && o.cached_outputs->buf->made_from == x.buf->id && (!x.buf->escaped || lazy::capturing())) {
+        const Storage& y = *o.cached_outputs;
+        switch (op) {
+          case RT_RELU: return lz_mul(g, lz_unary(RT_F_STEP, y));
+          case RT_EXP: return lz_mul(g, y);
+          case RT_TANH: return lz_mul(g, lz_unary(RT_F_ONE_MINUS_SQUARE, y));
+          case RT_SIGMOID: return lz_mul(g, lz_unary(RT_F_LOGISTIC_SLOPE, y));
+          default: break;
+        }
+      }
+      switch (op) {
+        case RT_RELU: return lz_mul(g, lz_unary(RT_F_STEP, x));
+        case RT_ELU: return lz_mul(g, lz_unary(RT_F_ELU_SLOPE, x, p0));
+        case RT_EXP: return lz_mul(g, lz_unary(RT_F_EXP, x));
+        case RT_LN: return lz_mul(g, lz_unary(RT_F_RECIP, x));
+        case RT_SIN: return lz_mul(lz_unary(RT_F_COS, x), g);
+        case RT_COS: return lz_mul(lz_unary(RT_F_NEG, lz_unary(RT_F_SIN, x)), g);
+        case RT_TAN: return lz_mul(g, lz_unary(RT_F_RECIP_SQUARE, lz_unary(RT_F_COS, x)));
+        case RT_TANH: return lz_mul(g, lz_unary(RT_F_ONE_MINUS_SQUARE, lz_unary(RT_F_TANH, x)));
+        case RT_SIGMOID: return lz_mul(g, lz_unary(RT_F_LOGISTIC_SLOPE, lz_unary(RT_F_SIGMOID, x)));
+        case RT_SOFTPLUS: return lz_mul(g, lz_unary(RT_F_SIGMOID, x));
+        case RT_SQUARE: return lz_mul(g, lz_imm(RT_F_MUL, x, 2.f));
+        case RT_SQRT: return lz_mul(g, lz_unary(RT_F_HALF_RSQRT, x));
+        case RT_ABS: return lz_mul(g, lz_unary(RT_F_SIGN, x));
+        case RT_CLIP: return lz_mul(g, lz_mul(lz_imm(RT_F_GE, x, p0), lz_imm(RT_F_LE, x, p1)));
+        default: break;
+      }
+    }
     Storage dx = alloc(x.shape);
     check(rt_unary_backward(ctx(), op, x.ptr(), g.ptr(), dx.ptr(), (int64_t)x.numel(), p0, p1));
     return dx;
@@ -207,11 +369,32 @@ struct B200Backend {
   }
   static bool is_operator_op(int op) { return op == RT_SUB || op == RT_DIV; }
   static Storage binary(int op, const Storage& a, const Storage& b, const char* name) {
-    Storage out = alloc(bshape(a.shape, b.shape, name, is_operator_op(op)));
+    const Shape os = bshape(a.shape, b.shape, name, is_operator_op(op));
+    if (deferrable(os)) return lz_binary((uint8_t)(RT_F_ADD + (op - RT_ADD)), a, b, os);
+    Storage out = alloc(os);
     auto as = dims(a.shape), bs = dims(b.shape);
     check(rt_binary(ctx(), op, a.ptr(), as.data(), (int)as.size(), b.ptr(), bs.data(), (int)bs.size(), out.ptr()));
     return out;
   }
+  // d/da (or d/db) of a binary op times g, over g's shape, in the form of the stand-alone kernels
+  static Storage binary_term(int op, const Storage& a, const Storage& b, const Storage& g, bool second) {
+    const Shape& s = g.shape;
+    switch (op) {
+      case RT_ADD: return g;
+      case RT_SUB: return second ? lz_unary(RT_F_NEG, g) : g;
+      case RT_MUL: return lz_binary(RT_F_MUL, g, second ? a : b, s);
+      case RT_DIV:
+        if (!second) return lz_binary(RT_F_MUL, g, lz_unary(RT_F_RECIP, b), s);
+        return lz_mul(g, lz_unary(RT_F_NEG, lz_binary(RT_F_DIV, a, lz_binary(RT_F_MUL, b, b, b.shape), s)));
+      case RT_POWF:
+        if (!second) return lz_mul(g, lz_binary(RT_F_MUL, b, lz_binary(RT_F_POWF, a, lz_imm(RT_F_SUB, b, 1.f), s), s));
+        return lz_mul(g, lz_binary(RT_F_MUL, lz_binary(RT_F_POWF, a, b, s), lz_unary(RT_F_LN, a), s));
+      case RT_MAXIMUM: return lz_mul(g, second ? lz_binary(RT_F_GT, b, a, s) : lz_binary(RT_F_GE, a, b, s));
+      case RT_MINIMUM: return lz_mul(g, second ? lz_binary(RT_F_LT, b, a, s) : lz_binary(RT_F_LE, a, b, s));
+      default: return filled(s, 0.f);  // comparisons
+    }
+  }
+  static Storage reduced(const Storage& term, const Shape& target) { return unbroadcast(term, target); }
   static std::pair<Storage, Storage> binary_bwd(int op, const OpB& o, const Storage& g, const char* name) {
     if (o.inputs.size() != 2) throw Error::invalid_op(std::string(name) + " requires 2 inputs");
     const Storage& a = o.inputs[0].data();
@@ -219,6 +402,14 @@ struct B200Backend {
     Shape os = bshape(a.shape, b.shape, name, is_operator_op(op));
     if (g.numel() != shape_numel(os)) throw Error::incompatible(name, os, g.shape);
     bool need_a = o.inputs[0].requires_grad(), need_b = o.inputs[1].requires_grad();
+    if (deferrable(os)) {
+      // each term over the full shape; the side that was stretched is then summed down to its own shape
+      Storage gf = g;
+      set_shape(gf, os);
+      Storage da = need_a ? reduced(binary_term(op, a, b, gf, false), a.shape) : Storage{nullptr, a.shape};
+      Storage db = need_b ? reduced(binary_term(op, a, b, gf, true), b.shape) : Storage{nullptr, b.shape};
+      return {std::move(da), std::move(db)};
+    }
     Storage da = need_a ? alloc(a.shape) : Storage{nullptr, a.shape};
     Storage db = need_b ? alloc(b.shape) : Storage{nullptr, b.shape};
     auto as = dims(a.shape), bs = dims(b.shape);
@@ -255,12 +446,10 @@ struct B200Backend {
     if (o.inputs.size() == 2 && o.inputs[0].data().shape == g.shape && g.numel() > 0 && stretches_onto(o.inputs[1].data().shape, g.shape)) {
       const Shape& bs = o.inputs[1].data().shape;
       const auto& bias = o.inputs[1];
-      if (bias.requires_grad() && bias.grad() && g.shape.size() == 2 && bs.size() == 1 && bs[0] == g.shape[1] && g.shape[0] <= 1024 &&
+      if (bias.requires_grad() && bias.grad() && deferrable(g.shape) && g.shape.size() == 2 && bs.size() == 1 && bs[0] == g.shape[1] &&
           bias.grad()->shape == bs) {
-        // the bias already holds a gradient (it is used at every timestep): add this one's column sums to it in place
-        Storage& acc = bias.grad_mut();
-        make_unique(acc);
-        check(rt_sum_rows_accumulate(ctx(), g.ptr(), (int64_t)g.shape[0], (int64_t)g.shape[1], acc.ptr()));
+        // the bias already holds a gradient (it is used at every timestep): this one's column sums join a list that is added in one go
+        append_terms(bias.grad_mut(), lazy::Tag::SumRows, {input(g)}, {(int64_t)g.shape[0], (int64_t)g.shape[1]}, run_sum_rows);
         return {g, unused_grad(bs)};
       }
       return {g, bias.requires_grad() ? unbroadcast(g, bs) : unused_grad(bs)};
@@ -330,6 +519,10 @@ struct B200Backend {
     size_t off = shape.size() - x.shape.size();
     for (size_t i = 0; i < x.shape.size(); ++i)
       if (x.shape[i] != shape[i + off] && x.shape[i] != 1) throw Error::incompatible("broadcast", x.shape, shape);
+    if (deferrable(shape)) {
+      if (x.shape == shape) return x;
+      return lz_box(lazy::Kind::Broadcast, x, shape, {});
+    }
     Storage y = alloc(shape);
     auto xs = dims(x.shape), os = dims(shape);
     check(rt_broadcast_to(ctx(), x.ptr(), xs.data(), (int)xs.size(), os.data(), (int)os.size(), y.ptr()));
@@ -349,6 +542,12 @@ struct B200Backend {
       }
       throw Error::incompatible("unbroadcast (final shape/size)", g.shape, target);
     }
+    if (deferrable(g.shape) && deferrable(t) && gs.size() == 2 && shape_numel(t) == g.shape[1] && !t.empty() && t.back() == g.shape[1])
+      // the column sums of a matrix (the gradient of a bias): deferred, because a bias that is used again takes more of them
+      return lz_opaque(lazy::Tag::SumRows, {-1}, {input(g)}, t, [](lazy::Node& n, float* o) {
+        const int64_t gd[2] = {(int64_t)n.in[0].shape[0], (int64_t)n.in[0].shape[1]}, td[1] = {gd[1]};
+        return rt_unbroadcast(ctx(), n.in[0].buf->data(), gd, 2, td, 1, o);
+      });
     Storage out = alloc(t);
     check(rt_unbroadcast(ctx(), g.ptr(), gs.data(), (int)gs.size(), ts.data(), (int)ts.size(), out.ptr()));
     return out;
@@ -361,6 +560,7 @@ struct B200Backend {
       os[i] = ranges[i].end - ranges[i].start;
       starts[i] = (int64_t)ranges[i].start;
     }
+    if (deferrable(os) && deferrable(x.shape)) return lz_box(lazy::Kind::Slice, x, os, Shape(starts.begin(), starts.end()));
     Storage y = alloc(os);
     auto xs = dims(x.shape), od = dims(os);
     check(rt_slice(ctx(), x.ptr(), xs.data(), (int)xs.size(), starts.data(), od.data(), y.ptr()));
@@ -376,6 +576,11 @@ struct B200Backend {
       gs.push_back(r.end - r.start);
     }
     if (shape_numel(gs) != g.numel()) throw Error::incompatible("slice_backward", gs, g.shape);
+    if (deferrable(is) && deferrable(gs)) {
+      Storage gb = g;
+      set_shape(gb, gs);
+      return lz_box(lazy::Kind::Pad, gb, is, Shape(starts.begin(), starts.end()));
+    }
     Storage dx = zeros(is);
     auto id = dims(is), gd = dims(gs);
     check(rt_slice_assign(ctx(), dx.ptr(), id.data(), (int)id.size(), starts.data(), g.ptr(), gd.data()));
@@ -393,6 +598,14 @@ struct B200Backend {
       total += x->shape[axis];
     }
     os[axis] = total;
+    bool defers = deferrable(os) && xs.size() <= 4;  // each piece costs a region of the program
+    for (auto* x : xs) defers = defers && x->numel() > 0;
+    if (defers) {
+      lazy::Node n{lazy::Kind::Concat};
+      n.starts = Shape{axis};
+      for (auto* x : xs) n.in.push_back(input(*x));
+      return defer(std::move(n), os);
+    }
     Storage y = alloc(os);
     auto od = dims(os);
     std::vector<int64_t> starts(os.size(), 0);
@@ -409,6 +622,10 @@ struct B200Backend {
     if (x.shape.size() != 2 || h.shape.size() != 2 || r0 > r1 || r1 > x.shape[0] || h.shape[0] != r1 - r0)
       throw Error(ErrorKind::ShapeError, "concat_rows_with: incompatible shapes");
     Shape os{r1 - r0, x.shape[1] + h.shape[1]};
+    if (deferrable(os) && r1 > r0 && x.shape[1] > 0 && h.shape[1] > 0) {
+      const Storage rows = slice(x, {{r0, r1}, {0, x.shape[1]}});
+      return concat({&rows, &h}, 1);
+    }
     Storage y = alloc(os);
     auto od = dims(os);
     std::vector<int64_t> starts{0, 0};
@@ -499,6 +716,10 @@ struct B200Backend {
   }
   static Storage reduce(int kind, const Storage& x, std::optional<size_t> axis) {
     Axis3 a = split(x.shape, axis);
+    if ((kind == RT_RED_SUM || kind == RT_RED_MEAN) && deferrable(x.shape))
+      return lz_opaque(lazy::Tag::Reduce, {kind, axis ? (int64_t)*axis : -1}, {input(x)}, a.out_shape, [a, kind](lazy::Node& n, float* out) {
+        return rt_reduce(ctx(), kind, n.in[0].buf->data(), a.outer, a.len, a.inner, out);
+      });
     Storage out = alloc(a.out_shape);
     check(rt_reduce(ctx(), kind, x.ptr(), a.outer, a.len, a.inner, out.ptr()));
     return out;
@@ -532,6 +753,10 @@ struct B200Backend {
   static Storage argmin(const Storage& x, size_t axis) { return reduce_or_empty(RT_RED_ARGMIN, x, axis); }
   static Storage log_softmax(const Storage& x, size_t axis) {
     Axis3 a = split(x.shape, axis);
+    if (deferrable(x.shape))
+      return lz_opaque(lazy::Tag::LogSoftmax, {(int64_t)axis}, {input(x)}, x.shape, [a](lazy::Node& n, float* out) {
+        return rt_log_softmax(ctx(), n.in[0].buf->data(), a.outer, a.len, a.inner, out);
+      });
     Storage y = alloc(x.shape);
     check(rt_log_softmax(ctx(), x.ptr(), a.outer, a.len, a.inner, y.ptr()));
     return y;
@@ -547,9 +772,23 @@ struct B200Backend {
   }
   static Storage sum_backward(const OpB& o, const Storage& g) {
     if (!o.op_type.axis && !g.shape.empty()) throw Error::shape_mismatch(Shape{}, g.shape);  // cpu.rs:1480-1485
-    return reduce_bwd(RT_RED_SUM, o, g, "sum");
+    return spread(RT_RED_SUM, o, g, "sum");
   }
-  static Storage mean_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_MEAN, o, g, "mean"); }
+  static Storage mean_backward(const OpB& o, const Storage& g) { return spread(RT_RED_MEAN, o, g, "mean"); }
+  // Gradient of a sum or mean: the upstream gradient repeated along the reduced axis (divided by its length for a mean).
+  static Storage spread(int kind, const OpB& o, const Storage& g, const char* name) {
+    if (o.inputs.size() != 1) throw Error::invalid_op(std::string(name) + " backward expects 1 input");
+    const Storage& x = o.inputs[0].data();
+    Axis3 a = split(x.shape, o.op_type.axis);
+    if ((int64_t)g.numel() != a.outer * a.inner) throw Error::incompatible(name, x.shape, g.shape);
+    if (!deferrable(x.shape)) return reduce_bwd(kind, o, g, name);
+    Storage gs = g;
+    Shape one = o.op_type.axis ? x.shape : Shape{};
+    if (o.op_type.axis) one[*o.op_type.axis] = 1;
+    gs = reshaped(gs, one);
+    Storage scaled = kind == RT_RED_MEAN ? lz_imm(RT_F_DIV, gs, (float)a.len) : gs;
+    return one == x.shape ? scaled : lz_box(lazy::Kind::Broadcast, scaled, x.shape, {});
+  }
   static Storage max_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_MAX, o, g, "max"); }
   static Storage min_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_MIN, o, g, "min"); }
   static Storage prod_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_PROD, o, g, "prod"); }
@@ -560,6 +799,16 @@ struct B200Backend {
     Axis3 a = split(x.shape, o.op_type.axis);
     if (g.shape != x.shape) throw Error::shape_mismatch(x.shape, g.shape);
     Storage dx = alloc(x.shape);
+    // upstream = constant * targets (a classification loss): without the product in memory
+    float c;
+    if (g.buf && g.buf->node && a.inner == 1 && a.len <= 4096)
+      if (const lazy::Input* t = lazy::times_constant(g.buf->node.get(), &c)) {
+        const float* tp = t->buf->data();
+        if (g.buf->node) {
+          check(rt_softmax_nll_scaled_backward(ctx(), x.ptr(), tp, a.outer, a.len, c, dx.ptr()));
+          return dx;
+        }
+      }
     check(rt_log_softmax_backward(ctx(), x.ptr(), g.ptr(), a.outer, a.len, a.inner, dx.ptr()));
     return dx;
   }
@@ -570,6 +819,15 @@ struct B200Backend {
     if (b.shape.size() != 2) throw Error(ErrorKind::ShapeError, "Input 'b' is not 2D");
     if (a.shape[1] != b.shape[0]) throw Error::incompatible("matmul", a.shape, b.shape);
     int64_t m = (int64_t)a.shape[0], k = (int64_t)a.shape[1], n = (int64_t)b.shape[1];
+    if (k > 0 && deferrable(Shape{a.shape[0], b.shape[1]})) {
+      // the operands are evaluated now (expressions do not grow through products); the product itself may still join a bias, an
+      // activation, or its siblings
+      a.ptr();
+      b.ptr();
+      return lz_opaque(lazy::Tag::Matmul, {}, {input(a), input(b)}, Shape{a.shape[0], b.shape[1]}, [m, n, k](lazy::Node& nd, float* out) {
+        return rt_gemm(ctx(), 0, 0, m, n, k, nd.in[0].buf->data(), k, nd.in[1].buf->data(), n, out, n, 0);
+      });
+    }
     Storage c = alloc(Shape{a.shape[0], b.shape[1]});
     check(rt_gemm(ctx(), 0, 0, m, n, k, a.ptr(), k, b.ptr(), n, c.ptr(), n, 0));
     return c;
@@ -596,14 +854,77 @@ struct B200Backend {
     if (g.shape != Shape{a.shape[0], b.shape[1]}) throw Error::incompatible("matmul", g.shape, b.shape);
     if (acc.shape != b.shape) throw Error::shape_mismatch(b.shape, acc.shape);
     Storage da = o.inputs[0].requires_grad() ? alloc(a.shape) : Storage{nullptr, a.shape};
+    if (deferrable(a.shape) && deferrable(g.shape) && deferrable(b.shape)) {
+      // the weight's gradient is a sum over all its uses: the products are collected and computed as one with a longer reduction
+      append_terms(acc, lazy::Tag::SumProducts, {input(a), input(g)}, {m, k, n}, run_sum_products);
+      if (da.buf) check(rt_gemm(ctx(), 0, 1, m, k, n, g.ptr(), n, b.ptr(), n, da.ptr(), k, 0));
+      return da;
+    }
     make_unique(acc);  // nobody else may see the sum appear in a buffer they share
     check(rt_matmul_backward_accumulate(ctx(), a.ptr(), b.ptr(), g.ptr(), m, k, n, da.ptr(), acc.ptr()));
     return da;
   }
   static bool is_accumulated(const Storage& s) { return !s.buf; }
-  // the accumulating epilogue of the product works on 128-bit pieces of a row; other widths keep product + addition
-  static bool accumulates_well(const Storage& b) { return b.shape.size() == 2 && b.shape[1] % 4 == 0; }
+  static bool accumulates_well(const Storage& b) { return b.shape.size() == 2 && (deferrable(b.shape) || b.shape[1] % 4 == 0); }
 
+  // acc += a term that is computed later, together with the others of its kind.  Node: in[0] is what was there before.
+  static constexpr size_t kMaxTerms = 192;
+  static void append_terms(Storage& acc, lazy::Tag tag, std::vector<lazy::Input> term, std::vector<int64_t> geo,
+                           void (*run)(lazy::Node&, DeviceBuffer*)) {
+    DeviceBuffer* b = acc.buf.get();
+    if (b->node && b->node->tag == tag && b->node->geo == geo && acc.buf.use_count() == 1 && b->readers.empty() &&
+        b->node->in.size() + term.size() <= 1 + kMaxTerms) {
+      for (auto& t : term) {
+        t.buf->readers.push_back(b);
+        b->node->in.push_back(std::move(t));
+      }
+      return;
+    }
+    acc.buf->data();
+    lazy::Node n{lazy::Kind::Opaque};
+    n.tag = tag;
+    n.geo = std::move(geo);
+    n.weight = 1 << 10;
+    n.in.push_back(input(acc));
+    for (auto& t : term) n.in.push_back(std::move(t));
+    n.run = run;
+    const Shape s = acc.shape;
+    acc = Storage{};  // the node now holds the old values, alone unless somebody else does too
+    acc = defer(std::move(n), s);
+  }
+  // The block in which a sum goes on: the old values' own one when nobody else needs it.
+  static float* sum_block(lazy::Node& n, DeviceBuffer* b) {
+    DeviceBuffer* base = n.in[0].buf.get();
+    if (n.in[0].buf.use_count() == 1 && !base->escaped && !base->owner) return std::exchange(base->ptr, nullptr);
+    float* out = lazy::new_block(b->ctx, b->numel);
+    check(rt_memcpy_d2d(ctx(), out, base->data(), sizeof(float) * b->numel));
+    return out;
+  }
+  static void run_sum_products(lazy::Node& n, DeviceBuffer* b) {
+    std::vector<const float*> as, gs;
+    for (size_t i = 1; i < n.in.size(); i += 2) {
+      as.push_back(n.in[i].buf->data());
+      gs.push_back(n.in[i + 1].buf->data());
+    }
+    b->ptr = sum_block(n, b);
+    check(rt_gemm_sum_products(ctx(), (int)as.size(), as.data(), gs.data(), n.geo[0], n.geo[1], n.geo[2], b->ptr));
+  }
+  // existing + g for a gradient that receives another contribution (Tensor::add_grad).
+  static Storage accumulate(Storage existing, const Storage& g) {
+    const lazy::Node* n = g.buf ? g.buf->node.get() : nullptr;
+    if (n && n->tag == lazy::Tag::SumRows && n->geo[0] < 0 && g.buf->readers.empty() && g.shape.size() == 1 && existing.buf && existing.shape == g.shape) {
+      const lazy::Input x = n->in[0];
+      append_terms(existing, lazy::Tag::SumRows, {x}, {(int64_t)x.shape[0], (int64_t)x.shape[1]}, run_sum_rows);
+      return existing;
+    }
+    return add(existing, g);
+  }
+  static void run_sum_rows(lazy::Node& n, DeviceBuffer* b) {
+    std::vector<const float*> xs;
+    for (size_t i = 1; i < n.in.size(); ++i) xs.push_back(n.in[i].buf->data());
+    b->ptr = sum_block(n, b);
+    check(rt_sum_rows_accumulate_list(ctx(), (int)xs.size(), xs.data(), n.geo[0], n.geo[1], b->ptr));
+  }
   static void conv_shapes(const Storage& x, const Storage& w, const char* name) {
     if (x.shape.size() != 4 || w.shape.size() != 4) throw Error::invalid_op(std::string(name) + " expects 4D input and weights");
   }
@@ -612,7 +933,21 @@ struct B200Backend {
     if (x.shape[1] != w.shape[1]) throw Error::invalid_op("conv2d: input channels != weight channels");
     if (bias && bias->numel() != w.shape[0]) throw Error::invalid_op("conv2d: bias shape mismatch");
     size_t ho = (x.shape[2] + 2 * p.first - w.shape[2]) / s.first + 1, wo = (x.shape[3] + 2 * p.second - w.shape[3]) / s.second + 1;
-    Storage y = alloc(Shape{x.shape[0], w.shape[0], ho, wo});
+    const Shape ys{x.shape[0], w.shape[0], ho, wo};
+    if (deferrable(ys) && deferrable(x.shape) && deferrable(w.shape)) {
+      x.ptr();
+      w.ptr();
+      std::vector<lazy::Input> in{input(x), input(w)};
+      if (bias) in.push_back(input(*bias));
+      const std::vector<int64_t> q{(int64_t)x.shape[0], (int64_t)x.shape[1], (int64_t)x.shape[2], (int64_t)x.shape[3], (int64_t)w.shape[0],
+                                   (int64_t)w.shape[2], (int64_t)w.shape[3], (int64_t)s.first, (int64_t)s.second, (int64_t)p.first, (int64_t)p.second};
+      return lz_opaque(lazy::Tag::Conv, q, std::move(in), ys, [](lazy::Node& n, float* out) {
+        const auto& q = n.geo;
+        return rt_conv2d(ctx(), n.in[0].buf->data(), n.in[1].buf->data(), n.in.size() > 2 ? n.in[2].buf->data() : nullptr, q[0], q[1], q[2], q[3],
+                         q[4], (int)q[5], (int)q[6], (int)q[7], (int)q[8], (int)q[9], (int)q[10], out);
+      });
+    }
+    Storage y = alloc(ys);
     check(rt_conv2d(ctx(), x.ptr(), w.ptr(), bias ? bias->ptr() : nullptr, (int64_t)x.shape[0], (int64_t)x.shape[1],
                     (int64_t)x.shape[2], (int64_t)x.shape[3], (int64_t)w.shape[0], (int)w.shape[2], (int)w.shape[3],
                     (int)s.first, (int)s.second, (int)p.first, (int)p.second, y.ptr()));
@@ -693,6 +1028,23 @@ struct B200Backend {
     if (x.shape.size() != 4) throw Error::invalid_op("max_pool2d expects 4D input (NCHW)");
     size_t ho = (x.shape[2] + 2 * p.first - k.first) / s.first + 1, wo = (x.shape[3] + 2 * p.second - k.second) / s.second + 1;
     Shape os{x.shape[0], x.shape[1], ho, wo};
+    if (const lazy::Node* act = x.buf ? x.buf->node.get() : nullptr; lazy::is_op(act, lazy::Kind::Unary, RT_F_RELU) && act->shape == x.shape) {
+      // relu in front of the pooling, its result not in memory: both in one kernel, with the convolution below it where that has one
+      const lazy::Input pre = act->in[0];
+      const lazy::Node* cv = lazy::tagged(pre, lazy::Tag::Conv);
+      Storage y = alloc(os), idx = alloc(os);
+      const bool halves = k == Pair{2, 2} && s == Pair{2, 2} && p == Pair{0, 0} && x.shape[2] % 2 == 0 && x.shape[3] % 2 == 0;
+      if (cv && halves && pre.buf->readers.size() == 1) {
+        const auto& q = cv->geo;
+        const float *px = cv->in[0].buf->data(), *pw = cv->in[1].buf->data(), *pb = cv->in.size() > 2 ? cv->in[2].buf->data() : nullptr;
+        check(rt_conv2d_relu_max_pool2x2(ctx(), px, pw, pb, q[0], q[1], q[2], q[3], q[4], (int)q[5], (int)q[6], (int)q[7], (int)q[8], (int)q[9],
+                                         (int)q[10], y.ptr(), idx.ptr()));
+      } else {
+        check(rt_relu_max_pool2d(ctx(), pre.buf->data(), (int64_t)x.shape[0], (int64_t)x.shape[1], (int64_t)x.shape[2], (int64_t)x.shape[3],
+                                 (int)k.first, (int)k.second, (int)s.first, (int)s.second, (int)p.first, (int)p.second, y.ptr(), idx.ptr()));
+      }
+      return {std::move(y), std::move(idx)};
+    }
     Storage y = alloc(os), idx = alloc(os);
     check(rt_max_pool2d(ctx(), x.ptr(), (int64_t)x.shape[0], (int64_t)x.shape[1], (int64_t)x.shape[2], (int64_t)x.shape[3],
                         (int)k.first, (int)k.second, (int)s.first, (int)s.second, (int)p.first, (int)p.second, y.ptr(),
@@ -706,6 +1058,19 @@ struct B200Backend {
     const Storage& idx = o.inputs[1].data();
     if (g.numel() != idx.numel()) throw Error::shape_mismatch(idx.shape, g.shape);
     Pair k = o.op_type.kernel_size, s = o.op_type.stride, p = o.op_type.padding;
+    const bool halves = k == Pair{2, 2} && s == Pair{2, 2} && p == Pair{0, 0} && is[2] % 2 == 0 && is[3] % 2 == 0;
+    if (deferrable(is) && g.numel() > 0) {
+      std::vector<lazy::Input> in{input(g), input(idx)};
+      const Storage& x = o.inputs[0].data();
+      if (halves && o.cached_outputs && lazy::is_op(x.buf->node.get(), lazy::Kind::Unary, RT_F_RELU)) in.push_back(input(*o.cached_outputs));
+      std::vector<int64_t> q{(int64_t)is[0], (int64_t)is[1], (int64_t)is[2], (int64_t)is[3], (int64_t)k.first, (int64_t)k.second,
+                             (int64_t)s.first, (int64_t)s.second, (int64_t)p.first, (int64_t)p.second, (int64_t)(intptr_t)x.buf.get()};
+      return lz_opaque(lazy::Tag::PoolGrad, std::move(q), std::move(in), is, [](lazy::Node& n, float* out) {
+        const auto& q = n.geo;
+        return rt_max_pool2d_backward(ctx(), n.in[0].buf->data(), n.in[1].buf->data(), q[0], q[1], q[2], q[3], (int)q[4], (int)q[5], (int)q[6],
+                                      (int)q[7], (int)q[8], (int)q[9], out);
+      });
+    }
     Storage dx = alloc(is);
     check(rt_max_pool2d_backward(ctx(), g.ptr(), idx.ptr(), (int64_t)is[0], (int64_t)is[1], (int64_t)is[2], (int64_t)is[3],
                                  (int)k.first, (int)k.second, (int)s.first, (int)s.second, (int)p.first, (int)p.second,
@@ -755,7 +1120,28 @@ struct B200Backend {
     return {std::move(dl), std::move(dt)};
   }
 
+  // Column block i of the [batch, 4 * hidden] gate pre-activations, activated; and a gradient put back into its block.
+  static Storage gate(const Storage& gates, const Shape& s, size_t i, uint8_t act) {
+    return lz_unary(act, lz_box(lazy::Kind::Slice, gates, s, Shape{0, i * s[1]}));
+  }
+  // What the forward pass has kept of a cell, unless the gates have been changed since.
+  static bool keeps(const OpB& o, const Storage& gates) {
+    return o.cached_outputs && o.cached_outputs->buf && !o.cached_outputs->buf->saved.empty() && o.cached_outputs->buf->made_from == gates.buf->id &&
+           (!gates.buf->escaped || lazy::capturing());
+  }
+  static Storage saved_gate(const OpB& o, size_t k, const Storage& gates, const Shape& s, size_t i, uint8_t act) {
+    return keeps(o, gates) ? Storage{o.cached_outputs->buf->saved[k], s} : gate(gates, s, i, act);
+  }
+  static Storage to_gate(const Storage& g, const Shape& gates, size_t i) { return lz_box(lazy::Kind::Pad, g, gates, Shape{0, i * g.shape[1]}); }
   static Storage lstm_cell_c(const Storage& gates, const Storage& c_prev) {
+    if (deferrable(gates.shape) && deferrable(c_prev.shape)) {  // joins the ops around it in one launch
+      const Shape& s = c_prev.shape;
+      const Storage i = gate(gates, s, 0, RT_F_SIGMOID), f = gate(gates, s, 1, RT_F_SIGMOID), gg = gate(gates, s, 2, RT_F_TANH);
+      Storage c = lz_binary(RT_F_ADD, lz_mul(f, c_prev), lz_mul(i, gg), s);
+      c.buf->made_from = gates.buf->id;
+      c.buf->saved = {i.buf, f.buf, gg.buf};
+      return c;
+    }
     Storage c = alloc(c_prev.shape);
     check(rt_lstm_cell_c(ctx(), gates.ptr(), c_prev.ptr(), (int64_t)c_prev.shape[0], (int64_t)c_prev.shape[1], c.ptr()));
     return c;
@@ -765,6 +1151,20 @@ struct B200Backend {
     const Storage& c_prev = o.inputs[1].data();
     if (g.shape != c_prev.shape) throw Error::shape_mismatch(c_prev.shape, g.shape);
     const bool ng = o.inputs[0].requires_grad(), nc = o.inputs[1].requires_grad();
+    if (deferrable(gates.shape) && deferrable(g.shape)) {
+      const Shape &s = g.shape, &gs = gates.shape;
+      const Storage i = saved_gate(o, 0, gates, s, 0, RT_F_SIGMOID), f = saved_gate(o, 1, gates, s, 1, RT_F_SIGMOID),
+                    gg = saved_gate(o, 2, gates, s, 2, RT_F_TANH);
+      Storage dgates = unused_grad(gs), dprev = unused_grad(s);
+      if (ng) {
+        const Storage di = to_gate(lz_mul(lz_mul(g, gg), lz_unary(RT_F_LOGISTIC_SLOPE, i)), gs, 0);
+        const Storage df = to_gate(lz_mul(lz_mul(g, c_prev), lz_unary(RT_F_LOGISTIC_SLOPE, f)), gs, 1);
+        const Storage dg = to_gate(lz_mul(lz_mul(g, i), lz_unary(RT_F_ONE_MINUS_SQUARE, gg)), gs, 2);
+        dgates = lz_binary(RT_F_ADD, lz_binary(RT_F_ADD, di, df, gs), dg, gs);
+      }
+      if (nc) dprev = lz_mul(g, f);
+      return {std::move(dgates), std::move(dprev)};
+    }
     Storage dg = ng ? alloc(gates.shape) : unused_grad(gates.shape);
     Storage dc = nc ? alloc(c_prev.shape) : unused_grad(c_prev.shape);
     check(rt_lstm_cell_c_backward(ctx(), gates.ptr(), c_prev.ptr(), g.ptr(), (int64_t)c_prev.shape[0], (int64_t)c_prev.shape[1],
@@ -772,6 +1172,13 @@ struct B200Backend {
     return {std::move(dg), std::move(dc)};
   }
   static Storage lstm_cell_h(const Storage& gates, const Storage& c) {
+    if (deferrable(gates.shape) && deferrable(c.shape)) {
+      const Storage og = gate(gates, c.shape, 3, RT_F_SIGMOID), th = lz_unary(RT_F_TANH, c);
+      Storage h = lz_mul(og, th);
+      h.buf->made_from = gates.buf->id;
+      h.buf->saved = {og.buf, th.buf};
+      return h;
+    }
     Storage h = alloc(c.shape);
     check(rt_lstm_cell_h(ctx(), gates.ptr(), c.ptr(), (int64_t)c.shape[0], (int64_t)c.shape[1], h.ptr()));
     return h;
@@ -781,11 +1188,56 @@ struct B200Backend {
     const Storage& c = o.inputs[1].data();
     if (g.shape != c.shape) throw Error::shape_mismatch(c.shape, g.shape);
     const bool ng = o.inputs[0].requires_grad(), nc = o.inputs[1].requires_grad();
+    if (deferrable(gates.shape) && deferrable(g.shape)) {
+      const Storage og = saved_gate(o, 0, gates, c.shape, 3, RT_F_SIGMOID);
+      const bool kept = keeps(o, gates) && o.cached_outputs->buf->saved[1]->made_from == c.buf->id;
+      const Storage th = kept ? Storage{o.cached_outputs->buf->saved[1], c.shape} : lz_unary(RT_F_TANH, c);
+      Storage dgates = ng ? to_gate(lz_mul(lz_mul(g, th), lz_unary(RT_F_LOGISTIC_SLOPE, og)), gates.shape, 3) : unused_grad(gates.shape);
+      Storage dc = nc ? lz_mul(lz_mul(g, og), lz_unary(RT_F_ONE_MINUS_SQUARE, th)) : unused_grad(c.shape);
+      return {std::move(dgates), std::move(dc)};
+    }
     Storage dg = ng ? alloc(gates.shape) : unused_grad(gates.shape);
     Storage dc = nc ? alloc(c.shape) : unused_grad(c.shape);
     check(rt_lstm_cell_h_backward(ctx(), gates.ptr(), c.ptr(), g.ptr(), (int64_t)c.shape[0], (int64_t)c.shape[1],
                                   ng ? dg.ptr() : nullptr, nc ? dc.ptr() : nullptr));
     return {std::move(dg), std::move(dc)};
+  }
+
+  // One launch for all parameters of an optimizer step.  kind as rt_optimizer_step_multi; s1 / s2: the optimizer's states.
+  static void step_all(int kind, const std::vector<Storage*>& ps, const std::vector<Storage>& gs, const std::vector<Storage*>& s1,
+                       const std::vector<Storage*>& s2, float lr, float b1, float b2, float eps, float momentum, size_t t) {
+    if (kind == 1 && t == 0) throw Error::internal("Adam step called with t=0");
+    std::vector<float*> p, a, b;
+    std::vector<const float*> g;
+    std::vector<int64_t> n;
+    auto launch = [&] {
+      if (!p.empty())
+        check(rt_optimizer_step_multi(ctx(), kind, (int)p.size(), p.data(), g.data(), a.data(), b.data(), n.data(), lr, b1, b2, eps, momentum,
+                                      (int64_t)t, 1.f, 0, 0.f, 0.f));
+      p.clear(); a.clear(); b.clear(); g.clear(); n.clear();
+    };
+    for (size_t i = 0; i < ps.size(); ++i) {
+      if (ps[i]->shape != gs[i].shape) throw Error::shape_mismatch(ps[i]->shape, gs[i].shape);
+      if (ps[i]->numel() == 0) continue;
+      g.push_back(gs[i].ptr());
+      if (std::find(p.begin(), p.end(), ps[i]->buf->ptr) != p.end()) launch();  // a parameter listed twice is updated twice, in order
+      make_unique(*ps[i]);
+      p.push_back(ps[i]->ptr());
+      if (kind != 0) {
+        make_unique(*s1[i]);
+        a.push_back(s1[i]->ptr());
+      } else {
+        a.push_back(nullptr);
+      }
+      if (kind == 1) {
+        make_unique(*s2[i]);
+        b.push_back(s2[i]->ptr());
+      } else {
+        b.push_back(nullptr);
+      }
+      n.push_back((int64_t)ps[i]->numel());
+    }
+    launch();
   }
 
   // ---- optimizer steps (mod.rs:18-36, 256-272) ---------------------------------------------------

@@ -154,6 +154,17 @@ struct DpTrainer {
     if (do_reduce) B200Backend::check(rt_dp_allreduce_sum(c, dst + begin, end - begin));
   }
 
+  // Everything a step leaves behind is evaluated as part of it (the loss and the gradients, which a captured graph writes on
+  // every replay); the recorded ops go, and with them the intermediate results that nobody has asked for.
+  void settle(const Tensor& loss) {
+    loss.data().ptr();
+    for (auto& p : tr->w.params)
+      if (p.grad()) p.grad()->ptr();
+    for (auto& x : inputs)
+      if (x.grad()) x.grad()->ptr();
+    loss.detach_graph();
+  }
+
   // forward + backward (+ gradient exchange when world > 1); everything asynchronous.
   // Data parallel: as soon as the backward walk has finalised at least half of the gradient elements (for a CNN the
   // fully connected layers, reached first), the largest contiguous run of ready parameters becomes the early slice,
@@ -176,6 +187,7 @@ struct DpTrainer {
     if (update_in_stream() || world == 1 || fused) {
       stamp(1);
       loss.backward();
+      settle(loss);
       stamp(2);
       if (update_in_stream()) update_on_device();
       stamp(6);
@@ -188,7 +200,6 @@ struct DpTrainer {
     int64_t ready_elems = 0, total = 0;
     for (int i = 0; i < n; ++i) total += sizes[i];
     bool fired = false;
-    rt_ctx* c = B200Backend::ctx();
     struct HookGuard {
       ~HookGuard() { Tensor::leaf_ready_hook() = nullptr; }
     } guard;
@@ -209,14 +220,16 @@ struct DpTrainer {
       }
       fired = true;
       if (capturing) {  // split the capture here; the exchange of the early slice runs between the two replays
-        B200Backend::check(rt_graph_end(c, &graph));
-        B200Backend::check(rt_graph_begin(c));
+        for (int i = early_lo; i < early_hi; ++i) w.params[i].grad()->ptr();  // evaluated inside the first part
+        B200Backend::end_capture(&graph);
+        B200Backend::begin_capture();
       } else {
         exchange_early();
       }
     };
     loss.backward();
     Tensor::leaf_ready_hook() = nullptr;
+    settle(loss);
     if (!capturing) exchange_rest();
     else if (!fused && !fired) {  // single exchange: the pack kernel is recorded with the backward pass
       pack_and_reduce(0, n, true, false);
@@ -227,6 +240,8 @@ struct DpTrainer {
   void exchange_early() {
     if (world == 1 || early_lo >= early_hi) return;
     rt_ctx* c = B200Backend::ctx();
+    for (int i = early_lo; i < early_hi; ++i)
+      if (tr->w.params[i].grad()) tr->w.params[i].grad()->ptr();  // a side-stream section must not allocate
     B200Backend::check(rt_side_stream_begin(c));
     try {
       pack_and_reduce(early_lo, early_hi);
@@ -415,12 +430,13 @@ struct DpTrainer {
     if (graph) return;
     captured_loss = Tensor();
     have_loss = false;
-    B200Backend::check(rt_graph_begin(c));
+    B200Backend::begin_capture();
     rt_graph* last = nullptr;
     try {
       captured_loss = forward_backward(true);
     } catch (...) {
       rt_graph* g = nullptr;
+      rt::lazy::capturing() = false;
       rt_graph_end(c, &g);
       if (g) rt_graph_destroy(c, g);
       if (graph) {
@@ -429,7 +445,7 @@ struct DpTrainer {
       }
       throw;
     }
-    B200Backend::check(rt_graph_end(c, &last));
+    B200Backend::end_capture(&last);
     if (graph) graph_b = last;  // the hook closed the first part
     else graph = last;
     have_loss = true;
@@ -662,12 +678,15 @@ int rth_shutdown() {
 }
 
 int rth_sync() {
-  return rt::capi::guarded<B200Backend>([&](auto&) { B200Backend::check(rt_sync(B200Backend::ctx())); });
+  return rt::capi::guarded<B200Backend>([&](auto&) {
+    rt::lazy::flush_all();  // everything asked for so far is done when this returns
+    B200Backend::check(rt_sync(B200Backend::ctx()));
+  });
 }
 
 // Device pointer of a tensor's data (for calling the raw C ABI on engine tensors).
 int rth_tensor_device_ptr(int64_t h, void** out) {
-  return rt::capi::guarded<B200Backend>([&](auto& r) { *out = r.get(h).data().ptr(); });
+  return rt::capi::guarded<B200Backend>([&](auto& r) { *out = B200Backend::escape(r.get(h).data()); });
 }
 
 // ---- data-parallel trainer ------------------------------------------------------------

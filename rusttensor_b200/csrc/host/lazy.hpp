@@ -1,0 +1,1064 @@
+// Deferred elementwise ops of the CUDA backend.
+//
+// A model written op by op asks for one small kernel after another, and inside a CUDA graph as well as outside of it every
+// kernel costs 1.3 - 2 us and a pass over memory however little it computes.  The backend therefore only notes down what an
+// elementwise op (arithmetic, activations and their gradients, broadcasting, slicing, padding, concatenation) is to compute:
+// the result's buffer holds an expression (Node) over its operands' buffers.  The first use that needs the values - a product,
+// a reduction, an optimizer step, a copy to the host, a device pointer - evaluates the expression together with all the
+// unevaluated ones below it in ONE launch of the interpreting kernel (rt_fused_elementwise).
+//
+// Rules that keep this invisible:
+//  * Buffers are immutable once produced.  What does change one in place (optimizer steps, update_from_host, accumulating
+//    kernels) first evaluates every expression that reads it (flush_readers).
+//  * A buffer whose address has been handed out may be written behind the engine's back, so expressions that read it are
+//    evaluated on the spot - except inside a graph capture, where the whole step is recorded anyway.
+//  * A capture starts with nothing unevaluated (flush_all), so that it records exactly the step's own work, and rth_sync leaves
+//    nothing unevaluated either.
+//  * Depth is bounded: a result whose expression has become kMaxDepth ops deep is evaluated at once.
+//
+// What is written to memory besides the asked-for result: intermediate results that somebody else still refers to, when the
+// tensor is small (a launch later on would cost more than the store), or when recomputing them would be expensive.
+#pragma once
+#include <algorithm>
+#include <cstring>
+#include <functional>
+#include <memory>
+#include <vector>
+
+#include "../../../include/rt_b200.h"
+#include "autograd.hpp"
+
+namespace rt {
+
+struct DeviceBuffer;
+void lazy_evaluate(DeviceBuffer* b);
+
+namespace lazy {
+
+struct Input {
+  std::shared_ptr<DeviceBuffer> buf;
+  Shape shape;
+};
+enum class Kind : uint8_t { Const, Unary, BinaryImm, Binary, Broadcast, Slice, Pad, Concat, Opaque };
+// Opaque: computed by a kernel of its own.  Deferred only because what it feeds may take a kernel that does both.
+enum class Tag : uint8_t { None, Matmul, Conv, LogSoftmax, Reduce, PoolGrad, SumProducts, SumRows };
+
+struct Node {
+  Kind kind;
+  uint8_t op = 0;
+  bool swap = false;  // BinaryImm: the immediate is the left operand
+  float imm = 0.f;
+  int depth = 1;
+  int weight = 0;     // cost of evaluating it from its evaluated inputs, in simple ops
+  Shape shape;
+  Shape starts;       // Slice, Pad: the box's origin; Concat: {axis}
+  std::vector<Input> in;
+  // Opaque only
+  Tag tag = Tag::None;
+  std::vector<int64_t> geo;  // its parameters, as its tag has them
+  std::function<void(Node&, DeviceBuffer*)> run;  // computes the buffer (sets ptr)
+};
+
+constexpr int kMaxDepth = 200;
+#ifndef RT_LAZY_SMALL
+#define RT_LAZY_SMALL ((size_t)1 << 20)
+#endif
+constexpr size_t kSmall = RT_LAZY_SMALL;    // elements up to which shared intermediate results are always written
+constexpr int kRecompute = 16;              // weight from which they are written whatever the size
+constexpr int kDuplicate = 2;               // most weight that is repeated for every element of a broadcast
+constexpr int kMaxChain = 512;              // depth of a sum of scalars (the losses of a sequence)
+
+// What evaluating an expression costs now, up to `limit`; products and the like count as evaluated, which they will be by then.
+int current_weight(const Node& n, int limit);
+
+}  // namespace lazy
+
+struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
+  rt_ctx* ctx;
+  float* ptr;
+  size_t numel;
+  bool escaped = false;
+  std::shared_ptr<DeviceBuffer> owner;  // set: ptr points into this buffer's block (contiguous rows of it)
+  uint64_t id = next_id();   // of the values: another one after every change in place
+  uint64_t made_from = 0;    // id of the operand's values, for results from which their gradient follows
+  std::vector<std::shared_ptr<DeviceBuffer>> saved;  // intermediate results of a fused op that its gradient uses
+  std::unique_ptr<lazy::Node> node;    // what to compute; null once the values are in memory
+  std::vector<DeviceBuffer*> readers;  // unevaluated buffers whose expression takes this one as an input
+  DeviceBuffer *prev = nullptr, *next = nullptr;  // list of all unevaluated buffers
+
+  static uint64_t next_id() {
+    static uint64_t n = 0;
+    return ++n;
+  }
+  static DeviceBuffer*& head() {
+    static DeviceBuffer* h = nullptr;
+    return h;
+  }
+  DeviceBuffer(rt_ctx* c, float* p, size_t n) : ctx(c), ptr(p), numel(n) {}
+  DeviceBuffer(rt_ctx* c, std::unique_ptr<lazy::Node> nd, size_t n) : ctx(c), ptr(nullptr), numel(n), node(std::move(nd)) {
+    for (auto& i : node->in) i.buf->readers.push_back(this);
+    next = head();
+    if (next) next->prev = this;
+    head() = this;
+  }
+  DeviceBuffer(const DeviceBuffer&) = delete;
+  DeviceBuffer& operator=(const DeviceBuffer&) = delete;
+  ~DeviceBuffer() {
+    drop_node();
+    if (ptr && !owner) rt_free(ctx, ptr);
+  }
+  void drop_node() {
+    if (!node) return;
+    std::unique_ptr<lazy::Node> gone = std::move(node);
+    if (prev) prev->next = next;
+    else head() = next;
+    if (next) next->prev = prev;
+    prev = next = nullptr;
+    for (auto& i : gone->in) {
+      auto& r = i.buf->readers;
+      for (size_t k = r.size(); k-- > 0;)
+        if (r[k] == this) {
+          r[k] = r.back();
+          r.pop_back();
+          break;
+        }
+    }
+  }
+  float* data() {
+    if (node) lazy_evaluate(this);
+    return ptr;
+  }
+  void flush_readers() {
+    while (!readers.empty()) lazy_evaluate(readers.back());
+  }
+};
+
+namespace lazy {
+
+int op_weight(uint8_t op);
+inline int current_weight(const Node& n, int limit) {
+  if (n.kind == Kind::Opaque) return 0;
+  int w = n.kind == Kind::Unary || n.kind == Kind::Binary || n.kind == Kind::BinaryImm ? op_weight(n.op) : 0;
+  for (auto& i : n.in) {
+    if (w > limit) break;
+    if (i.buf->node) w += current_weight(*i.buf->node, limit - w);
+  }
+  return w;
+}
+
+inline bool& capturing() {
+  static bool c = false;
+  return c;
+}
+inline void flush_all() {
+  while (DeviceBuffer::head()) lazy_evaluate(DeviceBuffer::head());
+}
+
+inline int op_weight(uint8_t op) {
+  switch (op) {
+    case RT_F_EXP: case RT_F_LN: case RT_F_SIN: case RT_F_COS: case RT_F_TAN: case RT_F_TANH: case RT_F_SIGMOID: case RT_F_SOFTPLUS:
+    case RT_F_ELU: case RT_F_ELU_SLOPE: case RT_F_POWF: return 4;
+    case RT_F_DIV: case RT_F_RECIP: case RT_F_SQRT: case RT_F_HALF_RSQRT: case RT_F_RECIP_SQUARE: return 3;
+    default: return 1;
+  }
+}
+
+// ---- from an expression to a program -----------------------------------------------------------------------------------------
+constexpr int kMaxRawDims = 8;
+
+// How a tensor's coordinates follow from the iteration coordinates: dimension j = (map[j] < 0 ? 0 : iteration[map[j]]) + off[j].
+struct View {
+  int nd = 0;
+  int8_t map[kMaxRawDims];
+  int64_t off[kMaxRawDims];
+  int region = RT_FUSED_NONE;
+  bool operator==(const View& o) const {
+    if (nd != o.nd || region != o.region) return false;
+    for (int j = 0; j < nd; ++j)
+      if (map[j] != o.map[j] || off[j] != o.off[j]) return false;
+    return true;
+  }
+};
+
+class Compiler {
+ public:
+  // Builds the program of `root`; false: it does not fit (the caller evaluates some inputs first and tries again).
+  bool build(DeviceBuffer* root, rt_fused_program* p, std::vector<DeviceBuffer*>* stored) {
+    const Node& n = *root->node;
+    nd_ = (int)n.shape.size();
+    if (nd_ > kMaxRawDims) return false;
+    for (int d = 0; d < nd_; ++d) shape_[d] = (int64_t)n.shape[d];
+    if (nd_ == 0) {
+      nd_ = 1;
+      shape_[0] = 1;
+    }
+    numel_ = root->numel;
+    View id;
+    id.nd = (int)n.shape.size();
+    for (int j = 0; j < id.nd; ++j) {
+      id.map[j] = (int8_t)j;
+      id.off[j] = 0;
+    }
+    views_.push_back(id);
+    root_ = root;
+    const int r = node_value(root, 0);
+    if (r < 0) return false;
+    outputs_.push_back({r, root});
+    for (auto& c : stored_) {
+      if ((int)outputs_.size() == RT_FUSED_MAX_OUTPUTS) break;
+      if (c.second->node) outputs_.push_back({c.first, c.second});  // not evaluated meanwhile, as part of some other program
+    }
+    if (!collapse(p)) return false;
+    for (int pre = std::min<int>((int)operands_.size(), RT_FUSED_PRELOAD); pre >= 0; --pre)
+      if (emit(p, pre)) {
+        for (auto& o : outputs_) stored->push_back(o.second);
+        return true;
+      }
+    return false;
+  }
+  const std::vector<std::pair<int, DeviceBuffer*>>& outputs() const { return outputs_; }
+
+ private:
+  struct Value {
+    uint8_t op;       // RT_F_*; RT_F_LOAD: operand `a`; RT_F_REG: the immediate
+    bool swap;
+    int a, b;         // value numbers; b < 0: none, or the immediate for a binary op
+    int region;       // RT_F_SELECT: a inside, b (or the immediate) outside
+    float imm;
+  };
+  struct Operand {
+    std::shared_ptr<DeviceBuffer> buf;  // stays allocated until the launch
+    const float* ptr;
+    int64_t stride[kMaxRawDims];
+    int region;
+  };
+  struct Box {
+    int64_t lo[kMaxRawDims], hi[kMaxRawDims];
+  };
+  struct Memo {
+    DeviceBuffer* b;
+    int view, value;
+  };
+  DeviceBuffer* root_ = nullptr;
+  int nd_ = 0;
+  int64_t shape_[kMaxRawDims];
+  size_t numel_ = 0;
+  std::vector<View> views_;
+  std::vector<Value> values_;
+  std::vector<Operand> operands_;
+  std::vector<Box> regions_;
+  std::vector<Memo> memo_;
+  std::vector<std::pair<int, DeviceBuffer*>> stored_, outputs_;
+
+  int view_id(const View& v) {
+    for (size_t i = 0; i < views_.size(); ++i)
+      if (views_[i] == v) return (int)i;
+    views_.push_back(v);
+    return (int)views_.size() - 1;
+  }
+  int add(uint8_t op, int a, int b, float imm, bool swap = false, int region = RT_FUSED_NONE) {
+    for (size_t i = values_.size(); i-- > 0;) {
+      const Value& v = values_[i];
+      if (v.op == op && v.a == a && v.b == b && v.swap == swap && v.region == region && std::memcmp(&v.imm, &imm, sizeof(float)) == 0)
+        return (int)i;
+    }
+    if (values_.size() >= RT_FUSED_MAX_CODE) return -1;
+    values_.push_back({op, swap, a, b, region, imm});
+    return (int)values_.size() - 1;
+  }
+  bool is_imm(int v) const { return values_[v].op == RT_F_REG; }
+
+  int region_id(const Box& b) {
+    for (size_t i = 0; i < regions_.size(); ++i) {
+      bool same = true;
+      for (int d = 0; d < nd_; ++d) same = same && regions_[i].lo[d] == b.lo[d] && regions_[i].hi[d] == b.hi[d];
+      if (same) return (int)i;
+    }
+    if (regions_.size() >= RT_FUSED_MAX_REGIONS) return -1;
+    regions_.push_back(b);
+    return (int)regions_.size() - 1;
+  }
+
+  // Maps a view of a node onto one of its inputs (right-aligned dimensions; extent 1 stretches).
+  View child_view(const View& v, const Shape& node, const Shape& child) const {
+    View c;
+    c.nd = (int)child.size();
+    c.region = v.region;
+    const int lead = (int)node.size() - c.nd;
+    for (int j = 0; j < c.nd; ++j) {
+      if (child[j] == 1 && node[j + lead] != 1) {
+        c.map[j] = -1;
+        c.off[j] = 0;
+      } else {
+        c.map[j] = v.map[j + lead];
+        c.off[j] = v.off[j + lead];
+      }
+    }
+    return c;
+  }
+  // Restricts a view to the box [start, start + extent) of its tensor and moves the origin there.  -1: no room for the region;
+  // false in `any`: nothing of the box is seen.
+  int box_view(const View& v, const Shape& starts, const Shape& extent, View* out, bool* any) {
+    Box b;
+    for (int d = 0; d < nd_; ++d) {
+      b.lo[d] = v.region == RT_FUSED_NONE ? 0 : regions_[v.region].lo[d];
+      b.hi[d] = v.region == RT_FUSED_NONE ? shape_[d] : regions_[v.region].hi[d];
+    }
+    *out = v;
+    *any = true;
+    for (int j = 0; j < v.nd; ++j) {
+      const int64_t s = (int64_t)starts[j], n = (int64_t)extent[j];
+      out->off[j] = v.off[j] - s;
+      if (v.map[j] < 0) {
+        if (v.off[j] < s || v.off[j] >= s + n) *any = false;
+        continue;
+      }
+      const int d = v.map[j];
+      b.lo[d] = std::max(b.lo[d], s - v.off[j]);
+      b.hi[d] = std::min(b.hi[d], s + n - v.off[j]);
+      if (b.lo[d] >= b.hi[d]) *any = false;
+    }
+    if (!*any) return RT_FUSED_NONE;
+    bool full = true;
+    for (int d = 0; d < nd_; ++d) full = full && b.lo[d] <= 0 && b.hi[d] >= shape_[d];
+    if (full) return out->region = RT_FUSED_NONE;
+    const int r = region_id(b);
+    if (r < 0) return -1;
+    return out->region = r;
+  }
+
+  // The view of a tensor as seen by an expression of the same values whose shape differs in extents of 1 only.
+  static bool squeezed_view(const View& v, const Shape& from, const Shape& to, View* w) {
+    w->nd = (int)to.size();
+    w->region = v.region;
+    size_t i = 0;
+    for (size_t j = 0; j < to.size(); ++j) {
+      w->map[j] = -1;
+      w->off[j] = 0;
+      if (to[j] == 1) continue;
+      while (i < from.size() && from[i] == 1) ++i;
+      if (i == from.size() || from[i] != to[j]) return false;
+      w->map[j] = v.map[i];
+      w->off[j] = v.off[i];
+      ++i;
+    }
+    while (i < from.size() && from[i] == 1) ++i;
+    return i == from.size();
+  }
+
+  int leaf(const Input& in, const View& v) {
+    Operand o;
+    for (int d = 0; d < kMaxRawDims; ++d) o.stride[d] = 0;
+    int64_t stride = 1, off = 0;
+    for (int j = v.nd - 1; j >= 0; --j) {
+      off += v.off[j] * stride;
+      if (v.map[j] >= 0 && shape_[v.map[j]] != 1) o.stride[v.map[j]] += stride;
+      stride *= (int64_t)in.shape[j];
+    }
+    if (stride >= (1ll << 31)) return -1;
+    o.buf = in.buf;
+    o.ptr = in.buf->ptr + off;
+    o.region = v.region;
+    for (size_t k = 0; k < operands_.size(); ++k) {
+      bool same = operands_[k].ptr == o.ptr && operands_[k].region == o.region;
+      for (int d = 0; d < nd_; ++d) same = same && operands_[k].stride[d] == o.stride[d];
+      if (same) return add(RT_F_LOAD, (int)k, -1, 0.f);
+    }
+    if (operands_.size() >= RT_FUSED_MAX_OPERANDS) return -1;
+    operands_.push_back(o);
+    return add(RT_F_LOAD, (int)operands_.size() - 1, -1, 0.f);
+  }
+
+  int input_value(const Input& in, const View& v) {
+    if (in.buf->node && in.buf->node->kind != Kind::Opaque && in.buf->node->shape != in.shape) {
+      if (in.buf->node->kind == Kind::Const) return add(RT_F_REG, -1, -1, in.buf->node->imm);
+      View w;
+      if (in.buf->node->weight <= kDuplicate && squeezed_view(v, in.shape, in.buf->node->shape, &w)) return node_value(in.buf.get(), view_id(w));
+      lazy_evaluate(in.buf.get());  // its own dimensions do not match the iteration's
+    }
+    if (in.buf->node && in.buf->node->kind != Kind::Const && in.buf->node->kind != Kind::Opaque && in.buf->node->weight > kDuplicate) {
+      // an expensive expression under a broadcast would be evaluated over and over
+      for (int d = 0; d < nd_; ++d) {
+        if (shape_[d] == 1) continue;
+        bool seen = false;
+        for (int j = 0; j < v.nd; ++j) seen = seen || v.map[j] == d;
+        if (!seen) {
+          lazy_evaluate(in.buf.get());
+          break;
+        }
+      }
+    }
+    if (in.buf->node && in.buf->node->kind == Kind::Opaque) lazy_evaluate(in.buf.get());
+    // seen through a window (not over its own full shape), costly, and part of several expressions: once, into memory
+    if (in.buf->node && in.buf->readers.size() >= 2 && !(v == views_[0] && in.shape == root_->node->shape) && current_weight(*in.buf->node, 4) > 3)
+      lazy_evaluate(in.buf.get());
+    if (!in.buf->node) return leaf(in, v);
+    return node_value(in.buf.get(), view_id(v));
+  }
+
+  int node_value(DeviceBuffer* b, int vid) {
+    for (auto& m : memo_)
+      if (m.b == b && m.view == vid) return m.value;
+    const int r = make_value(b, vid);
+    if (r >= 0) {
+      memo_.push_back({b, vid, r});
+      if (vid == 0 && b != root_ && b->node->shape == root_->node->shape && values_[r].op != RT_F_LOAD && values_[r].op != RT_F_REG && worth_storing(b))
+        stored_.push_back({r, b});
+    }
+    return r;
+  }
+  static bool worth_storing(DeviceBuffer* b) {
+    const Node& n = *b->node;
+    if (n.kind == Kind::Const || n.kind == Kind::Broadcast || n.kind == Kind::Slice) return false;
+    // whoever is not an unevaluated expression: tensors, recorded ops, callers
+    const long outside = b->weak_from_this().use_count() - (long)b->readers.size();
+    if (outside <= 0) return false;
+    return b->numel <= kSmall || n.weight >= kRecompute;
+  }
+
+  int make_value(DeviceBuffer* b, int vid) {
+    const Node& n = *b->node;
+    const View v = views_[vid];  // a copy: views_ grows below
+    switch (n.kind) {
+      case Kind::Const: return add(RT_F_REG, -1, -1, n.imm);
+      case Kind::Unary: {
+        const int a = input_value(n.in[0], child_view(v, n.shape, n.in[0].shape));
+        return a < 0 ? -1 : add(n.op, a, -1, n.imm);
+      }
+      case Kind::BinaryImm: {
+        const int a = input_value(n.in[0], child_view(v, n.shape, n.in[0].shape));
+        return a < 0 ? -1 : add(n.op, a, -1, n.imm, n.swap);
+      }
+      case Kind::Broadcast: return input_value(n.in[0], child_view(v, n.shape, n.in[0].shape));
+      case Kind::Binary: {
+        int a, c;
+        const View va = child_view(v, n.shape, n.in[0].shape), vb = child_view(v, n.shape, n.in[1].shape);
+        auto cost = [](const Input& i) { return i.buf->node ? 1 + current_weight(*i.buf->node, 64) : 0; };
+        if (cost(n.in[1]) > cost(n.in[0])) {  // the larger side first: fewer values are alive at a time
+          c = input_value(n.in[1], vb);
+          a = c < 0 ? -1 : input_value(n.in[0], va);
+        } else {
+          a = input_value(n.in[0], va);
+          c = a < 0 ? -1 : input_value(n.in[1], vb);
+        }
+        if (a < 0 || c < 0) return -1;
+        if (is_imm(c)) return add(n.op, a, -1, values_[c].imm);
+        if (is_imm(a)) return add(n.op, c, -1, values_[a].imm, true);
+        return add(n.op, a, c, 0.f);
+      }
+      case Kind::Slice: {
+        settle_shared(n.in[0]);
+        View c = v;
+        for (int j = 0; j < v.nd; ++j) c.off[j] += (int64_t)n.starts[j];
+        return input_value(n.in[0], c);
+      }
+      case Kind::Pad: return boxed(n.in[0], v, n.starts, -1);
+      case Kind::Concat: {
+        Shape starts(n.shape.size(), 0);
+        int r = -1;
+        for (auto& piece : n.in) {
+          settle_shared(piece);
+          r = boxed(piece, v, starts, r);
+          if (r < 0) return -1;
+          starts[n.starts[0]] += piece.shape[n.starts[0]];
+        }
+        return r;
+      }
+      case Kind::Opaque: break;
+    }
+    return -1;
+  }
+  // A costly result that others use too and that is seen here only through a window: it is written to memory now, because the
+  // program around the window cannot write it and whoever else asks would compute it again.
+  static void settle_shared(const Input& in) {
+    DeviceBuffer* b = in.buf.get();
+    if (b->node && b->weak_from_this().use_count() > (long)b->readers.size() && current_weight(*b->node, 4) > 3) lazy_evaluate(b);
+  }
+  // The value of `in` placed at `starts`, and `other` (0 when negative) elsewhere.
+  int boxed(const Input& in, const View& v, const Shape& starts, int other) {
+    View c;
+    bool any;
+    const int r = box_view(v, starts, in.shape, &c, &any);
+    if (r < 0) return -1;
+    if (!any) return other < 0 ? add(RT_F_REG, -1, -1, 0.f) : other;
+    const int a = input_value(in, c);
+    if (a < 0 || r == RT_FUSED_NONE) return a;
+    if (other < 0 && values_[a].op == RT_F_LOAD && operands_[values_[a].a].region == r) return a;  // 0 outside already
+    if (other < 0 || is_imm(other)) return add(RT_F_SELECT, a, -1, other < 0 ? 0.f : values_[other].imm, false, r);
+    return add(RT_F_SELECT, a, other, 0.f, false, r);
+  }
+
+  // Merges neighbouring dimensions that every operand walks as one and writes shape, operands and regions.
+  bool collapse(rt_fused_program* p) {
+    int nd = 0;
+    int keep[kMaxRawDims];
+    int64_t shape[kMaxRawDims];
+    std::vector<Operand> ops = operands_;
+    std::vector<Box> boxes = regions_;
+    for (int d = 0; d < nd_; ++d) {
+      if (shape_[d] == 1 && !(d == nd_ - 1 && nd == 0)) {
+        bool trivial = true;
+        for (auto& b : boxes) trivial = trivial && b.lo[d] <= 0 && b.hi[d] >= 1;
+        if (trivial) continue;
+      }
+      bool merge = nd > 0;
+      if (merge) {
+        const int q = keep[nd - 1];
+        for (auto& o : ops) merge = merge && o.stride[q] == o.stride[d] * shape_[d];
+        for (auto& b : boxes) merge = merge && b.lo[d] <= 0 && b.hi[d] >= shape_[d];
+        if (merge) {
+          for (auto& o : ops) o.stride[q] = o.stride[d];
+          for (auto& b : boxes) {
+            b.lo[q] *= shape_[d];
+            b.hi[q] *= shape_[d];
+          }
+          shape[nd - 1] *= shape_[d];
+          continue;
+        }
+      }
+      keep[nd] = d;
+      shape[nd++] = shape_[d];
+    }
+    if (nd == 0) {
+      keep[0] = nd_ - 1;
+      shape[0] = 1;
+      nd = 1;
+    }
+    if (nd > RT_FUSED_MAX_DIMS) return false;
+    p->nd = nd;
+    for (int i = 0; i < nd; ++i) p->shape[i] = (int32_t)shape[i];
+    p->n_operands = (int)ops.size();
+    for (size_t k = 0; k < ops.size(); ++k) {
+      p->operand[k].ptr = ops[k].ptr;
+      p->operand[k].region = ops[k].region;
+      for (int i = 0; i < RT_FUSED_MAX_DIMS; ++i) p->operand[k].stride[i] = i < nd ? (int32_t)ops[k].stride[keep[i]] : 0;
+    }
+    p->n_regions = (int)boxes.size();
+    for (size_t k = 0; k < boxes.size(); ++k)
+      for (int i = 0; i < RT_FUSED_MAX_DIMS; ++i) {
+        p->region[k].lo[i] = i < nd ? (int32_t)boxes[k].lo[keep[i]] : 0;
+        p->region[k].hi[i] = i < nd ? (int32_t)boxes[k].hi[keep[i]] : 1;
+      }
+    return true;
+  }
+
+  // ---- instructions and registers: one accumulator, a value goes to a register when the accumulator is overwritten before its
+  // last use (the instruction that produced it then also writes the register) -------------------------------------------------
+  struct Emitter {
+    rt_fused_program* p;
+    const std::vector<Value>& values;
+    std::vector<int> where, left;  // register of a value or -1; uses that are still to come
+    int acc = -1;
+    unsigned free_regs = (1u << RT_FUSED_REGS) - 1;
+    bool ok = true;
+
+    int take() {
+      for (int r = 0; r < RT_FUSED_REGS; ++r)
+        if (free_regs & (1u << r)) {
+          free_regs &= ~(1u << r);
+          return r;
+        }
+      return -1;
+    }
+    void keep_acc() {  // gives the accumulator's value a register
+      if (acc < 0 || where[acc] >= 0) return;
+      const int r = take();
+      if (r < 0) {
+        ok = ok && values[acc].op == RT_F_LOAD;  // an operand can be loaded again
+        return;
+      }
+      p->code[p->n_code - 1].dst = (uint8_t)r;
+      where[acc] = r;
+    }
+    void put(uint8_t op, uint8_t src, uint8_t swap, float imm, int value) {
+      if (value != acc && acc >= 0 && left[acc] > 0) keep_acc();
+      if (p->n_code >= RT_FUSED_MAX_CODE) ok = false;
+      if (!ok) return;
+      p->code[p->n_code++] = {op, src, RT_FUSED_NONE, swap, imm};
+      acc = value;
+    }
+    void release(int v) {
+      if (left[v] == 0 && where[v] >= 0) {
+        free_regs |= 1u << where[v];
+        where[v] = -1;
+      }
+    }
+    void to_acc(int v) {
+      if (acc == v || !ok) return;
+      if (where[v] >= 0) put(RT_F_REG, (uint8_t)where[v], 0, 0.f, v);
+      else if (values[v].op == RT_F_REG) put(RT_F_REG, RT_FUSED_IMM, 0, values[v].imm, v);
+      else if (values[v].op == RT_F_LOAD) put(RT_F_LOAD, (uint8_t)values[v].a, 0, 0.f, v);
+      else ok = false;
+    }
+    void to_register(int v) {
+      if (where[v] >= 0 || !ok) return;
+      to_acc(v);
+      keep_acc();
+      if (where[v] < 0) ok = false;
+    }
+  };
+
+  bool emit(rt_fused_program* p, int preload) {
+    Emitter e{p, values_, std::vector<int>(values_.size(), -1), std::vector<int>(values_.size(), 0)};
+    p->n_code = 0;
+    p->n_preload = preload;
+    std::vector<char> live(values_.size(), 0);
+    for (auto& o : outputs_) live[o.first] = 1;
+    for (int v = (int)values_.size() - 1; v >= 0; --v) {
+      if (!live[v]) continue;
+      const Value& x = values_[v];
+      if (x.op == RT_F_LOAD || x.op == RT_F_REG) continue;
+      live[x.a] = 1;
+      e.left[x.a]++;
+      if (x.b >= 0) {
+        live[x.b] = 1;
+        e.left[x.b]++;
+      }
+    }
+    for (size_t v = 0; v < values_.size(); ++v)
+      if (live[v] && values_[v].op == RT_F_LOAD && values_[v].a < preload) {
+        e.where[v] = values_[v].a;
+        e.free_regs &= ~(1u << values_[v].a);
+      }
+    auto store = [&](int v) {
+      for (size_t k = 0; k < outputs_.size(); ++k)
+        if (outputs_[k].first == v) e.put(RT_F_OUT, (uint8_t)k, 0, 0.f, v);
+    };
+    for (int v = 0; v < (int)values_.size() && e.ok; ++v) {
+      const Value& x = values_[v];
+      if (!live[v] || x.op == RT_F_LOAD || x.op == RT_F_REG) continue;
+      uint8_t src = RT_FUSED_IMM, swap = x.swap ? 1 : 0;
+      if (x.op == RT_F_SELECT) {
+        if (x.b >= 0) e.to_register(x.b);
+        e.to_acc(x.a);
+        if (!e.ok) return false;
+        if (x.b >= 0) src = (uint8_t)e.where[x.b];
+        swap = (uint8_t)x.region;
+      } else if (x.b < 0) {
+        e.to_acc(x.a);
+      } else if (x.a == x.b) {
+        e.to_register(x.a);
+        e.to_acc(x.a);
+        if (!e.ok) return false;
+        src = (uint8_t)e.where[x.a];
+      } else {
+        if (e.acc == x.b && e.where[x.a] >= 0) {
+          swap ^= 1;
+        } else if (!(e.acc == x.a && e.where[x.b] >= 0)) {
+          if (e.where[x.a] >= 0 && e.where[x.b] < 0) {
+            e.to_acc(x.b);
+            swap ^= 1;
+          } else {
+            e.to_register(x.b);
+            e.to_acc(x.a);
+          }
+        }
+        if (!e.ok) return false;
+        src = (uint8_t)e.where[e.acc == x.a ? x.b : x.a];
+      }
+      if (!e.ok) return false;
+      --e.left[x.a];
+      if (x.b >= 0) --e.left[x.b];
+      e.put(x.op, src, swap, x.imm, v);  // may give the old accumulator a register: `src` is still taken here
+      e.release(x.a);
+      if (x.b >= 0) e.release(x.b);
+      store(v);
+    }
+    for (size_t v = 0; v < values_.size() && e.ok; ++v)
+      if (live[v] && (values_[v].op == RT_F_LOAD || values_[v].op == RT_F_REG)) {
+        bool out = false;
+        for (auto& o : outputs_) out = out || o.first == (int)v;
+        if (!out) continue;
+        e.to_acc((int)v);
+        store((int)v);
+      }
+    p->n_outputs = (int)outputs_.size();
+    return e.ok;
+  }
+};
+
+inline void check(rt_ctx* ctx, rt_status st) {
+  if (st != RT_OK) throw Error((ErrorKind)st, rt_last_error(ctx));
+}
+inline float* new_block(rt_ctx* ctx, size_t numel) {
+  void* p = nullptr;
+  check(ctx, rt_malloc(ctx, sizeof(float) * std::max<size_t>(numel, 1), &p));
+  return (float*)p;
+}
+inline int unary_entry(uint8_t op) {  // the stand-alone kernel of an op, or -1
+  switch (op) {
+    case RT_F_RELU: return RT_RELU;
+    case RT_F_EXP: return RT_EXP;
+    case RT_F_LN: return RT_LN;
+    case RT_F_SIN: return RT_SIN;
+    case RT_F_COS: return RT_COS;
+    case RT_F_TAN: return RT_TAN;
+    case RT_F_TANH: return RT_TANH;
+    case RT_F_SIGMOID: return RT_SIGMOID;
+    case RT_F_SOFTPLUS: return RT_SOFTPLUS;
+    case RT_F_SQRT: return RT_SQRT;
+    case RT_F_ABS: return RT_ABS;
+    case RT_F_SQUARE: return RT_SQUARE;
+    case RT_F_ELU: return RT_ELU;
+    default: return -1;
+  }
+}
+inline int binary_entry(uint8_t op) {
+  static_assert(RT_F_LE - RT_F_ADD == RT_LESS_EQUAL - RT_ADD && RT_F_EQ - RT_F_ADD == RT_EQUAL - RT_ADD && RT_F_MAX - RT_F_ADD == RT_MAXIMUM - RT_ADD,
+                "binary ops are listed in the same order");
+  return op >= RT_F_ADD && op <= RT_F_LE ? op - RT_F_ADD + RT_ADD : -1;
+}
+inline std::vector<int64_t> dims64(const Shape& s) { return std::vector<int64_t>(s.begin(), s.end()); }
+
+// One op by its stand-alone kernel, its inputs in memory.  False: the op has none.
+inline bool evaluate_alone(DeviceBuffer* b) {
+  const Node& n = *b->node;
+  rt_ctx* c = b->ctx;
+  const int u = n.kind == Kind::Unary ? unary_entry(n.op) : -1, bi = n.kind == Kind::Binary ? binary_entry(n.op) : -1;
+  if ((n.kind == Kind::Unary && u < 0) || (n.kind == Kind::Binary && bi < 0) || n.kind == Kind::BinaryImm) return false;
+  float* out = new_block(c, b->numel);
+  auto nd = dims64(n.shape);
+  rt_status st = RT_OK;
+  auto place = [&](const Input& in, const std::vector<int64_t>& starts) {
+    auto id = dims64(in.shape);
+    if (st == RT_OK && shape_numel(in.shape) > 0)
+      st = rt_slice_assign(c, out, nd.data(), (int)nd.size(), starts.data(), in.buf->data(), id.data());
+  };
+  switch (n.kind) {
+    case Kind::Const: st = rt_fill(c, out, n.imm, (int64_t)b->numel); break;
+    case Kind::Unary: st = rt_unary(c, u, n.in[0].buf->data(), out, (int64_t)b->numel, n.imm, 0.f); break;
+    case Kind::Binary: {
+      auto as = dims64(n.in[0].shape), bs = dims64(n.in[1].shape);
+      st = rt_binary(c, bi, n.in[0].buf->data(), as.data(), (int)as.size(), n.in[1].buf->data(), bs.data(), (int)bs.size(), out);
+      break;
+    }
+    case Kind::Broadcast: {
+      auto xs = dims64(n.in[0].shape);
+      st = rt_broadcast_to(c, n.in[0].buf->data(), xs.data(), (int)xs.size(), nd.data(), (int)nd.size(), out);
+      break;
+    }
+    case Kind::Slice: {
+      auto xs = dims64(n.in[0].shape), s0 = dims64(n.starts);
+      st = rt_slice(c, n.in[0].buf->data(), xs.data(), (int)xs.size(), s0.data(), nd.data(), out);
+      break;
+    }
+    case Kind::Pad:
+      st = rt_fill(c, out, 0.f, (int64_t)b->numel);
+      place(n.in[0], dims64(n.starts));
+      break;
+    case Kind::Concat: {
+      std::vector<int64_t> s0(n.shape.size(), 0);
+      for (auto& piece : n.in) {
+        place(piece, s0);
+        s0[n.starts[0]] += (int64_t)piece.shape[n.starts[0]];
+      }
+      break;
+    }
+    default: break;
+  }
+  if (st != RT_OK) {
+    rt_free(c, out);
+    check(c, st);
+  }
+  b->ptr = out;
+  b->drop_node();
+  return true;
+}
+
+// ---- combinations that one kernel computes ---------------------------------------------------------------------------------
+inline Node* pending(const Input& i) { return i.buf->node.get(); }
+inline Node* tagged(const Input& i, Tag t) { return pending(i) && i.buf->node->tag == t ? i.buf->node.get() : nullptr; }
+inline bool is_op(const Node* n, Kind k, uint8_t op) { return n && n->kind == k && n->op == op; }
+
+// n = other * constant: the other factor, and the constant in `c`
+inline const Input* times_constant(const Node* n, float* c) {
+  if (is_op(n, Kind::BinaryImm, RT_F_MUL)) {
+    *c = n->imm;
+    return &n->in[0];
+  }
+  if (is_op(n, Kind::Binary, RT_F_MUL))
+    for (int i = 0; i < 2; ++i)
+      if (pending(n->in[i]) && n->in[i].buf->node->kind == Kind::Const && n->in[1 - i].shape == n->shape) {
+        *c = n->in[i].buf->node->imm;
+        return &n->in[1 - i];
+      }
+  return nullptr;
+}
+
+// act(a * b + bias), act one of none, relu, tanh, sigmoid: bias and activation in the product's epilogue.  Products of one shape
+// with the same b (a layer applied to every timestep) whose left operands are all there are computed in one launch.
+struct Linear {
+  DeviceBuffer* out;
+  Input a, b, bias;  // bias.buf null: none
+  int act;
+};
+inline bool match_linear(DeviceBuffer* out, Linear* l) {
+  const Node* n = out->node.get();
+  l->out = out;
+  l->act = RT_ACT_NONE;
+  if (n->tag == Tag::Matmul) {
+    l->a = n->in[0];
+    l->b = n->in[1];
+    l->bias = Input{};
+    return true;
+  }
+  const Node* sum = n;
+  if (n->kind == Kind::Unary && (n->op == RT_F_RELU || n->op == RT_F_TANH || n->op == RT_F_SIGMOID)) {
+    l->act = n->op == RT_F_RELU ? RT_ACT_RELU : (n->op == RT_F_TANH ? RT_ACT_TANH : RT_ACT_SIGMOID);
+    sum = pending(n->in[0]);
+    if (!sum || n->in[0].shape != sum->shape) return false;
+  }
+  if (!is_op(sum, Kind::Binary, RT_F_ADD)) return false;
+  for (int i = 0; i < 2; ++i) {
+    const Node* m = tagged(sum->in[i], Tag::Matmul);
+    if (!m || sum->in[i].buf->readers.size() != 1 || m->shape != sum->shape || sum->in[i].shape != m->shape) continue;
+    Input bias = sum->in[1 - i];
+    if (pending(bias) && pending(bias)->kind == Kind::Broadcast && pending(bias)->shape == bias.shape) bias = Input(pending(bias)->in[0]);
+    if (bias.shape.empty() || bias.shape.back() != m->shape[1] || shape_numel(bias.shape) != m->shape[1]) continue;
+    l->a = m->in[0];
+    l->b = m->in[1];
+    l->bias = bias;
+    return true;
+  }
+  return false;
+}
+// The expression around a product that is computed with it: the product itself, its sum with a bias, the activation of that.
+inline DeviceBuffer* epilogue_of(DeviceBuffer* product, int act, bool bias) {
+  if (!bias) return product;
+  if (product->readers.size() != 1) return nullptr;
+  DeviceBuffer* sum = product->readers[0];
+  if (act == RT_ACT_NONE) return sum;
+  return sum->readers.size() == 1 ? sum->readers[0] : nullptr;
+}
+inline bool rewrite_linear(DeviceBuffer* b) {
+  Linear first{};
+  if (!match_linear(b, &first)) return false;
+  std::vector<Linear> all{first};
+  const float *pa = first.a.buf->data(), *pb = first.b.buf->data(), *bias = first.bias.buf ? first.bias.buf->data() : nullptr;
+  const std::vector<DeviceBuffer*> others = first.b.buf->readers;
+  for (DeviceBuffer* r : others) {
+    if (all.size() == 256) break;
+    if (!r->node || r->node->tag != Tag::Matmul || r->node->in[1].buf != first.b.buf || r->node->in[0].buf->node) continue;
+    DeviceBuffer* e = epilogue_of(r, first.act, bias != nullptr);
+    Linear l;
+    if (!e || e == b || !match_linear(e, &l)) continue;
+    if (l.act != first.act || l.b.buf != first.b.buf || l.a.shape != first.a.shape || l.b.shape != first.b.shape || l.bias.buf != first.bias.buf) continue;
+    all.push_back(l);
+  }
+  const int64_t rows = (int64_t)first.a.shape[0], k = (int64_t)first.a.shape[1], cols = (int64_t)first.b.shape[1];
+  std::vector<std::shared_ptr<DeviceBuffer>> keep;
+  for (auto& l : all) keep.push_back(l.out->shared_from_this());
+  std::vector<const float*> as;
+  std::vector<float*> outs;
+  for (auto& l : all) {
+    as.push_back(l.a.buf->data());
+    outs.push_back(new_block(b->ctx, l.out->numel));
+  }
+  rt_status st;
+  if (all.size() > 1) st = rt_gemm_bias_act_list(b->ctx, (int)all.size(), as.data(), outs.data(), rows, cols, k, pb, bias, first.act);
+  else st = rt_gemm_bias_act(b->ctx, rows, cols, k, pa, k, pb, cols, bias, first.act, outs[0], cols);
+  if (st != RT_OK) {
+    for (float* o : outs) rt_free(b->ctx, o);
+    check(b->ctx, st);
+  }
+  for (size_t i = 0; i < all.size(); ++i) {
+    all[i].out->ptr = outs[i];
+    all[i].out->drop_node();
+  }
+  return true;
+}
+
+// constant * [mean or sum over rows] of [constant *] sum over classes of log_softmax(x) * y: a classification loss.
+struct Loss {
+  const Input *logits, *targets;
+  int64_t rows, classes;
+  float scale, divisor;
+  bool same_kind(const Loss& o) const { return rows == o.rows && classes == o.classes && scale == o.scale && divisor == o.divisor; }
+};
+inline bool match_loss(DeviceBuffer* b, Loss* l) {
+  float scale = 1.f, c = 1.f;
+  const Node* n = b->node.get();
+  if (const Input* f = times_constant(n, &c)) {
+    if (!tagged(*f, Tag::Reduce) || f->buf->readers.size() != 1) return false;
+    scale *= c;
+    n = pending(*f);
+  }
+  if (n->tag != Tag::Reduce || n->geo[1] >= 0) return false;  // over all elements
+  const bool mean = n->geo[0] == RT_RED_MEAN;
+  const Input* rows_of = &n->in[0];
+  if (pending(*rows_of))
+    if (const Input* f = times_constant(pending(*rows_of), &c)) {
+      scale *= c;
+      rows_of = f;
+    }
+  const Node* per_row = tagged(*rows_of, Tag::Reduce);
+  if (!per_row || per_row->geo[0] != RT_RED_SUM || per_row->geo[1] != 1 || per_row->in[0].shape.size() != 2) return false;
+  const Node* prod = pending(per_row->in[0]);
+  if (!is_op(prod, Kind::Binary, RT_F_MUL) || prod->shape != per_row->in[0].shape) return false;
+  for (int i = 0; i < 2; ++i) {
+    const Node* ls = tagged(prod->in[i], Tag::LogSoftmax);
+    if (!ls || ls->geo[0] != 1 || ls->shape != prod->shape || prod->in[1 - i].shape != prod->shape) continue;
+    const int64_t rows = (int64_t)ls->shape[0], classes = (int64_t)ls->shape[1];
+    if (classes > 4096 || rows > (1 << 22)) return false;
+    *l = Loss{&ls->in[0], &prod->in[1 - i], rows, classes, scale, mean ? (float)rows : 1.f};
+    return true;
+  }
+  return false;
+}
+inline bool rewrite_loss(DeviceBuffer* b) {
+  Loss l;
+  if (!match_loss(b, &l)) return false;
+  const Input logits = *l.logits, targets = *l.targets;  // kept through the evaluations
+  const float *x = logits.buf->data(), *y = targets.buf->data();
+  float* out = new_block(b->ctx, b->numel);
+  const rt_status st = rt_softmax_nll_scaled(b->ctx, x, y, l.rows, l.classes, l.scale, l.divisor, out);
+  if (st != RT_OK) {
+    rt_free(b->ctx, out);
+    check(b->ctx, st);
+  }
+  b->ptr = out;
+  b->drop_node();
+  return true;
+}
+
+// max_pool2d's gradient masked by the relu in front of the pooling: one pass.
+inline bool rewrite_pool(DeviceBuffer* b) {
+  const Node* n = b->node.get();
+  if (!is_op(n, Kind::Binary, RT_F_MUL)) return false;
+  for (int i = 0; i < 2; ++i) {
+    const Node* pg = tagged(n->in[i], Tag::PoolGrad);
+    const Node* st = pending(n->in[1 - i]);
+    if (!pg || !is_op(st, Kind::Unary, RT_F_STEP) || pg->shape != n->shape || st->shape != n->shape || n->in[i].shape != n->shape) continue;
+    if (n->in[i].buf->readers.size() != 1 || pg->in.size() != 3) continue;  // in: g, idx, pooled relu output
+    if (pg->geo[10] != (int64_t)(intptr_t)st->in[0].buf.get()) continue;    // the relu's output is what was pooled
+    const auto& q = pg->geo;
+    const float *y = pg->in[2].buf->data(), *g = pg->in[0].buf->data(), *idx = pg->in[1].buf->data();
+    float* out = new_block(b->ctx, b->numel);
+    const rt_status rc = rt_relu_max_pool2x2_backward_from_output(b->ctx, y, g, idx, q[0], q[1], q[2], q[3], out);
+    if (rc != RT_OK) {
+      rt_free(b->ctx, out);
+      check(b->ctx, rc);
+    }
+    b->ptr = out;
+    b->drop_node();
+    return true;
+  }
+  return false;
+}
+// A sum of scalars, among them several classification losses of one shape: the losses of a sequence, computed in one launch.
+inline bool rewrite_loss_sum(DeviceBuffer* b) {
+  if (b->numel != 1 || !is_op(b->node.get(), Kind::Binary, RT_F_ADD)) return false;
+  std::vector<Input> leaves;  // keeps the operands alive
+  std::vector<const Node*> open{b->node.get()};
+  for (size_t i = 0; i < open.size(); ++i)
+    for (auto& in : open[i]->in) {
+      const Node* n = pending(in);
+      // a partial sum that nobody else uses belongs to this sum
+      if (is_op(n, Kind::Binary, RT_F_ADD) && in.buf->numel == 1 && in.buf->readers.size() == 1) open.push_back(n);
+      else leaves.push_back(in);
+    }
+  std::vector<Loss> losses;
+  std::vector<Input> rest;
+  for (auto& l : leaves) {
+    Loss x;
+    if (pending(l) && match_loss(l.buf.get(), &x) && (losses.empty() || x.same_kind(losses[0])) && losses.size() < 256) losses.push_back(x);
+    else rest.push_back(l);
+  }
+  if (losses.size() < 2 || rest.size() > 16) return false;
+  std::vector<const float*> xs, ys, more;
+  std::vector<Input> keep;
+  for (auto& l : losses) {
+    keep.push_back(*l.logits);
+    keep.push_back(*l.targets);
+  }
+  const Loss first = losses[0];
+  for (size_t i = 0; i < keep.size(); i += 2) {
+    xs.push_back(keep[i].buf->data());
+    ys.push_back(keep[i + 1].buf->data());
+  }
+  for (auto& r : rest) more.push_back(r.buf->data());
+  float* out = new_block(b->ctx, 1);
+  const rt_status st = rt_softmax_nll_list(b->ctx, (int)xs.size(), xs.data(), ys.data(), first.rows, first.classes, first.scale, first.divisor,
+                                           (int)more.size(), more.data(), out);
+  if (st != RT_OK) {
+    rt_free(b->ctx, out);
+    check(b->ctx, st);
+  }
+  b->ptr = out;
+  b->drop_node();
+  return true;
+}
+// Rows of a tensor that is in memory: no copy, the result points into it.
+inline bool rewrite_rows(DeviceBuffer* b) {
+  const Node* n = b->node.get();
+  if (n->kind != Kind::Slice || (n->in[0].buf->escaped && !capturing())) return false;
+  const Input& base = n->in[0];
+  if (base.buf->node && base.buf->node->kind != Kind::Opaque) return false;
+  size_t d = 0;
+  while (d < n->shape.size() && n->shape[d] == 1) ++d;  // leading extents of 1, then one free extent, then whole ones
+  for (size_t j = d + 1; j < n->shape.size(); ++j)
+    if (n->shape[j] != base.shape[j]) return false;
+  int64_t off = 0;
+  for (size_t j = 0; j < n->shape.size(); ++j) off = off * (int64_t)base.shape[j] + (int64_t)n->starts[j];
+  std::shared_ptr<DeviceBuffer> root = base.buf;
+  const float* p = root->data();
+  while (root->owner) root = root->owner;
+  b->ptr = const_cast<float*>(p) + off;
+  b->owner = root;
+  b->drop_node();
+  return true;
+}
+inline bool rewrite(DeviceBuffer* b) {
+  if (b->node->kind == Kind::Const) return false;
+  return rewrite_rows(b) || rewrite_linear(b) || rewrite_loss(b) || rewrite_loss_sum(b) || rewrite_pool(b);
+}
+
+}  // namespace lazy
+
+inline void lazy_evaluate(DeviceBuffer* b) {
+  using namespace lazy;
+  if (!b->node) return;
+  std::shared_ptr<DeviceBuffer> guard = b->shared_from_this();
+  if (rewrite(b)) return;
+  if (b->node->kind == Kind::Opaque) {
+    b->node->run(*b->node, b);
+    b->drop_node();
+    return;
+  }
+  const bool lone = (b->node->kind == Kind::Unary || b->node->kind == Kind::Binary) &&
+                    std::all_of(b->node->in.begin(), b->node->in.end(), [](const Input& i) { return !i.buf->node; });
+  if ((lone || b->node->kind == Kind::Const) && evaluate_alone(b)) return;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    rt_fused_program p;
+    Compiler c;
+    std::vector<DeviceBuffer*> outs;
+    if (c.build(b, &p, &outs)) {
+      std::vector<float*> blocks;
+      rt_status st = RT_OK;
+      for (size_t k = 0; k < outs.size(); ++k) {
+        void* q = nullptr;
+        st = rt_malloc(b->ctx, sizeof(float) * std::max<size_t>(b->numel, 1), &q);
+        if (st != RT_OK) break;
+        blocks.push_back((float*)q);
+        p.out[k] = (float*)q;
+      }
+      if (st == RT_OK) st = rt_fused_elementwise(b->ctx, &p);
+      if (st != RT_OK) {
+        for (float* q : blocks) rt_free(b->ctx, q);
+        check(b->ctx, st);
+      }
+      std::vector<std::shared_ptr<DeviceBuffer>> keep;
+      for (auto* o : outs) keep.push_back(o->shared_from_this());
+      for (size_t k = 0; k < outs.size(); ++k) {
+        outs[k]->ptr = blocks[k];
+        outs[k]->drop_node();
+      }
+      return;
+    }
+    // too long, or more dimensions than the kernel walks: evaluate what lies below first
+    for (auto& i : b->node->in) i.buf->data();
+  }
+  if (!evaluate_alone(b)) throw Error::internal("an elementwise op could not be evaluated");
+}
+
+}  // namespace rt

@@ -1,0 +1,98 @@
+"""Deferred elementwise ops (one kernel per chain) against the oracle, which computes op by op: chains whose program is compiled
+ahead of time and ones that are interpreted, groups of four elements and single ones, windows, broadcasts and reductions in
+between, operands changed in place between an op and its evaluation."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+from helpers import assert_close
+
+pytestmark = pytest.mark.gpu
+
+# one element; rows of fewer / exactly / more than four; an odd row length; one tile of 512 elements and one more; above the size
+# up to which shared intermediate results are kept
+SHAPES = [(1, 1), (3, 3), (5, 4), (7, 36), (64, 577), (4, 128), (3, 171), (1100, 1000)]
+
+
+@pytest.fixture(scope="module")
+def engines():
+    import rusttensor_b200
+
+    return rusttensor_b200.engine(), oracle.engine()
+
+
+def chain(e, x, b, col):
+    o = e.ops
+    rows, cols = x.shape
+    t = o.tanh(o.add(o.mul(x, b), col))
+    u = o.div(o.sin(x), o.add(o.square(x), e.tensor(np.float32(1.5), ())))
+    v = o.elu(o.clip(o.sub(t, u), -0.7, 0.9), 0.5)
+    w = o.slice(o.softplus(v), [(0, rows), (cols // 2, cols)])
+    z = o.concat([w, o.sigmoid(x), w], 1)
+    return o.maximum(o.mul_scalar(z, -0.5), o.exp(o.mul_scalar(o.square(z), -1.0))), t, v
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_chain_forward_and_backward(engines, shape):
+    r = np.random.default_rng(shape[0] * 31 + shape[1])
+    data = [r.standard_normal(s).astype(np.float32) for s in (shape, shape[1:], (shape[0], 1))]
+    out = []
+    for e in engines:
+        x, b, col = (e.tensor(d, requires_grad=True) for d in data)
+        y, t, v = chain(e, x, b, col)
+        loss = e.ops.add(e.ops.mean(y), e.ops.sum(e.ops.logsumexp(v, 1)))
+        loss.backward()
+        out.append([y, v, t, loss] + [p.grad for p in (x, b, col)])
+    for got, ref in zip(*out):
+        assert_close(got.numpy(), ref.numpy())
+
+
+@pytest.mark.parametrize("shape", SHAPES[:-1])
+def test_operands_changed_in_place_after_the_op(engines, shape):
+    r = np.random.default_rng(7)
+    a, b = (r.standard_normal(shape).astype(np.float32) for _ in range(2))
+    out = []
+    for e in engines:
+        x = e.tensor(a, requires_grad=True)
+        y = e.ops.exp(e.ops.mul_scalar(x, 0.5))  # not asked for before x changes
+        loss = e.ops.mean(e.ops.square(x))
+        loss.backward()
+        x.update_from_host(b)
+        z = e.ops.tanh(x)
+        e.Sgd([x], 0.1).step()
+        out.append([y, z, x])
+    for got, ref in zip(*out):
+        assert_close(got.numpy(), ref.numpy())
+
+
+@pytest.mark.parametrize("rows,classes", [(1, 2), (7, 16), (33, 17), (64, 65), (5, 300)])
+@pytest.mark.parametrize("steps", [1, 2, 205])
+def test_losses_of_a_sequence(engines, rows, classes, steps):
+    r = np.random.default_rng(rows + classes + steps)
+    h = r.standard_normal((steps, rows, 9)).astype(np.float32)
+    w, bias = r.standard_normal((9, classes)).astype(np.float32), r.standard_normal(classes).astype(np.float32)
+    y = np.eye(classes, dtype=np.float32)[r.integers(0, classes, (steps, rows))]
+    out = []
+    for e in engines:
+        tw, tb = e.tensor(w, requires_grad=True), e.tensor(bias, requires_grad=True)
+        total = None
+        for t in range(steps):
+            logits = e.ops.add(e.ops.matmul(e.tensor(h[t]), tw), e.ops.broadcast_to(tb, (rows, classes)))
+            loss = e.ops.softmax_cross_entropy(logits, e.tensor(y[t]), 1)
+            total = loss if total is None else e.ops.add(total, loss)
+        total.backward()
+        out.append([total, tw.grad, tb.grad])
+    for got, ref in zip(*out):
+        assert_close(got.numpy(), ref.numpy())
+
+
+def test_a_malformed_program_is_refused():
+    from rusttensor_b200 import CApi
+    from rusttensor_b200.capi import RtError
+
+    api = CApi()
+    with pytest.raises(RtError):
+        api.call("fused_elementwise", C.create_string_buffer(8192))  # zero dimensions, no outputs
+    api.close()
