@@ -21,6 +21,8 @@ rt_status rt_gemm_tc_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, 
 
 rt_status rt_gemm_small_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
                                  const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
+rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
+                               int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
 rt_status rt_gemm_small_list_internal(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k,
                                       const float* b, const float* bias, int act);
 rt_status rt_gemm_list_tc_internal(rt_ctx* ctx, int count, const float* const* a, const float* const* g, int64_t m, int64_t k, int64_t n,
@@ -629,6 +631,12 @@ extern "C" {
 static bool small_product(int64_t m, int64_t n, int64_t k) {
   return k > 0 && k <= 2048 && m * n * k <= (32ll << 20);
 }
+// Products for the TMA-fed tensor-core kernel (k_gemm_tma.cu), which has no split of the reduction: from about 48 tiles of 128 x 128 on
+// it is ahead of the kernels with one (1024 x 256 x 1024, 64 tiles: 15 against 20 us; 700 x 1500 x 900, 48 tiles: 42 against 43 - 58 us;
+// 512^3, 16 tiles: 19 against 10 us).
+static bool large_product(rt_ctx* ctx, int64_t m, int64_t n, int64_t k) {
+  return ctx->use_tensor_cores && k >= 64 && n >= 48 && ((m + 127) / 128) * ((n + 127) / 128) >= 48;
+}
 rt_status rt_gemm_bias_act(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb,
                            const float* bias, int act, float* c, int64_t ldc) {
   RT_CHECK_CTX(ctx);
@@ -639,6 +647,10 @@ rt_status rt_gemm_bias_act(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const f
   RT_CHECK_PTR(ctx, c);
   if (small_product(m, n, k)) {
     rt_status st = rt_gemm_small_internal(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, bias, act, 0);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
+  if (large_product(ctx, m, n, k)) {
+    rt_status st = rt_gemm_tma_internal(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, bias, act, 0);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   rt_status st = rt_gemm(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, 0);
@@ -732,6 +744,10 @@ rt_status rt_gemm(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, i
   }
   if (small_product(m, n, k)) {
     rt_status st = rt_gemm_small_internal(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, nullptr, RT_ACT_NONE, accumulate);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
+  if (large_product(ctx, m, n, k)) {
+    rt_status st = rt_gemm_tma_internal(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, nullptr, RT_ACT_NONE, accumulate);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   if (ctx->use_tensor_cores && k >= 32 && m >= 32 && n >= 16 && m * n * k >= (1ll << 20)) {

@@ -38,7 +38,14 @@ def test_small_product(api, m, k, n, trans):
         close(c.numpy(), a.astype(np.float64) @ b + accumulate * c0, np.sqrt(k))
 
 
-@pytest.mark.parametrize("m,k,n", SIZES + [(300, 784, 300)])
+# one more than whole tiles and K-blocks, rows that TMA cannot fetch directly, 256- and 128-column tiles, chunks of 1, 2 and 4 K-blocks
+@pytest.mark.parametrize("m,k,n", [(769, 65, 1025), (1024, 64, 768), (1030, 1024, 900), (6200, 100, 70), (2100, 2081, 1900)])
+@pytest.mark.parametrize("trans", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_large_product(api, m, k, n, trans):
+    test_small_product(api, m, k, n, trans)
+
+
+@pytest.mark.parametrize("m,k,n", SIZES + [(300, 784, 300), (900, 70, 1000)])
 @pytest.mark.parametrize("act", [0, 1, 2, 3])
 def test_linear_layer(api, m, k, n, act):
     r = np.random.default_rng(m + k + n + act)
