@@ -23,6 +23,8 @@ rt_status rt_gemm_small_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t 
                                  const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
 rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
                                int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
+rt_status rt_conv_forward_tma_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y);
+rt_status rt_conv_gather_tma_internal(rt_ctx* ctx, const float* y, const float* w, const float* bias, const ConvGeom& g, int cm, float* out);
 rt_status rt_gemm_small_list_internal(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k,
                                       const float* b, const float* bias, int act);
 rt_status rt_gemm_list_tc_internal(rt_ctx* ctx, int count, const float* const* a, const float* const* g, int64_t m, int64_t k, int64_t n,
@@ -508,7 +510,9 @@ rt_status conv_forward_like(rt_ctx* ctx, const float* x, const float* w, const f
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   if (ctx->use_tensor_cores) {
-    rt_status st = rt_conv_forward_tc_internal(ctx, x, w, bias, g, y);
+    rt_status st = rt_conv_forward_tma_internal(ctx, x, w, bias, g, y);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+    st = rt_conv_forward_tc_internal(ctx, x, w, bias, g, y);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   MatA<false> la{w, K};
@@ -555,7 +559,9 @@ rt_status conv_gather_like(rt_ctx* ctx, const float* y, const float* w, const fl
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   if (ctx->use_tensor_cores) {
-    rt_status st = rt_conv_gather_tc_internal(ctx, y, w, bias, g, cm, out);
+    rt_status st = rt_conv_gather_tma_internal(ctx, y, w, bias, g, cm, out);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+    st = rt_conv_gather_tc_internal(ctx, y, w, bias, g, cm, out);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   WeightSecondIndexA la{w, cm, g};

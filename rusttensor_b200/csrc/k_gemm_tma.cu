@@ -36,22 +36,27 @@ constexpr int kThreads = (kEpilogueWarps + kConverterWarps + 2) * 32;  // 512: 1
 constexpr int kTmaWarp = kEpilogueWarps + kConverterWarps, kMmaWarp = kTmaWarp + 1;
 constexpr uint32_t kARaw = BM * BK * 4;  // 16 KB
 
-template <int BN>
+// SPLIT: B comes as two matrices, hi and lo (the packed weights of a convolution, used by every tile).
+template <int BN, bool SPLIT>
 struct Config {
   static constexpr int NU = BN < 128 ? BN : 128;  // columns of one MMA and of one accumulator
   static constexpr int halves = BN / NU;
-  static constexpr int NC = halves == 2 ? NU : NU / 2;  // columns that one accumulating thread sums
+  // The two groups of accumulating warps: each takes one half of a 256-column tile; or they take turns, a tile each, so that one writes a
+  // result while the other sums the next tile (convolutions: short reductions, scattered stores); or each takes half the columns.
+  static constexpr bool turns = SPLIT;
+  static constexpr int NC = halves == 2 || turns ? NU : NU / 2;
   static constexpr int ACC = BN == 256 ? 3 : 2;   // accumulators, used in turn
-  static constexpr int R = BN == 256 ? 3 : 4;     // raw A and B tiles in flight
   static constexpr int L = BN == 256 ? 2 : 4;     // converted A (tensor memory) and B lo
   static constexpr uint32_t b_raw = BN * BK * 4;
-  static constexpr uint32_t raw = kARaw + b_raw;
+  static constexpr uint32_t raw = kARaw + (SPLIT ? 2 : 1) * b_raw;
+  static constexpr int R = BN == 256 ? 3 : (BN == 64 && SPLIT ? 6 : 4);  // raw tiles in flight
   static constexpr uint32_t lo_offset = R * raw;
-  static constexpr uint32_t stage_offset = lo_offset + L * b_raw;  // result: one 32 x 17 tile per accumulating warp
+  static constexpr uint32_t stage_offset = lo_offset + (SPLIT ? 0 : L * b_raw);  // result: one 32 x 17 tile per accumulating warp
   static constexpr uint32_t bar_offset = stage_offset + kEpilogueWarps * 32 * 17 * 4;
-  static constexpr int n_bars = 2 * R + 2 * L + 2 * ACC;
+  static constexpr int n_bars = 2 * R + 2 * L + 3 * ACC;
   static constexpr uint32_t total = bar_offset + n_bars * 8 + 16 + 1024;  // + alignment of the base to 1024
   static constexpr uint32_t a_cols = 2 * BK;                              // tensor-memory columns of a converted A block
+  static constexpr int converters = SPLIT ? 4 : kConverterWarps;
   static_assert(ACC * NU + L * a_cols <= 512, "tensor memory");
   static_assert(total <= 232448, "shared memory");
 };
@@ -131,11 +136,11 @@ __device__ __forceinline__ float activated(float v, int act) {
   return v;
 }
 
-template <int BN>
+template <int BN, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p, int* status) {
   extern __shared__ char smem_raw[];
-  using C = Config<BN>;
+  using C = Config<BN, SPLIT>;
   __shared__ volatile int abort_flag;
   const uint32_t raw_base = smem_u32(smem_raw);
   const uint32_t base = (raw_base + 1023) & ~1023u;
@@ -146,8 +151,10 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   auto raw_empty = [&](int i) { return bars + 8 * (C::R + i); };
   auto conv_full = [&](int i) { return bars + 8 * (2 * C::R + i); };
   auto conv_empty = [&](int i) { return bars + 8 * (2 * C::R + C::L + i); };
-  auto acc_full = [&](int i) { return bars + 8 * (2 * C::R + 2 * C::L + i); };
-  auto acc_empty = [&](int i) { return bars + 8 * (2 * C::R + 2 * C::L + C::ACC + i); };
+  // one "full" barrier per accumulator and group of accumulating warps: a group sees only the uses that are its own, so that the phases
+  // of its barriers follow them
+  auto acc_full = [&](int group, int i) { return bars + 8 * (2 * C::R + 2 * C::L + group * C::ACC + i); };
+  auto acc_empty = [&](int i) { return bars + 8 * (2 * C::R + 2 * C::L + 2 * C::ACC + i); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::bar_offset + C::n_bars * 8);
 
   if (threadIdx.x == 0) {
@@ -157,12 +164,13 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       mbar_init(raw_empty(i), 1);
     }
     for (int i = 0; i < C::L; ++i) {
-      mbar_init(conv_full(i), kConverterWarps);
+      mbar_init(conv_full(i), C::converters);
       mbar_init(conv_empty(i), 1);
     }
     for (int i = 0; i < C::ACC; ++i) {
-      mbar_init(acc_full(i), 1);
-      mbar_init(acc_empty(i), C::halves == 2 ? kEpilogueWarps / 2 : kEpilogueWarps);
+      mbar_init(acc_full(0, i), 1);
+      mbar_init(acc_full(1, i), 1);
+      mbar_init(acc_empty(i), C::halves == 2 || C::turns ? kEpilogueWarps / 2 : kEpilogueWarps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -198,6 +206,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           else if (p.a_mode == kRowsMajorM) load_2d(dst, &map_a, mt * BM, kb * BK, raw_full(s));
           else load_4d(dst, &map_a, cb * BK, x0 + kx, y0 + ky, n0, raw_full(s));
           load_2d(dst + kARaw, &map_b, kb * BK, nt * BN, raw_full(s));
+          if (SPLIT) load_2d(dst + kARaw + C::b_raw, &map_b, kb * BK, p.N + nt * BN, raw_full(s));
           if (++cb == p.c_blocks) {
             cb = 0;
             if (++kx == p.kw) {
@@ -215,8 +224,8 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     // ---------------- MMAs ----------------
     constexpr uint32_t idesc = make_idesc(C::NU);
     constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // 8-row groups of 1024 bytes, 128-byte swizzle
-    int it = 0, chunks = 0;  // chunks that are complete
-    for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+    int it = 0, chunks = 0, t = 0;  // chunks that are complete
+    for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++t) {
       for (int kb = 0, in_chunk = 0; kb < p.k_blocks && ok; ++kb, ++it) {
         const int s = it % C::R, l = it % C::L;
         const bool first = in_chunk == 0, last = ++in_chunk == p.chunk || kb + 1 == p.k_blocks;
@@ -226,7 +235,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (!ok) break;
         tc_fence_after();
         const uint32_t b_hi = ((base + s * C::raw + kARaw) >> 4 & 0x3FFF) | (1u << 16);
-        const uint32_t b_lo = ((base + C::lo_offset + l * C::b_raw) >> 4 & 0x3FFF) | (1u << 16);
+        const uint32_t b_lo = ((SPLIT ? base + s * C::raw + kARaw + C::b_raw : base + C::lo_offset + l * C::b_raw) >> 4 & 0x3FFF) | (1u << 16);
         const uint32_t a_hi = tmem_a + l * C::a_cols, a_lo = a_hi + BK;
 #pragma unroll
         for (int h = 0; h < C::halves; ++h) {
@@ -241,7 +250,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             for (int j = 0; j < BK / 8; ++j)
               mma_step(tmem + acc * C::NU, a_hi + 8 * j, a_lo + 8 * j, b_hi + h * half_rows + 2 * j, b_lo + h * half_rows + 2 * j, desc_hi, idesc,
                        first && j == 0 ? 0u : 1u);
-            if (last) umma_commit_elect(acc_full(acc));
+            if (last) umma_commit_elect(acc_full(C::halves == 2 ? h : (C::turns ? t & 1 : 0), acc));
           }
         }
         if (ok) {
@@ -251,7 +260,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (last) ++chunks;
       }
     }
-  } else if (warp >= kEpilogueWarps && warp < kTmaWarp) {
+  } else if (warp >= kEpilogueWarps && warp < kEpilogueWarps + C::converters) {
     // ---------------- converters ----------------
     // Four of the six convert A (a row a thread; tensor-memory lanes 32 * (warp % 4) ..) and a smaller share of B than the other two.
     const int cw = warp - kEpilogueWarps, row = cw * 32 + lane;
@@ -296,7 +305,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const float4* b = reinterpret_cast<const float4*>(a + kARaw);
         float4* bl = reinterpret_cast<float4*>(smem + C::lo_offset + l * C::b_raw);
 #pragma unroll 5
-        for (int j = b_begin; j < b_end; j += 32) {
+        for (int j = b_begin; !SPLIT && j < b_end; j += 32) {
           const float4 v = b[j];
           bl[j] = make_float4(__uint_as_float(low_part(v.x)), __uint_as_float(low_part(v.y)), __uint_as_float(low_part(v.z)),
                               __uint_as_float(low_part(v.w)));
@@ -311,19 +320,23 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   } else if (warp < kEpilogueWarps) {
     // ---------------- sums over the K-blocks, result ----------------
     float* stage = reinterpret_cast<float*>(smem + C::stage_offset) + warp * 32 * 17;
-    const int quad = warp & 3, group = warp >> 2;
-    const int col0 = C::halves == 2 ? group * C::NU : group * C::NC;  // of this warp's columns in the tile
-    int it = 0;
-    for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+    const int quad = warp & 3, group = warp >> 2, full = C::halves == 2 || C::turns ? group : 0;
+    const int col0 = C::halves == 2 ? group * C::NU : (C::turns ? 0 : group * C::NC);  // of this warp's columns in the tile
+    const int chunks = (p.k_blocks + p.chunk - 1) / p.chunk;  // of a tile
+    int t = 0;
+    uint32_t phases = 0;  // bit i: parity of this group's next use of accumulator i
+    for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++t) {
+      if (C::turns && (t & 1) != group) continue;
       float sum[C::NC];
 #pragma unroll
       for (int j = 0; j < C::NC; ++j) sum[j] = 0.f;
-      for (int kb = 0; kb < p.k_blocks && ok; kb += p.chunk, ++it) {
-        const int unit = C::halves == 2 ? 2 * it + group : it, acc = unit % C::ACC, use = unit / C::ACC;
-        ok = __all_sync(0xffffffffu, wait(acc_full(acc), use & 1, status, 48, &abort_flag));
+      for (int i = 0; i < chunks && ok; ++i) {
+        const int unit = (t * chunks + i) * C::halves + (C::halves == 2 ? group : 0), acc = unit % C::ACC;
+        ok = __all_sync(0xffffffffu, wait(acc_full(full, acc), (phases >> acc) & 1, status, 48, &abort_flag));
         if (!ok) break;
+        phases ^= 1u << acc;
         tc_fence_after();
-        const uint32_t d = tmem + acc * C::NU + (C::halves == 2 ? 0 : group * C::NC) + ((uint32_t)(quad * 32) << 16);
+        const uint32_t d = tmem + acc * C::NU + (C::halves == 2 ? 0 : col0) + ((uint32_t)(quad * 32) << 16);
 #pragma unroll
         for (int c = 0; c < C::NC; c += 16) {
           uint32_t v[16];
@@ -340,7 +353,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
       if (!ok) break;
       const int mt = tile % p.m_tiles, n0 = tile / p.m_tiles * BN + col0, n_left = p.N - n0;
-      if (BN <= 128 && p.a_mode == kPixels) {
+      if (SPLIT) {
         const int tw = mt % p.tiles_w, r = mt / p.tiles_w, row = quad * 32 + lane;
         const int w = row % p.bw, q = row / p.bw;
         const int x = tw * p.bw + w, y = r % p.tiles_h * p.bh + q % p.bh, n = r / p.tiles_h * p.bn + q / p.bh;
@@ -411,13 +424,43 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ src
     if (r < rows && c < cols) d[(int64_t)c * ldd + r] = tile[tx][ty + j];
   }
 }
-// B operand of a convolution: row n, column ((ky * kw + kx) * c_blocks + channel block) * 32 + channel; zeros behind the last channel.
+// The transpose with 128-bit accesses on both sides: a block turns 32 rows x 128 columns, four independent loads a thread.  16-byte aligned
+// pointers and rows on both sides; bound by memory bandwidth (103 MB turned: see the figures at channels_last).
+__global__ void __launch_bounds__(256) transpose4_kernel(const float* __restrict__ src, float* __restrict__ dst, int rows, int cols, int64_t lds, int64_t ldd,
+                                                         int64_t batch_src, int64_t batch_dst) {
+  __shared__ float tile[32][129];
+  const float* s = src + (int64_t)blockIdx.z * batch_src;
+  float* d = dst + (int64_t)blockIdx.z * batch_dst;
+  const int c0 = blockIdx.x * 128, r0 = blockIdx.y * 32;
+  float4 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + (threadIdx.x >> 5) + 8 * i, c = c0 + (threadIdx.x & 31) * 4;
+    v[i] = r < rows && c < cols ? __ldcs(reinterpret_cast<const float4*>(s + (int64_t)r * lds + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float* t = &tile[(threadIdx.x >> 5) + 8 * i][(threadIdx.x & 31) * 4];
+    t[0] = v[i].x; t[1] = v[i].y; t[2] = v[i].z; t[3] = v[i].w;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = (threadIdx.x >> 3) + 32 * i, r = (threadIdx.x & 7) * 4;
+    if (c0 + c < cols && r0 + r < rows)
+      *reinterpret_cast<float4*>(d + (int64_t)(c0 + c) * ldd + r0 + r) = make_float4(tile[r][c], tile[r + 1][c], tile[r + 2][c], tile[r + 3][c]);
+  }
+}
+// B operand of a convolution, hi rows and then lo rows: row n, column ((ky * kw + kx) * c_blocks + channel block) * 32 + channel; zeros
+// behind the last channel.
 __global__ void __launch_bounds__(256) pack_taps_kernel(const float* __restrict__ w, float* __restrict__ dst, int N, int C, int c_blocks, int kw, int taps,
                                                         int64_t sn, int64_t sc, int64_t sky, int64_t skx, int64_t off0) {
   const int64_t cols = (int64_t)taps * c_blocks * BK;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N * cols; i += (int64_t)gridDim.x * blockDim.x) {
     const int n = (int)(i / cols), k = (int)(i % cols), tap = k / (c_blocks * BK), c = k % (c_blocks * BK);
-    dst[i] = c < C ? __ldg(w + n * sn + c * sc + tap / kw * sky + tap % kw * skx + off0) : 0.f;
+    const float v = c < C ? __ldg(w + n * sn + c * sc + tap / kw * sky + tap % kw * skx + off0) : 0.f;
+    dst[i] = v;
+    dst[N * cols + i] = __uint_as_float(low_part(v));
   }
 }
 
@@ -444,10 +487,10 @@ inline bool map_matrix(CUtensorMap* m, const float* t, int64_t cols, int64_t row
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
+template <int BN, bool SPLIT = false>
 rt_status launch(rt_ctx* ctx, const CUtensorMap& a, const CUtensorMap& b, const Params& p) {
-  using C = Config<BN>;
-  auto kern = tma_gemm_kernel<BN>;
+  using C = Config<BN, SPLIT>;
+  auto kern = tma_gemm_kernel<BN, SPLIT>;
   static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::total);
   if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "tensor-core product: %s", cudaGetErrorString(set));
   kern<<<p.tiles < ctx->sm_count ? p.tiles : ctx->sm_count, kThreads, C::total, ctx->stream>>>(a, b, p, ctx->device_status);
@@ -462,7 +505,10 @@ inline int64_t up4(int64_t v) { return (v + 3) & ~int64_t(3); }
 inline rt_status pack(rt_ctx* ctx, const float* src, float* dst, int64_t rows, int64_t cols, int64_t lds, int64_t ldd, bool transpose, int64_t batch,
                       int64_t batch_src, int64_t batch_dst) {
   const dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32), (unsigned)batch);
-  if (transpose) pack_kernel<true><<<grid, 256, 0, ctx->stream>>>(src, dst, (int)rows, (int)cols, lds, ldd, batch_src, batch_dst);
+  if (transpose && rt_aligned16(src) && rt_aligned16(dst) && ((rows | cols | lds | ldd | batch_src | batch_dst) & 3) == 0)
+    transpose4_kernel<<<dim3((unsigned)((cols + 127) / 128), grid.y, grid.z), 256, 0, ctx->stream>>>(src, dst, (int)rows, (int)cols, lds, ldd, batch_src,
+                                                                                                    batch_dst);
+  else if (transpose) pack_kernel<true><<<grid, 256, 0, ctx->stream>>>(src, dst, (int)rows, (int)cols, lds, ldd, batch_src, batch_dst);
   else pack_kernel<false><<<grid, 256, 0, ctx->stream>>>(src, dst, (int)rows, (int)cols, lds, ldd, batch_src, batch_dst);
   RT_LAUNCHED(ctx);
   return RT_OK;
@@ -529,4 +575,140 @@ rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m,
   p.chunk = chunk_of(k);
   p.kw = 1;
   return wide ? launch<256>(ctx, ma, mb, p) : launch<128>(ctx, ma, mb, p);
+}
+
+namespace tc {
+namespace tma {
+
+// A convolution-shaped product over the pixels (n, y, x) of the row side: out(n, co, y * osy + oy, x * osx + ox) (+ bias) =
+// sum over taps and channels of src(n, c, y * sy - py + ky, x * sx - px + kx) * w(co, c, ky, kx), zeros outside the source.
+struct PixelProduct {
+  int Nb, C, H, W;                      // source
+  int rows_h, rows_w;                   // row side
+  int N, kh, kw, sy, sx, py, px;
+  const float* w;                       // element (co, c, ky, kx) at co * sn + c * sc + ky * sky + kx * skx + off0
+  int64_t sn, sc, sky, skx, off0;
+  const float* bias;
+  float* out;
+  int out_h, out_w, osy, osx, oy, ox;
+};
+
+// The box of 128 pixels (powers of two) that wastes least at the edges; short runs along a row make scattered stores.
+inline void choose_box(int w, int h, int n, int* bw, int* bh, int* bn) {
+  double best = -1;
+  for (int a = 1; a <= 128; a *= 2)
+    for (int b = 1; a * b <= 128; b *= 2) {
+      const int c = 128 / (a * b);
+      auto used = [](int extent, int box) { return (double)extent / ((extent + box - 1) / box * box); };
+      const double score = used(w, a) * used(h, b) * used(n, c) * (a >= 8 ? 1.0 : (a == 4 ? 0.9 : (a == 2 ? 0.7 : 0.5)));
+      if (score > best + 1e-9) {
+        best = score;
+        *bw = a;
+        *bh = b;
+        *bn = c;
+      }
+    }
+}
+
+// src in channels-last form: [Nb][H * W][up4(C)].
+inline rt_status channels_last(rt_ctx* ctx, const float* src, int Nb, int C, int64_t hw, RtScratch* ws) {
+  const int64_t cp = up4(C);
+  rt_status st = ws->alloc(sizeof(float) * (size_t)Nb * hw * cp);
+  if (st != RT_OK) return st;
+  for (int n = 0; n < Nb && st == RT_OK; n += 32768)
+    st = pack(ctx, src + (int64_t)n * C * hw, ws->as<float>() + (int64_t)n * hw * cp, C, hw, hw, cp, true, Nb - n < 32768 ? Nb - n : 32768, C * hw, hw * cp);
+  return st;
+}
+
+inline rt_status pixel_product(rt_ctx* ctx, const PixelProduct& q, const float* nhwc) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return RT_ERR_UNIMPLEMENTED;
+  Params p{};
+  p.a_mode = kPixels;
+  choose_box(q.rows_w, q.rows_h, q.Nb, &p.bw, &p.bh, &p.bn);
+  const int64_t cp = up4(q.C);
+  CUtensorMap ma, mb;
+  const cuuint64_t dims[4] = {(cuuint64_t)q.C, (cuuint64_t)q.W, (cuuint64_t)q.H, (cuuint64_t)q.Nb};
+  const cuuint64_t strides[3] = {(cuuint64_t)cp * 4, (cuuint64_t)q.W * cp * 4, (cuuint64_t)q.H * q.W * cp * 4};
+  const cuuint32_t box[4] = {BK, (cuuint32_t)((p.bw - 1) * q.sx + 1), (cuuint32_t)((p.bh - 1) * q.sy + 1), (cuuint32_t)p.bn};
+  const cuuint32_t step[4] = {1, (cuuint32_t)q.sx, (cuuint32_t)q.sy, 1};
+  if (box[1] > 256 || box[2] > 256) return RT_ERR_UNIMPLEMENTED;
+  if (enc(&ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(nhwc), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return RT_ERR_UNIMPLEMENTED;
+  const int bn_cols = q.N <= 64 ? 64 : 128;
+  p.c_blocks = (q.C + BK - 1) / BK;
+  p.kw = q.kw;
+  p.k_blocks = p.c_blocks * q.kh * q.kw;
+  const int64_t cols = (int64_t)p.k_blocks * BK;
+  RtScratch wb(ctx);
+  rt_status st = wb.alloc(sizeof(float) * (size_t)(2 * q.N * cols));
+  if (st != RT_OK) return st;
+  pack_taps_kernel<<<rt_grid_for(ctx, q.N * cols, 256), 256, 0, ctx->stream>>>(q.w, wb.as<float>(), q.N, q.C, p.c_blocks, q.kw, q.kh * q.kw, q.sn, q.sc, q.sky,
+                                                                               q.skx, q.off0);
+  RT_LAUNCHED(ctx);
+  if (!map_matrix(&mb, wb.as<float>(), cols, 2 * q.N, cols, BK, bn_cols, true)) return RT_ERR_UNIMPLEMENTED;
+  p.tiles_w = (q.rows_w + p.bw - 1) / p.bw;
+  p.tiles_h = (q.rows_h + p.bh - 1) / p.bh;
+  p.rows_w = q.rows_w;
+  p.rows_h = q.rows_h;
+  p.rows_n = q.Nb;
+  p.m_tiles = p.tiles_w * p.tiles_h * ((q.Nb + p.bn - 1) / p.bn);
+  p.tiles = p.m_tiles * ((q.N + bn_cols - 1) / bn_cols);
+  p.N = q.N;
+  p.c = q.out;
+  p.bias = q.bias;
+  const int64_t k = (int64_t)q.C * q.kh * q.kw;
+  p.chunk = k < 512 ? 2 : (k < 1024 ? 3 : 4);  // the gather kernel's errors: 6e-7 at 300, 9e-7 at 576, 1.5e-6 at 1152
+  p.sx = q.sx; p.sy = q.sy; p.px = q.px; p.py = q.py;
+  p.out_h = q.out_h; p.out_w = q.out_w; p.osx = q.osx; p.osy = q.osy; p.ox = q.ox; p.oy = q.oy;
+  return bn_cols == 64 ? launch<64, true>(ctx, ma, mb, p) : launch<128, true>(ctx, ma, mb, p);
+}
+
+// Which convolutions: a whole wave of tiles, enough channels to fill most of a block of 32, strides that TMA steps over.
+inline bool worth_it(rt_ctx* ctx, int64_t pixels, int C, int N, int sy, int sx, int H, int W) {
+  return pixels >= 128ll * ctx->sm_count && pixels < (1ll << 31) && C >= 16 && N >= 16 && sy <= 8 && sx <= 8 && (int64_t)H * W < (1ll << 31);
+}
+
+}  // namespace tma
+}  // namespace tc
+
+// y[Nb,Cy,Hy,Wy] = conv(x, w[Cy,Cx,kh,kw]) (+ bias).
+rt_status rt_conv_forward_tma_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y) {
+  using namespace tc::tma;
+  if (!worth_it(ctx, (int64_t)g.Nb * g.Hy * g.Wy, g.Cx, g.Cy, g.sh, g.sw, g.Hx, g.Wx)) return RT_ERR_UNIMPLEMENTED;
+  RtScratch ws(ctx);
+  rt_status st = channels_last(ctx, x, g.Nb, g.Cx, (int64_t)g.Hx * g.Wx, &ws);
+  if (st != RT_OK) return st;
+  const int64_t taps = (int64_t)g.kh * g.kw;
+  PixelProduct q{g.Nb, g.Cx, g.Hx, g.Wx, g.Hy, g.Wy, g.Cy, g.kh, g.kw, g.sh, g.sw, g.ph, g.pw, w, g.Cx * taps, taps, g.kw, 1, 0, bias, y,
+                 g.Hy, g.Wy, 1, 1, 0, 0};
+  return pixel_product(ctx, q, ws.as<float>());
+}
+
+// out[Nb,Cm,Hx,Wx] (+ bias) = gather of y[Nb,Cy,Hy,Wy] with w[Cy,Cm,kh,kw]: input gradient of a convolution, forward of a transposed one.
+// The outputs of one stride phase (iy % sh, ix % sw) only meet the taps ky = ky0 + sh * a, kx = kx0 + sw * b; with those the phase is a
+// unit-stride convolution of y with the kernel turned round that writes every sh-th / sw-th output.
+rt_status rt_conv_gather_tma_internal(rt_ctx* ctx, const float* y, const float* w, const float* bias, const ConvGeom& g, int cm, float* out) {
+  using namespace tc::tma;
+  if (!worth_it(ctx, (int64_t)g.Nb * g.Hx * g.Wx / (g.sh * g.sw), g.Cy, cm, 1, 1, g.Hy, g.Wy)) return RT_ERR_UNIMPLEMENTED;
+  for (int ry = 0; ry < g.sh; ++ry)  // every phase needs a tap (otherwise its outputs are the bias alone)
+    if ((ry + g.ph) % g.sh >= g.kh) return RT_ERR_UNIMPLEMENTED;
+  for (int rx = 0; rx < g.sw; ++rx)
+    if ((rx + g.pw) % g.sw >= g.kw) return RT_ERR_UNIMPLEMENTED;
+  RtScratch ws(ctx);
+  rt_status st = channels_last(ctx, y, g.Nb, g.Cy, (int64_t)g.Hy * g.Wy, &ws);
+  const int64_t taps = (int64_t)g.kh * g.kw;
+  for (int ry = 0; ry < g.sh && st == RT_OK; ++ry)
+    for (int rx = 0; rx < g.sw && st == RT_OK; ++rx) {
+      const int rows_h = (g.Hx - ry + g.sh - 1) / g.sh, rows_w = (g.Wx - rx + g.sw - 1) / g.sw;
+      if (rows_h <= 0 || rows_w <= 0) continue;
+      const int ky0 = (ry + g.ph) % g.sh, kx0 = (rx + g.pw) % g.sw;
+      const int nay = (g.kh - ky0 + g.sh - 1) / g.sh, nax = (g.kw - kx0 + g.sw - 1) / g.sw;
+      const int py = (nay - 1) - (ry + g.ph - ky0) / g.sh, px = (nax - 1) - (rx + g.pw - kx0) / g.sw;
+      PixelProduct q{g.Nb, g.Cy, g.Hy, g.Wy, rows_h, rows_w, cm, nay, nax, 1, 1, py, px, w, taps, cm * taps, -(int64_t)g.sh * g.kw, -(int64_t)g.sw,
+                     (int64_t)(ky0 + g.sh * (nay - 1)) * g.kw + kx0 + g.sw * (nax - 1), bias, out, g.Hx, g.Wx, g.sh, g.sw, ry, rx};
+      st = pixel_product(ctx, q, ws.as<float>());
+    }
+  return st;
 }

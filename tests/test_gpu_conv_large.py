@@ -1,0 +1,44 @@
+"""Convolutions of the TMA-fed tensor-core kernel against float64: extents that its pixel boxes and 32-channel blocks do not divide,
+strides, output phases, one and several column tiles."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import ref_f64
+
+pytestmark = pytest.mark.gpu
+
+i64 = C.c_int64
+CASES = [(64, 33, 30, 30, 70, 3, 1, 1), (90, 48, 29, 37, 96, 5, 2, 2), (24, 16, 41, 33, 16, 3, 1, 0), (40, 130, 23, 31, 130, 1, 1, 0),
+         (48, 20, 50, 46, 65, 4, 2, 1), (16, 17, 64, 67, 24, 3, 3, 1)]
+
+
+@pytest.fixture(scope="module")
+def api():
+    from rusttensor_b200 import CApi
+
+    a = CApi()
+    yield a
+    a.close()
+
+
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("n,cin,h,w,cout,k,s,p", CASES)
+def test_convolution(api, n, cin, h, w, cout, k, s, p, transposed):
+    r = np.random.default_rng(n + cin + h)
+    x = r.standard_normal((n, cin, h, w)).astype(np.float32)
+    wt = r.standard_normal((cin, cout, k, k) if transposed else (cout, cin, k, k)).astype(np.float32)
+    b = r.standard_normal(cout).astype(np.float32)
+    some = [0, n // 2, n - 1]  # images that are checked (the reference takes its time)
+    name, fwd, bwd = (("conv2d_transpose", ref_f64.conv2d_transpose, ref_f64.conv2d_transpose_backward) if transposed
+                      else ("conv2d", ref_f64.conv2d, ref_f64.conv2d_backward))
+    ref = fwd(x[some], wt, b, (s, s), (p, p))
+    y, dx = api.empty((n,) + ref.shape[1:]), api.empty(x.shape)
+    g = r.standard_normal(y.shape).astype(np.float32)
+    dev = [api.to_device(v) for v in (x, wt, b, g)]
+    dims = (i64(n), i64(cin), i64(h), i64(w), i64(cout), k, k, s, s, p, p)
+    api.call(name, dev[0].ptr, dev[1].ptr, dev[2].ptr, *dims, y.ptr)
+    api.call(name + "_backward", dev[0].ptr, dev[1].ptr, dev[3].ptr, *dims, dx.ptr, None, None)
+    for got, want in ((y.numpy()[some], ref), (dx.numpy()[some], bwd(x[some], wt, g[some], (s, s), (p, p))[0])):
+        assert np.all(np.abs(got - want) <= 4e-6 * np.abs(want).max() + 1e-6 * np.abs(want))
