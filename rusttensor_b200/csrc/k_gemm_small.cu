@@ -3,12 +3,15 @@
 // What bounds them: with a few dozen output tiles a product of this size occupies a fraction of the chip for as long as one tile
 // walks its reduction, and a second launch that adds split-K partial sums costs as much as the product.  So
 //  * 32 x 64 tiles, and the reduction of a tile is split over the CTAs of a cluster (1, 2, 4 or 8), so that about one to two
-//    CTAs land on every SM; their partial tiles meet in distributed shared memory and each CTA finishes a slice of the rows:
+//    CTAs land on every SM; their partial tiles meet in distributed shared memory and each CTA finishes a share of them:
 //    bias, activation and accumulation included, one launch in all, sums in a fixed order;
-//  * inside a CTA two groups of four warps take alternate halves of every 64-deep K-block (4 x 4 outputs a thread);
+//  * inside a CTA four groups of four warps take a quarter of every 64-deep K-block each (4 x 4 outputs a thread);
 //  * operands arrive by cp.async, three K-blocks in flight, 16 bytes at a time where the rows allow it, else 4.
 // fp32 FMAs rather than tensor cores: below a few hundred MFLOP the splitting of operands into TF32 parts and the tensor-memory
 // set-up cost more than the arithmetic.
+// The partial sums leave a thread as 128-bit slots, so that a slot, and not an element, is what a thread adds up and writes.
+// Measured in a graph (M x K x N; with one group of threads and element-wise sums before): 64 x 64 x 64 3.5 us (4.5), of which the launch is
+// 0.65 and the first operands 1.15; 512 x 64 x 65 4.4 (5.1); 30 x 250 x 800 5.1 (5.2); 64 x 784 x 128 6.2 (6.5); 90 x 1000 x 100 6.3 (6.6).
 #include <cooperative_groups.h>
 
 #include "rt_internal.cuh"
@@ -17,7 +20,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int kBM = 32, kBN = 64, kBK = 64, kStages = 3, kThreads = 256;
+constexpr int kBM = 32, kBN = 64, kBK = 64, kStages = 3, kGroups = 4, kThreads = kGroups * 128;
 constexpr int kPad = 4;
 
 struct SmallGemm {
@@ -71,7 +74,7 @@ struct Shape {
   static constexpr int a_floats = TA ? kBK * (kBM + kPad) : kBM * (kBK + kPad);
   static constexpr int b_floats = TB ? kBN * (kBK + kPad) : kBK * (kBN + kPad);
   static constexpr size_t bytes = sizeof(float) * kStages * (a_floats + b_floats);
-  static_assert(kBM * (kBN + kPad) <= kStages * (a_floats + b_floats), "the partial tile reuses the stages");
+  static_assert(kGroups * kBM * kBN <= kStages * (a_floats + b_floats), "the partial tiles reuse the stages");
 };
 
 // Several left operands and results for one right operand: the row tiles of item i follow those of item i - 1.
@@ -84,7 +87,7 @@ struct SmallList {
 struct NoList {};
 
 template <bool TA, bool TB, class List>
-__global__ void __launch_bounds__(kThreads, 3) small_gemm_kernel(const SmallGemm args, const List list) {
+__global__ void __launch_bounds__(kThreads, 2) small_gemm_kernel(const SmallGemm args, const List list) {
   extern __shared__ __align__(16) float smem[];
   using S = Shape<TA, TB>;
   cg::cluster_group cluster = cg::this_cluster();
@@ -130,8 +133,8 @@ __global__ void __launch_bounds__(kThreads, 3) small_gemm_kernel(const SmallGemm
     const float* sa = smem + (it % kStages) * (S::a_floats + S::b_floats);
     const float* sb = sa + S::a_floats;
 #pragma unroll
-    for (int q = 0; q < kBK / 2; q += 4) {
-      const int k = group * (kBK / 2) + q;
+    for (int q = 0; q < kBK / kGroups; q += 4) {
+      const int k = group * (kBK / kGroups) + q;
       float av[4][4], bv[4][4];  // [row or column][k]
       if (TA) {
 #pragma unroll
@@ -169,58 +172,74 @@ __global__ void __launch_bounds__(kThreads, 3) small_gemm_kernel(const SmallGemm
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  // the two groups' sums, then the cluster's
-  float* part = smem;  // [kBM][kBN + kPad]
-  auto row_of = [&](int i) { return TA ? 4 * tm + i : tm + 8 * i; };
-  auto col_of = [&](int j) { return TB ? tn + 16 * j : 4 * tn + j; };
-  if (group == 1) {
+  // Every thread leaves its sums as four 128-bit slots; a slot is then added over the groups and the CTAs of the cluster by one thread
+  // of one of them and written out.  Slot i * 128 + t belongs to thread t of a group: row i of its block (column i when B is stored
+  // transposed, whose columns are 16 apart).
+  float4* part = reinterpret_cast<float4*>(smem);
+  constexpr int kSlots = 4 * 128;
+  const int t128 = threadIdx.x & 127;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) part[row_of(i) * (kBN + kPad) + col_of(j)] = acc[i][j];
-  }
+  for (int i = 0; i < 4; ++i) part[group * kSlots + i * 128 + t128] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
   __syncthreads();
-  if (group == 0) {
+  static_assert(kSlots == kThreads, "a slot a thread");
+  auto over_groups = [&](int slot) {
+    float4 v = part[slot];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) part[row_of(i) * (kBN + kPad) + col_of(j)] += acc[i][j];
-  }
-  if (splits > 1) cluster.sync();
-  else __syncthreads();
-  const int rows = kBM / splits;
-  for (int idx = threadIdx.x; idx < rows * (kBN / 4); idx += kThreads) {
-    const int r = rank * rows + idx / (kBN / 4), c = idx % (kBN / 4) * 4;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < splits; ++s) {
-      const float* q = splits > 1 ? cluster.map_shared_rank(part, s) : part;
-      const float4 t = *reinterpret_cast<const float4*>(q + r * (kBN + kPad) + c);
-      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+    for (int g = 1; g < kGroups; ++g) {
+      const float4 u = part[g * kSlots + slot];
+      v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
     }
-    const int m = m0 + r, n = n0 + c;
+    return v;
+  };
+  if (splits > 1) {
+    part[threadIdx.x] = over_groups(threadIdx.x);
+    cluster.sync();
+  }
+  const int share = kSlots / splits, slot = rank * share + threadIdx.x, i = slot >> 7, l = slot & 31, w = (slot >> 5) & 3;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if ((int)threadIdx.x < share) {
+    if (splits == 1) {
+      v = over_groups(slot);
+    } else {
+      float4 u[8];  // all remote reads are in flight before the first is added
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s < splits) u[s] = cluster.map_shared_rank(part, s)[slot];
+      v = u[0];
+#pragma unroll
+      for (int s = 1; s < 8; ++s)
+        if (s < splits) {
+          v.x += u[s].x; v.y += u[s].y; v.z += u[s].z; v.w += u[s].w;
+        }
+    }
+  }
+  // nobody leaves while its partial tile may still be read: the wait comes after the result is written
+  if (splits > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  if ((int)threadIdx.x < share) {
+    const int sm = (l >> 3) + 4 * (w & 1), sn = (l & 7) + 8 * (w >> 1);
+    const int m = m0 + (TA ? 4 * sm + i : sm + 8 * i), n = n0 + (TB ? sn : 4 * sn);
     if (m < p.m) {
       float* out = p.c + (int64_t)m * p.ldc + n;
-      const float e[4] = {v.x, v.y, v.z, v.w};
-      float o[4];
+      float o[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        o[j] = e[j];
-        if (n + j < p.n) {
-          if (p.bias) o[j] += __ldg(p.bias + n + j);
-          o[j] = activate(o[j], p.act);
-          if (p.accumulate) o[j] += out[j];
+        const int nj = TB ? 16 * j : j;
+        if (n + nj < p.n) {
+          if (p.bias) o[j] += __ldg(p.bias + n + nj);
+          if (p.act != RT_ACT_NONE) o[j] = activate(o[j], p.act);
+          if (p.accumulate) o[j] += out[nj];
         }
       }
-      if (n + 3 < p.n && rt_aligned16(out)) {
+      if (!TB && n + 3 < p.n && rt_aligned16(out)) {
         *reinterpret_cast<float4*>(out) = make_float4(o[0], o[1], o[2], o[3]);
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (n + j < p.n) out[j] = o[j];
+          if (n + (TB ? 16 * j : j) < p.n) out[TB ? 16 * j : j] = o[j];
       }
     }
   }
-  if (splits > 1) cluster.sync();  // nobody leaves while its partial tile may still be read
+  if (splits > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
 template <bool TA, bool TB, class List = NoList>
@@ -245,15 +264,21 @@ rt_status launch_small(rt_ctx* ctx, const SmallGemm& p, int splits, const List& 
   return RT_OK;
 }
 
+// As many splits as put a CTA on every SM, at least one K-block each.  (Two K-blocks in one CTA were slower than one in each of two,
+// 64 x 65 x 512: 5.5 and 5.1 us.)
+int choose_splits(rt_ctx* ctx, int64_t tiles, int64_t k) {
+  int splits = 1;
+  while (splits < 8 && tiles * splits <= (int64_t)ctx->sm_count && k > (int64_t)kBK * splits) splits *= 2;
+  return splits;
+}
+
 }  // namespace
 
 rt_status rt_gemm_small_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
                                  const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   const int64_t tiles = ((m + kBM - 1) / kBM) * ((n + kBN - 1) / kBN);
   if (m >= (1 << 20) || n >= (1 << 20) || k >= (1 << 28) || (m + kBM - 1) / kBM > 65535) return RT_ERR_UNIMPLEMENTED;
-  // as many splits as put a CTA and a half on every SM, at least one K-block each
-  int splits = 1;
-  while (splits < 8 && tiles * splits * 2 <= (int64_t)ctx->sm_count * 2 && k > (int64_t)kBK * splits) splits *= 2;
+  const int splits = choose_splits(ctx, tiles, k);
   int64_t per = (k + splits - 1) / splits;
   per = (per + kBK - 1) / kBK * kBK;
   SmallGemm p{a, b, bias, c, lda, ldb, ldc, (int)m, (int)n, (int)k, (int)per, act, rt_aligned16(a) && lda % 4 == 0, rt_aligned16(b) && ldb % 4 == 0,
@@ -268,8 +293,7 @@ rt_status rt_gemm_small_list_internal(rt_ctx* ctx, int count, const float* const
                                       const float* b, const float* bias, int act) {
   const int64_t row_tiles = (m + kBM - 1) / kBM, tiles = row_tiles * ((n + kBN - 1) / kBN) * (count < kListTerms ? count : kListTerms);
   if (m >= (1 << 20) || n >= (1 << 20) || k >= (1 << 28) || row_tiles * kListTerms > 65535) return RT_ERR_UNIMPLEMENTED;
-  int splits = 1;
-  while (splits < 8 && tiles * splits * 2 <= (int64_t)ctx->sm_count * 2 && k > (int64_t)kBK * splits) splits *= 2;
+  const int splits = choose_splits(ctx, tiles, k);
   int64_t per = (k + splits - 1) / splits;
   per = (per + kBK - 1) / kBK * kBK;
   for (int q = 0; q < count; q += kListTerms) {
