@@ -11,16 +11,19 @@
 //
 // This file is the exact-FP32 path.  Large, tile-aligned shapes are routed to the
 // tcgen05 3xTF32 kernels in k_gemm_tc.cu by the dispatchers at the bottom.
+#include "finish.cuh"
 #include "rt_internal.cuh"
 #include "conv_geom.cuh"
 
 rt_status rt_sum_axis_internal(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, int64_t inner, float* out,
                                float scale);
-rt_status rt_gemm_tc_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a,
-                              int64_t lda, const float* b, int64_t ldb, float* c, int64_t ldc, int accumulate);
+rt_status rt_gemm_tc_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
+                              int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
 
 rt_status rt_gemm_small_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
                                  const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
+float rt_gemm_small_estimate(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, bool wide);
+float rt_gemm_ts_estimate(rt_ctx* ctx, int64_t m, int64_t n, int64_t k);
 rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
                                int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
 rt_status rt_conv_forward_tma_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y);
@@ -366,7 +369,7 @@ constexpr int kSkinnyN = 16, kSkinnyRows = 32, kSkinnyKC = 128, kSkinnySlices = 
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(kSkinnyRows * kSkinnySlices)
 gemm_skinny_n_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ b, int64_t ldb, float* __restrict__ c,
-                     int64_t ldc, int M, int N, int K, int accumulate) {
+                     int64_t ldc, int M, int N, int K, const float* __restrict__ bias, int act, int accumulate) {
   constexpr int T = kSkinnyRows * kSkinnySlices;
   __shared__ float As[kSkinnyRows][kSkinnyKC + 1];
   __shared__ __align__(16) float Bs[kSkinnyKC][kSkinnyN];
@@ -434,6 +437,7 @@ gemm_skinny_n_kernel(const float* __restrict__ a, int64_t lda, const float* __re
 #pragma unroll
     for (int s2 = 0; s2 < kSkinnySlices; ++s2) v += red[s2][mm][j];
     float* dst = c + (int64_t)(m0 + mm) * ldc + j;
+    if (bias || act != RT_ACT_NONE) v = rt_finish4(make_float4(v, 0.f, 0.f, 0.f), bias ? bias + j : nullptr, act, nullptr, 1).x;
     *dst = accumulate ? *dst + v : v;
   }
 }
@@ -462,14 +466,14 @@ __global__ void __launch_bounds__(256) gemm_small_k_kernel(const float* __restri
 
 template <bool TA, bool TB>
 rt_status gemm_narrow_launch(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
-                             int64_t ldb, float* c, int64_t ldc, int accumulate) {
+                             int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   if (k <= 16) {
     gemm_small_k_kernel<TA, TB><<<rt_grid_for(ctx, m * n, 256), 256, 0, ctx->stream>>>(a, lda, b, ldb, c, ldc, m * n, (int)n,
                                                                                       (int)k, accumulate);
   } else {
     const int grid = (int)((m + kSkinnyRows - 1) / kSkinnyRows);
     gemm_skinny_n_kernel<TA, TB><<<grid, kSkinnyRows * kSkinnySlices, 0, ctx->stream>>>(a, lda, b, ldb, c, ldc, (int)m, (int)n,
-                                                                                        (int)k, accumulate);
+                                                                                        (int)k, bias, act, accumulate);
   }
   RT_LAUNCHED(ctx);
   return RT_OK;
@@ -477,15 +481,20 @@ rt_status gemm_narrow_launch(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const
 
 // Narrow products (K <= 16, or N <= 16 with a K one block can walk); RT_ERR_UNIMPLEMENTED for everything else.
 rt_status gemm_narrow(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
-                      const float* b, int64_t ldb, float* c, int64_t ldc, int accumulate) {
+                      const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   if (k < 1 || m >= (1ll << 31) || n >= (1ll << 31) || m * n >= (1ll << 40)) return RT_ERR_UNIMPLEMENTED;
-  const bool small_k = k <= 16;
-  const bool skinny_n = n <= kSkinnyN && (k <= 4096 || m >= 4096) && k < (1ll << 30) && m < (1ll << 30);
+  // A thread reads k values of both operands by itself: with a reduction that is contiguous in B, or rows that are in A, these reads
+  // do not coalesce, which shows from some millions of multiply-adds on (768 x 16 x 1196: B plain 10 us, B transposed 30, A transposed 16).
+  const bool small_k = k <= 16 && !((trans_a || trans_b) && m * n * k > (5ll << 19)) && !bias && act == RT_ACT_NONE;
+  // One block walks the whole reduction of its 32 rows: 1.8 us and 1.2 more per 100 of it, against 5 us and more in the small tiles
+  // (351 x 173 x 7: 4.5 us here; 173 x 351 x 7: 5.8 here, 5.2 there; 88 x 1288 x 16: 17 and 7).  Many rows fill the chip all the same.
+  const bool skinny_n = n <= kSkinnyN && k > 16 && k < (1ll << 30) && m < (1ll << 30) &&
+                        (m >= 4096 || 1.8f + 0.012f * (float)k <= rt_gemm_small_estimate(ctx, m, n, k, false));
   if (!small_k && !skinny_n) return RT_ERR_UNIMPLEMENTED;
-  if (!trans_a && !trans_b) return gemm_narrow_launch<false, false>(ctx, m, n, k, a, lda, b, ldb, c, ldc, accumulate);
-  if (!trans_a && trans_b) return gemm_narrow_launch<false, true>(ctx, m, n, k, a, lda, b, ldb, c, ldc, accumulate);
-  if (trans_a && !trans_b) return gemm_narrow_launch<true, false>(ctx, m, n, k, a, lda, b, ldb, c, ldc, accumulate);
-  return gemm_narrow_launch<true, true>(ctx, m, n, k, a, lda, b, ldb, c, ldc, accumulate);
+  if (!trans_a && !trans_b) return gemm_narrow_launch<false, false>(ctx, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
+  if (!trans_a && trans_b) return gemm_narrow_launch<false, true>(ctx, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
+  if (trans_a && !trans_b) return gemm_narrow_launch<true, false>(ctx, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
+  return gemm_narrow_launch<true, true>(ctx, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
 }
 
 rt_status check_conv_args(rt_ctx* ctx, int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int kh, int kw, int sh,
@@ -631,17 +640,44 @@ __global__ void __launch_bounds__(1024) col_sum_list_kernel(const RowList l, int
 
 extern "C" {
 
-// Products for the one-launch fp32 kernel (k_gemm_small.cu).  Above 32 M multiply-adds the tensor cores win (64 x 577 x 2048: 9.5 against
-// 11.8 us; 90 x 1000 x 100: 6.5 against 9.4), and a reduction of more than 8 x 256 leaves each CTA of the cluster a serial walk that the
-// tensor-core kernel splits over the whole chip.
+// Which kernel takes a product.
+//  * Small: the one-launch fp32 kernel (k_gemm_small.cu), exact and with the least to set up;
+//  * Tensor: tcgen05 with operands split by the producing warps (k_gemm_tc.cu); in its form for one wave of 128 x 64 tiles the
+//    reduction is split over clusters;
+//  * Tma: tcgen05 with operands fetched by TMA (k_gemm_tma.cu), no split, operands not in its form packed first;
+//  * Plain: fp32 tiles for what is left, and for everything that is too large for Small when tensor cores are off.
+// Where the 128 x 64 tiles fit one wave the estimates of the first two decide.  (Against Small alone: 512 x 133 x 405 11.4 and 8.6 us; against
+// Tensor alone: 514 x 247 x 92 8.2 and 6.6 us.)  Beyond one wave Tma is ahead (708 x 679 x 2336: 30 us, the 128 x 128 tiles of Tensor
+// 45; 948 x 920 x 3948: 54 and 84), but for short reductions (1129 x 66 x 1116: 13 and 9 us), longer ones too if it would have
+// to transpose the right operand first (1120 x 144 x 1748: 13.4 and 11.5 us).  Reductions below 32 fill no K-block: fp32, in small tiles while these come to one wave
+// (2023 x 20 x 814: 15 us in small tiles, 9 in large ones).
+enum class Route { Small, Tensor, Tma, Plain };
+static Route choose_route(rt_ctx* ctx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb) {
+  const int64_t work = m * n * k;
+  const bool wide = rt_aligned16(a) && rt_aligned16(b) && lda % 4 == 0 && ldb % 4 == 0;
+  if (!ctx->use_tensor_cores) return k > 0 && k <= 2048 && work <= (32ll << 20) ? Route::Small : Route::Plain;
+  if (k < 32 || work < (1ll << 18)) {
+    const int64_t tiles = ((m + 31) / 32) * ((n + 63) / 64);
+    return k > 0 && (tiles <= 2 * (int64_t)ctx->sm_count || work < (1ll << 22)) ? Route::Small : Route::Plain;
+  }
+  const float ts = rt_gemm_ts_estimate(ctx, m, n, k);
+  if (ts >= 0.f) return rt_gemm_small_estimate(ctx, m, n, k, wide) <= ts ? Route::Small : Route::Tensor;
+  if (k < 128 || n < 48 || (k < 256 && wide && !(!ta && tb))) return Route::Tensor;
+  return Route::Tma;
+}
+// Products that several left operands share a right one with (rt_gemm_bias_act_list) in the one-launch kernel.
 static bool small_product(int64_t m, int64_t n, int64_t k) {
   return k > 0 && k <= 2048 && m * n * k <= (32ll << 20);
 }
-// Products for the TMA-fed tensor-core kernel (k_gemm_tma.cu), which has no split of the reduction: from about 48 tiles of 128 x 128 on
-// it is ahead of the kernels with one (1024 x 256 x 1024, 64 tiles: 15 against 20 us; 700 x 1500 x 900, 48 tiles: 42 against 43 - 58 us;
-// 512^3, 16 tiles: 19 against 10 us).
-static bool large_product(rt_ctx* ctx, int64_t m, int64_t n, int64_t k) {
-  return ctx->use_tensor_cores && k >= 64 && n >= 48 && ((m + 127) / 128) * ((n + 127) / 128) >= 48;
+static rt_status routed(rt_ctx* ctx, Route route, int ta, int tb, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
+                        int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
+  if (route == Route::Small) return rt_gemm_small_internal(ctx, ta, tb, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
+  if (route == Route::Tma) {
+    rt_status st = rt_gemm_tma_internal(ctx, ta, tb, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
+  if (route == Route::Plain) return RT_ERR_UNIMPLEMENTED;
+  return rt_gemm_tc_internal(ctx, ta, tb, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
 }
 rt_status rt_gemm_bias_act(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb,
                            const float* bias, int act, float* c, int64_t ldc) {
@@ -651,14 +687,12 @@ rt_status rt_gemm_bias_act(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const f
   RT_CHECK_PTR(ctx, a);
   RT_CHECK_PTR(ctx, b);
   RT_CHECK_PTR(ctx, c);
-  if (small_product(m, n, k)) {
-    rt_status st = rt_gemm_small_internal(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, bias, act, 0);
+  if (ctx->use_tensor_cores) {
+    rt_status st = gemm_narrow(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, bias, act, 0);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
-  if (large_product(ctx, m, n, k)) {
-    rt_status st = rt_gemm_tma_internal(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, bias, act, 0);
-    if (st != RT_ERR_UNIMPLEMENTED) return st;
-  }
+  rt_status done = routed(ctx, choose_route(ctx, false, false, m, n, k, a, lda, b, ldb), 0, 0, m, n, k, a, lda, b, ldb, c, ldc, bias, act, 0);
+  if (done != RT_ERR_UNIMPLEMENTED) return done;
   rt_status st = rt_gemm(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, 0);
   if (st != RT_OK || (!bias && act == RT_ACT_NONE)) return st;
   bias_act_kernel<<<rt_grid_for(ctx, m * n, 256), 256, 0, ctx->stream>>>(c, bias, m, (int)n, ldc, act);
@@ -745,19 +779,12 @@ rt_status rt_gemm(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, i
     RT_FAIL(ctx, RT_ERR_SHAPE_MISMATCH, "rt_gemm: leading dimension smaller than the row length");
   bool acc = accumulate != 0;
   if (ctx->use_tensor_cores) {  // narrow products: dedicated FP32 kernels
-    rt_status st = gemm_narrow(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, accumulate);
+    rt_status st = gemm_narrow(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, nullptr, RT_ACT_NONE, accumulate);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
-  if (small_product(m, n, k)) {
-    rt_status st = rt_gemm_small_internal(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, nullptr, RT_ACT_NONE, accumulate);
-    if (st != RT_ERR_UNIMPLEMENTED) return st;
-  }
-  if (large_product(ctx, m, n, k)) {
-    rt_status st = rt_gemm_tma_internal(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, nullptr, RT_ACT_NONE, accumulate);
-    if (st != RT_ERR_UNIMPLEMENTED) return st;
-  }
-  if (ctx->use_tensor_cores && k >= 32 && m >= 32 && n >= 16 && m * n * k >= (1ll << 20)) {
-    rt_status st = rt_gemm_tc_internal(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, accumulate);
+  if (k > 0) {
+    rt_status st = routed(ctx, choose_route(ctx, trans_a, trans_b, m, n, k, a, lda, b, ldb), trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc,
+                          nullptr, RT_ACT_NONE, accumulate);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   if (!trans_a && !trans_b) return gemm_plain(ctx, MatA<false>{a, lda}, MatB<false>{b, ldb}, c, ldc, m, n, k, acc, true);

@@ -14,6 +14,7 @@
 // 0.65 and the first operands 1.15; 512 x 64 x 65 4.4 (5.1); 30 x 250 x 800 5.1 (5.2); 64 x 784 x 128 6.2 (6.5); 90 x 1000 x 100 6.3 (6.6).
 #include <cooperative_groups.h>
 
+#include "finish.cuh"
 #include "rt_internal.cuh"
 
 namespace cg = cooperative_groups;
@@ -57,15 +58,6 @@ __device__ __forceinline__ void load_piece(float* s, const float* g, int64_t ld,
       const bool in = row0 + r < row_end && col0 + c < col_end;
       async_copy(s + r * (COLS + kPad) + c, in ? g + (int64_t)(row0 + r) * ld + col0 + c : g, in ? 4 : 0, false);
     }
-  }
-}
-
-__device__ __forceinline__ float activate(float v, int act) {
-  switch (act) {
-    case RT_ACT_RELU: return fmaxf(v, 0.f);
-    case RT_ACT_TANH: return tanhf(v);
-    case RT_ACT_SIGMOID: return 1.f / (1.f + expf(-v));
-    default: return v;
   }
 }
 
@@ -215,27 +207,34 @@ __global__ void __launch_bounds__(kThreads, 2) small_gemm_kernel(const SmallGemm
   }
   // nobody leaves while its partial tile may still be read: the wait comes after the result is written
   if (splits > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  const bool plain = !p.bias && p.act == RT_ACT_NONE && !p.accumulate;
   if ((int)threadIdx.x < share) {
     const int sm = (l >> 3) + 4 * (w & 1), sn = (l & 7) + 8 * (w >> 1);
     const int m = m0 + (TA ? 4 * sm + i : sm + 8 * i), n = n0 + (TB ? sn : 4 * sn);
     if (m < p.m) {
       float* out = p.c + (int64_t)m * p.ldc + n;
-      float o[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int nj = TB ? 16 * j : j;
-        if (n + nj < p.n) {
-          if (p.bias) o[j] += __ldg(p.bias + n + nj);
-          if (p.act != RT_ACT_NONE) o[j] = activate(o[j], p.act);
-          if (p.accumulate) o[j] += out[nj];
+      if (!TB) {
+        const int left = p.n - n;
+        if (left > 0) {
+          if (!plain) v = rt_finish4(v, p.bias ? p.bias + n : nullptr, p.act, p.accumulate ? out : nullptr, left);
+          if (left >= 4 && rt_aligned16(out)) {
+            *reinterpret_cast<float4*>(out) = v;
+          } else {
+            out[0] = v.x;
+            if (left > 1) out[1] = v.y;
+            if (left > 2) out[2] = v.z;
+            if (left > 3) out[3] = v.w;
+          }
         }
-      }
-      if (!TB && n + 3 < p.n && rt_aligned16(out)) {
-        *reinterpret_cast<float4*>(out) = make_float4(o[0], o[1], o[2], o[3]);
       } else {
+        const float o[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (n + (TB ? 16 * j : j) < p.n) out[TB ? 16 * j : j] = o[j];
+          if (n + 16 * j < p.n) {
+            float r = o[j];
+            if (!plain) r = rt_finish4(make_float4(r, 0.f, 0.f, 0.f), p.bias ? p.bias + n + 16 * j : nullptr, p.act, p.accumulate ? out + 16 * j : nullptr, 1).x;
+            out[16 * j] = r;
+          }
       }
     }
   }
@@ -273,6 +272,16 @@ int choose_splits(rt_ctx* ctx, int64_t tiles, int64_t k) {
 }
 
 }  // namespace
+
+// Microseconds that a product takes here, fitted like rt_gemm_ts_estimate: a K-block costs 1.3 us where about one CTA comes to an SM and
+// 2.8 where two do, a third more where its copies are of 4 bytes.
+float rt_gemm_small_estimate(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, bool wide) {
+  const int64_t tiles = ((m + kBM - 1) / kBM) * ((n + kBN - 1) / kBN), blocks = (k + kBK - 1) / kBK;
+  const int splits = choose_splits(ctx, tiles, k);
+  const int64_t ctas = tiles * splits, waves = (ctas + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count);
+  const float block = ctas * 4 > (int64_t)ctx->sm_count * 3 ? 2.8f : 1.3f;
+  return (splits > 1 ? 3.7f : 2.7f) + block * (wide || k <= kBK ? 1.f : 1.3f) * (float)(waves * ((blocks + splits - 1) / splits));
+}
 
 rt_status rt_gemm_small_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda,
                                  const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {

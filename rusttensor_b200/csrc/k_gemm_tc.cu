@@ -17,10 +17,15 @@
 // Stages are handed over with mbarriers.  Every wait is bounded: on expiry the kernel
 // records an error code in the context's status word, skips the rest of its work, still
 // frees its TMEM columns and returns.
+#include <cooperative_groups.h>
+
 #include "rt_internal.cuh"
 #include "conv_geom.cuh"
+#include "finish.cuh"
 #include "tc_common.cuh"
 #include <type_traits>
+
+namespace cg = cooperative_groups;
 
 rt_status rt_sum_axis_internal(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, int64_t inner, float* out,
                                float scale);
@@ -796,28 +801,39 @@ tc_gemm_kernel(const LA la, const LB lb, const EPI epi, int K, int k_per_split, 
 }
 
 // ---- plain products with the A operand in tensor memory (TS form) -----------------------------------------------------
-// tc_gemm_kernel stages the hi / lo images of BOTH operands in shared memory and is bound by its bandwidth: per K-block of 32 the
-// producers write 64 KB and the twelve MMAs read 96 KB through a 128 B/cycle path (1 250 cycles against 780 cycles of tensor
-// work; measured 2 350 cycles per K-block).  Here the A tile never touches shared memory: every producer thread owns one row of
-// the tile (= one lane of tensor memory), loads 16 of its 32 k-values, splits them and writes hi and lo straight into tensor
-// memory with tcgen05.st; the MMAs read A from there (an MMA with A in tensor memory costs N/2 cycles for every N) and only
-// the 64-column B tile crosses shared memory (16 KB written, 24 KB read per K-block).  Used for products whose grid is small
-// enough to be latency-bound (the fully connected and recurrent layers); large products keep the 128 x 128 tile, whose wider B
-// tile halves the traffic from L2.
-struct PlainA {  // element(row, k) = trans ? p[k * ld + row] : p[row * ld + k]
+// For products whose grid of 128 x 64 tiles is small enough to be bound by latency (fully connected and recurrent layers); large
+// ones go to the TMA-fed kernel.
+//  * A never has its hi / lo images in shared memory: a producer thread owns a row of the tile (= one lane of tensor memory),
+//    splits it and writes hi and lo with tcgen05.st; only the 64-column B tile is staged as hi / lo for the MMAs.
+//  * Two groups of four producer warps take K-blocks in turn: a block is a chain of waits (copies, tensor-memory stores, fences), of
+//    which two run at a time.
+//  * What a warp converts it has also copied, by cp.async, up to kTsRaw K-blocks ahead, so that the copies need no barrier but
+//    __syncwarp.  (With the loads kept in registers the hardware waited for all of them at the first use: 0.85 us a K-block of 32,
+//    whatever the depth.)  Copies run along the contiguous direction, 16 bytes a lane where alignment allows, else 4.
+//  * The reduction of a tile is split over the CTAs of a cluster (up to 16).  Their partial tiles meet in distributed shared
+//    memory, each CTA adds up, finishes and writes a share of the rows, in a fixed order; a second launch that adds partial sums from
+//    a workspace cost 2.6 us and one for bias and activation 2.8.
+struct PlainMat {  // element(row, k) = trans ? p[k * ld + row] : p[row * ld + k]; wide: base and ld allow 16-byte copies
   const float* p;
   int64_t ld;
   int rows;
-  bool trans, vec;
+  bool wide;
 };
-constexpr int kTsBN = 64, kTsStages = 3, kTsAccs = 4;
+constexpr int kTsBN = 64, kTsStages = 3, kTsAccs = 4, kTsRaw = 4, kTsMaxSplits = 16;
 constexpr uint32_t kTsAccCols = kTsAccs * kTsBN;        // 256 accumulator columns
 constexpr uint32_t kTsAStageCols = 2 * BK;              // hi k 0..31, lo k 0..31
+constexpr int kTsTileLd = kTsBN + 4;                    // row stride of the partial tile in shared memory: 128-bit rows free of conflicts
 struct TsSmem {
   static constexpr uint32_t b_bytes = tile_bytes(kTsBN);
   static constexpr uint32_t stage_bytes = 2 * b_bytes;  // B hi, B lo
-  static constexpr uint32_t bar_offset = kTsStages * stage_bytes;
+  // raw copies of one warp: A 32 rows x 32 k or 32 k x 32 rows (stride 36); B 16 rows x 32 k (stride 36) or 8 k x 64 rows (stride 68)
+  static constexpr int a_raw = 32 * 36, b_raw = 16 * 36;
+  static constexpr uint32_t raw_offset = kTsStages * stage_bytes, raw_stage = kProducerWarps / 2 * (a_raw + b_raw) * 4;
+  static_assert(kTsRaw % 2 == 0, "each group has its own raw slots");
+  static constexpr uint32_t bar_offset = raw_offset + kTsRaw * raw_stage;
   static constexpr uint32_t total = bar_offset + (2 * kTsStages + 1) * 8 + 16;
+  static_assert(BM * kTsTileLd * 4 <= bar_offset, "the partial tile reuses the stages");
+  static_assert(total <= 232448, "shared memory");
 };
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
@@ -846,25 +862,92 @@ __device__ __forceinline__ void umma_tf32_step_ts_elect(uint32_t d_cross, uint32
       "r"(b_hi_lo32), "r"(b_lo_lo32), "r"(b_hi32), "r"(idesc), "r"(acc_cross), "r"(acc_main)
       : "memory");
 }
+// `left` floats (none if negative) of up to 4 (wide) or 1 to shared memory, zeros behind them
+__device__ __forceinline__ void copy_async(float* dst, const float* src, const float* valid, int left, bool wide) {
+  const uint32_t d = smem_u32(dst);
+  if (wide) {
+    const int n = left <= 0 ? 0 : (left >= 4 ? 16 : left * 4);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(n ? src : valid), "r"(n) : "memory");
+  } else {
+    const int n = left > 0 ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(n ? src : valid), "r"(n) : "memory");
+  }
+}
+// A warp's LINES lines of WIDTH floats (stride LD in shared memory); line and position bounded by n_lines and n_width.
+template <int LINES, int WIDTH, int LD>
+__device__ __forceinline__ void copy_lines(float* dst, const PlainMat& m, int line0, int n_lines, int pos0, int n_pos, int lane) {
+  if (m.wide) {
+    constexpr int kPer = 32 / (WIDTH / 4);
+    const int l = lane / (WIDTH / 4), c = lane % (WIDTH / 4) * 4;
+#pragma unroll
+    for (int i = 0; i < LINES / kPer; ++i) {
+      const int line = line0 + l + i * kPer;
+      copy_async(dst + (l + i * kPer) * LD + c, m.p + (int64_t)line * m.ld + pos0 + c, m.p, line < n_lines ? n_pos - (pos0 + c) : 0, true);
+    }
+  } else {
+    constexpr int kPer = WIDTH < 32 ? 32 / WIDTH : 1, kSteps = WIDTH < 32 ? 1 : WIDTH / 32;
+    const int l = WIDTH < 32 ? lane / WIDTH : 0, c = lane % WIDTH;
+#pragma unroll
+    for (int i = 0; i < LINES / kPer; ++i) {
+      const int line = line0 + l + i * kPer;
+#pragma unroll
+      for (int q = 0; q < kSteps; ++q)
+        copy_async(dst + (l + i * kPer) * LD + c + 32 * q, m.p + (int64_t)line * m.ld + pos0 + c + 32 * q, m.p,
+                   line < n_lines ? n_pos - (pos0 + c + 32 * q) : 0, false);
+    }
+  }
+}
 
-template <class LB, class EPI>
+// Where the result goes: c[m, n] = act(sum + bias[n]) (+ c[m, n]); with a workspace, partial sum z at c + z * split_stride.
+struct TsOut {
+  float* c;
+  int64_t ld, split_stride;
+  int M, N;
+  const float* bias;
+  int act;
+  bool accumulate;
+};
+
+template <bool TA, bool TB>
 __global__ void __launch_bounds__(kThreads, 1)
-tc_gemm_ts_kernel(const PlainA la, const LB lb, const EPI epi, int K, int k_per_split, int* status) {
+tc_gemm_ts_kernel(const PlainMat la, const PlainMat lb, const TsOut out, int K, int k_per_split, int* status) {
   extern __shared__ __align__(128) char smem[];
   using SL = TsSmem;
   constexpr int BN = kTsBN, STAGES = kTsStages;
   // broadcast from lane 0 so that the compiler knows the value is the same in every lane (uniform role branches and registers)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int kbeg = blockIdx.z * k_per_split;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int splits = cluster.num_blocks(), rank = cluster.block_rank();
+  const int m0 = blockIdx.y * BM, n0 = (int)(blockIdx.x / splits) * BN;
+  const int kbeg = ((int)blockIdx.z * splits + rank) * k_per_split;
   const int kend = min(K, kbeg + k_per_split);
   const int nkb = (kend - kbeg + BK - 1) / BK;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bars = smem_base + SL::bar_offset;  // full[s], empty[s], acc
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SL::bar_offset + (2 * STAGES + 1) * 8);
+  const int quad = warp & 3, group = warp >> 2;
+  float* raw = reinterpret_cast<float*>(smem + SL::raw_offset) + quad * (SL::a_raw + SL::b_raw);
+  constexpr int kRawStage = SL::raw_stage / 4;
+
+  // Copies of K-block `it`: of A this warp's 32 rows; of B (rows are columns of the result) 16 rows, or 8 k of all 64 rows.
+  auto fetch = [&](int it) {
+    if (it < nkb) {
+      float* ra = raw + (it % kTsRaw) * kRawStage;
+      float* rb = ra + SL::a_raw;
+      const int k0 = kbeg + it * BK;
+      if (TA) copy_lines<32, 32, 36>(ra, la, k0, kend, m0 + quad * 32, la.rows, lane);
+      else copy_lines<32, 32, 36>(ra, la, m0 + quad * 32, la.rows, k0, kend, lane);
+      if (TB) copy_lines<16, 32, 36>(rb, lb, n0 + quad * 16, lb.rows, k0, kend, lane);
+      else copy_lines<8, 64, 68>(rb, lb, k0 + quad * 8, kend, n0, lb.rows, lane);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (warp < kProducerWarps)
+    for (int i = 0; i < kTsRaw / 2; ++i) fetch(group + 2 * i);
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(bars + 8 * s, kProducerWarps);
+      mbar_init(bars + 8 * s, kProducerWarps / 2);
       mbar_init(bars + 8 * (STAGES + s), 1);
     }
     mbar_init(bars + 8 * (2 * STAGES), 1);
@@ -879,102 +962,97 @@ tc_gemm_ts_kernel(const PlainA la, const LB lb, const EPI epi, int K, int k_per_
 
   bool ok = true;
   if (warp < kProducerWarps) {
-    // ---------------- producers: every thread one row of A (16 k-values) and its share of the B tile ----------------
-    const int quad = warp & 3, khalf = warp >> 2;
-    const int row = m0 + quad * 32 + lane;
-    const bool row_ok = row < la.rows;
-    const float* arow = la.trans ? la.p + row : la.p + (int64_t)row * la.ld;
-    Producer<BN, LB> pb;
-    pb.init(lb, n0, warp, lane);
-    struct ABuf { float v[16]; };
-    auto fetch_a = [&](int k0, ABuf& b) {
-      const int kk = k0 + khalf * 16;
+    // ---------------- producers ----------------
+    for (int it = group; it < nkb && ok; it += 2) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kTsRaw / 2 - 1) : "memory");
+      __syncwarp();
+      const float* ra = raw + (it % kTsRaw) * kRawStage;
+      const float* rb = ra + SL::a_raw;
+      uint32_t hi[32];
+      float bv[4][4];  // four K-vectors of B: row and k-quad as below
+      if (TA) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) b.v[i] = 0.f;
-      if (!row_ok || kk >= kend) return;
-      if (!la.trans) {
-        if (la.vec && kk + 15 < kend) {
+        for (int i = 0; i < 32; ++i) hi[i] = __float_as_uint(ra[i * 36 + lane]);
+      } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float4 t = __ldg(reinterpret_cast<const float4*>(arow + kk) + j);
-            b.v[4 * j] = t.x; b.v[4 * j + 1] = t.y; b.v[4 * j + 2] = t.z; b.v[4 * j + 3] = t.w;
-          }
-        } else {
+        for (int i = 0; i < 8; ++i) {
+          const float4 t = *reinterpret_cast<const float4*>(ra + lane * 36 + 4 * i);
+          hi[4 * i] = __float_as_uint(t.x); hi[4 * i + 1] = __float_as_uint(t.y);
+          hi[4 * i + 2] = __float_as_uint(t.z); hi[4 * i + 3] = __float_as_uint(t.w);
+        }
+      }
+      auto b_row = [&](int h) { return TB ? quad * 16 + (lane & 7) + 8 * (h & 1) : 2 * lane + (h & 1); };
+      auto b_kq = [&](int h) { return TB ? (lane >> 3) * 2 + (h >> 1) : quad * 2 + (h >> 1); };
+      if (TB) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (kk + i < kend) b.v[i] = __ldg(arow + kk + i);
+        for (int h = 0; h < 4; ++h) {
+          const float4 t = *reinterpret_cast<const float4*>(rb + ((lane & 7) + 8 * (h & 1)) * 36 + b_kq(h) * 4);
+          bv[h][0] = t.x; bv[h][1] = t.y; bv[h][2] = t.z; bv[h][3] = t.w;
         }
       } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (kk + i < kend) b.v[i] = __ldg(arow + (int64_t)(kk + i) * la.ld);  // consecutive lanes read consecutive rows
+        for (int k = 0; k < 8; ++k) {
+          const float2 t = *reinterpret_cast<const float2*>(rb + k * 68 + 2 * lane);
+          bv[k >> 2 << 1][k & 3] = t.x; bv[(k >> 2 << 1) + 1][k & 3] = t.y;
+        }
       }
-    };
-    ABuf a0, a1;
-    typename Producer<BN, LB>::Buf b0, b1;
-    auto stage_out = [&](int it, const ABuf& ba, const typename Producer<BN, LB>::Buf& bb) -> bool {
+      __syncwarp();  // every lane has read before the slot is filled again
+      fetch(it + kTsRaw);
       const int s = it % STAGES;
-      if (it >= STAGES && !mbar_wait(bars + 8 * (STAGES + s), ((it / STAGES) - 1) & 1, status, 1)) return false;
-      char* st = smem + s * SL::stage_bytes;
-      pb.commit(bb, st, st + SL::b_bytes);
-      uint32_t hi[16], lo[16];
+      if (it >= STAGES) ok = mbar_wait(bars + 8 * (STAGES + s), ((it / STAGES) - 1) & 1, status, 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      const uint32_t ta = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)s * kTsAStageCols;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint32_t h = __float_as_uint(ba.v[i]) & 0xFFFFE000u;
-        hi[i] = h;
-        lo[i] = __float_as_uint(ba.v[i] - __uint_as_float(h));
+      for (int half = 0; half < 2; ++half) {
+        uint32_t h[16], lo[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          h[i] = hi[16 * half + i] & 0xFFFFE000u;
+          lo[i] = __float_as_uint(__uint_as_float(hi[16 * half + i]) - __uint_as_float(h[i]));
+        }
+        tmem_st16(ta + 16 * half, h);
+        tmem_st16(ta + 16 * half + BK, lo);
       }
-      const uint32_t ta = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)s * kTsAStageCols + (uint32_t)khalf * 16;
-      tmem_st16(ta, hi);
-      tmem_st16(ta + BK, lo);
-      tmem_wait_st();
+      char* st = smem + s * SL::stage_bytes;
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int row = b_row(h);
+        float4 vh, vl;
+        split4(bv[h], vh, vl);
+        const uint32_t off = (uint32_t)(row >> 3) * SBO + (uint32_t)b_kq(h) * LBO + (uint32_t)(row & 7) * 16;
+        *reinterpret_cast<float4*>(st + off) = vh;
+        *reinterpret_cast<float4*>(st + SL::b_bytes + off) = vl;
+      }
       fence_async_smem();  // the B stores -> async proxy
+      tmem_wait_st();
       tc_fence_before();   // the tensor-memory stores are ordered before the arrive
       __syncwarp();
       if (lane == 0) mbar_arrive(bars + 8 * s);
-      return true;
-    };
-    if (nkb > 0) {
-      fetch_a(kbeg, a0);
-      pb.fetch(lb, kbeg, kend, b0);
     }
-    for (int it = 0; it < nkb && ok; it += 2) {
-      if (it + 1 < nkb) {
-        fetch_a(kbeg + (it + 1) * BK, a1);
-        pb.fetch(lb, kbeg + (it + 1) * BK, kend, b1);
-      }
-      ok = stage_out(it, a0, b0);
-      if (ok && it + 1 < nkb) {
-        if (it + 2 < nkb) {
-          fetch_a(kbeg + (it + 2) * BK, a0);
-          pb.fetch(lb, kbeg + (it + 2) * BK, kend, b0);
-        }
-        ok = stage_out(it + 1, a1, b1);
-      }
-    }
-    // ---------------- epilogue ----------------
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // ---------------- partial tile -> shared memory (the stages are done with) ----------------
     if (ok && nkb > 0) ok = mbar_wait(bars + 8 * (2 * STAGES), 0, status, 2);
+    ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
-    if (ok) {
-      const int m = m0 + quad * 32 + lane;
-      const int c = khalf;  // two chunks of 32 columns: warps 0-3 the first, warps 4-7 the second
-      float v[32];
-      if (nkb > 0) {
-        const uint32_t t0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32);
-        tmem_ld32(t0, v);  // cross terms
+    float v[32];
+    if (ok && nkb > 0) {
+      const uint32_t t0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(group * 32);  // warps 0-3: columns 0-31, 4-7: 32-63
+      tmem_ld32(t0, v);  // cross terms
 #pragma unroll
-        for (int a = 1; a < kTsAccs; ++a) {
-          float u[32];
-          tmem_ld32(t0 + (uint32_t)(a * BN), u);
+      for (int a = 1; a < kTsAccs; ++a) {
+        float u[32];
+        tmem_ld32(t0 + (uint32_t)(a * BN), u);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += u[j];
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        for (int j = 0; j < 32; ++j) v[j] += u[j];
       }
-      epi.store32(m, n0 + c * 32, v, blockIdx.z);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = 0.f;
     }
+    float4* mine = reinterpret_cast<float4*>(smem + ((quad * 32 + lane) * kTsTileLd + group * 32) * 4);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mine[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
   } else {
     // ---------------- MMA issuer ----------------
     constexpr uint32_t idesc = make_idesc(BN);
@@ -1005,16 +1083,111 @@ tc_gemm_ts_kernel(const PlainA la, const LB lb, const EPI epi, int K, int k_per_
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  // ---------------- sums over the cluster, bias, activation, result: 16 threads a row ----------------
+  if (splits > 1) cluster.sync();
+  const int share = (BM + splits - 1) / splits, row0 = rank * share;  // rows of this CTA
+  const int pieces = min(share, max(BM - row0, 0)) * (BN / 4);        // 128-bit pieces in them
+  float* c = out.c + (int64_t)blockIdx.z * out.split_stride;
+  const bool plain = !out.bias && out.act == RT_ACT_NONE && !out.accumulate;
+  for (int first = 0; first < pieces; first += kProducerWarps * 32) {
+    const int i = first + (int)threadIdx.x, r = row0 + (i >> 4), col = (i & 15) * 4;
+    const bool mine = threadIdx.x < kProducerWarps * 32 && i < pieces && m0 + r < out.M && n0 + col < out.N;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (mine) {
+      const float* t = reinterpret_cast<const float*>(smem) + r * kTsTileLd + col;
+      if (splits == 1) {
+        v = *reinterpret_cast<const float4*>(t);
+      } else {
+        float4 u[8];  // eight remote reads are in flight before the first is added
+        for (int q0 = 0; q0 < splits; q0 += 8) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (q0 + q < splits) u[q] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(t, q0 + q));
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (q0 + q < splits) {
+              v.x += u[q].x; v.y += u[q].y; v.z += u[q].z; v.w += u[q].w;
+            }
+        }
+      }
+    }
+    if (mine) {
+      float* q = c + (int64_t)(m0 + r) * out.ld + n0 + col;
+      const int left = out.N - (n0 + col);
+      if (!plain) v = rt_finish4(v, out.bias ? out.bias + n0 + col : nullptr, out.act, out.accumulate ? q : nullptr, left);
+      if (left >= 4 && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
+        *reinterpret_cast<float4*>(q) = v;
+      } else {
+        q[0] = v.x;
+        if (left > 1) q[1] = v.y;
+        if (left > 2) q[2] = v.z;
+        if (left > 3) q[3] = v.w;
+      }
+    }
+  }
+  if (splits > 1) cluster.sync();  // nobody leaves while its partial tile may still be read
 }
 
-template <class LB, class EPI>
-rt_status launch_ts(rt_ctx* ctx, const PlainA& la, const LB& lb, const EPI& epi, int M, int N, int K, int splits, int kps) {
-  auto kern = tc_gemm_ts_kernel<LB, EPI>;
-  RT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TsSmem::total));
-  dim3 grid((N + kTsBN - 1) / kTsBN, (M + BM - 1) / BM, splits);
-  kern<<<grid, kThreads, TsSmem::total, ctx->stream>>>(la, lb, epi, K, kps, ctx->device_status);
+template <class Kernel>
+cudaError_t prepare_ts(Kernel kern) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TsSmem::total);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+// How many clusters of `splits` CTAs the chip holds at a time: clusters lie within a GPC, of which not all have the same number of
+// SMs, so that fewer CTAs fit in clusters than alone.
+inline int64_t ts_clusters(rt_ctx* ctx, int splits) {
+  struct Table {
+    int n[kTsMaxSplits + 1];
+  };
+  static const Table table = [] {
+    Table t{};
+    auto kern = tc_gemm_ts_kernel<false, false>;
+    for (int i = 2; i <= kTsMaxSplits && prepare_ts(kern) == cudaSuccess; ++i) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      cfg.gridDim = dim3((unsigned)i, 1, 1);
+      cfg.blockDim = dim3(kThreads, 1, 1);
+      cfg.dynamicSmemBytes = TsSmem::total;
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)i;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&t.n[i], kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        t.n[i] = 0;
+      }
+    }
+    return t;
+  }();
+  return splits == 1 ? ctx->sm_count : table.n[splits];
+}
+
+template <bool TA, bool TB>
+rt_status launch_ts(rt_ctx* ctx, const PlainMat& la, const PlainMat& lb, const TsOut& out, int K, int outer, int splits, int kps) {
+  auto kern = tc_gemm_ts_kernel<TA, TB>;
+  static const cudaError_t set = prepare_ts(kern);
+  if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "tensor-core product: %s", cudaGetErrorString(set));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((out.N + kTsBN - 1) / kTsBN * splits), (unsigned)((out.M + BM - 1) / BM), (unsigned)outer);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = TsSmem::total;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)splits;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  RT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, la, lb, out, K, kps, ctx->device_status));
   RT_LAUNCHED(ctx);
   return RT_OK;
+}
+inline rt_status launch_ts(rt_ctx* ctx, bool ta, bool tb, const PlainMat& la, const PlainMat& lb, const TsOut& out, int K, int outer, int splits, int kps) {
+  if (!ta && !tb) return launch_ts<false, false>(ctx, la, lb, out, K, outer, splits, kps);
+  if (!ta) return launch_ts<false, true>(ctx, la, lb, out, K, outer, splits, kps);
+  if (!tb) return launch_ts<true, false>(ctx, la, lb, out, K, outer, splits, kps);
+  return launch_ts<true, true>(ctx, la, lb, out, K, outer, splits, kps);
 }
 
 template <int BN, int STAGES, class LA, class LB, class EPI>
@@ -1093,35 +1266,44 @@ inline bool use_ts_tile(rt_ctx* ctx, int64_t M, int64_t N) {
   const int64_t tiles = ((M + BM - 1) / BM) * ((N + kTsBN - 1) / kTsBN);
   return tiles <= (int64_t)ctx->sm_count;
 }
-template <class LB>
-rt_status gemm_plain_ts(rt_ctx* ctx, const PlainA& la, const LB& lb, float* c, int64_t ldc, int64_t M, int64_t N, int64_t K,
-                        bool accumulate) {
-  const int64_t tiles = ((M + BM - 1) / BM) * ((N + kTsBN - 1) / kTsBN);
-  int splits = 1, kps = (int)((K + BK - 1) / BK * BK);
-  if (!accumulate && ldc == N) {  // one CTA per SM (the kernel takes all of tensor memory); at least 4 K-blocks per split
-    int64_t want = ((int64_t)ctx->sm_count + tiles - 1) / tiles;
-    int64_t max_s = K / (4 * BK);
-    if (max_s < 1) max_s = 1;
-    int64_t sp = want < max_s ? want : max_s;
-    if (sp < 1) sp = 1;
-    if (sp > 512) sp = 512;
-    int64_t per = (K + sp - 1) / sp;
-    per = (per + BK - 1) / BK * BK;
-    sp = (K + per - 1) / per;
-    splits = (int)(sp < 1 ? 1 : sp);
-    kps = (int)per;
+// A tile's cluster: of those of which all fit on the chip at a time, the one that leaves a CTA the fewest K-blocks of 32 (0.5 us each); not
+// split where that gains less than the cluster's meeting costs (1.3 us).
+inline int ts_splits(rt_ctx* ctx, int64_t tiles, int64_t blocks) {
+  int best = 1;
+  int64_t least = blocks - 3;
+  for (int s = 2; s <= kTsMaxSplits && s <= blocks; ++s) {
+    const int64_t each = (blocks + s - 1) / s;
+    if (each < least && tiles <= ts_clusters(ctx, s)) {
+      best = s;
+      least = each;
+    }
   }
-  if (splits == 1) {
-    PlainOut epi{c, ldc, 0, (int)M, (int)N, accumulate};
-    return launch_ts(ctx, la, lb, epi, (int)M, (int)N, (int)K, 1, kps);
+  return best;
+}
+// Only where a CTA is left more than 24 blocks is the reduction also split over partial sums in a workspace, whose addition is a second
+// launch of 2.6 us.
+inline rt_status gemm_plain_ts(rt_ctx* ctx, bool ta, bool tb, const PlainMat& la, const PlainMat& lb, float* c, int64_t ldc, int64_t M, int64_t N,
+                               int64_t K, const float* bias, int act, bool accumulate) {
+  const int64_t tiles = ((M + BM - 1) / BM) * ((N + kTsBN - 1) / kTsBN), blocks = (K + BK - 1) / BK;
+  const int splits = ts_splits(ctx, tiles, blocks);
+  int64_t outer = 1;
+  if (blocks / splits > 24 && !accumulate && ldc == N && !bias && act == RT_ACT_NONE) {
+    outer = ts_clusters(ctx, splits) / tiles;
+    if (outer > blocks / (splits * 8)) outer = blocks / (splits * 8);
+    if (outer < 1) outer = 1;
   }
+  const int kps = (int)((blocks + outer * splits - 1) / (outer * splits) * BK);
+  TsOut out{c, ldc, 0, (int)M, (int)N, bias, act, accumulate};
+  if (outer == 1) return launch_ts(ctx, ta, tb, la, lb, out, (int)K, 1, splits, kps);
   RtScratch ws(ctx);
-  rt_status st = ws.alloc(sizeof(float) * (size_t)splits * M * N);
+  rt_status st = ws.alloc(sizeof(float) * (size_t)outer * M * N);
   if (st != RT_OK) return st;
-  PlainOut epi{ws.as<float>(), N, M * N, (int)M, (int)N, false};
-  st = launch_ts(ctx, la, lb, epi, (int)M, (int)N, (int)K, splits, kps);
+  out.c = ws.as<float>();
+  out.ld = N;
+  out.split_stride = M * N;
+  st = launch_ts(ctx, ta, tb, la, lb, out, (int)K, (int)outer, splits, kps);
   if (st != RT_OK) return st;
-  return rt_sum_axis_internal(ctx, ws.as<float>(), 1, splits, M * N, c, 1.f);
+  return rt_sum_axis_internal(ctx, ws.as<float>(), 1, outer, M * N, c, 1.f);
 }
 
 inline PixelTapRows pixel_rows(const float* src, int C, int H, int W, int rows_h, int rows_w, int kh, int kw, int sh, int sw,
@@ -1148,19 +1330,30 @@ inline TapWeights tap_weights(const float* w, int rows, int kh, int kw, int sn, 
 
 }  // namespace tc
 
+// Microseconds that gemm_plain_ts takes, fitted to 150 products of 0.05 - 400 M multiply-adds (most within 10 %); negative when its tiles
+// do not fit one wave.
+float rt_gemm_ts_estimate(rt_ctx* ctx, int64_t m, int64_t n, int64_t k) {
+  using namespace tc;
+  const int64_t tiles = ((m + BM - 1) / BM) * ((n + kTsBN - 1) / kTsBN), blocks = (k + BK - 1) / BK;
+  if (!use_ts_tile(ctx, m, n)) return -1.f;
+  const int splits = ts_splits(ctx, tiles, blocks);
+  return 4.9f + 0.5f * (float)((blocks + splits - 1) / splits) + (splits > 1 ? 1.3f : 0.f);
+}
+
 // Tensor-core GEMM with the rt_gemm contract.  Returns RT_ERR_UNIMPLEMENTED when the shape is
-// not worth / not possible on this path, so that the caller can use the FP32 kernel.
+// not worth / not possible on this path, so that the caller can use the FP32 kernel; bias and activation only where they are part of
+// the kernel that writes the result.
 rt_status rt_gemm_tc_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a,
-                              int64_t lda, const float* b, int64_t ldb, float* c, int64_t ldc, int accumulate) {
+                              int64_t lda, const float* b, int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   using namespace tc;
   if (m <= 0 || n <= 0 || k <= 0) return RT_ERR_UNIMPLEMENTED;
   if (m >= (1ll << 31) || n >= (1ll << 31) || k >= (1ll << 31)) return RT_ERR_UNIMPLEMENTED;
   bool acc = accumulate != 0;
   if (use_ts_tile(ctx, m, n)) {
-    const PlainA pa{a, lda, (int)m, trans_a != 0, al16(a) && lda % 4 == 0};
-    if (!trans_b) return gemm_plain_ts(ctx, pa, MatMN{b, ldb, (int)n, al16(b) && ldb % 4 == 0}, c, ldc, m, n, k, acc);
-    return gemm_plain_ts(ctx, pa, MatK{b, ldb, (int)n, al16(b) && ldb % 4 == 0}, c, ldc, m, n, k, acc);
+    const PlainMat pa{a, lda, (int)m, al16(a) && lda % 4 == 0}, pb{b, ldb, (int)n, al16(b) && ldb % 4 == 0};
+    return gemm_plain_ts(ctx, trans_a != 0, trans_b != 0, pa, pb, c, ldc, m, n, k, bias, act, acc);
   }
+  if (bias || act != RT_ACT_NONE) return RT_ERR_UNIMPLEMENTED;
   // A(row=m, k): not transposed -> K-contiguous; transposed ([K,M] storage) -> M-contiguous
   // B(row=n, k): not transposed ([K,N] storage) -> N-contiguous; transposed ([N,K]) -> K-contiguous
   if (!trans_a && !trans_b)

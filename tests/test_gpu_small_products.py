@@ -38,6 +38,14 @@ def test_small_product(api, m, k, n, trans):
         close(c.numpy(), a.astype(np.float64) @ b + accumulate * c0, np.sqrt(k))
 
 
+# 128 x 64 tiles in one wave: one row and column more than a tile, a K-block and one, cluster splits 1 .. 16, partial sums in a workspace,
+# copies of 4 and of 16 bytes; and the first size past one wave with a short reduction
+@pytest.mark.parametrize("m,k,n", [(129, 321, 65), (128, 4100, 64), (37, 2049, 577), (300, 33, 2001), (96, 13000, 40), (1120, 144, 1748)])
+@pytest.mark.parametrize("trans", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_medium_product(api, m, k, n, trans):
+    test_small_product(api, m, k, n, trans)
+
+
 # one more than whole tiles and K-blocks, rows that TMA cannot fetch directly, 256- and 128-column tiles, chunks of 1, 2 and 4 K-blocks
 @pytest.mark.parametrize("m,k,n", [(769, 65, 1025), (1024, 64, 768), (1030, 1024, 900), (6200, 100, 70), (2100, 2081, 1900)])
 @pytest.mark.parametrize("trans", [(0, 0), (0, 1), (1, 0), (1, 1)])
