@@ -89,6 +89,9 @@ rt_status rt_upload_submit(rt_ctx* ctx, rt_upload* up, void* dst);
  * and ONE kernel on the context's stream copies every staging buffer to its destination, instead of one device-to-device
  * memcpy per input.  ups[i] must be distinct. */
 rt_status rt_upload_submit_all(rt_ctx* ctx, rt_upload* const* ups, void* const* dsts, int n);
+/* The same for ONE upload that holds several inputs: bytes[i] bytes at offsets[i] of its buffer go to dsts[i].  One host-to-device
+ * copy, one event and (for up to 8 parts) one kernel for all of them; offsets should be multiples of 16. */
+rt_status rt_upload_submit_parts(rt_ctx* ctx, rt_upload* up, int n, const int64_t* offsets, const int64_t* bytes, void* const* dsts);
 /* Writes n <= 4096 floats at src (device) to pinned host memory from rt_host_alloc with a one-block kernel on the context's
  * stream: the read-back of a loss (Backend::copy_to_host, mod.rs:248, without its synchronisation) costs a kernel launch
  * instead of a copy-engine round trip.  The values are visible to the host once an event recorded after this call has
@@ -259,6 +262,13 @@ rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* program);
 /* out[i, :] = src[idx[i], :] (idx: n_idx int32 row numbers in DEVICE memory): the row gather of data::get_random_batch
  * (src/data.rs:125-209), done on the device instead of through a host copy of the whole data set. */
 rt_status rt_gather_rows(rt_ctx* ctx, const float* src, int64_t rows, int64_t row_len, const int32_t* idx, int64_t n_idx, float* out);
+/* The same rows of n_src <= 8 matrices (all inputs of a step) in one launch: outs[s][i, :] = srcs[s][idx[i], :]. */
+rt_status rt_gather_rows_list(rt_ctx* ctx, int n_src, const float* const* srcs, const int64_t* row_lens, int64_t rows, const int32_t* idx,
+                              int64_t n_idx, float* const* outs);
+/* rt_gather_rows_list with the row numbers in an upload's current host buffer: they are copied to the device on its copy stream like the
+ * data of rt_upload_submit, and the gather on the context's stream reads them where they arrive. */
+rt_status rt_upload_gather_rows(rt_ctx* ctx, rt_upload* up, int n_src, const float* const* srcs, const int64_t* row_lens, int64_t rows,
+                                int64_t n_idx, float* const* outs);
 
 /* out[c] += sum over r of x[r, c] for a row-major x[rows, cols]: the gradient of a bias that already holds a gradient (a bias
  * used at every timestep of a recurrent layer), accumulated in place in one launch.  Eight row lanes per column: meant for few rows. */

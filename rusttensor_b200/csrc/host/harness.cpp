@@ -77,7 +77,8 @@ struct DpTrainer {
   bool nccl_in_graph = std::getenv("RT_B200_DP_NCCL_GRAPH") && std::getenv("RT_B200_DP_NCCL_GRAPH")[0] == '1';
   bool update_in_stream() const { return tr->w.optimizer != 0 && (world == 1 || fused || (nccl_in_graph && !overlap_exchange)); }
   // pipelined steps: double-buffered uploads, two loss slots with completion events
-  std::vector<rt_upload*> uploads;
+  rt_upload* upload = nullptr;               // all inputs, one behind another
+  std::vector<int64_t> upload_at, upload_bytes;
   float* pipe_loss[2] = {nullptr, nullptr};
   rt_event* pipe_done[2] = {nullptr, nullptr};
   int64_t pipe_steps = 0;
@@ -85,8 +86,7 @@ struct DpTrainer {
   // travel; the rows are gathered on the device straight into the step's input tensors
   std::vector<Storage> dataset;          // one [rows, sample elements] tensor per input
   int64_t dataset_rows = 0;
-  rt_upload* idx_upload = nullptr;  // row numbers of the next batch: pinned buffers, copy stream and staging like any input
-  Storage idx_dev;
+  rt_upload* idx_upload = nullptr;  // row numbers of the next batch
   // RT_B200_DP_OVERLAP=1 sends the early gradient slice while the backward pass is still running.  Off by default:
   // with this model (1.7 MB of gradients) on two B200s the extra NCCL launch and graph launch cost more than the
   // overlap hides (0.371 ms per step against 0.362 ms).
@@ -96,7 +96,7 @@ struct DpTrainer {
     rt_ctx* c = B200Backend::ctx_slot();
     if (!c) return;
     for (void* p : opened) rt_ipc_close(c, p);
-    for (rt_upload* u : uploads) rt_upload_destroy(c, u);
+    if (upload) rt_upload_destroy(c, upload);
     for (int i = 0; i < 2; ++i) {
       if (pipe_loss[i]) rt_host_free(c, pipe_loss[i]);
       if (pipe_done[i]) rt_event_destroy(c, pipe_done[i]);
@@ -525,42 +525,56 @@ struct DpTrainer {
   }
 
   // ---- pipelined steps: the host runs one step ahead of the device ----
-  void pipe_setup() {
-    if (!uploads.empty()) return;
+  void loss_setup() {
+    if (pipe_done[1]) return;
     rt_ctx* c = B200Backend::ctx();
-    for (auto& x : inputs) {
-      rt_upload* u = nullptr;
-      B200Backend::check(rt_upload_create(c, sizeof(float) * x.size(), &u));
-      uploads.push_back(u);
-    }
     for (int i = 0; i < 2; ++i) {
       void* lp = nullptr;
-      B200Backend::check(rt_host_alloc(c, sizeof(float), &lp));
-      pipe_loss[i] = (float*)lp;
-      B200Backend::check(rt_event_create(c, &pipe_done[i]));
+      if (!pipe_loss[i]) B200Backend::check(rt_host_alloc(c, sizeof(float), &lp));
+      if (lp) pipe_loss[i] = (float*)lp;
+      if (!pipe_done[i]) B200Backend::check(rt_event_create(c, &pipe_done[i]));
     }
   }
+  void upload_setup() {
+    if (upload) return;
+    size_t at = 0;
+    upload_at.clear();
+    upload_bytes.clear();
+    for (auto& x : inputs) {
+      upload_at.push_back((int64_t)at);
+      upload_bytes.push_back((int64_t)(sizeof(float) * x.size()));
+      at += (sizeof(float) * x.size() + 255) & ~size_t(255);
+    }
+    B200Backend::check(rt_upload_create(B200Backend::ctx(), at, &upload));
+  }
   float* pipe_buffer(int i) {
-    pipe_setup();
+    upload_setup();
     void* p = nullptr;
-    B200Backend::check(rt_upload_host_buffer(B200Backend::ctx(), uploads.at(i), &p));
-    return (float*)p;
+    const int64_t at = upload_at.at(i);
+    B200Backend::check(rt_upload_host_buffer(B200Backend::ctx(), upload, &p));
+    return reinterpret_cast<float*>(static_cast<char*>(p) + at);
   }
   // Submits the buffers handed out by pipe_buffer, enqueues the step and the read-back of its loss, and
   // returns the loss of the PREVIOUS pipelined step (its work finished while this one was being enqueued).
   bool step_pipelined(float* prev_loss) {
-    pipe_setup();
+    loss_setup();
+    upload_setup();
     if (!graph) capture();
     rt_ctx* c = B200Backend::ctx();
-    // all inputs in one staging -> tensor kernel (one call per 8 inputs), the loss by a store to pinned memory: no copy-engine
-    // round trip sits between two replays of the step
-    std::vector<void*> dsts;
-    for (auto& x : inputs) {
-      B200Backend::make_unique(x.data_mut());
-      dsts.push_back(x.data().ptr());
+    // all inputs in one copy and one staging -> tensor kernel, the loss by a store to pinned memory: no copy-engine round trip
+    // sits between two replays of the step
+    void* dsts[16];
+    std::vector<void*> more;
+    void** d = dsts;
+    if (inputs.size() > 16) {
+      more.resize(inputs.size());
+      d = more.data();
     }
-    for (size_t i = 0; i < inputs.size(); i += 8)
-      B200Backend::check(rt_upload_submit_all(c, uploads.data() + i, dsts.data() + i, (int)std::min<size_t>(8, inputs.size() - i)));
+    for (size_t i = 0; i < inputs.size(); ++i) {
+      B200Backend::make_unique(inputs[i].data_mut());
+      d[i] = inputs[i].data().ptr();
+    }
+    B200Backend::check(rt_upload_submit_parts(c, upload, (int)inputs.size(), upload_at.data(), upload_bytes.data(), d));
     replay();
     exchange_and_update();
     const int k = (int)(pipe_steps & 1);
@@ -586,33 +600,35 @@ struct DpTrainer {
       dataset.push_back(d);
     }
     dataset_rows = rows;
-    const size_t batch = inputs[0].shape()[0];
-    if (!idx_upload) B200Backend::check(rt_upload_create(B200Backend::ctx(), sizeof(int32_t) * batch, &idx_upload));
-    idx_dev = B200Backend::zeros(rt::Shape{batch});
+    if (inputs.size() > 8) throw Error::invalid_op("attach_dataset: at most 8 inputs");
+    if (!idx_upload) B200Backend::check(rt_upload_create(B200Backend::ctx(), sizeof(int32_t) * inputs[0].shape()[0], &idx_upload));
   }
   // Like step_pipelined, but the inputs are rows `indices` of the attached data set: 4 bytes per sample go to the device.
   bool step_dataset(const int64_t* indices, int64_t n, float* prev_loss) {
     if (dataset.empty()) throw Error::invalid_op("no data set attached");
     const int64_t batch = (int64_t)inputs[0].shape()[0];
     if (n != batch) throw Error(ErrorKind::DimensionMismatch, "step_dataset: one index per sample of the batch");
-    pipe_setup();
+    loss_setup();
     if (!graph) capture();
     rt_ctx* c = B200Backend::ctx();
     const int k = (int)(pipe_steps & 1);
     for (int64_t i = 0; i < n; ++i)
       if (indices[i] < 0 || indices[i] >= dataset_rows) throw Error(ErrorKind::InvalidIndex, "step_dataset: row outside the data set");
-    // the row numbers travel like an input of step_pipelined: host -> staging on the copy stream, staging -> idx_dev by a kernel
+    // the row numbers travel like an input of step_pipelined; all inputs are gathered by one kernel, which reads them where they arrive
     void* hp = nullptr;
     B200Backend::check(rt_upload_host_buffer(c, idx_upload, &hp));
     for (int64_t i = 0; i < n; ++i) static_cast<int32_t*>(hp)[i] = (int32_t)indices[i];
-    void* idx_dst = idx_dev.ptr();
-    B200Backend::check(rt_upload_submit_all(c, &idx_upload, &idx_dst, 1));
+    const float* srcs[8];
+    float* outs[8];
+    int64_t lens[8];
     for (size_t i = 0; i < inputs.size(); ++i) {
-      B200Backend::make_unique(inputs[i].data_mut());
-      const int64_t per = (int64_t)(inputs[i].size() / (size_t)batch);
-      B200Backend::check(rt_gather_rows(c, dataset[i].ptr(), dataset_rows, per, reinterpret_cast<const int32_t*>(idx_dev.ptr()), n,
-                                        inputs[i].data().ptr()));
+      auto& x = inputs[i];
+      B200Backend::make_unique(x.data_mut());
+      srcs[i] = dataset[i].ptr();
+      outs[i] = x.data().ptr();
+      lens[i] = (int64_t)(x.size() / (size_t)batch);
     }
+    B200Backend::check(rt_upload_gather_rows(c, idx_upload, (int)inputs.size(), srcs, lens, dataset_rows, n, outs));
     replay();
     exchange_and_update();
     B200Backend::check(rt_publish_to_host(c, pipe_loss[k], captured_loss.data().ptr(), 1));

@@ -103,6 +103,9 @@ rt_status rt_ctx_destroy(rt_ctx* ctx) {
     cudaEventDestroy(ctx->join_ev);
   }
   rt_dp_finalize(ctx);
+  rt_release_idle_uploads(ctx);
+  for (void* p : ctx->idle_host_blocks) cudaFreeHost(p);
+  for (auto& kv : ctx->host_blocks) cudaFreeHost(kv.first);
   for (auto& kv : ctx->free_blocks) cudaFree(kv.second);
   for (auto& kv : ctx->capture_free) cudaFree(kv.second);
   for (auto& kv : ctx->side_deferred) cudaFree(kv.second);
@@ -161,6 +164,7 @@ rt_status rt_malloc(rt_ctx* ctx, size_t bytes, void** out) {
         ctx->bytes_reserved -= (int64_t)kv.first;
       }
       ctx->free_blocks.clear();
+      rt_release_idle_uploads(ctx);
       e = cudaMalloc(&p, sz);
     }
   }
@@ -257,13 +261,35 @@ rt_status rt_memcpy_d2d(rt_ctx* ctx, void* dst, const void* src, size_t bytes) {
 rt_status rt_host_alloc(rt_ctx* ctx, size_t bytes, void** out) {
   RT_CHECK_CTX(ctx);
   RT_CHECK_PTR(ctx, out);
-  RT_CUDA(ctx, cudaHostAlloc(out, bytes ? bytes : 1, cudaHostAllocDefault));
+  if (bytes <= kHostBlock) {
+    if (!ctx->idle_host_blocks.empty()) {
+      *out = ctx->idle_host_blocks.back();
+      ctx->idle_host_blocks.pop_back();
+    } else {
+      RT_CUDA(ctx, cudaHostAlloc(out, kHostBlock, cudaHostAllocDefault));
+    }
+    ctx->host_blocks[*out] = kHostBlock;
+    return RT_OK;
+  }
+  RT_CUDA(ctx, cudaHostAlloc(out, bytes, cudaHostAllocDefault));
   return RT_OK;
 }
 
 rt_status rt_host_free(rt_ctx* ctx, void* ptr) {
   RT_CHECK_CTX(ctx);
-  if (ptr) RT_CUDA(ctx, cudaFreeHost(ptr));
+  if (!ptr) return RT_OK;
+  auto it = ctx->host_blocks.find(ptr);
+  if (it == ctx->host_blocks.end()) {
+    RT_CUDA(ctx, cudaFreeHost(ptr));
+    return RT_OK;
+  }
+  ctx->host_blocks.erase(it);
+  // as with cudaFreeHost, nothing queued may still use the block when its next owner gets it
+  if (!ctx->capturing && ctx->idle_host_blocks.size() < kIdleHostBlocks && cudaStreamSynchronize(ctx->stream) == cudaSuccess) {
+    ctx->idle_host_blocks.push_back(ptr);
+    return RT_OK;
+  }
+  RT_CUDA(ctx, cudaFreeHost(ptr));
   return RT_OK;
 }
 
@@ -277,7 +303,7 @@ void* rt_stream(rt_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
 // ---- double-buffered input upload ------------------------------------------------------------
 struct rt_upload {
-  size_t bytes = 0;
+  size_t bytes = 0, capacity = 0;
   cudaStream_t copy_stream = nullptr;
   void* pinned[2] = {nullptr, nullptr};
   void* staging[2] = {nullptr, nullptr};
@@ -287,11 +313,7 @@ struct rt_upload {
   int next = 0;
 };
 
-rt_status rt_upload_destroy(rt_ctx* ctx, rt_upload* up) {
-  RT_CHECK_CTX(ctx);
-  if (!up) return RT_OK;
-  if (up->copy_stream) cudaStreamSynchronize(up->copy_stream);
-  cudaStreamSynchronize(ctx->stream);
+static void free_upload(rt_upload* up) {
   for (int i = 0; i < 2; ++i) {
     if (up->pinned[i]) cudaFreeHost(up->pinned[i]);
     if (up->staging[i]) cudaFree(up->staging[i]);
@@ -300,6 +322,25 @@ rt_status rt_upload_destroy(rt_ctx* ctx, rt_upload* up) {
   }
   if (up->copy_stream) cudaStreamDestroy(up->copy_stream);
   delete up;
+}
+}  // extern "C"
+void rt_release_idle_uploads(rt_ctx* ctx) {
+  for (rt_upload* up : ctx->idle_uploads) free_upload(up);
+  ctx->idle_uploads.clear();
+  ctx->idle_upload_bytes = 0;
+}
+extern "C" {
+
+rt_status rt_upload_destroy(rt_ctx* ctx, rt_upload* up) {
+  RT_CHECK_CTX(ctx);
+  if (!up) return RT_OK;
+  const bool idle = (!up->copy_stream || cudaStreamSynchronize(up->copy_stream) == cudaSuccess) && cudaStreamSynchronize(ctx->stream) == cudaSuccess;
+  if (idle && up->consumed[1] && ctx->idle_uploads.size() < kIdleUploads && ctx->idle_upload_bytes + up->capacity <= kIdleUploadBytes) {
+    ctx->idle_uploads.push_back(up);
+    ctx->idle_upload_bytes += up->capacity;
+    return RT_OK;
+  }
+  free_upload(up);
   return RT_OK;
 }
 
@@ -307,18 +348,32 @@ rt_status rt_upload_create(rt_ctx* ctx, size_t bytes, rt_upload** out) {
   RT_CHECK_CTX(ctx);
   RT_CHECK_PTR(ctx, out);
   *out = nullptr;
+  bytes = bytes ? bytes : 1;
+  for (size_t i = 0; i < ctx->idle_uploads.size(); ++i) {
+    rt_upload* up = ctx->idle_uploads[i];
+    if (up->capacity < bytes || up->capacity / 4 > bytes + 16384) continue;
+    ctx->idle_uploads.erase(ctx->idle_uploads.begin() + i);
+    ctx->idle_upload_bytes -= up->capacity;
+    up->bytes = bytes;
+    up->used[0] = up->used[1] = false;
+    up->next = 0;
+    *out = up;
+    return RT_OK;
+  }
   RT_CUDA(ctx, cudaSetDevice(ctx->device));  // the calling thread's current device may be another one
   rt_upload* up = new rt_upload();
-  up->bytes = bytes ? bytes : 1;
+  up->bytes = bytes;
+  up->capacity = (bytes + 4095) & ~size_t(4095);
   cudaError_t e = cudaStreamCreateWithFlags(&up->copy_stream, cudaStreamNonBlocking);
   for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
-    e = cudaHostAlloc(&up->pinned[i], up->bytes, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaMalloc(&up->staging[i], up->bytes);
+    e = cudaHostAlloc(&up->pinned[i], up->capacity, cudaHostAllocDefault);
+    if (e == cudaSuccess) e = cudaMalloc(&up->staging[i], up->capacity);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&up->copied[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&up->consumed[i], cudaEventDisableTiming);
   }
   if (e != cudaSuccess) {
-    rt_upload_destroy(ctx, up);
+    cudaGetLastError();
+    free_upload(up);
     RT_FAIL(ctx, e == cudaErrorMemoryAllocation ? RT_ERR_OOM : RT_ERR_CUDA, "rt_upload_create: %s", cudaGetErrorString(e));
   }
   *out = up;
@@ -421,6 +476,66 @@ rt_status rt_upload_submit_all(rt_ctx* ctx, rt_upload* const* ups, void* const* 
     up->next = k ^ 1;
   }
   return RT_OK;
+}
+
+rt_status rt_upload_submit_parts(rt_ctx* ctx, rt_upload* up, int n, const int64_t* offsets, const int64_t* bytes, void* const* dsts) {
+  RT_CHECK_CTX(ctx);
+  RT_CHECK_PTR(ctx, up);
+  RT_CHECK_PTR(ctx, offsets);
+  RT_CHECK_PTR(ctx, bytes);
+  RT_CHECK_PTR(ctx, dsts);
+  if (n < 1) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_upload_submit_parts: no part");
+  if (ctx->capturing) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_upload_submit_parts during graph capture");
+  size_t end = 0;
+  for (int i = 0; i < n; ++i) {
+    RT_CHECK_PTR(ctx, dsts[i]);
+    if (offsets[i] < 0 || bytes[i] < 0 || (size_t)offsets[i] > up->bytes || (size_t)bytes[i] > up->bytes - (size_t)offsets[i])
+      RT_FAIL(ctx, RT_ERR_INVALID_INDEX, "rt_upload_submit_parts: part %d ends behind the upload's %zu bytes", i, up->bytes);
+    end = std::max(end, (size_t)(offsets[i] + bytes[i]));
+  }
+  const int k = up->next;
+  // the staging buffer may still be read by the staging -> dst copy of two submits ago
+  if (up->used[k]) RT_CUDA(ctx, cudaStreamWaitEvent(up->copy_stream, up->consumed[k], 0));
+  if (end) RT_CUDA(ctx, cudaMemcpyAsync(up->staging[k], up->pinned[k], end, cudaMemcpyHostToDevice, up->copy_stream));
+  RT_CUDA(ctx, cudaEventRecord(up->copied[k], up->copy_stream));
+  RT_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, up->copied[k], 0));
+  for (int first = 0; first < n; first += kMaxUploadsPerSubmit) {
+    const int parts = std::min(n - first, kMaxUploadsPerSubmit);
+    MultiCopyParams p{};
+    size_t most = 0;
+    for (int i = 0; i < parts; ++i) {
+      p.src[i] = static_cast<const char*>(up->staging[k]) + offsets[first + i];
+      p.dst[i] = static_cast<char*>(dsts[first + i]);
+      p.bytes[i] = (unsigned long long)bytes[first + i];
+      most = std::max(most, (size_t)bytes[first + i]);
+    }
+    const size_t units = (most + 15) / 16;
+    const unsigned blocks = (unsigned)std::min<size_t>((units + 255) / 256, (size_t)ctx->sm_count * 4);
+    multi_copy_kernel<<<dim3(blocks ? blocks : 1, (unsigned)parts), 256, 0, ctx->stream>>>(p);
+    RT_LAUNCHED(ctx);
+  }
+  RT_CUDA(ctx, cudaEventRecord(up->consumed[k], ctx->stream));
+  up->used[k] = true;
+  up->next = k ^ 1;
+  return RT_OK;
+}
+
+rt_status rt_upload_gather_rows(rt_ctx* ctx, rt_upload* up, int n_src, const float* const* srcs, const int64_t* row_lens, int64_t rows,
+                                int64_t n_idx, float* const* outs) {
+  RT_CHECK_CTX(ctx);
+  RT_CHECK_PTR(ctx, up);
+  if (ctx->capturing) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_upload_gather_rows during graph capture");
+  if (n_idx < 1 || (uint64_t)n_idx > up->bytes / sizeof(int32_t)) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_upload_gather_rows: more rows than the upload holds");
+  const int k = up->next;
+  if (up->used[k]) RT_CUDA(ctx, cudaStreamWaitEvent(up->copy_stream, up->consumed[k], 0));
+  RT_CUDA(ctx, cudaMemcpyAsync(up->staging[k], up->pinned[k], sizeof(int32_t) * (size_t)n_idx, cudaMemcpyHostToDevice, up->copy_stream));
+  RT_CUDA(ctx, cudaEventRecord(up->copied[k], up->copy_stream));
+  RT_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, up->copied[k], 0));
+  const rt_status st = rt_gather_rows_list(ctx, n_src, srcs, row_lens, rows, static_cast<const int32_t*>(up->staging[k]), n_idx, outs);
+  RT_CUDA(ctx, cudaEventRecord(up->consumed[k], ctx->stream));
+  up->used[k] = true;
+  up->next = k ^ 1;
+  return st;
 }
 
 __global__ void publish_kernel(const float* __restrict__ src, float* __restrict__ host_dst, int n) {

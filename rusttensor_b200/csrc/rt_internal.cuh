@@ -19,6 +19,9 @@ struct rt_graph {
   std::vector<std::pair<size_t, void*>> retired;
 };
 
+struct rt_upload;
+void rt_release_idle_uploads(struct rt_ctx* ctx);
+
 struct rt_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -31,6 +34,12 @@ struct rt_ctx {
   int64_t bytes_reserved = 0, bytes_in_use = 0, n_device_allocs = 0;
   int64_t launches = 0;
   bool capturing = false;
+  // Destroyed uploads (at most kIdleUploads of kIdleUploadBytes in all) and small pinned blocks (at most kIdleHostBlocks) wait here for
+  // the next owner: pinning memory and creating a stream cost milliseconds, which the first step of every new trainer paid.
+  std::vector<rt_upload*> idle_uploads;
+  size_t idle_upload_bytes = 0;
+  std::vector<void*> idle_host_blocks;
+  std::map<void*, size_t> host_blocks;  // pinned blocks of kHostBlock bytes that are in use
   std::multimap<size_t, void*> capture_free;  // released during capture: reusable only inside it
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   // side stream (rt_side_stream_*): `stream` points at it between begin and end
@@ -62,6 +71,7 @@ struct rt_ctx {
   int dp_rank = 0, dp_world = 1;
 };
 
+constexpr size_t kIdleUploads = 16, kIdleUploadBytes = size_t(256) << 20, kIdleHostBlocks = 64, kHostBlock = 16384;
 constexpr int kReduceCounterSlots = 4096;  // per stream half: tickets of the column reductions
 constexpr int kAuxCounterSlots = 128;      // per stream half, behind them: tickets of other kernels that hand partial sums over
 

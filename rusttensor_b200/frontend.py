@@ -236,11 +236,15 @@ class Engine:
         self.lib = lib
         self.prefix = prefix
         self.ops = _Ops(self)
+        self._fns = {}
         getattr(lib, f"{prefix}_last_error").restype = C.c_char_p
 
     def _call(self, name, *args):
-        fn = getattr(self.lib, f"{self.prefix}_{name}")
-        fn.restype = C.c_int
+        fn = self._fns.get(name)
+        if fn is None:
+            fn = getattr(self.lib, f"{self.prefix}_{name}")
+            fn.restype = C.c_int
+            self._fns[name] = fn
         rc = fn(*args)
         if rc != 0:
             msg = getattr(self.lib, f"{self.prefix}_last_error")()

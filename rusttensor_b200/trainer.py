@@ -37,6 +37,7 @@ class DataParallelTrainer:
                 break
             i += 1
         self._pinned = []
+        self._pipeline_views = {}
         for i, t in enumerate(self.inputs):
             p = _f32p()
             self._call("dp_pinned_input", C.c_int64(self.handle), C.c_int(i), C.byref(p))
@@ -196,9 +197,13 @@ class DataParallelTrainer:
     def pipeline_buffer(self, i):
         """numpy view of the pinned host buffer to fill with input ``i`` of the NEXT pipelined step
         (two buffers alternate; the call waits until the copy that last read this one has finished)."""
-        p = _f32p()
+        p = C.c_void_p()
         self._call("dp_pipeline_buffer", C.c_int64(self.handle), C.c_int(i), C.byref(p))
-        return np.ctypeslib.as_array(p, shape=tuple(self.inputs[i].shape))
+        view = self._pipeline_views.get((i, p.value))  # two buffers per input, for the trainer's lifetime
+        if view is None:
+            view = np.ctypeslib.as_array(C.cast(p, _f32p), shape=tuple(self.inputs[i].shape))
+            self._pipeline_views[(i, p.value)] = view
+        return view
 
     def step_pipelined(self):
         """Enqueues one step from the pipeline buffers and returns the loss of the previous pipelined

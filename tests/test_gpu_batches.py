@@ -1,0 +1,62 @@
+"""Inputs of a step: several parts of one upload, and rows of several matrices gathered by uploaded numbers."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def api():
+    from rusttensor_b200 import CApi
+
+    a = CApi()
+    yield a
+    a.close()
+
+
+@pytest.mark.parametrize("parts", [1, 2, 9])  # the kernel copies eight at a time
+def test_upload_parts(api, parts):
+    r = np.random.default_rng(parts)
+    sizes = [1 + 37 * i for i in range(parts)]
+    at = np.cumsum([0] + [(4 * n + 255) // 256 * 256 for n in sizes])
+    for _ in range(2):  # the second upload takes over what the first has left
+        up, dst = C.c_void_p(), [api.to_device(np.zeros(n, np.float32)) for n in sizes]
+        api.call("upload_create", C.c_size_t(int(at[-1])), C.byref(up))
+        offsets, nbytes = (C.c_int64 * parts)(*at[:-1].tolist()), (C.c_int64 * parts)(*[4 * n for n in sizes])
+        ptrs = (C.c_void_p * parts)(*[d.ptr.value for d in dst])
+        for _ in range(3):
+            p, data = C.c_void_p(), [r.random(n, dtype=np.float32) for n in sizes]
+            api.call("upload_host_buffer", up, C.byref(p))
+            for a, o in zip(data, at):
+                C.memmove(p.value + int(o), a.ctypes.data, a.nbytes)
+            api.call("upload_submit_parts", up, parts, offsets, nbytes, ptrs)
+            for a, d in zip(data, dst):
+                np.testing.assert_array_equal(a, d.numpy())
+        nbytes[0] = int(at[-1]) + 1
+        with pytest.raises(Exception, match="ends behind"):
+            api.call("upload_submit_parts", up, parts, offsets, nbytes, ptrs)
+        api.call("upload_destroy", up)
+
+
+@pytest.mark.parametrize("n_idx", [1, 7, 301, 5000])  # one to eight rows a block, the last of them not full
+def test_gather_rows_list(api, n_idx):
+    r = np.random.default_rng(n_idx)
+    rows, lens = 613, [1, 10, 784, 0]
+    data = [r.random((rows, n), dtype=np.float32) for n in lens]
+    src, dst = [api.to_device(d) for d in data[:3]], [api.to_device(np.ones((n_idx, n), np.float32)) for n in lens[:3]]
+    up, p = C.c_void_p(), C.c_void_p()
+    api.call("upload_create", C.c_size_t(4 * n_idx), C.byref(up))
+    ptrs = lambda ts: (C.c_void_p * 4)(*[t.ptr.value for t in ts], None)  # noqa: E731
+    for _ in range(3):
+        api.call("upload_host_buffer", up, C.byref(p))
+        idx = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_int32)), (n_idx,))
+        idx[:] = r.integers(0, rows, n_idx)
+        want = [d[idx] for d in data]
+        idx[-1] = rows  # outside: a row of zeros
+        api.call("upload_gather_rows", up, 4, ptrs(src), (C.c_int64 * 4)(*lens), C.c_int64(rows), C.c_int64(n_idx), ptrs(dst))
+        for w, d in zip(want, dst):
+            w[-1] = 0
+            np.testing.assert_array_equal(w, d.numpy())
+    api.call("upload_destroy", up)
