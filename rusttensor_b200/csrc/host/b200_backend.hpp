@@ -805,6 +805,21 @@ struct B200Backend {
       if (const lazy::Input* t = lazy::times_constant(g.buf->node.get(), &c)) {
         const float* tp = t->buf->data();
         if (g.buf->node) {
+          const float* xp = x.ptr();
+          lazy::Loss l;
+          DeviceBuffer* loss = lazy::loss_over(x.buf.get(), t->buf.get(), &l);
+          if (loss && l.rows == (int64_t)a.outer && l.classes == (int64_t)a.len) {  // the loss itself comes out of the same pass
+            auto keep = loss->shared_from_this();
+            float* out = lazy::new_block(loss->ctx, loss->numel);
+            const rt_status st = rt_softmax_nll_with_grad(ctx(), xp, tp, a.outer, a.len, l.scale, l.divisor, c, out, dx.ptr());
+            if (st != RT_OK) {
+              rt_free(ctx(), out);
+              check(st);
+            }
+            loss->ptr = out;
+            loss->drop_node();
+            return dx;
+          }
           check(rt_softmax_nll_scaled_backward(ctx(), x.ptr(), tp, a.outer, a.len, c, dx.ptr()));
           return dx;
         }

@@ -921,6 +921,20 @@ inline bool rewrite_loss(DeviceBuffer* b) {
   return true;
 }
 
+// The unevaluated classification loss that log_softmax of `logits` leads to, if nothing else reads any step of it.
+inline DeviceBuffer* loss_over(DeviceBuffer* logits, DeviceBuffer* targets, Loss* l) {
+  for (DeviceBuffer* r : logits->readers) {
+    if (!r->node || r->node->tag != Tag::LogSoftmax) continue;
+    DeviceBuffer* root = nullptr;
+    for (DeviceBuffer* b = r; b->readers.size() == 1;) {
+      b = b->readers[0];
+      if (b->node && match_loss(b, l)) root = b;
+    }
+    if (root && root->readers.empty() && match_loss(root, l) && l->logits->buf.get() == logits && l->targets->buf.get() == targets) return root;
+  }
+  return nullptr;
+}
+
 // max_pool2d's gradient masked by the relu in front of the pooling: one pass.
 inline bool rewrite_pool(DeviceBuffer* b) {
   const Node* n = b->node.get();

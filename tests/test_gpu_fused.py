@@ -96,3 +96,23 @@ def test_a_malformed_program_is_refused():
     with pytest.raises(RtError):
         api.call("fused_elementwise", C.create_string_buffer(8192))  # zero dimensions, no outputs
     api.close()
+
+
+# one block and several, a row more and less than a block of each form (128 rows; 8 rows), the change of form at 16 classes
+@pytest.mark.parametrize("rows,classes", [(1, 1), (127, 10), (129, 16), (9, 17), (1000, 16), (1003, 300)])
+def test_classification_loss_with_gradient(rows, classes):
+    import ctypes as C
+
+    from rusttensor_b200 import CApi
+
+    api, r = CApi(), np.random.default_rng(rows + classes)
+    x, t = r.standard_normal((rows, classes)).astype(np.float32), r.random((rows, classes), dtype=np.float32)
+    dx, dt, loss, grad = api.to_device(x), api.to_device(t), api.to_device(np.zeros(1, np.float32)), api.to_device(np.zeros_like(x))
+    ls = x - np.log(np.exp(x.astype(np.float64)).sum(1, keepdims=True))
+    for _ in range(2):  # the ticket has to be back at zero
+        api.call("softmax_nll_with_grad", dx.ptr, dt.ptr, C.c_int64(rows), C.c_int64(classes), C.c_float(-1), C.c_float(rows), C.c_float(-1 / rows),
+                 loss.ptr, grad.ptr)
+        np.testing.assert_allclose(loss.numpy()[0], -(ls * t).sum() / rows, rtol=2e-6, atol=1e-7)
+        want = -(t - np.exp(ls) * t.sum(1, keepdims=True, dtype=np.float64)) / rows
+        np.testing.assert_allclose(grad.numpy(), want, rtol=1e-4, atol=2e-6 * np.abs(want).max() + 1e-9)
+    api.close()
