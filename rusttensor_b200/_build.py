@@ -2,18 +2,21 @@
 
   rusttensor_b200/librt_b200.so       the C-ABI CUDA library (include/rt_b200.h), sm_100a only
   rusttensor_b200/librt_b200_host.so  the C++ host engine over that ABI (rth_* functions)
+  rusttensor_b200/_fastcall.so        CPython extension: the front end's most frequent calls
 
 nvcc cross-compiles without a GPU, so this runs on a CPU-only machine as well.
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "librt_b200.so")
 HOST_LIB = os.path.join(HERE, "librt_b200_host.so")
+FAST_LIB = os.path.join(HERE, "_fastcall.so")
 
 CU_SOURCES = ["rt_context.cu", "k_elementwise.cu", "k_fused.cu", "k_fused_known.cu", "k_fused_lstm.cu", "k_reduce.cu", "k_pool.cu", "k_optim.cu", "k_gemm.cu", "k_gemm_small.cu", "k_gemm_tma.cu", "k_gemm_tc.cu", "k_conv_tc.cu", "k_conv_thin.cu", "k_lstm.cu", "k_tc_probe.cu", "k_conv_dw_tc.cu", "k_random.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
@@ -32,6 +35,16 @@ def _headers():
     for root, _, files in os.walk(CSRC):
         out += [os.path.join(root, f) for f in files if f.endswith((".cuh", ".hpp", ".h", ".inc"))]
     return out
+
+
+def build_fastcall(verbose=False, force=False):
+    src = os.path.join(CSRC, "host", "fastcall.cpp")
+    if force or _newer(FAST_LIB, [src]):
+        cmd = [os.environ.get("CXX", "g++")] + HOST_FLAGS + ["-shared", "-I" + sysconfig.get_paths()["include"], src, "-o", FAST_LIB]
+        if verbose:
+            print(" ".join(cmd), file=sys.stderr)
+        subprocess.run(cmd, check=True)
+    return FAST_LIB
 
 
 def build(verbose=False, force=False):
@@ -63,6 +76,7 @@ def build(verbose=False, force=False):
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
         subprocess.run(cmd, check=True)
+    build_fastcall(verbose, force)
     return LIB, HOST_LIB
 
 

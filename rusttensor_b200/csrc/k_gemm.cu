@@ -485,7 +485,7 @@ rt_status gemm_narrow(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t 
   if (k < 1 || m >= (1ll << 31) || n >= (1ll << 31) || m * n >= (1ll << 40)) return RT_ERR_UNIMPLEMENTED;
   // A thread reads k values of both operands by itself: with a reduction that is contiguous in B, or rows that are in A, these reads
   // do not coalesce, which shows from some millions of multiply-adds on (768 x 16 x 1196: B plain 10 us, B transposed 30, A transposed 16).
-  const bool small_k = k <= 16 && !((trans_a || trans_b) && m * n * k > (5ll << 19)) && !bias && act == RT_ACT_NONE;
+  const bool small_k = k <= 16 && !((trans_a || trans_b) && m * n * k > (4ll << 20)) && !bias && act == RT_ACT_NONE;
   // One block walks the whole reduction of its 32 rows: 1.8 us and 1.2 more per 100 of it, against 5 us and more in the small tiles
   // (351 x 173 x 7: 4.5 us here; 173 x 351 x 7: 5.8 here, 5.2 there; 88 x 1288 x 16: 17 and 7).  Many rows fill the chip all the same.
   const bool skinny_n = n <= kSkinnyN && k > 16 && k < (1ll << 30) && m < (1ll << 30) &&

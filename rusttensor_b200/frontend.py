@@ -10,6 +10,14 @@ import ctypes as C
 
 import numpy as np
 
+try:
+    from ._fastcall import Calls, TensorBase
+except ImportError:  # not built yet; needs only a host compiler
+    from ._build import build_fastcall
+
+    build_fastcall()
+    from ._fastcall import Calls, TensorBase
+
 _i64p = C.POINTER(C.c_int64)
 _f32p = C.POINTER(C.c_float)
 _f64p = C.POINTER(C.c_double)
@@ -41,16 +49,8 @@ def _f64(values):
     return arr
 
 
-class Tensor:
-    def __init__(self, engine, handle):
-        self.engine = engine
-        self.handle = handle
-
-    def __del__(self):
-        try:
-            self.engine._call("tensor_free", C.c_int64(self.handle))
-        except Exception:
-            pass
+class Tensor(TensorBase):
+    """``engine``, ``handle`` and ``grad`` come from the base; so does the release of the handle."""
 
     @property
     def shape(self):
@@ -76,16 +76,6 @@ class Tensor:
     def update_from_host(self, data):
         a = np.require(data, dtype=np.float32, requirements='C')
         self.engine._call("tensor_update_from_host", C.c_int64(self.handle), a.ctypes.data_as(_f32p), C.c_int64(a.size))
-
-    @property
-    def grad(self):
-        has = C.c_int(0)
-        self.engine._call("tensor_has_grad", C.c_int64(self.handle), C.byref(has))
-        if not has.value:
-            return None
-        out = C.c_int64(0)
-        self.engine._call("tensor_grad", C.c_int64(self.handle), C.byref(out))
-        return Tensor(self.engine, out.value)
 
     def set_grad(self, grad):
         self.engine._call("tensor_set_grad", C.c_int64(self.handle), C.c_int64(grad.handle))
@@ -237,6 +227,7 @@ class Engine:
         self.prefix = prefix
         self.ops = _Ops(self)
         self._fns = {}
+        self._calls = Calls(*[C.cast(getattr(lib, f"{prefix}_{n}"), C.c_void_p).value for n in ("op", "tensor_free", "tensor_has_grad", "tensor_grad")])
         getattr(lib, f"{prefix}_last_error").restype = C.c_char_p
 
     def _call(self, name, *args):
@@ -247,8 +238,11 @@ class Engine:
             self._fns[name] = fn
         rc = fn(*args)
         if rc != 0:
-            msg = getattr(self.lib, f"{self.prefix}_last_error")()
-            raise EngineError(rc, msg.decode() if msg else "")
+            self._raise(rc)
+
+    def _raise(self, rc):
+        msg = getattr(self.lib, f"{self.prefix}_last_error")()
+        raise EngineError(rc, msg.decode() if msg else "")
 
     def tensor(self, data, shape=None, requires_grad=False):
         """``Tensor::from_vec(data, shape, requires_grad)`` (src/tensor.rs:948-950)."""
@@ -298,10 +292,7 @@ class Engine:
         return Tensor(self, ox.value), Tensor(self, oy.value)
 
     def op(self, name, inputs, ip=(), fp=()):
-        out = C.c_int64(0)
-        self._call("op", name.encode(), _i64([t.handle for t in inputs]), C.c_int(len(inputs)),
-                   _i64(ip), C.c_int(len(ip)), _f64(fp), C.c_int(len(fp)), C.byref(out))
-        return Tensor(self, out.value)
+        return self._calls.op(Tensor, self, name, inputs, ip, fp)
 
     def op_backward(self, output, grad):
         """Calls the backward closure of the op that produced ``output`` with ``grad`` directly."""
