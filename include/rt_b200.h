@@ -202,6 +202,9 @@ rt_status rt_slice_assign(rt_ctx* ctx, float* dst, const int64_t* dst_shape, int
 /* out[i] = x[starts + i]: slice mod.rs:522, concat_backward mod.rs:563. */
 rt_status rt_slice(rt_ctx* ctx, const float* x, const int64_t* x_shape, int ndim, const int64_t* starts,
                    const int64_t* out_shape, float* out);
+/* `count` pieces side by side: out[o, sum of the lens before i + j] = srcs[i][o * lens[i] + j] for o < outer, j < lens[i].  One launch
+ * for up to 256 pieces. */
+rt_status rt_concat_list(rt_ctx* ctx, int count, const float* const* srcs, const int64_t* lens, int64_t outer, float* out);
 
 /* ---- one kernel for a chain of elementwise ops -------------------------------------------------------------------
  * An expression over tensors is given as a short program that one kernel runs for every element of an iteration space of

@@ -105,6 +105,7 @@ __device__ __forceinline__ void execute(const FusedParams& p, const Quad<VEC>& e
 constexpr int kKnownThreads = 128;
 template <class P, bool VEC>
 __global__ void __launch_bounds__(kKnownThreads) known_kernel(const __grid_constant__ FusedParams p) {
+  RT_PDL_ENTRY();
   for (uint32_t tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
     Quad<VEC> e;
 #pragma unroll
@@ -131,8 +132,8 @@ rt_status launch_program(rt_ctx* ctx, FusedParams& p, bool vec, int64_t numel) {
   const int64_t tiles = (numel + kKnownThreads * 4 - 1) / (kKnownThreads * 4), cap = (int64_t)ctx->sm_count * 32;
   p.tiles = (uint32_t)tiles;
   const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-  if (vec) known_kernel<P, true><<<grid, kKnownThreads, 0, ctx->stream>>>(p);
-  else known_kernel<P, false><<<grid, kKnownThreads, 0, ctx->stream>>>(p);
+  if (vec) rt_launch(ctx, known_kernel<P, true>, grid, kKnownThreads, 0, p);
+  else rt_launch(ctx, known_kernel<P, false>, grid, kKnownThreads, 0, p);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

@@ -607,13 +607,15 @@ struct B200Backend {
       return defer(std::move(n), os);
     }
     Storage y = alloc(os);
-    auto od = dims(os);
-    std::vector<int64_t> starts(os.size(), 0);
+    int64_t outer = 1;
+    for (size_t d = 0; d < axis; ++d) outer *= (int64_t)os[d];
+    std::vector<const float*> srcs;
+    std::vector<int64_t> lens;
     for (auto* x : xs) {
-      auto xd = dims(x->shape);
-      check(rt_slice_assign(ctx(), y.ptr(), od.data(), (int)od.size(), starts.data(), x->ptr(), xd.data()));
-      starts[axis] += (int64_t)x->shape[axis];
+      srcs.push_back(x->numel() ? x->ptr() : nullptr);
+      lens.push_back(outer ? (int64_t)x->numel() / outer : 0);
     }
+    check(rt_concat_list(ctx(), (int)xs.size(), srcs.data(), lens.data(), outer, y.ptr()));
     return y;
   }
   // concat({x[r0:r1, :], h}, axis 1) for 2-D x and h without materialising the row slice: rows r0..r1 of a row-major matrix are

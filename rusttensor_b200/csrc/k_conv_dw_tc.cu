@@ -546,6 +546,7 @@ __global__ void __launch_bounds__(32 * GROUPS) conv_dw_finish_kernel(const float
                                                                float* __restrict__ dw, float* __restrict__ db, int Cout, int Cin,
                                                                int kh, int kw, int CIT, int n_cit, int NP, int cpc, int tile_elems,
                                                                int dw_elems, int db_elems) {
+  RT_PDL_ENTRY();
   __shared__ float red[GROUPS][33];
   const int lane_o = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int o = (int)blockIdx.x * 32 + lane_o;
@@ -603,6 +604,7 @@ __global__ void __launch_bounds__(32 * GROUPS) conv_dw_finish_vec_kernel(const f
                                                                    float* __restrict__ dw, float* __restrict__ db, int Cout, int Cin,
                                                                    int kh, int kw, int CIT, int n_cit, int NP, int cpc, int tile_elems,
                                                                    int dw_elems, int db_elems) {
+  RT_PDL_ENTRY();
   __shared__ float4 red[GROUPS][32];
   const int lane_o = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int o = ((int)blockIdx.x * 32 + lane_o) * 4;
@@ -788,10 +790,10 @@ rt_status rt_conv_dw_tma_internal(rt_ctx* ctx, const float* x, const float* y, c
   if (st != RT_OK) return st;
   const int tile_elems = kCoTile * p.row_len, dw_elems = p.n_combo * tile_elems, db_elems = db ? p.n_cot * kCoTile : 0;
   if (cit % 4 == 0)
-    conv_dw_finish_vec_kernel<16, 12><<<((dw_elems + db_elems) / 4 + 31) / 32, 512, 0, ctx->stream>>>(
+    rt_launch(ctx, conv_dw_finish_vec_kernel<16, 12>, ((dw_elems + db_elems) / 4 + 31) / 32, 512, 0, 
         p.ws, p.ws_db, dw, db, g.Cy, g.Cx, g.kh, g.kw, cit, p.n_cit, NP, p.cpc, tile_elems, dw_elems, db_elems);
   else
-    conv_dw_finish_kernel<8><<<(dw_elems + db_elems + 31) / 32, 256, 0, ctx->stream>>>(p.ws, p.ws_db, dw, db, g.Cy, g.Cx, g.kh, g.kw, cit, p.n_cit,
+    rt_launch(ctx, conv_dw_finish_kernel<8>, (dw_elems + db_elems + 31) / 32, 256, 0, p.ws, p.ws_db, dw, db, g.Cy, g.Cx, g.kh, g.kw, cit, p.n_cit,
                                                                                   NP, p.cpc, tile_elems, dw_elems, db_elems);
   RT_LAUNCHED(ctx);
   return RT_OK;

@@ -213,6 +213,7 @@ constexpr int kImgThreads = 512;
 // and the KH x (KW + 3) patch of the image as 64-bit shared-memory loads - which halves the instructions per multiply-add.
 template <int KH, int KW, bool QUAD>
 __global__ void __launch_bounds__(kImgThreads) thin_dw_image_kernel(const ImageDwParams p) {
+  RT_PDL_ENTRY();
   constexpr int T = KH * KW;
   extern __shared__ __align__(16) float tile[];  // Hp x Wp: the image with its halo
   __shared__ float phase1[8][4][T + 1];          // sums of the warps that took the odd pixel blocks
@@ -422,6 +423,7 @@ constexpr int kPoolChannelGroup = 16;
 __global__ void __launch_bounds__(kThreads) thin_conv_relu_pool_kernel(const ThinPoolParams p, const float* __restrict__ w,
                                                                         const float* __restrict__ bias, float* __restrict__ y,
                                                                         float* __restrict__ idx) {
+  RT_PDL_ENTRY();
   // weights transposed to [tap][channel]: one 128-bit broadcast load brings a tap's weights for four channels; channels past the
   // layer's last one hold zeros and are computed but not stored
   __shared__ __align__(16) float w_t[9][kPoolChannelGroup];
@@ -558,7 +560,7 @@ rt_status rt_conv_relu_pool_thin_internal(rt_ctx* ctx, const float* x, const flo
   const int groups = (g.Cy + kPoolChannelGroup - 1) / kPoolChannelGroup;
   if (groups > 65535) return RT_ERR_UNIMPLEMENTED;
   const dim3 grid(rt_grid_for(ctx, p.pooled, kThreads, 16), groups);
-  thin_conv_relu_pool_kernel<<<grid, kThreads, 0, ctx->stream>>>(p, w, bias, y, idx);
+  rt_launch(ctx, thin_conv_relu_pool_kernel, grid, kThreads, 0, p, w, bias, y, idx);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }
@@ -587,8 +589,8 @@ static rt_status weight_grad_image(rt_ctx* ctx, const float* x, const float* gy,
   p.d_Wo.init(g.Wy);
   p.d_Wp.init(p.Wp);
   p.d_Wq.init(g.Wy / 4 > 0 ? g.Wy / 4 : 1);
-  if (g.Wy % 4 == 0 && rt_aligned16(gy)) thin_dw_image_kernel<3, 3, true><<<grid, kImgThreads, smem, ctx->stream>>>(p);
-  else thin_dw_image_kernel<3, 3, false><<<grid, kImgThreads, smem, ctx->stream>>>(p);
+  if (g.Wy % 4 == 0 && rt_aligned16(gy)) rt_launch(ctx, thin_dw_image_kernel<3, 3, true>, grid, kImgThreads, smem, p);
+  else rt_launch(ctx, thin_dw_image_kernel<3, 3, false>, grid, kImgThreads, smem, p);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

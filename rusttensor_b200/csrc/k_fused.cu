@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) fused_kernel(const __grid_con
   using E = Elements<V, VEC>;
   extern __shared__ float4 file[];
   __shared__ uint2 code[RT_FUSED_MAX_CODE + 1];
+  RT_PDL_ENTRY();
   for (int i = threadIdx.x; i < p.n_code; i += THREADS) code[i] = p.code[i];
   __syncthreads();
   const Registers<V, THREADS> r{file + threadIdx.x};
@@ -235,7 +236,7 @@ rt_status launch_fused(rt_ctx* ctx, FusedParams& p, int64_t numel) {
   auto kern = fused_kernel<V, VEC, THREADS, BLOCKS>;
   static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "rt_fused_elementwise: %s", cudaGetErrorString(set));
-  kern<<<(unsigned)(tiles < cap ? tiles : cap), THREADS, smem, ctx->stream>>>(p);
+  rt_launch(ctx, kern, (unsigned)(tiles < cap ? tiles : cap), THREADS, smem, p);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

@@ -183,6 +183,7 @@ constexpr int BK = 16;
 
 template <int BM, int BN, int TM, int TN, class LA, class LB, class SC>
 __global__ void __launch_bounds__(256) gemm_tile_kernel(LA la, LB lb, SC sc, int M, int N, int K, int k_per_split) {
+  RT_PDL_ENTRY();
   static_assert((BM / TM) * (BN / TN) == 256, "256 threads per tile");
   static_assert(TM % 4 == 0 && TN % 4 == 0, "register tile is made of 4-wide groups");
   __shared__ __align__(16) float As[2][BK][BM + 4];
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(256) gemm_tile_kernel(LA la, LB lb, SC sc, int
 template <int BM, int BN, int TM, int TN, class LA, class LB, class SC>
 void launch_tile(rt_ctx* ctx, const LA& la, const LB& lb, const SC& sc, int M, int N, int K, int splits, int kps) {
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, splits);
-  gemm_tile_kernel<BM, BN, TM, TN, LA, LB, SC><<<grid, 256, 0, ctx->stream>>>(la, lb, sc, M, N, K, kps);
+  rt_launch(ctx, gemm_tile_kernel<BM, BN, TM, TN, LA, LB, SC>, grid, 256, 0, la, lb, sc, M, N, K, kps);
 }
 
 // Picks a tile shape for (M, N) and launches.  splits > 1 requires a PlainC store that
@@ -370,6 +371,7 @@ template <bool TA, bool TB>
 __global__ void __launch_bounds__(kSkinnyRows * kSkinnySlices)
 gemm_skinny_n_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ b, int64_t ldb, float* __restrict__ c,
                      int64_t ldc, int M, int N, int K, const float* __restrict__ bias, int act, int accumulate) {
+  RT_PDL_ENTRY();
   constexpr int T = kSkinnyRows * kSkinnySlices;
   __shared__ float As[kSkinnyRows][kSkinnyKC + 1];
   __shared__ __align__(16) float Bs[kSkinnyKC][kSkinnyN];
@@ -447,6 +449,7 @@ template <bool TA, bool TB>
 __global__ void __launch_bounds__(256) gemm_small_k_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ b,
                                                            int64_t ldb, float* __restrict__ c, int64_t ldc, int64_t MN, int N, int K,
                                                            int accumulate) {
+  RT_PDL_ENTRY();
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < MN; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = e / N;
     const int j = (int)(e - i * N);
@@ -468,11 +471,11 @@ template <bool TA, bool TB>
 rt_status gemm_narrow_launch(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
                              int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   if (k <= 16) {
-    gemm_small_k_kernel<TA, TB><<<rt_grid_for(ctx, m * n, 256), 256, 0, ctx->stream>>>(a, lda, b, ldb, c, ldc, m * n, (int)n,
+    rt_launch(ctx, gemm_small_k_kernel<TA, TB>, rt_grid_for(ctx, m * n, 256), 256, 0, a, lda, b, ldb, c, ldc, m * n, (int)n,
                                                                                       (int)k, accumulate);
   } else {
     const int grid = (int)((m + kSkinnyRows - 1) / kSkinnyRows);
-    gemm_skinny_n_kernel<TA, TB><<<grid, kSkinnyRows * kSkinnySlices, 0, ctx->stream>>>(a, lda, b, ldb, c, ldc, (int)m, (int)n,
+    rt_launch(ctx, gemm_skinny_n_kernel<TA, TB>, grid, kSkinnyRows * kSkinnySlices, 0, a, lda, b, ldb, c, ldc, (int)m, (int)n,
                                                                                         (int)k, bias, act, accumulate);
   }
   RT_LAUNCHED(ctx);
@@ -598,6 +601,7 @@ namespace {
 // c = act(c + bias) in place, for the products whose kernel has no epilogue of its own
 __global__ void __launch_bounds__(256) bias_act_kernel(float* __restrict__ c, const float* __restrict__ bias, int64_t m, int n, int64_t ldc,
                                                        int act) {
+  RT_PDL_ENTRY();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m * n; i += (int64_t)gridDim.x * blockDim.x) {
     float* q = c + i / n * ldc + i % n;
     float v = *q + (bias ? __ldg(bias + i % n) : 0.f);
@@ -616,6 +620,7 @@ struct RowList {
   int count;
 };
 __global__ void __launch_bounds__(1024) col_sum_list_kernel(const RowList l, int64_t total, int64_t cols, float* __restrict__ out) {
+  RT_PDL_ENTRY();
   __shared__ float red[32][33];
   const int64_t c = (int64_t)blockIdx.x * 32 + threadIdx.x;
   float acc = 0.f;
@@ -695,7 +700,7 @@ rt_status rt_gemm_bias_act(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const f
   if (done != RT_ERR_UNIMPLEMENTED) return done;
   rt_status st = rt_gemm(ctx, 0, 0, m, n, k, a, lda, b, ldb, c, ldc, 0);
   if (st != RT_OK || (!bias && act == RT_ACT_NONE)) return st;
-  bias_act_kernel<<<rt_grid_for(ctx, m * n, 256), 256, 0, ctx->stream>>>(c, bias, m, (int)n, ldc, act);
+  rt_launch(ctx, bias_act_kernel, rt_grid_for(ctx, m * n, 256), 256, 0, c, bias, m, (int)n, ldc, act);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }
@@ -760,7 +765,7 @@ rt_status rt_sum_rows_accumulate_list(rt_ctx* ctx, int count, const float* const
     l.count = count - i < kRowListTerms ? count - i : kRowListTerms;
     for (int j = 0; j < l.count; ++j) l.x[j] = x[i + j];
     l.d_rows.init((uint32_t)rows);
-    col_sum_list_kernel<<<(unsigned)((cols + 31) / 32), dim3(32, 32), 0, ctx->stream>>>(l, rows * l.count, cols, out);
+    rt_launch(ctx, col_sum_list_kernel, (unsigned)((cols + 31) / 32), dim3(32, 32), 0, l, rows * l.count, cols, out);
     RT_LAUNCHED(ctx);
   }
   return RT_OK;

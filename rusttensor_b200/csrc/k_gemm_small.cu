@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kThreads, 2) small_gemm_kernel(const SmallGemm
   using S = Shape<TA, TB>;
   cg::cluster_group cluster = cg::this_cluster();
   const int splits = cluster.num_blocks(), rank = cluster.block_rank();
+  RT_PDL_ENTRY();
   SmallGemm p = args;
   int row_tile = blockIdx.y;
   if constexpr (sizeof(List) > sizeof(NoList)) {
@@ -252,12 +253,14 @@ rt_status launch_small(rt_ctx* ctx, const SmallGemm& p, int splits, const List& 
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = S::bytes;
   cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)splits;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   RT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, p, list));
   RT_LAUNCHED(ctx);
   return RT_OK;

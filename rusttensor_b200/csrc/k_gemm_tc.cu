@@ -942,6 +942,7 @@ tc_gemm_ts_kernel(const PlainMat la, const PlainMat lb, const TsOut out, int K, 
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  if (!rt_pdl_wait()) return;
   if (warp < kProducerWarps)
     for (int i = 0; i < kTsRaw / 2; ++i) fetch(group + 2 * i);
 
@@ -957,6 +958,7 @@ tc_gemm_ts_kernel(const PlainMat la, const PlainMat lb, const TsOut out, int K, 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  rt_pdl_trigger();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tmem_a = tmem_base + kTsAccCols;  // A stages behind the accumulators
 
@@ -1173,12 +1175,14 @@ rt_status launch_ts(rt_ctx* ctx, const PlainMat& la, const PlainMat& lb, const T
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = TsSmem::total;
   cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)splits;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   RT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, la, lb, out, K, kps, ctx->device_status));
   RT_LAUNCHED(ctx);
   return RT_OK;

@@ -428,6 +428,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ src
 // pointers and rows on both sides; bound by memory bandwidth (103 MB turned: see the figures at channels_last).
 __global__ void __launch_bounds__(256) transpose4_kernel(const float* __restrict__ src, float* __restrict__ dst, int rows, int cols, int64_t lds, int64_t ldd,
                                                          int64_t batch_src, int64_t batch_dst) {
+  RT_PDL_ENTRY();
   __shared__ float tile[32][129];
   const float* s = src + (int64_t)blockIdx.z * batch_src;
   float* d = dst + (int64_t)blockIdx.z * batch_dst;
@@ -455,6 +456,7 @@ __global__ void __launch_bounds__(256) transpose4_kernel(const float* __restrict
 // behind the last channel.
 __global__ void __launch_bounds__(256) pack_taps_kernel(const float* __restrict__ w, float* __restrict__ dst, int N, int C, int c_blocks, int kw, int taps,
                                                         int64_t sn, int64_t sc, int64_t sky, int64_t skx, int64_t off0) {
+  RT_PDL_ENTRY();
   const int64_t cols = (int64_t)taps * c_blocks * BK;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N * cols; i += (int64_t)gridDim.x * blockDim.x) {
     const int n = (int)(i / cols), k = (int)(i % cols), tap = k / (c_blocks * BK), c = k % (c_blocks * BK);
@@ -506,7 +508,7 @@ inline rt_status pack(rt_ctx* ctx, const float* src, float* dst, int64_t rows, i
                       int64_t batch_src, int64_t batch_dst) {
   const dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32), (unsigned)batch);
   if (transpose && rt_aligned16(src) && rt_aligned16(dst) && ((rows | cols | lds | ldd | batch_src | batch_dst) & 3) == 0)
-    transpose4_kernel<<<dim3((unsigned)((cols + 127) / 128), grid.y, grid.z), 256, 0, ctx->stream>>>(src, dst, (int)rows, (int)cols, lds, ldd, batch_src,
+    rt_launch(ctx, transpose4_kernel, dim3((unsigned)((cols + 127) / 128), grid.y, grid.z), 256, 0, src, dst, (int)rows, (int)cols, lds, ldd, batch_src,
                                                                                                     batch_dst);
   else if (transpose) pack_kernel<true><<<grid, 256, 0, ctx->stream>>>(src, dst, (int)rows, (int)cols, lds, ldd, batch_src, batch_dst);
   else pack_kernel<false><<<grid, 256, 0, ctx->stream>>>(src, dst, (int)rows, (int)cols, lds, ldd, batch_src, batch_dst);
@@ -644,7 +646,7 @@ inline rt_status pixel_product(rt_ctx* ctx, const PixelProduct& q, const float* 
   RtScratch wb(ctx);
   rt_status st = wb.alloc(sizeof(float) * (size_t)(2 * q.N * cols));
   if (st != RT_OK) return st;
-  pack_taps_kernel<<<rt_grid_for(ctx, q.N * cols, 256), 256, 0, ctx->stream>>>(q.w, wb.as<float>(), q.N, q.C, p.c_blocks, q.kw, q.kh * q.kw, q.sn, q.sc, q.sky,
+  rt_launch(ctx, pack_taps_kernel, rt_grid_for(ctx, q.N * cols, 256), 256, 0, q.w, wb.as<float>(), q.N, q.C, p.c_blocks, q.kw, q.kh * q.kw, q.sn, q.sc, q.sky,
                                                                                q.skx, q.off0);
   RT_LAUNCHED(ctx);
   if (!map_matrix(&mb, wb.as<float>(), cols, 2 * q.N, cols, BK, bn_cols, true)) return RT_ERR_UNIMPLEMENTED;

@@ -112,6 +112,7 @@ __device__ __forceinline__ void update(float& p, float g, float& s1, float& s2, 
 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) optimizer_kernel(const __grid_constant__ OptArgs a) {
+  RT_PDL_ENTRY();
   float bc1, bc2;
   if (!optimizer_prologue<KIND>(a, bc1, bc2)) return;
   // locate the tensor this block works on
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(kThreads) optimizer_peer_kernel(const __grid_c
 
 // Starts a step: the exchange step number and the optimizer step count advance on the device.
 __global__ void dp_step_begin_kernel(int* ctrl) {
+  RT_PDL_ENTRY();
   if (threadIdx.x == 0) {
     ctrl[kCtrlStep] += 1;
     ctrl[kCtrlT] += 1;
@@ -396,10 +398,10 @@ rt_status launch_multi(rt_ctx* ctx, int kind, int n_tensors, float* const* param
       a.bc2 = 1.0f - powi_f32(beta2, (int)t);
     }
     switch (kind) {
-      case 0: optimizer_kernel<0><<<blocks, kThreads, 0, ctx->stream>>>(a); break;
-      case 1: optimizer_kernel<1><<<blocks, kThreads, 0, ctx->stream>>>(a); break;
-      case 2: optimizer_kernel<2><<<blocks, kThreads, 0, ctx->stream>>>(a); break;
-      default: optimizer_kernel<3><<<blocks, kThreads, 0, ctx->stream>>>(a); break;
+      case 0: rt_launch(ctx, optimizer_kernel<0>, blocks, kThreads, 0, a); break;
+      case 1: rt_launch(ctx, optimizer_kernel<1>, blocks, kThreads, 0, a); break;
+      case 2: rt_launch(ctx, optimizer_kernel<2>, blocks, kThreads, 0, a); break;
+      default: rt_launch(ctx, optimizer_kernel<3>, blocks, kThreads, 0, a); break;
     }
     RT_LAUNCHED(ctx);
   }
@@ -525,7 +527,7 @@ rt_status rt_pack_flat_signal(rt_ctx* ctx, int n_tensors, const float* const* sr
 rt_status rt_dp_step_begin(rt_ctx* ctx, int* step_state) {
   RT_CHECK_CTX(ctx);
   RT_CHECK_PTR(ctx, step_state);
-  dp_step_begin_kernel<<<1, 32, 0, ctx->stream>>>(step_state);
+  rt_launch(ctx, dp_step_begin_kernel, 1, 32, 0, step_state);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(kThreads) pool_fwd_general(const float* __rest
 template <bool RELU>
 __global__ void __launch_bounds__(kThreads) pool_fwd_2x2(const float* __restrict__ x, float* __restrict__ y,
                                                           float* __restrict__ idx, int64_t total, int w, int ho, int wo) {
+  RT_PDL_ENTRY();
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += stride) {
     int xo = (int)(o % wo);
@@ -81,6 +82,7 @@ template <bool RELU>  // RELU: dx is also masked with x > 0 (backward of the fus
 __global__ void __launch_bounds__(kThreads) pool_bwd_2x2(const float* __restrict__ g, const float* __restrict__ idx,
                                                           const float* __restrict__ x, float* __restrict__ dx, int64_t total,
                                                           int w, int ho, int wo) {
+  RT_PDL_ENTRY();
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += stride) {
     int xo = (int)(o % wo);
@@ -107,6 +109,7 @@ template <bool RELU>
 __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_pair(const float* __restrict__ g, const float* __restrict__ idx,
                                                                const float* __restrict__ x, float* __restrict__ dx,
                                                                int64_t total2, int w, int wo2) {
+  RT_PDL_ENTRY();
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total2; o += stride) {
     const int xo = (int)(o % wo2);
@@ -134,6 +137,7 @@ __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_pair(const float* __res
 __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_from_output(const float* __restrict__ y, const float* __restrict__ g,
                                                                       const float* __restrict__ idx, float* __restrict__ dx,
                                                                       int64_t total2, int w, int wo2) {
+  RT_PDL_ENTRY();
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total2; o += stride) {
     const int xo = (int)(o % wo2);
@@ -154,6 +158,7 @@ __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_from_output(const float
 __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_from_output_scalar(const float* __restrict__ y, const float* __restrict__ g,
                                                                              const float* __restrict__ idx, float* __restrict__ dx,
                                                                              int64_t total, int w, int wo) {
+  RT_PDL_ENTRY();
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += stride) {
     const int xo = (int)(o % wo);
@@ -246,8 +251,8 @@ static rt_status pool_forward(rt_ctx* ctx, bool relu, const float* x, int64_t n,
   bool fast = kh == 2 && kw == 2 && sh == 2 && sw == 2 && ph == 0 && pw == 0 && (h % 2 == 0) && (w % 2 == 0) &&
               (reinterpret_cast<uintptr_t>(x) % 8 == 0);
   if (fast) {
-    if (relu) pool_fwd_2x2<true><<<grid, kThreads, 0, ctx->stream>>>(x, y, idx, total, (int)w, (int)ho, (int)wo);
-    else pool_fwd_2x2<false><<<grid, kThreads, 0, ctx->stream>>>(x, y, idx, total, (int)w, (int)ho, (int)wo);
+    if (relu) rt_launch(ctx, pool_fwd_2x2<true>, grid, kThreads, 0, x, y, idx, total, (int)w, (int)ho, (int)wo);
+    else rt_launch(ctx, pool_fwd_2x2<false>, grid, kThreads, 0, x, y, idx, total, (int)w, (int)ho, (int)wo);
   } else {
     if (relu) pool_fwd_general<true><<<grid, kThreads, 0, ctx->stream>>>(x, y, idx, total, (int)h, (int)w, (int)ho, (int)wo, kh, kw, sh, sw, ph, pw);
     else pool_fwd_general<false><<<grid, kThreads, 0, ctx->stream>>>(x, y, idx, total, (int)h, (int)w, (int)ho, (int)wo, kh, kw, sh, sw, ph, pw);
@@ -287,18 +292,18 @@ static rt_status pool_backward(rt_ctx* ctx, const float* x, const float* g, cons
     if (pair) {  // w % 4 == 0 makes wo even: two windows per thread
       // one pair per thread up to 64 waves of blocks (a thread per pair measured 8.3 us on [256,32,28,28], eight waves 8.7)
       const int grid = rt_grid_for(ctx, total / 2, kThreads, 64);
-      if (x) pool_bwd_2x2_pair<true><<<grid, kThreads, 0, ctx->stream>>>(g, idx, x, dx, total / 2, (int)w, (int)(wo / 2));
-      else pool_bwd_2x2_pair<false><<<grid, kThreads, 0, ctx->stream>>>(g, idx, nullptr, dx, total / 2, (int)w, (int)(wo / 2));
+      if (x) rt_launch(ctx, pool_bwd_2x2_pair<true>, grid, kThreads, 0, g, idx, x, dx, total / 2, (int)w, (int)(wo / 2));
+      else rt_launch(ctx, pool_bwd_2x2_pair<false>, grid, kThreads, 0, g, idx, nullptr, dx, total / 2, (int)w, (int)(wo / 2));
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
     const int grid2 = rt_grid_for(ctx, total, kThreads * 2);
     if (x && reinterpret_cast<uintptr_t>(x) % 8 == 0) {
-      pool_bwd_2x2<true><<<grid2, kThreads, 0, ctx->stream>>>(g, idx, x, dx, total, (int)w, (int)ho, (int)wo);
+      rt_launch(ctx, pool_bwd_2x2<true>, grid2, kThreads, 0, g, idx, x, dx, total, (int)w, (int)ho, (int)wo);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
-    pool_bwd_2x2<false><<<grid2, kThreads, 0, ctx->stream>>>(g, idx, nullptr, dx, total, (int)w, (int)ho, (int)wo);
+    rt_launch(ctx, pool_bwd_2x2<false>, grid2, kThreads, 0, g, idx, nullptr, dx, total, (int)w, (int)ho, (int)wo);
     RT_LAUNCHED(ctx);
     return x ? rt_unary_backward(ctx, RT_RELU, x, dx, dx, in_total, 0.f, 0.f) : RT_OK;
   }
@@ -336,9 +341,9 @@ rt_status rt_relu_max_pool2x2_backward_from_output(rt_ctx* ctx, const float* y, 
   const bool pair = w % 4 == 0 && rt_aligned16(dx) && (reinterpret_cast<uintptr_t>(g) % 8 == 0) && (reinterpret_cast<uintptr_t>(idx) % 8 == 0) &&
                     (reinterpret_cast<uintptr_t>(y) % 8 == 0);
   if (pair)
-    pool_bwd_2x2_from_output<<<rt_grid_for(ctx, total / 2, kThreads, 64), kThreads, 0, ctx->stream>>>(y, g, idx, dx, total / 2, (int)w, (int)(w / 4));
+    rt_launch(ctx, pool_bwd_2x2_from_output, rt_grid_for(ctx, total / 2, kThreads, 64), kThreads, 0, y, g, idx, dx, total / 2, (int)w, (int)(w / 4));
   else
-    pool_bwd_2x2_from_output_scalar<<<rt_grid_for(ctx, total, kThreads, 16), kThreads, 0, ctx->stream>>>(y, g, idx, dx, total, (int)w, (int)(w / 2));
+    rt_launch(ctx, pool_bwd_2x2_from_output_scalar, rt_grid_for(ctx, total, kThreads, 16), kThreads, 0, y, g, idx, dx, total, (int)w, (int)(w / 2));
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

@@ -67,6 +67,7 @@ __device__ __forceinline__ float block_reduce(float v, float* smem) {  // smem: 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) row_reduce_warp(const float* __restrict__ x, float* __restrict__ out,
                                                              int64_t rows, int64_t len, float scale) {
+  RT_PDL_ENTRY();
   int lane = threadIdx.x & 31;
   int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(kThreads) row_reduce_warp(const float* __restr
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) row_reduce_thread(const float* __restrict__ x, float* __restrict__ out,
                                                                int64_t rows, int len, float scale) {
+  RT_PDL_ENTRY();
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += stride) {
     const float* p = x + r * len;
@@ -113,6 +115,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kThreads) row_reduce_block(const float* __restrict__ x, float* __restrict__ out,
                                                               int64_t rows, int64_t len, int64_t chunks,
                                                               int64_t chunk_len, float scale) {
+  RT_PDL_ENTRY();
   __shared__ float smem[kThreads / 32];
   for (int64_t job = blockIdx.x; job < rows * chunks; job += gridDim.x) {
     int64_t r = job / chunks, c = job % chunks;
@@ -145,6 +148,7 @@ __global__ void __launch_bounds__(kThreads) row_reduce_block(const float* __rest
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) row_reduce_warp_vec(const float* __restrict__ x, float* __restrict__ out,
                                                                  int64_t rows, int len, float scale) {
+  RT_PDL_ENTRY();
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -195,6 +199,7 @@ __device__ __forceinline__ void load_row_vec(const float* __restrict__ p, int n4
 template <int KIND, int VPT>
 __global__ void __launch_bounds__(kThreads) row_reduce_regs(const float* __restrict__ x, float* __restrict__ out,
                                                              int64_t rows, int len, float scale) {
+  RT_PDL_ENTRY();
   __shared__ float smem[kThreads / 32];
   const int n4 = len >> 2;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -214,6 +219,7 @@ __global__ void __launch_bounds__(kThreads) row_reduce_regs(const float* __restr
 template <int KIND, bool VEC, int TX = 32>
 __global__ void __launch_bounds__(256) col_reduce(const float* __restrict__ x, float* __restrict__ out, int64_t len,
                                                    int64_t inner, int64_t splits, int64_t rows_per_split, float scale) {
+  RT_PDL_ENTRY();
   constexpr int W = VEC ? 4 : 1;
   constexpr int TY = 256 / TX;  // row lanes; a block reads TX*W contiguous columns of TY rows at a time
   __shared__ float red[TY][TX * W + 1];
@@ -278,6 +284,7 @@ template <int KIND, int TX>
 __global__ void __launch_bounds__(256) col_reduce_single(const float* __restrict__ x, float* __restrict__ part,
                                                           float* __restrict__ out, int64_t len, int64_t inner, int splits,
                                                           int64_t rows_per_split, float scale, unsigned* __restrict__ counters) {
+  RT_PDL_ENTRY();
   constexpr int TY = 256 / TX, U = 8;
   __shared__ __align__(16) float red[TY][TX * 4 + 4];
   __shared__ bool last;
@@ -343,6 +350,7 @@ __global__ void __launch_bounds__(256) col_reduce_single(const float* __restrict
 template <int KIND>
 __global__ void __launch_bounds__(1024) col_reduce_short(const float* __restrict__ x, float* __restrict__ out, int64_t len, int64_t inner,
                                                           float scale) {
+  RT_PDL_ENTRY();
   __shared__ float part[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * 32 + tx, o = blockIdx.y;
@@ -380,28 +388,28 @@ rt_status reduce_float(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, 
   if (inner == 1) {
     int64_t rows = outer;
     if (len <= 16) {
-      row_reduce_thread<KIND><<<rt_grid_for(ctx, rows, kThreads), kThreads, 0, ctx->stream>>>(x, out, rows, (int)len, scale);
+      rt_launch(ctx, row_reduce_thread<KIND>, rt_grid_for(ctx, rows, kThreads), kThreads, 0, x, out, rows, (int)len, scale);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
     if (len <= 1024) {
       int grid = rt_grid_for(ctx, rows, kThreads / 32);
-      row_reduce_warp<KIND><<<grid, kThreads, 0, ctx->stream>>>(x, out, rows, len, scale);
+      rt_launch(ctx, row_reduce_warp<KIND>, grid, kThreads, 0, x, out, rows, len, scale);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
     if (len > 8192 && len <= 65536 && (len & 3) == 0 && rt_aligned16(x) && rows >= (int64_t)ctx->sm_count * 16) {
       // plenty of very long rows: a warp per row keeps the most loads in flight (up to 8192 elements the block-per-row
       // kernel below, which holds the row in registers, is faster: 12.6 against 14.5 us on 4096 x 4096)
-      row_reduce_warp_vec<KIND><<<rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, ctx->stream>>>(x, out, rows, (int)len, scale);
+      rt_launch(ctx, row_reduce_warp_vec<KIND>, rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, x, out, rows, (int)len, scale);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
     if (len <= 8192 && (len & 3) == 0 && rt_aligned16(x) && rows >= 64) {
       const int grid = (int)(rows < (1 << 20) ? rows : (1 << 20));  // a block per row: rows in different phases overlap
-      if (len <= 2048) row_reduce_regs<KIND, 2><<<grid, kThreads, 0, ctx->stream>>>(x, out, rows, (int)len, scale);
-      else if (len <= 4096) row_reduce_regs<KIND, 4><<<grid, kThreads, 0, ctx->stream>>>(x, out, rows, (int)len, scale);
-      else row_reduce_regs<KIND, 8><<<grid, kThreads, 0, ctx->stream>>>(x, out, rows, (int)len, scale);
+      if (len <= 2048) rt_launch(ctx, row_reduce_regs<KIND, 2>, grid, kThreads, 0, x, out, rows, (int)len, scale);
+      else if (len <= 4096) rt_launch(ctx, row_reduce_regs<KIND, 4>, grid, kThreads, 0, x, out, rows, (int)len, scale);
+      else rt_launch(ctx, row_reduce_regs<KIND, 8>, grid, kThreads, 0, x, out, rows, (int)len, scale);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
@@ -417,14 +425,14 @@ rt_status reduce_float(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, 
     chunks = (len + chunk_len - 1) / chunk_len;
     int grid = (int)((rows * chunks < target_blocks * 2) ? rows * chunks : target_blocks * 2);
     if (chunks == 1) {
-      row_reduce_block<KIND><<<grid, kThreads, 0, ctx->stream>>>(x, out, rows, len, 1, chunk_len, scale);
+      rt_launch(ctx, row_reduce_block<KIND>, grid, kThreads, 0, x, out, rows, len, 1, chunk_len, scale);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
     RtScratch part(ctx);
     rt_status st = part.alloc(sizeof(float) * rows * chunks);
     if (st != RT_OK) return st;
-    row_reduce_block<KIND><<<grid, kThreads, 0, ctx->stream>>>(x, part.as<float>(), rows, len, chunks, chunk_len, 1.f);
+    rt_launch(ctx, row_reduce_block<KIND>, grid, kThreads, 0, x, part.as<float>(), rows, len, chunks, chunk_len, 1.f);
     RT_LAUNCHED(ctx);
     return reduce_float<KIND>(ctx, part.as<float>(), rows, chunks, 1, out, scale);
   }
@@ -457,7 +465,7 @@ rt_status reduce_float(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, 
   }
   if (short_reduction && len >= 16 && outer * inner <= 4096 && outer <= 65535) {
     // few rows, narrow output: one latency-bound launch with all loads in flight (6 us -> 2.5 us for a [256, 10] bias gradient)
-    col_reduce_short<KIND><<<dim3((unsigned)((inner + 31) / 32), (unsigned)outer), 1024, 0, ctx->stream>>>(x, out, len, inner, scale);
+    rt_launch(ctx, col_reduce_short<KIND>, dim3((unsigned)((inner + 31) / 32), (unsigned)outer), 1024, 0, x, out, len, inner, scale);
     RT_LAUNCHED(ctx);
     return RT_OK;
   }
@@ -483,9 +491,9 @@ rt_status reduce_float(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, 
       unsigned* counters = ctx->reduce_counters + (ctx->on_side ? kReduceCounterSlots : 0);
       const dim3 grid1((unsigned)tiles1, (unsigned)sp, (unsigned)outer);
       if (tile_cols1 == 64)
-        col_reduce_single<KIND, 16><<<grid1, 256, 0, ctx->stream>>>(x, partial.as<float>(), out, len, inner, (int)sp, rows_per, scale, counters);
+        rt_launch(ctx, col_reduce_single<KIND, 16>, grid1, 256, 0, x, partial.as<float>(), out, len, inner, (int)sp, rows_per, scale, counters);
       else
-        col_reduce_single<KIND, 32><<<grid1, 256, 0, ctx->stream>>>(x, partial.as<float>(), out, len, inner, (int)sp, rows_per, scale, counters);
+        rt_launch(ctx, col_reduce_single<KIND, 32>, grid1, 256, 0, x, partial.as<float>(), out, len, inner, (int)sp, rows_per, scale, counters);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
@@ -501,9 +509,9 @@ rt_status reduce_float(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, 
     dst = part.as<float>();
   }
   float sc = splits > 1 ? 1.f : scale;
-  if (wide) col_reduce<KIND, true, 128><<<grid, dim3(128, 2), 0, ctx->stream>>>(x, dst, len, inner, splits, rps, sc);
-  else if (vec) col_reduce<KIND, true><<<grid, block, 0, ctx->stream>>>(x, dst, len, inner, splits, rps, sc);
-  else col_reduce<KIND, false><<<grid, block, 0, ctx->stream>>>(x, dst, len, inner, splits, rps, sc);
+  if (wide) rt_launch(ctx, col_reduce<KIND, true, 128>, grid, dim3(128, 2), 0, x, dst, len, inner, splits, rps, sc);
+  else if (vec) rt_launch(ctx, col_reduce<KIND, true>, grid, block, 0, x, dst, len, inner, splits, rps, sc);
+  else rt_launch(ctx, col_reduce<KIND, false>, grid, block, 0, x, dst, len, inner, splits, rps, sc);
   RT_LAUNCHED(ctx);
   if (splits > 1) return reduce_float<KIND>(ctx, dst, outer, splits, inner, out, scale);
   return RT_OK;
@@ -529,6 +537,7 @@ __device__ __forceinline__ float group_reduce_sum(float v, float* smem) {
 template <int MODE, int G>
 __global__ void __launch_bounds__(kThreads) row_softmax_kernel(const float* __restrict__ x, const float* __restrict__ g,
                                                                 float* __restrict__ out, int64_t rows, int64_t len) {
+  RT_PDL_ENTRY();
   __shared__ float smem[kThreads / 32];
   int lane = threadIdx.x % G;
   int64_t group = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -616,6 +625,7 @@ __global__ void __launch_bounds__(kThreads) slice_softmax_kernel(const float* __
 template <int MODE, int VPT>
 __global__ void __launch_bounds__(kThreads) row_softmax_regs(const float* __restrict__ x, const float* __restrict__ g,
                                                               float* __restrict__ out, int64_t rows, int len) {
+  RT_PDL_ENTRY();
   __shared__ float smem[kThreads / 32];
   const int n4 = len >> 2;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -674,16 +684,16 @@ rt_status launch_softmax_family(rt_ctx* ctx, const float* x, const float* g, flo
   if (inner == 1) {
     if (len <= 1024) {
       int grid = rt_grid_for(ctx, outer, kThreads / 32);
-      row_softmax_kernel<MODE, 32><<<grid, kThreads, 0, ctx->stream>>>(x, g, out, outer, len);
+      rt_launch(ctx, row_softmax_kernel<MODE, 32>, grid, kThreads, 0, x, g, out, outer, len);
     } else if (len <= 8192 && (len & 3) == 0 && rt_aligned16(x) && (MODE == ROW_LSE_FWD || rt_aligned16(out)) &&
                (MODE != ROW_LSM_BWD || rt_aligned16(g))) {
       const int grid = (int)(outer < (1 << 20) ? outer : (1 << 20));  // a block per row: rows in different phases overlap
-      if (len <= 2048) row_softmax_regs<MODE, 2><<<grid, kThreads, 0, ctx->stream>>>(x, g, out, outer, (int)len);
-      else if (len <= 4096) row_softmax_regs<MODE, 4><<<grid, kThreads, 0, ctx->stream>>>(x, g, out, outer, (int)len);
-      else row_softmax_regs<MODE, 8><<<grid, kThreads, 0, ctx->stream>>>(x, g, out, outer, (int)len);
+      if (len <= 2048) rt_launch(ctx, row_softmax_regs<MODE, 2>, grid, kThreads, 0, x, g, out, outer, (int)len);
+      else if (len <= 4096) rt_launch(ctx, row_softmax_regs<MODE, 4>, grid, kThreads, 0, x, g, out, outer, (int)len);
+      else rt_launch(ctx, row_softmax_regs<MODE, 8>, grid, kThreads, 0, x, g, out, outer, (int)len);
     } else {
       int grid = rt_grid_for(ctx, outer, 1);
-      row_softmax_kernel<MODE, kThreads><<<grid, kThreads, 0, ctx->stream>>>(x, g, out, outer, len);
+      rt_launch(ctx, row_softmax_kernel<MODE, kThreads>, grid, kThreads, 0, x, g, out, outer, len);
     }
   } else {
     int grid = rt_grid_for(ctx, outer * inner, kThreads);
@@ -729,6 +739,7 @@ __global__ void __launch_bounds__(kThreads) expand_axis_kernel(const float* __re
 // dx[:] = g[0] (/ scale): gradient of a global sum / mean
 __global__ void __launch_bounds__(kThreads) fill_from_scalar_kernel(const float* __restrict__ g, float* __restrict__ dx,
                                                                      int64_t n, float scale, bool divide) {
+  RT_PDL_ENTRY();
   float v = divide ? g[0] / scale : g[0];
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -867,12 +878,12 @@ rt_status rt_reduce_backward(rt_ctx* ctx, int kind, const float* x, const float*
   int grid = rt_grid_for(ctx, n, kThreads * 2);
   switch (kind) {
     case RT_RED_SUM:
-      if (outer * inner == 1) fill_from_scalar_kernel<<<rt_grid_for(ctx, (n + 3) / 4, kThreads * 2), kThreads, 0, ctx->stream>>>(g, dx, n, 1.f, false);
+      if (outer * inner == 1) rt_launch(ctx, fill_from_scalar_kernel, rt_grid_for(ctx, (n + 3) / 4, kThreads * 2), kThreads, 0, g, dx, n, 1.f, false);
       else expand_axis_kernel<<<grid, kThreads, 0, ctx->stream>>>(g, dx, n, len, inner, 1.f, false);
       RT_LAUNCHED(ctx);
       return RT_OK;
     case RT_RED_MEAN:  // div_scalar(broadcast(g), len)  (src/ops/cpu_backward.rs:716,764)
-      if (outer * inner == 1) fill_from_scalar_kernel<<<rt_grid_for(ctx, (n + 3) / 4, kThreads * 2), kThreads, 0, ctx->stream>>>(g, dx, n, (float)len, true);
+      if (outer * inner == 1) rt_launch(ctx, fill_from_scalar_kernel, rt_grid_for(ctx, (n + 3) / 4, kThreads * 2), kThreads, 0, g, dx, n, (float)len, true);
       else expand_axis_kernel<<<grid, kThreads, 0, ctx->stream>>>(g, dx, n, len, inner, (float)len, true);
       RT_LAUNCHED(ctx);
       return RT_OK;
@@ -1004,12 +1015,12 @@ extern "C" rt_status rt_reduce_sum_static_scratch(rt_ctx* ctx, const float* x, i
   if (inner == 1) {
     const int64_t rows = outer;
     if (len <= 16) {
-      row_reduce_thread<RT_RED_SUM><<<rt_grid_for(ctx, rows, kThreads), kThreads, 0, ctx->stream>>>(x, out, rows, (int)len, 1.f);
+      rt_launch(ctx, row_reduce_thread<RT_RED_SUM>, rt_grid_for(ctx, rows, kThreads), kThreads, 0, x, out, rows, (int)len, 1.f);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
     if (len <= 1024) {
-      row_reduce_warp<RT_RED_SUM><<<rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, ctx->stream>>>(x, out, rows, len, 1.f);
+      rt_launch(ctx, row_reduce_warp<RT_RED_SUM>, rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, x, out, rows, len, 1.f);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
@@ -1027,7 +1038,7 @@ extern "C" rt_status rt_reduce_sum_static_scratch(rt_ctx* ctx, const float* x, i
     chunks = (len + chunk_len - 1) / chunk_len;
     const int grid = (int)((rows * chunks < target_blocks * 2) ? rows * chunks : target_blocks * 2);
     if (chunks == 1) {
-      row_reduce_block<RT_RED_SUM><<<grid, kThreads, 0, ctx->stream>>>(x, out, rows, len, 1, chunk_len, 1.f);
+      rt_launch(ctx, row_reduce_block<RT_RED_SUM>, grid, kThreads, 0, x, out, rows, len, 1, chunk_len, 1.f);
       RT_LAUNCHED(ctx);
       return RT_OK;
     }
@@ -1035,12 +1046,12 @@ extern "C" rt_status rt_reduce_sum_static_scratch(rt_ctx* ctx, const float* x, i
       RT_FAIL(ctx, RT_ERR_INVALID_OPERATION,
               "rt_reduce_sum_static_scratch: %lld partial sums needed, the fixed workspace holds %lld", (long long)(rows * chunks),
               (long long)kStaticScratchFloats);
-    row_reduce_block<RT_RED_SUM><<<grid, kThreads, 0, ctx->stream>>>(x, scratch, rows, len, chunks, chunk_len, 1.f);
+    rt_launch(ctx, row_reduce_block<RT_RED_SUM>, grid, kThreads, 0, x, scratch, rows, len, chunks, chunk_len, 1.f);
     RT_LAUNCHED(ctx);
     if (chunks <= 16)
-      row_reduce_thread<RT_RED_SUM><<<rt_grid_for(ctx, rows, kThreads), kThreads, 0, ctx->stream>>>(scratch, out, rows, (int)chunks, 1.f);
+      rt_launch(ctx, row_reduce_thread<RT_RED_SUM>, rt_grid_for(ctx, rows, kThreads), kThreads, 0, scratch, out, rows, (int)chunks, 1.f);
     else
-      row_reduce_warp<RT_RED_SUM><<<rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, ctx->stream>>>(scratch, out, rows, chunks, 1.f);
+      rt_launch(ctx, row_reduce_warp<RT_RED_SUM>, rt_grid_for(ctx, rows, kThreads / 32), kThreads, 0, scratch, out, rows, chunks, 1.f);
     RT_LAUNCHED(ctx);
     return RT_OK;
   }
@@ -1063,15 +1074,15 @@ extern "C" rt_status rt_reduce_sum_static_scratch(rt_ctx* ctx, const float* x, i
             (long long)(outer * splits * inner), (long long)kStaticScratchFloats);
   dim3 grid((unsigned)tiles, (unsigned)splits, (unsigned)outer), block(32, 8);
   float* dst = splits > 1 ? scratch : out;
-  if (vec) col_reduce<RT_RED_SUM, true><<<grid, block, 0, ctx->stream>>>(x, dst, len, inner, splits, rps, 1.f);
-  else col_reduce<RT_RED_SUM, false><<<grid, block, 0, ctx->stream>>>(x, dst, len, inner, splits, rps, 1.f);
+  if (vec) rt_launch(ctx, col_reduce<RT_RED_SUM, true>, grid, block, 0, x, dst, len, inner, splits, rps, 1.f);
+  else rt_launch(ctx, col_reduce<RT_RED_SUM, false>, grid, block, 0, x, dst, len, inner, splits, rps, 1.f);
   RT_LAUNCHED(ctx);
   if (splits > 1) {
     // second pass in one launch: the partial sums [outer, splits, inner] are 256-byte aligned, inner % 4 decides the width
     const bool vec2 = inner % 4 == 0;
     dim3 grid2((unsigned)((inner + (vec2 ? 128 : 32) - 1) / (vec2 ? 128 : 32)), 1, (unsigned)outer);
-    if (vec2) col_reduce<RT_RED_SUM, true><<<grid2, block, 0, ctx->stream>>>(scratch, out, splits, inner, 1, splits, 1.f);
-    else col_reduce<RT_RED_SUM, false><<<grid2, block, 0, ctx->stream>>>(scratch, out, splits, inner, 1, splits, 1.f);
+    if (vec2) rt_launch(ctx, col_reduce<RT_RED_SUM, true>, grid2, block, 0, scratch, out, splits, inner, 1, splits, 1.f);
+    else rt_launch(ctx, col_reduce<RT_RED_SUM, false>, grid2, block, 0, scratch, out, splits, inner, 1, splits, 1.f);
     RT_LAUNCHED(ctx);
   }
   return RT_OK;
@@ -1123,6 +1134,7 @@ __device__ __forceinline__ void sce_finish_loss(const SceArgs& a, float block_su
 
 constexpr int kSceRows = 128, kSceFew = 16;
 __global__ void __launch_bounds__(kSceRows) sce_rows_kernel(const SceArgs a) {
+  RT_PDL_ENTRY();
   __shared__ float smem[kSceRows / 32];
   const float scale = a.g ? -__ldg(a.g) / (float)a.rows : a.c;
   float acc = 0.f;
@@ -1187,6 +1199,7 @@ __device__ __forceinline__ void row_max_lse_warp(const float* x, int classes, in
 }
 
 __global__ void __launch_bounds__(kThreads) sce_warp_kernel(const SceArgs a) {
+  RT_PDL_ENTRY();
   constexpr int nw = kThreads / 32;
   __shared__ float smem[nw];
   const float scale = a.g ? -__ldg(a.g) / (float)a.rows : a.c;
@@ -1235,8 +1248,8 @@ rt_status sce_launch(rt_ctx* ctx, SceArgs a) {
     a.part = part.as<float>();
     a.ticket = ctx->reduce_counters + 2 * kReduceCounterSlots + (ctx->on_side ? kAuxCounterSlots : 0) + kAuxCounterSlots - 2;
   }
-  if (a.classes <= kSceFew) sce_rows_kernel<<<(unsigned)grid, kSceRows, 0, ctx->stream>>>(a);
-  else sce_warp_kernel<<<(unsigned)grid, kThreads, 0, ctx->stream>>>(a);
+  if (a.classes <= kSceFew) rt_launch(ctx, sce_rows_kernel, (unsigned)grid, kSceRows, 0, a);
+  else rt_launch(ctx, sce_warp_kernel, (unsigned)grid, kThreads, 0, a);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }
@@ -1325,6 +1338,7 @@ struct NllList {
 };
 // part[block] = sum over the block's rows of sum_k log_softmax * t; a warp per row
 __global__ void __launch_bounds__(kThreads) nll_list_kernel(const NllList l, float* __restrict__ part) {
+  RT_PDL_ENTRY();
   __shared__ float smem[kThreads / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float acc = 0.f;
@@ -1352,6 +1366,7 @@ struct Scalars {
 };
 __global__ void __launch_bounds__(32) nll_list_finish_kernel(const float* __restrict__ part, int n, const Scalars more, float* __restrict__ loss,
                                                              float scale, float divisor) {
+  RT_PDL_ENTRY();
   float v = 0.f;
   for (int i = threadIdx.x; i < n; i += 32) v += part[i];
   v = warp_sum_all(v);
@@ -1387,13 +1402,13 @@ extern "C" rt_status rt_softmax_nll_list(rt_ctx* ctx, int count, const float* co
       l.x[i] = logits[q * kNllTerms + i];
       l.t[i] = targets[q * kNllTerms + i];
     }
-    nll_list_kernel<<<grid, kThreads, 0, ctx->stream>>>(l, part.as<float>() + (size_t)q * grid);
+    rt_launch(ctx, nll_list_kernel, grid, kThreads, 0, l, part.as<float>() + (size_t)q * grid);
     RT_LAUNCHED(ctx);
   }
   Scalars s{};
   s.n = n_more;
   for (int i = 0; i < n_more; ++i) s.p[i] = more[i];
-  nll_list_finish_kernel<<<1, 32, 0, ctx->stream>>>(part.as<float>(), grid * lists, s, loss, scale, divisor);
+  rt_launch(ctx, nll_list_finish_kernel, 1, 32, 0, part.as<float>(), grid * lists, s, loss, scale, divisor);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

@@ -420,6 +420,7 @@ struct MultiCopyParams {
 };
 // blockIdx.y = which copy; 16-byte units when both ends are 16-byte aligned, single bytes for the rest
 __global__ void multi_copy_kernel(const MultiCopyParams p) {
+  RT_PDL_ENTRY();
   const int seg = blockIdx.y;
   const char* __restrict__ src = p.src[seg];
   char* __restrict__ dst = p.dst[seg];
@@ -466,7 +467,7 @@ rt_status rt_upload_submit_all(rt_ctx* ctx, rt_upload* const* ups, void* const* 
   }
   const size_t units = (most + 15) / 16;
   const unsigned blocks = (unsigned)std::min<size_t>((units + 255) / 256, (size_t)ctx->sm_count * 4);
-  multi_copy_kernel<<<dim3(blocks ? blocks : 1, (unsigned)n), 256, 0, ctx->stream>>>(p);
+  rt_launch(ctx, multi_copy_kernel, dim3(blocks ? blocks : 1, (unsigned)n), 256, 0, p);
   RT_LAUNCHED(ctx);
   for (int i = 0; i < n; ++i) {
     rt_upload* up = ups[i];
@@ -511,7 +512,7 @@ rt_status rt_upload_submit_parts(rt_ctx* ctx, rt_upload* up, int n, const int64_
     }
     const size_t units = (most + 15) / 16;
     const unsigned blocks = (unsigned)std::min<size_t>((units + 255) / 256, (size_t)ctx->sm_count * 4);
-    multi_copy_kernel<<<dim3(blocks ? blocks : 1, (unsigned)parts), 256, 0, ctx->stream>>>(p);
+    rt_launch(ctx, multi_copy_kernel, dim3(blocks ? blocks : 1, (unsigned)parts), 256, 0, p);
     RT_LAUNCHED(ctx);
   }
   RT_CUDA(ctx, cudaEventRecord(up->consumed[k], ctx->stream));
@@ -539,6 +540,7 @@ rt_status rt_upload_gather_rows(rt_ctx* ctx, rt_upload* up, int n_src, const flo
 }
 
 __global__ void publish_kernel(const float* __restrict__ src, float* __restrict__ host_dst, int n) {
+  RT_PDL_ENTRY();
   for (int i = threadIdx.x; i < n; i += blockDim.x) host_dst[i] = src[i];
   __threadfence_system();
 }
@@ -555,7 +557,7 @@ rt_status rt_publish_to_host(rt_ctx* ctx, float* pinned_dst, const float* src, i
     if (e != cudaSuccess) cudaGetLastError();
     RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_publish_to_host: the destination is not pinned host memory (use rt_host_alloc)");
   }
-  publish_kernel<<<1, n < 256 ? 32 : 256, 0, ctx->stream>>>(src, static_cast<float*>(attr.devicePointer), (int)n);
+  rt_launch(ctx, publish_kernel, 1, n < 256 ? 32 : 256, 0, src, static_cast<float*>(attr.devicePointer), (int)n);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

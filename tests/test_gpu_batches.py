@@ -1,4 +1,4 @@
-"""Inputs of a step: several parts of one upload, and rows of several matrices gathered by uploaded numbers."""
+"""Inputs of a step: several parts of one upload, rows of several matrices gathered by uploaded numbers, concatenation of many pieces."""
 import ctypes as C
 
 import numpy as np
@@ -60,3 +60,13 @@ def test_gather_rows_list(api, n_idx):
             w[-1] = 0
             np.testing.assert_array_equal(w, d.numpy())
     api.call("upload_destroy", up)
+
+
+@pytest.mark.parametrize("outer,lens", [(1, [5]), (1, [4] * 300), (7, [3, 0, 8, 129]), (3, [4, 2000, 16])])  # more pieces than a launch takes
+def test_concat_list(api, outer, lens):
+    r = np.random.default_rng(len(lens))
+    data = [r.random((outer, n), dtype=np.float32) for n in lens]
+    src, out = [api.to_device(d) if d.size else None for d in data], api.to_device(np.zeros((outer, sum(lens)), np.float32))
+    ptrs = (C.c_void_p * len(lens))(*[s.ptr.value if s else None for s in src])
+    api.call("concat_list", len(lens), ptrs, (C.c_int64 * len(lens))(*lens), C.c_int64(outer), out.ptr)
+    np.testing.assert_array_equal(out.numpy(), np.concatenate(data, 1))
