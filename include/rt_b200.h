@@ -387,6 +387,9 @@ rt_status rt_gemm_bias_act_list(rt_ctx* ctx, int count, const float* const* a, f
 rt_status rt_gemm_sum_products(rt_ctx* ctx, int count, const float* const* a, const float* const* g, int64_t m, int64_t k, int64_t n, float* c);
 /* out[c] += sum over i < count and rows r of x_i[rows, cols][r, c]: the same for a bias. */
 rt_status rt_sum_rows_accumulate_list(rt_ctx* ctx, int count, const float* const* x, int64_t rows, int64_t cols, float* out);
+/* outs[i][c] = sum over r of xs[i][r, c] for count row-major matrices of rows[i] x cols[i] (the gradients of several biases), one launch for
+ * up to 32 of them.  32 row lanes per column: meant for some thousand rows at most. */
+rt_status rt_column_sums_list(rt_ctx* ctx, int count, const float* const* xs, const int64_t* rows, const int64_t* cols, float* const* outs);
 /* da[M,K] = g * b^T, db[K,N] = a^T * g   (matmul_backward mod.rs:324); NULL skips one. */
 rt_status rt_matmul_backward(rt_ctx* ctx, const float* a, const float* b, const float* g, int64_t m, int64_t k,
                              int64_t n, float* da, float* db);
@@ -492,6 +495,11 @@ rt_status rt_optimizer_step_multi_device_t(rt_ctx* ctx, int kind, int n_tensors,
                                            float* const* state1, float* const* state2, const int64_t* sizes, float lr, float beta1,
                                            float beta2, float epsilon, float momentum, const int* step_state, float grad_scale,
                                            int clip, float clip_lo, float clip_hi);
+/* rt_dp_step_begin and then rt_optimizer_step_multi_device_t, in one launch: the step of one GPU, where nothing else asks for the count. */
+rt_status rt_optimizer_step_multi_next(rt_ctx* ctx, int kind, int n_tensors, float* const* params, const float* const* grads,
+                                       float* const* state1, float* const* state2, const int64_t* sizes, float lr, float beta1,
+                                       float beta2, float epsilon, float momentum, int* step_state, float grad_scale, int clip, float clip_lo,
+                                       float clip_hi);
 /* rt_pack_flat into flat0 or flat1, whichever the step number selects (buffer = step & 1). */
 rt_status rt_pack_flat_alternating(rt_ctx* ctx, int n_tensors, const float* const* srcs, const int64_t* sizes, float* flat0,
                                    float* flat1, const int* step_state, int clip, float clip_lo, float clip_hi);

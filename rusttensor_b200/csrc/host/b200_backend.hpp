@@ -552,6 +552,36 @@ struct B200Backend {
     check(rt_unbroadcast(ctx(), g.ptr(), gs.data(), (int)gs.size(), ts.data(), (int)ts.size(), out.ptr()));
     return out;
   }
+  // Those of `grads` that are unevaluated column sums of matrices of up to 2048 rows (more are better split over blocks), in one launch.
+  static void evaluate_column_sums(const std::vector<const Storage*>& grads) {
+    std::vector<std::shared_ptr<DeviceBuffer>> sums;
+    std::vector<const float*> xs;
+    std::vector<int64_t> rows, cols;
+    std::vector<float*> outs;
+    for (auto* g : grads) {
+      const lazy::Node* n = g->buf ? g->buf->node.get() : nullptr;
+      if (n && n->tag == lazy::Tag::SumRows && n->geo[0] < 0 && n->in[0].shape[0] <= 2048 && n->in[0].shape[1] == g->buf->numel) sums.push_back(g->buf);
+    }
+    if (sums.size() < 2) return;
+    for (auto& b : sums) {
+      const std::shared_ptr<DeviceBuffer> x = b->node->in[0].buf;
+      rows.push_back((int64_t)b->node->in[0].shape[0]);
+      cols.push_back((int64_t)b->node->in[0].shape[1]);
+      xs.push_back(x->data());
+      if (!b->node) return;  // evaluated on the way
+      outs.push_back(lazy::new_block(b->ctx, b->numel));
+    }
+    const rt_status st = rt_column_sums_list(ctx(), (int)sums.size(), xs.data(), rows.data(), cols.data(), outs.data());
+    for (size_t i = 0; i < sums.size(); ++i) {
+      if (st != RT_OK) {
+        rt_free(ctx(), outs[i]);
+        continue;
+      }
+      sums[i]->ptr = outs[i];
+      sums[i]->drop_node();
+    }
+    check(st);
+  }
   static Storage slice(const Storage& x, const std::vector<Range>& ranges) {
     if (ranges.size() != x.shape.size()) throw Error::invalid_op("Slice ranges do not match input dimensionality");
     Shape os(ranges.size());

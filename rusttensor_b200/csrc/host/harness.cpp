@@ -158,8 +158,11 @@ struct DpTrainer {
   // every replay); the recorded ops go, and with them the intermediate results that nobody has asked for.
   void settle(const Tensor& loss) {
     loss.data().ptr();
+    std::vector<const Storage*> grads;
     for (auto& p : tr->w.params)
-      if (p.grad()) p.grad()->ptr();
+      if (p.grad()) grads.push_back(&*p.grad());
+    B200Backend::evaluate_column_sums(grads);
+    for (auto* g : grads) g->ptr();
     for (auto& x : inputs)
       if (x.grad()) x.grad()->ptr();
     loss.detach_graph();
@@ -178,7 +181,7 @@ struct DpTrainer {
     if (update_in_stream()) {
       own_buffers();  // the launches below (and the graph, when capturing) keep these pointers
       stamp(0);
-      B200Backend::check(rt_dp_step_begin(cx, ctrl_ptr()));
+      if (world > 1 || fused) B200Backend::check(rt_dp_step_begin(cx, ctrl_ptr()));  // else part of the optimizer's launch
     }
     for (auto& p : w.params) p.zero_grad();
     for (auto& x : inputs) x.zero_grad();
@@ -350,7 +353,7 @@ struct DpTrainer {
     }
     if (!fused) {
       UpdatePointers u = update_pointers(nullptr);
-      B200Backend::check(rt_optimizer_step_multi_device_t(c, kind, (int)u.ps.size(), u.ps.data(), u.gs.data(), u.s1.data(), u.s2.data(),
+      B200Backend::check(rt_optimizer_step_multi_next(c, kind, (int)u.ps.size(), u.ps.data(), u.gs.data(), u.s1.data(), u.s2.data(),
                                                           sizes.data(), w.lr, w.beta1, w.beta2, w.eps, w.momentum, ctrl_ptr(), 1.0f,
                                                           w.clip_grads ? 1 : 0, w.clip_lo, w.clip_hi));
       return;

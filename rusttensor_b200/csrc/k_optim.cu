@@ -45,6 +45,9 @@ struct OptArgs {
   // being complete for this step (rt_dp_wait_peers).
   const int* ctrl;
   int need_ready;
+  // Not null: this launch is the step's rt_dp_step_begin as well.  Every block counts with t + 1, the last one to finish writes it back.
+  int* advance;
+  unsigned* ticket;
 };
 
 // Words of the step state.
@@ -74,7 +77,7 @@ __device__ __forceinline__ bool optimizer_prologue(const OptArgs& a, float& bc1,
     int go = 1;
     if (a.ctrl) {
       if (KIND == 1) {
-        const int t = a.ctrl[kCtrlT];
+        const int t = a.ctrl[kCtrlT] + (a.advance ? 1 : 0);
         b1 = 1.0f - powi_f32(a.beta1, t);
         b2 = 1.0f - powi_f32(a.beta2, t);
       }
@@ -150,6 +153,12 @@ __global__ void __launch_bounds__(kThreads) optimizer_kernel(const __grid_consta
     p[i] = pv;
     if (KIND != 0) s1[i] = m;
     if (KIND == 1) s2[i] = v;
+  }
+  // the block has read the step count long before it draws its ticket
+  if (a.advance && threadIdx.x == 0 && atomicAdd(a.ticket, 1u) == gridDim.x - 1) {
+    *a.ticket = 0;
+    a.advance[kCtrlStep] += 1;
+    a.advance[kCtrlT] += 1;
   }
 }
 
@@ -364,7 +373,7 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(const __grid_constant__ 
 rt_status launch_multi(rt_ctx* ctx, int kind, int n_tensors, float* const* params, const float* const* grads,
                        float* const* s1, float* const* s2, const int64_t* sizes, float lr, float beta1, float beta2,
                        float eps, float momentum, int64_t t, float grad_scale, int clip, float clip_lo, float clip_hi,
-                       const int* ctrl = nullptr) {
+                       const int* ctrl = nullptr, int* advance = nullptr) {
   if (kind < 0 || kind > 3) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "optimizer kind %d", kind);
   if (kind == 1 && t <= 0 && !ctrl) RT_FAIL(ctx, RT_ERR_INTERNAL, "Adam step called with t=0");
   const int chunk = chunk_for(ctx, sizes, n_tensors);
@@ -393,6 +402,8 @@ rt_status launch_multi(rt_ctx* ctx, int kind, int n_tensors, float* const* param
     a.bc1 = a.bc2 = 1.f;
     a.ctrl = ctrl;
     a.need_ready = 0;
+    a.advance = advance;
+    a.ticket = advance ? ctx->reduce_counters + 2 * kReduceCounterSlots + (ctx->on_side ? kAuxCounterSlots : 0) + kAuxCounterSlots - 3 : nullptr;
     if (kind == 1 && !ctrl) {
       a.bc1 = 1.0f - powi_f32(beta1, (int)t);
       a.bc2 = 1.0f - powi_f32(beta2, (int)t);
@@ -546,6 +557,26 @@ rt_status rt_optimizer_step_multi_device_t(rt_ctx* ctx, int kind, int n_tensors,
                       clip, clip_lo, clip_hi, step_state);
 }
 
+rt_status rt_optimizer_step_multi_next(rt_ctx* ctx, int kind, int n_tensors, float* const* params, const float* const* grads,
+                                       float* const* state1, float* const* state2, const int64_t* sizes, float lr, float beta1,
+                                       float beta2, float epsilon, float momentum, int* step_state, float grad_scale, int clip, float clip_lo,
+                                       float clip_hi) {
+  RT_CHECK_CTX(ctx);
+  RT_CHECK_PTR(ctx, step_state);
+  int live = 0;
+  for (int i = 0; i < n_tensors; ++i) live += sizes && sizes[i] > 0;
+  if (n_tensors > kMaxTensors || live == 0 || !ctx->reduce_counters) {  // several launches, or none, share one step count
+    const rt_status st = rt_dp_step_begin(ctx, step_state);
+    if (st != RT_OK) return st;
+    return rt_optimizer_step_multi_device_t(ctx, kind, n_tensors, params, grads, state1, state2, sizes, lr, beta1, beta2, epsilon, momentum, step_state,
+                                            grad_scale, clip, clip_lo, clip_hi);
+  }
+  RT_CHECK_PTR(ctx, params);
+  RT_CHECK_PTR(ctx, grads);
+  return launch_multi(ctx, kind, n_tensors, params, grads, state1, state2, sizes, lr, beta1, beta2, epsilon, momentum, 0, grad_scale,
+                      clip, clip_lo, clip_hi, step_state, step_state);
+}
+
 rt_status rt_dp_signal_peers(rt_ctx* ctx, int* const* peer_flags, int rank, int world, const int* step_state) {
   RT_CHECK_CTX(ctx);
   RT_CHECK_PTR(ctx, peer_flags);
@@ -621,6 +652,7 @@ rt_status rt_optimizer_step_multi_peers(rt_ctx* ctx, int kind, int n_tensors, fl
   a.lr = lr; a.beta1 = beta1; a.beta2 = beta2; a.eps = epsilon; a.momentum = momentum;
   a.grad_scale = grad_scale; a.clip = 0; a.clip_lo = 0.f; a.clip_hi = 0.f;
   a.bc1 = a.bc2 = 1.f;
+  a.advance = nullptr;
   a.ctrl = step_state;
   a.need_ready = 1;
   switch (kind) {

@@ -377,6 +377,49 @@ __global__ void __launch_bounds__(1024) col_reduce_short(const float* __restrict
   }
 }
 
+// col_reduce_short for several matrices: the bias gradients of a step's layers, whose launches (2 us each, 3.5 - 4.7 at 1000 rows) cost
+// more than their sums.
+constexpr int kColumnSums = 32;
+struct ColumnSums {
+  const float* x[kColumnSums];
+  float* out[kColumnSums];
+  int64_t rows[kColumnSums], cols[kColumnSums];
+  int first[kColumnSums + 1];  // first block of each
+};
+__global__ void __launch_bounds__(1024) column_sums_kernel(const __grid_constant__ ColumnSums l) {
+  RT_PDL_ENTRY();
+  __shared__ float part[32][33];
+  int i = 0;
+  while ((int)blockIdx.x >= l.first[i + 1]) ++i;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t rows = l.rows[i], cols = l.cols[i], c = (int64_t)((int)blockIdx.x - l.first[i]) * 32 + tx;
+  float acc = 0.f;
+  if (c < cols) {
+    const float* base = l.x[i] + c;
+    int64_t r = ty;
+    for (; r + 15 * 32 < rows; r += 16 * 32) {
+      float v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = __ldg(base + (r + 32 * u) * cols);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) acc += v[u];
+    }
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = r + 32 * u < rows ? __ldg(base + (r + 32 * u) * cols) : 0.f;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) acc += v[u];
+  }
+  part[ty][tx] = acc;
+  __syncthreads();
+  if (ty == 0 && c < cols) {
+    float s = part[0][tx];
+#pragma unroll
+    for (int y = 1; y < 32; ++y) s += part[y][tx];
+    l.out[i][c] = s;
+  }
+}
+
 template <int KIND>
 rt_status reduce_float(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, int64_t inner, float* out, float scale) {
   if (outer * inner == 0) return RT_OK;
@@ -1255,6 +1298,32 @@ rt_status sce_launch(rt_ctx* ctx, SceArgs a) {
 }
 
 }  // namespace
+
+extern "C" rt_status rt_column_sums_list(rt_ctx* ctx, int count, const float* const* xs, const int64_t* rows, const int64_t* cols,
+                                         float* const* outs) {
+  RT_CHECK_CTX(ctx);
+  for (int q = 0; q < count; q += kColumnSums) {
+    ColumnSums l;
+    int n = 0, blocks = 0;
+    for (int i = q; i < count && i < q + kColumnSums; ++i) {
+      if (rows[i] < 0 || cols[i] < 0 || cols[i] > (1ll << 30)) RT_FAIL(ctx, RT_ERR_INVALID_INDEX, "rt_column_sums_list: bad extent");
+      if (cols[i] == 0) continue;
+      RT_CHECK_PTR(ctx, outs[i]);
+      if (rows[i] > 0) RT_CHECK_PTR(ctx, xs[i]);
+      l.x[n] = xs[i];
+      l.out[n] = outs[i];
+      l.rows[n] = rows[i];
+      l.cols[n] = cols[i];
+      l.first[n++] = blocks;
+      blocks += (int)((cols[i] + 31) / 32);
+    }
+    l.first[n] = blocks;
+    if (!n) continue;
+    rt_launch(ctx, column_sums_kernel, blocks, 1024, 0, l);
+    RT_LAUNCHED(ctx);
+  }
+  return RT_OK;
+}
 
 extern "C" rt_status rt_softmax_nll_scaled(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes,
                                            float scale, float divisor, float* loss) {

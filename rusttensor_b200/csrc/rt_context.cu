@@ -541,8 +541,7 @@ rt_status rt_upload_gather_rows(rt_ctx* ctx, rt_upload* up, int n_src, const flo
 
 __global__ void publish_kernel(const float* __restrict__ src, float* __restrict__ host_dst, int n) {
   RT_PDL_ENTRY();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) host_dst[i] = src[i];
-  __threadfence_system();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) host_dst[i] = src[i];  // visible to the host once the kernel is complete
 }
 
 rt_status rt_publish_to_host(rt_ctx* ctx, float* pinned_dst, const float* src, int64_t n) {

@@ -1,4 +1,5 @@
-"""Inputs of a step: several parts of one upload, rows of several matrices gathered by uploaded numbers, concatenation of many pieces."""
+"""Inputs of a step: several parts of one upload, rows of several matrices gathered by uploaded numbers, concatenation of many pieces,
+sums of several matrices' columns; and the optimizer's launch that advances the step count."""
 import ctypes as C
 
 import numpy as np
@@ -70,3 +71,39 @@ def test_concat_list(api, outer, lens):
     ptrs = (C.c_void_p * len(lens))(*[s.ptr.value if s else None for s in src])
     api.call("concat_list", len(lens), ptrs, (C.c_int64 * len(lens))(*lens), C.c_int64(outer), out.ptr)
     np.testing.assert_array_equal(out.numpy(), np.concatenate(data, 1))
+
+
+@pytest.mark.parametrize("shapes", [[(1, 1)], [(31, 33), (513, 32), (0, 5), (2048, 7)], [(64, 10 + i) for i in range(35)]])  # more than a launch takes
+def test_column_sums_list(api, shapes):
+    r = np.random.default_rng(len(shapes))
+    data = [r.random(s, dtype=np.float32) for s in shapes]
+    src, out = [api.to_device(d) if d.size else None for d in data], [api.to_device(np.ones(s[1], np.float32)) for s in shapes]
+    n = len(shapes)
+    api.call("column_sums_list", n, (C.c_void_p * n)(*[s.ptr.value if s else None for s in src]), (C.c_int64 * n)(*[s[0] for s in shapes]),
+             (C.c_int64 * n)(*[s[1] for s in shapes]), (C.c_void_p * n)(*[o.ptr.value for o in out]))
+    for d, o in zip(data, out):
+        np.testing.assert_allclose(o.numpy(), d.sum(0, dtype=np.float64), rtol=1e-6)
+
+
+@pytest.mark.parametrize("tensors", [1, 3, 200])  # one block; several; more tensors than a launch takes
+@pytest.mark.parametrize("kind", [1, 2])
+def test_optimizer_step_counts_itself(api, kind, tensors):
+    r = np.random.default_rng(tensors)
+    sizes = [int(n) for n in r.integers(1, 3000, tensors)]
+    new = lambda: [r.standard_normal(n).astype(np.float32) for n in sizes]  # noqa: E731
+    p, g, s1, s2 = new(), new(), new(), [x * x for x in new()]
+    f = C.c_float
+    got = []
+    for name in ("device_t", "next"):
+        dev = [[api.to_device(x) for x in xs] for xs in (p, g, s1, s2)]
+        lists = [(C.c_void_p * tensors)(*[d.ptr.value for d in ds]) for ds in dev]
+        state = api.to_device(np.array([0, 0, 7, 0], np.int32).view(np.float32))
+        for _ in range(3):
+            if name == "device_t":
+                api.call("dp_step_begin", state.ptr)
+            api.call("optimizer_step_multi_" + name, kind, tensors, *lists, (C.c_int64 * tensors)(*sizes), f(1e-2), f(0.9), f(0.999), f(1e-8), f(0.9),
+                     state.ptr, f(1.0), 0, f(0), f(0))
+        assert state.numpy().view(np.int32).tolist() == [3, 0, 10, 0]
+        got.append([d.numpy() for ds in dev for d in ds])
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
