@@ -1241,6 +1241,9 @@ __device__ __forceinline__ void row_max_lse_warp(const float* x, int classes, in
   lse = logf(warp_sum_all(ss));
 }
 
+// REGS values of the row a lane, in registers, for up to 32 * REGS classes; 0: the row is read again for each pass (4.0 us for the 64 x
+// 65 gradient of a recurrent head, most of it the latency of three passes and four sums over the warp).
+template <int REGS>
 __global__ void __launch_bounds__(kThreads) sce_warp_kernel(const SceArgs a) {
   RT_PDL_ENTRY();
   constexpr int nw = kThreads / 32;
@@ -1252,6 +1255,42 @@ __global__ void __launch_bounds__(kThreads) sce_warp_kernel(const SceArgs a) {
   for (int64_t r = (int64_t)blockIdx.x * nw + warp; r < a.rows; r += (int64_t)gridDim.x * nw) {
     const float* x = a.logits + r * a.classes;
     const float* t = a.targets + r * a.classes;
+    if constexpr (REGS > 0) {
+      float xv[REGS], tv[REGS], m = -INFINITY, s = 0.f, st = 0.f;
+#pragma unroll
+      for (int j = 0; j < REGS; ++j) {
+        const int k = lane + 32 * j;
+        xv[j] = k < a.classes ? __ldg(x + k) : -INFINITY;
+        tv[j] = k < a.classes ? __ldg(t + k) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < REGS; ++j) m = fmaxf(m, xv[j]);
+      m = warp_max_all(m);
+#pragma unroll
+      for (int j = 0; j < REGS; ++j) {
+        if (lane + 32 * j < a.classes) s += expf(xv[j] - m);
+        st += tv[j] * scale;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {  // both sums at once
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        st += __shfl_xor_sync(0xffffffffu, st, o);
+      }
+      const float lse = logf(s);
+      float e = 0.f;
+#pragma unroll
+      for (int j = 0; j < REGS; ++j) {
+        const int k = lane + 32 * j;
+        if (k < a.classes) {
+          const float ls = (xv[j] - m) - lse;
+          e += ls * tv[j];
+          if (a.dlogits) a.dlogits[r * a.classes + k] = tv[j] * scale - expf(ls) * st;
+          if (a.dtargets) a.dtargets[r * a.classes + k] = ls * scale;
+        }
+      }
+      if (a.loss) acc += warp_sum_all(e);
+      continue;
+    }
     float m, lse;
     row_max_lse_warp(x, a.classes, lane, m, lse);
     if (a.loss) {
@@ -1292,7 +1331,8 @@ rt_status sce_launch(rt_ctx* ctx, SceArgs a) {
     a.ticket = ctx->reduce_counters + 2 * kReduceCounterSlots + (ctx->on_side ? kAuxCounterSlots : 0) + kAuxCounterSlots - 2;
   }
   if (a.classes <= kSceFew) rt_launch(ctx, sce_rows_kernel, (unsigned)grid, kSceRows, 0, a);
-  else rt_launch(ctx, sce_warp_kernel, (unsigned)grid, kThreads, 0, a);
+  else if (a.classes <= 128) rt_launch(ctx, sce_warp_kernel<4>, (unsigned)grid, kThreads, 0, a);
+  else rt_launch(ctx, sce_warp_kernel<0>, (unsigned)grid, kThreads, 0, a);
   RT_LAUNCHED(ctx);
   return RT_OK;
 }

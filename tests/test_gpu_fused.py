@@ -99,7 +99,7 @@ def test_a_malformed_program_is_refused():
 
 
 # one block and several, a row more and less than a block of each form (128 rows; 8 rows), the change of form at 16 classes
-@pytest.mark.parametrize("rows,classes", [(1, 1), (127, 10), (129, 16), (9, 17), (1000, 16), (1003, 300)])
+@pytest.mark.parametrize("rows,classes", [(1, 1), (127, 10), (129, 16), (9, 17), (1000, 16), (64, 65), (9, 128), (1003, 129), (300, 300)])
 def test_classification_loss_with_gradient(rows, classes):
     import ctypes as C
 
