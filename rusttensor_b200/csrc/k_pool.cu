@@ -13,6 +13,7 @@
 // no zero-fill.  Overlapping windows are gathered per input element in the reference's order of additions.
 #include <cmath>
 
+#include "conv_geom.cuh"
 #include "rt_internal.cuh"
 
 namespace {
@@ -53,28 +54,47 @@ __global__ void __launch_bounds__(kThreads) pool_fwd_general(const float* __rest
 }
 
 // 2x2 window, stride 2, no padding, even H and W: one thread per output, two 8-byte loads.
-template <bool RELU>
+// PAIR: two windows a thread, 128-bit loads.  Bound by memory; positions are 32-bit with a precomputed division (two 64-bit divisions a
+// window took as long as its memory accesses: 1000 x 64 x 14 x 14 13.8 us; see for_window_rows for the limit).
+__device__ __forceinline__ void window_max(float a, float b, float c, float d, float& mv, float& mi) {
+  mv = -INFINITY;
+  mi = 0.f;
+  if (a > mv) { mv = a; mi = 0.f; }
+  if (b > mv) { mv = b; mi = 1.f; }
+  if (c > mv) { mv = c; mi = 2.f; }
+  if (d > mv) { mv = d; mi = 3.f; }
+}
+template <bool RELU, bool PAIR>
 __global__ void __launch_bounds__(kThreads) pool_fwd_2x2(const float* __restrict__ x, float* __restrict__ y,
-                                                          float* __restrict__ idx, int64_t total, int w, int ho, int wo) {
+                                                          float* __restrict__ idx, uint32_t total, int w, const FastDiv d_row) {
   RT_PDL_ENTRY();
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += stride) {
-    int xo = (int)(o % wo);
-    int64_t row = o / wo;  // = bc * ho + yo ; the input row pair starts at 2 * row (H = 2 * ho)
-    const float2* p = reinterpret_cast<const float2*>(x + (row * 2) * w) + xo;
-    float2 a = __ldg(p), b = __ldg(p + (w >> 1));
-    if (RELU) {
-      a.x = fmaxf(a.x, 0.f); a.y = fmaxf(a.y, 0.f);
-      b.x = fmaxf(b.x, 0.f); b.y = fmaxf(b.y, 0.f);
+  const uint32_t stride = gridDim.x * kThreads;
+  for (uint32_t o = blockIdx.x * kThreads + threadIdx.x; o < total; o += stride) {
+    uint32_t row, xo;
+    d_row.divmod(o, row, xo);  // row = bc * ho + yo ; the input row pair starts at 2 * row (H = 2 * ho)
+    const float* q = x + (int64_t)row * 2 * w;
+    if (PAIR) {
+      float4 a = __ldg(reinterpret_cast<const float4*>(q) + xo), b = __ldg(reinterpret_cast<const float4*>(q + w) + xo);
+      if (RELU) {
+        a.x = fmaxf(a.x, 0.f); a.y = fmaxf(a.y, 0.f); a.z = fmaxf(a.z, 0.f); a.w = fmaxf(a.w, 0.f);
+        b.x = fmaxf(b.x, 0.f); b.y = fmaxf(b.y, 0.f); b.z = fmaxf(b.z, 0.f); b.w = fmaxf(b.w, 0.f);
+      }
+      float2 mv, mi;
+      window_max(a.x, a.y, b.x, b.y, mv.x, mi.x);
+      window_max(a.z, a.w, b.z, b.w, mv.y, mi.y);
+      reinterpret_cast<float2*>(y)[o] = mv;
+      reinterpret_cast<float2*>(idx)[o] = mi;
+    } else {
+      float2 a = __ldg(reinterpret_cast<const float2*>(q) + xo), b = __ldg(reinterpret_cast<const float2*>(q + w) + xo);
+      if (RELU) {
+        a.x = fmaxf(a.x, 0.f); a.y = fmaxf(a.y, 0.f);
+        b.x = fmaxf(b.x, 0.f); b.y = fmaxf(b.y, 0.f);
+      }
+      float mv, mi;
+      window_max(a.x, a.y, b.x, b.y, mv, mi);
+      y[o] = mv;
+      idx[o] = mi;
     }
-    float mv = -INFINITY;
-    int mi = 0;
-    if (a.x > mv) { mv = a.x; mi = 0; }
-    if (a.y > mv) { mv = a.y; mi = 1; }
-    if (b.x > mv) { mv = b.x; mi = 2; }
-    if (b.y > mv) { mv = b.y; mi = 3; }
-    y[o] = mv;
-    idx[o] = (float)mi;
   }
 }
 
@@ -136,12 +156,12 @@ __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_pair(const float* __res
 // and nowhere otherwise.  Two windows per thread like pool_bwd_2x2_pair; the un-pooled tensor is not read.
 __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_from_output(const float* __restrict__ y, const float* __restrict__ g,
                                                                       const float* __restrict__ idx, float* __restrict__ dx,
-                                                                      int64_t total2, int w, int wo2) {
+                                                                      uint32_t total2, int w, const FastDiv d_row) {
   RT_PDL_ENTRY();
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total2; o += stride) {
-    const int xo = (int)(o % wo2);
-    const int64_t row = o / wo2;
+  const uint32_t stride = gridDim.x * kThreads;
+  for (uint32_t o = blockIdx.x * kThreads + threadIdx.x; o < total2; o += stride) {
+    uint32_t row, xo;
+    d_row.divmod(o, row, xo);
     float2 gv = __ldcs(reinterpret_cast<const float2*>(g) + o);
     const float2 iv = __ldcs(reinterpret_cast<const float2*>(idx) + o);
     const float2 yv = __ldg(reinterpret_cast<const float2*>(y) + o);
@@ -150,22 +170,22 @@ __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_from_output(const float
     const int m0 = (int)lrintf(iv.x), m1 = (int)lrintf(iv.y);
     const float4 a = make_float4(m0 == 0 ? gv.x : 0.f, m0 == 1 ? gv.x : 0.f, m1 == 0 ? gv.y : 0.f, m1 == 1 ? gv.y : 0.f);
     const float4 b = make_float4(m0 == 2 ? gv.x : 0.f, m0 == 3 ? gv.x : 0.f, m1 == 2 ? gv.y : 0.f, m1 == 3 ? gv.y : 0.f);
-    float4* p = reinterpret_cast<float4*>(dx + (row * 2) * w) + xo;
+    float4* p = reinterpret_cast<float4*>(dx + (int64_t)row * 2 * w) + xo;
     p[0] = a;
     p[w >> 2] = b;
   }
 }
 __global__ void __launch_bounds__(kThreads) pool_bwd_2x2_from_output_scalar(const float* __restrict__ y, const float* __restrict__ g,
                                                                              const float* __restrict__ idx, float* __restrict__ dx,
-                                                                             int64_t total, int w, int wo) {
+                                                                             uint32_t total, int w, const FastDiv d_row) {
   RT_PDL_ENTRY();
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += stride) {
-    const int xo = (int)(o % wo);
-    const int64_t row = o / wo;
+  const uint32_t stride = gridDim.x * kThreads;
+  for (uint32_t o = blockIdx.x * kThreads + threadIdx.x; o < total; o += stride) {
+    uint32_t row, xo;
+    d_row.divmod(o, row, xo);
     const float gv = __ldg(y + o) > 0.f ? __ldg(g + o) : 0.f;
     const int mi = (int)lrintf(__ldg(idx + o));
-    float* p = dx + (row * 2) * w + 2 * xo;
+    float* p = dx + (int64_t)row * 2 * w + 2 * xo;
     p[0] = mi == 0 ? gv : 0.f;
     p[1] = mi == 1 ? gv : 0.f;
     p[w] = mi == 2 ? gv : 0.f;
@@ -236,6 +256,23 @@ static rt_status pool_dims(rt_ctx* ctx, int64_t h, int64_t w, int kh, int kw, in
   return RT_OK;
 }
 
+}  // extern "C"
+// launch(first row of windows, items, division of an item into row and position, blocks) for rows of `wo` windows, an item a window or
+// two: all at once, or parts of a billion items, which 32-bit positions hold.  The forward pass takes 8 blocks per SM, so that all run
+// at once and the next kernel's may wait beside them (64: 3 us more from pooling to the end of an image evaluation of 120).
+template <class Launch>
+static rt_status for_window_rows(rt_ctx* ctx, int64_t rows, int64_t wo, bool pair, int waves, const Launch& launch) {
+  const int64_t per_row = pair ? wo / 2 : wo, most = (1ll << 30) / per_row;
+  FastDiv d;
+  d.init((uint32_t)per_row);
+  for (int64_t row = 0; row < rows; row += most) {
+    const int64_t items = (rows - row < most ? rows - row : most) * per_row;
+    launch(row, (uint32_t)items, d, rt_grid_for(ctx, items, kThreads, waves));
+    RT_LAUNCHED(ctx);
+  }
+  return RT_OK;
+}
+extern "C" {
 static rt_status pool_forward(rt_ctx* ctx, bool relu, const float* x, int64_t n, int64_t c, int64_t h, int64_t w, int kh, int kw,
                               int sh, int sw, int ph, int pw, float* y, float* idx) {
   RT_CHECK_CTX(ctx);
@@ -251,8 +288,15 @@ static rt_status pool_forward(rt_ctx* ctx, bool relu, const float* x, int64_t n,
   bool fast = kh == 2 && kw == 2 && sh == 2 && sw == 2 && ph == 0 && pw == 0 && (h % 2 == 0) && (w % 2 == 0) &&
               (reinterpret_cast<uintptr_t>(x) % 8 == 0);
   if (fast) {
-    if (relu) rt_launch(ctx, pool_fwd_2x2<true>, grid, kThreads, 0, x, y, idx, total, (int)w, (int)ho, (int)wo);
-    else rt_launch(ctx, pool_fwd_2x2<false>, grid, kThreads, 0, x, y, idx, total, (int)w, (int)ho, (int)wo);
+    const bool pair = w % 4 == 0 && rt_aligned16(x) && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(idx)) & 7) == 0;
+    return for_window_rows(ctx, n * c * ho, wo, pair, 8, [&](int64_t row, uint32_t items, const FastDiv& d, int blocks) {
+      const float* xs = x + row * 2 * w;
+      float *ys = y + row * wo, *is = idx + row * wo;
+      if (relu && pair) rt_launch(ctx, pool_fwd_2x2<true, true>, blocks, kThreads, 0, xs, ys, is, items, (int)w, d);
+      else if (relu) rt_launch(ctx, pool_fwd_2x2<true, false>, blocks, kThreads, 0, xs, ys, is, items, (int)w, d);
+      else if (pair) rt_launch(ctx, pool_fwd_2x2<false, true>, blocks, kThreads, 0, xs, ys, is, items, (int)w, d);
+      else rt_launch(ctx, pool_fwd_2x2<false, false>, blocks, kThreads, 0, xs, ys, is, items, (int)w, d);
+    });
   } else {
     if (relu) pool_fwd_general<true><<<grid, kThreads, 0, ctx->stream>>>(x, y, idx, total, (int)h, (int)w, (int)ho, (int)wo, kh, kw, sh, sw, ph, pw);
     else pool_fwd_general<false><<<grid, kThreads, 0, ctx->stream>>>(x, y, idx, total, (int)h, (int)w, (int)ho, (int)wo, kh, kw, sh, sw, ph, pw);
@@ -340,12 +384,11 @@ rt_status rt_relu_max_pool2x2_backward_from_output(rt_ctx* ctx, const float* y, 
   RT_CHECK_PTR(ctx, dx);
   const bool pair = w % 4 == 0 && rt_aligned16(dx) && (reinterpret_cast<uintptr_t>(g) % 8 == 0) && (reinterpret_cast<uintptr_t>(idx) % 8 == 0) &&
                     (reinterpret_cast<uintptr_t>(y) % 8 == 0);
-  if (pair)
-    rt_launch(ctx, pool_bwd_2x2_from_output, rt_grid_for(ctx, total / 2, kThreads, 64), kThreads, 0, y, g, idx, dx, total / 2, (int)w, (int)(w / 4));
-  else
-    rt_launch(ctx, pool_bwd_2x2_from_output_scalar, rt_grid_for(ctx, total, kThreads, 16), kThreads, 0, y, g, idx, dx, total, (int)w, (int)(w / 2));
-  RT_LAUNCHED(ctx);
-  return RT_OK;
+  return for_window_rows(ctx, n * c * (h / 2), w / 2, pair, 64, [&](int64_t row, uint32_t items, const FastDiv& d, int blocks) {
+    const int64_t o = row * (w / 2);
+    if (pair) rt_launch(ctx, pool_bwd_2x2_from_output, blocks, kThreads, 0, y + o, g + o, idx + o, dx + 4 * o, items, (int)w, d);
+    else rt_launch(ctx, pool_bwd_2x2_from_output_scalar, blocks, kThreads, 0, y + o, g + o, idx + o, dx + 4 * o, items, (int)w, d);
+  });
 }
 
 rt_status rt_max_pool2d_backward(rt_ctx* ctx, const float* g, const float* idx, int64_t n, int64_t c, int64_t h, int64_t w,
