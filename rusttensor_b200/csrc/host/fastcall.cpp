@@ -1,5 +1,5 @@
 // The calls of the Python front end that a program makes many times a step - applying an op, reading a gradient, letting go of a tensor -
-// as a CPython extension over the engine's C API.
+// and those of a trainer's pipelined steps, as a CPython extension over the engine's C API.
 //
 // A small eager step is bound by the host: of 165 us for an MLP of three layers, most went into ctypes, which converts every
 // argument by way of Python objects (4 us an op, 2.5 a gradient, 1.2 a tensor released).  Here a call is a C call with arguments taken
@@ -218,7 +218,49 @@ PyMethodDef calls_methods[] = {
 };
 PyTypeObject CallsType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+// ---- pipelined steps of a trainer (function address, trainer's handle, ..) ----
+bool addresses(PyObject* const* args, Py_ssize_t nargs, Py_ssize_t want, unsigned long long* fn, int64_t* handle) {
+  if (nargs != want) {
+    PyErr_SetString(PyExc_TypeError, "wrong number of arguments");
+    return false;
+  }
+  *fn = PyLong_AsUnsignedLongLong(args[0]);
+  *handle = PyLong_AsLongLong(args[1]);
+  if (!*fn && !PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "a function's address is null");
+  return !PyErr_Occurred();
+}
+// pointer(fn, handle, index) -> (status, address)
+PyObject* module_pointer(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  unsigned long long fn;
+  int64_t handle;
+  if (!addresses(args, nargs, 3, &fn, &handle)) return nullptr;
+  const long index = PyLong_AsLong(args[2]);
+  if (index == -1 && PyErr_Occurred()) return nullptr;
+  float* out = nullptr;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = reinterpret_cast<int (*)(int64_t, int, float**)>(fn)(handle, (int)index, &out);
+  Py_END_ALLOW_THREADS
+  return Py_BuildValue("iK", rc, (unsigned long long)(uintptr_t)out);
+}
+// step(fn, handle) -> (status, loss of the previous step or None)
+PyObject* module_step(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  unsigned long long fn;
+  int64_t handle;
+  if (!addresses(args, nargs, 2, &fn, &handle)) return nullptr;
+  float loss = 0.f;
+  int has = 0, rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = reinterpret_cast<int (*)(int64_t, float*, int*)>(fn)(handle, &loss, &has);
+  Py_END_ALLOW_THREADS
+  return has ? Py_BuildValue("id", rc, (double)loss) : Py_BuildValue("iO", rc, Py_None);
+}
+PyMethodDef module_methods[] = {
+    {"pointer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(module_pointer)), METH_FASTCALL, nullptr},
+    {"step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(module_step)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 

@@ -551,7 +551,13 @@ rt_status rt_publish_to_host(rt_ctx* ctx, float* pinned_dst, const float* src, i
   if (n < 1 || n > 4096) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_publish_to_host: 1 to 4096 values, got %lld", (long long)n);
   // The kernel stores through the host pointer, so it must be pinned memory the device can reach (rt_host_alloc).
   cudaPointerAttributes attr{};
-  cudaError_t e = cudaPointerGetAttributes(&attr, pinned_dst);
+  cudaError_t e = cudaSuccess;
+  if (ctx->host_blocks.count(pinned_dst)) {  // known to be pinned; host and device addresses are the same
+    attr.type = cudaMemoryTypeHost;
+    attr.devicePointer = pinned_dst;
+  } else {
+    e = cudaPointerGetAttributes(&attr, pinned_dst);
+  }
   if (e != cudaSuccess || attr.type != cudaMemoryTypeHost || attr.devicePointer == nullptr) {
     if (e != cudaSuccess) cudaGetLastError();
     RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_publish_to_host: the destination is not pinned host memory (use rt_host_alloc)");

@@ -9,6 +9,7 @@ import ctypes as C
 import numpy as np
 
 from .frontend import Tensor, EngineError, _i64, _f64
+from . import _fastcall
 
 _f32p = C.POINTER(C.c_float)
 
@@ -38,6 +39,7 @@ class DataParallelTrainer:
             i += 1
         self._pinned = []
         self._pipeline_views = {}
+        self._buffer_fn, self._step_fn = (C.cast(getattr(self.host, "rth_" + n), C.c_void_p).value for n in ("dp_pipeline_buffer", "dp_step_pipelined"))
         for i, t in enumerate(self.inputs):
             p = _f32p()
             self._call("dp_pinned_input", C.c_int64(self.handle), C.c_int(i), C.byref(p))
@@ -197,20 +199,22 @@ class DataParallelTrainer:
     def pipeline_buffer(self, i):
         """numpy view of the pinned host buffer to fill with input ``i`` of the NEXT pipelined step
         (two buffers alternate; the call waits until the copy that last read this one has finished)."""
-        p = C.c_void_p()
-        self._call("dp_pipeline_buffer", C.c_int64(self.handle), C.c_int(i), C.byref(p))
-        view = self._pipeline_views.get((i, p.value))  # two buffers per input, for the trainer's lifetime
+        rc, address = _fastcall.pointer(self._buffer_fn, self.handle, i)
+        if rc != 0:
+            self.engine._raise(rc)
+        view = self._pipeline_views.get((i, address))  # two buffers per input, for the trainer's lifetime
         if view is None:
-            view = np.ctypeslib.as_array(C.cast(p, _f32p), shape=tuple(self.inputs[i].shape))
-            self._pipeline_views[(i, p.value)] = view
+            view = np.ctypeslib.as_array(C.cast(address, _f32p), shape=tuple(self.inputs[i].shape))
+            self._pipeline_views[(i, address)] = view
         return view
 
     def step_pipelined(self):
         """Enqueues one step from the pipeline buffers and returns the loss of the previous pipelined
         step (None for the first one): the host never waits for the step it has just enqueued."""
-        loss, has = C.c_float(0), C.c_int(0)
-        self._call("dp_step_pipelined", C.c_int64(self.handle), C.byref(loss), C.byref(has))
-        return loss.value if has.value else None
+        rc, loss = _fastcall.step(self._step_fn, self.handle)
+        if rc != 0:
+            self.engine._raise(rc)
+        return loss
 
     # ---- steps fed from a data set resident on the device (src/data.rs:125-209 without the host round trip) ----
     def attach_dataset(self, arrays):
