@@ -60,10 +60,7 @@ struct Node {
 };
 
 constexpr int kMaxDepth = 200;
-#ifndef RT_LAZY_SMALL
-#define RT_LAZY_SMALL ((size_t)1 << 20)
-#endif
-constexpr size_t kSmall = RT_LAZY_SMALL;    // elements up to which shared intermediate results are always written
+constexpr size_t kSmall = (size_t)1 << 20;    // elements up to which shared intermediate results are always written
 constexpr int kRecompute = 16;              // weight from which they are written whatever the size
 constexpr int kDuplicate = 2;               // most weight that is repeated for every element of a broadcast
 constexpr int kMaxChain = 512;              // depth of a sum of scalars (the losses of a sequence)
