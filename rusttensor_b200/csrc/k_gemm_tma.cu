@@ -5,7 +5,8 @@
 //  * feeds the raw fp32 tile to the MMA as the hi operand - the tensor core ignores the low 13 mantissa bits of a TF32 operand,
 //    which is the truncation hi = a & 0xffffe000 - so that only lo = a - hi has to be made;
 //  * keeps the A operand (hi and lo) in tensor memory, from which an MMA reads at no cost to shared memory;
-//  * uses 128 x 256 output tiles for products: per K-step of 8, 57 KB over shared memory against 384 cycles of MMAs.
+//  * uses 128 x 256 output tiles for products where these fill their waves: per K-step of 8, 57 KB over shared memory against 384 cycles
+//    of MMAs.
 // The tensor core adds every partial product into its fp32 accumulator with truncation: on one accumulator over the whole reduction
 // the error grows to 2.9e-5 of the result at 4096.  An accumulator is therefore emptied after every K-block of 32, or every
 // few, and these are summed in registers with rounding (error 3.5e-7 - 1e-6 whatever the length); accumulators are used in turn, so
@@ -527,6 +528,8 @@ rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m,
   const int64_t mt = (m + BM - 1) / BM, t256 = mt * ((n + 255) / 256), t128 = mt * ((n + 127) / 128);
   if ((m + 31) / 32 > 65535 || (k + 31) / 32 > 65535 || (n + 31) / 32 > 65535) return RT_ERR_UNIMPLEMENTED;
   const auto waves = [&](int64_t t) { return (t + ctx->sm_count - 1) / ctx->sm_count; };
+  // 256 columns cost twice the time of 128 and less of shared memory, unless the last wave of the larger tiles stands emptier (4096^3: 4 waves
+  // of 512 tiles against 7 of 1024, so 128)
   const bool wide = waves(t256) * 2 <= waves(t128);
   auto direct = [](const float* p, int64_t ld) { return rt_aligned16(p) && ld % 4 == 0; };
   RtScratch wa(ctx), wb(ctx);
