@@ -327,9 +327,10 @@ rt_status rt_softmax_nll_scaled(rt_ctx* ctx, const float* logits, const float* t
                                 float divisor, float* loss);
 rt_status rt_softmax_nll_scaled_backward(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes, float c,
                                          float* dlogits);
-/* rt_softmax_nll_scaled and rt_softmax_nll_scaled_backward of the same rows in one launch. */
+/* rt_softmax_nll_scaled and rt_softmax_nll_scaled_backward of the same rows in one launch; with g, the gradient is that of
+ * rt_softmax_cross_entropy_backward instead (c unused). */
 rt_status rt_softmax_nll_with_grad(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes, float scale,
-                                   float divisor, float c, float* loss, float* dlogits);
+                                   float divisor, const float* g, float c, float* loss, float* dlogits);
 
 /* loss[0] = the sum of `count` such losses (logits_i, targets_i) and of n_more scalars: the loss of a sequence. */
 rt_status rt_softmax_nll_list(rt_ctx* ctx, int count, const float* const* logits, const float* const* targets, int64_t rows, int64_t classes,

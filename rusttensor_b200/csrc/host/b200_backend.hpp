@@ -843,7 +843,7 @@ struct B200Backend {
           if (loss && l.rows == (int64_t)a.outer && l.classes == (int64_t)a.len) {  // the loss itself comes out of the same pass
             auto keep = loss->shared_from_this();
             float* out = lazy::new_block(loss->ctx, loss->numel);
-            const rt_status st = rt_softmax_nll_with_grad(ctx(), xp, tp, a.outer, a.len, l.scale, l.divisor, c, out, dx.ptr());
+            const rt_status st = rt_softmax_nll_with_grad(ctx(), xp, tp, a.outer, a.len, l.scale, l.divisor, nullptr, c, out, dx.ptr());
             if (st != RT_OK) {
               rt_free(ctx(), out);
               check(st);
@@ -1150,6 +1150,12 @@ struct B200Backend {
     return dx;
   }
   static Storage softmax_nll(const Storage& logits, const Storage& targets) {
+    // deferred, unless it is a size to be refused at once: its gradient, asked for first, brings the loss with it
+    if (deferrable(logits.shape) && logits.shape[1] <= 4096 && logits.shape[0] <= ((size_t)1 << 24))
+      return lz_opaque(lazy::Tag::FusedLoss, {}, {input(logits), input(targets)}, Shape{}, [](lazy::Node& n, float* out) {
+        const float *x = n.in[0].buf->data(), *t = n.in[1].buf->data();
+        return rt_softmax_cross_entropy(ctx(), x, t, (int64_t)n.in[0].shape[0], (int64_t)n.in[0].shape[1], out);
+      });
     Storage loss = alloc(Shape{});
     check(rt_softmax_cross_entropy(ctx(), logits.ptr(), targets.ptr(), (int64_t)logits.shape[0], (int64_t)logits.shape[1],
                                    loss.ptr()));
@@ -1162,6 +1168,23 @@ struct B200Backend {
     const bool need_l = o.inputs[0].requires_grad(), need_t = o.inputs[1].requires_grad();
     Storage dl = need_l ? alloc(logits.shape) : unused_grad(logits.shape);
     Storage dt = need_t ? alloc(targets.shape) : unused_grad(targets.shape);
+    if (need_l && !need_t && logits.buf) {
+      const float *x = logits.ptr(), *t = targets.ptr(), *gp = g.ptr();
+      for (DeviceBuffer* r : logits.buf->readers) {
+        if (!r->node || r->node->tag != lazy::Tag::FusedLoss || r->node->in[0].buf != logits.buf || r->node->in[1].buf != targets.buf) continue;
+        auto loss = r->shared_from_this();
+        float* out = lazy::new_block(loss->ctx, loss->numel);
+        const int64_t rows = (int64_t)logits.shape[0];
+        const rt_status st = rt_softmax_nll_with_grad(ctx(), x, t, rows, (int64_t)logits.shape[1], -1.f, (float)rows, gp, 0.f, out, dl.ptr());
+        if (st != RT_OK) {
+          rt_free(ctx(), out);
+          check(st);
+        }
+        loss->ptr = out;
+        loss->drop_node();
+        return {std::move(dl), std::move(dt)};
+      }
+    }
     check(rt_softmax_cross_entropy_backward(ctx(), logits.ptr(), targets.ptr(), g.ptr(), (int64_t)logits.shape[0],
                                             (int64_t)logits.shape[1], need_l ? dl.ptr() : nullptr, need_t ? dt.ptr() : nullptr));
     return {std::move(dl), std::move(dt)};

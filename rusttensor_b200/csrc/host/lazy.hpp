@@ -41,7 +41,7 @@ struct Input {
 };
 enum class Kind : uint8_t { Const, Unary, BinaryImm, Binary, Broadcast, Slice, Pad, Concat, Opaque };
 // Opaque: computed by a kernel of its own.  Deferred only because what it feeds may take a kernel that does both.
-enum class Tag : uint8_t { None, Matmul, Conv, LogSoftmax, Reduce, PoolGrad, SumProducts, SumRows };
+enum class Tag : uint8_t { None, Matmul, Conv, LogSoftmax, Reduce, PoolGrad, SumProducts, SumRows, FusedLoss };
 
 struct Node {
   Kind kind;

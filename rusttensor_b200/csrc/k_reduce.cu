@@ -1384,7 +1384,7 @@ extern "C" rt_status rt_softmax_nll_scaled(rt_ctx* ctx, const float* logits, con
 }
 
 extern "C" rt_status rt_softmax_nll_with_grad(rt_ctx* ctx, const float* logits, const float* targets, int64_t rows, int64_t classes, float scale,
-                                              float divisor, float c, float* loss, float* dlogits) {
+                                              float divisor, const float* g, float c, float* loss, float* dlogits) {
   RT_CHECK_CTX(ctx);
   if (rows <= 0 || classes <= 0) RT_FAIL(ctx, RT_ERR_EMPTY_TENSOR, "rt_softmax_nll: empty input");
   if (classes > 4096 || rows > (int64_t(1) << 24))
@@ -1394,6 +1394,7 @@ extern "C" rt_status rt_softmax_nll_with_grad(rt_ctx* ctx, const float* logits, 
   RT_CHECK_PTR(ctx, loss);
   RT_CHECK_PTR(ctx, dlogits);
   SceArgs a{logits, targets};
+  a.g = g;
   a.c = c;
   a.dlogits = dlogits;
   a.loss = loss;

@@ -110,7 +110,7 @@ def test_classification_loss_with_gradient(rows, classes):
     dx, dt, loss, grad = api.to_device(x), api.to_device(t), api.to_device(np.zeros(1, np.float32)), api.to_device(np.zeros_like(x))
     ls = x - np.log(np.exp(x.astype(np.float64)).sum(1, keepdims=True))
     for _ in range(2):  # the ticket has to be back at zero
-        api.call("softmax_nll_with_grad", dx.ptr, dt.ptr, C.c_int64(rows), C.c_int64(classes), C.c_float(-1), C.c_float(rows), C.c_float(-1 / rows),
+        api.call("softmax_nll_with_grad", dx.ptr, dt.ptr, C.c_int64(rows), C.c_int64(classes), C.c_float(-1), C.c_float(rows), None, C.c_float(-1 / rows),
                  loss.ptr, grad.ptr)
         np.testing.assert_allclose(loss.numpy()[0], -(ls * t).sum() / rows, rtol=2e-6, atol=1e-7)
         want = -(t - np.exp(ls) * t.sum(1, keepdims=True, dtype=np.float64)) / rows
