@@ -154,14 +154,27 @@ struct B200Backend {
     };
     return defer(std::move(n), shape);
   }
+  // Rows that point into another tensor's block (a slice taken inside a capture) get a block of their own.
+  static void own(const Storage& s) {
+    if (!s.buf) return;
+    const float* p = s.buf->data();
+    if (!s.buf->owner) return;
+    float* block = lazy::new_block(ctx(), s.buf->numel);
+    const rt_status st = rt_memcpy_d2d(ctx(), block, p, sizeof(float) * s.buf->numel);
+    if (st != RT_OK) {
+      rt_free(ctx(), block);
+      check(st);
+    }
+    s.buf->ptr = block;
+    s.buf->owner.reset();
+  }
   // The address of a tensor's values for use outside the engine: whoever has it may write there at any time.
   static float* escape(const Storage& s) {
     if (!s.buf) return nullptr;
+    own(s);
     s.buf->flush_readers();
-    float* p = s.buf->data();
     s.buf->escaped = true;
-    if (s.buf->owner) s.buf->owner->escaped = true;
-    return p;
+    return s.buf->ptr;
   }
   static void begin_capture() {
     lazy::flush_all();  // what was asked for before the capture must not become part of the graph

@@ -154,17 +154,17 @@ struct DpTrainer {
     if (do_reduce) B200Backend::check(rt_dp_allreduce_sum(c, dst + begin, end - begin));
   }
 
-  // Everything a step leaves behind is evaluated as part of it (the loss and the gradients, which a captured graph writes on
-  // every replay); the recorded ops go, and with them the intermediate results that nobody has asked for.
+  // Everything a step leaves behind is evaluated as part of it, in blocks of its own (the loss and the gradients, which a captured
+  // graph writes on every replay); the recorded ops go, and with them the intermediate results that nobody has asked for.
   void settle(const Tensor& loss) {
-    loss.data().ptr();
+    B200Backend::own(loss.data());
     std::vector<const Storage*> grads;
     for (auto& p : tr->w.params)
       if (p.grad()) grads.push_back(&*p.grad());
     B200Backend::evaluate_column_sums(grads);
-    for (auto* g : grads) g->ptr();
+    for (auto* g : grads) B200Backend::own(*g);
     for (auto& x : inputs)
-      if (x.grad()) x.grad()->ptr();
+      if (x.grad()) B200Backend::own(*x.grad());
     loss.detach_graph();
   }
 
@@ -223,7 +223,7 @@ struct DpTrainer {
       }
       fired = true;
       if (capturing) {  // split the capture here; the exchange of the early slice runs between the two replays
-        for (int i = early_lo; i < early_hi; ++i) w.params[i].grad()->ptr();  // evaluated inside the first part
+        for (int i = early_lo; i < early_hi; ++i) B200Backend::own(*w.params[i].grad());  // evaluated inside the first part
         B200Backend::end_capture(&graph);
         B200Backend::begin_capture();
       } else {

@@ -12,6 +12,9 @@
 //    kernels) first evaluates every expression that reads it (flush_readers).
 //  * A buffer whose address has been handed out may be written behind the engine's back, so expressions that read it are
 //    evaluated on the spot - except inside a graph capture, where the whole step is recorded anyway.
+//  * A slice of whole rows points into its base's block only inside a capture, where nothing outside the engine sees either of them
+//    before the step is recorded; what a step leaves behind gets a block of its own (B200Backend::own).  Elsewhere the address of one
+//    of the two may be handed out and written through, and a slice would keep its base's memory.
 //  * A capture starts with nothing unevaluated (flush_all), so that it records exactly the step's own work, and rth_sync leaves
 //    nothing unevaluated either.
 //  * Depth is bounded: a result whose expression has become kMaxDepth ops deep is evaluated at once.
@@ -999,10 +1002,10 @@ inline bool rewrite_loss_sum(DeviceBuffer* b) {
   b->drop_node();
   return true;
 }
-// Rows of a tensor that is in memory: no copy, the result points into it.
+// Rows of a tensor that is in memory, inside a capture: no copy, the result points into it.
 inline bool rewrite_rows(DeviceBuffer* b) {
   const Node* n = b->node.get();
-  if (n->kind != Kind::Slice || (n->in[0].buf->escaped && !capturing())) return false;
+  if (n->kind != Kind::Slice || !capturing()) return false;
   const Input& base = n->in[0];
   if (base.buf->node && base.buf->node->kind != Kind::Opaque) return false;
   size_t d = 0;

@@ -1,0 +1,140 @@
+// Checks of the CUDA backend's host logic (host/b200_backend.hpp, host/lazy.hpp) without a GPU: the few C-ABI entry points that they
+// reach are stubs over host memory, which count blocks and fail on demand.  Usage: engine_checks NAME; test_engine_host.py runs them.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+
+#include "../../rusttensor_b200/csrc/host/b200_backend.hpp"
+
+using namespace rt;
+using B = B200Backend;
+
+namespace {
+std::map<void*, size_t> live;  // blocks that are allocated
+int failures;                  // of the checks
+int mallocs_left = -1;         // rt_malloc fails once they are used up; < 0: never
+bool kernels_fail = false;
+
+void expect(bool ok, const char* what, int line) {
+  if (ok) return;
+  std::printf("line %d: %s\n", line, what);
+  ++failures;
+}
+#define EXPECT(x) expect((x), #x, __LINE__)
+
+B::Storage make(const Shape& s, float first, float step = 1.f) {
+  B::Storage x = B::alloc(s);
+  for (size_t i = 0; i < x.numel(); ++i) x.buf->ptr[i] = first + step * (float)i;
+  return x;
+}
+bool holds(const B::Storage& x, float first, float step = 1.f) {
+  const float* p = x.ptr();
+  for (size_t i = 0; i < x.numel(); ++i)
+    if (p[i] != first + step * (float)i) return false;
+  return true;
+}
+void scribble(float* p, size_t n) {
+  for (size_t i = 0; i < n; ++i) p[i] = -77.f;
+}
+}  // namespace
+
+// ---- the stubs ------------------------------------------------------------------------------------------------------------
+extern "C" {
+const char* rt_last_error(rt_ctx*) { return "stub"; }
+rt_status rt_malloc(rt_ctx*, size_t bytes, void** out) {
+  if (mallocs_left == 0) return RT_ERR_OOM;
+  if (mallocs_left > 0) --mallocs_left;
+  *out = std::calloc(1, bytes);
+  live[*out] = bytes;
+  return RT_OK;
+}
+rt_status rt_free(rt_ctx*, void* p) {
+  if (!p) return RT_OK;
+  if (!live.erase(p)) {
+    std::printf("a block is freed twice, or is none\n");
+    ++failures;
+    return RT_OK;
+  }
+  std::free(p);
+  return RT_OK;
+}
+rt_status rt_memcpy_d2d(rt_ctx*, void* d, const void* s, size_t n) {
+  std::memmove(d, s, n);
+  return RT_OK;
+}
+rt_status rt_unary(rt_ctx*, int op, const float* x, float* y, int64_t n, float, float) {
+  if (kernels_fail || op != RT_SQUARE) return RT_ERR_CUDA;
+  for (int64_t i = 0; i < n; ++i) y[i] = x[i] * x[i];
+  return RT_OK;
+}
+rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of two-dimensional windows are all that the checks need
+  if (kernels_fail || p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_ERR_CUDA;
+  const int rows = p->nd == 2 ? p->shape[0] : 1, cols = p->shape[p->nd - 1];
+  const rt_fused_operand& o = p->operand[0];
+  for (int i = 0; i < rows; ++i)
+    for (int j = 0; j < cols; ++j) p->out[0][i * cols + j] = o.ptr[(p->nd == 2 ? i * o.stride[0] : 0) + j * o.stride[p->nd - 1]];
+  return RT_OK;
+}
+}
+
+// ---- the checks -----------------------------------------------------------------------------------------------------------
+namespace {
+
+// A slice of whole rows and its base do not see each other's writes through a device pointer.
+void rows_do_not_alias() {
+  const Shape s{6, 4};
+  for (int first : {0, 2}) {
+    B::Storage x = make(s, 1.f), y = B::slice(x, {{2, 4}, {0, 4}}), z = B::unary(RT_SQUARE, y);
+    EXPECT(holds(y, 9.f));
+    scribble(B::escape(first == 0 ? x : y), first == 0 ? 24 : 8);
+    EXPECT(first == 0 ? holds(y, 9.f) : holds(x, 1.f));
+    for (int i = 0; i < 8; ++i) EXPECT(z.ptr()[i] == (9.f + i) * (9.f + i));  // asked for before the write
+  }
+  {  // a slice of a slice, of one row
+    B::Storage x = make(s, 1.f), y = B::slice(x, {{1, 5}, {0, 4}}), w = B::slice(y, {{3, 4}, {1, 3}});
+    EXPECT(holds(w, 18.f));
+    scribble(B::escape(y), 16);
+    scribble(B::escape(x), 24);
+    EXPECT(holds(w, 18.f));
+  }
+  {  // the base's memory goes with the base
+    B::Storage x = make(s, 1.f), y = B::slice(x, {{2, 4}, {0, 4}});
+    y.ptr();
+    x = B::Storage{};
+    EXPECT(live.size() == 1 && live.begin()->second == 8 * sizeof(float));
+  }
+  EXPECT(live.empty());
+}
+// Inside a capture rows are not copied; what a step leaves behind has a block of its own.
+void rows_in_a_capture() {
+  B::Storage x = make({6, 4}, 1.f);
+  lazy::capturing() = true;
+  B::Storage y = B::slice(x, {{2, 4}, {0, 4}});
+  EXPECT(y.ptr() == x.ptr() + 8);
+  B::Storage w = B::slice(y, {{1, 2}, {0, 4}});
+  EXPECT(w.ptr() == x.ptr() + 12);
+  B::own(y);
+  lazy::capturing() = false;
+  scribble(B::escape(x), 24);
+  EXPECT(holds(y, 9.f));
+  EXPECT(B::escape(w) != x.ptr() + 12);
+}
+
+const struct {
+  const char* name;
+  void (*run)();
+} kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture}};
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  B::ctx_slot() = reinterpret_cast<rt_ctx*>(&failures);  // never looked into
+  for (auto& c : kChecks)
+    if (argc == 2 && std::strcmp(argv[1], c.name) == 0) {
+      c.run();
+      return failures ? 1 : 0;
+    }
+  std::printf("unknown check\n");
+  return 2;
+}
