@@ -1124,7 +1124,7 @@ struct B200Backend {
       const Storage& x = o.inputs[0].data();
       if (halves && o.cached_outputs && lazy::is_op(x.buf->node.get(), lazy::Kind::Unary, RT_F_RELU)) in.push_back(input(*o.cached_outputs));
       std::vector<int64_t> q{(int64_t)is[0], (int64_t)is[1], (int64_t)is[2], (int64_t)is[3], (int64_t)k.first, (int64_t)k.second,
-                             (int64_t)s.first, (int64_t)s.second, (int64_t)p.first, (int64_t)p.second, (int64_t)(intptr_t)x.buf.get()};
+                             (int64_t)s.first, (int64_t)s.second, (int64_t)p.first, (int64_t)p.second, (int64_t)x.buf->id};
       return lz_opaque(lazy::Tag::PoolGrad, std::move(q), std::move(in), is, [](lazy::Node& n, float* out) {
         const auto& q = n.geo;
         return rt_max_pool2d_backward(ctx(), n.in[0].buf->data(), n.in[1].buf->data(), q[0], q[1], q[2], q[3], (int)q[4], (int)q[5], (int)q[6],

@@ -944,7 +944,7 @@ inline bool rewrite_pool(DeviceBuffer* b) {
     const Node* st = pending(n->in[1 - i]);
     if (!pg || !is_op(st, Kind::Unary, RT_F_STEP) || pg->shape != n->shape || st->shape != n->shape || n->in[i].shape != n->shape) continue;
     if (n->in[i].buf->readers.size() != 1 || pg->in.size() != 3) continue;  // in: g, idx, pooled relu output
-    if (pg->geo[10] != (int64_t)(intptr_t)st->in[0].buf.get()) continue;    // the relu's output is what was pooled
+    if (pg->geo[10] != (int64_t)st->in[0].buf->id) continue;                // the relu's output is what was pooled
     const auto& q = pg->geo;
     const float *y = pg->in[2].buf->data(), *g = pg->in[0].buf->data(), *idx = pg->in[1].buf->data();
     float* out = new_block(b->ctx, b->numel);

@@ -15,6 +15,8 @@ std::map<void*, size_t> live;  // blocks that are allocated
 int failures;                  // of the checks
 int mallocs_left = -1;         // rt_malloc fails once they are used up; < 0: never
 bool kernels_fail = false;
+int masked_pool_gradients;     // launches of the pooling gradient that masks by the relu in front
+
 
 void expect(bool ok, const char* what, int line) {
   if (ok) return;
@@ -68,8 +70,19 @@ rt_status rt_unary(rt_ctx*, int op, const float* x, float* y, int64_t n, float, 
   for (int64_t i = 0; i < n; ++i) y[i] = x[i] * x[i];
   return RT_OK;
 }
-rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of two-dimensional windows are all that the checks need
-  if (kernels_fail || p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_ERR_CUDA;
+rt_status rt_relu_max_pool2d(rt_ctx*, const float*, int64_t, int64_t, int64_t, int64_t, int, int, int, int, int, int, float*, float*) {
+  return RT_OK;
+}
+rt_status rt_max_pool2d_backward(rt_ctx*, const float*, const float*, int64_t, int64_t, int64_t, int64_t, int, int, int, int, int, int, float*) {
+  return RT_OK;
+}
+rt_status rt_relu_max_pool2x2_backward_from_output(rt_ctx*, const float*, const float*, const float*, int64_t, int64_t, int64_t, int64_t, float*) {
+  ++masked_pool_gradients;
+  return RT_OK;
+}
+rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of windows; results of other programs stay zero
+  if (kernels_fail) return RT_ERR_CUDA;
+  if (p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_OK;
   const int rows = p->nd == 2 ? p->shape[0] : 1, cols = p->shape[p->nd - 1];
   const rt_fused_operand& o = p->operand[0];
   for (int i = 0; i < rows; ++i)
@@ -120,11 +133,41 @@ void rows_in_a_capture() {
   EXPECT(holds(y, 9.f));
   EXPECT(B::escape(w) != x.ptr() + 12);
 }
+// The gradient of a pooling is masked by the relu in front of it, not by one whose buffer happens to lie where that one's was.
+void pooling_knows_its_relu() {
+  const Shape s{1, 1, 4, 4};
+  for (bool same : {true, false}) {
+    masked_pool_gradients = 0;
+    B::Storage gradient, mask, other = make(s, 3.f);
+    const DeviceBuffer* old;
+    {
+      B::Storage x = B::unary(RT_RELU, make(s, -5.f));
+      old = x.buf.get();
+      auto pooled = B::max_pool2d(x, {2, 2}, {2, 2}, {0, 0});
+      OpType t(OpType::MaxPool2D);
+      t.kernel_size = t.stride = {2, 2};
+      t.padding = {0, 0};
+      Op<B> op(t, {Tensor<B>(x, true), Tensor<B>(pooled.second, false)}, nullptr);
+      op.cached_outputs = pooled.first;
+      gradient = B::max_pool2d_backward(op, make(pooled.first.shape, 1.f));
+      if (same) mask = B::lz_unary(RT_F_STEP, x);
+    }
+    std::vector<B::Storage> tried;
+    for (int i = 0; i < 1000 && !same && !mask.buf; ++i) {
+      tried.push_back(B::unary(RT_RELU, other));
+      if (tried.back().buf.get() == old) mask = B::lz_unary(RT_F_STEP, tried.back());
+    }
+    if (!mask.buf) continue;  // the address was not used again
+    B::lz_mul(gradient, mask).ptr();
+    EXPECT(masked_pool_gradients == (same ? 1 : 0));
+  }
+}
 
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture}};
+} kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
+               {"pooling_knows_its_relu", pooling_knows_its_relu}};
 
 }  // namespace
 
