@@ -76,6 +76,13 @@ struct B200Backend {
     return n > 0 && n < ((size_t)1 << 31) && s.size() <= (size_t)lazy::kMaxRawDims;
   }
   static Storage defer(lazy::Node n, const Shape& shape) {
+    bool now;
+    Storage s = pend(std::move(n), shape, &now);
+    if (now) s.buf->data();
+    return s;
+  }
+  // The same, but left to the caller to evaluate when it has to be done `now`.
+  static Storage pend(lazy::Node n, const Shape& shape, bool* at_once) {
     n.shape = shape;
     bool now = false;
     for (auto& i : n.in) {
@@ -88,9 +95,8 @@ struct B200Backend {
     const bool scalar_sum = n.kind == lazy::Kind::Binary && n.op == RT_F_ADD && shape_numel(shape) == 1;
     now = now || n.depth >= (scalar_sum ? lazy::kMaxChain : lazy::kMaxDepth);
     n.weight = std::min(n.weight, 1 << 20);
-    Storage s{std::make_shared<DeviceBuffer>(ctx(), std::make_unique<lazy::Node>(std::move(n)), shape_numel(shape)), shape};
-    if (now) s.buf->data();
-    return s;
+    *at_once = now;
+    return Storage{std::make_shared<DeviceBuffer>(ctx(), std::make_unique<lazy::Node>(std::move(n)), shape_numel(shape)), shape};
   }
   static lazy::Input input(const Storage& x) { return lazy::Input{x.buf, x.shape}; }
   static bool is_const(const Storage& x) { return x.buf && x.buf->node && x.buf->node->kind == lazy::Kind::Const; }
@@ -144,13 +150,9 @@ struct B200Backend {
     n.in = std::move(in);
     n.weight = 1 << 10;
     n.run = [run](lazy::Node& nd, DeviceBuffer* b) {
-      float* out = lazy::new_block(b->ctx, b->numel);
-      const rt_status st = run(nd, out);
-      if (st != RT_OK) {
-        rt_free(b->ctx, out);
-        check(st);
-      }
-      b->ptr = out;
+      lazy::Block out(b->ctx, b->numel);
+      check(run(nd, out.ptr));
+      b->ptr = out.release();
     };
     return defer(std::move(n), shape);
   }
@@ -159,13 +161,9 @@ struct B200Backend {
     if (!s.buf) return;
     const float* p = s.buf->data();
     if (!s.buf->owner) return;
-    float* block = lazy::new_block(ctx(), s.buf->numel);
-    const rt_status st = rt_memcpy_d2d(ctx(), block, p, sizeof(float) * s.buf->numel);
-    if (st != RT_OK) {
-      rt_free(ctx(), block);
-      check(st);
-    }
-    s.buf->ptr = block;
+    lazy::Block block(ctx(), s.buf->numel);
+    check(rt_memcpy_d2d(ctx(), block.ptr, p, sizeof(float) * s.buf->numel));
+    s.buf->ptr = block.release();
     s.buf->owner.reset();
   }
   // The address of a tensor's values for use outside the engine: whoever has it may write there at any time.
@@ -264,10 +262,11 @@ struct B200Backend {
     }
     Storage out = alloc(Shape{idx.size(), row_len});
     if (idx.empty() || row_len == 0) return out;
+    const float* src = x.ptr();
     void* d = nullptr;
     check(rt_malloc(ctx(), sizeof(int32_t) * h.size(), &d));
     rt_status st = rt_memcpy_h2d(ctx(), d, h.data(), sizeof(int32_t) * h.size());
-    if (st == RT_OK) st = rt_gather_rows(ctx(), x.ptr(), (int64_t)rows, (int64_t)row_len, static_cast<const int32_t*>(d), (int64_t)h.size(), out.ptr());
+    if (st == RT_OK) st = rt_gather_rows(ctx(), src, (int64_t)rows, (int64_t)row_len, static_cast<const int32_t*>(d), (int64_t)h.size(), out.ptr());
     rt_free(ctx(), d);
     check(st);
     return out;
@@ -568,32 +567,33 @@ struct B200Backend {
   // Those of `grads` that are unevaluated column sums of matrices of up to 2048 rows (more are better split over blocks), in one launch.
   static void evaluate_column_sums(const std::vector<const Storage*>& grads) {
     std::vector<std::shared_ptr<DeviceBuffer>> sums;
+    for (auto* g : grads) {
+      const lazy::Node* n = g->buf ? g->buf->node.get() : nullptr;
+      if (n && n->tag == lazy::Tag::SumRows && n->geo[0] < 0 && n->in[0].shape[0] <= 2048 && n->in[0].shape[1] == g->buf->numel &&
+          std::find(sums.begin(), sums.end(), g->buf) == sums.end())
+        sums.push_back(g->buf);
+    }
+    if (sums.size() < 2) return;
+    for (auto& b : sums)
+      if (b->node) {
+        const std::shared_ptr<DeviceBuffer> x = b->node->in[0].buf;
+        x->data();
+      }
+    sums.erase(std::remove_if(sums.begin(), sums.end(), [](auto& b) { return !b->node; }), sums.end());  // evaluated on the way
     std::vector<const float*> xs;
     std::vector<int64_t> rows, cols;
     std::vector<float*> outs;
-    for (auto* g : grads) {
-      const lazy::Node* n = g->buf ? g->buf->node.get() : nullptr;
-      if (n && n->tag == lazy::Tag::SumRows && n->geo[0] < 0 && n->in[0].shape[0] <= 2048 && n->in[0].shape[1] == g->buf->numel) sums.push_back(g->buf);
-    }
-    if (sums.size() < 2) return;
+    std::vector<lazy::Block> blocks;
     for (auto& b : sums) {
-      const std::shared_ptr<DeviceBuffer> x = b->node->in[0].buf;
-      rows.push_back((int64_t)b->node->in[0].shape[0]);
-      cols.push_back((int64_t)b->node->in[0].shape[1]);
-      xs.push_back(x->data());
-      if (!b->node) return;  // evaluated on the way
-      outs.push_back(lazy::new_block(b->ctx, b->numel));
+      const lazy::Input& x = b->node->in[0];
+      xs.push_back(x.buf->data());
+      rows.push_back((int64_t)x.shape[0]);
+      cols.push_back((int64_t)x.shape[1]);
+      blocks.emplace_back(b->ctx, b->numel);
+      outs.push_back(blocks.back().ptr);
     }
-    const rt_status st = rt_column_sums_list(ctx(), (int)sums.size(), xs.data(), rows.data(), cols.data(), outs.data());
-    for (size_t i = 0; i < sums.size(); ++i) {
-      if (st != RT_OK) {
-        rt_free(ctx(), outs[i]);
-        continue;
-      }
-      sums[i]->ptr = outs[i];
-      sums[i]->drop_node();
-    }
-    check(st);
+    check(rt_column_sums_list(ctx(), (int)sums.size(), xs.data(), rows.data(), cols.data(), outs.data()));
+    for (size_t i = 0; i < sums.size(); ++i) blocks[i].to(sums[i].get());
   }
   static Storage slice(const Storage& x, const std::vector<Range>& ranges) {
     if (ranges.size() != x.shape.size()) throw Error::invalid_op("Slice ranges do not match input dimensionality");
@@ -855,14 +855,9 @@ struct B200Backend {
           DeviceBuffer* loss = lazy::loss_over(x.buf.get(), t->buf.get(), &l);
           if (loss && l.rows == (int64_t)a.outer && l.classes == (int64_t)a.len) {  // the loss itself comes out of the same pass
             auto keep = loss->shared_from_this();
-            float* out = lazy::new_block(loss->ctx, loss->numel);
-            const rt_status st = rt_softmax_nll_with_grad(ctx(), xp, tp, a.outer, a.len, l.scale, l.divisor, nullptr, c, out, dx.ptr());
-            if (st != RT_OK) {
-              rt_free(ctx(), out);
-              check(st);
-            }
-            loss->ptr = out;
-            loss->drop_node();
+            lazy::Block out(loss->ctx, loss->numel);
+            check(rt_softmax_nll_with_grad(ctx(), xp, tp, a.outer, a.len, l.scale, l.divisor, nullptr, c, out.ptr, dx.ptr()));
+            out.to(loss);
             return dx;
           }
           check(rt_softmax_nll_scaled_backward(ctx(), x.ptr(), tp, a.outer, a.len, c, dx.ptr()));
@@ -949,16 +944,26 @@ struct B200Backend {
     for (auto& t : term) n.in.push_back(std::move(t));
     n.run = run;
     const Shape s = acc.shape;
+    bool now;
     acc = Storage{};  // the node now holds the old values, alone unless somebody else does too
-    acc = defer(std::move(n), s);
+    acc = pend(std::move(n), s, &now);
+    if (now) acc.buf->data();
   }
-  // The block in which a sum goes on: the old values' own one when nobody else needs it.
-  static float* sum_block(lazy::Node& n, DeviceBuffer* b) {
+  // Adds to the old values: in their own block when nobody else needs it.  After an error the old values still have their block.
+  template <class F>
+  static void add_to(lazy::Node& n, DeviceBuffer* b, F add) {
     DeviceBuffer* base = n.in[0].buf.get();
-    if (n.in[0].buf.use_count() == 1 && !base->escaped && !base->owner) return std::exchange(base->ptr, nullptr);
-    float* out = lazy::new_block(b->ctx, b->numel);
-    check(rt_memcpy_d2d(ctx(), out, base->data(), sizeof(float) * b->numel));
-    return out;
+    float* old = base->data();
+    if (n.in[0].buf.use_count() == 1 && !base->escaped && !base->owner) {
+      check(add(old));
+      base->ptr = nullptr;
+      b->ptr = old;
+      return;
+    }
+    lazy::Block out(b->ctx, b->numel);
+    check(rt_memcpy_d2d(ctx(), out.ptr, old, sizeof(float) * b->numel));
+    check(add(out.ptr));
+    b->ptr = out.release();
   }
   static void run_sum_products(lazy::Node& n, DeviceBuffer* b) {
     std::vector<const float*> as, gs;
@@ -966,8 +971,7 @@ struct B200Backend {
       as.push_back(n.in[i].buf->data());
       gs.push_back(n.in[i + 1].buf->data());
     }
-    b->ptr = sum_block(n, b);
-    check(rt_gemm_sum_products(ctx(), (int)as.size(), as.data(), gs.data(), n.geo[0], n.geo[1], n.geo[2], b->ptr));
+    add_to(n, b, [&](float* out) { return rt_gemm_sum_products(ctx(), (int)as.size(), as.data(), gs.data(), n.geo[0], n.geo[1], n.geo[2], out); });
   }
   // existing + g for a gradient that receives another contribution (Tensor::add_grad).
   static Storage accumulate(Storage existing, const Storage& g) {
@@ -982,8 +986,7 @@ struct B200Backend {
   static void run_sum_rows(lazy::Node& n, DeviceBuffer* b) {
     std::vector<const float*> xs;
     for (size_t i = 1; i < n.in.size(); ++i) xs.push_back(n.in[i].buf->data());
-    b->ptr = sum_block(n, b);
-    check(rt_sum_rows_accumulate_list(ctx(), (int)xs.size(), xs.data(), n.geo[0], n.geo[1], b->ptr));
+    add_to(n, b, [&](float* out) { return rt_sum_rows_accumulate_list(ctx(), (int)xs.size(), xs.data(), n.geo[0], n.geo[1], out); });
   }
   static void conv_shapes(const Storage& x, const Storage& w, const char* name) {
     if (x.shape.size() != 4 || w.shape.size() != 4) throw Error::invalid_op(std::string(name) + " expects 4D input and weights");
@@ -1186,15 +1189,10 @@ struct B200Backend {
       for (DeviceBuffer* r : logits.buf->readers) {
         if (!r->node || r->node->tag != lazy::Tag::FusedLoss || r->node->in[0].buf != logits.buf || r->node->in[1].buf != targets.buf) continue;
         auto loss = r->shared_from_this();
-        float* out = lazy::new_block(loss->ctx, loss->numel);
+        lazy::Block out(loss->ctx, loss->numel);
         const int64_t rows = (int64_t)logits.shape[0];
-        const rt_status st = rt_softmax_nll_with_grad(ctx(), x, t, rows, (int64_t)logits.shape[1], -1.f, (float)rows, gp, 0.f, out, dl.ptr());
-        if (st != RT_OK) {
-          rt_free(ctx(), out);
-          check(st);
-        }
-        loss->ptr = out;
-        loss->drop_node();
+        check(rt_softmax_nll_with_grad(ctx(), x, t, rows, (int64_t)logits.shape[1], -1.f, (float)rows, gp, 0.f, out.ptr, dl.ptr()));
+        out.to(loss.get());
         return {std::move(dl), std::move(dt)};
       }
     }

@@ -680,11 +680,26 @@ class Compiler {
 inline void check(rt_ctx* ctx, rt_status st) {
   if (st != RT_OK) throw Error((ErrorKind)st, rt_last_error(ctx));
 }
-inline float* new_block(rt_ctx* ctx, size_t numel) {
-  void* p = nullptr;
-  check(ctx, rt_malloc(ctx, sizeof(float) * std::max<size_t>(numel, 1), &p));
-  return (float*)p;
-}
+// A new block for a result; given back unless it becomes a buffer's.
+struct Block {
+  rt_ctx* ctx;
+  float* ptr = nullptr;
+  Block(rt_ctx* c, size_t numel) : ctx(c) {
+    void* p = nullptr;
+    check(ctx, rt_malloc(ctx, sizeof(float) * std::max<size_t>(numel, 1), &p));
+    ptr = (float*)p;
+  }
+  Block(Block&& o) noexcept : ctx(o.ctx), ptr(std::exchange(o.ptr, nullptr)) {}
+  Block& operator=(Block&&) = delete;
+  ~Block() {
+    if (ptr) rt_free(ctx, ptr);
+  }
+  float* release() { return std::exchange(ptr, nullptr); }
+  void to(DeviceBuffer* b) {
+    b->ptr = release();
+    b->drop_node();
+  }
+};
 inline int unary_entry(uint8_t op) {  // the stand-alone kernel of an op, or -1
   switch (op) {
     case RT_F_RELU: return RT_RELU;
@@ -716,7 +731,8 @@ inline bool evaluate_alone(DeviceBuffer* b) {
   rt_ctx* c = b->ctx;
   const int u = n.kind == Kind::Unary ? unary_entry(n.op) : -1, bi = n.kind == Kind::Binary ? binary_entry(n.op) : -1;
   if ((n.kind == Kind::Unary && u < 0) || (n.kind == Kind::Binary && bi < 0) || n.kind == Kind::BinaryImm) return false;
-  float* out = new_block(c, b->numel);
+  Block block(c, b->numel);
+  float* out = block.ptr;
   auto nd = dims64(n.shape);
   rt_status st = RT_OK;
   auto place = [&](const Input& in, const std::vector<int64_t>& starts) {
@@ -756,12 +772,8 @@ inline bool evaluate_alone(DeviceBuffer* b) {
     }
     default: break;
   }
-  if (st != RT_OK) {
-    rt_free(c, out);
-    check(c, st);
-  }
-  b->ptr = out;
-  b->drop_node();
+  check(c, st);
+  block.to(b);
   return true;
 }
 
@@ -850,21 +862,17 @@ inline bool rewrite_linear(DeviceBuffer* b) {
   for (auto& l : all) keep.push_back(l.out->shared_from_this());
   std::vector<const float*> as;
   std::vector<float*> outs;
+  std::vector<Block> blocks;
   for (auto& l : all) {
     as.push_back(l.a.buf->data());
-    outs.push_back(new_block(b->ctx, l.out->numel));
+    blocks.emplace_back(b->ctx, l.out->numel);
+    outs.push_back(blocks.back().ptr);
   }
   rt_status st;
   if (all.size() > 1) st = rt_gemm_bias_act_list(b->ctx, (int)all.size(), as.data(), outs.data(), rows, cols, k, pb, bias, first.act);
   else st = rt_gemm_bias_act(b->ctx, rows, cols, k, pa, k, pb, cols, bias, first.act, outs[0], cols);
-  if (st != RT_OK) {
-    for (float* o : outs) rt_free(b->ctx, o);
-    check(b->ctx, st);
-  }
-  for (size_t i = 0; i < all.size(); ++i) {
-    all[i].out->ptr = outs[i];
-    all[i].out->drop_node();
-  }
+  check(b->ctx, st);
+  for (size_t i = 0; i < all.size(); ++i) blocks[i].to(all[i].out);
   return true;
 }
 
@@ -910,14 +918,9 @@ inline bool rewrite_loss(DeviceBuffer* b) {
   if (!match_loss(b, &l)) return false;
   const Input logits = *l.logits, targets = *l.targets;  // kept through the evaluations
   const float *x = logits.buf->data(), *y = targets.buf->data();
-  float* out = new_block(b->ctx, b->numel);
-  const rt_status st = rt_softmax_nll_scaled(b->ctx, x, y, l.rows, l.classes, l.scale, l.divisor, out);
-  if (st != RT_OK) {
-    rt_free(b->ctx, out);
-    check(b->ctx, st);
-  }
-  b->ptr = out;
-  b->drop_node();
+  Block out(b->ctx, b->numel);
+  check(b->ctx, rt_softmax_nll_scaled(b->ctx, x, y, l.rows, l.classes, l.scale, l.divisor, out.ptr));
+  out.to(b);
   return true;
 }
 
@@ -947,14 +950,9 @@ inline bool rewrite_pool(DeviceBuffer* b) {
     if (pg->geo[10] != (int64_t)st->in[0].buf->id) continue;                // the relu's output is what was pooled
     const auto& q = pg->geo;
     const float *y = pg->in[2].buf->data(), *g = pg->in[0].buf->data(), *idx = pg->in[1].buf->data();
-    float* out = new_block(b->ctx, b->numel);
-    const rt_status rc = rt_relu_max_pool2x2_backward_from_output(b->ctx, y, g, idx, q[0], q[1], q[2], q[3], out);
-    if (rc != RT_OK) {
-      rt_free(b->ctx, out);
-      check(b->ctx, rc);
-    }
-    b->ptr = out;
-    b->drop_node();
+    Block out(b->ctx, b->numel);
+    check(b->ctx, rt_relu_max_pool2x2_backward_from_output(b->ctx, y, g, idx, q[0], q[1], q[2], q[3], out.ptr));
+    out.to(b);
     return true;
   }
   return false;
@@ -991,15 +989,10 @@ inline bool rewrite_loss_sum(DeviceBuffer* b) {
     ys.push_back(keep[i + 1].buf->data());
   }
   for (auto& r : rest) more.push_back(r.buf->data());
-  float* out = new_block(b->ctx, 1);
-  const rt_status st = rt_softmax_nll_list(b->ctx, (int)xs.size(), xs.data(), ys.data(), first.rows, first.classes, first.scale, first.divisor,
-                                           (int)more.size(), more.data(), out);
-  if (st != RT_OK) {
-    rt_free(b->ctx, out);
-    check(b->ctx, st);
-  }
-  b->ptr = out;
-  b->drop_node();
+  Block out(b->ctx, 1);
+  check(b->ctx, rt_softmax_nll_list(b->ctx, (int)xs.size(), xs.data(), ys.data(), first.rows, first.classes, first.scale, first.divisor,
+                                    (int)more.size(), more.data(), out.ptr));
+  out.to(b);
   return true;
 }
 // Rows of a tensor that is in memory, inside a capture: no copy, the result points into it.
@@ -1047,26 +1040,15 @@ inline void lazy_evaluate(DeviceBuffer* b) {
     Compiler c;
     std::vector<DeviceBuffer*> outs;
     if (c.build(b, &p, &outs)) {
-      std::vector<float*> blocks;
-      rt_status st = RT_OK;
+      std::vector<Block> blocks;
       for (size_t k = 0; k < outs.size(); ++k) {
-        void* q = nullptr;
-        st = rt_malloc(b->ctx, sizeof(float) * std::max<size_t>(b->numel, 1), &q);
-        if (st != RT_OK) break;
-        blocks.push_back((float*)q);
-        p.out[k] = (float*)q;
+        blocks.emplace_back(b->ctx, b->numel);
+        p.out[k] = blocks.back().ptr;
       }
-      if (st == RT_OK) st = rt_fused_elementwise(b->ctx, &p);
-      if (st != RT_OK) {
-        for (float* q : blocks) rt_free(b->ctx, q);
-        check(b->ctx, st);
-      }
+      check(b->ctx, rt_fused_elementwise(b->ctx, &p));
       std::vector<std::shared_ptr<DeviceBuffer>> keep;
       for (auto* o : outs) keep.push_back(o->shared_from_this());
-      for (size_t k = 0; k < outs.size(); ++k) {
-        outs[k]->ptr = blocks[k];
-        outs[k]->drop_node();
-      }
+      for (size_t k = 0; k < outs.size(); ++k) blocks[k].to(outs[k]);
       return;
     }
     // too long, or more dimensions than the kernel walks: evaluate what lies below first

@@ -80,6 +80,21 @@ rt_status rt_relu_max_pool2x2_backward_from_output(rt_ctx*, const float*, const 
   ++masked_pool_gradients;
   return RT_OK;
 }
+rt_status rt_column_sums_list(rt_ctx*, int count, const float* const* xs, const int64_t* rows, const int64_t* cols, float* const* outs) {
+  if (kernels_fail) return RT_ERR_CUDA;
+  for (int k = 0; k < count; ++k)
+    for (int64_t i = 0; i < rows[k] * cols[k]; ++i) outs[k][i % cols[k]] = (i < cols[k] ? 0.f : outs[k][i % cols[k]]) + xs[k][i];
+  return RT_OK;
+}
+rt_status rt_sum_rows_accumulate_list(rt_ctx*, int count, const float* const* xs, int64_t rows, int64_t cols, float* out) {
+  if (kernels_fail) return RT_ERR_CUDA;
+  for (int k = 0; k < count; ++k)
+    for (int64_t i = 0; i < rows * cols; ++i) out[i % cols] += xs[k][i];
+  return RT_OK;
+}
+rt_status rt_gemm_bias_act_list(rt_ctx*, int, const float* const*, float* const*, int64_t, int64_t, int64_t, const float*, const float*, int) {
+  return kernels_fail ? RT_ERR_CUDA : RT_OK;
+}
 rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of windows; results of other programs stay zero
   if (kernels_fail) return RT_ERR_CUDA;
   if (p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_OK;
@@ -162,12 +177,68 @@ void pooling_knows_its_relu() {
     EXPECT(masked_pool_gradients == (same ? 1 : 0));
   }
 }
+// A launch or an allocation that fails leaves nothing behind: no block is lost, and asking again gives the values.
+template <class F>
+void fails_and_recovers(size_t most_blocks, F ask) {
+  const size_t before = live.size();
+  for (size_t k = 0; k <= most_blocks; ++k) {
+    mallocs_left = k < most_blocks ? (int)k : -1;
+    kernels_fail = k == most_blocks;
+    bool threw = false;
+    try {
+      ask();
+    } catch (const Error&) {
+      threw = true;
+    }
+    EXPECT(threw);
+    EXPECT(live.size() == before);
+  }
+  mallocs_left = -1;
+  kernels_fail = false;
+  ask();
+}
+void errors_lose_nothing() {
+  {  // the bias gradients of several layers
+    std::vector<B::Storage> g;
+    for (int i = 0; i < 3; ++i) g.push_back(B::unbroadcast(make({2, 4}, (float)i), {4}));
+    fails_and_recovers(3, [&] { B::evaluate_column_sums({&g[0], &g[1], &g[2], &g[1]}); });
+    for (int i = 0; i < 3; ++i) EXPECT(holds(g[i], 2 * i + 4.f, 2.f));
+  }
+  for (bool shared : {false, true}) {  // terms added to a gradient, in its own block or in a new one
+    B::Storage x = make({2, 4}, 1.f), acc = make({4}, 10.f), other;
+    if (shared) other = acc;
+    B::append_terms(acc, lazy::Tag::SumRows, {B::input(x)}, {2, 4}, B::run_sum_rows);
+    fails_and_recovers(shared ? 1 : 0, [&] { acc.ptr(); });
+    EXPECT(holds(acc, 16.f, 3.f));
+    if (shared) EXPECT(holds(other, 10.f));
+  }
+  {  // at once, because the term's address has been handed out
+    B::Storage x = make({2, 4}, 1.f), acc = make({4}, 10.f);
+    B::escape(x);
+    kernels_fail = true;
+    try {
+      B::append_terms(acc, lazy::Tag::SumRows, {B::input(x)}, {2, 4}, B::run_sum_rows);
+      EXPECT(false);
+    } catch (const Error&) {
+    }
+    kernels_fail = false;
+    EXPECT(acc.buf && holds(acc, 16.f, 3.f));
+  }
+  {  // products of one layer in a list
+    const B::Storage w = make({4, 3}, 0.f);
+    std::vector<B::Storage> y;
+    for (int i = 0; i < 4; ++i) y.push_back(B::matmul(make({2, 4}, 0.f), w));
+    fails_and_recovers(4, [&] { y[0].ptr(); });
+  }
+  EXPECT(live.empty());
+}
 
 const struct {
   const char* name;
   void (*run)();
 } kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
-               {"pooling_knows_its_relu", pooling_knows_its_relu}};
+               {"pooling_knows_its_relu", pooling_knows_its_relu},
+               {"errors_lose_nothing", errors_lose_nothing}};
 
 }  // namespace
 
