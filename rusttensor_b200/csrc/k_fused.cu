@@ -234,8 +234,8 @@ rt_status launch_fused(rt_ctx* ctx, FusedParams& p, int64_t numel) {
   const int64_t cap = (int64_t)ctx->sm_count * BLOCKS * 4;
   const size_t smem = (size_t)RT_FUSED_REGS * V * THREADS * sizeof(float);
   auto kern = fused_kernel<V, VEC, THREADS, BLOCKS>;
-  static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "rt_fused_elementwise: %s", cudaGetErrorString(set));
+  static RtDeviceOnce once;
+  RT_CUDA(ctx, once([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
   rt_launch(ctx, kern, (unsigned)(tiles < cap ? tiles : cap), THREADS, smem, p);
   RT_LAUNCHED(ctx);
   return RT_OK;

@@ -246,8 +246,8 @@ template <bool TA, bool TB, class List = NoList>
 rt_status launch_small(rt_ctx* ctx, const SmallGemm& p, int splits, const List& list = List{}, int items = 1) {
   auto kern = small_gemm_kernel<TA, TB, List>;
   using S = Shape<TA, TB>;
-  static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes);
-  if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "small product: %s", cudaGetErrorString(set));
+  static RtDeviceOnce once;
+  RT_CUDA(ctx, once([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes); }));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((p.n + kBN - 1) / kBN * splits), (unsigned)((p.m + kBM - 1) / kBM * items), 1);
   cfg.blockDim = dim3(kThreads, 1, 1);

@@ -1130,21 +1130,24 @@ tc_gemm_ts_kernel(const PlainMat la, const PlainMat lb, const TsOut out, int K, 
   if (splits > 1) cluster.sync();  // nobody leaves while its partial tile may still be read
 }
 
-template <class Kernel>
-cudaError_t prepare_ts(Kernel kern) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TsSmem::total);
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+template <bool TA, bool TB>
+cudaError_t prepare_ts() {
+  static RtDeviceOnce once;
+  return once([] {
+    auto kern = tc_gemm_ts_kernel<TA, TB>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TsSmem::total);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
 }
 // How many clusters of `splits` CTAs the chip holds at a time: clusters lie within a GPC, of which not all have the same number of
 // SMs, so that fewer CTAs fit in clusters than alone.
 inline int64_t ts_clusters(rt_ctx* ctx, int splits) {
-  struct Table {
-    int n[kTsMaxSplits + 1];
-  };
-  static const Table table = [] {
-    Table t{};
-    auto kern = tc_gemm_ts_kernel<false, false>;
-    for (int i = 2; i <= kTsMaxSplits && prepare_ts(kern) == cudaSuccess; ++i) {
+  static_assert(sizeof(ctx->ts_clusters) == sizeof(int) * (kTsMaxSplits + 1), "a count for every size of cluster");
+  int current = -1;
+  if (!ctx->ts_clusters[1] && cudaGetDevice(&current) == cudaSuccess && current == ctx->device) {
+    int* n = ctx->ts_clusters;
+    n[1] = ctx->sm_count;
+    for (int i = 2; i <= kTsMaxSplits && prepare_ts<false, false>() == cudaSuccess; ++i) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
       cfg.gridDim = dim3((unsigned)i, 1, 1);
@@ -1155,21 +1158,19 @@ inline int64_t ts_clusters(rt_ctx* ctx, int splits) {
       at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
       cfg.attrs = at;
       cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&t.n[i], kern, &cfg) != cudaSuccess) {
+      if (cudaOccupancyMaxActiveClusters(&n[i], tc_gemm_ts_kernel<false, false>, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        t.n[i] = 0;
+        n[i] = 0;
       }
     }
-    return t;
-  }();
-  return splits == 1 ? ctx->sm_count : table.n[splits];
+  }
+  return splits == 1 ? ctx->sm_count : ctx->ts_clusters[splits];
 }
 
 template <bool TA, bool TB>
 rt_status launch_ts(rt_ctx* ctx, const PlainMat& la, const PlainMat& lb, const TsOut& out, int K, int outer, int splits, int kps) {
   auto kern = tc_gemm_ts_kernel<TA, TB>;
-  static const cudaError_t set = prepare_ts(kern);
-  if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "tensor-core product: %s", cudaGetErrorString(set));
+  RT_CUDA(ctx, (prepare_ts<TA, TB>()));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((out.N + kTsBN - 1) / kTsBN * splits), (unsigned)((out.M + BM - 1) / BM), (unsigned)outer);
   cfg.blockDim = dim3(kThreads, 1, 1);

@@ -494,8 +494,8 @@ template <int BN, bool SPLIT = false>
 rt_status launch(rt_ctx* ctx, const CUtensorMap& a, const CUtensorMap& b, const Params& p) {
   using C = Config<BN, SPLIT>;
   auto kern = tma_gemm_kernel<BN, SPLIT>;
-  static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::total);
-  if (set != cudaSuccess) RT_FAIL(ctx, RT_ERR_CUDA, "tensor-core product: %s", cudaGetErrorString(set));
+  static RtDeviceOnce once;
+  RT_CUDA(ctx, once([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::total); }));
   kern<<<p.tiles < ctx->sm_count ? p.tiles : ctx->sm_count, kThreads, C::total, ctx->stream>>>(a, b, p, ctx->device_status);
   RT_LAUNCHED(ctx);
   return RT_OK;

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/rt_b200.h"
+#include "device_once.cuh"
 
 struct rt_graph {
   cudaGraph_t graph = nullptr;
@@ -64,6 +65,8 @@ struct rt_ctx {
   // Unit-stride convolution weight gradients through the TMA-fed kernel with the pixels as the reduction index
   // (k_conv_dw_tc.cu); RT_B200_CONV_DW_TMA=0 keeps the general implicit-GEMM kernel.
   bool use_tma_weight_grad = true;
+  // How many clusters of 2 .. 16 CTAs of the medium products' kernel this device holds at a time ([1]: set once that is known).
+  int ts_clusters[17] = {};
   // NCCL (loaded at run time on first use)
   void* nccl_comm = nullptr;
   bool nccl_nonblocking = false;  // the communicator was created in NCCL's non-blocking mode: calls may answer "in progress"

@@ -1,5 +1,6 @@
 """Host logic of the CUDA backend that needs no GPU: tests/host/engine_checks.cpp over stubs of the C ABI."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -20,3 +21,17 @@ def checks(tmp_path_factory):
 def test_engine(checks, name):
     r = subprocess.run([checks, name], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, f"exit code {r.returncode}\n{r.stdout}{r.stderr}"
+
+
+def test_kernel_attributes_are_set_on_every_device(tmp_path):
+    """An attribute of a kernel belongs to a device: the helper that sets it sets it on each, and no source file keeps the answer in a
+    static of its own."""
+    exe, csrc = tmp_path / "device_once", os.path.join(os.path.dirname(HERE), "rusttensor_b200", "csrc")
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-I/usr/local/cuda/include", "-o", str(exe),
+                    os.path.join(HERE, "host", "device_once_checks.cpp")], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+    for name in os.listdir(csrc):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(csrc, name)) as f:
+                assert not re.search(r"static\s+(const\s+)?(cudaError_t|auto|int|bool)\s+\w+\s*=[^;]*cuda(FuncSetAttribute|Occupancy)", f.read()), name
