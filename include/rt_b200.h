@@ -265,7 +265,7 @@ rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* program);
 /* out[i, :] = src[idx[i], :] (idx: n_idx int32 row numbers in DEVICE memory): the row gather of data::get_random_batch
  * (src/data.rs:125-209), done on the device instead of through a host copy of the whole data set. */
 rt_status rt_gather_rows(rt_ctx* ctx, const float* src, int64_t rows, int64_t row_len, const int32_t* idx, int64_t n_idx, float* out);
-/* The same rows of n_src <= 8 matrices (all inputs of a step) in one launch: outs[s][i, :] = srcs[s][idx[i], :]. */
+/* The same rows of n_src matrices (all inputs of a step), eight of them a launch: outs[s][i, :] = srcs[s][idx[i], :]. */
 rt_status rt_gather_rows_list(rt_ctx* ctx, int n_src, const float* const* srcs, const int64_t* row_lens, int64_t rows, const int32_t* idx,
                               int64_t n_idx, float* const* outs);
 /* rt_gather_rows_list with the row numbers in an upload's current host buffer: they are copied to the device on its copy stream like the

@@ -603,7 +603,6 @@ struct DpTrainer {
       dataset.push_back(d);
     }
     dataset_rows = rows;
-    if (inputs.size() > 8) throw Error::invalid_op("attach_dataset: at most 8 inputs");
     if (!idx_upload) B200Backend::check(rt_upload_create(B200Backend::ctx(), sizeof(int32_t) * inputs[0].shape()[0], &idx_upload));
   }
   // Like step_pipelined, but the inputs are rows `indices` of the attached data set: 4 bytes per sample go to the device.
@@ -621,9 +620,9 @@ struct DpTrainer {
     void* hp = nullptr;
     B200Backend::check(rt_upload_host_buffer(c, idx_upload, &hp));
     for (int64_t i = 0; i < n; ++i) static_cast<int32_t*>(hp)[i] = (int32_t)indices[i];
-    const float* srcs[8];
-    float* outs[8];
-    int64_t lens[8];
+    std::vector<const float*> srcs(inputs.size());
+    std::vector<float*> outs(inputs.size());
+    std::vector<int64_t> lens(inputs.size());
     for (size_t i = 0; i < inputs.size(); ++i) {
       auto& x = inputs[i];
       B200Backend::make_unique(x.data_mut());
@@ -631,7 +630,7 @@ struct DpTrainer {
       outs[i] = x.data().ptr();
       lens[i] = (int64_t)(x.size() / (size_t)batch);
     }
-    B200Backend::check(rt_upload_gather_rows(c, idx_upload, (int)inputs.size(), srcs, lens, dataset_rows, n, outs));
+    B200Backend::check(rt_upload_gather_rows(c, idx_upload, (int)inputs.size(), srcs.data(), lens.data(), dataset_rows, n, outs.data()));
     replay();
     exchange_and_update();
     B200Backend::check(rt_publish_to_host(c, pipe_loss[k], captured_loss.data().ptr(), 1));

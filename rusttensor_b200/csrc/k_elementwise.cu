@@ -1040,7 +1040,7 @@ rt_status rt_concat_list(rt_ctx* ctx, int count, const float* const* srcs, const
 rt_status rt_gather_rows_list(rt_ctx* ctx, int n_src, const float* const* srcs, const int64_t* row_lens, int64_t rows, const int32_t* idx,
                               int64_t n_idx, float* const* outs) {
   RT_CHECK_CTX(ctx);
-  if (n_src < 1 || n_src > kGatherSources) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_gather_rows_list: 1 to %d matrices, got %d", kGatherSources, n_src);
+  if (n_src < 1) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_gather_rows_list: one matrix or more, got %d", n_src);
   if (rows < 0 || n_idx < 0) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_gather_rows_list: negative size");
   if (n_idx == 0) return RT_OK;
   RT_CHECK_PTR(ctx, srcs);
@@ -1048,24 +1048,29 @@ rt_status rt_gather_rows_list(rt_ctx* ctx, int n_src, const float* const* srcs, 
   RT_CHECK_PTR(ctx, outs);
   RT_CHECK_PTR(ctx, idx);
   if (rows < 1 || rows >= (1ll << 31) || n_idx >= (1ll << 31)) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_gather_rows_list: size out of range");
-  GatherList g{};
   for (int s = 0; s < n_src; ++s) {
     if (row_lens[s] < 0 || row_lens[s] >= (1ll << 31)) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_gather_rows_list: bad row length");
     if (row_lens[s] == 0) continue;
     RT_CHECK_PTR(ctx, srcs[s]);
     RT_CHECK_PTR(ctx, outs[s]);
-    g.src[g.n_src] = srcs[s];
-    g.out[g.n_src] = outs[s];
-    g.row_len[g.n_src++] = row_lens[s];
   }
-  if (g.n_src == 0) return RT_OK;
   // two blocks per SM before a block gets a second row
-  int64_t per = n_idx / (2 * (int64_t)ctx->sm_count);
-  g.rows_per_block = (int)(per < 1 ? 1 : (per > kGatherRows ? kGatherRows : per));
-  g.rows = rows;
-  g.n_idx = n_idx;
-  rt_launch(ctx, gather_list_kernel, (unsigned)((n_idx + g.rows_per_block - 1) / g.rows_per_block), kThreads, 0, g, idx);
-  RT_LAUNCHED(ctx);
+  const int64_t per = n_idx / (2 * (int64_t)ctx->sm_count);
+  for (int s = 0; s < n_src;) {  // kGatherSources matrices a launch
+    GatherList g{};
+    for (; s < n_src && g.n_src < kGatherSources; ++s) {
+      if (row_lens[s] == 0) continue;
+      g.src[g.n_src] = srcs[s];
+      g.out[g.n_src] = outs[s];
+      g.row_len[g.n_src++] = row_lens[s];
+    }
+    if (g.n_src == 0) break;
+    g.rows_per_block = (int)(per < 1 ? 1 : (per > kGatherRows ? kGatherRows : per));
+    g.rows = rows;
+    g.n_idx = n_idx;
+    rt_launch(ctx, gather_list_kernel, (unsigned)((n_idx + g.rows_per_block - 1) / g.rows_per_block), kThreads, 0, g, idx);
+    RT_LAUNCHED(ctx);
+  }
   return RT_OK;
 }
 

@@ -63,6 +63,24 @@ def test_gather_rows_list(api, n_idx):
     api.call("upload_destroy", up)
 
 
+@pytest.mark.parametrize("n_src", [8, 9, 17])  # a launch takes eight; one of them is empty
+def test_gather_rows_of_many_matrices(api, n_src):
+    r = np.random.default_rng(n_src)
+    rows, n_idx, lens = 61, 40, [(3 * i) % 29 for i in range(n_src)]
+    data, pick = [r.random((rows, n), dtype=np.float32) for n in lens], r.integers(0, rows, n_idx)
+    src, dst = [api.to_device(d) if d.size else None for d in data], [api.to_device(np.ones((n_idx, n), np.float32)) if n else None for n in lens]
+    up, p = C.c_void_p(), C.c_void_p()
+    api.call("upload_create", C.c_size_t(4 * n_idx), C.byref(up))
+    api.call("upload_host_buffer", up, C.byref(p))
+    np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_int32)), (n_idx,))[:] = pick
+    ptrs = lambda ts: (C.c_void_p * n_src)(*[t.ptr.value if t else None for t in ts])  # noqa: E731
+    api.call("upload_gather_rows", up, n_src, ptrs(src), (C.c_int64 * n_src)(*lens), C.c_int64(rows), C.c_int64(n_idx), ptrs(dst))
+    for d, o in zip(data, dst):
+        if o:
+            np.testing.assert_array_equal(d[pick], o.numpy())
+    api.call("upload_destroy", up)
+
+
 @pytest.mark.parametrize("outer,lens", [(1, [5]), (1, [4] * 300), (7, [3, 0, 8, 129]), (3, [4, 2000, 16])])  # more pieces than a launch takes
 def test_concat_list(api, outer, lens):
     r = np.random.default_rng(len(lens))
