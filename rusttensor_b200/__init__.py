@@ -67,9 +67,9 @@ def engine(device=None):
     """The autograd engine on the CUDA backend: ``engine().tensor(...)``, ``engine().ops.add(...)`` ..."""
     global _engine
     if _engine is None:
-        from .frontend import Engine
+        from .fast import FastEngine
 
-        _engine = Engine(init(device), "rth")
+        _engine = FastEngine(init(device), "rth")
     return _engine
 
 

@@ -5,18 +5,13 @@ oracle (prefix ``orc``), so a test builds one graph on both and compares, which
 is the scheme of the reference's differential tests
 (tests/ops_cuda_backward_tests.rs:74-144).  Names follow the reference's public
 API: ``ops.add``, ``Tensor.backward``, ``Tensor.grad``, ``Adam.step`` ...
+
+``fast.py`` derives the CUDA library's engine from this one, with the most
+frequent calls in an extension; this module itself loads no native code.
 """
 import ctypes as C
 
 import numpy as np
-
-try:
-    from ._fastcall import Calls, TensorBase
-except ImportError:  # not built yet; needs only a host compiler
-    from ._build import build_fastcall
-
-    build_fastcall()
-    from ._fastcall import Calls, TensorBase
 
 _i64p = C.POINTER(C.c_int64)
 _f32p = C.POINTER(C.c_float)
@@ -49,8 +44,8 @@ def _f64(values):
     return arr
 
 
-class Tensor(TensorBase):
-    """``engine``, ``handle`` and ``grad`` come from the base; so does the release of the handle."""
+class Tensor:
+    """What all tensors share.  The engine's own type adds ``engine``, ``handle``, ``grad`` and the release of the handle."""
 
     @property
     def shape(self):
@@ -91,6 +86,28 @@ class Tensor(TensorBase):
 
     def broadcast_to(self, shape):
         return self.engine.ops.broadcast_to(self, shape)
+
+
+class CtypesTensor(Tensor):
+    def __init__(self, engine, handle):
+        self.engine = engine
+        self.handle = handle
+
+    def __del__(self):
+        try:
+            self.engine._call("tensor_free", C.c_int64(self.handle))
+        except Exception:
+            pass
+
+    @property
+    def grad(self):
+        has = C.c_int(0)
+        self.engine._call("tensor_has_grad", C.c_int64(self.handle), C.byref(has))
+        if not has.value:
+            return None
+        out = C.c_int64(0)
+        self.engine._call("tensor_grad", C.c_int64(self.handle), C.byref(out))
+        return self.engine._tensor(out.value)
 
 
 class _Ops:
@@ -169,7 +186,7 @@ class Optimizer:
     def state(self, which, idx):
         out = C.c_int64(0)
         self.engine._call("optim_state", C.c_int64(self.handle), C.c_int(which), C.c_int(idx), C.byref(out))
-        return Tensor(self.engine, out.value)
+        return self.engine._tensor(out.value)
 
 
 class Trainer:
@@ -186,7 +203,7 @@ class Trainer:
         for i in range(n.value):
             h = C.c_int64(0)
             engine._call("trainer_param", C.c_int64(self.handle), C.c_int(i), C.byref(h))
-            self.params.append(Tensor(engine, h.value))
+            self.params.append(engine._tensor(h.value))
 
     def __del__(self):
         try:
@@ -201,7 +218,7 @@ class Trainer:
         out = C.c_int64(0)
         self.engine._call("trainer_run", C.c_int64(self.handle), _i64([t.handle for t in inputs]),
                           C.c_int(len(inputs)), C.c_int(mode), C.byref(out))
-        return Tensor(self.engine, out.value)
+        return self.engine._tensor(out.value)
 
     def forward(self, inputs):
         return self._run(inputs, 0)
@@ -218,17 +235,21 @@ class Trainer:
     def optim_state(self, which, idx):
         out = C.c_int64(0)
         self.engine._call("trainer_optim_state", C.c_int64(self.handle), C.c_int(which), C.c_int(idx), C.byref(out))
-        return Tensor(self.engine, out.value)
+        return self.engine._tensor(out.value)
 
 
 class Engine:
+    tensor_type = CtypesTensor
+
     def __init__(self, lib, prefix):
         self.lib = lib
         self.prefix = prefix
         self.ops = _Ops(self)
         self._fns = {}
-        self._calls = Calls(*[C.cast(getattr(lib, f"{prefix}_{n}"), C.c_void_p).value for n in ("op", "tensor_free", "tensor_has_grad", "tensor_grad")])
         getattr(lib, f"{prefix}_last_error").restype = C.c_char_p
+
+    def _tensor(self, handle):
+        return self.tensor_type(self, handle)
 
     def _call(self, name, *args):
         fn = self._fns.get(name)
@@ -256,7 +277,7 @@ class Engine:
         out = C.c_int64(0)
         self._call("tensor_from_host", a.ctypes.data_as(_f32p), _i64(shape), C.c_int(len(shape)),
                    C.c_int(1 if requires_grad else 0), C.byref(out))
-        return Tensor(self, out.value)
+        return self._tensor(out.value)
 
     # ---- random factories (Backend::random_uniform / random_normal / bernoulli / kaiming_uniform, src/backend/mod.rs:57-69) ----
     def manual_seed(self, seed):
@@ -282,24 +303,27 @@ class Engine:
         ox, oy = C.c_int64(0), C.c_int64(0)
         self._call("get_batch", C.c_int64(x.handle), C.c_int64(y.handle), _i64(indices), C.c_int(len(indices)), C.c_int64(0),
                    C.c_uint64(0), C.byref(ox), C.byref(oy))
-        return Tensor(self, ox.value), Tensor(self, oy.value)
+        return self._tensor(ox.value), self._tensor(oy.value)
 
     def get_random_batch(self, x, y, batch_size, seed=0):
         """``batch_size`` distinct random rows of x and y (sampling without replacement, seeded)."""
         ox, oy = C.c_int64(0), C.c_int64(0)
         self._call("get_batch", C.c_int64(x.handle), C.c_int64(y.handle), _i64([]), C.c_int(0), C.c_int64(int(batch_size)),
                    C.c_uint64(int(seed)), C.byref(ox), C.byref(oy))
-        return Tensor(self, ox.value), Tensor(self, oy.value)
+        return self._tensor(ox.value), self._tensor(oy.value)
 
     def op(self, name, inputs, ip=(), fp=()):
-        return self._calls.op(Tensor, self, name, inputs, ip, fp)
+        out = C.c_int64(0)
+        self._call("op", name.encode(), _i64([t.handle for t in inputs]), C.c_int(len(inputs)),
+                   _i64(ip), C.c_int(len(ip)), _f64(fp), C.c_int(len(fp)), C.byref(out))
+        return self._tensor(out.value)
 
     def op_backward(self, output, grad):
         """Calls the backward closure of the op that produced ``output`` with ``grad`` directly."""
         outs = (C.c_int64 * 16)()
         n = C.c_int(0)
         self._call("op_backward", C.c_int64(output.handle), C.c_int64(grad.handle), outs, C.c_int(16), C.byref(n))
-        return [Tensor(self, outs[i]) for i in range(n.value)]
+        return [self._tensor(outs[i]) for i in range(n.value)]
 
     def Sgd(self, params, lr):
         return Optimizer(self, 0, params, [lr])

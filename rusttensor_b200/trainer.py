@@ -8,8 +8,7 @@ import ctypes as C
 
 import numpy as np
 
-from .frontend import Tensor, EngineError, _i64, _f64
-from . import _fastcall
+from .frontend import EngineError, _i64, _f64
 
 _f32p = C.POINTER(C.c_float)
 
@@ -19,6 +18,9 @@ class DataParallelTrainer:
         from . import engine
 
         self.engine = engine(device)
+        from . import _fastcall  # the engine has it
+
+        self._fastcall = _fastcall
         self.host = self.engine.lib
         self.rank, self.world = rank, world
         idbuf = (C.c_uint8 * 128)(*(nccl_id if nccl_id is not None else [0] * 128))
@@ -51,7 +53,7 @@ class DataParallelTrainer:
     def _tensor(self, fn, i, *extra):
         h = C.c_int64(0)
         self._call(fn, C.c_int64(self.handle), *extra, C.c_int(i), C.byref(h))
-        return Tensor(self.engine, h.value)
+        return self.engine._tensor(h.value)
 
     def __del__(self):
         try:
@@ -199,7 +201,7 @@ class DataParallelTrainer:
     def pipeline_buffer(self, i):
         """numpy view of the pinned host buffer to fill with input ``i`` of the NEXT pipelined step
         (two buffers alternate; the call waits until the copy that last read this one has finished)."""
-        rc, address = _fastcall.pointer(self._buffer_fn, self.handle, i)
+        rc, address = self._fastcall.pointer(self._buffer_fn, self.handle, i)
         if rc != 0:
             self.engine._raise(rc)
         view = self._pipeline_views.get((i, address))  # two buffers per input, for the trainer's lifetime
@@ -211,7 +213,7 @@ class DataParallelTrainer:
     def step_pipelined(self):
         """Enqueues one step from the pipeline buffers and returns the loss of the previous pipelined
         step (None for the first one): the host never waits for the step it has just enqueued."""
-        rc, loss = _fastcall.step(self._step_fn, self.handle)
+        rc, loss = self._fastcall.step(self._step_fn, self.handle)
         if rc != 0:
             self.engine._raise(rc)
         return loss
@@ -242,7 +244,7 @@ class DataParallelTrainer:
     def loss_tensor(self):
         h = C.c_int64(0)
         self._call("dp_loss_tensor", C.c_int64(self.handle), C.byref(h))
-        return Tensor(self.engine, h.value)
+        return self.engine._tensor(h.value)
 
     def graph_nodes(self):
         n = C.c_int64(0)

@@ -159,3 +159,20 @@ def test_data_parallel_gradient_mean_equals_global_batch_on_two_gloo_ranks(tmp_p
 
     res = json.loads(line.split(" ", 1)[1])
     assert res["err"] <= 1e-5 * max(res["scale"], 1.0), res
+
+
+def test_the_oracle_runs_without_the_product_s_native_code():
+    """The CPU restatement is what the product is measured against: its engine, through the same Python classes, loads none of the
+    package's own libraries."""
+    code = ("import numpy as np, oracle\n"
+            "e = oracle.engine()\n"
+            "w = e.tensor(np.ones((3, 2)), requires_grad=True)\n"
+            "e.ops.mean(e.ops.matmul(e.tensor(np.ones((4, 3))), w)).backward()\n"
+            "assert w.grad.shape == (3, 2) and e.Sgd([w], 0.1).step() is None and w.grad.grad is None\n"
+            "from rusttensor_b200.workloads import setup_trainer, workload_data\n"
+            "params, inputs = workload_data(1, [6, 12, 8, 4], seed=0)\n"
+            "setup_trainer(e, 1, [6, 12, 8, 4], params).step([e.tensor(a) for a in inputs]).numpy()\n"
+            "import rusttensor_b200\n"
+            "print([l.split()[-1] for l in open('/proc/self/maps') if 'rusttensor_b200' in l and l.strip().endswith('.so')])\n")
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT)
+    assert out.returncode == 0 and out.stdout.strip() == "[]", out.stdout + out.stderr
