@@ -328,8 +328,9 @@ struct B200Backend {
     const Storage& x = o.inputs[0].data();
     if (x.shape != g.shape) throw Error::shape_mismatch(x.shape, g.shape);
     if (deferrable(x.shape)) {  // g * f'(x), each f' in the form of the stand-alone kernel
-      // where f' follows from f(x), which the forward pass has (unless x has been changed since)
-      if (o.cached_outputs && o.cached_outputs->buf && o.cached_outputs->buf->made_from == x.buf->id && (!x.buf->escaped || lazy::capturing())) {
+      // where f' follows from f(x), which the forward pass has (unless x or the result may have been changed since)
+      if (o.cached_outputs && o.cached_outputs->buf && o.cached_outputs->buf->made_from == x.buf->id &&
+          ((!x.buf->escaped && !o.cached_outputs->buf->escaped) || lazy::capturing())) {
         const Storage& y = *o.cached_outputs;
         switch (op) {
           case RT_RELU: return lz_mul(g, lz_unary(RT_F_STEP, y));
@@ -929,10 +930,13 @@ struct B200Backend {
     DeviceBuffer* b = acc.buf.get();
     if (b->node && b->node->tag == tag && b->node->geo == geo && acc.buf.use_count() == 1 && b->readers.empty() &&
         b->node->in.size() + term.size() <= 1 + kMaxTerms) {
+      bool now = false;
       for (auto& t : term) {
+        now = now || (t.buf->escaped && !lazy::capturing());
         t.buf->readers.push_back(b);
         b->node->in.push_back(std::move(t));
       }
+      if (now) b->data();
       return;
     }
     acc.buf->data();

@@ -232,13 +232,44 @@ void errors_lose_nothing() {
   }
   EXPECT(live.empty());
 }
+// What has been handed out may be written at any time: a gradient does not count on a forward result whose address is known outside,
+// and a term that joins others is added on the spot.
+bool reads(const DeviceBuffer* b, const DeviceBuffer* of) {
+  if (b == of) return true;
+  if (b->node)
+    for (auto& i : b->node->in)
+      if (reads(i.buf.get(), of)) return true;
+  return false;
+}
+void written_from_outside() {
+  for (int op : {RT_RELU, RT_EXP, RT_TANH, RT_SIGMOID})
+    for (bool known : {false, true}) {
+      B::Storage x = make({2, 3}, 1.f), y = B::unary(op, x);
+      Op<B> o(OpType(OpType::Relu), {Tensor<B>(x, true)}, nullptr);
+      o.cached_outputs = y;
+      y.buf->drop_node();  // as if it had been computed
+      y.buf->ptr = lazy::Block(B::ctx(), 6).release();
+      if (known) B::escape(y);
+      B::Storage d = B::unary_bwd(op, o, make({2, 3}, 1.f));
+      EXPECT(reads(d.buf.get(), y.buf.get()) == !known);
+      EXPECT(reads(d.buf.get(), x.buf.get()) == known);
+    }
+  B::Storage a = make({2, 4}, 1.f), b = make({2, 4}, 1.f), acc = make({4}, 10.f);
+  float* p = B::escape(b);
+  B::append_terms(acc, lazy::Tag::SumRows, {B::input(a)}, {2, 4}, B::run_sum_rows);
+  EXPECT(acc.buf->node != nullptr);
+  B::append_terms(acc, lazy::Tag::SumRows, {B::input(b)}, {2, 4}, B::run_sum_rows);
+  scribble(p, 8);
+  EXPECT(holds(acc, 22.f, 5.f));
+}
 
 const struct {
   const char* name;
   void (*run)();
 } kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"pooling_knows_its_relu", pooling_knows_its_relu},
-               {"errors_lose_nothing", errors_lose_nothing}};
+               {"errors_lose_nothing", errors_lose_nothing},
+               {"written_from_outside", written_from_outside}};
 
 }  // namespace
 
