@@ -73,7 +73,7 @@ struct B200Backend {
   // ---- deferred elementwise ops (lazy.hpp) --------------------------------------------------------------------------
   static bool deferrable(const Shape& s) {
     const size_t n = shape_numel(s);
-    return n > 0 && n < ((size_t)1 << 31) && s.size() <= (size_t)lazy::kMaxRawDims;
+    return lazy::deferring() && n > 0 && n < ((size_t)1 << 31) && s.size() <= (size_t)lazy::kMaxRawDims;
   }
   static Storage defer(lazy::Node n, const Shape& shape) {
     bool now;

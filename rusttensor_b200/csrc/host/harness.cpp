@@ -702,6 +702,15 @@ int rth_sync() {
   });
 }
 
+// Diagnostic: 0 runs every op at once by its own kernel, 1 (the state at the start) defers elementwise ops and what may join them.
+// Belongs to the engine of rth_init; not while a step is being captured, and not between steps of a captured trainer.
+int rth_set_deferred_ops(int on) {
+  return rt::capi::guarded<B200Backend>([&](auto&) {
+    rt::lazy::flush_all();
+    rt::lazy::deferring() = on != 0;
+  });
+}
+
 // Device pointer of a tensor's data (for calling the raw C ABI on engine tensors).
 int rth_tensor_device_ptr(int64_t h, void** out) {
   return rt::capi::guarded<B200Backend>([&](auto& r) { *out = B200Backend::escape(r.get(h).data()); });

@@ -150,6 +150,11 @@ inline bool& capturing() {
   static bool c = false;
   return c;
 }
+// Off: every op runs at once by its own kernel, as tensors of 2^31 and more elements always do (rth_set_deferred_ops).
+inline bool& deferring() {
+  static bool d = true;
+  return d;
+}
 inline void flush_all() {
   while (DeviceBuffer::head()) lazy_evaluate(DeviceBuffer::head());
 }
