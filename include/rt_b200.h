@@ -115,6 +115,8 @@ rt_status rt_event_synchronize(rt_ctx* ctx, rt_event* ev);
 void* rt_stream(rt_ctx* ctx);                                                        /* the cudaStream_t */
 rt_status rt_mem_stats(rt_ctx* ctx, int64_t* bytes_reserved, int64_t* bytes_in_use, int64_t* n_device_allocs);
 rt_status rt_kernel_launch_count(rt_ctx* ctx, int64_t* launches);                    /* kernels launched by this library so far */
+/* Launches of rt_fused_elementwise so far, by what ran the program: a kernel compiled for it, or the interpreter. */
+rt_status rt_fused_launch_counts(rt_ctx* ctx, int64_t* compiled, int64_t* interpreted);
 /* Synchronises and reads the device error word: kernels that wait on barriers give up after a bounded
  * number of polls, record a code there and return; non-zero -> RT_ERR_TIMEOUT (and the word is cleared). */
 rt_status rt_device_status(rt_ctx* ctx, int* code);

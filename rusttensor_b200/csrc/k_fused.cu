@@ -328,7 +328,11 @@ extern "C" rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* f
   for (int k = 0; k < f->n_regions; ++k) p.region[k] = f->region[k];
   for (int i = 0; i < f->n_code; ++i) p.code[i] = encode(f->code[i]);
   if (p.nd <= 2)
-    if (const KnownProgram* k = find_known(p)) return k->launch(ctx, p, vec && regions_in_quads(p), numel);
+    if (const KnownProgram* k = find_known(p)) {
+      ctx->fused_compiled++;
+      return k->launch(ctx, p, vec && regions_in_quads(p), numel);
+    }
+  ctx->fused_interpreted++;
   // Eight elements per thread halve the decoding per element, four give twice the warps: the line lies where eight still fill
   // every SM with its 512 threads.
   const bool wide = numel >= (int64_t)ctx->sm_count * 512 * 8;

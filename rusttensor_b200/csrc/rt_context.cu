@@ -209,6 +209,15 @@ rt_status rt_kernel_launch_count(rt_ctx* ctx, int64_t* launches) {
   return RT_OK;
 }
 
+rt_status rt_fused_launch_counts(rt_ctx* ctx, int64_t* compiled, int64_t* interpreted) {
+  RT_CHECK_CTX(ctx);
+  RT_CHECK_PTR(ctx, compiled);
+  RT_CHECK_PTR(ctx, interpreted);
+  *compiled = ctx->fused_compiled;
+  *interpreted = ctx->fused_interpreted;
+  return RT_OK;
+}
+
 rt_status rt_memcpy_h2d(rt_ctx* ctx, void* dst, const void* src, size_t bytes) {
   RT_CHECK_CTX(ctx);
   if (bytes == 0) return RT_OK;

@@ -33,7 +33,7 @@ struct rt_ctx {
   std::multimap<size_t, void*> free_blocks;
   std::map<void*, size_t> live_blocks;
   int64_t bytes_reserved = 0, bytes_in_use = 0, n_device_allocs = 0;
-  int64_t launches = 0;
+  int64_t launches = 0, fused_compiled = 0, fused_interpreted = 0;
   bool capturing = false;
   // Destroyed uploads (at most kIdleUploads of kIdleUploadBytes in all) and small pinned blocks (at most kIdleHostBlocks) wait here for
   // the next owner: pinning memory and creating a stream cost milliseconds, which the first step of every new trainer paid.

@@ -116,3 +116,23 @@ def test_classification_loss_with_gradient(rows, classes):
         want = -(t - np.exp(ls) * t.sum(1, keepdims=True, dtype=np.float64)) / rows
         np.testing.assert_allclose(grad.numpy(), want, rtol=1e-4, atol=2e-6 * np.abs(want).max() + 1e-9)
     api.close()
+
+
+# A changed order of a program's instructions or registers would miss every compiled program without a wrong value: the steps of the
+# workloads have to find theirs.  The recurrent one is not covered as a whole: its first and last timesteps are interpreted.
+@pytest.mark.parametrize("config,dims,interpreted", [(1, [64, 784, 128, 10], 0), (101, [7, 13, 5, 3], 0), (2, [33, 57], 0), (2, [1100, 1000], 0),
+                                                     (3, [16, 28, 32, 64, 128, 10], 0), (103, [5, 8, 3, 4, 7, 3], 0), (4, [2, 3, 6, 5], 0),
+                                                     (104, [8, 64, 56, 128], 0), (5, [50, 200, 60, 30], 8), (105, [50, 200, 60, 30], 8)])
+def test_the_workloads_find_their_compiled_programs(capi, config, dims, interpreted):
+    import rusttensor_b200
+
+    def counts():
+        n = C.c_int64(0), C.c_int64(0)
+        capi.call("fused_launch_counts", C.byref(n[0]), C.byref(n[1]))
+        return n[0].value, n[1].value
+
+    tr = rusttensor_b200.DataParallelTrainer(config, dims)
+    before = counts()
+    tr.capture()
+    found, missed = (b - a for a, b in zip(before, counts()))
+    assert missed <= interpreted and found >= (3 * dims[2] if config % 100 == 5 else 1), (found, missed)
