@@ -561,7 +561,7 @@ struct DpTrainer {
   // returns the loss of the PREVIOUS pipelined step (its work finished while this one was being enqueued).
   bool step_pipelined(float* prev_loss) {
     loss_setup();
-    upload_setup();
+    if (!inputs.empty()) upload_setup();
     if (!graph) capture();
     rt_ctx* c = B200Backend::ctx();
     // all inputs in one copy and one staging -> tensor kernel, the loss by a store to pinned memory: no copy-engine round trip
@@ -577,7 +577,7 @@ struct DpTrainer {
       B200Backend::make_unique(inputs[i].data_mut());
       d[i] = inputs[i].data().ptr();
     }
-    B200Backend::check(rt_upload_submit_parts(c, upload, (int)inputs.size(), upload_at.data(), upload_bytes.data(), d));
+    if (!inputs.empty()) B200Backend::check(rt_upload_submit_parts(c, upload, (int)inputs.size(), upload_at.data(), upload_bytes.data(), d));
     replay();
     exchange_and_update();
     const int k = (int)(pipe_steps & 1);
@@ -594,6 +594,7 @@ struct DpTrainer {
   // ---- steps fed from a data set that lives on the device ----
   void attach_dataset(const float* const* host_arrays, int n_arrays, int64_t rows) {
     if (n_arrays != (int)inputs.size()) throw Error::invalid_op("attach_dataset: one array per input");
+    if (inputs.empty()) throw Error::invalid_op("attach_dataset: the step has no inputs");
     if (rows <= 0 || rows >= (1ll << 31)) throw Error::invalid_op("attach_dataset: row count out of range");
     dataset.clear();
     for (int i = 0; i < n_arrays; ++i) {

@@ -1,6 +1,8 @@
 """The five benchmark workloads: CUDA backend vs CPU oracle on the same seeded inputs.
 Gradients, updated parameters and optimizer state within 1e-4 (max-abs-rel with the documented
 floor for near-zero sums)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -211,6 +213,22 @@ def test_pipelined_steps_equal_plain_steps(gpu_engine):
     assert got == ref
     for a, b in zip(plain.params, piped.params):
         assert np.array_equal(a.numpy(), b.numpy())
+
+
+def test_pipelined_steps_without_inputs(gpu_engine):
+    """A workload whose operands are all parameters has nothing to upload; its steps are pipelined all the same."""
+    dims = [33, 57]
+    params, _ = workload_data(2, dims, seed=0)
+    tr = rusttensor_b200.DataParallelTrainer(2, dims)
+    for t, p in zip(tr.params, params):
+        t.update_from_host(p)
+    assert tr.step_pipelined() is None
+    losses = [tr.step_pipelined(), tr.step_pipelined(), tr.pipeline_flush()]
+    x, b = (p.astype(np.float64) for p in params)
+    y = np.tanh(x * b) + np.exp(-x * x) + np.sin(x) / (x * x + 1)
+    np.testing.assert_allclose(losses, np.log(np.exp(y).sum(1)).sum(), rtol=1e-5)
+    with pytest.raises(Exception, match="no inputs"):
+        tr._call("dp_attach_dataset", C.c_int64(tr.handle), None, C.c_int(0), C.c_int64(5))
 
 
 @pytest.mark.parametrize("config", [1, 3, 4, 5])
