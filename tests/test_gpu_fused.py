@@ -67,6 +67,26 @@ def test_operands_changed_in_place_after_the_op(engines, shape):
         assert_close(got.numpy(), ref.numpy())
 
 
+@pytest.mark.parametrize("written", ["base", "slice", "slice of a slice"])
+def test_rows_and_their_base_written_through_a_device_pointer(capi, written):
+    import rusttensor_b200
+
+    e, data = rusttensor_b200.engine(), np.arange(24, dtype=np.float32).reshape(6, 4)
+    x = e.tensor(data)
+    y = e.ops.slice(x, [(1, 5), (0, 4)])
+    y.numpy()
+    w = e.ops.slice(y, [(2, 3), (0, 4)])
+    w.numpy()
+    z = e.ops.square(y)  # not asked for before the write
+    tensors = {"base": x, "slice": y, "slice of a slice": w}
+    p, other = C.c_void_p(), np.full(tensors[written].shape, -77, np.float32)
+    e._call("tensor_device_ptr", C.c_int64(tensors[written].handle), C.byref(p))
+    capi.call("memcpy_h2d", p, other.ctypes.data_as(C.c_void_p), C.c_size_t(other.nbytes))
+    for name, want in (("base", data), ("slice", data[1:5]), ("slice of a slice", data[3:4])):
+        np.testing.assert_array_equal(tensors[name].numpy(), other if name == written else want)
+    np.testing.assert_array_equal(z.numpy(), data[1:5] ** 2)
+
+
 @pytest.mark.parametrize("rows,classes", [(1, 2), (7, 16), (33, 17), (64, 65), (5, 300)])
 @pytest.mark.parametrize("steps", [1, 2, 205])
 def test_losses_of_a_sequence(engines, rows, classes, steps):
