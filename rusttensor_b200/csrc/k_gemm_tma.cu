@@ -11,9 +11,9 @@
 // the error grows to 2.9e-5 of the result at 4096.  An accumulator is therefore emptied after every K-block of 32, or every
 // few, and these are summed in registers with rounding (error 3.5e-7 - 1e-6 whatever the length); accumulators are used in turn, so
 // that the MMAs do not wait for it.
-// Roles of a CTA (one per SM, walking over tiles): one TMA warp several K-blocks ahead; four converter warps (A raw -> tensor
-// memory hi / lo; B raw -> B lo at the same swizzled address, so the swizzle needs no decoding); one MMA warp; eight accumulating
-// warps, which also write the result.
+// Roles of a CTA (one per SM, walking over tiles): one TMA warp several K-blocks ahead; six converter warps (A raw -> tensor
+// memory hi / lo; B raw -> B lo at the same swizzled address, so the swizzle needs no decoding), four of them at work where B comes
+// already split; one MMA warp; eight accumulating warps, which also write the result.
 // Measured: 4096^3 0.66 ms = 208 TFLOP/s of fp32-equivalent work, before 0.92 - 1.37 ms; 1024^3 31 us, before 40 - 45 us.  Without the
 // conversions (in a copy made for timing) the MMAs and copies alone take 0.43 ms: shared memory is what is full.
 // A operand: a matrix with the reduction contiguous, one with the rows contiguous, or the pixels of a channels-last image at one
