@@ -219,7 +219,7 @@ class Tensor {
     if (ds != gs) throw Error::incompatible("add_grad on Tensor ID " + std::to_string(id()), ds, gs);
     if (inner->grad) {
       if constexpr (KeepsOutputs<B>::value) {  // a backend that defers work may join this contribution to earlier ones
-        inner->grad = B::accumulate(std::move(*inner->grad), g);
+        B::accumulate(*inner->grad, g);
         return;
       }
       Storage existing = *inner->grad;

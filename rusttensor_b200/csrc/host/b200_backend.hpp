@@ -977,15 +977,15 @@ struct B200Backend {
     }
     add_to(n, b, [&](float* out) { return rt_gemm_sum_products(ctx(), (int)as.size(), as.data(), gs.data(), n.geo[0], n.geo[1], n.geo[2], out); });
   }
-  // existing + g for a gradient that receives another contribution (Tensor::add_grad).
-  static Storage accumulate(Storage existing, const Storage& g) {
+  // existing += g for a gradient that receives another contribution (Tensor::add_grad).  After an error it is what it was.
+  static void accumulate(Storage& existing, const Storage& g) {
     const lazy::Node* n = g.buf ? g.buf->node.get() : nullptr;
     if (n && n->tag == lazy::Tag::SumRows && n->geo[0] < 0 && g.buf->readers.empty() && g.shape.size() == 1 && existing.buf && existing.shape == g.shape) {
       const lazy::Input x = n->in[0];
       append_terms(existing, lazy::Tag::SumRows, {x}, {(int64_t)x.shape[0], (int64_t)x.shape[1]}, run_sum_rows);
-      return existing;
+      return;
     }
-    return add(existing, g);
+    existing = add(existing, g);
   }
   static void run_sum_rows(lazy::Node& n, DeviceBuffer* b) {
     std::vector<const float*> xs;

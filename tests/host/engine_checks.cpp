@@ -70,6 +70,9 @@ rt_status rt_unary(rt_ctx*, int op, const float* x, float* y, int64_t n, float, 
   for (int64_t i = 0; i < n; ++i) y[i] = x[i] * x[i];
   return RT_OK;
 }
+rt_status rt_binary(rt_ctx*, int, const float*, const int64_t*, int, const float*, const int64_t*, int, float*) {
+  return kernels_fail ? RT_ERR_CUDA : RT_OK;
+}
 rt_status rt_relu_max_pool2d(rt_ctx*, const float*, int64_t, int64_t, int64_t, int64_t, int, int, int, int, int, int, float*, float*) {
   return RT_OK;
 }
@@ -223,6 +226,20 @@ void errors_lose_nothing() {
     }
     kernels_fail = false;
     EXPECT(acc.buf && holds(acc, 16.f, 3.f));
+  }
+  {  // another contribution to a gradient, likewise
+    B::Storage g = make({4}, 1.f);
+    Tensor<B> p(make({4}, 0.f), true);
+    p.set_grad(make({4}, 10.f));
+    B::escape(g);
+    kernels_fail = true;
+    try {
+      p.add_grad(g);
+      EXPECT(false);
+    } catch (const Error&) {
+    }
+    kernels_fail = false;
+    EXPECT(p.grad()->buf && holds(*p.grad(), 10.f));
   }
   {  // products of one layer in a list
     const B::Storage w = make({4, 3}, 0.f);
