@@ -858,7 +858,8 @@ inline bool rewrite_linear(DeviceBuffer* b) {
     if (!r->node || r->node->tag != Tag::Matmul || r->node->in[1].buf != first.b.buf || r->node->in[0].buf->node) continue;
     DeviceBuffer* e = epilogue_of(r, first.act, bias != nullptr);
     Linear l;
-    if (!e || e == b || !match_linear(e, &l)) continue;
+    // a product of a matrix with itself reads it twice
+    if (!e || std::any_of(all.begin(), all.end(), [e](const Linear& x) { return x.out == e; }) || !match_linear(e, &l)) continue;
     if (l.act != first.act || l.b.buf != first.b.buf || l.a.shape != first.a.shape || l.b.shape != first.b.shape || l.bias.buf != first.bias.buf) continue;
     all.push_back(l);
   }

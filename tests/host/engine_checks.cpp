@@ -280,13 +280,26 @@ void written_from_outside() {
   EXPECT(holds(acc, 22.f, 5.f));
 }
 
+// A matrix that is both operands of a product is listed twice among its readers; the product is computed once.
+void a_product_of_a_matrix_with_itself() {
+  {
+    const B::Storage x = make({3, 3}, 1.f), y = make({3, 3}, 2.f);
+    std::vector<B::Storage> p{B::matmul(y, x), B::matmul(x, x), B::matmul(x, x)};
+    p[0].ptr();
+    for (auto& q : p) EXPECT(!q.buf->node);
+    EXPECT(live.size() == 5);
+  }
+  EXPECT(live.empty());
+}
+
 const struct {
   const char* name;
   void (*run)();
 } kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"pooling_knows_its_relu", pooling_knows_its_relu},
                {"errors_lose_nothing", errors_lose_nothing},
-               {"written_from_outside", written_from_outside}};
+               {"written_from_outside", written_from_outside},
+               {"a_product_of_a_matrix_with_itself", a_product_of_a_matrix_with_itself}};
 
 }  // namespace
 
