@@ -532,10 +532,7 @@ struct B200Backend {
     size_t off = shape.size() - x.shape.size();
     for (size_t i = 0; i < x.shape.size(); ++i)
       if (x.shape[i] != shape[i + off] && x.shape[i] != 1) throw Error::incompatible("broadcast", x.shape, shape);
-    if (deferrable(shape)) {
-      if (x.shape == shape) return x;
-      return lz_box(lazy::Kind::Broadcast, x, shape, {});
-    }
+    if (deferrable(shape)) return lz_box(lazy::Kind::Broadcast, x, shape, {});  // also to its own shape: a tensor of its own
     Storage y = alloc(shape);
     auto xs = dims(x.shape), os = dims(shape);
     check(rt_broadcast_to(ctx(), x.ptr(), xs.data(), (int)xs.size(), os.data(), (int)os.size(), y.ptr()));

@@ -137,6 +137,12 @@ void rows_do_not_alias() {
   }
   EXPECT(live.empty());
 }
+// A tensor broadcast to its own shape is a tensor of its own.
+void broadcast_does_not_alias() {
+  B::Storage x = make({2, 3}, 1.f), y = B::broadcast_to(x, {2, 3});
+  scribble(B::escape(y), 6);
+  EXPECT(holds(x, 1.f));
+}
 // Inside a capture rows are not copied; what a step leaves behind has a block of its own.
 void rows_in_a_capture() {
   B::Storage x = make({6, 4}, 1.f);
@@ -296,6 +302,7 @@ const struct {
   const char* name;
   void (*run)();
 } kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
+               {"broadcast_does_not_alias", broadcast_does_not_alias},
                {"pooling_knows_its_relu", pooling_knows_its_relu},
                {"errors_lose_nothing", errors_lose_nothing},
                {"written_from_outside", written_from_outside},
