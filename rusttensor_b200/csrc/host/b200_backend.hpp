@@ -1272,7 +1272,7 @@ struct B200Backend {
     const bool ng = o.inputs[0].requires_grad(), nc = o.inputs[1].requires_grad();
     if (deferrable(gates.shape) && deferrable(g.shape)) {
       const Storage og = saved_gate(o, 0, gates, c.shape, 3, RT_F_SIGMOID);
-      const bool kept = keeps(o, gates) && o.cached_outputs->buf->saved[1]->made_from == c.buf->id;
+      const bool kept = keeps(o, gates) && o.cached_outputs->buf->saved[1]->made_from == c.buf->id && (!c.buf->escaped || lazy::capturing());
       const Storage th = kept ? Storage{o.cached_outputs->buf->saved[1], c.shape} : lz_unary(RT_F_TANH, c);
       Storage dgates = ng ? to_gate(lz_mul(lz_mul(g, th), lz_unary(RT_F_LOGISTIC_SLOPE, og)), gates.shape, 3) : unused_grad(gates.shape);
       Storage dc = nc ? lz_mul(lz_mul(g, og), lz_unary(RT_F_ONE_MINUS_SQUARE, th)) : unused_grad(c.shape);

@@ -66,8 +66,8 @@ rt_status rt_memcpy_d2d(rt_ctx*, void* d, const void* s, size_t n) {
   return RT_OK;
 }
 rt_status rt_unary(rt_ctx*, int op, const float* x, float* y, int64_t n, float, float) {
-  if (kernels_fail || op != RT_SQUARE) return RT_ERR_CUDA;
-  for (int64_t i = 0; i < n; ++i) y[i] = x[i] * x[i];
+  if (kernels_fail) return RT_ERR_CUDA;
+  for (int64_t i = 0; i < n && op == RT_SQUARE; ++i) y[i] = x[i] * x[i];
   return RT_OK;
 }
 rt_status rt_binary(rt_ctx*, int, const float*, const int64_t*, int, const float*, const int64_t*, int, float*) {
@@ -277,6 +277,16 @@ void written_from_outside() {
       EXPECT(reads(d.buf.get(), y.buf.get()) == !known);
       EXPECT(reads(d.buf.get(), x.buf.get()) == known);
     }
+  for (int known : {0, 1, 2}) {  // the gradient of an LSTM cell's output takes the gate and tanh(c) that the forward pass has kept
+    const B::Storage gates = make({2, 12}, 0.f, 0.1f), c = make({2, 3}, 0.f, 0.1f), h = B::lstm_cell_h(gates, c);
+    Op<B> o(OpType(OpType::FusedLstmCellH), {Tensor<B>(gates, true), Tensor<B>(c, true)}, nullptr);
+    o.cached_outputs = h;
+    const auto gate = h.buf->saved[0], th = h.buf->saved[1];
+    if (known) B::escape(known == 1 ? gates : c);
+    const auto d = B::lstm_cell_h_backward(o, make({2, 3}, 1.f));
+    EXPECT(reads(d.second.buf.get(), gate.get()) == (known != 1));
+    EXPECT(reads(d.second.buf.get(), th.get()) == (known == 0));
+  }
   B::Storage a = make({2, 4}, 1.f), b = make({2, 4}, 1.f), acc = make({4}, 10.f);
   float* p = B::escape(b);
   B::append_terms(acc, lazy::Tag::SumRows, {B::input(a)}, {2, 4}, B::run_sum_rows);
