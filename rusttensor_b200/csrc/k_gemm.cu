@@ -26,6 +26,10 @@ float rt_gemm_small_estimate(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, bool 
 float rt_gemm_ts_estimate(rt_ctx* ctx, int64_t m, int64_t n, int64_t k);
 rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
                                int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
+rt_status rt_gemm_parts_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
+                                 int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
+rt_status rt_matmul_backward_parts_internal(rt_ctx* ctx, const float* a, const float* b, const float* g, int64_t m, int64_t k, int64_t n, float* da,
+                                            float* db, int accumulate_db);
 rt_status rt_conv_forward_tma_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y);
 rt_status rt_conv_gather_tma_internal(rt_ctx* ctx, const float* y, const float* w, const float* bias, const ConvGeom& g, int cm, float* out);
 rt_status rt_gemm_small_list_internal(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k,
@@ -650,13 +654,17 @@ extern "C" {
 //  * Tensor: tcgen05 with operands split by the producing warps (k_gemm_tc.cu); in its form for one wave of 128 x 64 tiles the
 //    reduction is split over clusters;
 //  * Tma: tcgen05 with operands fetched by TMA (k_gemm_tma.cu), no split, operands not in its form packed first;
+//  * Parts: tcgen05 with operands split into 16-bit parts by a pass beforehand (k_gemm_parts.cu);
 //  * Plain: fp32 tiles for what is left, and for everything that is too large for Small when tensor cores are off.
 // Where the 128 x 64 tiles fit one wave the estimates of the first two decide.  (Against Small alone: 512 x 133 x 405 11.4 and 8.6 us; against
 // Tensor alone: 514 x 247 x 92 8.2 and 6.6 us.)  Beyond one wave Tma is ahead (708 x 679 x 2336: 30 us, the 128 x 128 tiles of Tensor
 // 45; 948 x 920 x 3948: 54 and 84), but for short reductions (1129 x 66 x 1116: 13 and 9 us), longer ones too if it would have
 // to transpose the right operand first (1120 x 144 x 1748: 13.4 and 11.5 us).  Reductions below 32 fill no K-block: fp32, in small tiles while these come to one wave
 // (2023 x 20 x 814: 15 us in small tiles, 9 in large ones).
-enum class Route { Small, Tensor, Tma, Plain };
+enum class Route { Small, Tensor, Tma, Parts, Plain };
+// Above this many multiply-adds two more passes over the operands and two more launches are worth having MMAs of half the cost: 676 x 2102 x 41
+// 14.4 us (Tma) and 20.1 (Parts), 1598 x 1740 x 33 14.4 and 20.9, 721 x 1600 x 171 22.6 and 20.4, 2016 x 3898 x 49 45 and 31, 4096^3 670 and 368.
+constexpr int64_t kPartsWork = int64_t(1) << 27;
 static Route choose_route(rt_ctx* ctx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb) {
   const int64_t work = m * n * k;
   const bool wide = rt_aligned16(a) && rt_aligned16(b) && lda % 4 == 0 && ldb % 4 == 0;
@@ -668,7 +676,7 @@ static Route choose_route(rt_ctx* ctx, bool ta, bool tb, int64_t m, int64_t n, i
   const float ts = rt_gemm_ts_estimate(ctx, m, n, k);
   if (ts >= 0.f) return rt_gemm_small_estimate(ctx, m, n, k, wide) <= ts ? Route::Small : Route::Tensor;
   if (k < 128 || n < 48 || (k < 256 && wide && !(!ta && tb))) return Route::Tensor;
-  return Route::Tma;
+  return work >= kPartsWork ? Route::Parts : Route::Tma;
 }
 // Products that several left operands share a right one with (rt_gemm_bias_act_list) in the one-launch kernel.
 static bool small_product(int64_t m, int64_t n, int64_t k) {
@@ -677,7 +685,11 @@ static bool small_product(int64_t m, int64_t n, int64_t k) {
 static rt_status routed(rt_ctx* ctx, Route route, int ta, int tb, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
                         int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   if (route == Route::Small) return rt_gemm_small_internal(ctx, ta, tb, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
-  if (route == Route::Tma) {
+  if (route == Route::Parts) {
+    rt_status st = rt_gemm_parts_internal(ctx, ta, tb, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
+  if (route == Route::Tma || route == Route::Parts) {
     rt_status st = rt_gemm_tma_internal(ctx, ta, tb, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
@@ -801,6 +813,12 @@ rt_status rt_gemm(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, i
 static rt_status matmul_backward_impl(rt_ctx* ctx, const float* a, const float* b, const float* g, int64_t m, int64_t k, int64_t n,
                                       float* da, float* db, int accumulate_db) {
   RT_CHECK_CTX(ctx);
+  // Both large: in one call, one after the other, since either fills the chip
+  if (da && db && a && b && g && m > 0 && k > 0 && n > 0 && choose_route(ctx, true, false, k, n, m, a, k, g, n) == Route::Parts &&
+      choose_route(ctx, false, true, m, k, n, g, n, b, n) == Route::Parts) {
+    rt_status st = rt_matmul_backward_parts_internal(ctx, a, b, g, m, k, n, da, db, accumulate_db);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
   // da[M,K] = g[M,N] * b[K,N]^T ; db[K,N] (+)= a[M,K]^T * g[M,N]: independent, so db goes to the side stream
   RtFork fork(ctx, da && db);
   rt_status st = RT_OK, st2 = RT_OK;
