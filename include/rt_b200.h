@@ -115,7 +115,8 @@ rt_status rt_event_synchronize(rt_ctx* ctx, rt_event* ev);
 void* rt_stream(rt_ctx* ctx);                                                        /* the cudaStream_t */
 rt_status rt_mem_stats(rt_ctx* ctx, int64_t* bytes_reserved, int64_t* bytes_in_use, int64_t* n_device_allocs);
 rt_status rt_kernel_launch_count(rt_ctx* ctx, int64_t* launches);                    /* kernels launched by this library so far */
-/* Launches of rt_fused_elementwise so far, by what ran the program: a kernel compiled for it, or the interpreter. */
+/* Elementwise programs run so far, by what ran them: a kernel compiled for them, or the interpreter.  A program is a launch of
+ * rt_fused_elementwise, or one of the two that a timestep of rt_lstm_sequence or of its backward pass holds. */
 rt_status rt_fused_launch_counts(rt_ctx* ctx, int64_t* compiled, int64_t* interpreted);
 /* Synchronises and reads the device error word: kernels that wait on barriers give up after a bounded
  * number of polls, record a code there and return; non-zero -> RT_ERR_TIMEOUT (and the word is cleared). */
@@ -312,6 +313,15 @@ rt_status rt_lstm_cell_c_backward(rt_ctx* ctx, const float* gates, const float* 
 rt_status rt_lstm_cell_h(rt_ctx* ctx, const float* gates, const float* c, int64_t batch, int64_t hidden, float* h);
 rt_status rt_lstm_cell_h_backward(rt_ctx* ctx, const float* gates, const float* c, const float* dh, int64_t batch,
                                   int64_t hidden, float* dgates, float* dc);
+/* The recurrence of a whole sequence of such cells (examples/lstm_char_rnn_cpu.rs:98-138 for every timestep), time-major:
+ * gates_t = pre_t + h_{t-1} w, pre [steps*batch, 4*hidden] (the inputs' product and the bias), w [hidden, 4*hidden] with rows ldw floats
+ * apart; h0, c0 [batch, hidden] or NULL for zeros.  h [steps*batch, hidden]; saved: six such planes for the backward pass, sigmoid(i),
+ * sigmoid(f), tanh(g), sigmoid(o), c, tanh(c).  Backward: dgates [steps*batch, 4*hidden] = d/d pre from dh [steps*batch, hidden]; dh0, dc0
+ * may be NULL. */
+rt_status rt_lstm_sequence(rt_ctx* ctx, const float* pre, const float* w, int64_t ldw, const float* h0, const float* c0, int64_t steps,
+                           int64_t batch, int64_t hidden, float* saved, float* h);
+rt_status rt_lstm_sequence_backward(rt_ctx* ctx, const float* saved, const float* w, int64_t ldw, const float* c0, const float* dh, int64_t steps,
+                                    int64_t batch, int64_t hidden, float* dgates, float* dh0, float* dc0);
 
 /* Fused classification loss (no counterpart in the reference, whose examples spell the chain out:
  * examples/train_mnist_cpu.rs:63-97): loss[0] = -(1/rows) * sum over rows and classes of targets * log_softmax(logits).

@@ -100,7 +100,7 @@ struct OpType {
     Sigmoid, Sqrt, Tanh, Softplus, Max, Min, Prod, LogSumExp, ArgMax, ArgMin, Powf, Square,
     Maximum, Minimum, Elu, Transpose, Sin, Cos, Tan, Conv2d, MaxPool2D, Conv2DTranspose, Slice,
     Concat, ExpandDims, Squeeze, Clip, DivScalar, MulScalar,
-    FusedReluMaxPool2D, FusedSoftmaxNll, FusedLstmCellC, FusedLstmCellH, FusedConvReluMaxPool2D  // fused forward ops added beside the reference's (ops::fused_*)
+    FusedReluMaxPool2D, FusedSoftmaxNll, FusedLstmCellC, FusedLstmCellH, FusedConvReluMaxPool2D, FusedLstmSequence  // fused forward ops added beside the reference's (ops::fused_*)
   } kind;
   std::optional<size_t> axis;          // Mean/Sum/Max/Min/Prod/LogSumExp(Option), LogSoftmax/ArgMax/...
   float scalar = 0.f;                  // Elu(alpha), MulScalar, DivScalar
@@ -120,7 +120,7 @@ struct OpType {
       "Div", "Exp", "Ln", "Broadcast", "View", "Abs", "Sigmoid", "Sqrt", "Tanh", "Softplus", "Max",
       "Min", "Prod", "LogSumExp", "ArgMax", "ArgMin", "Powf", "Square", "Maximum", "Minimum", "Elu",
       "Transpose", "Sin", "Cos", "Tan", "Conv2d", "MaxPool2D", "Conv2DTranspose", "Slice", "Concat",
-      "ExpandDims", "Squeeze", "Clip", "DivScalar", "MulScalar", "FusedReluMaxPool2D", "FusedSoftmaxNll", "FusedLstmCellC", "FusedLstmCellH", "FusedConvReluMaxPool2D"};
+      "ExpandDims", "Squeeze", "Clip", "DivScalar", "MulScalar", "FusedReluMaxPool2D", "FusedSoftmaxNll", "FusedLstmCellC", "FusedLstmCellH", "FusedConvReluMaxPool2D", "FusedLstmSequence"};
     return n[(int)kind];
   }
 };
@@ -1002,6 +1002,37 @@ Tensor<B> fused_lstm_cell_h(const Tensor<B>& gates, const Tensor<B>& c) {
         auto p = B::lstm_cell_h_backward(op, g);
         return Grads<B>{std::move(p.first), std::move(p.second)};
       }));
+      t.inner->op->cached_outputs = t.data();
+    }
+    return t;
+  }
+}
+
+// The hidden states [steps * batch, H] of an LSTM over a time-major input [steps * batch, V], from zero states: what the reference's
+// char-LSTM example does timestep by timestep (examples/lstm_char_rnn_cpu.rs:98-138), gates_t = concat(x_t, h_{t-1}) w + b with w [V + H, 4H].
+template <class B>
+Tensor<B> fused_lstm_sequence(const Tensor<B>& x, const Tensor<B>& w, const Tensor<B>& b, size_t steps) {
+  const Shape xs = x.shape(), ws = w.shape();
+  if (xs.size() != 2 || ws.size() != 2 || steps == 0 || xs[0] == 0 || xs[0] % steps != 0) throw Error::invalid_op("fused_lstm_sequence expects a time-major input [steps * batch, features]");
+  const size_t H = ws[1] / 4, Bn = xs[0] / steps;
+  if (H == 0 || ws[1] != 4 * H || ws[0] != xs[1] + H) throw Error::incompatible("fused_lstm_sequence", xs, ws);
+  if (b.shape() != Shape{4 * H}) throw Error::incompatible("fused_lstm_sequence", ws, b.shape());
+  if constexpr (!HasFusedForward<B>::value) {
+    Tensor<B> h = Tensor<B>::zeros({Bn, H}, false), c = Tensor<B>::zeros({Bn, H}, false);
+    std::vector<Tensor<B>> hs;
+    for (size_t t = 0; t < steps; ++t) {
+      Tensor<B> gates = add(matmul(fused_rows_concat(x, t * Bn, (t + 1) * Bn, h), w), b);
+      c = fused_lstm_cell_c(gates, c);
+      h = fused_lstm_cell_h(gates, c);
+      hs.push_back(h);
+    }
+    return concat<B>(hs, 0);
+  } else {
+    St<B> out = B::lstm_sequence(x.data(), w.data(), b.data(), steps);
+    bool rg = x.requires_grad() || w.requires_grad() || b.requires_grad();
+    Tensor<B> t(std::move(out), rg);
+    if (rg) {
+      t.set_op(Op<B>(OpType(OpType::FusedLstmSequence), {x, w, b}, [steps](const Op<B>& op, const St<B>& g) { return B::lstm_sequence_backward(op, g, steps); }));
       t.inner->op->cached_outputs = t.data();
     }
     return t;

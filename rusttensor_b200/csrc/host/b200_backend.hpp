@@ -1285,6 +1285,53 @@ struct B200Backend {
     return {std::move(dg), std::move(dc)};
   }
 
+  // The recurrence in one kernel.  Kept for the gradient: the activated gates, the cell states and their tangents.
+  static Storage lstm_sequence(const Storage& x, const Storage& w, const Storage& b, size_t steps) {
+    const int64_t rows = (int64_t)x.shape[0], V = (int64_t)x.shape[1], H = (int64_t)w.shape[1] / 4;
+    const float *px = x.ptr(), *pw = w.ptr(), *pb = b.ptr();
+    Storage h = alloc({x.shape[0], (size_t)H}), saved = alloc({6 * x.shape[0], (size_t)H});
+    lazy::Block pre(ctx(), (size_t)(rows * 4 * H));
+    if (V > 0) {
+      check(rt_gemm_bias_act(ctx(), rows, 4 * H, V, px, V, pw, 4 * H, pb, RT_ACT_NONE, pre.ptr, 4 * H));
+    } else {
+      const int64_t bs[2] = {1, 4 * H}, os[2] = {rows, 4 * H};
+      check(rt_broadcast_to(ctx(), pb, bs, 2, os, 2, pre.ptr));
+    }
+    check(rt_lstm_sequence(ctx(), pre.ptr, pw + V * 4 * H, 4 * H, nullptr, nullptr, (int64_t)steps, rows / (int64_t)steps, H, saved.ptr(), h.ptr()));
+    h.buf->saved = {saved.buf};
+    return h;
+  }
+  static std::vector<Storage> lstm_sequence_backward(const OpB& o, const Storage& g, size_t steps) {
+    const Storage &x = o.inputs[0].data(), &w = o.inputs[1].data(), &h = *o.cached_outputs;
+    if (g.shape != h.shape) throw Error::shape_mismatch(h.shape, g.shape);
+    const int64_t rows = (int64_t)x.shape[0], V = (int64_t)x.shape[1], H = (int64_t)w.shape[1] / 4, batch = rows / (int64_t)steps;
+    const float *saved = h.buf->saved[0]->data(), *pw = w.ptr(), *px = x.ptr(), *pg = g.ptr();
+    Storage dgates = alloc({x.shape[0], w.shape[1]});
+    check(rt_lstm_sequence_backward(ctx(), saved, pw + V * 4 * H, 4 * H, nullptr, pg, (int64_t)steps, batch, H, dgates.ptr(), nullptr, nullptr));
+    std::vector<Storage> out{unused_grad(x.shape), unused_grad(w.shape), unused_grad(o.inputs[2].shape())};
+    if (o.inputs[0].requires_grad()) {
+      out[0] = alloc(x.shape);
+      if (V > 0) check(rt_gemm(ctx(), 0, 1, rows, V, 4 * H, dgates.ptr(), 4 * H, pw, 4 * H, out[0].ptr(), V, 0));
+    }
+    if (o.inputs[1].requires_grad()) {
+      out[1] = alloc(w.shape);
+      float *dx_rows = out[1].ptr(), *dh_rows = dx_rows + V * 4 * H;
+      if (V > 0) check(rt_gemm(ctx(), 1, 0, V, 4 * H, rows, px, V, dgates.ptr(), 4 * H, dx_rows, 4 * H, 0));
+      const int64_t later = rows - batch;  // every timestep but the first multiplies the weights with the state before it
+      const float* states = h.ptr();
+      lazy::Block own_states(ctx(), h.buf->escaped && !lazy::capturing() ? (size_t)(rows * H) : 1);
+      if (h.buf->escaped && !lazy::capturing()) {  // may have been written since: h = o * tanh(c) once more
+        const int64_t n[1] = {rows * H};
+        check(rt_binary(ctx(), RT_MUL, saved + 3 * rows * H, n, 1, saved + 5 * rows * H, n, 1, own_states.ptr));
+        states = own_states.ptr;
+      }
+      if (later > 0) check(rt_gemm(ctx(), 1, 0, H, 4 * H, later, states, H, dgates.ptr() + batch * 4 * H, 4 * H, dh_rows, 4 * H, 0));
+      else check(rt_fill(ctx(), dh_rows, 0.f, H * 4 * H));
+    }
+    if (o.inputs[2].requires_grad()) out[2] = unbroadcast(dgates, o.inputs[2].shape());
+    return out;
+  }
+
   // One launch for all parameters of an optimizer step.  kind as rt_optimizer_step_multi; s1 / s2: the optimizer's states.
   static void step_all(int kind, const std::vector<Storage*>& ps, const std::vector<Storage>& gs, const std::vector<Storage*>& s1,
                        const std::vector<Storage*>& s2, float lr, float b1, float b2, float eps, float momentum, size_t t) {

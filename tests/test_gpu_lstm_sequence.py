@@ -1,0 +1,79 @@
+"""The recurrence of a whole sequence in one kernel (rt_lstm_sequence and its gradient) against float64: batches and hidden sizes at the
+edges of the blocks' 16 rows and 8 / 16 units, given and zero initial states, a strided weight matrix, and sizes that run timestep by
+timestep because their blocks would not all be resident."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import rng
+
+pytestmark = pytest.mark.gpu
+
+i64 = C.c_int64
+# (steps, batch, hidden); the last two do not fit
+SIZES = [(1, 1, 1), (2, 16, 8), (5, 17, 9), (3, 15, 64), (7, 30, 200), (4, 33, 129), (9, 64, 512), (3, 8, 1000), (3, 90, 512), (2, 40, 700)]
+
+
+def sigmoid(v):
+    return 1 / (1 + np.exp(-v))
+
+
+def reference(pre, w, h, c, dh_all, steps, batch, hidden):
+    pre, w, h, c, dh_all = (v.astype(np.float64) for v in (pre, w, h, c, dh_all))
+    hs, kept = [], []
+    for t in range(steps):
+        z = pre[t * batch : (t + 1) * batch] + h @ w
+        i, f, g, o = sigmoid(z[:, :hidden]), sigmoid(z[:, hidden : 2 * hidden]), np.tanh(z[:, 2 * hidden : 3 * hidden]), sigmoid(z[:, 3 * hidden :])
+        kept.append((i, f, g, o, c))
+        c = f * c + i * g
+        h = o * np.tanh(c)
+        kept[-1] += (np.tanh(c),)
+        hs.append(h)
+    dh, dc, dz = np.zeros_like(h), np.zeros_like(h), [None] * steps
+    for t in reversed(range(steps)):
+        i, f, g, o, before, tc = kept[t]
+        d = dh + dh_all[t * batch : (t + 1) * batch]
+        dc = dc + d * o * (1 - tc * tc)
+        dz[t] = np.concatenate([dc * g * i * (1 - i), dc * before * f * (1 - f), dc * i * (1 - g * g), d * tc * o * (1 - o)], 1)
+        dc = dc * f
+        dh = dz[t] @ w.T
+    return np.concatenate(hs), np.concatenate(dz), dh, dc
+
+
+@pytest.mark.parametrize("initial", [False, True])
+@pytest.mark.parametrize("steps,batch,hidden", SIZES)
+def test_sequence_and_gradient(capi, steps, batch, hidden, initial):
+    r = rng(steps * 7 + batch + hidden)
+    ld = 4 * hidden + 4 * initial
+    pre = r.standard_normal((steps * batch, 4 * hidden)).astype(np.float32)
+    w = (r.uniform(-1, 1, (hidden, ld)) / np.sqrt(hidden)).astype(np.float32)
+    h0, c0 = (r.uniform(-1, 1, (batch, hidden)).astype(np.float32) * initial for _ in range(2))
+    dh = r.standard_normal((steps * batch, hidden)).astype(np.float32)
+    want = reference(pre, w[:, : 4 * hidden], h0, c0, dh, steps, batch, hidden)
+    d = [capi.to_device(v) for v in (pre, w, h0, c0, dh)]
+    h, saved, dgates, dh0, dc0 = (capi.empty(s) for s in ((steps * batch, hidden), (6, steps * batch, hidden), (steps * batch, 4 * hidden),
+                                                            (batch, hidden), (batch, hidden)))
+    sizes = (i64(steps), i64(batch), i64(hidden))
+    state = (d[2].ptr, d[3].ptr) if initial else (None, None)
+    for _ in range(2):  # the second time in memory that the first has used
+        capi.call("lstm_sequence", d[0].ptr, d[1].ptr, i64(ld), *state, *sizes, saved.ptr, h.ptr)
+        capi.call("lstm_sequence_backward", saved.ptr, d[1].ptr, i64(ld), state[1], d[4].ptr, *sizes, dgates.ptr, dh0.ptr if initial else None,
+                  dc0.ptr if initial else None)
+    code = C.c_int(0)
+    capi.call("device_status", C.byref(code))
+    assert code.value == 0
+    got = [h.numpy(), dgates.numpy()] + ([dh0.numpy(), dc0.numpy()] if initial else [])
+    # fp32 sums of `hidden` terms per timestep (4 hidden in the gradient), carried through at most `steps` contracting timesteps
+    bound = 2.0**-24 * (20 + 2 * np.sqrt(hidden)) * steps
+    for a, b in zip(got, want):
+        assert np.max(np.abs(a - b)) <= bound * max(1.0, np.abs(b).max())
+
+
+def test_sizes_are_checked(capi):
+    x = capi.empty((4, 16))
+    for sizes in ((0, 2, 4), (1, 0, 4), (1, 2, 0)):
+        with pytest.raises(Exception, match="extents must be positive"):
+            capi.call("lstm_sequence", x.ptr, x.ptr, i64(16), None, None, *[i64(s) for s in sizes], x.ptr, x.ptr)
+    with pytest.raises(Exception, match="leading dimension"):
+        capi.call("lstm_sequence", x.ptr, x.ptr, i64(15), None, None, i64(1), i64(2), i64(4), x.ptr, x.ptr)
