@@ -168,6 +168,12 @@ struct KeepsOutputs : std::false_type {};
 template <class B>
 struct KeepsOutputs<B, std::void_t<decltype(&B::relu_max_pool2d)>> : std::true_type {};
 
+// A backend that has computed a recurrence as one may take it backward as one.
+template <class B, class = void>
+struct HasSequences : std::false_type {};
+template <class B>
+struct HasSequences<B, std::void_t<decltype(&B::sequence_backward)>> : std::true_type {};
+
 template <class B>
 class Tensor {
  public:
@@ -280,6 +286,25 @@ class Tensor {
     }
     auto nodes = build_topo_sort();
     std::unordered_set<size_t> visited;
+    if constexpr (HasSequences<B>::value) {
+      // sequences go last: of the rest nothing but leaves depends on them
+      const auto sequences = B::sequences(nodes);
+      std::vector<Tensor<B>> leaves;
+      for (auto& s : sequences) {
+        visited.insert(s.members.begin(), s.members.end());
+        for (const Tensor<B>& leaf : {s.w, s.b})
+          if (visited.insert(leaf.id()).second) leaves.push_back(leaf);
+      }
+      walk_back(nodes, visited);
+      for (auto& s : sequences) B::sequence_backward(s);
+      for (const Tensor<B>& leaf : leaves)
+        if (leaf.inner->grad && leaf.requires_grad() && leaf_ready_hook()) leaf_ready_hook()(leaf);
+    } else {
+      walk_back(nodes, visited);
+    }
+  }
+  // The gradients of `nodes`, the last first, but for those that have been visited.
+  static void walk_back(const std::vector<Tensor<B>>& nodes, std::unordered_set<size_t>& visited) {
     for (auto it = nodes.rbegin(); it != nodes.rend(); ++it) {
       const Tensor<B>& node = *it;
       if (!visited.insert(node.id()).second) continue;

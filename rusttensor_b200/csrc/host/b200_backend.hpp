@@ -12,9 +12,11 @@
 #include <algorithm>
 #include <memory>
 #include <cmath>
+#include <cstring>
 #include <optional>
 #include <random>
 #include <tuple>
+#include <unordered_map>
 #include <vector>
 
 #include "../../../include/rt_b200.h"
@@ -95,6 +97,7 @@ struct B200Backend {
     const bool scalar_sum = n.kind == lazy::Kind::Binary && n.op == RT_F_ADD && shape_numel(shape) == 1;
     now = now || n.depth >= (scalar_sum ? lazy::kMaxChain : lazy::kMaxDepth);
     n.weight = std::min(n.weight, 1 << 20);
+    if (n.tag == lazy::Tag::Matmul) n.depth = 1;  // of a sequence, which is evaluated from its first timestep on
     *at_once = now;
     return Storage{std::make_shared<DeviceBuffer>(ctx(), std::make_unique<lazy::Node>(std::move(n)), shape_numel(shape)), shape};
   }
@@ -841,7 +844,6 @@ struct B200Backend {
     const Storage& x = o.inputs[0].data();
     Axis3 a = split(x.shape, o.op_type.axis);
     if (g.shape != x.shape) throw Error::shape_mismatch(x.shape, g.shape);
-    Storage dx = alloc(x.shape);
     // upstream = constant * targets (a classification loss): without the product in memory
     float c;
     if (g.buf && g.buf->node && a.inner == 1 && a.len <= 4096)
@@ -849,19 +851,30 @@ struct B200Backend {
         const float* tp = t->buf->data();
         if (g.buf->node) {
           const float* xp = x.ptr();
+          Storage dx;
           lazy::Loss l;
           DeviceBuffer* loss = lazy::loss_over(x.buf.get(), t->buf.get(), &l);
           if (loss && l.rows == (int64_t)a.outer && l.classes == (int64_t)a.len) {  // the loss itself comes out of the same pass
             auto keep = loss->shared_from_this();
             lazy::Block out(loss->ctx, loss->numel);
+            dx = alloc(x.shape);
             check(rt_softmax_nll_with_grad(ctx(), xp, tp, a.outer, a.len, l.scale, l.divisor, nullptr, c, out.ptr, dx.ptr()));
             out.to(loss);
             return dx;
           }
+          if (lazy::capturing() && deferrable(x.shape)) {  // may join those of the other timesteps
+            int64_t bits = 0;
+            std::memcpy(&bits, &c, sizeof(float));
+            return lz_opaque(lazy::Tag::NllGrad, {a.outer, a.len, bits}, {input(x), *t}, x.shape, [c](lazy::Node& n, float* out) {
+              return rt_softmax_nll_scaled_backward(ctx(), n.in[0].buf->data(), n.in[1].buf->data(), n.geo[0], n.geo[1], c, out);
+            });
+          }
+          dx = alloc(x.shape);
           check(rt_softmax_nll_scaled_backward(ctx(), x.ptr(), tp, a.outer, a.len, c, dx.ptr()));
           return dx;
         }
       }
+    Storage dx = alloc(x.shape);
     check(rt_log_softmax_backward(ctx(), x.ptr(), g.ptr(), a.outer, a.len, a.inner, dx.ptr()));
     return dx;
   }
@@ -874,16 +887,27 @@ struct B200Backend {
     int64_t m = (int64_t)a.shape[0], k = (int64_t)a.shape[1], n = (int64_t)b.shape[1];
     if (k > 0 && deferrable(Shape{a.shape[0], b.shape[1]})) {
       // the operands are evaluated now (expressions do not grow through products); the product itself may still join a bias, an
-      // activation, or its siblings
-      a.ptr();
+      // activation, or its siblings.  In a capture the timesteps of an LSTM wait for the last one, and so does what takes their states.
       b.ptr();
-      return lz_opaque(lazy::Tag::Matmul, {}, {input(a), input(b)}, Shape{a.shape[0], b.shape[1]}, [m, n, k](lazy::Node& nd, float* out) {
+      std::vector<int64_t> geo;
+      lazy::Cell cell;
+      if (const int64_t t = a.buf->node ? lazy::timestep_of(input(a), input(b)) : 0) geo.push_back(t);
+      else if (!(lazy::capturing() && a.buf->node && a.shape == a.buf->node->shape && lazy::match_cell(a.buf.get(), &cell))) a.ptr();
+      return lz_opaque(lazy::Tag::Matmul, std::move(geo), {input(a), input(b)}, Shape{a.shape[0], b.shape[1]}, [m, n, k](lazy::Node& nd, float* out) {
         return rt_gemm(ctx(), 0, 0, m, n, k, nd.in[0].buf->data(), k, nd.in[1].buf->data(), n, out, n, 0);
       });
     }
     Storage c = alloc(Shape{a.shape[0], b.shape[1]});
     check(rt_gemm(ctx(), 0, 0, m, n, k, a.ptr(), k, b.ptr(), n, c.ptr(), n, 0));
     return c;
+  }
+  // In a capture: a state of a sequence that was computed as one, whose gradient comes from all its timesteps at once.
+  static bool of_a_sequence(const Storage& a) { return lazy::capturing() && a.buf && a.buf->sequence; }
+  static Storage state_gradient(const Storage& g, const Storage& b, const Shape& shape) {
+    return lz_opaque(lazy::Tag::MatmulNT, {}, {input(g), input(b)}, shape, [](lazy::Node& n, float* out) {
+      const int64_t m = (int64_t)n.in[0].shape[0], cols = (int64_t)n.in[0].shape[1], k = (int64_t)n.in[1].shape[0];
+      return rt_gemm(ctx(), 0, 1, m, k, cols, n.in[0].buf->data(), cols, n.in[1].buf->data(), cols, out, k, 0);
+    });
   }
   static std::pair<Storage, Storage> matmul_backward(const OpB& o, const Storage& g) {
     if (o.inputs.size() != 2) throw Error::invalid_op("Matmul requires 2 inputs");
@@ -892,6 +916,14 @@ struct B200Backend {
     int64_t m = (int64_t)a.shape[0], k = (int64_t)a.shape[1], n = (int64_t)b.shape[1];
     if (g.shape != Shape{a.shape[0], b.shape[1]}) throw Error::incompatible("matmul", g.shape, b.shape);
     bool need_a = o.inputs[0].requires_grad(), need_b = o.inputs[1].requires_grad();
+    if (of_a_sequence(a) && deferrable(b.shape)) {  // the other timesteps' products follow: both wait for them
+      Storage db{nullptr, b.shape};
+      if (need_b) {
+        db = filled(b.shape, 0.f);
+        append_terms(db, lazy::Tag::SumProducts, {input(a), input(g)}, {m, k, n}, run_sum_products);
+      }
+      return {need_a ? state_gradient(g, b, a.shape) : Storage{nullptr, a.shape}, std::move(db)};
+    }
     Storage da = need_a ? alloc(a.shape) : Storage{nullptr, a.shape};
     Storage db = need_b ? alloc(b.shape) : Storage{nullptr, b.shape};
     check(rt_matmul_backward(ctx(), a.ptr(), b.ptr(), g.ptr(), m, k, n, da.ptr(), db.ptr()));
@@ -906,6 +938,10 @@ struct B200Backend {
     int64_t m = (int64_t)a.shape[0], k = (int64_t)a.shape[1], n = (int64_t)b.shape[1];
     if (g.shape != Shape{a.shape[0], b.shape[1]}) throw Error::incompatible("matmul", g.shape, b.shape);
     if (acc.shape != b.shape) throw Error::shape_mismatch(b.shape, acc.shape);
+    if (of_a_sequence(a) && deferrable(b.shape)) {
+      append_terms(acc, lazy::Tag::SumProducts, {input(a), input(g)}, {m, k, n}, run_sum_products);
+      return o.inputs[0].requires_grad() ? state_gradient(g, b, a.shape) : Storage{nullptr, a.shape};
+    }
     Storage da = o.inputs[0].requires_grad() ? alloc(a.shape) : Storage{nullptr, a.shape};
     if (deferrable(a.shape) && deferrable(g.shape) && deferrable(b.shape)) {
       // the weight's gradient is a sum over all its uses: the products are collected and computed as one with a longer reduction
@@ -921,7 +957,7 @@ struct B200Backend {
   static bool accumulates_well(const Storage& b) { return b.shape.size() == 2 && (deferrable(b.shape) || b.shape[1] % 4 == 0); }
 
   // acc += a term that is computed later, together with the others of its kind.  Node: in[0] is what was there before.
-  static constexpr size_t kMaxTerms = 192;
+  static constexpr size_t kMaxTerms = 512;  // operands: twice what one launch of rt_gemm_sum_products takes
   static void append_terms(Storage& acc, lazy::Tag tag, std::vector<lazy::Input> term, std::vector<int64_t> geo,
                            void (*run)(lazy::Node&, DeviceBuffer*)) {
     DeviceBuffer* b = acc.buf.get();
@@ -979,7 +1015,14 @@ struct B200Backend {
     const lazy::Node* n = g.buf ? g.buf->node.get() : nullptr;
     if (n && n->tag == lazy::Tag::SumRows && n->geo[0] < 0 && g.buf->readers.empty() && g.shape.size() == 1 && existing.buf && existing.shape == g.shape) {
       const lazy::Input x = n->in[0];
-      append_terms(existing, lazy::Tag::SumRows, {x}, {(int64_t)x.shape[0], (int64_t)x.shape[1]}, run_sum_rows);
+      const lazy::Node* e = existing.buf->node.get();
+      const std::vector<int64_t> geo{(int64_t)x.shape[0], (int64_t)x.shape[1]};
+      if (lazy::capturing() && e && e->tag == lazy::Tag::SumRows && e->geo[0] < 0 && existing.buf.use_count() == 1 && existing.buf->readers.empty()) {
+        const lazy::Input first = e->in[0];  // the first of a sequence's waits with the others
+        existing = filled(existing.shape, 0.f);
+        append_terms(existing, lazy::Tag::SumRows, {first}, {(int64_t)first.shape[0], (int64_t)first.shape[1]}, run_sum_rows);
+      }
+      append_terms(existing, lazy::Tag::SumRows, {x}, geo, run_sum_rows);
       return;
     }
     existing = add(existing, g);
@@ -1301,35 +1344,205 @@ struct B200Backend {
     h.buf->saved = {saved.buf};
     return h;
   }
+  // From the gradient of the states: that of the gates [rows, 4H], of the weights and of the input.
+  struct SequenceGradients {
+    Storage dgates, dw, dx;
+  };
+  static SequenceGradients sequence_gradients(const float* saved, const float* x, int64_t features, const float* h, const float* w, const float* dh,
+                                              int64_t steps, int64_t batch, int64_t H, bool need_w, bool need_x) {
+    const int64_t rows = steps * batch, V = features, G = 4 * H;
+    SequenceGradients r{alloc({(size_t)rows, (size_t)G}), {}, {}};
+    const float* dz = r.dgates.ptr();
+    check(rt_lstm_sequence_backward(ctx(), saved, w + V * G, G, nullptr, dh, steps, batch, H, r.dgates.ptr(), nullptr, nullptr));
+    if (need_x) {
+      r.dx = alloc({(size_t)rows, (size_t)V});
+      if (V > 0) check(rt_gemm(ctx(), 0, 1, rows, V, G, dz, G, w, G, r.dx.ptr(), V, 0));
+    }
+    if (need_w) {
+      r.dw = alloc({(size_t)(V + H), (size_t)G});
+      float *of_x = r.dw.ptr(), *of_h = of_x + V * G;
+      if (V > 0) check(rt_gemm(ctx(), 1, 0, V, G, rows, x, V, dz, G, of_x, G, 0));
+      // every timestep but the first multiplies the weights with the state before it
+      if (steps > 1) check(rt_gemm(ctx(), 1, 0, H, G, rows - batch, h, H, dz + batch * G, G, of_h, G, 0));
+      else check(rt_fill(ctx(), of_h, 0.f, H * G));
+    }
+    return r;
+  }
   static std::vector<Storage> lstm_sequence_backward(const OpB& o, const Storage& g, size_t steps) {
     const Storage &x = o.inputs[0].data(), &w = o.inputs[1].data(), &h = *o.cached_outputs;
     if (g.shape != h.shape) throw Error::shape_mismatch(h.shape, g.shape);
-    const int64_t rows = (int64_t)x.shape[0], V = (int64_t)x.shape[1], H = (int64_t)w.shape[1] / 4, batch = rows / (int64_t)steps;
-    const float *saved = h.buf->saved[0]->data(), *pw = w.ptr(), *px = x.ptr(), *pg = g.ptr();
-    Storage dgates = alloc({x.shape[0], w.shape[1]});
-    check(rt_lstm_sequence_backward(ctx(), saved, pw + V * 4 * H, 4 * H, nullptr, pg, (int64_t)steps, batch, H, dgates.ptr(), nullptr, nullptr));
+    const int64_t rows = (int64_t)x.shape[0], H = (int64_t)w.shape[1] / 4;
+    const float *saved = h.buf->saved[0]->data(), *pw = w.ptr(), *px = x.ptr(), *pg = g.ptr(), *states = h.ptr();
+    const bool written = h.buf->escaped && !lazy::capturing();  // perhaps, since: h = o * tanh(c) once more
+    lazy::Block again(ctx(), written ? (size_t)(rows * H) : 1);
+    if (written) {
+      const int64_t n[1] = {rows * H};
+      check(rt_binary(ctx(), RT_MUL, saved + 3 * rows * H, n, 1, saved + 5 * rows * H, n, 1, again.ptr));
+      states = again.ptr;
+    }
+    SequenceGradients r = sequence_gradients(saved, px, (int64_t)x.shape[1], states, pw, pg, (int64_t)steps, rows / (int64_t)steps, H,
+                                             o.inputs[1].requires_grad(), o.inputs[0].requires_grad());
     std::vector<Storage> out{unused_grad(x.shape), unused_grad(w.shape), unused_grad(o.inputs[2].shape())};
-    if (o.inputs[0].requires_grad()) {
-      out[0] = alloc(x.shape);
-      if (V > 0) check(rt_gemm(ctx(), 0, 1, rows, V, 4 * H, dgates.ptr(), 4 * H, pw, 4 * H, out[0].ptr(), V, 0));
-    }
-    if (o.inputs[1].requires_grad()) {
-      out[1] = alloc(w.shape);
-      float *dx_rows = out[1].ptr(), *dh_rows = dx_rows + V * 4 * H;
-      if (V > 0) check(rt_gemm(ctx(), 1, 0, V, 4 * H, rows, px, V, dgates.ptr(), 4 * H, dx_rows, 4 * H, 0));
-      const int64_t later = rows - batch;  // every timestep but the first multiplies the weights with the state before it
-      const float* states = h.ptr();
-      lazy::Block own_states(ctx(), h.buf->escaped && !lazy::capturing() ? (size_t)(rows * H) : 1);
-      if (h.buf->escaped && !lazy::capturing()) {  // may have been written since: h = o * tanh(c) once more
-        const int64_t n[1] = {rows * H};
-        check(rt_binary(ctx(), RT_MUL, saved + 3 * rows * H, n, 1, saved + 5 * rows * H, n, 1, own_states.ptr));
-        states = own_states.ptr;
-      }
-      if (later > 0) check(rt_gemm(ctx(), 1, 0, H, 4 * H, later, states, H, dgates.ptr() + batch * 4 * H, 4 * H, dh_rows, 4 * H, 0));
-      else check(rt_fill(ctx(), dh_rows, 0.f, H * 4 * H));
-    }
-    if (o.inputs[2].requires_grad()) out[2] = unbroadcast(dgates, o.inputs[2].shape());
+    if (r.dx.buf) out[0] = std::move(r.dx);
+    if (r.dw.buf) out[1] = std::move(r.dw);
+    if (o.inputs[2].requires_grad()) out[2] = unbroadcast(r.dgates, o.inputs[2].shape());
     return out;
+  }
+
+  // ---- sequences on the tape (Tensor::backward) ----------------------------------------------------------------------------------
+  // An LSTM that was written op by op and computed as one (lazy::rewrite_recurrence) goes backward as one, too: its nodes take no part in the
+  // walk, and once everything else is done the gradients of all its states go through rt_lstm_sequence_backward.  Its weights and bias are
+  // leaves and its inputs take no gradient, so nothing but leaves waits for it; nobody but the tape holds its intermediate tensors, whose
+  // own gradients are therefore not missed.
+  using T = Tensor<B200Backend>;
+  struct TapeSequence {
+    std::vector<T> h;
+    T w, b;
+    std::vector<size_t> members;
+  };
+  static bool is_plain(const T& t) { return !t.inner->op && !t.requires_grad(); }
+  struct TapeCell {
+    const T *h, *c, *h_prev, *c_prev, *w, *b;
+    std::vector<const T*> inner;  // everything between: used once each, z four times
+    const T* z;
+  };
+  static const T* input_of(const T& t, OpType::Kind kind, size_t inputs = 1) {
+    const auto& op = t.inner->op;
+    return op && op->op_type.kind == kind && op->inputs.size() == inputs ? op->inputs.data() : nullptr;
+  }
+  static const T* tape_gate(const T& t, OpType::Kind act, size_t block, TapeCell* q) {
+    const T* s = input_of(t, act);
+    const T* z = s ? input_of(*s, OpType::Slice) : nullptr;
+    if (!z || t.shape().size() != 2) return nullptr;
+    const size_t B = t.shape()[0], H = t.shape()[1];
+    const auto& r = s->inner->op->op_type.ranges;
+    if (z->shape() != Shape{B, 4 * H} || r.size() != 2 || r[0].start != 0 || r[0].end != B || r[1].start != block * H || r[1].end != (block + 1) * H) return nullptr;
+    q->inner.push_back(&t);
+    q->inner.push_back(s);
+    return z;
+  }
+  static bool tape_cell(const T& h, TapeCell* out) {
+    const T* m = input_of(h, OpType::Mul, 2);
+    if (!m) return false;
+    const Shape s = h.shape();
+    for (int k = 0; k < 2; ++k) {
+      TapeCell q{};
+      const T* z = tape_gate(m[k], OpType::Sigmoid, 3, &q);
+      const T* c = z && m[1 - k].shape() == s ? input_of(m[1 - k], OpType::Tanh) : nullptr;
+      const T* sum = c ? input_of(*c, OpType::Add, 2) : nullptr;
+      if (!sum) continue;
+      q.inner.push_back(&m[1 - k]);
+      for (int e = 0; e < 8; ++e) {
+        TapeCell p = q;
+        const T &fc = sum[e & 1], &ig = sum[1 - (e & 1)];
+        const T *u = input_of(fc, OpType::Mul, 2), *v = input_of(ig, OpType::Mul, 2);
+        if (!u || !v || fc.shape() != s || ig.shape() != s) continue;
+        const T &f = u[e >> 1 & 1], &before = u[1 - (e >> 1 & 1)], &i = v[e >> 2], &g = v[1 - (e >> 2)];
+        if (before.shape() != s) continue;
+        const T *zf = tape_gate(f, OpType::Sigmoid, 1, &p), *zi = tape_gate(i, OpType::Sigmoid, 0, &p), *zg = tape_gate(g, OpType::Tanh, 2, &p);
+        if (!zf || !zi || !zg || zf->id() != z->id() || zi->id() != z->id() || zg->id() != z->id()) continue;
+        const T* zs = input_of(*z, OpType::Add, 2);
+        if (!zs) return false;
+        for (int w = 0; w < 2; ++w) {
+          const T* mm = input_of(zs[w], OpType::Matmul, 2);
+          if (!mm) continue;
+          const T* cat = input_of(mm[0], OpType::Concat, 2);
+          if (cat ? *mm[0].inner->op->op_type.axis != 1 : !is_plain(mm[0])) continue;  // the first timestep's takes no gradient
+          const T* bias = &zs[1 - w];
+          p.inner.push_back(&zs[w]);
+          if (cat) p.inner.push_back(&mm[0]);
+          p.inner.push_back(&fc);
+          p.inner.push_back(&ig);
+          if (const T* b0 = input_of(*bias, OpType::Broadcast)) {
+            p.inner.push_back(bias);
+            bias = b0;
+          }
+          if (bias->inner->op || mm[1].inner->op || bias->shape() != Shape{4 * s[1]}) return false;
+          if (cat && (cat[0].requires_grad() || cat[1].shape() != s)) return false;
+          p.h = &h; p.c = c; p.z = z; p.h_prev = cat ? &cat[1] : nullptr; p.c_prev = &before; p.w = &mm[1]; p.b = bias;
+          *out = p;
+          return true;
+        }
+      }
+    }
+    return false;
+  }
+  static std::vector<TapeSequence> sequences(const std::vector<T>& nodes) {
+    std::vector<TapeSequence> found;
+    if (!lazy::capturing()) return found;
+    std::unordered_map<size_t, long> uses;
+    std::unordered_map<size_t, TapeCell> next;  // by the id of the state before
+    for (const T& n : nodes)
+      if (n.inner->op)
+        for (const T& i : n.inner->op->inputs) ++uses[i.id()];
+    std::vector<TapeCell> firsts;
+    for (const T& n : nodes) {
+      TapeCell q;
+      if (!tape_cell(n, &q)) continue;
+      if (!q.h_prev || is_plain(*q.h_prev)) {
+        if (is_plain(*q.c_prev)) firsts.push_back(q);
+      } else if (!next.emplace(q.h_prev->id(), q).second) {
+        return {};  // a state that two cells go on from
+      }
+    }
+    auto only = [&](const T& t, long n) { return uses[t.id()] == n && t.inner.use_count() == n + 1 && !t.inner->grad; };  // + 1: `nodes`
+    for (const TapeCell& first : firsts) {
+      TapeSequence s;
+      bool ok = true;
+      for (const TapeCell* q = &first; q;) {
+        auto it = next.find(q->h->id());
+        const TapeCell* after = it == next.end() ? nullptr : &it->second;
+        if (after && (after->c_prev->id() != q->c->id() || after->w->id() != q->w->id() || after->b->id() != q->b->id())) after = nullptr;
+        for (const T* t : q->inner) ok = ok && only(*t, 1);
+        ok = ok && only(*q->z, 4) && only(*q->c, after ? 2 : 1) && q->h->inner.use_count() == uses[q->h->id()] + 1 && !q->h->inner->grad;
+        s.h.push_back(*q->h);
+        for (const T* t : q->inner) s.members.push_back(t->id());
+        for (const T* t : {q->h, q->c, q->z}) s.members.push_back(t->id());
+        s.w = *q->w;
+        s.b = *q->b;
+        q = after;
+      }
+      if (s.h.size() < 2) continue;
+      s.h.back().data().ptr();  // computes the sequence, which the walk needs in any case
+      if (!ok) continue;
+      const auto& seq = s.h[0].data().buf->sequence;
+      ok = seq && seq->steps == (int64_t)s.h.size() && seq->w == s.w.data().buf;
+      for (size_t t = 0; t < s.h.size() && ok; ++t) ok = s.h[t].data().buf->sequence == seq && s.h[t].data().buf->timestep == (int64_t)t;
+      if (ok) found.push_back(std::move(s));
+    }
+    return found;
+  }
+  static void sequence_backward(const TapeSequence& s) {
+    const std::shared_ptr<Recurrence> q = s.h[0].data().buf->sequence;
+    const int64_t n = q->batch * q->hidden;
+    lazy::Block dh(ctx(), (size_t)(q->steps * n));
+    for (int64_t t = 0; t < q->steps;) {
+      float* out = dh.ptr + t * n;
+      const auto& g = s.h[t].grad();
+      auto product = [&](int64_t i) -> const lazy::Node* {  // the gradient is a product that nobody else has asked for
+        if (i >= q->steps || !s.h[i].grad() || !s.h[i].grad()->buf) return nullptr;
+        const DeviceBuffer* b = s.h[i].grad()->buf.get();
+        return b->node && b->node->tag == lazy::Tag::MatmulNT && b->readers.empty() ? b->node.get() : nullptr;
+      };
+      if (const lazy::Node* p = product(t)) {  // and those after it, as long as their operands follow in memory
+        const int64_t m = (int64_t)p->in[0].shape[0], cols = (int64_t)p->in[0].shape[1], k = (int64_t)p->in[1].shape[0];
+        const float* first = p->in[0].buf->data();
+        int64_t count = 1;
+        for (const lazy::Node* r; (r = product(t + count)) && r->in[1].buf == p->in[1].buf && r->in[0].shape == p->in[0].shape &&
+                                  r->in[0].buf->data() == first + count * m * cols;)
+          ++count;
+        check(rt_gemm(ctx(), 0, 1, count * m, k, cols, first, cols, p->in[1].buf->data(), cols, out, k, 0));
+        t += count;
+      } else {
+        if (g) check(rt_memcpy_d2d(ctx(), out, g->ptr(), sizeof(float) * (size_t)n));
+        else check(rt_fill(ctx(), out, 0.f, n));
+        ++t;
+      }
+    }
+    SequenceGradients r = sequence_gradients(q->saved->ptr, q->x_rows, q->features, q->h->ptr, q->w->ptr, dh.ptr, q->steps, q->batch, q->hidden,
+                                             s.w.requires_grad(), false);
+    if (r.dw.buf) s.w.add_grad(std::move(r.dw));
+    if (s.b.requires_grad()) s.b.add_grad(unbroadcast(r.dgates, s.b.shape()));
   }
 
   // One launch for all parameters of an optimizer step.  kind as rt_optimizer_step_multi; s1 / s2: the optimizer's states.

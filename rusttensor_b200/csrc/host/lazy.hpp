@@ -44,7 +44,7 @@ struct Input {
 };
 enum class Kind : uint8_t { Const, Unary, BinaryImm, Binary, Broadcast, Slice, Pad, Concat, Opaque };
 // Opaque: computed by a kernel of its own.  Deferred only because what it feeds may take a kernel that does both.
-enum class Tag : uint8_t { None, Matmul, Conv, LogSoftmax, Reduce, PoolGrad, SumProducts, SumRows, FusedLoss };
+enum class Tag : uint8_t { None, Matmul, Conv, LogSoftmax, Reduce, PoolGrad, SumProducts, SumRows, FusedLoss, NllGrad, MatmulNT };
 
 struct Node {
   Kind kind;
@@ -73,6 +73,13 @@ int current_weight(const Node& n, int limit);
 
 }  // namespace lazy
 
+// An LSTM over a sequence that was written op by op and has been computed as one (lazy::rewrite_recurrence).
+struct Recurrence {
+  std::shared_ptr<DeviceBuffer> saved, h, x, w;  // six planes and the states [steps * batch, hidden]; inputs; weights
+  const float* x_rows = nullptr;                 // [steps * batch, features]
+  int64_t steps = 0, batch = 0, hidden = 0, features = 0;
+};
+
 struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
   rt_ctx* ctx;
   float* ptr;
@@ -81,6 +88,8 @@ struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
   std::shared_ptr<DeviceBuffer> owner;  // set: ptr points into this buffer's block (contiguous rows of it)
   uint64_t id = next_id();   // of the values: another one after every change in place
   uint64_t made_from = 0;    // id of the operand's values, for results from which their gradient follows
+  std::shared_ptr<Recurrence> sequence;  // set: the state after timestep `timestep` of it
+  int64_t timestep = 0;
   std::vector<std::shared_ptr<DeviceBuffer>> saved;  // intermediate results of a fused op that its gradient uses
   std::unique_ptr<lazy::Node> node;    // what to compute; null once the values are in memory
   std::vector<DeviceBuffer*> readers;  // unevaluated buffers whose expression takes this one as an input
@@ -802,6 +811,159 @@ inline const Input* times_constant(const Node* n, float* c) {
   return nullptr;
 }
 
+// Several results computed as one matrix, in a capture: each is rows of the common block.
+inline std::shared_ptr<DeviceBuffer> common_block(rt_ctx* ctx, size_t numel) {
+  Block block(ctx, numel);
+  auto b = std::make_shared<DeviceBuffer>(ctx, block.ptr, numel);
+  block.release();
+  return b;
+}
+inline void place(DeviceBuffer* b, const std::shared_ptr<DeviceBuffer>& block, size_t offset) {
+  b->ptr = block->ptr + offset;
+  b->owner = block;
+  b->drop_node();
+}
+
+// ---- LSTM cells written op by op ---------------------------------------------------------------------------------------------
+//   z = concat(x_t, h_prev) w + b;  i, f, g, o = the column blocks of z, activated;  c = f c_prev + i g;  h = o tanh(c)
+// A capture records a whole step, so the product of such a cell need not be computed when it is asked for: matmul leaves it pending as long
+// as every cell below it is of this form and the states before the first are zeros, and whoever asks for a state then gets the sequence from
+// rt_lstm_sequence, every timestep at once.
+struct Cell {
+  std::shared_ptr<DeviceBuffer> h, c, i, f, g, o, tc, product;
+  Input z, xh, h_prev, c_prev, w, bias;
+};
+inline const Input* unary_of(const Input& x, uint8_t op) {
+  return pending(x) && pending(x)->kind == Kind::Unary && pending(x)->op == op && pending(x)->shape == x.shape ? &pending(x)->in[0] : nullptr;
+}
+// x = act(columns block * H .. of z)
+inline const Input* gate_of(const Input& x, uint8_t act, size_t block) {
+  const Input* s = unary_of(x, act);
+  const Node* n = s ? pending(*s) : nullptr;
+  if (!n || n->kind != Kind::Slice || n->shape != x.shape || s->shape != x.shape || x.shape.size() != 2) return nullptr;
+  if (n->starts != Shape{0, block * x.shape[1]} || n->in[0].shape != Shape{x.shape[0], 4 * x.shape[1]}) return nullptr;
+  return &n->in[0];
+}
+inline bool match_cell(DeviceBuffer* b, Cell* q) {
+  const Node* n = b->node.get();
+  if (!is_op(n, Kind::Binary, RT_F_MUL) || n->shape.size() != 2) return false;
+  const Shape& s = n->shape;
+  for (int k = 0; k < 2; ++k) {
+    const Input &o = n->in[k], &tc = n->in[1 - k];
+    const Input *zo = o.shape == s ? gate_of(o, RT_F_SIGMOID, 3) : nullptr, *c = zo && tc.shape == s ? unary_of(tc, RT_F_TANH) : nullptr;
+    if (!c || c->shape != s || !is_op(pending(*c), Kind::Binary, RT_F_ADD)) continue;
+    for (int a = 0; a < 2; ++a) {
+      const Input &fc = pending(*c)->in[a], &ig = pending(*c)->in[1 - a];
+      if (fc.shape != s || ig.shape != s || !is_op(pending(fc), Kind::Binary, RT_F_MUL) || !is_op(pending(ig), Kind::Binary, RT_F_MUL)) continue;
+      for (int e = 0; e < 4; ++e) {
+        const Input &f = pending(fc)->in[e & 1], &before = pending(fc)->in[1 - (e & 1)], &i = pending(ig)->in[e >> 1], &g = pending(ig)->in[1 - (e >> 1)];
+        if (f.shape != s || before.shape != s || i.shape != s || g.shape != s) continue;
+        const Input *zf = gate_of(f, RT_F_SIGMOID, 1), *zi = gate_of(i, RT_F_SIGMOID, 0), *zg = gate_of(g, RT_F_TANH, 2);
+        if (!zf || !zi || !zg || zf->buf != zo->buf || zi->buf != zo->buf || zg->buf != zo->buf) continue;
+        const Node* z = pending(*zo);
+        if (!is_op(z, Kind::Binary, RT_F_ADD) || z->shape != zo->shape) return false;
+        for (int p = 0; p < 2; ++p) {
+          const Node* m = tagged(z->in[p], Tag::Matmul);
+          Input bias = z->in[1 - p];
+          if (!m || m->geo.empty() || m->shape != z->shape || z->in[p].shape != m->shape) continue;
+          if (pending(bias) && pending(bias)->kind == Kind::Broadcast && pending(bias)->shape == bias.shape) bias = Input(pending(bias)->in[0]);
+          if (bias.shape.empty() || bias.shape.back() != m->shape[1] || shape_numel(bias.shape) != m->shape[1] || bias.buf->node) continue;
+          const Node* cat = pending(m->in[0]);
+          if (!cat || cat->kind != Kind::Concat || cat->in.size() != 2) return false;
+          *q = Cell{b->shared_from_this(), c->buf, i.buf, f.buf, g.buf, o.buf, tc.buf, z->in[p].buf, *zo, m->in[0], cat->in[1], before, m->in[1], bias};
+          return true;
+        }
+      }
+    }
+  }
+  return false;
+}
+inline bool is_zero(const Input& x) { return pending(x) && pending(x)->kind == Kind::Const && pending(x)->imm == 0.f; }
+// The rows of a matrix in memory that a cell's input is.
+inline bool rows_of(const Input& x, Input* base, int64_t* first) {
+  const Node* n = pending(x);
+  if (!n || n->kind != Kind::Slice || n->shape != x.shape || n->in[0].shape.size() != 2 || n->in[0].buf->node) return false;
+  if (n->starts[1] != 0 || n->in[0].shape[1] != x.shape[1]) return false;
+  *base = n->in[0];
+  *first = (int64_t)n->starts[0];
+  return true;
+}
+// The timestep, counted from 1, whose product a * w would be in a sequence whose cells are all pending; 0: none.
+inline int64_t timestep_of(const Input& a, const Input& w) {
+  const Node* cat = pending(a);
+  if (!capturing() || !cat || cat->kind != Kind::Concat || cat->in.size() != 2 || cat->starts[0] != 1 || a.shape != cat->shape || a.shape.size() != 2) return 0;
+  if (w.shape.size() != 2 || w.shape[0] != a.shape[1] || w.buf->node) return 0;
+  const Input &x = cat->in[0], &h = cat->in[1];
+  Input base;
+  int64_t first;
+  if (h.shape.size() != 2 || w.shape[1] != 4 * h.shape[1] || !rows_of(x, &base, &first)) return 0;
+  if (is_zero(h)) return 1;
+  Cell q;
+  if (!h.buf->node || !match_cell(h.buf.get(), &q) || q.w.buf != w.buf) return 0;
+  Input before;
+  int64_t at;
+  if (!rows_of(pending(q.xh)->in[0], &before, &at) || before.buf != base.buf || at + (int64_t)x.shape[0] != first || q.h_prev.shape != h.shape) return 0;
+  const int64_t t = pending(Input{q.product, {}})->geo[0];
+  if (t == 1 ? !is_zero(q.c_prev) : !q.c_prev.buf->node) return 0;
+  if (t > 1) {  // the cell state must be that of the cell whose h this one takes
+    Cell r;
+    if (!match_cell(q.h_prev.buf.get(), &r) || r.c != q.c_prev.buf || r.bias.buf != q.bias.buf) return 0;
+  }
+  q.c->node->depth = 1;  // like the products: the sequence is evaluated from its first timestep on, however long it is
+  return t + 1;
+}
+inline bool rewrite_recurrence(DeviceBuffer* b) {
+  if (!capturing() || !is_op(b->node.get(), Kind::Binary, RT_F_MUL)) return false;
+  std::vector<Cell> cells;  // the last first
+  for (DeviceBuffer* at = b;;) {
+    Cell q;
+    if (!at->node || !match_cell(at, &q)) return false;
+    if (!cells.empty() && (cells.back().c_prev.buf != q.c || cells.back().w.buf != q.w.buf || cells.back().bias.buf != q.bias.buf)) return false;
+    at = q.h_prev.buf.get();
+    cells.push_back(std::move(q));
+    if (is_zero(cells.back().h_prev) && is_zero(cells.back().c_prev)) break;
+  }
+  std::reverse(cells.begin(), cells.end());
+  auto seq = std::make_shared<Recurrence>();
+  const Input& w = cells[0].w;
+  Input x;
+  int64_t first = 0;
+  for (size_t t = 0; t < cells.size(); ++t) {  // as timestep_of has found them
+    Input base;
+    int64_t at;
+    if (!rows_of(pending(cells[t].xh)->in[0], &base, &at)) return false;
+    if (t == 0) {
+      x = base;
+      first = at;
+    }
+    if (base.buf != x.buf || at != first + (int64_t)(t * cells[0].h_prev.shape[0])) return false;
+  }
+  seq->steps = (int64_t)cells.size();
+  seq->batch = (int64_t)cells[0].h_prev.shape[0];
+  seq->hidden = (int64_t)cells[0].h_prev.shape[1];
+  seq->features = (int64_t)x.shape[1];
+  const int64_t rows = seq->steps * seq->batch, H = seq->hidden, n = seq->batch * H;
+  seq->x = x.buf;
+  seq->w = w.buf;
+  seq->x_rows = x.buf->ptr + first * seq->features;
+  seq->saved = common_block(b->ctx, (size_t)(6 * rows * H));
+  seq->h = common_block(b->ctx, (size_t)(rows * H));
+  Block pre(b->ctx, (size_t)(rows * 4 * H));
+  check(b->ctx, rt_gemm_bias_act(b->ctx, rows, 4 * H, seq->features, seq->x_rows, seq->features, w.buf->ptr, 4 * H, cells[0].bias.buf->ptr, RT_ACT_NONE,
+                                 pre.ptr, 4 * H));
+  check(b->ctx, rt_lstm_sequence(b->ctx, pre.ptr, w.buf->ptr + seq->features * 4 * H, 4 * H, nullptr, nullptr, seq->steps, seq->batch, H, seq->saved->ptr,
+                                 seq->h->ptr));
+  for (size_t t = 0; t < cells.size(); ++t) {
+    Cell& q = cells[t];
+    DeviceBuffer* planes[6] = {q.i.get(), q.f.get(), q.g.get(), q.o.get(), q.c.get(), q.tc.get()};
+    for (int k = 0; k < 6; ++k) place(planes[k], seq->saved, (size_t)(k * rows * H + (int64_t)t * n));
+    place(q.h.get(), seq->h, (size_t)((int64_t)t * n));
+    q.h->sequence = seq;
+    q.h->timestep = (int64_t)t;
+  }
+  return true;
+}
+
 // act(a * b + bias), act one of none, relu, tanh, sigmoid: bias and activation in the product's epilogue.  Products of one shape
 // with the same b (a layer applied to every timestep) whose left operands are all there are computed in one launch.
 struct Linear {
@@ -864,6 +1026,19 @@ inline bool rewrite_linear(DeviceBuffer* b) {
     all.push_back(l);
   }
   const int64_t rows = (int64_t)first.a.shape[0], k = (int64_t)first.a.shape[1], cols = (int64_t)first.b.shape[1];
+  if (capturing() && all.size() > 1) {  // left operands that follow one another in memory (the states of a sequence) are one
+    std::sort(all.begin(), all.end(), [](const Linear& x, const Linear& y) { return x.a.buf->ptr < y.a.buf->ptr; });
+    bool together = true;
+    for (size_t i = 1; i < all.size(); ++i) together = together && all[i].a.buf->ptr == all[i - 1].a.buf->ptr + rows * k;
+    if (together && (int64_t)all.size() * rows * std::max(cols, k) < (int64_t(1) << 31)) {
+      const auto block = common_block(b->ctx, all.size() * (size_t)(rows * cols));
+      std::vector<std::shared_ptr<DeviceBuffer>> outs;
+      for (auto& l : all) outs.push_back(l.out->shared_from_this());
+      check(b->ctx, rt_gemm_bias_act(b->ctx, (int64_t)all.size() * rows, cols, k, all[0].a.buf->ptr, k, pb, cols, bias, first.act, block->ptr, cols));
+      for (size_t i = 0; i < outs.size(); ++i) place(outs[i].get(), block, i * (size_t)(rows * cols));
+      return true;
+    }
+  }
   std::vector<std::shared_ptr<DeviceBuffer>> keep;
   for (auto& l : all) keep.push_back(l.out->shared_from_this());
   std::vector<const float*> as;
@@ -942,6 +1117,36 @@ inline DeviceBuffer* loss_over(DeviceBuffer* logits, DeviceBuffer* targets, Loss
     if (root && root->readers.empty() && match_loss(root, l) && l->logits->buf.get() == logits && l->targets->buf.get() == targets) return root;
   }
   return nullptr;
+}
+
+// Gradients of classification losses of one kind (Tag::NllGrad), in a capture: those whose rows follow one another in one launch.
+inline bool rewrite_nll_grad(DeviceBuffer* b) {
+  if (b->node->tag != Tag::NllGrad || !capturing()) return false;
+  const int64_t rows = b->node->geo[0], classes = b->node->geo[1], n = rows * classes;
+  std::vector<std::shared_ptr<DeviceBuffer>> all;
+  const std::vector<int64_t> geo = b->node->geo;
+  for (DeviceBuffer* p = DeviceBuffer::head(); p; p = p->next)
+    if (p->node->tag == Tag::NllGrad && p->node->geo == geo && !p->node->in[0].buf->node) all.push_back(p->shared_from_this());
+  for (auto& p : all) p->node->in[1].buf->data();
+  std::sort(all.begin(), all.end(), [](auto& x, auto& y) { return x->node->in[0].buf->ptr < y->node->in[0].buf->ptr; });
+  size_t lo = 0, at = 0;
+  while (at < all.size() && all[at].get() != b) ++at;
+  if (at == all.size()) return false;
+  auto follows = [&](size_t i) {
+    return all[i]->node->in[0].buf->ptr == all[i - 1]->node->in[0].buf->ptr + n && all[i]->node->in[1].buf->ptr == all[i - 1]->node->in[1].buf->ptr + n;
+  };
+  size_t hi = lo = at;
+  while (lo > 0 && follows(lo)) --lo;
+  while (hi + 1 < all.size() && follows(hi + 1)) ++hi;
+  const size_t count = hi - lo + 1;
+  if (count < 2 || (int64_t)count * rows > (1 << 22)) return false;
+  float c;
+  std::memcpy(&c, &geo[2], sizeof(float));
+  const auto block = common_block(b->ctx, count * (size_t)n);
+  check(b->ctx, rt_softmax_nll_scaled_backward(b->ctx, all[lo]->node->in[0].buf->ptr, all[lo]->node->in[1].buf->ptr, (int64_t)count * rows, classes, c,
+                                               block->ptr));
+  for (size_t i = 0; i < count; ++i) place(all[lo + i].get(), block, i * (size_t)n);
+  return true;
 }
 
 // max_pool2d's gradient masked by the relu in front of the pooling: one pass.
@@ -1023,7 +1228,7 @@ inline bool rewrite_rows(DeviceBuffer* b) {
 }
 inline bool rewrite(DeviceBuffer* b) {
   if (b->node->kind == Kind::Const) return false;
-  return rewrite_rows(b) || rewrite_linear(b) || rewrite_loss(b) || rewrite_loss_sum(b) || rewrite_pool(b);
+  return rewrite_rows(b) || rewrite_recurrence(b) || rewrite_linear(b) || rewrite_nll_grad(b) || rewrite_loss(b) || rewrite_loss_sum(b) || rewrite_pool(b);
 }
 
 }  // namespace lazy

@@ -28,6 +28,7 @@ rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m,
                                int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
 rt_status rt_gemm_parts_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
                                  int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate);
+float rt_gemm_parts_estimate(const rt_ctx* ctx, int64_t m, int64_t n, int64_t k);
 rt_status rt_matmul_backward_parts_internal(rt_ctx* ctx, const float* a, const float* b, const float* g, int64_t m, int64_t k, int64_t n, float* da,
                                             float* db, int accumulate_db);
 rt_status rt_conv_forward_tma_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y);
@@ -674,7 +675,11 @@ static Route choose_route(rt_ctx* ctx, bool ta, bool tb, int64_t m, int64_t n, i
     return k > 0 && (tiles <= 2 * (int64_t)ctx->sm_count || work < (1ll << 22)) ? Route::Small : Route::Plain;
   }
   const float ts = rt_gemm_ts_estimate(ctx, m, n, k);
+  // one wave, but so long that MMAs of half the cost are worth the passes beforehand: 512 x 2048 x 8128 205 us as Tensor
+  // (estimated 132, beyond 40 us the estimate is 1.35 times too low), 1024 x 1024 x 4096 70 and 65
+  if (ts > 40.f && rt_gemm_parts_estimate(ctx, m, n, k) < 1.35f * ts) return Route::Parts;
   if (ts >= 0.f) return rt_gemm_small_estimate(ctx, m, n, k, wide) <= ts ? Route::Small : Route::Tensor;
+  if (n >= 48 && work >= 2 * kPartsWork) return Route::Parts;  // short reductions, too: 3216 x 2880 x 94 40 us as Tensor, 32 as Parts
   if (k < 128 || n < 48 || (k < 256 && wide && !(!ta && tb))) return Route::Tensor;
   return work >= kPartsWork ? Route::Parts : Route::Tma;
 }
@@ -742,6 +747,12 @@ rt_status rt_gemm_sum_products(rt_ctx* ctx, int count, const float* const* a, co
   RT_CHECK_PTR(ctx, a);
   RT_CHECK_PTR(ctx, g);
   RT_CHECK_PTR(ctx, c);
+  // Operands that follow one another in memory, either way (the timesteps of a sequence, which the gradient meets last first): one product
+  for (int way = -1; way <= 1 && count > 1; way += 2) {
+    bool together = m * count < (1ll << 31);
+    for (int i = 1; i < count && together; ++i) together = a[i] == a[i - 1] + way * m * k && g[i] == g[i - 1] + way * m * n;
+    if (together) return rt_gemm(ctx, 1, 0, k, n, m * count, way > 0 ? a[0] : a[count - 1], k, way > 0 ? g[0] : g[count - 1], n, c, n, 1);
+  }
   if (ctx->use_tensor_cores && k >= 32 && n >= 16 && count > 1 && m * count < (1ll << 31) && m * n * k * count >= (1ll << 20)) {
     RtScratch sum(ctx);
     rt_status st = sum.alloc(sizeof(float) * (size_t)(k * n));
@@ -765,6 +776,11 @@ rt_status rt_sum_rows_accumulate_list(rt_ctx* ctx, int count, const float* const
   if (count <= 0 || rows <= 0 || cols <= 0) return RT_OK;
   RT_CHECK_PTR(ctx, x);
   RT_CHECK_PTR(ctx, out);
+  for (int way = -1; way <= 1 && count > 1; way += 2) {  // matrices that follow one another in memory, either way: one
+    bool together = rows * count < (1ll << 31);
+    for (int i = 1; i < count && together; ++i) together = x[i] == x[i - 1] + way * rows * cols;
+    if (together) return rt_sum_rows_accumulate(ctx, way > 0 ? x[0] : x[count - 1], rows * count, cols, out);
+  }
   if (rows >= (1 << 22)) {
     for (int i = 0; i < count; ++i) {
       rt_status st = rt_sum_rows_accumulate(ctx, x[i], rows, cols, out);

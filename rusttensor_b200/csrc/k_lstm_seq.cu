@@ -55,7 +55,8 @@ __device__ __forceinline__ void post2(uint4* p, float v, float w, uint32_t tag) 
 }
 __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
-// Waits until N pieces of mail carry `tag`.  False: the wait ran out, here or in another block.
+// Waits until N pieces of mail carry `tag`.  False: the wait ran out, here or in another block.  (Polling one piece until it is there and
+// only then the others is a round trip more: 693 -> 714 us for 128 timesteps at batch 64, H 512.)
 template <int N>
 __device__ __forceinline__ bool receive(const uint4* const (&from)[N], const bool (&want)[N], uint32_t tag, uint4 (&v)[N], const SeqArgs& a) {
   for (uint32_t i = 0; i < kPolls; ++i) {

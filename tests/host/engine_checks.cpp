@@ -16,6 +16,7 @@ int failures;                  // of the checks
 int mallocs_left = -1;         // rt_malloc fails once they are used up; < 0: never
 bool kernels_fail = false;
 int masked_pool_gradients;     // launches of the pooling gradient that masks by the relu in front
+int forward_sequences, backward_sequences;
 
 
 void expect(bool ok, const char* what, int line) {
@@ -105,6 +106,27 @@ rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies 
   const rt_fused_operand& o = p->operand[0];
   for (int i = 0; i < rows; ++i)
     for (int j = 0; j < cols; ++j) p->out[0][i * cols + j] = o.ptr[(p->nd == 2 ? i * o.stride[0] : 0) + j * o.stride[p->nd - 1]];
+  return RT_OK;
+}
+// their results stay zero
+rt_status rt_graph_begin(rt_ctx*) { return RT_OK; }
+rt_status rt_graph_end(rt_ctx*, rt_graph**) { return RT_OK; }
+rt_status rt_fill(rt_ctx*, float*, float, int64_t) { return RT_OK; }
+rt_status rt_gemm(rt_ctx*, int, int, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, float*, int64_t, int) { return RT_OK; }
+rt_status rt_gemm_bias_act(rt_ctx*, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, const float*, int, float*, int64_t) { return RT_OK; }
+rt_status rt_matmul_backward(rt_ctx*, const float*, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) { return RT_OK; }
+rt_status rt_gemm_sum_products(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, int64_t, float*) { return RT_OK; }
+rt_status rt_reduce(rt_ctx*, int, const float*, int64_t, int64_t, int64_t, float*) { return RT_OK; }
+rt_status rt_unbroadcast(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return RT_OK; }
+rt_status rt_broadcast_to(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return RT_OK; }
+rt_status rt_slice_assign(rt_ctx*, float*, const int64_t*, int, const int64_t*, const float*, const int64_t*) { return RT_OK; }
+rt_status rt_lstm_sequence(rt_ctx*, const float*, const float*, int64_t, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) {
+  ++forward_sequences;
+  return RT_OK;
+}
+rt_status rt_lstm_sequence_backward(rt_ctx*, const float*, const float*, int64_t, const float*, const float*, int64_t, int64_t, int64_t, float*, float*,
+                                    float*) {
+  ++backward_sequences;
   return RT_OK;
 }
 }
@@ -308,10 +330,56 @@ void a_product_of_a_matrix_with_itself() {
   EXPECT(live.empty());
 }
 
+// An LSTM written op by op, in a capture: one sequence forward; backward one, unless somebody could miss a gradient of what lies between.
+void cells_become_a_sequence() {
+  using Tn = Tensor<B>;
+  const size_t T = 5, Bn = 3, V = 4, H = 2;
+  enum { kPlain, kHeld, kCellUsed, kOtherGates, kStateUsedTwice, kInputsOutOfOrder, kGivenState, kCases };
+  for (int way = 0; way < kCases; ++way) {
+    forward_sequences = backward_sequences = 0;
+    {
+      const Tn x(make({(T + 1) * Bn, V}, 0.f, .01f), false), w(make({V + H, 4 * H}, 0.f, .01f), true), b(make({4 * H}, 0.f, .01f), true);
+      const Tn given(make({Bn, H}, 0.f), false);
+      std::vector<Tn> held;
+      Tn total;
+      B::begin_capture();
+      {
+        Tn h = way == kGivenState ? given : Tn::zeros({Bn, H}, false), c = Tn::zeros({Bn, H}, false), sum;
+        for (size_t t = 0; t < T; ++t) {
+          const size_t r = (way == kInputsOutOfOrder && t == 2 ? t + 2 : t) * Bn;
+          const Tn xh = ops::concat<B>({ops::slice(x, {{r, r + Bn}, {0, V}}), h}, 1);
+          const Tn z = ops::add(ops::matmul(xh, w), b.broadcast_to({Bn, 4 * H}));
+          auto gate = [&](size_t k) { return ops::slice(z, {{0, Bn}, {k * H, (k + 1) * H}}); };
+          const Tn f = ops::sigmoid(gate(way == kOtherGates ? 0 : 1)), i = ops::sigmoid(gate(way == kOtherGates ? 1 : 0));
+          c = ops::add(ops::mul(f, c), ops::mul(i, ops::tanh(gate(2))));
+          h = ops::mul(ops::sigmoid(gate(3)), ops::tanh(c));
+          if (way == kHeld && t == 2) held.push_back(c);
+          Tn out = ops::sum(way == kStateUsedTwice ? ops::mul(h, h) : h, std::nullopt);
+          if (way == kCellUsed && t == 2) out = ops::add(out, ops::sum(c, std::nullopt));
+          sum = t ? ops::add(sum, out) : out;
+        }
+        total = sum;
+      }
+      total.backward();
+      EXPECT(w.grad().has_value() && b.grad().has_value());
+      for (auto& g : {*w.grad(), *b.grad()}) g.ptr();
+      if (way == kHeld) EXPECT(held[0].grad().has_value());
+      total.detach_graph();
+      rt_graph* graph = nullptr;
+      B::end_capture(&graph);
+    }
+    const bool cells = way != kOtherGates && way != kGivenState;  // out of order: the first two timesteps
+    EXPECT(forward_sequences == (cells ? 1 : 0));
+    EXPECT(backward_sequences == (way == kPlain || way == kStateUsedTwice ? 1 : 0));
+    EXPECT(live.empty());
+  }
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
+} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence},
+               {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},
                {"pooling_knows_its_relu", pooling_knows_its_relu},
                {"errors_lose_nothing", errors_lose_nothing},

@@ -6,7 +6,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from helpers import rng
+import rusttensor_b200
+from helpers import assert_close, rng, workload_data
 
 pytestmark = pytest.mark.gpu
 
@@ -77,3 +78,23 @@ def test_sizes_are_checked(capi):
             capi.call("lstm_sequence", x.ptr, x.ptr, i64(16), None, None, *[i64(s) for s in sizes], x.ptr, x.ptr)
     with pytest.raises(Exception, match="leading dimension"):
         capi.call("lstm_sequence", x.ptr, x.ptr, i64(15), None, None, i64(1), i64(2), i64(4), x.ptr, x.ptr)
+
+
+@pytest.mark.parametrize("vocab,hidden,steps,batch", [(7, 9, 2, 3), (65, 24, 2, 17), (30, 200, 33, 16), (50, 130, 5, 40), (12, 64, 140, 4), (20, 512, 3, 90)])
+def test_cells_written_op_by_op_become_a_sequence_in_a_capture(capi, vocab, hidden, steps, batch):
+    dims = [vocab, hidden, steps, batch]
+    params, inputs = workload_data(5, dims, seed=steps)
+    results, launches = [], []
+    for mode in ("step_eager", "step"):
+        tr = rusttensor_b200.DataParallelTrainer(5, dims)
+        for t, p in zip(tr.params, params):
+            t.update_from_host(p)
+        before = capi.launches()
+        for _ in range(2):
+            getattr(tr, mode)(inputs)
+        launches.append(capi.launches() - before)
+        results.append([p.numpy() for p in tr.params] + [tr.state(0, i).numpy() for i in range(len(params))] + [np.array(tr.last_loss())])
+    if steps > 10:
+        assert launches[1] < 2 * steps < launches[0]
+    for a, b in zip(*results):  # two orders of the same fp32 sums, an Adam step of 1e-3 behind them
+        assert_close(b, a, 1e-4, "captured and eager", abs_floor=5e-7)
