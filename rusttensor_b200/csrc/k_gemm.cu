@@ -31,6 +31,12 @@ rt_status rt_gemm_parts_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t 
 float rt_gemm_parts_estimate(const rt_ctx* ctx, int64_t m, int64_t n, int64_t k);
 rt_status rt_matmul_backward_parts_internal(rt_ctx* ctx, const float* a, const float* b, const float* g, int64_t m, int64_t k, int64_t n, float* da,
                                             float* db, int accumulate_db);
+rt_status rt_conv_forward_parts_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y);
+rt_status rt_conv_gather_parts_internal(rt_ctx* ctx, const float* y, const float* w, const float* bias, const ConvGeom& g, int cm, float* out);
+rt_status rt_conv_backward_parts_internal(rt_ctx* ctx, const float* x, const float* w, const float* y, const ConvGeom& g, float* dx, float* dw, float* db);
+rt_status rt_conv_transpose_backward_parts_internal(rt_ctx* ctx, const float* x, const float* w, const float* y, const ConvGeom& g, float* dy, float* dw,
+                                                    float* db);
+rt_status rt_conv_weight_grad_parts_internal(rt_ctx* ctx, const float* x, const float* y, const ConvGeom& g, float* dw, float* db);
 rt_status rt_conv_forward_tma_internal(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y);
 rt_status rt_conv_gather_tma_internal(rt_ctx* ctx, const float* y, const float* w, const float* bias, const ConvGeom& g, int cm, float* out);
 rt_status rt_gemm_small_list_internal(rt_ctx* ctx, int count, const float* const* a, float* const* c, int64_t m, int64_t n, int64_t k,
@@ -513,6 +519,19 @@ rt_status check_conv_args(rt_ctx* ctx, int64_t n, int64_t cin, int64_t h, int64_
   return RT_OK;
 }
 
+int64_t conv_work(const ConvGeom& g) { return (int64_t)g.Nb * g.Hy * g.Wy * g.Cy * g.Cx * g.kh * g.kw; }
+// Which kernels take a convolution, after those for single channels and for up to 64 output channels at unit stride: 16-bit parts from about 2^30
+// multiply-adds on (64 x 33 x 30 x 30 to 70 channels 55 us, as 3xTF32 70; 90 x 48 x 29 x 37 to 96 at stride 2 68 and 87), then TMA-fed 3xTF32.
+// Gradients: where both are wanted, the images' parts serve both.  At unit stride the kernels that read fp32 rows directly are ahead until
+// there is more to do, and with few input channels (both gradients, multiply-adds: 64 x 64 x 28 x 28 to 64, 1.9 G, 99 us and 74; 1000 x 32 x 14
+// x 14 to 64, 3.6 G, 214 and 142; 128 x 40 x 40 x 40 to 80, 5.9 G, 324 and 463; 128 x 64 x 56 x 56 to 128, 30 G, 693 and 890); strided ones are
+// not (transposed 128 x 80 x 20 x 20 to 40, 2.6 G, 172 and 194; 128 x 128 x 28 x 28 to 64, 13 G, 301 and 515).
+constexpr int64_t kPartsGradWork = int64_t(1) << 31;
+bool parts_backward(const rt_ctx* ctx, const ConvGeom& g) {
+  if (!ctx->use_tensor_cores || !ctx->use_tma_weight_grad) return false;
+  return g.sh > 1 || g.sw > 1 ? conv_work(g) >= kPartsGradWork : conv_work(g) >= 2 * kPartsGradWork && g.Cx > 32;
+}
+
 // y[Nb,Cy,Hy,Wy] = conv(x[Nb,Cx,Hx,Wx], w[Cy,Cx,kh,kw]) (+bias)
 rt_status conv_forward_like(rt_ctx* ctx, const float* x, const float* w, const float* bias, const ConvGeom& g, float* y) {
   int64_t M = g.Cy, N = (int64_t)g.Nb * g.Hy * g.Wy, K = (int64_t)g.Cx * g.kh * g.kw;
@@ -527,7 +546,9 @@ rt_status conv_forward_like(rt_ctx* ctx, const float* x, const float* w, const f
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   if (ctx->use_tensor_cores) {
-    rt_status st = rt_conv_forward_tma_internal(ctx, x, w, bias, g, y);
+    rt_status st = rt_conv_forward_parts_internal(ctx, x, w, bias, g, y);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+    st = rt_conv_forward_tma_internal(ctx, x, w, bias, g, y);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
     st = rt_conv_forward_tc_internal(ctx, x, w, bias, g, y);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
@@ -546,6 +567,11 @@ rt_status conv_weight_grad_like(rt_ctx* ctx, const float* x, const float* y, con
                                 bool* db_done = nullptr) {
   int64_t M = g.Cy, N = (int64_t)g.Cx * g.kh * g.kw, K = (int64_t)g.Nb * g.Hy * g.Wy;
   if (db_done) *db_done = false;
+  if (ctx->use_tensor_cores && (g.sh > 1 || g.sw > 1) && conv_work(g) >= kPartsGradWork) {
+    rt_status st = rt_conv_weight_grad_parts_internal(ctx, x, y, g, dw, db);
+    if (st == RT_OK && db && db_done) *db_done = true;
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+  }
   if (ctx->use_tensor_cores && ctx->use_tma_weight_grad && M > 0 && N > 0 && K > 0) {  // unit stride: TMA-fed, pixels as K
     rt_status st = rt_conv_dw_tma_internal(ctx, x, y, g, dw, db);
     if (st == RT_OK && db && db_done) *db_done = true;
@@ -576,7 +602,9 @@ rt_status conv_gather_like(rt_ctx* ctx, const float* y, const float* w, const fl
     if (st != RT_ERR_UNIMPLEMENTED) return st;
   }
   if (ctx->use_tensor_cores) {
-    rt_status st = rt_conv_gather_tma_internal(ctx, y, w, bias, g, cm, out);
+    rt_status st = rt_conv_gather_parts_internal(ctx, y, w, bias, g, cm, out);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+    st = rt_conv_gather_tma_internal(ctx, y, w, bias, g, cm, out);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
     st = rt_conv_gather_tc_internal(ctx, y, w, bias, g, cm, out);
     if (st != RT_ERR_UNIMPLEMENTED) return st;
@@ -903,6 +931,11 @@ rt_status rt_conv2d_backward(rt_ctx* ctx, const float* x, const float* w, const 
   if (st != RT_OK) return st;
   if (h + 2 * ph < kh || wd + 2 * pw < kw) RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "conv2d_backward: kernel larger than padded input");
   ConvGeom g = make_geom(n, cin, h, wd, cout, kh, kw, sh, sw, ph, pw);
+  if (dx && dw && parts_backward(ctx, g)) {
+    st = rt_conv_backward_parts_internal(ctx, x, w, gr, g, dx, dw, db);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+    st = RT_OK;
+  }
   // The three gradients are independent.  The bias gradient (bandwidth-bound, small footprint) goes to the side stream,
   // where it overlaps the contraction kernels.
   RtFork fork(ctx, db && (dw || dx));
@@ -959,6 +992,11 @@ rt_status rt_conv2d_transpose_backward(rt_ctx* ctx, const float* x, const float*
   g.Hy = (int)h;
   g.Wy = (int)wd;
   g.finish();
+  if (dx && dw && parts_backward(ctx, g)) {
+    st = rt_conv_transpose_backward_parts_internal(ctx, gr, w, x, g, dx, dw, db);
+    if (st != RT_ERR_UNIMPLEMENTED) return st;
+    st = RT_OK;
+  }
   // as in rt_conv2d_backward: bias gradient (and the weight gradient, when dx is wanted too) on the side stream
   RtFork fork(ctx, db && (dw || dx));
   rt_status st_side = RT_OK;

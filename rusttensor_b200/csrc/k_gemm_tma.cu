@@ -1,12 +1,11 @@
-// Large products and convolutions on the tensor cores (tcgen05 3xTF32), operands fetched by TMA.
+// Products of more than one wave of small tiles and convolutions on the tensor cores (tcgen05 3xTF32), operands fetched by TMA; the largest of
+// either go to k_gemm_parts.cu and k_conv_parts.cu.
 //
 // What bounds a 3xTF32 product is the 128 B/cycle shared-memory path, not the tensor pipe: an fp32 operand element is 4 bytes as
 // TMA brings it, and every copy, split and operand read of an MMA crosses that path.  This kernel therefore
 //  * feeds the raw fp32 tile to the MMA as the hi operand - the tensor core ignores the low 13 mantissa bits of a TF32 operand,
 //    which is the truncation hi = a & 0xffffe000 - so that only lo = a - hi has to be made;
-//  * keeps the A operand (hi and lo) in tensor memory, from which an MMA reads at no cost to shared memory;
-//  * uses 128 x 256 output tiles for products where these fill their waves: per K-step of 8, 57 KB over shared memory against 384 cycles
-//    of MMAs.
+//  * keeps the A operand (hi and lo) in tensor memory, from which an MMA reads at no cost to shared memory.
 // The tensor core adds every partial product into its fp32 accumulator with truncation: on one accumulator over the whole reduction
 // the error grows to 2.9e-5 of the result at 4096.  An accumulator is therefore emptied after every K-block of 32, or every
 // few, and these are summed in registers with rounding (error 3.5e-7 - 1e-6 whatever the length); accumulators are used in turn, so
@@ -14,8 +13,8 @@
 // Roles of a CTA (one per SM, walking over tiles): one TMA warp several K-blocks ahead; six converter warps (A raw -> tensor
 // memory hi / lo; B raw -> B lo at the same swizzled address, so the swizzle needs no decoding), four of them at work where B comes
 // already split; one MMA warp; eight accumulating warps, which also write the result.
-// Measured: 4096^3 0.66 ms = 208 TFLOP/s of fp32-equivalent work, before 0.92 - 1.37 ms; 1024^3 31 us, before 40 - 45 us.  Without the
-// conversions (in a copy made for timing) the MMAs and copies alone take 0.43 ms: shared memory is what is full.
+// Measured: 1024^3 31 us.  Without the conversions (in a copy made for timing) the MMAs and copies of a large product take two thirds of its
+// time: shared memory is what is full.
 // A operand: a matrix with the reduction contiguous, one with the rows contiguous, or the pixels of a channels-last image at one
 // kernel tap (4-D boxes, zeros outside the image, element strides for strided convolutions: no im2col buffer).  B operand: a
 // matrix with the reduction contiguous.  Whatever is not in such a form or not 16-byte aligned is brought into it by one pass of
@@ -40,17 +39,16 @@ constexpr uint32_t kARaw = BM * BK * 4;  // 16 KB
 // SPLIT: B comes as two matrices, hi and lo (the packed weights of a convolution, used by every tile).
 template <int BN, bool SPLIT>
 struct Config {
-  static constexpr int NU = BN < 128 ? BN : 128;  // columns of one MMA and of one accumulator
-  static constexpr int halves = BN / NU;
-  // The two groups of accumulating warps: each takes one half of a 256-column tile; or they take turns, a tile each, so that one writes a
-  // result while the other sums the next tile (convolutions: short reductions, scattered stores); or each takes half the columns.
+  static_assert(BN <= 128, "columns of one MMA and of one accumulator");
+  // The two groups of accumulating warps: each takes half the columns; or they take turns, a tile each, so that one writes a
+  // result while the other sums the next tile (convolutions: short reductions, scattered stores).
   static constexpr bool turns = SPLIT;
-  static constexpr int NC = halves == 2 || turns ? NU : NU / 2;
-  static constexpr int ACC = BN == 256 ? 3 : 2;   // accumulators, used in turn
-  static constexpr int L = BN == 256 ? 2 : 4;     // converted A (tensor memory) and B lo
+  static constexpr int NC = turns ? BN : BN / 2;
+  static constexpr int ACC = 2;                   // accumulators, used in turn
+  static constexpr int L = 4;                     // converted A (tensor memory) and B lo
   static constexpr uint32_t b_raw = BN * BK * 4;
   static constexpr uint32_t raw = kARaw + (SPLIT ? 2 : 1) * b_raw;
-  static constexpr int R = BN == 256 ? 3 : (BN == 64 && SPLIT ? 6 : 4);  // raw tiles in flight
+  static constexpr int R = BN == 64 && SPLIT ? 6 : 4;  // raw tiles in flight
   static constexpr uint32_t lo_offset = R * raw;
   static constexpr uint32_t stage_offset = lo_offset + (SPLIT ? 0 : L * b_raw);  // result: one 32 x 17 tile per accumulating warp
   static constexpr uint32_t bar_offset = stage_offset + kEpilogueWarps * 32 * 17 * 4;
@@ -58,7 +56,7 @@ struct Config {
   static constexpr uint32_t total = bar_offset + n_bars * 8 + 16 + 1024;  // + alignment of the base to 1024
   static constexpr uint32_t a_cols = 2 * BK;                              // tensor-memory columns of a converted A block
   static constexpr int converters = SPLIT ? 4 : kConverterWarps;
-  static_assert(ACC * NU + L * a_cols <= 512, "tensor memory");
+  static_assert(ACC * BN + L * a_cols <= 512, "tensor memory");
   static_assert(total <= 232448, "shared memory");
 };
 
@@ -171,7 +169,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     for (int i = 0; i < C::ACC; ++i) {
       mbar_init(acc_full(0, i), 1);
       mbar_init(acc_full(1, i), 1);
-      mbar_init(acc_empty(i), C::halves == 2 || C::turns ? kEpilogueWarps / 2 : kEpilogueWarps);
+      mbar_init(acc_empty(i), C::turns ? kEpilogueWarps / 2 : kEpilogueWarps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -180,7 +178,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  const uint32_t tmem_a = tmem + C::ACC * C::NU;
+  const uint32_t tmem_a = tmem + C::ACC * BN;
   bool ok = true;
 
   if (warp == kTmaWarp) {
@@ -223,7 +221,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else if (warp == kMmaWarp) {
     // ---------------- MMAs ----------------
-    constexpr uint32_t idesc = make_idesc(C::NU);
+    constexpr uint32_t idesc = make_idesc(BN);
     constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // 8-row groups of 1024 bytes, 128-byte swizzle
     int it = 0, chunks = 0, t = 0;  // chunks that are complete
     for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++t) {
@@ -238,21 +236,16 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const uint32_t b_hi = ((base + s * C::raw + kARaw) >> 4 & 0x3FFF) | (1u << 16);
         const uint32_t b_lo = ((SPLIT ? base + s * C::raw + kARaw + C::b_raw : base + C::lo_offset + l * C::b_raw) >> 4 & 0x3FFF) | (1u << 16);
         const uint32_t a_hi = tmem_a + l * C::a_cols, a_lo = a_hi + BK;
+        const int acc = chunks % C::ACC, use = chunks / C::ACC;
+        if (first && use > 0) {
+          ok = __all_sync(0xffffffffu, wait(acc_empty(acc), (use - 1) & 1, status, 43, &abort_flag));
+          tc_fence_after();
+        }
+        if (ok) {
 #pragma unroll
-        for (int h = 0; h < C::halves; ++h) {
-          const int unit = chunks * C::halves + h, acc = unit % C::ACC, use = unit / C::ACC;
-          if (first && use > 0 && ok) {
-            ok = __all_sync(0xffffffffu, wait(acc_empty(acc), (use - 1) & 1, status, 43, &abort_flag));
-            tc_fence_after();
-          }
-          if (ok) {
-            constexpr uint32_t half_rows = C::NU * 128 / 16;
-#pragma unroll
-            for (int j = 0; j < BK / 8; ++j)
-              mma_step(tmem + acc * C::NU, a_hi + 8 * j, a_lo + 8 * j, b_hi + h * half_rows + 2 * j, b_lo + h * half_rows + 2 * j, desc_hi, idesc,
-                       first && j == 0 ? 0u : 1u);
-            if (last) umma_commit_elect(acc_full(C::halves == 2 ? h : (C::turns ? t & 1 : 0), acc));
-          }
+          for (int j = 0; j < BK / 8; ++j)
+            mma_step(tmem + acc * BN, a_hi + 8 * j, a_lo + 8 * j, b_hi + 2 * j, b_lo + 2 * j, desc_hi, idesc, first && j == 0 ? 0u : 1u);
+          if (last) umma_commit_elect(acc_full(C::turns ? t & 1 : 0, acc));
         }
         if (ok) {
           umma_commit_elect(raw_empty(s));
@@ -321,8 +314,8 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   } else if (warp < kEpilogueWarps) {
     // ---------------- sums over the K-blocks, result ----------------
     float* stage = reinterpret_cast<float*>(smem + C::stage_offset) + warp * 32 * 17;
-    const int quad = warp & 3, group = warp >> 2, full = C::halves == 2 || C::turns ? group : 0;
-    const int col0 = C::halves == 2 ? group * C::NU : (C::turns ? 0 : group * C::NC);  // of this warp's columns in the tile
+    const int quad = warp & 3, group = warp >> 2, full = C::turns ? group : 0;
+    const int col0 = C::turns ? 0 : group * C::NC;  // of this warp's columns in the tile
     const int chunks = (p.k_blocks + p.chunk - 1) / p.chunk;  // of a tile
     int t = 0;
     uint32_t phases = 0;  // bit i: parity of this group's next use of accumulator i
@@ -332,12 +325,12 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
       for (int j = 0; j < C::NC; ++j) sum[j] = 0.f;
       for (int i = 0; i < chunks && ok; ++i) {
-        const int unit = (t * chunks + i) * C::halves + (C::halves == 2 ? group : 0), acc = unit % C::ACC;
+        const int acc = (t * chunks + i) % C::ACC;
         ok = __all_sync(0xffffffffu, wait(acc_full(full, acc), (phases >> acc) & 1, status, 48, &abort_flag));
         if (!ok) break;
         phases ^= 1u << acc;
         tc_fence_after();
-        const uint32_t d = tmem + acc * C::NU + (C::halves == 2 ? 0 : col0) + ((uint32_t)(quad * 32) << 16);
+        const uint32_t d = tmem + acc * BN + col0 + ((uint32_t)(quad * 32) << 16);
 #pragma unroll
         for (int c = 0; c < C::NC; c += 16) {
           uint32_t v[16];
@@ -525,12 +518,8 @@ rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m,
                                int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   using namespace tc::tma;
   if (m >= (1 << 24) || n >= (1 << 24) || k >= (1 << 24)) return RT_ERR_UNIMPLEMENTED;
-  const int64_t mt = (m + BM - 1) / BM, t256 = mt * ((n + 255) / 256), t128 = mt * ((n + 127) / 128);
+  const int64_t mt = (m + BM - 1) / BM, nt = (n + 127) / 128;
   if ((m + 31) / 32 > 65535 || (k + 31) / 32 > 65535 || (n + 31) / 32 > 65535) return RT_ERR_UNIMPLEMENTED;
-  const auto waves = [&](int64_t t) { return (t + ctx->sm_count - 1) / ctx->sm_count; };
-  // 256 columns cost twice the time of 128 and less of shared memory, unless the last wave of the larger tiles stands emptier (4096^3: 4 waves
-  // of 512 tiles against 7 of 1024, so 128)
-  const bool wide = waves(t256) * 2 <= waves(t128);
   auto direct = [](const float* p, int64_t ld) { return rt_aligned16(p) && ld % 4 == 0; };
   RtScratch wa(ctx), wb(ctx);
   Params p{};
@@ -538,7 +527,7 @@ rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m,
   CUtensorMap ma, mb;
   bool mapped = true;
   rt_status st = RT_OK;
-  // A with the rows contiguous is read from shared memory a word at a time; from eight tile columns on, turning it once is cheaper
+  // A with the rows contiguous is read from shared memory a word at a time; from sixteen tile columns on, turning it once is cheaper
   // (4096^3: 0.70 against 0.76 ms)
   if (trans_a && direct(a, lda) && n < 2048) {
     p.a_mode = kRowsMajorM;
@@ -564,7 +553,7 @@ rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m,
     st = trans_b ? pack(ctx, b, wb.as<float>(), n, k, ldb, ld, false, 1, 0, 0) : pack(ctx, b, wb.as<float>(), k, n, ldb, ld, true, 1, 0, 0);
     if (st != RT_OK) return st;
   }
-  mapped = mapped && map_matrix(&mb, q, k, n, ld, BK, wide ? 256 : 128, true);
+  mapped = mapped && map_matrix(&mb, q, k, n, ld, BK, 128, true);
   if (!mapped) return RT_ERR_UNIMPLEMENTED;
   p.M = (int)m;
   p.N = (int)n;
@@ -574,12 +563,12 @@ rt_status rt_gemm_tma_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t m,
   p.act = act;
   p.accumulate = accumulate;
   p.m_tiles = (int)mt;
-  p.tiles = (int)(wide ? t256 : t128);
+  p.tiles = (int)(mt * nt);
   p.k_blocks = (int)((k + BK - 1) / BK);
   p.c_blocks = p.k_blocks;
   p.chunk = chunk_of(k);
   p.kw = 1;
-  return wide ? launch<256>(ctx, ma, mb, p) : launch<128>(ctx, ma, mb, p);
+  return launch<128>(ctx, ma, mb, p);
 }
 
 namespace tc {

@@ -42,3 +42,39 @@ def test_convolution(api, n, cin, h, w, cout, k, s, p, transposed):
     api.call(name + "_backward", dev[0].ptr, dev[1].ptr, dev[3].ptr, *dims, dx.ptr, None, None)
     for got, want in ((y.numpy()[some], ref), (dx.numpy()[some], bwd(x[some], wt, g[some], (s, s), (p, p))[0])):
         assert np.all(np.abs(got - want) <= 4e-6 * np.abs(want).max() + 1e-6 * np.abs(want))
+
+
+# The 16-bit parts (k_conv_parts.cu): from 2^30 multiply-adds on, both gradients from 2^31 (strided) and 2^32.  Channels that leave K-blocks and
+# column tiles ragged, boxes that overhang, odd output extents of a stride of two, and inputs that need three parts.
+PARTS = [(65, 70, 29, 31, 66, 3, 1, 1), (130, 40, 40, 38, 84, 3, 1, 1), (96, 33, 37, 35, 97, 4, 2, 1), (70, 66, 33, 30, 68, 5, 2, 2)]
+
+
+@pytest.mark.parametrize("spread", [False, True])
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("n,cin,h,w,cout,k,s,p", PARTS)
+def test_convolution_of_parts(api, n, cin, h, w, cout, k, s, p, transposed, spread):
+    r = np.random.default_rng(n + cin + h)
+    x = r.standard_normal((n, cin, h, w)).astype(np.float32)
+    if spread:  # one channel far below the others
+        x[:, cin // 2] *= np.float32(2.0**-30)
+    wt = (r.standard_normal((cin, cout, k, k) if transposed else (cout, cin, k, k)) / k).astype(np.float32)
+    b = r.standard_normal(cout).astype(np.float32)
+    some = [0, n // 2, n - 1]
+    name, fwd, bwd = (("conv2d_transpose", ref_f64.conv2d_transpose, ref_f64.conv2d_transpose_backward) if transposed
+                      else ("conv2d", ref_f64.conv2d, ref_f64.conv2d_backward))
+    ref = fwd(x[some], wt, b, (s, s), (p, p))
+    y, dx, dw, db = api.empty((n,) + ref.shape[1:]), api.empty(x.shape), api.empty(wt.shape), api.empty(b.shape)
+    g = np.zeros(y.shape, np.float32)  # the weight gradient is checked too: upstream gradient in the images that the reference looks at
+    g[some] = r.standard_normal((3,) + y.shape[1:]).astype(np.float32)
+    dev = [api.to_device(v) for v in (x, wt, b, g)]
+    dims = (i64(n), i64(cin), i64(h), i64(w), i64(cout), k, k, s, s, p, p)
+    api.call(name, dev[0].ptr, dev[1].ptr, dev[2].ptr, *dims, y.ptr)
+    api.call(name + "_backward", dev[0].ptr, dev[1].ptr, dev[3].ptr, *dims, dx.ptr, dw.ptr, db.ptr)
+    want = bwd(x[some], wt, g[some], (s, s), (p, p))
+    rows, cols = cin * k * k, y.shape[2] * y.shape[3] * 3
+    # relative to the root of the number of terms: 32 additions with truncation between roundings, the parts' own 2^-22
+    for got, ref_, terms in ((y.numpy()[some], ref, rows), (dx.numpy()[some], want[0], cout * k * k), (dw.numpy(), want[1], cols), (db.numpy(), want[2], cols)):
+        assert np.abs(got - ref_).max() <= (32 * 2.0**-23 + 2.0**-21) * (np.abs(ref_).max() + np.sqrt(terms))
+    if spread and not transposed:  # the small channel's weight gradient has its own scale
+        small, ref_ = dw.numpy()[:, cin // 2], want[1][:, cin // 2]
+        assert np.abs(small - ref_).max() <= 4e-6 * np.abs(ref_).max() + 1e-6 * np.abs(ref_).max()

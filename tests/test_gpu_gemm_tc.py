@@ -95,7 +95,7 @@ def test_product_of_parts(capi, m, n, k, ta, tb, inputs):
         A, B = A * np.float32(1e-25), B * np.float32(3e20)
     before = capi.launches()
     got = gemm(capi, ta, tb, m, n, k, np.ascontiguousarray(A.T) if ta else A, np.ascontiguousarray(B.T) if tb else B)
-    assert capi.launches() - before <= 3 + (k < 256)  # magnitudes, parts, product (short reductions go to another kernel)
+    assert capi.launches() - before <= 4  # a sample, two parts, perhaps three, the product
     assert parts_error(got, A, B) < PARTS_BOUND
 
 
