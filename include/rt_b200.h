@@ -116,7 +116,8 @@ void* rt_stream(rt_ctx* ctx);                                                   
 rt_status rt_mem_stats(rt_ctx* ctx, int64_t* bytes_reserved, int64_t* bytes_in_use, int64_t* n_device_allocs);
 rt_status rt_kernel_launch_count(rt_ctx* ctx, int64_t* launches);                    /* kernels launched by this library so far */
 /* Elementwise programs run so far, by what ran them: a kernel compiled for them, or the interpreter.  A program is a launch of
- * rt_fused_elementwise, or one of the two that a timestep of rt_lstm_sequence or of its backward pass holds. */
+ * rt_fused_elementwise, rt_fused_column_sums or rt_fused_logsumexp, or one of the two that a timestep of rt_lstm_sequence or of its backward
+ * pass holds. */
 rt_status rt_fused_launch_counts(rt_ctx* ctx, int64_t* compiled, int64_t* interpreted);
 /* Synchronises and reads the device error word: kernels that wait on barriers give up after a bounded
  * number of polls, record a code there and return; non-zero -> RT_ERR_TIMEOUT (and the word is cleared). */
@@ -264,6 +265,11 @@ typedef struct {
   rt_fused_instr code[RT_FUSED_MAX_CODE];
 } rt_fused_program;
 rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* program);
+/* The same for a program over [rows, columns] (nd = 2), with a reduction of one of its outputs in the same launch, where a kernel has been
+ * compiled for that (otherwise RT_ERR_UNIMPLEMENTED, and nothing has been done): the column sums of output `which`, which itself is not
+ * written (its pointer only has to be valid); the logsumexp of the rows of output 0, which is. */
+rt_status rt_fused_column_sums(rt_ctx* ctx, const rt_fused_program* program, int which, float* sums);
+rt_status rt_fused_logsumexp(rt_ctx* ctx, const rt_fused_program* program, float* out);
 
 /* out[i, :] = src[idx[i], :] (idx: n_idx int32 row numbers in DEVICE memory): the row gather of data::get_random_batch
  * (src/data.rs:125-209), done on the device instead of through a host copy of the whole data set. */

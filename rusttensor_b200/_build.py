@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, "librt_b200.so")
 HOST_LIB = os.path.join(HERE, "librt_b200_host.so")
 FAST_LIB = os.path.join(HERE, "_fastcall.so")
 
-CU_SOURCES = ["rt_context.cu", "k_elementwise.cu", "k_fused.cu", "k_fused_known.cu", "k_fused_lstm.cu", "k_reduce.cu", "k_pool.cu", "k_optim.cu", "k_gemm.cu", "k_gemm_small.cu", "k_gemm_tma.cu", "k_gemm_tc.cu", "k_gemm_parts.cu", "k_conv_parts.cu", "k_conv_tc.cu", "k_conv_thin.cu", "k_lstm.cu", "k_lstm_seq.cu", "k_tc_probe.cu", "k_conv_dw_tc.cu", "k_random.cu"]
+CU_SOURCES = ["rt_context.cu", "k_elementwise.cu", "k_fused.cu", "k_fused_known.cu", "k_fused_lstm.cu", "k_fused_reduced.cu", "k_reduce.cu", "k_pool.cu", "k_optim.cu", "k_gemm.cu", "k_gemm_small.cu", "k_gemm_tma.cu", "k_gemm_tc.cu", "k_gemm_parts.cu", "k_conv_parts.cu", "k_conv_tc.cu", "k_conv_thin.cu", "k_lstm.cu", "k_lstm_seq.cu", "k_tc_probe.cu", "k_conv_dw_tc.cu", "k_random.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-Wno-unused-function"]
 

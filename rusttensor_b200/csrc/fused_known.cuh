@@ -8,10 +8,9 @@
 // op more or in another form, and the first and last timesteps of the recurrent network, are not (rt_fused_launch_counts tells).
 //
 // Measured, kernel time inside a graph: the gate gradient of the LSTM cell (30 instructions, 12 operands, 4 windows) on [64, 2048]
-// 12.5 us interpreted, 4.2 us compiled; the 33 instructions of an elementwise gradient with four transcendentals on [4096, 4096] 300
-// us interpreted, 77 us compiled (its 268 MB take 41 us at the copy bandwidth: bound by instruction issue).  Mean of the logsumexp of
-// exp(-x^2) + tanh(x b) + sin(x) / (1 + x^2) over such a matrix, forward and backward from the front end: 465 us with square(x), where two
-// of three programs are listed, 560 us with x * x, where one is.
+// 12.5 us interpreted, 4.2 us compiled; an elementwise gradient with four transcendentals on [4096, 4096] 300 us interpreted, 77 us
+// compiled (its 268 MB take 41 us at the copy bandwidth: bound by instruction issue, as everything here that has more than two or three
+// transcendentals an element is).  Issue slots that a warp takes for one: exp 9, tanh 19, sin 27, cos 29, both by sincosf 34, 1/x 14, x/y 15.
 #pragma once
 #define RT_FUSED_EXPAND_MATH
 #include "fused_common.cuh"
@@ -72,20 +71,58 @@ __device__ __forceinline__ float apply_one(float x, float y, float imm) {
   return x;
 }
 
-template <class P, int PC, bool VEC>
-__device__ __forceinline__ void execute(const FusedParams& p, const Quad<VEC>& e, float (&r)[RT_FUSED_REGS][4], float (&acc)[4]) {
+// What becomes of an output: it is written.
+struct Store {
+  template <int OUT, bool VEC>
+  __device__ __forceinline__ void put(const FusedParams& p, const Quad<VEC>& e, const float (&acc)[4]) {
+#pragma unroll
+    for (int g = 0; g < Quad<VEC>::G; ++g)
+      if (e.live[g]) {
+        if constexpr (VEC) *reinterpret_cast<float4*>(p.out[OUT] + e.at[g]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        else p.out[OUT][e.at[g]] = acc[g];
+      }
+  }
+};
+
+// A sine and a cosine of one register's value, the earlier (first) and the later instruction: sincosf reduces the argument once for both (the
+// program with column sums over [4096, 4096] that has them: 98 us apart, 88 us together, without a spill).
+struct Pair {
+  int first = -1, later = -1;
+};
+template <class P>
+__host__ __device__ constexpr Pair find_pair() {
+  auto op = [](int i) { return P::code[i] & 0xff; };
+  for (int i = 1; i < P::n; ++i)
+    for (int j = i + 2; j < P::n && op(i - 1) == RT_F_REG; ++j) {
+      const uint32_t reg = (P::code[i - 1] >> 8) & 0xff;
+      bool same = ((op(i) == RT_F_SIN && op(j) == RT_F_COS) || (op(i) == RT_F_COS && op(j) == RT_F_SIN)) && op(j - 1) == RT_F_REG &&
+                  ((P::code[j - 1] >> 8) & 0xff) == reg;
+      for (int k = i; k < j && same; ++k) same = ((P::code[k] >> 16) & 0xff) != reg;
+      if (same) return {i, j};
+    }
+  return {};
+}
+
+template <class P, int PC, bool VEC, class Sink>
+__device__ __forceinline__ void execute(const FusedParams& p, const Quad<VEC>& e, float (&r)[RT_FUSED_REGS][4], float (&other)[4], float (&acc)[4], Sink& sink) {
   if constexpr (PC < P::n) {
     constexpr uint32_t word = P::code[PC];
     constexpr int op = word & 0xff, src = (word >> 8) & 0xff, dst = (word >> 16) & 0xff, region = word >> 24;
+    constexpr Pair pair = find_pair<P>();
     if constexpr (op == RT_F_LOAD) {
       load_operand<src, VEC>(p, e, acc);
     } else if constexpr (op == RT_F_OUT) {
+      sink.template put<src, VEC>(p, e, acc);
+    } else if constexpr (PC == pair.later) {
 #pragma unroll
-      for (int g = 0; g < Quad<VEC>::G; ++g)
-        if (e.live[g]) {
-          if constexpr (VEC) *reinterpret_cast<float4*>(p.out[src] + e.at[g]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-          else p.out[src][e.at[g]] = acc[g];
-        }
+      for (int i = 0; i < 4; ++i) acc[i] = other[i];
+    } else if constexpr (PC == pair.first) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float x = acc[i];
+        if constexpr (op == RT_F_SIN) sincosf(x, &acc[i], &other[i]);
+        else sincosf(x, &other[i], &acc[i]);
+      }
     } else {
       const float imm = __uint_as_float(p.code[PC].y);
 #pragma unroll
@@ -101,8 +138,19 @@ __device__ __forceinline__ void execute(const FusedParams& p, const Quad<VEC>& e
 #pragma unroll
       for (int i = 0; i < 4; ++i) r[dst][i] = acc[i];
     }
-    execute<P, PC + 1, VEC>(p, e, r, acc);
+    execute<P, PC + 1, VEC>(p, e, r, other, acc, sink);
   }
+}
+// The program for four elements.
+template <class P, bool VEC, class Sink>
+__device__ __forceinline__ void run(const FusedParams& p, const Quad<VEC>& e, Sink& sink) {
+  float r[RT_FUSED_REGS][4], other[4], acc[4];
+  if constexpr (P::preload > 0) load_operand<0, VEC>(p, e, r[0]);
+  if constexpr (P::preload > 1) load_operand<1, VEC>(p, e, r[1]);
+  if constexpr (P::preload > 2) load_operand<2, VEC>(p, e, r[2]);
+  if constexpr (P::preload > 3) load_operand<3, VEC>(p, e, r[3]);
+  if constexpr (P::preload > 4) load_operand<4, VEC>(p, e, r[4]);
+  execute<P, 0, VEC>(p, e, r, other, acc, sink);
 }
 
 constexpr int kKnownThreads = 128;
@@ -120,13 +168,8 @@ __global__ void __launch_bounds__(kKnownThreads) known_kernel(const __grid_const
       e.c0[g] = (int)q;
       e.c1[g] = (int)m;
     }
-    float r[RT_FUSED_REGS][4], acc[4];
-    if constexpr (P::preload > 0) load_operand<0, VEC>(p, e, r[0]);
-    if constexpr (P::preload > 1) load_operand<1, VEC>(p, e, r[1]);
-    if constexpr (P::preload > 2) load_operand<2, VEC>(p, e, r[2]);
-    if constexpr (P::preload > 3) load_operand<3, VEC>(p, e, r[3]);
-    if constexpr (P::preload > 4) load_operand<4, VEC>(p, e, r[4]);
-    execute<P, 0, VEC>(p, e, r, acc);
+    Store sink;
+    run<P, VEC>(p, e, sink);
   }
 }
 

@@ -605,10 +605,13 @@ Tensor<B> log_softmax(const Tensor<B>& x, size_t axis) {
   Tensor<B> fname(const Tensor<B>& x, std::optional<size_t> axis) {                               \
     St<B> out = B::fname(x.data(), axis);                                                         \
     bool rg = x.requires_grad();                                                                  \
-    return Tensor<B>::new_with_op(std::move(out), rg,                                             \
-                                  rg ? std::optional<OpType>(OpType::with_axis(OpType::KIND, axis)) \
-                                     : std::nullopt,                                              \
-                                  {x});                                                           \
+    Tensor<B> t = Tensor<B>::new_with_op(std::move(out), rg,                                      \
+                                         rg ? std::optional<OpType>(OpType::with_axis(OpType::KIND, axis)) \
+                                            : std::nullopt,                                       \
+                                         {x});                                                    \
+    if constexpr (KeepsOutputs<B>::value && OpType::KIND == OpType::LogSumExp)                     \
+      if (rg) t.inner->op->cached_outputs = t.data();                                             \
+    return t;                                                                                     \
   }
 RT_REDUCE_OP(mean, Mean)            // src/ops/mod.rs:614-632
 RT_REDUCE_OP(max, Max)              // src/ops/mod.rs:885-903

@@ -767,7 +767,10 @@ struct B200Backend {
         return rt_reduce(ctx(), kind, n.in[0].buf->data(), a.outer, a.len, a.inner, out);
       });
     Storage out = alloc(a.out_shape);
-    check(rt_reduce(ctx(), kind, x.ptr(), a.outer, a.len, a.inner, out.ptr()));
+    const bool fused = kind == RT_RED_LOGSUMEXP && a.inner == 1 && !x.shape.empty() && a.len == (int64_t)x.shape.back() && x.buf && x.buf->node &&
+                       x.buf->node->shape == x.shape && lazy::evaluate_with_logsumexp(x.buf.get(), out.buf->ptr);
+    if (!fused) check(rt_reduce(ctx(), kind, x.ptr(), a.outer, a.len, a.inner, out.ptr()));
+    if (x.buf) out.buf->made_from = x.buf->id;
     return out;
   }
   static Storage sum_along_axis(const Storage& x, size_t axis) { return reduce(RT_RED_SUM, x, axis); }
@@ -838,7 +841,20 @@ struct B200Backend {
   static Storage max_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_MAX, o, g, "max"); }
   static Storage min_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_MIN, o, g, "min"); }
   static Storage prod_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_PROD, o, g, "prod"); }
-  static Storage logsumexp_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_LOGSUMEXP, o, g, "logsumexp"); }
+  static Storage logsumexp_backward(const OpB& o, const Storage& g) {
+    // g exp(x - logsumexp(x)): elementwise, with the forward result, unless it or x may have been changed since
+    if (o.inputs.size() == 1 && o.cached_outputs && o.cached_outputs->buf) {
+      const Storage &x = o.inputs[0].data(), &lse = *o.cached_outputs;
+      const Axis3 a = split(x.shape, o.op_type.axis);
+      if (x.buf && a.inner == 1 && !x.shape.empty() && a.len == (int64_t)x.shape.back() && deferrable(x.shape) && lse.buf->made_from == x.buf->id &&
+          (int64_t)g.numel() == a.outer && lse.numel() == g.numel() && ((!x.buf->escaped && !lse.buf->escaped) || lazy::capturing())) {
+        Shape rows = x.shape;
+        rows.back() = 1;
+        return lz_binary(RT_F_MUL, reshaped(g, rows), lz_unary(RT_F_EXP, lz_binary(RT_F_SUB, x, reshaped(lse, rows), x.shape)), x.shape);
+      }
+    }
+    return reduce_bwd(RT_RED_LOGSUMEXP, o, g, "logsumexp");
+  }
   static Storage log_softmax_backward(const OpB& o, const Storage& g) {
     if (o.inputs.empty()) throw Error::invalid_op("LogSoftmax requires 1 input");
     const Storage& x = o.inputs[0].data();

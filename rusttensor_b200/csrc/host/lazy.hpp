@@ -194,10 +194,24 @@ struct View {
   }
 };
 
+// While it lives, expressions are being walked over: an evaluation is under way, or a program is being built.  What is evaluated meanwhile lies
+// below them; reductions over the same values, which do not, are taken along only where nothing is being walked (they would disappear from under
+// whoever walks).
+struct Walk {
+  static int& depth() {
+    static int n = 0;
+    return n;
+  }
+  Walk() { ++depth(); }
+  ~Walk() { --depth(); }
+  Walk(const Walk&) = delete;
+};
+
 class Compiler {
  public:
   // Builds the program of `root`; false: it does not fit (the caller evaluates some inputs first and tries again).
   bool build(DeviceBuffer* root, rt_fused_program* p, std::vector<DeviceBuffer*>* stored) {
+    const Walk walk;
     const Node& n = *root->node;
     nd_ = (int)n.shape.size();
     if (nd_ > kMaxRawDims) return false;
@@ -215,12 +229,20 @@ class Compiler {
     }
     views_.push_back(id);
     root_ = root;
+    root_shape_ = n.shape;
     const int r = node_value(root, 0);
     if (r < 0) return false;
     outputs_.push_back({r, root});
+    std::pair<int, DeviceBuffer*> sum{-1, nullptr};
+    if (keep_rows_ && nd_ == 2) sum = waiting_sum();
+    if (!root->node) return false;
     for (auto& c : stored_) {
-      if ((int)outputs_.size() == RT_FUSED_MAX_OUTPUTS) break;
-      if (c.second->node) outputs_.push_back({c.first, c.second});  // not evaluated meanwhile, as part of some other program
+      if ((int)outputs_.size() + (sum.second ? 1 : 0) == RT_FUSED_MAX_OUTPUTS) break;
+      if (c.second->node && wanted_later(c.second)) outputs_.push_back({c.first, c.second});  // not evaluated meanwhile, as part of some other program
+    }
+    if (sum.second) {
+      sums_ = (int)outputs_.size();
+      outputs_.push_back(sum);
     }
     if (!collapse(p)) return false;
     for (int pre = std::min<int>((int)operands_.size(), RT_FUSED_PRELOAD); pre >= 0; --pre)
@@ -231,6 +253,10 @@ class Compiler {
     return false;
   }
   const std::vector<std::pair<int, DeviceBuffer*>>& outputs() const { return outputs_; }
+  // The dimensions stay those of the root (two), for a reduction over one of them.
+  void keep_rows() { keep_rows_ = true; }
+  // Among the outputs, the pending column sums of a term that shares values with the root (its buffer in the outputs is the sums'); -1: none.
+  int sums() const { return sums_; }
 
  private:
   struct Value {
@@ -251,9 +277,12 @@ class Compiler {
   };
   struct Memo {
     DeviceBuffer* b;
+    uint64_t id;  // b's: what is evaluated on the way may free a buffer that has been walked over
     int view, value;
+    bool of(const DeviceBuffer* x, int v) const { return b == x && id == x->id && view == v; }
   };
   DeviceBuffer* root_ = nullptr;
+  Shape root_shape_;
   int nd_ = 0;
   int64_t shape_[kMaxRawDims];
   size_t numel_ = 0;
@@ -263,6 +292,39 @@ class Compiler {
   std::vector<Box> regions_;
   std::vector<Memo> memo_;
   std::vector<std::pair<int, DeviceBuffer*>> stored_, outputs_;
+
+  bool keep_rows_ = false;
+  int sums_ = -1;
+  // A bias that is broadcast over the rows gets the column sums of a product of something that is computed here anyway: the term's value
+  // and the buffer of the sums.
+  std::pair<int, DeviceBuffer*> waiting_sum() {
+    const std::pair<int, DeviceBuffer*> none{-1, nullptr};
+    for (DeviceBuffer* x = DeviceBuffer::head(); x; x = x->next) {  // what was walked over and is still pending
+      if (std::none_of(memo_.begin(), memo_.end(), [&](const Memo& m) { return m.of(x, 0); })) continue;
+      for (DeviceBuffer* r : x->readers) {
+        if (!r->node || r->node->kind == Kind::Opaque || r->node->shape != root_shape_ || r->readers.size() != 1) continue;
+        DeviceBuffer* s = r->readers[0];
+        if (!s->node || s->node->tag != Tag::SumRows || s->node->geo[0] >= 0 || s->node->in[0].shape != root_shape_ || (int64_t)s->numel != shape_[1]) continue;
+        const std::weak_ptr<DeviceBuffer> term = r->weak_from_this(), sum = s->weak_from_this();
+        const int v = node_value(r, 0);
+        // what the term needs besides may have been evaluated on the way, and with it the term or the root
+        if (v < 0 || is_imm(v) || sum.expired() || !s->node || term.expired() || !r->node || !root_->node) return none;
+        return {v, s};
+      }
+    }
+    return none;
+  }
+  // In a capture a large intermediate result whose readers are all part of this program is left to whoever asks for it after all (the tape holds
+  // every tensor's gradient): writing it would cost as much as the program.
+  bool wanted_later(DeviceBuffer* b) const {
+    if (!capturing() || b->numel <= kSmall) return true;
+    for (DeviceBuffer* r : b->readers) {
+      bool here = false;
+      for (auto& m : memo_) here = here || m.of(r, 0);
+      if (!here) return true;
+    }
+    return false;
+  }
 
   int view_id(const View& v) {
     for (size_t i = 0; i < views_.size(); ++i)
@@ -404,7 +466,7 @@ class Compiler {
     }
     if (in.buf->node && in.buf->node->kind == Kind::Opaque) lazy_evaluate(in.buf.get());
     // seen through a window (not over its own full shape), costly, and part of several expressions: once, into memory
-    if (in.buf->node && in.buf->readers.size() >= 2 && !(v == views_[0] && in.shape == root_->node->shape) && current_weight(*in.buf->node, 4) > 3)
+    if (in.buf->node && in.buf->readers.size() >= 2 && !(v == views_[0] && in.shape == root_shape_) && current_weight(*in.buf->node, 4) > 3)
       lazy_evaluate(in.buf.get());
     if (!in.buf->node) return leaf(in, v);
     return node_value(in.buf.get(), view_id(v));
@@ -412,11 +474,11 @@ class Compiler {
 
   int node_value(DeviceBuffer* b, int vid) {
     for (auto& m : memo_)
-      if (m.b == b && m.view == vid) return m.value;
+      if (m.of(b, vid)) return m.value;
     const int r = make_value(b, vid);
     if (r >= 0) {
-      memo_.push_back({b, vid, r});
-      if (vid == 0 && b != root_ && b->node->shape == root_->node->shape && values_[r].op != RT_F_LOAD && values_[r].op != RT_F_REG && worth_storing(b))
+      memo_.push_back({b, b->id, vid, r});
+      if (vid == 0 && b != root_ && b->node->shape == root_shape_ && values_[r].op != RT_F_LOAD && values_[r].op != RT_F_REG && worth_storing(b))
         stored_.push_back({r, b});
     }
     return r;
@@ -510,12 +572,12 @@ class Compiler {
     std::vector<Operand> ops = operands_;
     std::vector<Box> boxes = regions_;
     for (int d = 0; d < nd_; ++d) {
-      if (shape_[d] == 1 && !(d == nd_ - 1 && nd == 0)) {
+      if (!keep_rows_ && shape_[d] == 1 && !(d == nd_ - 1 && nd == 0)) {
         bool trivial = true;
         for (auto& b : boxes) trivial = trivial && b.lo[d] <= 0 && b.hi[d] >= 1;
         if (trivial) continue;
       }
-      bool merge = nd > 0;
+      bool merge = nd > 0 && !keep_rows_;
       if (merge) {
         const int q = keep[nd - 1];
         for (auto& o : ops) merge = merge && o.stride[q] == o.stride[d] * shape_[d];
@@ -1231,12 +1293,58 @@ inline bool rewrite(DeviceBuffer* b) {
   return rewrite_rows(b) || rewrite_recurrence(b) || rewrite_linear(b) || rewrite_nll_grad(b) || rewrite_loss(b) || rewrite_loss_sum(b) || rewrite_pool(b);
 }
 
+// Whether column sums over an expression of b's shape are pending.
+inline bool column_sum_waits(DeviceBuffer* b) {
+  for (DeviceBuffer* p = DeviceBuffer::head(); p; p = p->next)
+    if (p->node->tag == Tag::SumRows && p->node->geo[0] < 0 && p->node->in[0].shape == b->node->shape && pending(p->node->in[0]) &&
+        pending(p->node->in[0])->kind != Kind::Opaque && p->node->in[0].buf.get() != b)
+      return true;
+  return false;
+}
+// A program and its outputs' blocks, launched by `run`; false: not a form that it has.
+template <class Run>
+inline bool evaluate_reduced(DeviceBuffer* b, Compiler& c, Run run) {
+  rt_fused_program p;
+  std::vector<DeviceBuffer*> outs;
+  if (!c.build(b, &p, &outs)) return !b->node;  // evaluated on the way
+  std::vector<Block> blocks;
+  for (size_t k = 0; k < outs.size(); ++k) {
+    blocks.emplace_back(b->ctx, outs[k]->numel);
+    p.out[k] = blocks.back().ptr;
+  }
+  const rt_status st = run(p);
+  if (st == RT_ERR_UNIMPLEMENTED) return false;
+  check(b->ctx, st);
+  std::vector<std::shared_ptr<DeviceBuffer>> keep;
+  for (auto* o : outs) keep.push_back(o->shared_from_this());
+  for (size_t k = 0; k < outs.size(); ++k) blocks[k].to(outs[k]);
+  return true;
+}
+// An expression over [rows, columns] together with the pending column sums of a term that it shares values with.
+inline bool evaluate_with_sums(DeviceBuffer* b) {
+  if (Walk::depth() > 1 || b->node->shape.size() != 2 || b->numel == 0 || !column_sum_waits(b)) return false;
+  Compiler c;
+  c.keep_rows();
+  return evaluate_reduced(b, c, [&](rt_fused_program& p) {
+    return c.sums() < 0 ? RT_ERR_UNIMPLEMENTED : rt_fused_column_sums(b->ctx, &p, c.sums(), p.out[c.sums()]);
+  });
+}
+// The rows of an expression and their logsumexp.
+inline bool evaluate_with_logsumexp(DeviceBuffer* b, float* out) {
+  if (Walk::depth() > 0 || !b->node || b->node->kind == Kind::Opaque || b->node->kind == Kind::Const || b->node->shape.size() != 2 || b->numel == 0) return false;
+  std::shared_ptr<DeviceBuffer> guard = b->shared_from_this();
+  Compiler c;
+  c.keep_rows();
+  return evaluate_reduced(b, c, [&](rt_fused_program& p) { return c.sums() >= 0 ? RT_ERR_UNIMPLEMENTED : rt_fused_logsumexp(b->ctx, &p, out); });
+}
+
 }  // namespace lazy
 
 inline void lazy_evaluate(DeviceBuffer* b) {
   using namespace lazy;
   if (!b->node) return;
   std::shared_ptr<DeviceBuffer> guard = b->shared_from_this();
+  const Walk walk;
   if (rewrite(b)) return;
   if (b->node->kind == Kind::Opaque) {
     b->node->run(*b->node, b);
@@ -1246,6 +1354,7 @@ inline void lazy_evaluate(DeviceBuffer* b) {
   const bool lone = (b->node->kind == Kind::Unary || b->node->kind == Kind::Binary) &&
                     std::all_of(b->node->in.begin(), b->node->in.end(), [](const Input& i) { return !i.buf->node; });
   if ((lone || b->node->kind == Kind::Const) && evaluate_alone(b)) return;
+  if (evaluate_with_sums(b)) return;
   for (int attempt = 0; attempt < 2; ++attempt) {
     rt_fused_program p;
     Compiler c;

@@ -275,7 +275,7 @@ bool regions_in_quads(const FusedParams& p) {
 
 }  // namespace
 
-extern "C" rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* f) {
+rt_status fused::prepare(rt_ctx* ctx, const rt_fused_program* f, FusedParams* out, bool* in_vectors, int64_t* count) {
   RT_CHECK_CTX(ctx);
   RT_CHECK_PTR(ctx, f);
   if (f->nd < 1 || f->nd > RT_FUSED_MAX_DIMS || f->n_operands < 0 || f->n_operands > RT_FUSED_MAX_OPERANDS || f->n_regions < 0 ||
@@ -301,8 +301,9 @@ extern "C" rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* f
     if (f->operand[k].region != RT_FUSED_NONE && (f->operand[k].region < 0 || f->operand[k].region >= f->n_regions))
       RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_fused_elementwise: operand %d names region %d", k, f->operand[k].region);
   }
+  *count = numel;
   if (numel == 0) return RT_OK;
-  FusedParams p;
+  FusedParams& p = *out;
   p.nd = f->nd;
   p.n_preload = f->n_preload;
   p.n_code = f->n_code;
@@ -327,10 +328,20 @@ extern "C" rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* f
   }
   for (int k = 0; k < f->n_regions; ++k) p.region[k] = f->region[k];
   for (int i = 0; i < f->n_code; ++i) p.code[i] = encode(f->code[i]);
+  *in_vectors = vec && regions_in_quads(p);
+  return RT_OK;
+}
+
+extern "C" rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* f) {
+  FusedParams p;
+  bool vec;
+  int64_t numel;
+  rt_status st = prepare(ctx, f, &p, &vec, &numel);
+  if (st != RT_OK || numel == 0) return st;
   if (p.nd <= 2)
     if (const KnownProgram* k = find_known(p)) {
       ctx->fused_compiled++;
-      return k->launch(ctx, p, vec && regions_in_quads(p), numel);
+      return k->launch(ctx, p, vec, numel);
     }
   ctx->fused_interpreted++;
   // Eight elements per thread halve the decoding per element, four give twice the warps: the line lies where eight still fill

@@ -99,6 +99,8 @@ rt_status rt_sum_rows_accumulate_list(rt_ctx*, int count, const float* const* xs
 rt_status rt_gemm_bias_act_list(rt_ctx*, int, const float* const*, float* const*, int64_t, int64_t, int64_t, const float*, const float*, int) {
   return kernels_fail ? RT_ERR_CUDA : RT_OK;
 }
+rt_status rt_fused_column_sums(rt_ctx*, const rt_fused_program*, int, float*) { return RT_ERR_UNIMPLEMENTED; }
+rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of windows; results of other programs stay zero
   if (kernels_fail) return RT_ERR_CUDA;
   if (p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_OK;
