@@ -3,26 +3,31 @@
 // Timestep by timestep the recurrence is a product of [batch, H] x [H, 4H] and a few element operations, each a kernel that is over before
 // it has started: 8 + 4 us of a timestep at batch 64, H 512, of which the arithmetic is two.  Here the kernel stays: every block keeps its
 // slice of the recurrent weights in shared memory for the whole sequence, and what the blocks tell one another per timestep is written to
-// and polled in memory, value and timestep number side by side in 8 bytes, so that seeing the number is having the value: no barrier.
+// and polled in memory, the value and what tells its timestep in the same 4 or 8 bytes, so that seeing the one is having the other: no
+// barrier.
 //
 // A block has 16 rows of the batch and U hidden units (all four gates of them).  Rows are independent of one another, so only the blocks
-// of the same rows exchange anything.  Forward a block publishes h of its units and gathers everybody's: the 16 warps split the reduction
-// and add up in shared memory.  Backward a block has the gate gradients of its own units and multiplies them with its slice (its columns
-// of the weights) into a partial gradient of ALL units, which it sends to the blocks that own them: 32 KB in and out either way, where
-// gathering the gate gradients would take 128.  All sums are fp32 in a fixed order.
+// of the same rows exchange anything.  Forward a block publishes h of its units and gathers everybody's (4 bytes a value): the 16 warps
+// split the reduction and add up in shared memory.  Backward a block has the gate gradients of its own units and multiplies them with its
+// slice (its columns of the weights) into a partial gradient of ALL units, which it sends to the blocks that own them (8 bytes a value):
+// 64 KB in and out at H 512, where gathering the gate gradients would take twice that.  All sums are fp32 in a fixed order.
+// Operands lie as pairs of reduction indices, even and odd sums apart, for two multiply-adds an instruction: that halves what the warps
+// issue, though not the time of the multiply-adds themselves (36 cycles for 16 of these, 32 for 32 single ones).  A lane's results
+// backward are 16 units apart, so that eight lanes write 128 bytes together.
 // The blocks wait for one another, so they are launched cooperatively (all resident or an error).  Every wait is bounded; a block whose wait
 // expires records a code in the status word and goes on without waiting.
 //
-// Bound by latency.  Measured at batch 30, H 200: 2.3 us a timestep forward, 4.2 backward; as kernels of their own the product, the cell and
-// the concatenation took 9.7 forward, 12.3 backward.  Sizes whose blocks do not fit beside one another, or whose slice of the weights does not
-// fit into a block, run timestep by timestep.
+// Bound by latency; at H 512 forward two of the 5.3 us are multiply-adds.  Measured, a timestep: batch 30, H 200: 2.3 us forward, 3.0
+// backward (2.4 and 3.9 before the pairs and the shorter mail); batch 64, H 512: 5.3 and 6.5 (5.4 and 7.9).  As kernels of their own the
+// product, the cell and the concatenation took 9.7 forward, 12.3 backward at the first size.  Sizes whose blocks do not fit beside one
+// another, or whose slice of the weights does not fit into a block, run timestep by timestep.
 #include "rt_internal.cuh"
 #include "tc_common.cuh"
 
 namespace {
 
 constexpr int kRows = 16, kWarps = 16, kThreads = kWarps * 32;
-constexpr int kPitch = 20;  // words between the 16 rows' values of one reduction index and the next: 16-byte aligned, few bank conflicts
+constexpr int kPitch = 36;  // words between the 16 rows' values of two reduction indices and those of the next two: 16-byte aligned, few bank conflicts
 constexpr uint32_t kPolls = 1u << 21;
 
 struct SeqArgs {
@@ -47,25 +52,51 @@ __device__ __forceinline__ uint4 peek(const uint4* p) {
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void post(uint2* p, float v, uint32_t tag) {
-  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(v)), "r"(tag) : "memory");
-}
 __device__ __forceinline__ void post2(uint4* p, float v, float w, uint32_t tag) {
   asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %3, %2, %3};" ::"l"(p), "r"(__float_as_uint(v)), "r"(__float_as_uint(w)), "r"(tag) : "memory");
 }
+// Two multiply-adds in one instruction: what the accumulators hold apart are the sums over the even and over the odd reduction indices.
+struct Pair {
+  unsigned long long v = 0;
+  __device__ __forceinline__ float sum() const {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a + b;
+  }
+};
+__device__ __forceinline__ void fma2(Pair& c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c.v) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ ulonglong2 pairs_at(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
-// Waits until N pieces of mail carry `tag`.  False: the wait ran out, here or in another block.  (Polling one piece until it is there and
-// only then the others is a round trip more: 693 -> 714 us for 128 timesteps at batch 64, H 512.)
-template <int N>
-__device__ __forceinline__ bool receive(const uint4* const (&from)[N], const bool (&want)[N], uint32_t tag, uint4 (&v)[N], const SeqArgs& a) {
+// Forward a value carries the number of its timestep in one bit: h lies within [-1, 1], whose floats leave bit 30 zero, and a place is
+// written every second timestep, so that the bit need only tell a message from the one before it.  NaN goes as a number that h cannot be.
+// (With the number beside the value, twice the bytes to poll: 5.5 us a timestep at batch 64, H 512.)
+constexpr uint32_t kTurnBit = 1u << 30, kNanCode = 0x3fffffffu;
+__device__ __forceinline__ uint32_t turn_bit(int t) { return (t >> 1) & 1 ? 0u : kTurnBit; }  // memory starts as zeros
+__device__ __forceinline__ void post_output(uint32_t* p, float h, uint32_t bit) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"((h == h ? __float_as_uint(h) : kNanCode) | bit) : "memory");
+}
+__device__ __forceinline__ uint32_t output_of(uint32_t v) {
+  v &= ~kTurnBit;
+  return v == kNanCode ? 0x7fc00000u : v;
+}
+
+// Waits until the wanted ones of N pieces of mail, STRIDE apart, have arrived.  False: the wait ran out, here or in another block.  (Polling
+// one piece until it is there and only then the others is a round trip more: 693 -> 714 us for 128 timesteps at batch 64, H 512.)
+template <int STRIDE, int N, class Arrived>
+__device__ __forceinline__ bool receive(const uint4* from, bool (&want)[N], uint4 (&v)[N], const SeqArgs& a, const Arrived& arrived) {
   for (uint32_t i = 0; i < kPolls; ++i) {
-    bool there = true;
 #pragma unroll
     for (int j = 0; j < N; ++j)
-      if (want[j]) v[j] = peek(from[j]);
+      if (want[j]) v[j] = peek(from + j * STRIDE);
+    bool there = true;
 #pragma unroll
-    for (int j = 0; j < N; ++j) there = there && (!want[j] || (v[j].y == tag && v[j].w == tag));
+    for (int j = 0; j < N; ++j) {
+      want[j] = want[j] && !arrived(v[j]);
+      there = there && !want[j];
+    }
     if (__all_sync(0xffffffffu, there)) return true;
     if ((i & 1023) == 1023 && *(volatile int*)a.gave_up) return false;
   }
@@ -78,19 +109,24 @@ template <int U>
 __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const SeqArgs a) {
   extern __shared__ float4 smem4[];
   constexpr int kRegion = kRows * U;  // 16-byte pieces of a warp's region: its sums, before that 2 U reduction indices of h
-  static_assert(2 * U * kPitch * 4 <= kRegion * 16, "region");
-  constexpr int UL = U / 8, P = 32 / U, NL = U / 4;
+  static_assert(U * kPitch * 4 <= kRegion * 16, "region");
+  constexpr int UL = U / 8, P = 32 / U, NL = U / 8, quads = U / 4;  // quads: 16-byte pieces of a row's mail
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane >> 3, cg = lane & 7;
   const int H = a.hidden, group = blockIdx.x % a.groups, row0 = blockIdx.x / a.groups * kRows;
   const int first_block = blockIdx.x - group, padded = a.groups * U;
   float4* const regions = smem4 + padded * U;
   float* const stage = reinterpret_cast<float*>(regions + warp * kRegion);
-  for (int i = threadIdx.x; i < padded * U; i += kThreads) {  // [reduction index][unit]: the four gates
-    const int k = i / U, unit = group * U + i % U;
+  for (int i = threadIdx.x; i < padded * U; i += kThreads) {  // [pair of reduction indices][pair of gates][unit]: gate, index within the pairs
+    const int pair = i / (2 * U), gate = i / U % 2 * 2, unit = group * U + i % U;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (k < H && unit < H) {
-      const float* q = a.w + (int64_t)k * a.ldw + unit;
-      v = make_float4(__ldg(q), __ldg(q + H), __ldg(q + 2 * H), __ldg(q + 3 * H));
+    if (2 * pair < H && unit < H) {
+      const float* q = a.w + (int64_t)(2 * pair) * a.ldw + (int64_t)gate * H + unit;
+      v.x = __ldg(q);
+      v.z = __ldg(q + H);
+      if (2 * pair + 1 < H) {
+        v.y = __ldg(q + a.ldw);
+        v.w = __ldg(q + a.ldw + H);
+      }
     }
     smem4[i] = v;
   }
@@ -109,51 +145,61 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const SeqArg
 #pragma unroll
       for (int g = 0; g < 4; ++g) pre[g] = __ldg(q + (int64_t)g * H);
     }
-    float acc[UL][4][4] = {};
+    Pair acc[UL][4][4];
     if (t > 0 || a.h0) {
       for (int q = q_begin; q < q_end; q += 2) {
+        // piece j of the lane: rows of U / 4 pieces, sources of 16 rows, all one after the other
         uint4 v[2 * NL] = {};
-        int at[2 * NL];
-        const uint4* from[2 * NL];
         bool want[2 * NL];
+        const int quad = lane % quads, r0 = lane / quads;
 #pragma unroll
-        for (int j = 0; j < 2 * NL; ++j) {
-          const int piece = j % NL * 32 + lane, r = piece / (U / 2), pair = piece % (U / 2);
-          want[j] = q + j / NL < q_end;
-          at[j] = (j / NL * U + 2 * pair) * kPitch + r;
-          from[j] = a.mail + (((int64_t)((t - 1) & 1) * gridDim.x + first_block + q + j / NL) * kRows + r) * (U / 2) + pair;
-          if (t == 0 && want[j] && row0 + r < a.batch) {
-            const int k = (q + j / NL) * U + 2 * pair;
+        for (int j = 0; j < 2 * NL; ++j) want[j] = j < NL || q + 1 < q_end;
+        if (t > 0) {
+          const uint32_t bit = turn_bit(t - 1);
+          const uint4* from = a.mail + ((int64_t)((t - 1) & 1) * gridDim.x + first_block + q) * kRows * quads + lane;
+          if (ok)
+            ok = receive<32>(from, want, v, a, [bit](const uint4& m) { return (((m.x ^ bit) | (m.y ^ bit) | (m.z ^ bit) | (m.w ^ bit)) & kTurnBit) == 0; });
+#pragma unroll
+          for (int j = 0; j < 2 * NL; ++j) v[j] = make_uint4(output_of(v[j].x), output_of(v[j].y), output_of(v[j].z), output_of(v[j].w));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 2 * NL; ++j) {
+            const int r = j % NL * (128 / U) + r0, k = (q + j / NL) * U + 4 * quad;
             const float* h = a.h0 + (int64_t)(row0 + r) * H + k;
-            v[j].x = k < H ? __float_as_uint(__ldg(h)) : 0u;
-            v[j].z = k + 1 < H ? __float_as_uint(__ldg(h + 1)) : 0u;
+            if (want[j] && row0 + r < a.batch) {
+              v[j].x = k < H ? __float_as_uint(__ldg(h)) : 0u;
+              v[j].y = k + 1 < H ? __float_as_uint(__ldg(h + 1)) : 0u;
+              v[j].z = k + 2 < H ? __float_as_uint(__ldg(h + 2)) : 0u;
+              v[j].w = k + 3 < H ? __float_as_uint(__ldg(h + 3)) : 0u;
+            }
           }
         }
-        if (t > 0 && ok) ok = receive(from, want, (uint32_t)t, v, a);
+        float* const to = stage + 2 * quad * kPitch + 2 * r0;
 #pragma unroll
         for (int j = 0; j < 2 * NL; ++j) {
-          stage[at[j]] = __uint_as_float(v[j].x);
-          stage[at[j] + kPitch] = __uint_as_float(v[j].z);
+          float* const o = to + j / NL * (U / 2) * kPitch + j % NL * (256 / U);
+          *reinterpret_cast<uint2*>(o) = make_uint2(v[j].x, v[j].y);
+          *reinterpret_cast<uint2*>(o + kPitch) = make_uint2(v[j].z, v[j].w);
         }
         __syncwarp();
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           if (q + half >= q_end) break;
-          const float4* w = smem4 + (q + half) * U * U + cg;
-          const float* h = stage + half * U * kPitch + 4 * rg;
-#pragma unroll 8
-          for (int k = 0; k < U; ++k) {
-            const float4 x = *reinterpret_cast<const float4*>(h + k * kPitch);
-            const float xs[4] = {x.x, x.y, x.z, x.w};
+          const float* w = reinterpret_cast<const float*>(smem4 + (q + half) * U * U + cg);
+          const float* h = stage + half * (U / 2) * kPitch + 8 * rg;
+#pragma unroll 4
+          for (int k = 0; k < U / 2; ++k) {
+            const ulonglong2 x01 = pairs_at(h + k * kPitch), x23 = pairs_at(h + k * kPitch + 4);
+            const unsigned long long xs[4] = {x01.x, x01.y, x23.x, x23.y};
 #pragma unroll
             for (int j = 0; j < UL; ++j) {
-              const float4 y = w[k * U + 8 * j];
+              const ulonglong2 y01 = pairs_at(w + (k * 2 * U + 8 * j) * 4), y23 = pairs_at(w + (k * 2 * U + U + 8 * j) * 4);
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
-                acc[j][i][0] = fmaf(xs[i], y.x, acc[j][i][0]);
-                acc[j][i][1] = fmaf(xs[i], y.y, acc[j][i][1]);
-                acc[j][i][2] = fmaf(xs[i], y.z, acc[j][i][2]);
-                acc[j][i][3] = fmaf(xs[i], y.w, acc[j][i][3]);
+                fma2(acc[j][i][0], xs[i], y01.x);
+                fma2(acc[j][i][1], xs[i], y01.y);
+                fma2(acc[j][i][2], xs[i], y23.x);
+                fma2(acc[j][i][3], xs[i], y23.y);
               }
             }
           }
@@ -165,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const SeqArg
     for (int j = 0; j < UL; ++j)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        regions[warp * kRegion + (4 * rg + i) * U + cg + 8 * j] = make_float4(acc[j][i][0], acc[j][i][1], acc[j][i][2], acc[j][i][3]);
+        regions[warp * kRegion + (4 * rg + i) * U + cg + 8 * j] = make_float4(acc[j][i][0].sum(), acc[j][i][1].sum(), acc[j][i][2].sum(), acc[j][i][3].sum());
     __syncthreads();
     float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -186,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const SeqArg
     if (part == 0) {
       // the padding's h is never used: it meets weights of zero, and must therefore be finite
       if (t + 1 < a.steps)
-        post(reinterpret_cast<uint2*>(a.mail) + (((int64_t)(t & 1) * gridDim.x + blockIdx.x) * kRows + warp) * U + u, active ? h : 0.f, (uint32_t)t + 1);
+        post_output(reinterpret_cast<uint32_t*>(a.mail) + (((int64_t)(t & 1) * gridDim.x + blockIdx.x) * kRows + warp) * U + u, active ? h : 0.f, turn_bit(t));
       if (active) {
         const int64_t e = t * per_step + cell;
         a.ig[e] = ig; a.fg[e] = fg; a.gg[e] = gg; a.og[e] = og; a.c[e] = c; a.tc[e] = tc; a.h[e] = h;
@@ -202,11 +248,11 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_backward_kernel(con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane >> 3, cg = lane & 7;
   const int H = a.hidden, S = a.groups, group = blockIdx.x % S, rows = blockIdx.x / S, row0 = rows * kRows;
   const int pitch_w = (S * U + 31) / 32 * 32;
-  float* const ws = reinterpret_cast<float*>(smem4);           // [gate * U + unit][unit of the gradient]
-  float* const dgs = ws + 4 * U * pitch_w;                       // two turns of [gate * U + unit][row]
+  float* const ws = reinterpret_cast<float*>(smem4);           // [pair of gate * U + unit][unit of the gradient][index within the pair]
+  float* const dgs = ws + 4 * U * pitch_w;                       // two turns of [pair of gate * U + unit][row][index within the pair]
   for (int i = threadIdx.x; i < 4 * U * pitch_w; i += kThreads) {
     const int u = i % U, gate = i / U % 4, j = i / (4 * U), unit = group * U + u;
-    ws[(gate * U + u) * pitch_w + j] = j < H && unit < H ? __ldg(a.w + (int64_t)j * a.ldw + (int64_t)gate * H + unit) : 0.f;
+    ws[((gate * U + u) / 2 * pitch_w + j) * 2 + u % 2] = j < H && unit < H ? __ldg(a.w + (int64_t)j * a.ldw + (int64_t)gate * H + unit) : 0.f;
   }
   const int row = row0 + warp, u = lane % U, unit = group * U + u;
   const bool active = row < a.batch && unit < H;
@@ -229,21 +275,17 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_backward_kernel(con
       float x = 0.f, y = 0.f;
       for (int s0 = 0; s0 < S; s0 += N * at_once) {
         uint4 v[N] = {};
-        const uint4* from[N];
         bool want[N];
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
-          const int src = s0 + j * at_once + lane / pairs;
-          want[j] = src < S;
-          from[j] = box((step - 1) & 1, group, src) + warp * pairs + lane % pairs;
-        }
-        if (ok) ok = receive(from, want, (uint32_t)step, v, a);
+        for (int j = 0; j < N; ++j) want[j] = s0 + j * at_once + lane / pairs < S;
+        const uint4* from = box((step - 1) & 1, group, s0 + lane / pairs) + warp * pairs + lane % pairs;
+        const uint32_t tag = (uint32_t)step;
+        if (ok) ok = receive<at_once * kRows * pairs>(from, want, v, a, [tag](const uint4& m) { return m.y == tag && m.w == tag; });
 #pragma unroll
-        for (int j = 0; j < N; ++j)
-          if (want[j]) {
-            x += __uint_as_float(v[j].x);
-            y += __uint_as_float(v[j].z);
-          }
+        for (int j = 0; j < N; ++j) {  // zeros where there is no source
+          x += __uint_as_float(v[j].x);
+          y += __uint_as_float(v[j].z);
+        }
       }
 #pragma unroll
       for (int d = pairs; d < 32; d *= 2) {
@@ -258,41 +300,43 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_backward_kernel(con
       if (active && lane < U) a.dh0[cell] = dh;
       break;
     }
-    float* const turn = dgs + (step & 1) * 4 * U * kPitch;
+    float* const turn = dgs + (step & 1) * 2 * U * kPitch;
     dc += dh * og * (1.f - tc * tc);
     const float d[4] = {dc * gg * ig * (1.f - ig), dc * before * fg * (1.f - fg), dc * ig * (1.f - gg * gg), dh * tc * og * (1.f - og)};
     dc *= fg;
     if (lane < U) {
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        turn[(g * U + u) * kPitch + warp] = active ? d[g] : 0.f;
+        turn[(g * U + u) / 2 * kPitch + 2 * warp + u % 2] = active ? d[g] : 0.f;
         if (active) a.dgates[((int64_t)t * a.batch + row) * 4 * H + (int64_t)g * H + unit] = d[g];
       }
     }
     if (t == 0 && !a.dh0) break;
     __syncthreads();
     for (int j0 = warp * 32; j0 < pitch_w; j0 += kWarps * 32) {
-      float acc[4][4] = {};
-      const float *w = ws + j0 + 4 * cg, *x = turn + 4 * rg;
-#pragma unroll 8
-      for (int k = 0; k < 4 * U; ++k) {
-        const float4 p = *reinterpret_cast<const float4*>(x + k * kPitch), q = *reinterpret_cast<const float4*>(w + k * pitch_w);
-        const float xs[4] = {p.x, p.y, p.z, p.w};
+      // a lane has four rows and the units j0 + 2 cg, j0 + 16 + 2 cg and those after them
+      Pair acc[4][4];
+      const float *w = ws + (j0 + 2 * cg) * 2, *x = turn + 8 * rg;
+#pragma unroll 4
+      for (int k = 0; k < 2 * U; ++k) {
+        const ulonglong2 p01 = pairs_at(x + k * kPitch), p23 = pairs_at(x + k * kPitch + 4);
+        const ulonglong2 q01 = pairs_at(w + k * 2 * pitch_w), q23 = pairs_at(w + k * 2 * pitch_w + 32);
+        const unsigned long long xs[4] = {p01.x, p01.y, p23.x, p23.y};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          acc[i][0] = fmaf(xs[i], q.x, acc[i][0]);
-          acc[i][1] = fmaf(xs[i], q.y, acc[i][1]);
-          acc[i][2] = fmaf(xs[i], q.z, acc[i][2]);
-          acc[i][3] = fmaf(xs[i], q.w, acc[i][3]);
+          fma2(acc[i][0], xs[i], q01.x);
+          fma2(acc[i][1], xs[i], q01.y);
+          fma2(acc[i][2], xs[i], q23.x);
+          fma2(acc[i][3], xs[i], q23.y);
         }
       }
-      const int j = j0 + 4 * cg, dest = j / U;
-      if (dest < S) {
-        uint4* to = box(step & 1, dest, group) + 4 * rg * pairs + j % U / 2;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          post2(to + i * pairs, acc[i][0], acc[i][1], (uint32_t)step + 1);
-          post2(to + i * pairs + 1, acc[i][2], acc[i][3], (uint32_t)step + 1);
+      for (int half = 0; half < 2; ++half) {
+        const int j = j0 + 16 * half + 2 * cg, dest = j / U;
+        if (dest < S) {
+          uint4* to = box(step & 1, dest, group) + 4 * rg * pairs + j % U / 2;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) post2(to + i * pairs, acc[i][2 * half].sum(), acc[i][2 * half + 1].sum(), (uint32_t)step + 1);
         }
       }
     }
@@ -345,7 +389,7 @@ Fit fit(const rt_ctx* ctx, int64_t batch, int64_t hidden, bool backward) {
     f.groups = (int)((hidden + u - 1) / u);
     const int64_t blocks = (batch + kRows - 1) / kRows * f.groups;
     const size_t pitch_w = ((size_t)f.groups * u + 31) / 32 * 32;
-    f.smem = backward ? sizeof(float) * 4 * u * (pitch_w + 2 * kPitch)
+    f.smem = backward ? sizeof(float) * 4 * u * (pitch_w + kPitch)
                       : 16 * ((size_t)f.groups * u * u + kWarps * kRows * u);
     f.blocks = (int)blocks;
     if (blocks <= ctx->sm_count && f.smem <= 232448) return f;
@@ -368,14 +412,14 @@ rt_status launch_together(rt_ctx* ctx, void (*kern)(SeqArgs), RtDeviceOnce& once
   RT_LAUNCHED(ctx);
   return RT_OK;
 }
-// `mail`: 8 bytes a value and a word for giving up, cleared.
-rt_status clear_mail(rt_ctx* ctx, RtScratch* mem, size_t values, SeqArgs* a) {
-  const size_t bytes = 8 * values + 16;
+// `mail` and a word for giving up, cleared.
+rt_status clear_mail(rt_ctx* ctx, RtScratch* mem, size_t mail, SeqArgs* a) {
+  const size_t bytes = mail + 16;
   rt_status st = mem->alloc(bytes);
   if (st != RT_OK) return st;
   RT_CUDA(ctx, cudaMemsetAsync(mem->ptr, 0, bytes, ctx->stream));
   a->mail = mem->as<uint4>();
-  a->gave_up = reinterpret_cast<int*>(mem->as<char>() + 8 * values);
+  a->gave_up = reinterpret_cast<int*>(mem->as<char>() + mail);
   return RT_OK;
 }
 rt_status check_sizes(rt_ctx* ctx, const char* name, int64_t steps, int64_t batch, int64_t hidden, int64_t ldw) {
@@ -419,7 +463,7 @@ rt_status rt_lstm_sequence(rt_ctx* ctx, const float* pre, const float* w, int64_
   if (f.units) {
     a.groups = f.groups;
     RtScratch mail(ctx);
-    if ((st = clear_mail(ctx, &mail, (size_t)2 * f.blocks * kRows * f.units, &a)) != RT_OK) return st;
+    if ((st = clear_mail(ctx, &mail, (size_t)2 * f.blocks * kRows * f.units * 4, &a)) != RT_OK) return st;
     static RtDeviceOnce once8, once16;
     return f.units == 8 ? launch_together(ctx, lstm_sequence_kernel<8>, once8, f, a) : launch_together(ctx, lstm_sequence_kernel<16>, once16, f, a);
   }
@@ -463,7 +507,7 @@ rt_status rt_lstm_sequence_backward(rt_ctx* ctx, const float* saved, const float
   if (f.units) {
     a.groups = f.groups;
     RtScratch mail(ctx);
-    if ((st = clear_mail(ctx, &mail, (size_t)2 * f.blocks * f.groups * kRows * f.units, &a)) != RT_OK) return st;
+    if ((st = clear_mail(ctx, &mail, (size_t)2 * f.blocks * f.groups * kRows * f.units * 8, &a)) != RT_OK) return st;
     static RtDeviceOnce once8, once16;
     return f.units == 8 ? launch_together(ctx, lstm_sequence_backward_kernel<8>, once8, f, a)
                         : launch_together(ctx, lstm_sequence_backward_kernel<16>, once16, f, a);

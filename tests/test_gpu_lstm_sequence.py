@@ -71,6 +71,24 @@ def test_sequence_and_gradient(capi, steps, batch, hidden, initial):
         assert np.max(np.abs(a - b)) <= bound * max(1.0, np.abs(b).max())
 
 
+def test_nan_travels_like_a_value(capi):
+    """An output that is NaN goes from block to block as a code; its row is NaN from then on, the others are what they are without it."""
+    steps, batch, hidden = 6, 18, 40
+    r = rng(5)
+    pre = r.standard_normal((steps, batch, 4 * hidden)).astype(np.float32)
+    w = (r.uniform(-1, 1, (hidden, 4 * hidden)) / np.sqrt(hidden)).astype(np.float32)
+    got = []
+    for bad in (False, True):
+        if bad:
+            pre[1, 17, 3] = np.nan
+        p, d = capi.to_device(pre), capi.to_device(w)
+        h, saved = capi.empty((steps, batch, hidden)), capi.empty((6, steps * batch, hidden))
+        capi.call("lstm_sequence", p.ptr, d.ptr, i64(4 * hidden), None, None, i64(steps), i64(batch), i64(hidden), saved.ptr, h.ptr)
+        got.append(h.numpy())
+    assert np.isnan(got[1][2:, 17]).all() and np.isnan(got[1][1, 17, 3]) and np.isnan(got[1][1]).sum() == 1
+    assert np.array_equal(got[0][:, :17], got[1][:, :17]) and np.array_equal(got[0][0], got[1][0])
+
+
 def test_sizes_are_checked(capi):
     x = capi.empty((4, 16))
     for sizes in ((0, 2, 4), (1, 0, 4), (1, 2, 0)):
