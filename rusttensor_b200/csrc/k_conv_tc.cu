@@ -16,10 +16,16 @@
 //
 // The weights are packed once per call by a small kernel into the exact shared-memory image
 // (per tap a K-major [BN x Cp] tile, hi and lo) and stay resident in shared memory while the
-// persistent CTA walks over its position tiles.  Roles per CTA: 8 producer / epilogue warps, one
-// MMA-issuing thread.  Window stages and the two accumulator sets in tensor memory are handed
+// persistent CTA walks over its position tiles.  Roles per CTA: 8 producer warps, 8 epilogue warps,
+// one MMA-issuing thread.  Window stages and the two accumulator sets in tensor memory are handed
 // over with mbarriers; every wait is bounded and on expiry the kernel records a code in the
 // context's status word, skips the remaining work, frees its tensor memory and returns.
+//
+// Bound by shared memory: the MMAs read about 112 x 128 bytes for 8 channels of a tap and the producers'
+// stores take a quarter of that again (ncu: tensor pipe active 57 %, 20 of 81 thousand cycles are the
+// stores').  With the epilogue done by the producers in between, a tile of 32 -> 64 channels took 4.1 us,
+// in warps of its own 3.7: [1000,32,14,14] 58.5 -> 51.5 us.  Four epilogue warps are too few (55.7), a
+// second group of producers changes nothing.
 #include "rt_internal.cuh"
 #include "conv_geom.cuh"
 #include "tc_common.cuh"
@@ -28,7 +34,8 @@ namespace tc {
 namespace conv {
 
 constexpr int kProducerWarps = 8;
-constexpr int kThreads = (kProducerWarps + 1) * 32;
+constexpr int kEpilogueWarps = 8, kMmaWarp = kProducerWarps + kEpilogueWarps;
+constexpr int kThreads = (kMmaWarp + 1) * 32;
 constexpr int kTileM = 128;
 // Accumulator columns per set: [hi*hi | hi*lo] (2*BN, one MMA against the stacked hi/lo weight tile) and lo*hi (BN).
 // The reduction of one tile is at most a few hundred K-steps, short enough for a single accumulation chain.
@@ -79,7 +86,7 @@ __global__ void pack_weights_kernel(const float* __restrict__ w, float* __restri
 }
 
 // CGQ = channel quads per window stage (2, 4, 6 or 8), a compile-time constant so that the producers' load / convert /
-// store loops are straight-line code: these nine warps are issue-bound, every predicate and address computation in the
+// store loops are straight-line code: these warps are issue-bound, every predicate and address computation in the
 // per-element path shows up in the kernel's run time.
 template <int BN, int CGQ>
 __global__ void __launch_bounds__(kThreads, 1) conv_window_kernel(const Params p, int* status) {
@@ -109,12 +116,12 @@ __global__ void __launch_bounds__(kThreads, 1) conv_window_kernel(const Params p
       mbar_init(bars + 8 * s, kProducerWarps);        // a_full
       mbar_init(bars + 8 * (2 + s), 1);               // a_empty
       mbar_init(bars + 8 * (4 + s), 1);               // acc_full
-      mbar_init(bars + 8 * (6 + s), kProducerWarps);  // acc_empty
+      mbar_init(bars + 8 * (6 + s), kEpilogueWarps);  // acc_empty
     }
     mbar_init(bars + 8 * 8, 1);                       // b_full: the resident weights have landed
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kProducerWarps) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
+  if (warp == kMmaWarp) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
   if (threadIdx.x < BN) bias_s[threadIdx.x] = (p.bias && (int)threadIdx.x < p.N) ? __ldg(p.bias + threadIdx.x) : 0.f;
   tc_fence_before();
   __syncthreads();
@@ -125,46 +132,9 @@ __global__ void __launch_bounds__(kThreads, 1) conv_window_kernel(const Params p
   bool ok = true;
 
   if (warp < kProducerWarps) {
-    // ---------------- window producers, then epilogue of the previous tile ----------------
+    // ---------------- window producers ----------------
     const int tid = threadIdx.x;  // position within the window (threads beyond the window idle in the producer part)
     const int hw = p.H * p.W;
-    auto epilogue = [&](int tile, int tcnt) -> bool {
-      const int set = tcnt & 1;
-      if (!mbar_wait(bars + 8 * (4 + set), (tcnt >> 1) & 1, status, 5)) return false;
-      tc_fence_after();
-      const int quad = warp & 3, half = warp >> 2;
-      const int P = tile * kTileM + quad * 32 + lane;
-      uint32_t b, r, y, x;
-      p.d_HpWp.divmod(P, b, r);
-      p.d_Wp.divmod(r, y, x);
-      const bool valid = (int)b < p.Nb && (int)y < p.Ho && (int)x < p.Wo;
-      const int howo = p.Ho * p.Wo;
-      float* q = p.out + (int64_t)b * p.N * howo + (int)y * p.Wo + (int)x;
-      // this warp's share: 32 rows (its lane quadrant) x BN/2 columns, in pieces of 16 columns
-      constexpr int CW = BN / 2;
-#pragma unroll
-      for (int c0 = 0; c0 < CW; c0 += 16) {
-        const int col = half * CW + c0;
-        const uint32_t t0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(set * kAccCols * BN + col);
-        uint32_t r[kAccCols][16];
-#pragma unroll
-        for (int a = 0; a < kAccCols; ++a) tmem_ld16_nowait(t0 + (uint32_t)(a * BN), r[a]);
-        tmem_wait_ld();
-        if (valid) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int n = col + j;
-            const float v = __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
-            if (n < p.N) q[(int64_t)n * howo] = v + bias_s[n];
-          }
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + 8 * (6 + set));
-      return true;
-    };
-
     // A stage is (tile, channel group).  The loads of stage s+1 are issued before stage s is converted
     // and stored, so that their latency overlaps the wait for the stage buffer and the conversion.
     struct Pos { bool inside; int soff; };
@@ -235,7 +205,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv_window_kernel(const Params p
         load(ps, ng, nxt);
       }
       if (!store(s, g, cur)) return false;
-      if (g == p.groups - 1 && ti > 0 && !epilogue((int)blockIdx.x + (ti - 1) * (int)gridDim.x, ti - 1)) return false;
       ti = nti;
       g = ng;
       return true;
@@ -244,8 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_window_kernel(const Params p
       ok = step(s, b0, b1);
       if (ok && s + 1 < total) ok = step(s + 1, b1, b0);
     }
-    if (ok && my_tiles > 0) ok = epilogue((int)blockIdx.x + (my_tiles - 1) * (int)gridDim.x, my_tiles - 1);
-  } else {
+  } else if (warp == kMmaWarp) {
     // ---------------- MMA issuer: the whole warp runs the loop, one elected lane issues ----------------
     // Descriptors are kept as 32-bit low words (start address, in 16-byte units, plus the constant
     // leading-dimension field) that advance by additions; the issue loop has no divisions.
@@ -299,10 +267,48 @@ __global__ void __launch_bounds__(kThreads, 1) conv_window_kernel(const Params p
       }
       if (ok) umma_commit_elect(bars + 8 * (4 + set));  // accumulator set complete
     }
+  } else {
+    // ---------------- epilogue ----------------
+    const int quad = warp & 3, half = (warp - kProducerWarps) >> 2;  // a warp reads the quarter of the lanes that its index says
+    for (int i = 0; i < my_tiles && ok; ++i) {
+      const int set = i & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * (4 + set), (i >> 1) & 1, status, 5));
+      if (!ok) break;
+      tc_fence_after();
+      const int P = ((int)blockIdx.x + i * (int)gridDim.x) * kTileM + quad * 32 + lane;
+      uint32_t b, r, y, x;
+      p.d_HpWp.divmod(P, b, r);
+      p.d_Wp.divmod(r, y, x);
+      const bool valid = (int)b < p.Nb && (int)y < p.Ho && (int)x < p.Wo;
+      const int howo = p.Ho * p.Wo;
+      float* q = p.out + (int64_t)b * p.N * howo + (int)y * p.Wo + (int)x;
+      // this warp's share: 32 rows (its lane quadrant) x BN/2 columns, in pieces of 16 columns
+      constexpr int CW = BN / 2;
+#pragma unroll
+      for (int c0 = 0; c0 < CW; c0 += 16) {
+        const int col = half * CW + c0;
+        const uint32_t t0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(set * kAccCols * BN + col);
+        uint32_t r[kAccCols][16];
+#pragma unroll
+        for (int a = 0; a < kAccCols; ++a) tmem_ld16_nowait(t0 + (uint32_t)(a * BN), r[a]);
+        tmem_wait_ld();
+        if (valid) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int n = col + j;
+            const float v = __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
+            if (n < p.N) q[(int64_t)n * howo] = v + bias_s[n];
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + 8 * (6 + set));
+    }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == kProducerWarps) {
+  if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
