@@ -374,33 +374,40 @@ rt_status gemm_plain(rt_ctx* ctx, const LA& la, const LB& lb, float* c, int64_t 
 // ---- narrow products -------------------------------------------------------------------------------------------
 // A classifier head (N <= 16 output columns) or its input gradient (K <= 16) gives a tile kernel one or two CTAs that
 // walk K serially; these two kernels spread the same arithmetic over the block instead.
-constexpr int kSkinnyN = 16, kSkinnyRows = 32, kSkinnyKC = 128, kSkinnySlices = 8;
+constexpr int kSkinnyN = 16, kSkinnyThreads = 256;
 
-// C[M, N<=16] = A x B.  A block owns 32 rows of C: A and B chunks of 128 k are staged in shared memory with coalesced
-// loads whatever the storage order, thread (row, slice) accumulates every 8th k, the 8 slices are added in a fixed order.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(kSkinnyRows * kSkinnySlices)
+// C[M, N<=16] = A x B.  A block owns ROWS rows of C: chunks of A and B are staged in shared memory with coalesced loads whatever the
+// storage order, the next chunk on its way while one is multiplied; thread (row, slice) accumulates every SLICES-th k, the slices are added
+// in a fixed order.  Bound by latency, of which a chunk is a round trip to memory: blocks of 8 rows and chunks of 256 while all of them (two
+// an SM, for their registers) run at once; each block reads all of B, so that with more rows 32 a block are cheaper.  us in blocks of 8 and
+// of 32 rows, 64 x 10 x 128: 2.6, 3.3; 1000 x 10 x 300: 3.8, 6.2; 2000 x 10 x 1000: 9.0, 13.5; 4700 x 16 x 600: 12.5, 9.4.
+template <int ROWS>
+struct Skinny {
+  static constexpr int slices = kSkinnyThreads / ROWS, chunk = ROWS == 32 ? 128 : 256;
+  static constexpr int pitch = chunk + 32 / ROWS;  // a warp has 32 / ROWS consecutive k of each row
+};
+template <bool TA, bool TB, int ROWS>
+__global__ void __launch_bounds__(kSkinnyThreads)
 gemm_skinny_n_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ b, int64_t ldb, float* __restrict__ c,
                      int64_t ldc, int M, int N, int K, const float* __restrict__ bias, int act, int accumulate) {
   RT_PDL_ENTRY();
-  constexpr int T = kSkinnyRows * kSkinnySlices;
-  __shared__ float As[kSkinnyRows][kSkinnyKC + 1];
-  __shared__ __align__(16) float Bs[kSkinnyKC][kSkinnyN];
-  __shared__ float red[kSkinnySlices][kSkinnyRows][kSkinnyN + 1];
-  const int tid = threadIdx.x, ml = tid & 31, ks = tid >> 5;
-  const int m0 = blockIdx.x * kSkinnyRows;
+  constexpr int T = kSkinnyThreads, KC = Skinny<ROWS>::chunk, S = Skinny<ROWS>::slices;
+  __shared__ float As[ROWS][Skinny<ROWS>::pitch];
+  __shared__ __align__(16) float Bs[KC][kSkinnyN];
+  __shared__ float red[S][ROWS][kSkinnyN + 1];
+  const int tid = threadIdx.x, ml = tid % ROWS, ks = tid / ROWS;
+  const int m0 = blockIdx.x * ROWS;
   float acc[kSkinnyN];
 #pragma unroll
   for (int j = 0; j < kSkinnyN; ++j) acc[j] = 0.f;
-  for (int k0 = 0; k0 < K; k0 += kSkinnyKC) {
-    // all loads of the chunk are issued before the first store, so the chunk costs one memory round trip
-    constexpr int kALoads = kSkinnyRows * kSkinnyKC / T, kBLoads = kSkinnyKC * kSkinnyN / T;
-    float ar[kALoads], br_[kBLoads];
+  constexpr int kALoads = ROWS * KC / T, kBLoads = KC * kSkinnyN / T;
+  float ar[kALoads], br_[kBLoads];
+  auto load = [&](int k0) {
 #pragma unroll
     for (int u = 0; u < kALoads; ++u) {
       const int i = tid + u * T;
       int mm, kk;
-      if (TA) { mm = i % kSkinnyRows; kk = i / kSkinnyRows; } else { kk = i % kSkinnyKC; mm = i / kSkinnyKC; }
+      if (TA) { mm = i % ROWS; kk = i / ROWS; } else { kk = i % KC; mm = i / KC; }
       const bool in = m0 + mm < M && k0 + kk < K;
       const int64_t off = TA ? (int64_t)(k0 + kk) * lda + m0 + mm : (int64_t)(m0 + mm) * lda + k0 + kk;
       ar[u] = in ? __ldg(a + off) : 0.f;
@@ -409,24 +416,29 @@ gemm_skinny_n_kernel(const float* __restrict__ a, int64_t lda, const float* __re
     for (int u = 0; u < kBLoads; ++u) {
       const int i = tid + u * T;
       int j, kk;
-      if (TB) { kk = i % kSkinnyKC; j = i / kSkinnyKC; } else { j = i % kSkinnyN; kk = i / kSkinnyN; }
+      if (TB) { kk = i % KC; j = i / KC; } else { j = i % kSkinnyN; kk = i / kSkinnyN; }
       const bool in = j < N && k0 + kk < K;
       const int64_t off = TB ? (int64_t)j * ldb + k0 + kk : (int64_t)(k0 + kk) * ldb + j;
       br_[u] = in ? __ldg(b + off) : 0.f;
     }
+  };
+  load(0);
+  for (int k0 = 0; k0 < K; k0 += KC) {
 #pragma unroll
     for (int u = 0; u < kALoads; ++u) {
       const int i = tid + u * T;
-      if (TA) As[i % kSkinnyRows][i / kSkinnyRows] = ar[u]; else As[i / kSkinnyKC][i % kSkinnyKC] = ar[u];
+      if (TA) As[i % ROWS][i / ROWS] = ar[u]; else As[i / KC][i % KC] = ar[u];
     }
 #pragma unroll
     for (int u = 0; u < kBLoads; ++u) {
       const int i = tid + u * T;
-      if (TB) Bs[i % kSkinnyKC][i / kSkinnyKC] = br_[u]; else Bs[i / kSkinnyN][i % kSkinnyN] = br_[u];
+      if (TB) Bs[i % KC][i / KC] = br_[u]; else Bs[i / kSkinnyN][i % kSkinnyN] = br_[u];
     }
     __syncthreads();
+    if (K - k0 > KC) load(k0 + KC);
+    const int end = min(KC, K - k0);
 #pragma unroll 4
-    for (int kk = ks; kk < kSkinnyKC; kk += kSkinnySlices) {
+    for (int kk = ks; kk < end; kk += S) {
       const float av = As[ml][kk];
       const float4* br = reinterpret_cast<const float4*>(&Bs[kk][0]);
 #pragma unroll
@@ -443,12 +455,12 @@ gemm_skinny_n_kernel(const float* __restrict__ a, int64_t lda, const float* __re
 #pragma unroll
   for (int j = 0; j < kSkinnyN; ++j) red[ks][ml][j] = acc[j];
   __syncthreads();
-  for (int o = tid; o < kSkinnyRows * kSkinnyN; o += T) {
+  for (int o = tid; o < ROWS * kSkinnyN; o += T) {
     const int mm = o / kSkinnyN, j = o % kSkinnyN;
     if (m0 + mm >= M || j >= N) continue;
     float v = 0.f;
 #pragma unroll
-    for (int s2 = 0; s2 < kSkinnySlices; ++s2) v += red[s2][mm][j];
+    for (int s2 = 0; s2 < S; ++s2) v += red[s2][mm][j];
     float* dst = c + (int64_t)(m0 + mm) * ldc + j;
     if (bias || act != RT_ACT_NONE) v = rt_finish4(make_float4(v, 0.f, 0.f, 0.f), bias ? bias + j : nullptr, act, nullptr, 1).x;
     *dst = accumulate ? *dst + v : v;
@@ -478,6 +490,8 @@ __global__ void __launch_bounds__(256) gemm_small_k_kernel(const float* __restri
   }
 }
 
+bool skinny_few(const rt_ctx* ctx, int64_t m) { return m <= 16 * (int64_t)ctx->sm_count; }
+
 template <bool TA, bool TB>
 rt_status gemm_narrow_launch(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b,
                              int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
@@ -485,9 +499,10 @@ rt_status gemm_narrow_launch(rt_ctx* ctx, int64_t m, int64_t n, int64_t k, const
     rt_launch(ctx, gemm_small_k_kernel<TA, TB>, rt_grid_for(ctx, m * n, 256), 256, 0, a, lda, b, ldb, c, ldc, m * n, (int)n,
                                                                                       (int)k, accumulate);
   } else {
-    const int grid = (int)((m + kSkinnyRows - 1) / kSkinnyRows);
-    rt_launch(ctx, gemm_skinny_n_kernel<TA, TB>, grid, kSkinnyRows * kSkinnySlices, 0, a, lda, b, ldb, c, ldc, (int)m, (int)n,
-                                                                                        (int)k, bias, act, accumulate);
+    const bool few = skinny_few(ctx, m);
+    const int rows = few ? 8 : 32;
+    rt_launch(ctx, few ? gemm_skinny_n_kernel<TA, TB, 8> : gemm_skinny_n_kernel<TA, TB, 32>, (int)((m + rows - 1) / rows), kSkinnyThreads, 0, a, lda, b,
+              ldb, c, ldc, (int)m, (int)n, (int)k, bias, act, accumulate);
   }
   RT_LAUNCHED(ctx);
   return RT_OK;
@@ -500,10 +515,12 @@ rt_status gemm_narrow(rt_ctx* ctx, int trans_a, int trans_b, int64_t m, int64_t 
   // A thread reads k values of both operands by itself: with a reduction that is contiguous in B, or rows that are in A, these reads
   // do not coalesce, which shows from some millions of multiply-adds on (768 x 16 x 1196: B plain 10 us, B transposed 30, A transposed 16).
   const bool small_k = k <= 16 && !((trans_a || trans_b) && m * n * k > (4ll << 20)) && !bias && act == RT_ACT_NONE;
-  // One block walks the whole reduction of its 32 rows: 1.8 us and 1.2 more per 100 of it, against 5 us and more in the small tiles
-  // (351 x 173 x 7: 4.5 us here; 173 x 351 x 7: 5.8 here, 5.2 there; 88 x 1288 x 16: 17 and 7).  Many rows fill the chip all the same.
+  // One block walks the whole reduction of its rows: 1.2 us and 1.4 - 1.9 more per chunk of 256 with few rows, 1.8 and 1.2 per 100 with many,
+  // against 5 us and more in the small tiles (351 x 173 x 7: 2.5 us here; 173 x 351 x 7: 3.5 here, 5.2 there; 88 x 1288 x 16: 7.3 there).  Very many
+  // rows fill the chip all the same.
+  const float skinny = skinny_few(ctx, m) ? 1.2f + 1.6f * (float)((k + 255) / 256) : 1.8f + 0.012f * (float)k;
   const bool skinny_n = n <= kSkinnyN && k > 16 && k < (1ll << 30) && m < (1ll << 30) &&
-                        (m >= 4096 || 1.8f + 0.012f * (float)k <= rt_gemm_small_estimate(ctx, m, n, k, false));
+                        (m >= 4096 || skinny <= rt_gemm_small_estimate(ctx, m, n, k, false));
   if (!small_k && !skinny_n) return RT_ERR_UNIMPLEMENTED;
   if (!trans_a && !trans_b) return gemm_narrow_launch<false, false>(ctx, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);
   if (!trans_a && trans_b) return gemm_narrow_launch<false, true>(ctx, m, n, k, a, lda, b, ldb, c, ldc, bias, act, accumulate);

@@ -53,6 +53,13 @@ def test_large_product(api, m, k, n, trans):
     test_small_product(api, m, k, n, trans)
 
 
+# up to 16 columns: blocks of 8 rows and chunks of 256 up to 16 rows an SM (2368 on 148), of 32 and 128 beyond
+@pytest.mark.parametrize("m,k,n", [(7, 17, 1), (9, 255, 16), (8, 256, 3), (33, 257, 15), (2368, 513, 10), (2369, 129, 10), (4099, 300, 16)])
+@pytest.mark.parametrize("trans", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_product_of_few_columns(api, m, k, n, trans):
+    test_small_product(api, m, k, n, trans)
+
+
 @pytest.mark.parametrize("m,k,n", SIZES + [(300, 784, 300), (900, 70, 1000)])
 @pytest.mark.parametrize("act", [0, 1, 2, 3])
 def test_linear_layer(api, m, k, n, act):
