@@ -64,7 +64,7 @@ struct B200Backend {
     if (!s.buf->escaped)
       for (auto* r : s.buf->readers) costly = costly || r->node->kind == lazy::Kind::Opaque;
     if (!costly) s.buf->flush_readers();
-    if (s.buf.use_count() > 1 || s.buf->owner) {
+    if (s.buf.use_count() > 1 || s.buf->shares_rows()) {
       Storage c = alloc(s.shape);
       check(rt_memcpy_d2d(ctx(), c.ptr(), s.ptr(), sizeof(float) * s.numel()));
       s.buf = std::move(c.buf);
@@ -159,11 +159,12 @@ struct B200Backend {
     };
     return defer(std::move(n), shape);
   }
-  // Rows that point into another tensor's block (a slice taken inside a capture) get a block of their own.
+  // Rows that point into another tensor's block (a slice taken inside a capture) get a block of their own.  Results that were computed as
+  // rows of one matrix have theirs to themselves already, and replays of the capture go on writing there.
   static void own(const Storage& s) {
     if (!s.buf) return;
     const float* p = s.buf->data();
-    if (!s.buf->owner) return;
+    if (!s.buf->shares_rows()) return;
     lazy::Block block(ctx(), s.buf->numel);
     check(rt_memcpy_d2d(ctx(), block.ptr, p, sizeof(float) * s.buf->numel));
     s.buf->ptr = block.release();

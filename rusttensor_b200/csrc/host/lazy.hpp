@@ -14,7 +14,8 @@
 //    evaluated on the spot - except inside a graph capture, where the whole step is recorded anyway.
 //  * A slice of whole rows points into its base's block only inside a capture, where nothing outside the engine sees either of them
 //    before the step is recorded; what a step leaves behind gets a block of its own (B200Backend::own).  Elsewhere the address of one
-//    of the two may be handed out and written through, and a slice would keep its base's memory.
+//    of the two may be handed out and written through, and a slice would keep its base's memory.  Results that a capture computes as one
+//    matrix (place) are rows of a block that no tensor has as a whole: they stay there, where every replay writes them.
 //  * A capture starts with nothing unevaluated (flush_all), so that it records exactly the step's own work, and rth_sync leaves
 //    nothing unevaluated either.
 //  * Depth is bounded: a result whose expression has become kMaxDepth ops deep is evaluated at once.
@@ -86,6 +87,7 @@ struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
   size_t numel;
   bool escaped = false;
   std::shared_ptr<DeviceBuffer> owner;  // set: ptr points into this buffer's block (contiguous rows of it)
+  bool apart = false;        // with an owner: these rows of its block are this buffer's alone, and no tensor is the whole block
   uint64_t id = next_id();   // of the values: another one after every change in place
   uint64_t made_from = 0;    // id of the operand's values, for results from which their gradient follows
   std::shared_ptr<Recurrence> sequence;  // set: the state after timestep `timestep` of it
@@ -133,6 +135,8 @@ struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
         }
     }
   }
+  // Whether the values are also those of another buffer (a slice's, of its base).
+  bool shares_rows() const { return owner && !apart; }
   float* data() {
     if (node) lazy_evaluate(this);
     return ptr;
@@ -873,7 +877,7 @@ inline const Input* times_constant(const Node* n, float* c) {
   return nullptr;
 }
 
-// Several results computed as one matrix, in a capture: each is rows of the common block.
+// Several results computed as one matrix, in a capture: each is rows of the common block, and the only one to be so.
 inline std::shared_ptr<DeviceBuffer> common_block(rt_ctx* ctx, size_t numel) {
   Block block(ctx, numel);
   auto b = std::make_shared<DeviceBuffer>(ctx, block.ptr, numel);
@@ -883,6 +887,7 @@ inline std::shared_ptr<DeviceBuffer> common_block(rt_ctx* ctx, size_t numel) {
 inline void place(DeviceBuffer* b, const std::shared_ptr<DeviceBuffer>& block, size_t offset) {
   b->ptr = block->ptr + offset;
   b->owner = block;
+  b->apart = true;
   b->drop_node();
 }
 
@@ -1282,7 +1287,7 @@ inline bool rewrite_rows(DeviceBuffer* b) {
   for (size_t j = 0; j < n->shape.size(); ++j) off = off * (int64_t)base.shape[j] + (int64_t)n->starts[j];
   std::shared_ptr<DeviceBuffer> root = base.buf;
   const float* p = root->data();
-  while (root->owner) root = root->owner;
+  while (root->shares_rows()) root = root->owner;
   b->ptr = const_cast<float*>(p) + off;
   b->owner = root;
   b->drop_node();

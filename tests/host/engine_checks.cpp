@@ -116,6 +116,11 @@ rt_status rt_graph_end(rt_ctx*, rt_graph**) { return RT_OK; }
 rt_status rt_fill(rt_ctx*, float*, float, int64_t) { return RT_OK; }
 rt_status rt_gemm(rt_ctx*, int, int, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, float*, int64_t, int) { return RT_OK; }
 rt_status rt_gemm_bias_act(rt_ctx*, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, const float*, int, float*, int64_t) { return RT_OK; }
+rt_status rt_softmax_nll_list(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, float, float, int, const float* const*, float*) {
+  return RT_OK;
+}
+rt_status rt_softmax_nll_with_grad(rt_ctx*, const float*, const float*, int64_t, int64_t, float, float, const float*, float, float*, float*) { return RT_OK; }
+rt_status rt_softmax_nll_scaled_backward(rt_ctx*, const float*, const float*, int64_t, int64_t, float, float*) { return RT_OK; }
 rt_status rt_matmul_backward(rt_ctx*, const float*, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) { return RT_OK; }
 rt_status rt_gemm_sum_products(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, int64_t, float*) { return RT_OK; }
 rt_status rt_reduce(rt_ctx*, int, const float*, int64_t, int64_t, int64_t, float*) { return RT_OK; }
@@ -377,10 +382,70 @@ void cells_become_a_sequence() {
   }
 }
 
+// What a captured step computes as rows of one matrix (the states of a sequence, the output layer's results, the gradients of the losses) and
+// somebody keeps stays where every replay writes it when its address is asked for; a slice of it goes elsewhere.
+void kept_results_stay_where_they_are_written() {
+  using Tn = Tensor<B>;
+  const size_t T = 4, Bn = 2, V = 3, H = 2;
+  for (bool states : {true, false}) {  // with states kept the backward pass goes timestep by timestep
+    const Tn x(make({T * Bn, V}, 0.f, .01f), false), y(make({T * Bn, V}, 0.f, .01f), false), w(make({V + H, 4 * H}, 0.f, .01f), true);
+    const Tn b(make({4 * H}, 0.f, .01f), true), wo(make({H, V}, 0.f, .1f), true), bo(make({V}, 0.f, .1f), true);
+    std::vector<Tn> kept;
+    std::vector<B::Storage> slices;
+    B::begin_capture();
+    Tn sum;
+    {
+      Tn h = Tn::zeros({Bn, H}, false), c = Tn::zeros({Bn, H}, false);
+      for (size_t t = 0; t < T; ++t) {
+        const Tn xh = ops::concat<B>({ops::slice(x, {{t * Bn, (t + 1) * Bn}, {0, V}}), h}, 1);
+        const Tn z = ops::add(ops::matmul(xh, w), b.broadcast_to({Bn, 4 * H}));
+        auto gate = [&](size_t k) { return ops::slice(z, {{0, Bn}, {k * H, (k + 1) * H}}); };
+        const Tn i = ops::sigmoid(gate(0)), f = ops::sigmoid(gate(1));
+        c = ops::add(ops::mul(f, c), ops::mul(i, ops::tanh(gate(2))));
+        h = ops::mul(ops::sigmoid(gate(3)), ops::tanh(c));
+        const Tn logits = ops::add(ops::matmul(h, wo), bo.broadcast_to({Bn, V}));
+        const Tn l = ops::softmax_cross_entropy(logits, ops::slice(y, {{t * Bn, (t + 1) * Bn}, {0, V}}), 1, Reduction::Mean);
+        sum = t ? ops::add(sum, l) : l;
+        if (t == 1) kept = states ? std::vector<Tn>{logits, h, c, i} : std::vector<Tn>{logits};
+      }
+    }
+    sum.backward();
+    for (auto& g : {sum.data(), *w.grad(), *b.grad(), *wo.grad(), *bo.grad()}) B::own(g);
+    slices = {B::slice(kept[0].data(), {{1, 2}, {0, V}}), B::slice(kept[0].data(), {{1, 2}, {0, V}})};
+    sum.detach_graph();
+    std::vector<B::Storage> all;
+    for (auto& k : kept) all.push_back(k.data());
+    if (!states) all.push_back(*kept[0].grad());
+    std::vector<float*> where;
+    for (auto& s : all) where.push_back(s.ptr());
+    for (auto& s : all) EXPECT(s.buf->owner != nullptr);
+    for (auto& s : slices) EXPECT(s.ptr() == where[0] + V);
+    rt_graph* graph = nullptr;
+    B::end_capture(&graph);
+    for (size_t k = 0; k < all.size(); ++k) {
+      EXPECT(B::escape(all[k]) == where[k]);
+      scribble(where[k], all[k].numel());
+      EXPECT(all[k].ptr() == where[k]);
+    }
+    EXPECT(B::escape(slices[0]) != where[0] + V);
+    B::Storage logits = kept[0].data();
+    all.clear();
+    kept.clear();
+    B::make_unique(logits);  // the other slice still reads the rows
+    EXPECT(logits.ptr() != where[0] && slices[1].ptr() == where[0] + V);
+    slices.clear();
+    float* const own = logits.ptr();
+    B::make_unique(logits);
+    EXPECT(logits.ptr() == own);
+  }
+  EXPECT(live.empty());
+}
+
 const struct {
   const char* name;
   void (*run)();
 } kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence},
+               {"kept_results_stay_where_they_are_written", kept_results_stay_where_they_are_written},
                {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},
                {"pooling_knows_its_relu", pooling_knows_its_relu},
