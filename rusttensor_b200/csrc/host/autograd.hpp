@@ -153,6 +153,23 @@ struct TensorData {
   std::optional<typename B::Storage> grad;
   bool requires_grad;
   std::shared_ptr<Op<B>> op;
+  // Ops are let go of one after another, not each within the one that takes its result: a tape may be as long as a sequence.
+  ~TensorData() {
+    if (!op || op.use_count() > 1) return;
+    thread_local std::vector<std::shared_ptr<Op<B>>>* dying = nullptr;  // of the call that is at it
+    if (dying) {
+      dying->push_back(std::move(op));
+      return;
+    }
+    std::vector<std::shared_ptr<Op<B>>> all;
+    dying = &all;
+    all.push_back(std::move(op));
+    while (!all.empty()) {
+      const std::shared_ptr<Op<B>> o = std::move(all.back());
+      all.pop_back();
+    }
+    dying = nullptr;
+  }
 };
 
 // A backend may add a product's weight gradient to the gradient the weight already holds (a weight used at every timestep

@@ -18,7 +18,8 @@
 //    matrix (place) are rows of a block that no tensor has as a whole: they stay there, where every replay writes them.
 //  * A capture starts with nothing unevaluated (flush_all), so that it records exactly the step's own work, and rth_sync leaves
 //    nothing unevaluated either.
-//  * Depth is bounded: a result whose expression has become kMaxDepth ops deep is evaluated at once.
+//  * Depth is bounded: a result whose expression has become kMaxDepth ops deep is evaluated at once.  The timesteps of a recurrence in a
+//    capture, which wait for the last one, are evaluated from the first one on where they do not become one sequence.
 //
 // What is written to memory besides the asked-for result: intermediate results that somebody else still refers to, when the
 // tensor is small (a launch later on would cost more than the store), or when recomputing them would be expensive.
@@ -27,6 +28,7 @@
 #include <cstring>
 #include <functional>
 #include <memory>
+#include <unordered_set>
 #include <vector>
 
 #include "../../../include/rt_b200.h"
@@ -61,6 +63,7 @@ struct Node {
   Tag tag = Tag::None;
   std::vector<int64_t> geo;  // its parameters, as its tag has them
   std::function<void(Node&, DeviceBuffer*)> run;  // computes the buffer (sets ptr)
+  bool waits() const { return tag == Tag::Matmul && !geo.empty(); }  // the product of a recurrence's timestep, for the last one
 };
 
 constexpr int kMaxDepth = 200;
@@ -105,9 +108,15 @@ struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
     static DeviceBuffer* h = nullptr;
     return h;
   }
+  // How many products of timesteps wait for their last one.
+  static size_t& waiting() {
+    static size_t n = 0;
+    return n;
+  }
   DeviceBuffer(rt_ctx* c, float* p, size_t n) : ctx(c), ptr(p), numel(n) {}
   DeviceBuffer(rt_ctx* c, std::unique_ptr<lazy::Node> nd, size_t n) : ctx(c), ptr(nullptr), numel(n), node(std::move(nd)) {
     for (auto& i : node->in) i.buf->readers.push_back(this);
+    if (node->waits()) ++waiting();
     next = head();
     if (next) next->prev = this;
     head() = this;
@@ -125,6 +134,10 @@ struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
     else head() = next;
     if (next) next->prev = prev;
     prev = next = nullptr;
+    // The operands are let go of one after another, not each within the one that reads it: an expression may be as deep as a sequence is long.
+    static auto& dying = *new std::vector<std::shared_ptr<DeviceBuffer>>;  // used until the last buffer goes, at exit
+    static bool busy = false;
+    if (gone->waits()) --waiting();
     for (auto& i : gone->in) {
       auto& r = i.buf->readers;
       for (size_t k = r.size(); k-- > 0;)
@@ -133,7 +146,15 @@ struct DeviceBuffer : std::enable_shared_from_this<DeviceBuffer> {
           r.pop_back();
           break;
         }
+      dying.push_back(std::move(i.buf));
     }
+    if (busy) return;
+    busy = true;
+    while (!dying.empty()) {
+      const std::shared_ptr<DeviceBuffer> b = std::move(dying.back());
+      dying.pop_back();
+    }
+    busy = false;
   }
   // Whether the values are also those of another buffer (a slice's, of its base).
   bool shares_rows() const { return owner && !apart; }
@@ -979,31 +1000,65 @@ inline int64_t timestep_of(const Input& a, const Input& w) {
   q.c->node->depth = 1;  // like the products: the sequence is evaluated from its first timestep on, however long it is
   return t + 1;
 }
+// The states of the cells, the first first, each by itself: what becomes of a recurrence that is not a sequence (any more, since somebody has
+// asked for something within it).  Whether b is among what has been evaluated.
+inline bool evaluate_in_order(const std::vector<Cell>& cells, DeviceBuffer* b) {
+  for (const Cell& q : cells)
+    if (q.h.get() != b) lazy_evaluate(q.h.get());
+  return !b->node;
+}
+// The states of such cells that the expression b reads, the last first, which brings the others along.  Walking through them would be as deep as the
+// recurrence is long: a cell state reads the one before.
+inline void settle_states(DeviceBuffer* b) {
+  if (!capturing() || DeviceBuffer::waiting() == 0) return;
+  std::vector<std::pair<int64_t, std::shared_ptr<DeviceBuffer>>> states;
+  std::unordered_set<const DeviceBuffer*> seen;
+  std::vector<const Node*> open{b->node.get()};
+  while (!open.empty()) {
+    const Node* n = open.back();
+    open.pop_back();
+    for (const Input& i : n->in) {
+      const Node* m = pending(i);
+      Cell q;
+      if (!m || !seen.insert(i.buf.get()).second) continue;
+      if (match_cell(i.buf.get(), &q)) states.push_back({q.product->node->geo[0], i.buf});
+      else if (m->kind != Kind::Opaque || m->waits()) open.push_back(m);
+    }
+  }
+  std::stable_sort(states.begin(), states.end(), [](auto& x, auto& y) { return x.first > y.first; });
+  for (auto& s : states) lazy_evaluate(s.second.get());
+}
 inline bool rewrite_recurrence(DeviceBuffer* b) {
   if (!capturing() || !is_op(b->node.get(), Kind::Binary, RT_F_MUL)) return false;
   std::vector<Cell> cells;  // the last first
-  for (DeviceBuffer* at = b;;) {
+  bool whole = false;
+  for (DeviceBuffer* at = b; !whole;) {
     Cell q;
-    if (!at->node || !match_cell(at, &q)) return false;
-    if (!cells.empty() && (cells.back().c_prev.buf != q.c || cells.back().w.buf != q.w.buf || cells.back().bias.buf != q.bias.buf)) return false;
+    if (!at->node || !match_cell(at, &q)) break;
+    if (!cells.empty() && (cells.back().c_prev.buf != q.c || cells.back().w.buf != q.w.buf || cells.back().bias.buf != q.bias.buf)) break;
     at = q.h_prev.buf.get();
     cells.push_back(std::move(q));
-    if (is_zero(cells.back().h_prev) && is_zero(cells.back().c_prev)) break;
+    whole = is_zero(cells.back().h_prev) && is_zero(cells.back().c_prev);
   }
   std::reverse(cells.begin(), cells.end());
+  if (!whole) return !cells.empty() && evaluate_in_order(cells, b);
   auto seq = std::make_shared<Recurrence>();
   const Input& w = cells[0].w;
   Input x;
   int64_t first = 0;
-  for (size_t t = 0; t < cells.size(); ++t) {  // as timestep_of has found them
+  for (size_t t = 0; t < cells.size(); ++t) {  // as timestep_of has found them, unless a timestep's inputs have been asked for
     Input base;
-    int64_t at;
-    if (!rows_of(pending(cells[t].xh)->in[0], &base, &at)) return false;
-    if (t == 0) {
+    int64_t at = 0;
+    const bool rows = rows_of(pending(cells[t].xh)->in[0], &base, &at);
+    if (rows && t == 0) {
       x = base;
       first = at;
     }
-    if (base.buf != x.buf || at != first + (int64_t)(t * cells[0].h_prev.shape[0])) return false;
+    if (!rows || base.buf != x.buf || at != first + (int64_t)(t * cells[0].h_prev.shape[0])) {
+      if (t == 0) return evaluate_in_order(cells, b);
+      lazy_evaluate(cells[t - 1].h.get());  // those before it are a sequence
+      return evaluate_in_order(cells, b);
+    }
   }
   seq->steps = (int64_t)cells.size();
   seq->batch = (int64_t)cells[0].h_prev.shape[0];
@@ -1037,6 +1092,7 @@ struct Linear {
   DeviceBuffer* out;
   Input a, b, bias;  // bias.buf null: none
   int act;
+  bool waits;  // of a recurrence's timestep: those after it need its result
 };
 inline bool match_linear(DeviceBuffer* out, Linear* l) {
   const Node* n = out->node.get();
@@ -1046,6 +1102,7 @@ inline bool match_linear(DeviceBuffer* out, Linear* l) {
     l->a = n->in[0];
     l->b = n->in[1];
     l->bias = Input{};
+    l->waits = n->waits();
     return true;
   }
   const Node* sum = n;
@@ -1064,6 +1121,7 @@ inline bool match_linear(DeviceBuffer* out, Linear* l) {
     l->a = m->in[0];
     l->b = m->in[1];
     l->bias = bias;
+    l->waits = m->waits();
     return true;
   }
   return false;
@@ -1081,7 +1139,8 @@ inline bool rewrite_linear(DeviceBuffer* b) {
   if (!match_linear(b, &first)) return false;
   std::vector<Linear> all{first};
   const float *pa = first.a.buf->data(), *pb = first.b.buf->data(), *bias = first.bias.buf ? first.bias.buf->data() : nullptr;
-  const std::vector<DeviceBuffer*> others = first.b.buf->readers;
+  std::vector<DeviceBuffer*> others;
+  if (!first.waits) others = first.b.buf->readers;
   for (DeviceBuffer* r : others) {
     if (all.size() == 256) break;
     if (!r->node || r->node->tag != Tag::Matmul || r->node->in[1].buf != first.b.buf || r->node->in[0].buf->node) continue;
@@ -1356,6 +1415,8 @@ inline void lazy_evaluate(DeviceBuffer* b) {
     b->drop_node();
     return;
   }
+  settle_states(b);
+  if (!b->node) return;
   const bool lone = (b->node->kind == Kind::Unary || b->node->kind == Kind::Binary) &&
                     std::all_of(b->node->in.begin(), b->node->in.end(), [](const Input& i) { return !i.buf->node; });
   if ((lone || b->node->kind == Kind::Const) && evaluate_alone(b)) return;

@@ -441,10 +441,51 @@ void kept_results_stay_where_they_are_written() {
   EXPECT(live.empty());
 }
 
+// However long a recurrence in a capture is, evaluating it and letting go of it takes a bounded stack, whatever is asked for first.
+void long_recurrences() {
+  using Tn = Tensor<B>;
+  const size_t T = 20000, Bn = 1, V = 1, H = 1;
+  enum { kGateFirst, kInputFirst, kLastGateAlone, kCellState, kOfTheLastState, kNothing, kWays };
+  for (int way = 0; way < kWays; ++way) {
+    forward_sequences = 0;
+    {
+      const Tn x(make({T * Bn, V}, 0.f, .01f), false), w(make({V + H, 4 * H}, 0.f, .01f), true), b(make({4 * H}, 0.f, .01f), true);
+      B::begin_capture();
+      {
+        Tn h = Tn::zeros({Bn, H}, false), c = Tn::zeros({Bn, H}, false), asked;
+        for (size_t t = 0; t < T; ++t) {
+          const Tn xt = ops::slice(x, {{t * Bn, (t + 1) * Bn}, {0, V}}), xh = ops::concat<B>({xt, h}, 1);
+          const Tn z = ops::add(ops::matmul(xh, w), b.broadcast_to({Bn, 4 * H}));
+          auto gate = [&](size_t k) { return ops::slice(z, {{0, Bn}, {k * H, (k + 1) * H}}); };
+          const Tn i = ops::sigmoid(gate(0)), f = ops::sigmoid(gate(1));
+          c = ops::add(ops::mul(f, c), ops::mul(i, ops::tanh(gate(2))));
+          h = ops::mul(ops::sigmoid(gate(3)), ops::tanh(c));
+          if (way == kGateFirst && t == 3) asked = f;
+          if (way == kInputFirst && t == 3) asked = xt;
+          if (way == kLastGateAlone && t + 1 == T) asked = i;
+          if (way == kCellState && t + 1 == T) asked = c;
+          if (way == kOfTheLastState && t + 1 == T) asked = ops::square(ops::exp(h));
+          if (way == kLastGateAlone) {  // no tape: nothing but the next timestep holds a state
+            h.detach_graph();
+            c.detach_graph();
+          }
+        }
+        if (way == kLastGateAlone) h = c = Tn();
+        if (asked.inner) asked.data().ptr();
+        if (way == kGateFirst || way == kInputFirst) h.data().ptr();
+      }
+      rt_graph* graph = nullptr;
+      B::end_capture(&graph);
+    }
+    EXPECT(forward_sequences == (way == kNothing ? 0 : 1));  // of the timesteps that are one still
+    EXPECT(live.empty() && !DeviceBuffer::head());
+  }
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence},
+} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences},
                {"kept_results_stay_where_they_are_written", kept_results_stay_where_they_are_written},
                {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},
