@@ -37,8 +37,9 @@ struct ConvSplitArgs {
   ImageSplit image[kMaxImages];
   TapSplit taps;        // w null: none
   int images, sample_blocks;
-  const uint2* samples; // [source][block]; the weights, the last source, are looked at as a whole
-  uint2* stats;         // [image][block] of conv_split_kernel<false>
+  uint32_t most_faint[kMaxSources];
+  const Magnitudes* samples;  // [source][block]; the weights, the last source, are looked at as a whole
+  Magnitudes* stats;          // [source][block] of conv_split_kernel<false>; of the weights only how many are faint
   Decision* decision;
 };
 // Bound by memory: 4 bytes read and 4 written an element.  A block turns 32 channels x 128 pixels at a time through shared memory; what is
@@ -46,15 +47,20 @@ struct ConvSplitArgs {
 template <bool AGAIN>
 __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) {
   RT_PDL_ENTRY();
-  __shared__ uint32_t red[2][8];
+  __shared__ uint32_t red[3][8];
   __shared__ float tile[32][kSplitPixels + 1];
   constexpr int depth = AGAIN ? 16 : 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, weights = a.taps.w ? 1 : 0;
   Decision d{};
   for (int q = 0; q < a.images + weights; ++q) {
-    const uint2 v = extremes_of(a.samples + q * a.sample_blocks, a.sample_blocks, red);
-    d.exponent[q] = exponent_for(v.x);
-    if (AGAIN && out_of_range(q < a.images ? extremes_of(a.stats + q * gridDim.x, gridDim.x, red) : v, d.exponent[q])) d.wide = 1;
+    Magnitudes v = over_blocks(a.samples + q * a.sample_blocks, a.sample_blocks, red);
+    d.exponent[q] = exponent_for(v.most);
+    if (AGAIN) {
+      const Magnitudes seen = over_blocks(a.stats + q * gridDim.x, gridDim.x, red);
+      if (q < a.images) v = seen;
+      v.faint = seen.faint;
+      if (out_of_range(v, d.exponent[q], a.most_faint[q])) d.wide = 1;
+    }
   }
   if (AGAIN) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.decision = d;
@@ -63,7 +69,8 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
   for (int q = 0; q < a.images; ++q) {
     const ImageSplit& s = a.image[q];
     const float scale = AGAIN ? 1.f : ldexpf(1.f, d.exponent[q]);
-    uint32_t most = 0, least = 0xffffffffu;
+    const uint32_t faint = faint_below(d.exponent[q]);
+    Magnitudes all;
     for (int i0 = blockIdx.x; i0 < s.tiles; i0 += gridDim.x) {
       uint32_t im, t;
       s.d_tiles.divmod((uint32_t)i0, im, t);
@@ -78,6 +85,7 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
           for (int j = 0; j < 4; ++j) v[i][j] = c0 + c < s.C && lane + 32 * j < left ? __ldcs(src + (int64_t)c * s.HW + lane + 32 * j) : 0.f;
         }
         __syncthreads();  // the tile before has been read
+        uint32_t low = 0xffffffffu;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int c = warp * 4 + i;
@@ -85,12 +93,14 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             tile[c][lane + 32 * j] = v[i][j];
-            row = max(row, __float_as_uint(v[i][j]) & 0x7fffffffu);
+            const uint32_t m = __float_as_uint(v[i][j]) & 0x7fffffffu;
+            row = max(row, m);
+            low = lower(low, m);
           }
           if (AGAIN) continue;
           row = __reduce_max_sync(0xffffffffu, row);
-          most = max(most, row);
-          if (row) least = min(least, row);
+          all.most = max(all.most, row);
+          if (row) all.least = min(all.least, row);
           if (s.sums) {
             float sum = (v[i][0] + v[i][1]) + (v[i][2] + v[i][3]);
 #pragma unroll
@@ -98,6 +108,7 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
             if (lane == 0 && c0 + c < s.C) s.sums[(int64_t)i0 * s.C + c0 + c] = sum;
           }
         }
+        all.faint += low < faint;
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < 2; ++i) {  // eight channels of a pixel
@@ -121,8 +132,8 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
       }
     }
     if (!AGAIN) {
-      const uint2 v = block_extremes(most, least, red);
-      if (threadIdx.x == 0) a.stats[q * gridDim.x + blockIdx.x] = v;
+      all = over_block(all, red);
+      if (threadIdx.x == 0) a.stats[q * gridDim.x + blockIdx.x] = all;
     }
   }
   if (!weights) return;
@@ -130,6 +141,8 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
   const float scale = AGAIN ? 1.f : ldexpf(1.f, d.exponent[a.images]);
   const int eighths = (s.C + depth - 1) / depth * depth / 8, taps = s.kh * s.kw;
   const int64_t total = (int64_t)s.N * taps * eighths;
+  const uint32_t faint = faint_below(d.exponent[a.images]);
+  Magnitudes all;
   // from the last block on, which has had the least to do
   for (int64_t i = (int64_t)(gridDim.x - 1 - blockIdx.x) * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
     const int c = (int)(i % eighths) * 8, tap = (int)(i / eighths % taps), n = (int)(i / eighths / taps);
@@ -144,8 +157,13 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
     }
     const float* w = s.w + row * s.sn + ky * s.sky + kx * s.skx + s.off;
     float x[8];
+    uint32_t low = 0xffffffffu;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = there && c + j < s.C ? __ldg(w + (c + j) * s.sc) : 0.f;
+    for (int j = 0; j < 8; ++j) {
+      x[j] = there && c + j < s.C ? __ldg(w + (c + j) * s.sc) : 0.f;
+      low = lower(low, __float_as_uint(x[j]) & 0x7fffffffu);
+    }
+    all.faint += low < faint;
     uint4 part[4];
     split8(x, AGAIN, scale, part);
     uint16_t* o = s.out + n * s.pitch + ((int64_t)tap * (eighths * 8 / depth) + c / depth) * 64 + c % depth;
@@ -155,6 +173,10 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
       *reinterpret_cast<uint4*>(o + 2 * depth) = part[2];
       *reinterpret_cast<uint4*>(o + 3 * depth) = part[3];
     }
+  }
+  if (!AGAIN) {
+    all = over_block(all, red);
+    if (threadIdx.x == 0) a.stats[a.images * gridDim.x + blockIdx.x] = all;
   }
 }
 
@@ -460,11 +482,11 @@ inline void choose_box(int pixels, int w, int h, int n, int* bw, int* bh, int* b
 // Parts of images and weights (taps null: none).
 inline rt_status split_conv(rt_ctx* ctx, Image* const* images, int n_images, Taps* taps, RtScratch* work, Decision** decision) {
   const int sample_blocks = ctx->sm_count, blocks = 4 * ctx->sm_count;
-  rt_status st = work->alloc(sizeof(uint2) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
+  rt_status st = work->alloc(sizeof(Magnitudes) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
   if (st != RT_OK) return st;
   SampleArgs a{};
   ConvSplitArgs b{};
-  uint2* samples = work->as<uint2>();
+  Magnitudes* samples = work->as<Magnitudes>();
   a.count = n_images + (taps ? 1 : 0);
   b.sample_blocks = sample_blocks;
   b.samples = samples;
@@ -476,6 +498,7 @@ inline rt_status split_conv(rt_ctx* ctx, Image* const* images, int n_images, Tap
     if ((st = im.alloc()) != RT_OK) return st;
     const int64_t hw = (int64_t)im.H * im.W;
     a.s[q] = sample_of(ctx, im.p, hw, (int64_t)im.Nb * im.C, hw, false);
+    b.most_faint[q] = most_faint((int64_t)im.Nb * im.C * hw);
     ImageSplit& s = b.image[q];
     s.p = im.p;
     s.out = im.mem.as<uint16_t>();
@@ -490,6 +513,7 @@ inline rt_status split_conv(rt_ctx* ctx, Image* const* images, int n_images, Tap
     if ((st = taps->alloc()) != RT_OK) return st;
     b.taps = taps->t;
     a.s[n_images] = sample_of(ctx, taps->all, taps->all_cols, taps->all_rows, taps->all_cols, true);
+    b.most_faint[n_images] = most_faint(taps->all_rows * taps->all_cols);
   }
   rt_launch(ctx, sample_kernel, sample_blocks, 256, 0, a, samples);
   RT_LAUNCHED(ctx);

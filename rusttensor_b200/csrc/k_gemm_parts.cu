@@ -5,10 +5,13 @@
 // another that is scaled down at the end.  That is three MMAs of kind::f16 where 3xTF32 takes three of kind::tf32 at half the rate and twice
 // the bytes, and it drops less: lo * lo is below 2^-24 of a product, 2^-20 with the truncated TF32 parts.
 // The scale comes from a sample of the operand, whose largest magnitude becomes 2^9; the pass that splits looks at all of it.  lo is exact
-// to 2^-36.  If an element reaches 2^15 after scaling, or a segment (128 columns of a row, 64 rows of a column) lies wholly below 2^-9, or
-// there are infinities, NaN or scales beyond 2^100, a third pass, which otherwise ends at once, splits again into three bf16 parts (8 + 8 + 8
-// bits, exact, the exponents of fp32) and the same kernel runs six MMAs where it otherwise runs three.  Within these lines an element keeps its
-// 22 bits or is off by less than 2^-27 of its own segment.  The decision is made on the device; nothing waits for it on the host.
+// to 2^-36.  If an element reaches 2^15 after scaling, or a segment (128 columns of a row, 64 rows of a column) lies wholly below 2^-9, or more
+// elements than one in 2^20 are not zero and below 2^-22, or there are infinities, NaN or scales beyond 2^100, a third pass, which otherwise ends
+// at once, splits again into three bf16 parts (8 + 8 + 8 bits, exact, the exponents of fp32) and the same kernel runs six MMAs where it otherwise
+// runs three.  Within these lines an element keeps its 22 bits or is off by less than 2^-36 after scaling, which is 2^-27 of its segment's largest
+// and 2^-14 of itself.  Where the terms of a result all weigh the same, what the parts drop is 1.1e-7 of |A| |B| with magnitudes spread evenly over
+// 2^31, 3.3e-7 with 3xTF32; over 2^33, where the line is crossed, 8e-7 and 5e-7, over 2^40 6e-5.
+// The decision is made on the device; nothing waits for it on the host.
 //
 // A K-block in memory is four slots of 16 along the reduction: hi hi lo lo of 32 elements, or the three bf16 parts of 16 and the first once
 // more, with zeros for infinities and NaN: the cross terms take that one, so that an infinity meets no zero which is none.  A row of it is
@@ -49,13 +52,14 @@ struct SplitSource {
 struct SplitArgs {
   SplitSource s[kMaxSplits];
   int count, sources, sample_blocks;
-  const uint2* samples;  // [source][block] of sample_kernel
-  uint2* stats;          // [source][block] of split_kernel<false>
+  uint32_t most_faint[kMaxSources];
+  const Magnitudes* samples;  // [source][block] of sample_kernel
+  Magnitudes* stats;          // [source][block] of split_kernel<false>
   Decision* decision;
 };
 // A tile of 64 rows x 128 columns: a warp has eight rows, two at a time, a lane eight columns of one.
 template <bool VEC, bool AGAIN>
-__device__ __forceinline__ void split_tiles(const SplitSource& s, float scale, uint32_t (*cols)[16][kTileCols], uint32_t& most, uint32_t& least) {
+__device__ __forceinline__ void split_tiles(const SplitSource& s, float scale, uint32_t faint, uint32_t (*cols)[16][kTileCols], Magnitudes& all) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, piece = lane & 15;
   constexpr int depth = AGAIN ? 16 : 32;  // elements of a K-block
   // the padding behind the reduction is written as zeros
@@ -86,17 +90,19 @@ __device__ __forceinline__ void split_tiles(const SplitSource& s, float scale, u
     for (int i = 0; i < 4; ++i) {
       const int r = r0 + 2 * i;
       if (!AGAIN) {
-        uint32_t row = 0;
+        uint32_t row = 0, low = 0xffffffffu;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const uint32_t m = __float_as_uint(x[i][j]) & 0x7fffffffu;
           row = max(row, m);
+          low = lower(low, m);
           col[j] = max(col[j], m);
         }
+        all.faint += low < faint;
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) row = max(row, __shfl_xor_sync(0xffffffffu, row, o));
-        most = max(most, row);
-        if (row) least = min(least, row);
+        all.most = max(all.most, row);
+        if (row) all.least = min(all.least, row);
       }
       if (r < rows && c < width) {
         uint4 part[4];
@@ -121,7 +127,7 @@ __device__ __forceinline__ void split_tiles(const SplitSource& s, float scale, u
       uint32_t m = 0;
 #pragma unroll
       for (int i = 0; i < 16; ++i) m = max(m, cols[turn][i][threadIdx.x]);
-      if (m) least = min(least, m);
+      if (m) all.least = min(all.least, m);
     }
   }
 }
@@ -129,12 +135,12 @@ __device__ __forceinline__ void split_tiles(const SplitSource& s, float scale, u
 template <bool AGAIN>
 __global__ void __launch_bounds__(256) split_kernel(const SplitArgs a) {
   RT_PDL_ENTRY();
-  __shared__ uint32_t red[2][8];
+  __shared__ uint32_t red[3][8];
   __shared__ uint32_t cols[AGAIN ? 1 : 2][16][kTileCols];
   Decision d{};
   for (int q = 0; q < a.sources; ++q) {
-    d.exponent[q] = exponent_for(extremes_of(a.samples + q * a.sample_blocks, a.sample_blocks, red).x);
-    if (AGAIN && out_of_range(extremes_of(a.stats + q * gridDim.x, gridDim.x, red), d.exponent[q])) d.wide = 1;
+    d.exponent[q] = exponent_for(over_blocks(a.samples + q * a.sample_blocks, a.sample_blocks, red).most);
+    if (AGAIN && out_of_range(over_blocks(a.stats + q * gridDim.x, gridDim.x, red), d.exponent[q], a.most_faint[q])) d.wide = 1;
   }
   if (AGAIN) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.decision = d;
@@ -143,12 +149,13 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitArgs a) {
   for (int q = 0; q < a.count; ++q) {
     const SplitSource& s = a.s[q];
     const float scale = AGAIN ? 1.f : ldexpf(1.f, d.exponent[s.source]);
-    uint32_t most = 0, least = 0xffffffffu;
-    if (s.vec) split_tiles<true, AGAIN>(s, scale, cols, most, least);
-    else split_tiles<false, AGAIN>(s, scale, cols, most, least);
+    const uint32_t faint = faint_below(d.exponent[s.source]);
+    Magnitudes all;
+    if (s.vec) split_tiles<true, AGAIN>(s, scale, faint, cols, all);
+    else split_tiles<false, AGAIN>(s, scale, faint, cols, all);
     if (AGAIN || !s.look) continue;
-    const uint2 v = block_extremes(most, least, red);
-    if (threadIdx.x == 0) a.stats[s.source * gridDim.x + blockIdx.x] = v;
+    all = over_block(all, red);
+    if (threadIdx.x == 0) a.stats[s.source * gridDim.x + blockIdx.x] = all;
   }
 }
 
@@ -177,11 +184,11 @@ struct Split {
 // Splits matrices, the first `sources` of which are all different; decision: device memory of one Decision.
 inline rt_status split_all(rt_ctx* ctx, Split* const* s, int count, int sources, RtScratch* work, Decision** decision) {
   const int sample_blocks = ctx->sm_count, blocks = 4 * ctx->sm_count;
-  rt_status st = work->alloc(sizeof(uint2) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
+  rt_status st = work->alloc(sizeof(Magnitudes) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
   if (st != RT_OK) return st;
   SampleArgs a{};
   SplitArgs b{};
-  uint2* samples = work->as<uint2>();
+  Magnitudes* samples = work->as<Magnitudes>();
   a.count = b.sources = sources;
   b.count = count;
   b.sample_blocks = sample_blocks;
@@ -191,7 +198,10 @@ inline rt_status split_all(rt_ctx* ctx, Split* const* s, int count, int sources,
   for (int q = 0; q < count; ++q) {
     if ((st = s[q]->alloc()) != RT_OK) return st;
     const Sample m = sample_of(ctx, s[q]->p, s[q]->ld, s[q]->rows, s[q]->cols, false);
-    if (q < sources) a.s[q] = m;
+    if (q < sources) {
+      a.s[q] = m;
+      b.most_faint[q] = most_faint((int64_t)s[q]->rows * s[q]->cols);
+    }
     b.s[q] = {s[q]->p, s[q]->mem.as<uint16_t>(), s[q]->ld, s[q]->ldo, s[q]->rows, s[q]->cols, m.tiles_c, m.tiles, s[q]->along_rows, m.vec, s[q]->source,
               q < sources};
   }

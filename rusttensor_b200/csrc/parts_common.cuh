@@ -28,6 +28,11 @@ constexpr int kMaxSources = 3;
 constexpr int kTileRows = 64, kTileCols = 128;
 constexpr int kSampleExponent = 9;                         // where the sample's largest magnitude is scaled to
 constexpr int kLargestExponent = 14, kSmallestExponent = -9;  // of any element, of a segment's largest
+// Elements that are not zero and stay below 2^-22 after scaling are faint: they keep fewer than 14 bits, which shows where the other operand is large.
+// Two parts will do while there are next to none.  Of 2^24 numbers from a normal distribution 0.03 are, of the gate gradients of a recurrent network
+// 4; of magnitudes spread evenly over 2^31 none, over 2^33 one in 20.
+constexpr int kFaintExponent = -22;
+inline uint32_t most_faint(int64_t elements) { return 4 + (uint32_t)(elements >> 20); }
 
 struct Decision {
   int wide;                   // three bf16 parts
@@ -35,7 +40,10 @@ struct Decision {
 };
 
 // ---- magnitudes: the largest, and the smallest of the non-zero segments' largest, as the bits of floats (which order as they do; NaN
-// above infinity) ----------------------------------------------------------------------------------------------------------------
+// above infinity), and in how many pieces (of eight or sixteen elements) there is a faint one ------------------------------------------
+struct alignas(16) Magnitudes {
+  uint32_t most = 0, least = 0xffffffffu, faint = 0, unused = 0;
+};
 struct Sample {
   const float* p;
   int64_t ld;
@@ -51,45 +59,55 @@ inline Sample sample_of(const rt_ctx* ctx, const float* p, int64_t ld, int64_t r
   return {p, ld, (int)rows, (int)cols, (int)tiles_c, rt_aligned16(p) && ld % 4 == 0 && cols % 4 == 0, (uint32_t)tiles,
           all ? 1u : (uint32_t)((tiles + ctx->sm_count - 1) / ctx->sm_count)};
 }
-// The block's largest and smallest, in all its threads.  red: 2 x 8 words; 256 threads.
-__device__ __forceinline__ uint2 block_extremes(uint32_t most, uint32_t least, uint32_t (*red)[8]) {
+// The block's, in all its threads.  red: 3 x 8 words; 256 threads.
+__device__ __forceinline__ Magnitudes over_block(Magnitudes m, uint32_t (*red)[8]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  most = __reduce_max_sync(0xffffffffu, most);
-  least = __reduce_min_sync(0xffffffffu, least);
+  m.most = __reduce_max_sync(0xffffffffu, m.most);
+  m.least = __reduce_min_sync(0xffffffffu, m.least);
+  m.faint = __reduce_add_sync(0xffffffffu, m.faint);
   __syncthreads();
   if (lane == 0) {
-    red[0][warp] = most;
-    red[1][warp] = least;
+    red[0][warp] = m.most;
+    red[1][warp] = m.least;
+    red[2][warp] = m.faint;
   }
   __syncthreads();
-  return make_uint2(__reduce_max_sync(0xffffffffu, red[0][lane & 7]), __reduce_min_sync(0xffffffffu, red[1][lane & 7]));
+  m.most = __reduce_max_sync(0xffffffffu, red[0][lane & 7]);
+  m.least = __reduce_min_sync(0xffffffffu, red[1][lane & 7]);
+  m.faint = __reduce_add_sync(0xffffffffu, lane < 8 ? red[2][lane] : 0u);
+  return m;
 }
-__device__ __forceinline__ uint2 extremes_of(const uint2* stats, int n, uint32_t (*red)[8]) {
-  uint32_t most = 0, least = 0xffffffffu;
+__device__ __forceinline__ Magnitudes over_blocks(const Magnitudes* stats, int n, uint32_t (*red)[8]) {
+  Magnitudes m;
   for (int i = threadIdx.x; i < n; i += 256) {
-    const uint2 v = __ldg(stats + i);
-    most = max(most, v.x);
-    least = min(least, v.y);
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(stats + i));
+    m.most = max(m.most, v.x);
+    m.least = min(m.least, v.y);
+    m.faint += v.z;
   }
-  return block_extremes(most, least, red);
+  return over_block(m, red);
 }
 // The exponent that a sample asks for; more than 100 either way is refused by out_of_range.
 __device__ __forceinline__ int exponent_for(uint32_t most) { return most == 0 || most >= 0x7f800000u ? 0 : kSampleExponent + 127 - (int)(most >> 23); }
-__device__ __forceinline__ bool out_of_range(uint2 v, int exponent) {
-  if (v.x == 0) return false;
-  return v.x >= 0x7f800000u || exponent > 100 || exponent < -100 || (int)(v.x >> 23) - 127 + exponent > kLargestExponent ||
-         (int)(v.y >> 23) - 127 + exponent < kSmallestExponent;
+// An element of magnitude m (its bits) is faint if m - 1 is below this: zero is not.
+__device__ __forceinline__ uint32_t faint_below(int exponent) { return max(__float_as_uint(ldexpf(1.f, kFaintExponent - exponent)), 1u) - 1u; }
+// The least of m - 1 over a piece, an element more.
+__device__ __forceinline__ uint32_t lower(uint32_t least, uint32_t m) { return __viaddmin_u32(m, 0xffffffffu, least); }
+__device__ __forceinline__ bool out_of_range(const Magnitudes& v, int exponent, uint32_t most_faint) {
+  if (v.most == 0) return false;
+  return v.most >= 0x7f800000u || exponent > 100 || exponent < -100 || (int)(v.most >> 23) - 127 + exponent > kLargestExponent ||
+         (int)(v.least >> 23) - 127 + exponent < kSmallestExponent || v.faint > most_faint;
 }
 // A warp has eight rows of a tile of 64 x 128, eight 128-bit loads in flight.
-static __global__ void __launch_bounds__(256) sample_kernel(const SampleArgs a, uint2* __restrict__ out) {
+static __global__ void __launch_bounds__(256) sample_kernel(const SampleArgs a, Magnitudes* __restrict__ out) {
   RT_PDL_ENTRY();
   __shared__ uint32_t cols[2][8][kTileCols];
-  __shared__ uint32_t red[2][8];
+  __shared__ uint32_t red[3][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int turn = 0;
   for (int q = 0; q < a.count; ++q) {
     const Sample& s = a.s[q];
-    uint32_t most = 0, least = 0xffffffffu;
+    Magnitudes all;
     for (uint32_t k = blockIdx.x; k * s.step < s.tiles; k += gridDim.x) {
       // not always the same place of `step` tiles: rows of them may repeat
       const uint32_t t = min(k * s.step + (s.step > 1 ? (k * 40503u >> 8) % s.step : 0), s.tiles - 1);
@@ -119,8 +137,8 @@ static __global__ void __launch_bounds__(256) sample_kernel(const SampleArgs a, 
           col[j] = max(col[j], m);
         }
         row = __reduce_max_sync(0xffffffffu, row);
-        most = max(most, row);
-        if (row) least = min(least, row);
+        all.most = max(all.most, row);
+        if (row) all.least = min(all.least, row);
       }
       turn ^= 1;  // two buffers, so that one barrier a tile is enough
 #pragma unroll
@@ -130,11 +148,11 @@ static __global__ void __launch_bounds__(256) sample_kernel(const SampleArgs a, 
         uint32_t m = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) m = max(m, cols[turn][i][threadIdx.x]);
-        if (m) least = min(least, m);
+        if (m) all.least = min(all.least, m);
       }
     }
-    const uint2 v = block_extremes(most, least, red);
-    if (threadIdx.x == 0) out[q * gridDim.x + blockIdx.x] = v;
+    all = over_block(all, red);
+    if (threadIdx.x == 0) out[q * gridDim.x + blockIdx.x] = all;
     __syncthreads();
   }
 }

@@ -78,3 +78,29 @@ def test_convolution_of_parts(api, n, cin, h, w, cout, k, s, p, transposed, spre
     if spread and not transposed:  # the small channel's weight gradient has its own scale
         small, ref_ = dw.numpy()[:, cin // 2], want[1][:, cin // 2]
         assert np.abs(small - ref_).max() <= 4e-6 * np.abs(ref_).max() + 1e-6 * np.abs(ref_).max()
+
+
+@pytest.mark.parametrize("octaves", [28, 31, 40])
+def test_convolution_of_parts_of_wide_ranges(api, octaves):
+    """Magnitudes spread over so many powers of two in every channel and filter, and results whose terms all weigh the same: what the small elements
+    keep shows."""
+    n, cin, h, w, cout = 65, 70, 28, 32, 128  # no short segments at the ends, which would be told from their largest element
+    r = np.random.default_rng(octaves)
+
+    def spread(*shape):
+        return (np.exp2(r.uniform(-octaves / 2, octaves / 2, shape)) * r.choice([-1, 1], shape)).astype(np.float32)
+
+    x, g, wt = spread(n, cin, h, w), spread(n, cout, h, w), spread(cout, cin, 3, 3)
+    g[:, 2] = 1 / np.abs(x[:, 1])                                   # the weight gradient of channels 1 -> 2, middle tap
+    wt[:, 3] = 1 / np.abs(g[4, :, 9:12, 11:14])[:, ::-1, ::-1]      # the input gradient of image 4, channel 3, pixel (10, 12)
+    wt[0] = 1 / np.abs(x[3, :, 9:12, 11:14])                        # the output of image 3, channel 0, pixel (10, 12)
+    y, dx, dw, db = api.empty(g.shape), api.empty(x.shape), api.empty(wt.shape), api.empty((cout,))
+    dev = [api.to_device(v) for v in (x, wt, np.zeros(cout, np.float32), g)]
+    dims = (i64(n), i64(cin), i64(h), i64(w), i64(cout), 3, 3, 1, 1, 1, 1)
+    api.call("conv2d", dev[0].ptr, dev[1].ptr, dev[2].ptr, *dims, y.ptr)
+    api.call("conv2d_backward", dev[0].ptr, dev[1].ptr, dev[3].ptr, *dims, dx.ptr, dw.ptr, db.ptr)
+    for got, a, b in ((y.numpy()[3, 0, 10, 12], x[3, :, 9:12, 11:14], wt[0]), (dx.numpy()[4, 3, 10, 12], g[4, :, 9:12, 11:14], wt[:, 3, ::-1, ::-1]),
+                      (dw.numpy()[2, 1, 1, 1], g[:, 2], x[:, 1])):
+        terms = a.astype(np.float64) * b
+        # 32 additions with truncation between two roundings, the parts' own 2^-22
+        assert abs(got - terms.sum()) <= (32 * 2.0**-23 + 2.0**-21) * np.abs(terms).sum()

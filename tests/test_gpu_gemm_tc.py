@@ -69,6 +69,7 @@ def test_tensor_core_gemm_is_deterministic(capi):
 
 
 # ---- operands split into 16-bit parts (k_gemm_parts.cu): work of 2^27 and more, more than one wave of 128 x 64 tiles -------------
+# Only the fourth has no short segments at its ends, by which the largest element of a segment tells that the range is wide.
 PARTS = [(1300, 1000, 129), (1281, 1089, 257), (2049, 640, 1055), (1024, 1216, 2080), (1409, 901, 300)]
 # Error relative to |A| |B|: at most 32 additions to an accumulator between two roundings, each truncated (2^-23), the parts' own 2^-22 and
 # the sums over the chunks.
@@ -80,7 +81,7 @@ def parts_error(got, A, B):
     return float(np.max(np.abs(got - A @ B) / (np.abs(A) @ np.abs(B))))
 
 
-@pytest.mark.parametrize("inputs", ["normal", "one row far below the rest", "scales that cancel along the reduction", "tiny times huge"])
+@pytest.mark.parametrize("inputs", ["normal", "one row far below the rest", "scales that cancel along the reduction", "tiny times huge", 28, 31, 35, 40, 50])
 @pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
 @pytest.mark.parametrize("m,n,k", PARTS, ids=str)
 def test_product_of_parts(capi, m, n, k, ta, tb, inputs):
@@ -93,6 +94,9 @@ def test_product_of_parts(capi, m, n, k, ta, tb, inputs):
         A, B = A * s, B / s[:, None]
     elif inputs == "tiny times huge":
         A, B = A * np.float32(1e-25), B * np.float32(3e20)
+    elif inputs != "normal":  # magnitudes spread over so many powers of two, in every row and column, and columns that give each the same weight
+        A = (np.exp2(r.uniform(-inputs / 2, inputs / 2, (m, k))) * r.choice([-1, 1], (m, k))).astype(np.float32)
+        B = np.ascontiguousarray((1 / np.abs(A[np.arange(n) % m])).T)
     before = capi.launches()
     got = gemm(capi, ta, tb, m, n, k, np.ascontiguousarray(A.T) if ta else A, np.ascontiguousarray(B.T) if tb else B)
     assert capi.launches() - before <= 4  # a sample, two parts, perhaps three, the product
