@@ -3,8 +3,8 @@
 // Timestep by timestep the recurrence is a product of [batch, H] x [H, 4H] and a few element operations, each a kernel that is over before
 // it has started: 8 + 4 us of a timestep at batch 64, H 512, of which the arithmetic is two.  Here the kernel stays: every block keeps its
 // slice of the recurrent weights in shared memory for the whole sequence, and what the blocks tell one another per timestep is written to
-// and polled in memory, the value and what tells its timestep in the same 4 or 8 bytes, so that seeing the one is having the other: no
-// barrier.
+// and polled in memory, the value and what tells its timestep in one element of 4 or 8 bytes, so that seeing the one is having the other: no
+// barrier.  (A vector access is one access per element, in no order: value and number must not be two of them.)
 //
 // A block has 16 rows of the batch and U hidden units (all four gates of them).  Rows are independent of one another, so only the blocks
 // of the same rows exchange anything.  Forward a block publishes h of its units and gathers everybody's (4 bytes a value): the 16 warps
@@ -47,13 +47,34 @@ struct SeqArgs {
   float *dgates, *dh0, *dc0;
 };
 
+// Forward mail: four values, each with its turn.
 __device__ __forceinline__ uint4 peek(const uint4* p) {
   uint4 v;
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+// Backward mail: two elements of {value, number of the timestep}.  (848 us for 128 timesteps at batch 64, H 512; as four elements of 32 bits, which
+// would say nothing about their order, 840.)
+__device__ __forceinline__ uint4 peek2(const uint4* p) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .b64 a, b;\n\t"
+      "ld.relaxed.gpu.global.v2.b64 {a, b}, [%4];\n\t"
+      "mov.b64 {%0, %1}, a;\n\t"
+      "mov.b64 {%2, %3}, b;\n\t}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p)
+      : "memory");
+  return v;
+}
 __device__ __forceinline__ void post2(uint4* p, float v, float w, uint32_t tag) {
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %3, %2, %3};" ::"l"(p), "r"(__float_as_uint(v)), "r"(__float_as_uint(w)), "r"(tag) : "memory");
+  asm volatile(
+      "{\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "st.relaxed.gpu.global.v2.b64 [%0], {a, b};\n\t}" ::"l"(p),
+      "r"(__float_as_uint(v)), "r"(__float_as_uint(w)), "r"(tag)
+      : "memory");
 }
 // Two multiply-adds in one instruction: what the accumulators hold apart are the sums over the even and over the odd reduction indices.
 struct Pair {
@@ -85,12 +106,12 @@ __device__ __forceinline__ uint32_t output_of(uint32_t v) {
 
 // Waits until the wanted ones of N pieces of mail, STRIDE apart, have arrived.  False: the wait ran out, here or in another block.  (Polling
 // one piece until it is there and only then the others is a round trip more: 693 -> 714 us for 128 timesteps at batch 64, H 512.)
-template <int STRIDE, int N, class Arrived>
-__device__ __forceinline__ bool receive(const uint4* from, bool (&want)[N], uint4 (&v)[N], const SeqArgs& a, const Arrived& arrived) {
+template <int STRIDE, int N, class Peek, class Arrived>
+__device__ __forceinline__ bool receive(const uint4* from, bool (&want)[N], uint4 (&v)[N], const SeqArgs& a, const Peek& look, const Arrived& arrived) {
   for (uint32_t i = 0; i < kPolls; ++i) {
 #pragma unroll
     for (int j = 0; j < N; ++j)
-      if (want[j]) v[j] = peek(from + j * STRIDE);
+      if (want[j]) v[j] = look(from + j * STRIDE);
     bool there = true;
 #pragma unroll
     for (int j = 0; j < N; ++j) {
@@ -158,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const SeqArg
           const uint32_t bit = turn_bit(t - 1);
           const uint4* from = a.mail + ((int64_t)((t - 1) & 1) * gridDim.x + first_block + q) * kRows * quads + lane;
           if (ok)
-            ok = receive<32>(from, want, v, a, [bit](const uint4& m) { return (((m.x ^ bit) | (m.y ^ bit) | (m.z ^ bit) | (m.w ^ bit)) & kTurnBit) == 0; });
+            ok = receive<32>(from, want, v, a, peek, [bit](const uint4& m) { return (((m.x ^ bit) | (m.y ^ bit) | (m.z ^ bit) | (m.w ^ bit)) & kTurnBit) == 0; });
 #pragma unroll
           for (int j = 0; j < 2 * NL; ++j) v[j] = make_uint4(output_of(v[j].x), output_of(v[j].y), output_of(v[j].z), output_of(v[j].w));
         } else {
@@ -280,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_backward_kernel(con
         for (int j = 0; j < N; ++j) want[j] = s0 + j * at_once + lane / pairs < S;
         const uint4* from = box((step - 1) & 1, group, s0 + lane / pairs) + warp * pairs + lane % pairs;
         const uint32_t tag = (uint32_t)step;
-        if (ok) ok = receive<at_once * kRows * pairs>(from, want, v, a, [tag](const uint4& m) { return m.y == tag && m.w == tag; });
+        if (ok) ok = receive<at_once * kRows * pairs>(from, want, v, a, peek2, [tag](const uint4& m) { return m.y == tag && m.w == tag; });
 #pragma unroll
         for (int j = 0; j < N; ++j) {  // zeros where there is no source
           x += __uint_as_float(v[j].x);

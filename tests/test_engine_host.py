@@ -35,3 +35,17 @@ def test_kernel_attributes_are_set_on_every_device(tmp_path):
         if name.endswith((".cu", ".cuh")):
             with open(os.path.join(csrc, name)) as f:
                 assert not re.search(r"static\s+(const\s+)?(cudaError_t|auto|int|bool)\s+\w+\s*=[^;]*cuda(FuncSetAttribute|Occupancy)", f.read()), name
+
+
+def test_a_piece_of_mail_is_one_element_of_its_access():
+    """A vector access is one access per element, in no order.  Where blocks tell one another values beside a number that says which timestep they
+    are of (the backward recurrence), both are halves of one 64-bit element; forward the number is a bit of the 32-bit value."""
+    with open(os.path.join(os.path.dirname(HERE), "rusttensor_b200", "csrc", "k_lstm_seq.cu")) as f:
+        source = f.read()
+    forward, backward = source.split("lstm_sequence_backward_kernel(const SeqArgs a) {", 1)
+    accesses = [(re.findall(r"__forceinline__ \S+ (\w+)\(", source[: m.start()])[-1], m.group()) for m in re.finditer(r"(ld|st)\.relaxed\.[\w.]+", source)]
+    assert sorted(accesses) == [("peek", "ld.relaxed.gpu.global.v4.u32"), ("peek2", "ld.relaxed.gpu.global.v2.b64"),
+                                ("post2", "st.relaxed.gpu.global.v2.b64"), ("post_output", "st.relaxed.gpu.global.u32")]
+    forward = forward[forward.index("lstm_sequence_kernel(const SeqArgs a) {"):]
+    assert re.findall(r"a, (peek2?), \[", forward) == ["peek"] and "post2" not in forward
+    assert re.findall(r"a, (peek2?), \[", backward) == ["peek2"] and "post_output" not in backward
