@@ -181,63 +181,74 @@ struct Split {
 };
 
 
-// Splits matrices, the first `sources` of which are all different; decision: device memory of one Decision.
-inline rt_status split_all(rt_ctx* ctx, Split* const* s, int count, int sources, RtScratch* work, Decision** decision) {
-  const int sample_blocks = ctx->sm_count, blocks = 4 * ctx->sm_count;
-  rt_status st = work->alloc(sizeof(Magnitudes) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
-  if (st != RT_OK) return st;
-  SampleArgs a{};
-  SplitArgs b{};
-  Magnitudes* samples = work->as<Magnitudes>();
-  a.count = b.sources = sources;
-  b.count = count;
-  b.sample_blocks = sample_blocks;
-  b.samples = samples;
-  b.stats = samples + (size_t)sample_blocks * kMaxSources;
-  *decision = b.decision = reinterpret_cast<Decision*>(b.stats + (size_t)blocks * kMaxSources);
-  for (int q = 0; q < count; ++q) {
-    if ((st = s[q]->alloc()) != RT_OK) return st;
-    const Sample m = sample_of(ctx, s[q]->p, s[q]->ld, s[q]->rows, s[q]->cols, false);
-    if (q < sources) {
-      a.s[q] = m;
-      b.most_faint[q] = most_faint((int64_t)s[q]->rows * s[q]->cols);
+// The passes that split matrices, the first `sources` of which are all different.  Preparing takes the memory and makes the tensor maps, so that
+// what can be missing is missing before anything has been launched: a caller that takes another kernel then may be adding to what is there.
+struct Splitting {
+  SampleArgs sample{};
+  SplitArgs split{};
+  RtScratch work;
+  explicit Splitting(rt_ctx* ctx) : work(ctx) {}
+  rt_status prepare(rt_ctx* ctx, Split* const* s, int count, int sources) {
+    const int sample_blocks = ctx->sm_count, blocks = 4 * ctx->sm_count;
+    rt_status st = work.alloc(sizeof(Magnitudes) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
+    if (st != RT_OK) return st;
+    Magnitudes* samples = work.as<Magnitudes>();
+    sample.count = split.sources = sources;
+    split.count = count;
+    split.sample_blocks = sample_blocks;
+    split.samples = samples;
+    split.stats = samples + (size_t)sample_blocks * kMaxSources;
+    split.decision = reinterpret_cast<Decision*>(split.stats + (size_t)blocks * kMaxSources);
+    for (int q = 0; q < count; ++q) {
+      if ((st = s[q]->alloc()) != RT_OK) return st;
+      const Sample m = sample_of(ctx, s[q]->p, s[q]->ld, s[q]->rows, s[q]->cols, false);
+      if (q < sources) {
+        sample.s[q] = m;
+        split.most_faint[q] = most_faint((int64_t)s[q]->rows * s[q]->cols);
+      }
+      split.s[q] = {s[q]->p, s[q]->mem.as<uint16_t>(), s[q]->ld, s[q]->ldo, s[q]->rows, s[q]->cols, m.tiles_c, m.tiles, s[q]->along_rows, m.vec,
+                    s[q]->source, q < sources};
     }
-    b.s[q] = {s[q]->p, s[q]->mem.as<uint16_t>(), s[q]->ld, s[q]->ldo, s[q]->rows, s[q]->cols, m.tiles_c, m.tiles, s[q]->along_rows, m.vec, s[q]->source,
-              q < sources};
+    return RT_OK;
   }
-  rt_launch(ctx, sample_kernel, sample_blocks, 256, 0, a, samples);
-  RT_LAUNCHED(ctx);
-  rt_launch(ctx, split_kernel<false>, blocks, 256, 0, b);
-  RT_LAUNCHED(ctx);
-  rt_launch(ctx, split_kernel<true>, blocks, 256, 0, b);
-  RT_LAUNCHED(ctx);
-  return RT_OK;
-}
+  rt_status run(rt_ctx* ctx) {
+    rt_launch(ctx, sample_kernel, split.sample_blocks, 256, 0, sample, work.as<Magnitudes>());
+    RT_LAUNCHED(ctx);
+    rt_launch(ctx, split_kernel<false>, 4 * ctx->sm_count, 256, 0, split);
+    RT_LAUNCHED(ctx);
+    rt_launch(ctx, split_kernel<true>, 4 * ctx->sm_count, 256, 0, split);
+    RT_LAUNCHED(ctx);
+    return RT_OK;
+  }
+};
 
 // C = act(op(A) op(B) + bias) (+ C) of two split matrices.
-inline rt_status product(rt_ctx* ctx, Split& a, bool trans_a, Split& b, bool trans_b, const Decision* decision, float* c, int64_t ldc, const float* bias,
-                         int act, int accumulate) {
+struct Product {
+  CUtensorMap map_a, map_b;
   Params p{};
-  CUtensorMap ma, mb;
-  if (!a.map(&ma) || !b.map(&mb)) return RT_ERR_UNIMPLEMENTED;
-  p.decision = decision;
-  p.source_a = a.source;
-  p.source_b = b.source;
-  p.a_along_m = a.along_rows;
-  p.b_along_n = b.along_rows;
-  p.M = trans_a ? a.cols : a.rows;
-  p.K = trans_a ? a.rows : a.cols;
-  p.N = trans_b ? b.rows : b.cols;
-  p.chunk = p.K < 1024 ? 6 : (p.K < 2048 ? 8 : 16);
-  p.m_tiles = (p.M + BM - 1) / BM;
-  choose_tiles(ctx, &p);
-  p.c = c;
-  p.ldc = ldc;
-  p.bias = bias;
-  p.act = act;
-  p.accumulate = accumulate;
-  return launch<kMatrices>(ctx, ma, mb, p);
-}
+  rt_status prepare(rt_ctx* ctx, Split& a, bool trans_a, Split& b, bool trans_b, const Decision* decision, float* c, int64_t ldc, const float* bias, int act,
+                    int accumulate) {
+    if (!a.map(&map_a) || !b.map(&map_b)) return RT_ERR_UNIMPLEMENTED;
+    p.decision = decision;
+    p.source_a = a.source;
+    p.source_b = b.source;
+    p.a_along_m = a.along_rows;
+    p.b_along_n = b.along_rows;
+    p.M = trans_a ? a.cols : a.rows;
+    p.K = trans_a ? a.rows : a.cols;
+    p.N = trans_b ? b.rows : b.cols;
+    p.chunk = p.K < 1024 ? 6 : (p.K < 2048 ? 8 : 16);
+    p.m_tiles = (p.M + BM - 1) / BM;
+    choose_tiles(ctx, &p);
+    p.c = c;
+    p.ldc = ldc;
+    p.bias = bias;
+    p.act = act;
+    p.accumulate = accumulate;
+    return RT_OK;
+  }
+  rt_status run(rt_ctx* ctx) { return launch<kMatrices>(ctx, map_a, map_b, p); }
+};
 inline bool extents_fit(int64_t m, int64_t n, int64_t k) { return m < (1 << 24) && n < (1 << 24) && k < (1 << 24); }
 
 }  // namespace parts
@@ -259,27 +270,30 @@ rt_status rt_gemm_parts_internal(rt_ctx* ctx, int trans_a, int trans_b, int64_t 
                                  int64_t ldb, float* c, int64_t ldc, const float* bias, int act, int accumulate) {
   using namespace tc::parts;
   if (!extents_fit(m, n, k)) return RT_ERR_UNIMPLEMENTED;
-  RtScratch work(ctx);
   Split sa(ctx, 0, a, lda, trans_a ? k : m, trans_a ? m : k, trans_a), sb(ctx, 1, b, ldb, trans_b ? n : k, trans_b ? k : n, !trans_b);
   Split* both[2] = {&sa, &sb};
-  Decision* decision;
-  rt_status st = split_all(ctx, both, 2, 2, &work, &decision);
-  if (st == RT_ERR_OOM) return RT_ERR_UNIMPLEMENTED;
-  if (st != RT_OK) return st;
-  return product(ctx, sa, trans_a, sb, trans_b, decision, c, ldc, bias, act, accumulate);
+  Splitting splitting(ctx);
+  Product product;
+  rt_status st = splitting.prepare(ctx, both, 2, 2);
+  if (st == RT_OK) st = product.prepare(ctx, sa, trans_a, sb, trans_b, splitting.split.decision, c, ldc, bias, act, accumulate);
+  if (st != RT_OK) return st == RT_ERR_OOM ? RT_ERR_UNIMPLEMENTED : st;
+  if ((st = splitting.run(ctx)) != RT_OK) return st;
+  return product.run(ctx);
 }
 // da[m,k] = g[m,n] b[k,n]^T and db[k,n] (+)= a[m,k]^T g[m,n], the upstream gradient looked at once for both.
 rt_status rt_matmul_backward_parts_internal(rt_ctx* ctx, const float* a, const float* b, const float* g, int64_t m, int64_t k, int64_t n, float* da,
                                             float* db, int accumulate_db) {
   using namespace tc::parts;
   if (!extents_fit(m, n, k)) return RT_ERR_UNIMPLEMENTED;
-  RtScratch work(ctx);
   Split sa(ctx, 0, a, k, m, k, true), sb(ctx, 1, b, n, k, n, false), g_rows(ctx, 2, g, n, m, n, false), g_cols(ctx, 2, g, n, m, n, true);
   Split* all[4] = {&sa, &sb, &g_rows, &g_cols};
-  Decision* decision;
-  rt_status st = split_all(ctx, all, 4, 3, &work, &decision);
-  if (st == RT_ERR_OOM) return RT_ERR_UNIMPLEMENTED;
-  if (st == RT_OK) st = product(ctx, sa, true, g_cols, false, decision, db, n, nullptr, RT_ACT_NONE, accumulate_db);
-  if (st == RT_OK) st = product(ctx, g_rows, false, sb, true, decision, da, k, nullptr, RT_ACT_NONE, 0);
-  return st;
+  Splitting splitting(ctx);
+  Product of_b, of_a;
+  rt_status st = splitting.prepare(ctx, all, 4, 3);
+  if (st == RT_OK) st = of_b.prepare(ctx, sa, true, g_cols, false, splitting.split.decision, db, n, nullptr, RT_ACT_NONE, accumulate_db);
+  if (st == RT_OK) st = of_a.prepare(ctx, g_rows, false, sb, true, splitting.split.decision, da, k, nullptr, RT_ACT_NONE, 0);
+  if (st != RT_OK) return st == RT_ERR_OOM ? RT_ERR_UNIMPLEMENTED : st;
+  if ((st = splitting.run(ctx)) != RT_OK) return st;
+  if ((st = of_b.run(ctx)) != RT_OK) return st;
+  return of_a.run(ctx);
 }

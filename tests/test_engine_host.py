@@ -37,6 +37,16 @@ def test_kernel_attributes_are_set_on_every_device(tmp_path):
                 assert not re.search(r"static\s+(const\s+)?(cudaError_t|auto|int|bool)\s+\w+\s*=[^;]*cuda(FuncSetAttribute|Occupancy)", f.read()), name
 
 
+def test_both_gradients_of_parts_launch_all_or_nothing(tmp_path):
+    obj, exe = str(tmp_path / "parts.o"), str(tmp_path / "parts_checks")
+    subprocess.run([os.environ.get("NVCC", "nvcc"), "-gencode", "arch=compute_100a,code=compute_100a", "-std=c++17", "-c",
+                    os.path.join(os.path.dirname(HERE), "rusttensor_b200", "csrc", "k_gemm_parts.cu"), "-o", obj], check=True)
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-I/usr/local/cuda/include", "-o", exe,
+                    os.path.join(HERE, "host", "parts_checks.cpp"), obj], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_a_piece_of_mail_is_one_element_of_its_access():
     """A vector access is one access per element, in no order.  Where blocks tell one another values beside a number that says which timestep they
     are of (the backward recurrence), both are halves of one 64-bit element; forward the number is a bit of the 32-bit value."""
