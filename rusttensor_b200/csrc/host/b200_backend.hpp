@@ -187,6 +187,13 @@ struct B200Backend {
     lazy::capturing() = false;
     check(rt_graph_end(ctx(), out));
   }
+  // Goes on in another graph.  What is still deferred belongs to the first: between the two it would be computed once, and no replay would
+  // compute it again.
+  static void split_capture(rt_graph** first) {
+    lazy::flush_all();
+    end_capture(first);
+    begin_capture();
+  }
 
   // ---- factories / access (mod.rs:44-88, 248-252) --------------------------------------
   static Storage filled(const Shape& s, float v) {

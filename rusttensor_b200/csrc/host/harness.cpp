@@ -224,8 +224,7 @@ struct DpTrainer {
       fired = true;
       if (capturing) {  // split the capture here; the exchange of the early slice runs between the two replays
         for (int i = early_lo; i < early_hi; ++i) B200Backend::own(*w.params[i].grad());  // evaluated inside the first part
-        B200Backend::end_capture(&graph);
-        B200Backend::begin_capture();
+        B200Backend::split_capture(&graph);
       } else {
         exchange_early();
       }

@@ -17,7 +17,12 @@ int mallocs_left = -1;         // rt_malloc fails once they are used up; < 0: ne
 bool kernels_fail = false;
 int masked_pool_gradients;     // launches of the pooling gradient that masks by the relu in front
 int forward_sequences, backward_sequences;
-
+bool recording = false;
+int unrecorded;                // kernels while nothing is recorded
+rt_status kernel() {
+  unrecorded += !recording;
+  return kernels_fail ? RT_ERR_CUDA : RT_OK;
+}
 
 void expect(bool ok, const char* what, int line) {
   if (ok) return;
@@ -67,12 +72,12 @@ rt_status rt_memcpy_d2d(rt_ctx*, void* d, const void* s, size_t n) {
   return RT_OK;
 }
 rt_status rt_unary(rt_ctx*, int op, const float* x, float* y, int64_t n, float, float) {
-  if (kernels_fail) return RT_ERR_CUDA;
+  if (kernel() != RT_OK) return RT_ERR_CUDA;
   for (int64_t i = 0; i < n && op == RT_SQUARE; ++i) y[i] = x[i] * x[i];
   return RT_OK;
 }
 rt_status rt_binary(rt_ctx*, int, const float*, const int64_t*, int, const float*, const int64_t*, int, float*) {
-  return kernels_fail ? RT_ERR_CUDA : RT_OK;
+  return kernel();
 }
 rt_status rt_relu_max_pool2d(rt_ctx*, const float*, int64_t, int64_t, int64_t, int64_t, int, int, int, int, int, int, float*, float*) {
   return RT_OK;
@@ -85,24 +90,24 @@ rt_status rt_relu_max_pool2x2_backward_from_output(rt_ctx*, const float*, const 
   return RT_OK;
 }
 rt_status rt_column_sums_list(rt_ctx*, int count, const float* const* xs, const int64_t* rows, const int64_t* cols, float* const* outs) {
-  if (kernels_fail) return RT_ERR_CUDA;
+  if (kernel() != RT_OK) return RT_ERR_CUDA;
   for (int k = 0; k < count; ++k)
     for (int64_t i = 0; i < rows[k] * cols[k]; ++i) outs[k][i % cols[k]] = (i < cols[k] ? 0.f : outs[k][i % cols[k]]) + xs[k][i];
   return RT_OK;
 }
 rt_status rt_sum_rows_accumulate_list(rt_ctx*, int count, const float* const* xs, int64_t rows, int64_t cols, float* out) {
-  if (kernels_fail) return RT_ERR_CUDA;
+  if (kernel() != RT_OK) return RT_ERR_CUDA;
   for (int k = 0; k < count; ++k)
     for (int64_t i = 0; i < rows * cols; ++i) out[i % cols] += xs[k][i];
   return RT_OK;
 }
 rt_status rt_gemm_bias_act_list(rt_ctx*, int, const float* const*, float* const*, int64_t, int64_t, int64_t, const float*, const float*, int) {
-  return kernels_fail ? RT_ERR_CUDA : RT_OK;
+  return kernel();
 }
 rt_status rt_fused_column_sums(rt_ctx*, const rt_fused_program*, int, float*) { return RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of windows; results of other programs stay zero
-  if (kernels_fail) return RT_ERR_CUDA;
+  if (kernel() != RT_OK) return RT_ERR_CUDA;
   if (p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_OK;
   const int rows = p->nd == 2 ? p->shape[0] : 1, cols = p->shape[p->nd - 1];
   const rt_fused_operand& o = p->operand[0];
@@ -111,30 +116,30 @@ rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies 
   return RT_OK;
 }
 // their results stay zero
-rt_status rt_graph_begin(rt_ctx*) { return RT_OK; }
-rt_status rt_graph_end(rt_ctx*, rt_graph**) { return RT_OK; }
-rt_status rt_fill(rt_ctx*, float*, float, int64_t) { return RT_OK; }
-rt_status rt_gemm(rt_ctx*, int, int, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, float*, int64_t, int) { return RT_OK; }
-rt_status rt_gemm_bias_act(rt_ctx*, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, const float*, int, float*, int64_t) { return RT_OK; }
+rt_status rt_graph_begin(rt_ctx*) { return recording = true, RT_OK; }
+rt_status rt_graph_end(rt_ctx*, rt_graph**) { return recording = false, RT_OK; }
+rt_status rt_fill(rt_ctx*, float*, float, int64_t) { return kernel(); }
+rt_status rt_gemm(rt_ctx*, int, int, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, float*, int64_t, int) { return kernel(); }
+rt_status rt_gemm_bias_act(rt_ctx*, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, const float*, int, float*, int64_t) { return kernel(); }
 rt_status rt_softmax_nll_list(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, float, float, int, const float* const*, float*) {
-  return RT_OK;
+  return kernel();
 }
-rt_status rt_softmax_nll_with_grad(rt_ctx*, const float*, const float*, int64_t, int64_t, float, float, const float*, float, float*, float*) { return RT_OK; }
-rt_status rt_softmax_nll_scaled_backward(rt_ctx*, const float*, const float*, int64_t, int64_t, float, float*) { return RT_OK; }
-rt_status rt_matmul_backward(rt_ctx*, const float*, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) { return RT_OK; }
-rt_status rt_gemm_sum_products(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, int64_t, float*) { return RT_OK; }
-rt_status rt_reduce(rt_ctx*, int, const float*, int64_t, int64_t, int64_t, float*) { return RT_OK; }
-rt_status rt_unbroadcast(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return RT_OK; }
-rt_status rt_broadcast_to(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return RT_OK; }
-rt_status rt_slice_assign(rt_ctx*, float*, const int64_t*, int, const int64_t*, const float*, const int64_t*) { return RT_OK; }
+rt_status rt_softmax_nll_with_grad(rt_ctx*, const float*, const float*, int64_t, int64_t, float, float, const float*, float, float*, float*) { return kernel(); }
+rt_status rt_softmax_nll_scaled_backward(rt_ctx*, const float*, const float*, int64_t, int64_t, float, float*) { return kernel(); }
+rt_status rt_matmul_backward(rt_ctx*, const float*, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) { return kernel(); }
+rt_status rt_gemm_sum_products(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, int64_t, float*) { return kernel(); }
+rt_status rt_reduce(rt_ctx*, int, const float*, int64_t, int64_t, int64_t, float*) { return kernel(); }
+rt_status rt_unbroadcast(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return kernel(); }
+rt_status rt_broadcast_to(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return kernel(); }
+rt_status rt_slice_assign(rt_ctx*, float*, const int64_t*, int, const int64_t*, const float*, const int64_t*) { return kernel(); }
 rt_status rt_lstm_sequence(rt_ctx*, const float*, const float*, int64_t, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) {
   ++forward_sequences;
-  return RT_OK;
+  return kernel();
 }
 rt_status rt_lstm_sequence_backward(rt_ctx*, const float*, const float*, int64_t, const float*, const float*, int64_t, int64_t, int64_t, float*, float*,
                                     float*) {
   ++backward_sequences;
-  return RT_OK;
+  return kernel();
 }
 }
 
@@ -482,10 +487,48 @@ void long_recurrences() {
   }
 }
 
+// A capture that goes on in another graph in the middle of the backward pass (an exchange of the gradients that are ready runs between the two):
+// everything is in one of the graphs.
+void a_capture_in_two_parts() {
+  using Tn = Tensor<B>;
+  const size_t T = 4, Bn = 2, V = 3, H = 2;
+  {
+    const Tn x(make({T * Bn, V}, 0.f, .01f), false), w(make({V + H, 4 * H}, 0.f, .01f), true), b(make({4 * H}, 0.f, .01f), true);
+    const Tn wo(make({H, V}, 0.f, .1f), true), bo(make({V}, 0.f, .1f), true);
+    rt_graph *first = nullptr, *second = nullptr;
+    int ready = 0;
+    B::begin_capture();
+    unrecorded = 0;
+    {
+      Tn h = Tn::zeros({Bn, H}, false), c = Tn::zeros({Bn, H}, false), sum;
+      for (size_t t = 0; t < T; ++t) {
+        const Tn z = ops::add(ops::matmul(ops::concat<B>({ops::slice(x, {{t * Bn, (t + 1) * Bn}, {0, V}}), h}, 1), w), b.broadcast_to({Bn, 4 * H}));
+        auto gate = [&](size_t k) { return ops::slice(z, {{0, Bn}, {k * H, (k + 1) * H}}); };
+        c = ops::add(ops::mul(ops::sigmoid(gate(1)), c), ops::mul(ops::sigmoid(gate(0)), ops::tanh(gate(2))));
+        h = ops::mul(ops::sigmoid(gate(3)), ops::tanh(c));
+        const Tn l = ops::sum(ops::square(ops::add(ops::matmul(h, wo), bo.broadcast_to({Bn, V}))), std::nullopt);
+        sum = t ? ops::add(sum, l) : l;
+      }
+      Tn::leaf_ready_hook() = [&](const Tn& leaf) {
+        if (ready++ > 0) return;
+        B::own(*leaf.grad());
+        B::split_capture(&first);
+      };
+      sum.backward();
+      Tn::leaf_ready_hook() = nullptr;
+      for (auto& g : {sum.data(), *w.grad(), *b.grad(), *wo.grad(), *bo.grad()}) B::own(g);
+      sum.detach_graph();
+    }
+    B::end_capture(&second);
+    EXPECT(ready == 4 && unrecorded == 0);
+  }
+  EXPECT(live.empty());
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences},
+} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"a_capture_in_two_parts", a_capture_in_two_parts},
                {"kept_results_stay_where_they_are_written", kept_results_stay_where_they_are_written},
                {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},
