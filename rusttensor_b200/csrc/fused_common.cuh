@@ -82,6 +82,7 @@ struct KnownProgram {
 };
 // Checks a program and brings it into the kernels' form; vec: groups of four consecutive elements may be read and written as vectors.
 rt_status prepare(rt_ctx* ctx, const rt_fused_program* f, FusedParams* p, bool* vec, int64_t* numel);  // k_fused.cu
+uint2 encode(const rt_fused_instr& in);                  // k_fused.cu
 const KnownProgram* known_programs(int* n);            // k_fused_known.cu
 const KnownProgram* known_recurrent_programs(int* n);  // k_fused_lstm.cu
 

@@ -1365,20 +1365,22 @@ inline bool column_sum_waits(DeviceBuffer* b) {
       return true;
   return false;
 }
-// A program and its outputs' blocks, launched by `run`; false: not a form that it has.
-template <class Run>
-inline bool evaluate_reduced(DeviceBuffer* b, Compiler& c, Run run) {
+// A program with a reduction of one of its outputs: column sums of output c.sums(), or with `lse` the logsumexp of the rows.  False: not a form that
+// there is a kernel for, and no memory has been taken for it.
+inline bool evaluate_reduced(DeviceBuffer* b, Compiler& c, float* lse) {
   rt_fused_program p;
   std::vector<DeviceBuffer*> outs;
   if (!c.build(b, &p, &outs)) return !b->node;  // evaluated on the way
+  if ((c.sums() < 0) != (lse != nullptr)) return false;
+  const rt_status known = rt_fused_reduction_known(b->ctx, &p, c.sums());
+  if (known == RT_ERR_UNIMPLEMENTED) return false;
+  check(b->ctx, known);
   std::vector<Block> blocks;
   for (size_t k = 0; k < outs.size(); ++k) {
     blocks.emplace_back(b->ctx, outs[k]->numel);
     p.out[k] = blocks.back().ptr;
   }
-  const rt_status st = run(p);
-  if (st == RT_ERR_UNIMPLEMENTED) return false;
-  check(b->ctx, st);
+  check(b->ctx, lse ? rt_fused_logsumexp(b->ctx, &p, lse) : rt_fused_column_sums(b->ctx, &p, c.sums(), p.out[c.sums()]));
   std::vector<std::shared_ptr<DeviceBuffer>> keep;
   for (auto* o : outs) keep.push_back(o->shared_from_this());
   for (size_t k = 0; k < outs.size(); ++k) blocks[k].to(outs[k]);
@@ -1389,9 +1391,7 @@ inline bool evaluate_with_sums(DeviceBuffer* b) {
   if (Walk::depth() > 1 || b->node->shape.size() != 2 || b->numel == 0 || !column_sum_waits(b)) return false;
   Compiler c;
   c.keep_rows();
-  return evaluate_reduced(b, c, [&](rt_fused_program& p) {
-    return c.sums() < 0 ? RT_ERR_UNIMPLEMENTED : rt_fused_column_sums(b->ctx, &p, c.sums(), p.out[c.sums()]);
-  });
+  return evaluate_reduced(b, c, nullptr);
 }
 // The rows of an expression and their logsumexp.
 inline bool evaluate_with_logsumexp(DeviceBuffer* b, float* out) {
@@ -1399,7 +1399,7 @@ inline bool evaluate_with_logsumexp(DeviceBuffer* b, float* out) {
   std::shared_ptr<DeviceBuffer> guard = b->shared_from_this();
   Compiler c;
   c.keep_rows();
-  return evaluate_reduced(b, c, [&](rt_fused_program& p) { return c.sums() >= 0 ? RT_ERR_UNIMPLEMENTED : rt_fused_logsumexp(b->ctx, &p, out); });
+  return evaluate_reduced(b, c, out);
 }
 
 }  // namespace lazy

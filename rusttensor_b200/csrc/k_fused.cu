@@ -205,28 +205,6 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) fused_kernel(const __grid_con
   }
 }
 
-// The instruction as the kernel decodes it: reversed operands become ops of their own.
-uint2 encode(const rt_fused_instr& in) {
-  int op = in.op;
-  if (in.swap && op != RT_F_SELECT) switch (op) {
-      case RT_F_SUB: op = kReverseSub; break;
-      case RT_F_DIV: op = kReverseDiv; break;
-      case RT_F_POWF: op = kReversePow; break;
-      case RT_F_GT: op = RT_F_LT; break;
-      case RT_F_GE: op = RT_F_LE; break;
-      case RT_F_LT: op = RT_F_GT; break;
-      case RT_F_LE: op = RT_F_GE; break;
-      default: break;
-    }
-  const bool unary = op >= RT_F_RELU && op <= RT_F_ELU_SLOPE;
-  const uint32_t src = unary ? 0u : in.src, region = in.op == RT_F_SELECT ? in.swap : 0u;
-  uint2 w;
-  w.x = (uint32_t)op | src << 8 | (uint32_t)in.dst << 16 | region << 24;
-  static_assert(sizeof(in.imm) == 4, "");
-  memcpy(&w.y, &in.imm, 4);
-  return w;
-}
-
 template <int V, bool VEC, int THREADS, int BLOCKS>
 rt_status launch_fused(rt_ctx* ctx, FusedParams& p, int64_t numel) {
   const int64_t per_block = (int64_t)V * THREADS, tiles = (numel + per_block - 1) / per_block;
@@ -274,6 +252,28 @@ bool regions_in_quads(const FusedParams& p) {
 }
 
 }  // namespace
+
+// The instruction as the kernel decodes it: reversed operands become ops of their own.
+uint2 fused::encode(const rt_fused_instr& in) {
+  int op = in.op;
+  if (in.swap && op != RT_F_SELECT) switch (op) {
+      case RT_F_SUB: op = kReverseSub; break;
+      case RT_F_DIV: op = kReverseDiv; break;
+      case RT_F_POWF: op = kReversePow; break;
+      case RT_F_GT: op = RT_F_LT; break;
+      case RT_F_GE: op = RT_F_LE; break;
+      case RT_F_LT: op = RT_F_GT; break;
+      case RT_F_LE: op = RT_F_GE; break;
+      default: break;
+    }
+  const bool unary = op >= RT_F_RELU && op <= RT_F_ELU_SLOPE;
+  const uint32_t src = unary ? 0u : in.src, region = in.op == RT_F_SELECT ? in.swap : 0u;
+  uint2 w;
+  w.x = (uint32_t)op | src << 8 | (uint32_t)in.dst << 16 | region << 24;
+  static_assert(sizeof(in.imm) == 4, "");
+  memcpy(&w.y, &in.imm, 4);
+  return w;
+}
 
 rt_status fused::prepare(rt_ctx* ctx, const rt_fused_program* f, FusedParams* out, bool* in_vectors, int64_t* count) {
   RT_CHECK_CTX(ctx);

@@ -157,19 +157,34 @@ constexpr Reduced with_logsumexp{P::code, P::n, P::preload, &logsumexp_kernel<P,
 
 #include "fused_programs_reduced.inc"
 
-template <int N>
-const Reduced* find(const Reduced (&list)[N], const FusedParams& p) {
+// word(i): the i-th instruction as the kernels decode it.
+template <int N, class Word>
+const Reduced* find(const Reduced (&list)[N], int n_code, int n_preload, const Word& word) {
   for (const Reduced& k : list) {
-    bool same = k.n_code == p.n_code && k.n_preload == p.n_preload;
-    for (int i = 0; i < p.n_code && same; ++i) same = k.code[i] == p.code[i].x;
+    bool same = k.n_code == n_code && k.n_preload == n_preload;
+    for (int i = 0; i < n_code && same; ++i) same = k.code[i] == word(i);
     if (same) return &k;
   }
   return nullptr;
+}
+template <int N>
+const Reduced* find(const Reduced (&list)[N], const FusedParams& p) {
+  return find(list, p.n_code, p.n_preload, [&](int i) { return p.code[i].x; });
 }
 
 }  // namespace
 
 extern "C" {
+
+rt_status rt_fused_reduction_known(rt_ctx* ctx, const rt_fused_program* f, int which) {
+  RT_CHECK_CTX(ctx);
+  RT_CHECK_PTR(ctx, f);
+  if (f->nd != 2 || f->n_code < 1 || f->n_code > RT_FUSED_MAX_CODE || which < -1 || which >= f->n_outputs)
+    RT_FAIL(ctx, RT_ERR_INVALID_OPERATION, "rt_fused_reduction_known: an output of a two-dimensional program, or -1");
+  if (f->shape[0] <= 0 || f->shape[1] <= 0 || (which < 0 && f->shape[1] > kLongestRow)) return RT_ERR_UNIMPLEMENTED;
+  auto word = [&](int i) { return fused::encode(f->code[i]).x; };
+  return (which < 0 ? find(kWithLogsumexp, f->n_code, f->n_preload, word) : find(kWithSums, f->n_code, f->n_preload, word)) ? RT_OK : RT_ERR_UNIMPLEMENTED;
+}
 
 rt_status rt_fused_column_sums(rt_ctx* ctx, const rt_fused_program* f, int which, float* sums) {
   ReducedParams q{};

@@ -14,6 +14,7 @@ namespace {
 std::map<void*, size_t> live;  // blocks that are allocated
 int failures;                  // of the checks
 int mallocs_left = -1;         // rt_malloc fails once they are used up; < 0: never
+int mallocs;
 bool kernels_fail = false;
 int masked_pool_gradients;     // launches of the pooling gradient that masks by the relu in front
 int forward_sequences, backward_sequences;
@@ -53,6 +54,7 @@ const char* rt_last_error(rt_ctx*) { return "stub"; }
 rt_status rt_malloc(rt_ctx*, size_t bytes, void** out) {
   if (mallocs_left == 0) return RT_ERR_OOM;
   if (mallocs_left > 0) --mallocs_left;
+  ++mallocs;
   *out = std::calloc(1, bytes);
   live[*out] = bytes;
   return RT_OK;
@@ -104,6 +106,7 @@ rt_status rt_sum_rows_accumulate_list(rt_ctx*, int count, const float* const* xs
 rt_status rt_gemm_bias_act_list(rt_ctx*, int, const float* const*, float* const*, int64_t, int64_t, int64_t, const float*, const float*, int) {
   return kernel();
 }
+rt_status rt_fused_reduction_known(rt_ctx*, const rt_fused_program*, int) { return RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_column_sums(rt_ctx*, const rt_fused_program*, int, float*) { return RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of windows; results of other programs stay zero
@@ -525,10 +528,27 @@ void a_capture_in_two_parts() {
   EXPECT(live.empty());
 }
 
+// A program that no kernel with a reduction has been compiled for takes no memory before it is refused.
+void refused_programs_take_no_memory() {
+  {
+    const B::Storage x = make({4, 8}, 0.f), b = make({8}, 0.f);
+    const B::Storage y = B::add(B::tanh(B::mul(x, b)), x);
+    mallocs = 0;
+    const B::Storage lse = B::logsumexp(y, 1);
+    EXPECT(!y.buf->node && mallocs == 2);
+    const B::Storage u = B::mul(x, b), v = B::exp(u), sums = B::unbroadcast(B::mul(B::tanh(u), x), {8});
+    mallocs = 0;
+    v.ptr();
+    EXPECT(!v.buf->node && mallocs <= 2);  // v, and u beside it, which somebody holds
+    sums.ptr();
+  }
+  EXPECT(live.empty());
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"a_capture_in_two_parts", a_capture_in_two_parts},
+} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"refused_programs_take_no_memory", refused_programs_take_no_memory}, {"a_capture_in_two_parts", a_capture_in_two_parts},
                {"kept_results_stay_where_they_are_written", kept_results_stay_where_they_are_written},
                {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},
