@@ -116,8 +116,7 @@ void* rt_stream(rt_ctx* ctx);                                                   
 rt_status rt_mem_stats(rt_ctx* ctx, int64_t* bytes_reserved, int64_t* bytes_in_use, int64_t* n_device_allocs);
 rt_status rt_kernel_launch_count(rt_ctx* ctx, int64_t* launches);                    /* kernels launched by this library so far */
 /* Elementwise programs run so far, by what ran them: a kernel compiled for them, or the interpreter.  A program is a launch of
- * rt_fused_elementwise, rt_fused_column_sums or rt_fused_logsumexp, or one of the two that a timestep of rt_lstm_sequence or of its backward
- * pass holds. */
+ * rt_fused_elementwise, rt_fused_column_sums or rt_fused_logsumexp. */
 rt_status rt_fused_launch_counts(rt_ctx* ctx, int64_t* compiled, int64_t* interpreted);
 /* Synchronises and reads the device error word: kernels that wait on barriers give up after a bounded
  * number of polls, record a code there and return; non-zero -> RT_ERR_TIMEOUT (and the word is cleared). */

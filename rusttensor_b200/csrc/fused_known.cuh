@@ -5,7 +5,8 @@
 // gradients, a mean squared error, the LSTM cell) consist of are therefore listed in fused_programs_*.inc and compiled: the same
 // instruction words as template arguments, registers and operand numbers become constants, immediates and shapes stay run-time.
 // An unlisted program is interpreted, with the same results: a program is found by its instructions, so a user's expression with one
-// op more or in another form, and the first and last timesteps of the recurrent network, are not (rt_fused_launch_counts tells).
+// op more or in another form is not (rt_fused_launch_counts tells).  Those of the LSTM written op by op serve steps that are not captured (in a
+// capture its timesteps are one sequence, k_lstm_seq.cu); there the first and last timesteps are interpreted.
 //
 // Measured, kernel time inside a graph: the gate gradient of the LSTM cell (30 instructions, 12 operands, 4 windows) on [64, 2048]
 // 12.5 us interpreted, 4.2 us compiled; an elementwise gradient with four transcendentals on [4096, 4096] 300 us interpreted, 77 us

@@ -479,7 +479,6 @@ rt_status rt_lstm_sequence(rt_ctx* ctx, const float* pre, const float* w, int64_
   a.h = h;
   a.status = ctx->device_status;
   set_saved(&a, saved, steps * n);
-  ctx->fused_compiled += 2 * steps;
   const Fit f = fit(ctx, batch, hidden, false);
   if (f.units) {
     a.groups = f.groups;
@@ -523,7 +522,6 @@ rt_status rt_lstm_sequence_backward(rt_ctx* ctx, const float* saved, const float
   a.dc0 = dc0;
   a.status = ctx->device_status;
   set_saved(&a, saved, steps * n);
-  ctx->fused_compiled += 2 * steps;
   const Fit f = fit(ctx, batch, hidden, true);
   if (f.units) {
     a.groups = f.groups;
