@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
       if (q < a.images) v = seen;
       v.faint = seen.faint;
       if (out_of_range(v, d.exponent[q], a.most_faint[q])) d.wide = 1;
+      if (v.most >= 0x7f800000u) d.special = 1;
     }
   }
   if (AGAIN) {
@@ -420,6 +421,37 @@ __global__ void __launch_bounds__(256) parts_grad_finish_kernel(const GradFinish
   }
 }
 
+// The columns of the phases have weights of zero at the taps that are not theirs, which an infinity or NaN makes NaN of: with such in the images or
+// weights an output that came out NaN is computed once more from its own taps.  Otherwise over at once.
+struct Repair {
+  const Decision* decision;
+  const float *y, *w, *bias;
+  float* out;
+  int64_t total;
+  int Cm, Cy, Hy, Wy, Hx, Wx, kh, kw, sh, sw, ph, pw;
+};
+__global__ void __launch_bounds__(256) repair_gather_kernel(const Repair p) {
+  RT_PDL_ENTRY();
+  if (!p.decision->special) return;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < p.total; i += (int64_t)gridDim.x * 256) {
+    if (p.out[i] == p.out[i]) continue;
+    const int u = (int)(i % p.Wx), v = (int)(i / p.Wx % p.Hx), c = (int)(i / p.Wx / p.Hx % p.Cm);
+    const float* y = p.y + i / p.Wx / p.Hx / p.Cm * p.Cy * p.Hy * p.Wy;
+    double sum = p.bias ? __ldg(p.bias + c) : 0.f;
+    for (int ky = 0; ky < p.kh; ++ky) {
+      const int yo = (v + p.ph - ky) / p.sh;
+      if (v + p.ph < ky || (v + p.ph - ky) % p.sh || yo >= p.Hy) continue;
+      for (int kx = 0; kx < p.kw; ++kx) {
+        const int xo = (u + p.pw - kx) / p.sw;
+        if (u + p.pw < kx || (u + p.pw - kx) % p.sw || xo >= p.Wy) continue;
+        for (int k = 0; k < p.Cy; ++k)
+          sum += (double)__ldg(y + ((int64_t)k * p.Hy + yo) * p.Wy + xo) * __ldg(p.w + (((int64_t)k * p.Cm + c) * p.kh + ky) * p.kw + kx);
+      }
+    }
+    p.out[i] = (float)sum;
+  }
+}
+
 // ---- host ---------------------------------------------------------------------------------------------------------------------
 // An image [Nb][C][H][W] and its parts.
 struct Image {
@@ -613,8 +645,13 @@ struct Gather {
     rows_w = (g.Wx + 1) / 2;
     return true;
   }
-  rt_status run(rt_ctx* ctx, Image& y, int source_w, const Decision* decision, const ConvGeom& g, const float* bias, float* out) {
-    return pixel_product(ctx, y, taps, source_w, decision, rows_h, rows_w, 1, 1, py, px, bias, out, g.Hx, g.Wx);
+  rt_status run(rt_ctx* ctx, Image& y, int source_w, const Decision* decision, const ConvGeom& g, int cm, const float* bias, float* out) {
+    rt_status st = pixel_product(ctx, y, taps, source_w, decision, rows_h, rows_w, 1, 1, py, px, bias, out, g.Hx, g.Wx);
+    if (st != RT_OK || !taps.t.phases) return st;
+    const Repair r{decision, y.p, taps.all, bias, out, (int64_t)g.Nb * cm * g.Hx * g.Wx, cm, g.Cy, g.Hy, g.Wy, g.Hx, g.Wx, g.kh, g.kw, g.sh, g.sw, g.ph, g.pw};
+    rt_launch(ctx, repair_gather_kernel, 4 * ctx->sm_count, 256, 0, r);
+    RT_LAUNCHED(ctx);
+    return RT_OK;
   }
 };
 inline bool gather_worth_it(const ConvGeom& g, int cm) {
@@ -689,7 +726,7 @@ rt_status rt_conv_gather_parts_internal(rt_ctx* ctx, const float* y, const float
   RtScratch work(ctx);
   Decision* decision;
   rt_status st = split_conv(ctx, images, 1, &gather.taps, &work, &decision);
-  if (st == RT_OK) st = gather.run(ctx, src, 1, decision, g, bias, out);
+  if (st == RT_OK) st = gather.run(ctx, src, 1, decision, g, cm, bias, out);
   return or_another_kernel(st);
 }
 // dw[Cy,Cx,kh,kw] = sum over images and pixels of y * (x at the tap); db[Cy] = sum of y.
@@ -715,7 +752,7 @@ rt_status rt_conv_backward_parts_internal(rt_ctx* ctx, const float* x, const flo
   Decision* decision;
   rt_status st = split_conv(ctx, images, 2, &gather.taps, &work, &decision);
   if (st == RT_OK) st = weight_grad(ctx, ix, iy, decision, g, dw, db, iy);
-  if (st == RT_OK) st = gather.run(ctx, iy, 2, decision, g, nullptr, dx);
+  if (st == RT_OK) st = gather.run(ctx, iy, 2, decision, g, g.Cx, nullptr, dx);
   return or_another_kernel(st);
 }
 // The same of a transposed convolution: y is its input, x (the wide side) the upstream gradient, whose channel sums db is.

@@ -36,6 +36,7 @@ inline uint32_t most_faint(int64_t elements) { return 4 + (uint32_t)(elements >>
 
 struct Decision {
   int wide;                   // three bf16 parts
+  int special;                // convolutions: there are infinities or NaN
   int exponent[kMaxSources];  // an element is split after multiplication with 2^exponent
 };
 

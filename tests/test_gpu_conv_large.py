@@ -104,3 +104,43 @@ def test_convolution_of_parts_of_wide_ranges(api, octaves):
         terms = a.astype(np.float64) * b
         # 32 additions with truncation between two roundings, the parts' own 2^-22
         assert abs(got - terms.sum()) <= (32 * 2.0**-23 + 2.0**-21) * np.abs(terms).sum()
+
+
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("n,cin,h,w,cout,k,s,p", [(65, 70, 29, 31, 66, 3, 1, 1), (96, 33, 37, 35, 97, 4, 2, 1), (70, 66, 33, 30, 68, 5, 2, 2)])
+def test_infinities_and_nan_stay_where_they_belong(api, n, cin, h, w, cout, k, s, p, transposed):
+    """An infinity or NaN in the input (the upstream gradient) shows in the outputs that it is a term of, and in no others."""
+    r = np.random.default_rng(n)
+    name, fwd, bwd = (("conv2d_transpose", ref_f64.conv2d_transpose, ref_f64.conv2d_transpose_backward) if transposed
+                      else ("conv2d", ref_f64.conv2d, ref_f64.conv2d_backward))
+    x = r.standard_normal((n, cin, h, w)).astype(np.float32)
+    wt = (r.standard_normal((cin, cout, k, k) if transposed else (cout, cin, k, k)) / k).astype(np.float32)
+    b, some = r.standard_normal(cout).astype(np.float32), [1, n - 1]
+    clean = fwd(x[some], wt, b, (s, s), (p, p))
+    y, dx = api.empty((n,) + clean.shape[1:]), api.empty(x.shape)
+    g = r.standard_normal(y.shape).astype(np.float32)
+
+    def spoil(a):
+        a[some[0], 3, a.shape[2] // 2, 4], a[some[0], 5, 2, a.shape[3] - 2], a[some[1], 0, 0, 0] = np.inf, np.nan, -np.inf
+        return a
+
+    # which elements a spoiled one is a term of: those that change with it
+    def touched(f, a):
+        zero = np.zeros_like(a[some])
+        return f(np.where(np.isfinite(a[some]), zero, 1.0)) != 0
+
+    def run():
+        dev = [api.to_device(v) for v in (x, wt, b, g)]
+        dims = (i64(n), i64(cin), i64(h), i64(w), i64(cout), k, k, s, s, p, p)
+        api.call(name, dev[0].ptr, dev[1].ptr, dev[2].ptr, *dims, y.ptr)
+        api.call(name + "_backward", dev[0].ptr, dev[1].ptr, dev[3].ptr, *dims, dx.ptr, None, None)
+        return y.numpy()[some], dx.numpy()[some]
+
+    before = run()
+    spoil(x), spoil(g)
+    after = run()
+    positive = np.abs(wt)
+    for was, now, hit in ((before[0], after[0], touched(lambda v: fwd(v, positive, None, (s, s), (p, p)), x)),
+                          (before[1], after[1], touched(lambda v: bwd(np.ones_like(x[some]), positive, v, (s, s), (p, p))[0], g))):
+        assert not np.isfinite(now[hit]).any()
+        assert np.isfinite(now[~hit]).all() and np.abs(now - was)[~hit].max() <= 1e-5 * np.abs(was).max()
