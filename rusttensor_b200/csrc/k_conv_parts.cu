@@ -366,6 +366,8 @@ parts_grad_kernel(const __grid_constant__ CUtensorMap map_y, const __grid_consta
 
 // dw[cy][cx][tap] = sum over the splits and the pairs of parts; db[c] = sum over the tiles of the upstream gradient's image.
 // A warp has a column's 32 rows of a channel block at a time: coalesced reads.  Fixed order.
+// Where a box overhangs the image y there are zeros, which x is multiplied with all the same: an infinity among it makes NaN.  With infinities or
+// NaN in the images an element that came out NaN is therefore computed once more from the images themselves.
 struct GradFinish {
   const Decision* decision;
   const float* partial;
@@ -374,37 +376,61 @@ struct GradFinish {
   const float* sums;
   float* db;
   int sum_tiles, sum_C;
+  const float *x, *y;
+  int Nb, Hx, Wx, Hy, Wy, kw, sx, sy, px, py;
 };
-__global__ void __launch_bounds__(256) parts_grad_finish_kernel(const GradFinish p) {
+__device__ __noinline__ float grad_from_images(const GradFinish& p, int cy, int cx, int tap) {
+  const int lane = threadIdx.x & 31, ky = tap / p.kw, kx = tap % p.kw, pixels = p.Nb * p.Hy * p.Wy;
+  double sum = 0;
+  for (int i = lane; i < pixels; i += 32) {
+    const int xo = i % p.Wy, yo = i / p.Wy % p.Hy, n = i / p.Wy / p.Hy, v = yo * p.sy - p.py + ky, u = xo * p.sx - p.px + kx;
+    const bool in = v >= 0 && v < p.Hx && u >= 0 && u < p.Wx;
+    sum += (double)__ldg(p.y + (((int64_t)n * p.Cy + cy) * p.Hy + yo) * p.Wy + xo) * (in ? __ldg(p.x + (((int64_t)n * p.Cx + cx) * p.Hx + v) * p.Wx + u) : 0.f);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  return (float)sum;
+}
+__global__ void __launch_bounds__(256) parts_grad_finish_kernel(const __grid_constant__ GradFinish p) {
   RT_PDL_ENTRY();
-  const int wide = p.decision->wide, depth = wide ? 16 : 32;
+  const int wide = p.decision->wide, special = p.decision->special, depth = wide ? 16 : 32;
   const GradTiles g = grad_tiles(p.Cy, p.Cx, p.taps, wide);
-  const int tiles = g.m_tiles * g.n_tiles;
+  const int tiles = g.m_tiles * g.n_tiles, lane = threadIdx.x & 31;
   const int exponent = wide ? 0 : -(p.decision->exponent[p.source_y] + p.decision->exponent[p.source_x]);
   const float f1 = ldexpf(1.f, exponent / 2), f2 = ldexpf(1.f, exponent - exponent / 2);
   const int64_t cy_padded = (int64_t)g.c_rows * depth;
   const int64_t total = cy_padded * p.Cx * p.taps;
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
+  for (int64_t first = (int64_t)blockIdx.x * 256 + (threadIdx.x & ~31u); first < total; first += (int64_t)gridDim.x * 256) {
+    const int64_t i = first + lane;
     const int cy = (int)(i % cy_padded), rest = (int)(i / cy_padded), cx = rest % p.Cx, tap = rest / p.Cx;
-    if (cy >= p.Cy) continue;
-    const int rb = cy / depth, column_block = tap * g.c_cols + cx / depth;
-    const int tile = rb / 2 + column_block / 4 * g.m_tiles;
-    const int row = rb % 2 * 64 + cy % depth, col = column_block % 4 * 64 + cx % depth;
-    const float* q = p.partial + ((int64_t)tile * 256 + col) * BM + row;
-    auto at = [&](const float* t, int part_y, int part_x) { return __ldcs(t + (int64_t)part_x * depth * BM + part_y * depth); };
-    float main = 0.f, cross = 0.f;
+    float v = 0.f;
+    if (i < total && cy < p.Cy) {
+      const int rb = cy / depth, column_block = tap * g.c_cols + cx / depth;
+      const int tile = rb / 2 + column_block / 4 * g.m_tiles;
+      const int row = rb % 2 * 64 + cy % depth, col = column_block % 4 * 64 + cx % depth;
+      const float* q = p.partial + ((int64_t)tile * 256 + col) * BM + row;
+      auto at = [&](const float* t, int part_y, int part_x) { return __ldcs(t + (int64_t)part_x * depth * BM + part_y * depth); };
+      float main = 0.f, cross = 0.f;
 #pragma unroll 4
-    for (int s = 0; s < p.splits; ++s) {
-      const float* t = q + (int64_t)s * tiles * 256 * BM;
-      main += at(t, 0, 0);
-      if (wide) cross += (at(t, 3, 1) + at(t, 1, 3)) + (at(t, 1, 1) + (at(t, 3, 2) + at(t, 2, 3)));
-      else cross += (at(t, 0, 1) + at(t, 1, 0)) + at(t, 1, 1) * (1.f / 2048.f);
+      for (int s = 0; s < p.splits; ++s) {
+        const float* t = q + (int64_t)s * tiles * 256 * BM;
+        main += at(t, 0, 0);
+        if (wide) cross += (at(t, 3, 1) + at(t, 1, 3)) + (at(t, 1, 1) + (at(t, 3, 2) + at(t, 2, 3)));
+        else cross += (at(t, 0, 1) + at(t, 1, 0)) + at(t, 1, 1) * (1.f / 2048.f);
+      }
+      v = (main + cross * (wide ? 1.f : 1.f / 2048.f)) * f1 * f2;
     }
-    p.dw[((int64_t)cy * p.Cx + cx) * p.taps + tap] = (main + cross * (wide ? 1.f : 1.f / 2048.f)) * f1 * f2;
+    if (special)
+      for (unsigned bad = __ballot_sync(0xffffffffu, v != v); bad; bad &= bad - 1) {
+        const int of = __ffs((int)bad) - 1;
+        const float again = grad_from_images(p, __shfl_sync(0xffffffffu, cy, of), __shfl_sync(0xffffffffu, cx, of), __shfl_sync(0xffffffffu, tap, of));
+        if (lane == of) v = again;
+      }
+    if (i < total && cy < p.Cy) p.dw[((int64_t)cy * p.Cx + cx) * p.taps + tap] = v;
   }
   if (!p.db) return;
   __shared__ float red[8];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
   for (int c = blockIdx.x; c < p.sum_C; c += gridDim.x) {
     float v = 0.f;
 #pragma unroll 4
@@ -689,7 +715,7 @@ inline rt_status weight_grad(rt_ctx* ctx, Image& x, Image& y, const Decision* de
   rt_launch(ctx, parts_grad_kernel, ctx->sm_count, kThreads, kGradSmem, my, mx, p, ctx->device_status);
   RT_LAUNCHED(ctx);
   GradFinish f{decision, p.partial, dw, p.Cy, p.Cx, p.taps, p.splits, y.source, x.source, static_cast<const float*>(of.sum_mem.ptr), db, of.Nb * of.tiles(),
-               of.C};
+               of.C, x.p, y.p, g.Nb, g.Hx, g.Wx, g.Hy, g.Wy, g.kw, g.sw, g.sh, g.pw, g.ph};
   rt_launch(ctx, parts_grad_finish_kernel, rt_grid_for(ctx, (int64_t)t.c_rows * 32 * p.Cx * p.taps, 256), 256, 0, f);
   RT_LAUNCHED(ctx);
   return RT_OK;

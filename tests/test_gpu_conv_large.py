@@ -144,3 +144,31 @@ def test_infinities_and_nan_stay_where_they_belong(api, n, cin, h, w, cout, k, s
                           (before[1], after[1], touched(lambda v: bwd(np.ones_like(x[some]), positive, v, (s, s), (p, p))[0], g))):
         assert not np.isfinite(now[hit]).any()
         assert np.isfinite(now[~hit]).all() and np.abs(now - was)[~hit].max() <= 1e-5 * np.abs(was).max()
+
+
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("n,cin,h,w,cout,k,s,p", [(130, 40, 40, 38, 84, 3, 1, 1), (96, 33, 37, 35, 97, 4, 2, 1), (70, 66, 33, 30, 68, 5, 2, 2)])
+def test_infinities_and_nan_in_weight_gradients(api, n, cin, h, w, cout, k, s, p, transposed):
+    """Of the wide side (the input, the upstream gradient of a transposed convolution), whose elements meet the padding of the other side's boxes."""
+    r = np.random.default_rng(n)
+    name, bwd = ("conv2d_transpose", ref_f64.conv2d_transpose_backward) if transposed else ("conv2d", ref_f64.conv2d_backward)
+    x = r.standard_normal((n, cin, h, w)).astype(np.float32)
+    wt = (r.standard_normal((cin, cout, k, k) if transposed else (cout, cin, k, k)) / k).astype(np.float32)
+    side = (lambda v: (v - 1) * s + k - 2 * p) if transposed else (lambda v: (v + 2 * p - k) // s + 1)
+    g = r.standard_normal((n, cout, side(h), side(w))).astype(np.float32)
+    some, wide = [1, n - 1], g if transposed else x
+
+    def run():
+        dev = [api.to_device(v) for v in (x, wt, g)]
+        dx, dw, db = api.empty(x.shape), api.empty(wt.shape), api.empty((cout,))
+        api.call(name + "_backward", *[d.ptr for d in dev], i64(n), i64(cin), i64(h), i64(w), i64(cout), k, k, s, s, p, p, dx.ptr, dw.ptr, db.ptr)
+        return dw.numpy()
+
+    was = run()
+    wide[1, 3, wide.shape[2] // 2, 4], wide[1, 5, 2, -1], wide[n - 1, 0, -1, 7], wide[n - 1, 7, 0, 0] = np.inf, np.nan, -np.inf, np.inf
+    marks = np.where(np.isfinite(wide[some]), 0.0, 1.0)
+    hit = (bwd(np.ones_like(x[some]), wt, marks, (s, s), (p, p)) if transposed else bwd(marks, wt, np.ones_like(g[some]), (s, s), (p, p)))[1] != 0
+    now = run()
+    assert not np.isfinite(now[hit]).any() and np.isfinite(now[~hit]).all()
+    # 32 additions with truncation between roundings, the parts' own 2^-22, on either side
+    assert np.abs(now - was)[~hit].max() <= 2 * (32 * 2.0**-23 + 2.0**-21) * (np.abs(was).max() + np.sqrt(n * side(h) * side(w)))
