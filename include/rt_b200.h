@@ -324,7 +324,9 @@ rt_status rt_lstm_cell_h_backward(rt_ctx* ctx, const float* gates, const float* 
  * gates_t = pre_t + h_{t-1} w, pre [steps*batch, 4*hidden] (the inputs' product and the bias), w [hidden, 4*hidden] with rows ldw floats
  * apart; h0, c0 [batch, hidden] or NULL for zeros.  h [steps*batch, hidden]; saved: six such planes for the backward pass, sigmoid(i),
  * sigmoid(f), tanh(g), sigmoid(o), c, tanh(c).  Backward: dgates [steps*batch, 4*hidden] = d/d pre from dh [steps*batch, hidden]; dh0, dc0
- * may be NULL. */
+ * may be NULL.  Blocks of these kernels wait for one another's results, looking that often at most before they record a code in the status word
+ * (rt_device_status) and go on without: rt_lstm_sequence_polls sets how often, for calls to come; a negative number: the default, seconds. */
+rt_status rt_lstm_sequence_polls(rt_ctx* ctx, int64_t polls);
 rt_status rt_lstm_sequence(rt_ctx* ctx, const float* pre, const float* w, int64_t ldw, const float* h0, const float* c0, int64_t steps,
                            int64_t batch, int64_t hidden, float* saved, float* h);
 rt_status rt_lstm_sequence_backward(rt_ctx* ctx, const float* saved, const float* w, int64_t ldw, const float* c0, const float* dh, int64_t steps,

@@ -28,7 +28,6 @@ namespace {
 
 constexpr int kRows = 16, kWarps = 16, kThreads = kWarps * 32;
 constexpr int kPitch = 36;  // words between the 16 rows' values of two reduction indices and those of the next two: 16-byte aligned, few bank conflicts
-constexpr uint32_t kPolls = 1u << 21;
 
 struct SeqArgs {
   int steps, batch, hidden, groups;  // groups of U units
@@ -38,6 +37,7 @@ struct SeqArgs {
   uint4* mail;                       // zeroed before the launch
   int* gave_up;                      // zeroed before the launch
   int* status;
+  uint32_t polls;
   // forward: the part of the gates' inputs that does not depend on h; activated gates, cell, its hyperbolic tangent and the output,
   // each [steps * batch][hidden]
   const float *pre, *h0;
@@ -108,7 +108,7 @@ __device__ __forceinline__ uint32_t output_of(uint32_t v) {
 // one piece until it is there and only then the others is a round trip more: 693 -> 714 us for 128 timesteps at batch 64, H 512.)
 template <int STRIDE, int N, class Peek, class Arrived>
 __device__ __forceinline__ bool receive(const uint4* from, bool (&want)[N], uint4 (&v)[N], const SeqArgs& a, const Peek& look, const Arrived& arrived) {
-  for (uint32_t i = 0; i < kPolls; ++i) {
+  for (uint32_t i = 0; i < a.polls; ++i) {
 #pragma unroll
     for (int j = 0; j < N; ++j)
       if (want[j]) v[j] = look(from + j * STRIDE);
@@ -457,6 +457,13 @@ void set_saved(SeqArgs* a, const float* saved, int64_t plane) {
 
 extern "C" {
 
+rt_status rt_lstm_sequence_polls(rt_ctx* ctx, int64_t polls) {
+  RT_CHECK_CTX(ctx);
+  if (polls > UINT32_MAX) RT_FAIL(ctx, RT_ERR_INVALID_INDEX, "rt_lstm_sequence_polls: 2^32 and more");
+  ctx->sequence_polls = polls < 0 ? rt_ctx().sequence_polls : (uint32_t)polls;
+  return RT_OK;
+}
+
 rt_status rt_lstm_sequence(rt_ctx* ctx, const float* pre, const float* w, int64_t ldw, const float* h0, const float* c0, int64_t steps, int64_t batch,
                            int64_t hidden, float* saved, float* h) {
   RT_CHECK_CTX(ctx);
@@ -478,6 +485,7 @@ rt_status rt_lstm_sequence(rt_ctx* ctx, const float* pre, const float* w, int64_
   a.c0 = c0;
   a.h = h;
   a.status = ctx->device_status;
+  a.polls = ctx->sequence_polls;
   set_saved(&a, saved, steps * n);
   const Fit f = fit(ctx, batch, hidden, false);
   if (f.units) {
@@ -521,6 +529,7 @@ rt_status rt_lstm_sequence_backward(rt_ctx* ctx, const float* saved, const float
   a.dh0 = dh0;
   a.dc0 = dc0;
   a.status = ctx->device_status;
+  a.polls = ctx->sequence_polls;
   set_saved(&a, saved, steps * n);
   const Fit f = fit(ctx, batch, hidden, true);
   if (f.units) {

@@ -67,6 +67,7 @@ struct rt_ctx {
   bool use_tma_weight_grad = true;
   // How many clusters of 2 .. 16 CTAs of the medium products' kernel this device holds at a time ([1]: set once that is known).
   int ts_clusters[17] = {};
+  uint32_t sequence_polls = 1u << 21;  // looks at mail that has not arrived (k_lstm_seq.cu)
   // NCCL (loaded at run time on first use)
   void* nccl_comm = nullptr;
   bool nccl_nonblocking = false;  // the communicator was created in NCCL's non-blocking mode: calls may answer "in progress"

@@ -172,3 +172,35 @@ def test_infinities_and_nan_in_weight_gradients(api, n, cin, h, w, cout, k, s, p
     assert not np.isfinite(now[hit]).any() and np.isfinite(now[~hit]).all()
     # 32 additions with truncation between roundings, the parts' own 2^-22, on either side
     assert np.abs(now - was)[~hit].max() <= 2 * (32 * 2.0**-23 + 2.0**-21) * (np.abs(was).max() + np.sqrt(n * side(h) * side(w)))
+
+
+# Kernels, strides and paddings that differ between the dimensions, strides of three and eight, padding of the kernel's size and more (work as above).
+FORMS = [(64, 48, 40, 44, 80, (3, 5), (1, 1), (1, 2)), (64, 64, 40, 48, 96, (5, 3), (1, 2), (2, 1)), (128, 64, 60, 63, 80, (3, 3), (3, 3), (1, 1)),
+         (128, 70, 96, 90, 80, (4, 5), (8, 7), (0, 2)), (104, 48, 28, 28, 80, (3, 3), (1, 1), (4, 5)), (96, 64, 30, 32, 72, (4, 3), (2, 2), (5, 3))]
+
+
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("n,cin,h,w,cout,k,s,p", FORMS)
+def test_forms_of_convolutions_of_parts(api, n, cin, h, w, cout, k, s, p, transposed):
+    r = np.random.default_rng(n + cin + h)
+    if transposed and s[0] > 2:
+        h, w = h // s[0], w // s[1]
+    x = r.standard_normal((n, cin, h, w)).astype(np.float32)
+    wt = (r.standard_normal((cin, cout, *k) if transposed else (cout, cin, *k)) / k[0]).astype(np.float32)
+    b = r.standard_normal(cout).astype(np.float32)
+    some = [0, n - 1]
+    name, fwd, bwd = (("conv2d_transpose", ref_f64.conv2d_transpose, ref_f64.conv2d_transpose_backward) if transposed
+                      else ("conv2d", ref_f64.conv2d, ref_f64.conv2d_backward))
+    ref = fwd(x[some], wt, b, s, p)
+    y, dx, dw, db = api.empty((n,) + ref.shape[1:]), api.empty(x.shape), api.empty(wt.shape), api.empty(b.shape)
+    g = np.zeros(y.shape, np.float32)
+    g[some] = r.standard_normal((2,) + y.shape[1:]).astype(np.float32)
+    dev = [api.to_device(v) for v in (x, wt, b, g)]
+    dims = (i64(n), i64(cin), i64(h), i64(w), i64(cout), *k, *s, *p)
+    api.call(name, dev[0].ptr, dev[1].ptr, dev[2].ptr, *dims, y.ptr)
+    api.call(name + "_backward", dev[0].ptr, dev[1].ptr, dev[3].ptr, *dims, dx.ptr, dw.ptr, db.ptr)
+    want = bwd(x[some], wt, g[some], s, p)
+    taps = k[0] * k[1]
+    for got, ref_, terms in ((y.numpy()[some], ref, cin * taps), (dx.numpy()[some], want[0], cout * taps), (dw.numpy(), want[1], 2 * y.shape[2] * y.shape[3]),
+                             (db.numpy(), want[2], 2 * y.shape[2] * y.shape[3])):
+        assert np.abs(got - ref_).max() <= (32 * 2.0**-23 + 2.0**-21) * (np.abs(ref_).max() + np.sqrt(terms))

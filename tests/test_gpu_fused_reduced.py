@@ -3,6 +3,8 @@ through the front end: rows and columns at the edges of the kernels' tiles, of v
 import numpy as np
 import pytest
 
+import oracle
+
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1), (3, 4), (5, 31), (33, 57), (16, 128), (17, 129), (64, 1000), (130, 1025), (1100, 1000), (1025, 1027), (3, 8192), (3, 8193), (2, 8200)]
@@ -51,3 +53,32 @@ def test_the_chain_over_other_axes(gpu_engine, shape, axis):
     dx = np.exp(Y - L) * ((1 - t * t) / 2 + np.cos(X) / q - 2 * X * np.exp(-X * X) - 2 * X * np.sin(X) / q**2)
     np.testing.assert_allclose(lse.numpy().reshape(-1), L.reshape(-1), rtol=2e-6, atol=2e-6)
     assert np.abs(x.grad.numpy() - dx).max() <= 4e-6 * max(1.0, np.abs(dx).max())
+
+
+def special_rows(rows, cols):
+    x = np.random.default_rng(rows + cols).standard_normal((rows, cols)).astype(np.float32)
+    x[1], x[2, 3], x[3, 1], x[4, 0], x[5] = -np.inf, -np.inf, np.inf, np.nan, np.inf
+    x[6, 0], x[6, 1], x[7, 2], x[7, 3] = np.inf, -np.inf, np.inf, np.nan
+    return x
+
+
+@pytest.mark.parametrize("rows,cols", [(8, 9), (20, 128), (9, 1030)])
+@pytest.mark.parametrize("chain", ["alone", "scaled", "workload"])
+def test_rows_of_infinities_and_nan(gpu_engine, rows, cols, chain):
+    """Row by row what the reference gives, also through the gradient, which is elementwise in the forward result: an infinity of either sign that is the
+    largest of its row, one that is not, NaN, and rows beside them."""
+    xv, out = special_rows(rows, cols), []
+    for e in (gpu_engine, oracle.engine()):
+        o = e.ops
+        x, b = e.tensor(xv, requires_grad=True), e.tensor(np.full(cols, 0.5, np.float32), requires_grad=True)
+        if chain == "workload":  # the program that logsumexp_kernel carries; the sine of an infinity is NaN
+            sq = o.square(x)
+            y = o.add(o.add(o.tanh(o.mul(x, b)), o.exp(o.mul_scalar(sq, -1.0))), o.div(o.sin(x), o.add(sq, e.tensor(np.float32(1).reshape(())))))
+        else:
+            y = o.mul_scalar(x, 0.5) if chain == "scaled" else x
+        lse = o.logsumexp(y, 1)
+        o.sum(lse).backward()
+        out.append([lse.numpy(), x.grad.numpy()])
+    for got, want in zip(*out):
+        # exp and its sum to a few units in the last place of values of order one
+        np.testing.assert_allclose(got, want, rtol=1e-5, atol=2e-6)

@@ -89,6 +89,41 @@ def test_nan_travels_like_a_value(capi):
     assert np.array_equal(got[0][:, :17], got[1][:, :17]) and np.array_equal(got[0][0], got[1][0])
 
 
+@pytest.mark.parametrize("backward", [False, True])
+@pytest.mark.parametrize("batch,hidden", [(20, 40), (64, 512)])
+def test_a_wait_that_runs_out_is_reported(batch, hidden, backward):
+    """Blocks that do not wait for one another at all: the kernel ends, the next synchronising call says so, and the calls after it are right."""
+    api, steps, r = rusttensor_b200.CApi(), 4, rng(batch)
+    pre, dh = (r.standard_normal((steps * batch, c * hidden)).astype(np.float32) for c in (4, 1))
+    w, zero = (r.uniform(-1, 1, (hidden, 4 * hidden)) / np.sqrt(hidden)).astype(np.float32), np.zeros((batch, hidden), np.float32)
+    d = [api.to_device(v) for v in (pre, w, dh)]
+    h, saved, dgates = (api.empty(s) for s in ((steps * batch, hidden), (6, steps * batch, hidden), (steps * batch, 4 * hidden)))
+    sizes = (i64(steps), i64(batch), i64(hidden))
+
+    def forward():
+        api.call("lstm_sequence", d[0].ptr, d[1].ptr, i64(4 * hidden), None, None, *sizes, saved.ptr, h.ptr)
+
+    def gradient():
+        api.call("lstm_sequence_backward", saved.ptr, d[1].ptr, i64(4 * hidden), None, d[2].ptr, *sizes, dgates.ptr, None, None)
+
+    forward()
+    api.call("lstm_sequence_polls", i64(0))
+    gradient() if backward else forward()
+    code = C.c_int(0)
+    with pytest.raises(Exception, match="gave up"):
+        api.call("device_status", C.byref(code))
+    assert code.value == 81
+    api.call("device_status", C.byref(code))
+    assert code.value == 0
+    api.call("lstm_sequence_polls", i64(-1))
+    forward()
+    gradient()
+    want = reference(pre, w, zero, zero, dh, steps, batch, hidden)
+    for a, b in zip((h.numpy(), dgates.numpy()), want):
+        assert np.max(np.abs(a - b)) <= 2.0**-24 * (20 + 2 * np.sqrt(hidden)) * steps * max(1.0, np.abs(b).max())
+    api.close()
+
+
 def test_sizes_are_checked(capi):
     x = capi.empty((4, 16))
     for sizes in ((0, 2, 4), (1, 0, 4), (1, 2, 0)):
