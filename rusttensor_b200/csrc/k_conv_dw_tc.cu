@@ -25,11 +25,10 @@
 //
 // Every wait is bounded; on expiry the kernel records a code in the context's status word, raises a CTA-wide abort flag
 // that every other wait polls, frees its tensor memory and returns.
-#include <cuda.h>
-
 #include "conv_geom.cuh"
 #include "rt_internal.cuh"
 #include "tc_common.cuh"
+#include "tensor_map.cuh"
 
 namespace tc {
 namespace dw {
@@ -666,21 +665,6 @@ __global__ void __launch_bounds__(32 * GROUPS) conv_dw_finish_vec_kernel(const f
     if (n_out > 2) out[2 * out_step] = t.z;
     if (n_out > 3) out[3 * out_step] = t.w;
   }
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-inline EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-    cudaGetLastError();
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
 }
 
 // 3-D map over t[Nb][C][HW] (fp32) with a box of (bw, ct, 1) elements; elements outside the tensor read as zero.

@@ -8,6 +8,7 @@
 // tap_t(b,p) = x[b, c, yo*sh-ph+ky, xo*sw-pw+kx] for t = (c,ky,kx), zero outside the image.
 #include "rt_internal.cuh"
 #include "conv_geom.cuh"
+#include "packed_fma.cuh"
 
 rt_status rt_sum_axis_internal(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, int64_t inner, float* out,
                                float scale);
@@ -436,9 +437,6 @@ struct ThinPoolParams {
 // Bound by instruction issue: two channels are one packed multiply-add (the same roundings), and the pooling needs no conversions.
 // [1000,1,28,28] to 32 channels: 20.6 -> 17.9 us, [256,1,28,28] 6.9 -> 6.4.
 constexpr int kPoolChannelGroup = 16;
-__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
   unsigned long long v;
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));

@@ -21,11 +21,10 @@
 // pack_kernel beforehand.
 // Every wait is bounded; on expiry the kernel records a code in the status word, raises a flag that all other waits poll, lets its
 // own copies land, frees tensor memory and returns.
-#include <cuda.h>
-
 #include "conv_geom.cuh"
 #include "rt_internal.cuh"
 #include "tc_common.cuh"
+#include "tensor_map.cuh"
 
 namespace tc {
 namespace tma {
@@ -460,18 +459,6 @@ __global__ void __launch_bounds__(256) pack_taps_kernel(const float* __restrict_
   }
 }
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-inline EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-    cudaGetLastError();
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
 // [rows][cols] floats, rows ld floats apart, boxes of box_cols x box_rows, zeros outside.
 inline bool map_matrix(CUtensorMap* m, const float* t, int64_t cols, int64_t rows, int64_t ld, int box_cols, int box_rows, bool swizzle) {
   EncodeTiledFn enc = encode_tiled();

@@ -21,6 +21,7 @@
 // backward (2.4 and 3.9 before the pairs and the shorter mail); batch 64, H 512: 5.3 and 6.5 (5.4 and 7.9).  As kernels of their own the
 // product, the cell and the concatenation took 9.7 forward, 12.3 backward at the first size.  Sizes whose blocks do not fit beside one
 // another, or whose slice of the weights does not fit into a block, run timestep by timestep.
+#include "packed_fma.cuh"
 #include "rt_internal.cuh"
 #include "tc_common.cuh"
 
@@ -85,9 +86,6 @@ struct Pair {
     return a + b;
   }
 };
-__device__ __forceinline__ void fma2(Pair& c, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c.v) : "l"(a), "l"(b));
-}
 __device__ __forceinline__ ulonglong2 pairs_at(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
@@ -217,10 +215,10 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const SeqArg
               const ulonglong2 y01 = pairs_at(w + (k * 2 * U + 8 * j) * 4), y23 = pairs_at(w + (k * 2 * U + U + 8 * j) * 4);
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
-                fma2(acc[j][i][0], xs[i], y01.x);
-                fma2(acc[j][i][1], xs[i], y01.y);
-                fma2(acc[j][i][2], xs[i], y23.x);
-                fma2(acc[j][i][3], xs[i], y23.y);
+                fma2(acc[j][i][0].v, xs[i], y01.x);
+                fma2(acc[j][i][1].v, xs[i], y01.y);
+                fma2(acc[j][i][2].v, xs[i], y23.x);
+                fma2(acc[j][i][3].v, xs[i], y23.y);
               }
             }
           }
@@ -345,10 +343,10 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_backward_kernel(con
         const unsigned long long xs[4] = {p01.x, p01.y, p23.x, p23.y};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          fma2(acc[i][0], xs[i], q01.x);
-          fma2(acc[i][1], xs[i], q01.y);
-          fma2(acc[i][2], xs[i], q23.x);
-          fma2(acc[i][3], xs[i], q23.y);
+          fma2(acc[i][0].v, xs[i], q01.x);
+          fma2(acc[i][1].v, xs[i], q01.y);
+          fma2(acc[i][2].v, xs[i], q23.x);
+          fma2(acc[i][3].v, xs[i], q23.y);
         }
       }
 #pragma unroll

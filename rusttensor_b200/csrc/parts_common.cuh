@@ -1,7 +1,6 @@
 // What the products of operands in 16-bit parts share (k_gemm_parts.cu, k_conv_parts.cu): the scale and the decision between two fp16 and three
 // bf16 parts, splitting, PTX wrappers, the product kernel.  k_gemm_parts.cu says how they work.
 #pragma once
-#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include <climits>
@@ -9,6 +8,7 @@
 #include "conv_geom.cuh"
 #include "rt_internal.cuh"
 #include "tc_common.cuh"
+#include "tensor_map.cuh"
 
 namespace tc {
 namespace parts {
@@ -548,18 +548,6 @@ parts_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
 }
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-inline EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-    cudaGetLastError();
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
 // [rows][cols] 16-bit values, rows ld apart, boxes of 64 x 64, zeros outside.
 inline bool map_parts(CUtensorMap* m, uint16_t* t, int64_t cols, int64_t rows, int64_t ld) {
   EncodeTiledFn enc = encode_tiled();
