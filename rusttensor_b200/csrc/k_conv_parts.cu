@@ -38,39 +38,46 @@ struct ConvSplitArgs {
   TapSplit taps;        // w null: none
   int images, sample_blocks;
   uint32_t most_faint[kMaxSources];
-  const Magnitudes* samples;  // [source][block]; the weights, the last source, are looked at as a whole
-  Magnitudes* stats;          // [source][block] of conv_split_kernel<false>; of the weights only how many are faint
+  const uint2* samples;       // [source][block]; the weights, the last source, are looked at as a whole
+  uint32_t* verdicts;         // [source][block] of conv_split_kernel<false>
   Decision* decision;
 };
 // Bound by memory: 4 bytes read and 4 written an element.  A block turns 32 channels x 128 pixels at a time through shared memory; what is
 // looked at is 128 pixels of a channel.  AGAIN: into three parts, if the first pass has found that two will not do.
 template <bool AGAIN>
-__global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) {
+__global__ void __launch_bounds__(256, 4) conv_split_kernel(const ConvSplitArgs a) {
   RT_PDL_ENTRY();
-  __shared__ uint32_t red[3][8];
+  __shared__ uint32_t red[2 * kMaxSources][8];
   __shared__ float tile[32][kSplitPixels + 1];
   constexpr int depth = AGAIN ? 16 : 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, weights = a.taps.w ? 1 : 0;
   Decision d{};
-  for (int q = 0; q < a.images + weights; ++q) {
-    Magnitudes v = over_blocks(a.samples + q * a.sample_blocks, a.sample_blocks, red);
-    d.exponent[q] = exponent_for(v.most);
-    if (AGAIN) {
-      const Magnitudes seen = over_blocks(a.stats + q * gridDim.x, gridDim.x, red);
-      if (q < a.images) v = seen;
-      v.faint = seen.faint;
-      if (out_of_range(v, d.exponent[q], a.most_faint[q])) d.wide = 1;
-      if (v.most >= 0x7f800000u) d.special = 1;
-    }
-  }
+  Magnitudes of_weights;
   if (AGAIN) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *a.decision = d;
+    d = decide(a.verdicts, a.images + weights, gridDim.x, a.most_faint, red);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      a.decision->wide = d.wide;
+      a.decision->special = d.special;
+    }
     if (!d.wide) return;
+  } else {
+    uint2 v[kMaxSources];
+    over_samples(a.samples, a.images + weights, a.sample_blocks, red, v);
+#pragma unroll
+    for (int q = 0; q < kMaxSources; ++q) {
+      d.exponent[q] = exponent_for(v[q].x);
+      if (blockIdx.x == 0 && threadIdx.x == 0) a.decision->exponent[q] = d.exponent[q];
+      if (q == a.images) {
+        of_weights.most = v[q].x;
+        of_weights.least = v[q].y;
+      }
+    }
   }
   for (int q = 0; q < a.images; ++q) {
     const ImageSplit& s = a.image[q];
-    const float scale = AGAIN ? 1.f : ldexpf(1.f, d.exponent[q]);
-    const uint32_t faint = faint_below(d.exponent[q]);
+    const int exponent = q == 0 ? d.exponent[0] : d.exponent[1];
+    const float scale = AGAIN ? 1.f : ldexpf(1.f, exponent);
+    const uint32_t faint = faint_below(exponent);
     Magnitudes all;
     for (int i0 = blockIdx.x; i0 < s.tiles; i0 += gridDim.x) {
       uint32_t im, t;
@@ -134,16 +141,16 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
     }
     if (!AGAIN) {
       all = over_block(all, red);
-      if (threadIdx.x == 0) a.stats[q * gridDim.x + blockIdx.x] = all;
+      if (threadIdx.x == 0) a.verdicts[q * gridDim.x + blockIdx.x] = verdict(all, exponent);
     }
   }
   if (!weights) return;
   const TapSplit& s = a.taps;
-  const float scale = AGAIN ? 1.f : ldexpf(1.f, d.exponent[a.images]);
+  const int exponent = a.images == 0 ? d.exponent[0] : (a.images == 1 ? d.exponent[1] : d.exponent[2]);
+  const float scale = AGAIN ? 1.f : ldexpf(1.f, exponent);
   const int eighths = (s.C + depth - 1) / depth * depth / 8, taps = s.kh * s.kw;
   const int64_t total = (int64_t)s.N * taps * eighths;
-  const uint32_t faint = faint_below(d.exponent[a.images]);
-  Magnitudes all;
+  const uint32_t faint = faint_below(exponent);
   // from the last block on, which has had the least to do
   for (int64_t i = (int64_t)(gridDim.x - 1 - blockIdx.x) * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
     const int c = (int)(i % eighths) * 8, tap = (int)(i / eighths % taps), n = (int)(i / eighths / taps);
@@ -164,7 +171,7 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
       x[j] = there && c + j < s.C ? __ldg(w + (c + j) * s.sc) : 0.f;
       low = lower(low, __float_as_uint(x[j]) & 0x7fffffffu);
     }
-    all.faint += low < faint;
+    of_weights.faint += low < faint;
     uint4 part[4];
     split8(x, AGAIN, scale, part);
     uint16_t* o = s.out + n * s.pitch + ((int64_t)tap * (eighths * 8 / depth) + c / depth) * 64 + c % depth;
@@ -176,8 +183,8 @@ __global__ void __launch_bounds__(256) conv_split_kernel(const ConvSplitArgs a) 
     }
   }
   if (!AGAIN) {
-    all = over_block(all, red);
-    if (threadIdx.x == 0) a.stats[a.images * gridDim.x + blockIdx.x] = all;
+    of_weights = over_block(of_weights, red);
+    if (threadIdx.x == 0) a.verdicts[a.images * gridDim.x + blockIdx.x] = verdict(of_weights, exponent);
   }
 }
 
@@ -540,16 +547,16 @@ inline void choose_box(int pixels, int w, int h, int n, int* bw, int* bh, int* b
 // Parts of images and weights (taps null: none).
 inline rt_status split_conv(rt_ctx* ctx, Image* const* images, int n_images, Taps* taps, RtScratch* work, Decision** decision) {
   const int sample_blocks = ctx->sm_count, blocks = 4 * ctx->sm_count;
-  rt_status st = work->alloc(sizeof(Magnitudes) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
+  rt_status st = work->alloc((sizeof(uint2) * (size_t)sample_blocks + sizeof(uint32_t) * (size_t)blocks) * kMaxSources + sizeof(Decision));
   if (st != RT_OK) return st;
   SampleArgs a{};
   ConvSplitArgs b{};
-  Magnitudes* samples = work->as<Magnitudes>();
+  uint2* samples = work->as<uint2>();
   a.count = n_images + (taps ? 1 : 0);
   b.sample_blocks = sample_blocks;
   b.samples = samples;
-  b.stats = samples + (size_t)sample_blocks * kMaxSources;
-  *decision = b.decision = reinterpret_cast<Decision*>(b.stats + (size_t)blocks * kMaxSources);
+  b.verdicts = reinterpret_cast<uint32_t*>(samples + (size_t)sample_blocks * kMaxSources);
+  *decision = b.decision = reinterpret_cast<Decision*>(b.verdicts + (size_t)blocks * kMaxSources);
   b.images = n_images;
   for (int q = 0; q < n_images; ++q) {
     Image& im = *images[q];

@@ -53,8 +53,8 @@ struct SplitArgs {
   SplitSource s[kMaxSplits];
   int count, sources, sample_blocks;
   uint32_t most_faint[kMaxSources];
-  const Magnitudes* samples;  // [source][block] of sample_kernel
-  Magnitudes* stats;          // [source][block] of split_kernel<false>
+  const uint2* samples;       // [source][block] of sample_kernel
+  uint32_t* verdicts;         // [source][block] of split_kernel<false>
   Decision* decision;
 };
 // A tile of 64 rows x 128 columns: a warp has eight rows, two at a time, a lane eight columns of one.
@@ -133,29 +133,38 @@ __device__ __forceinline__ void split_tiles(const SplitSource& s, float scale, u
 }
 // Bound by memory: 4 bytes read and 4 written an element.  AGAIN: into three parts, if the first pass has found that two will not do.
 template <bool AGAIN>
-__global__ void __launch_bounds__(256) split_kernel(const SplitArgs a) {
+__global__ void __launch_bounds__(256, 4) split_kernel(const SplitArgs a) {
   RT_PDL_ENTRY();
-  __shared__ uint32_t red[3][8];
+  __shared__ uint32_t red[2 * kMaxSources][8];
   __shared__ uint32_t cols[AGAIN ? 1 : 2][16][kTileCols];
   Decision d{};
-  for (int q = 0; q < a.sources; ++q) {
-    d.exponent[q] = exponent_for(over_blocks(a.samples + q * a.sample_blocks, a.sample_blocks, red).most);
-    if (AGAIN && out_of_range(over_blocks(a.stats + q * gridDim.x, gridDim.x, red), d.exponent[q], a.most_faint[q])) d.wide = 1;
-  }
   if (AGAIN) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *a.decision = d;
+    d = decide(a.verdicts, a.sources, gridDim.x, a.most_faint, red);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      a.decision->wide = d.wide;
+      a.decision->special = d.special;
+    }
     if (!d.wide) return;
+  } else {
+    uint2 v[kMaxSources];
+    over_samples(a.samples, a.sources, a.sample_blocks, red, v);
+#pragma unroll
+    for (int q = 0; q < kMaxSources; ++q) {
+      d.exponent[q] = exponent_for(v[q].x);
+      if (blockIdx.x == 0 && threadIdx.x == 0) a.decision->exponent[q] = d.exponent[q];
+    }
   }
   for (int q = 0; q < a.count; ++q) {
     const SplitSource& s = a.s[q];
-    const float scale = AGAIN ? 1.f : ldexpf(1.f, d.exponent[s.source]);
-    const uint32_t faint = faint_below(d.exponent[s.source]);
+    const int exponent = s.source == 0 ? d.exponent[0] : (s.source == 1 ? d.exponent[1] : d.exponent[2]);
+    const float scale = AGAIN ? 1.f : ldexpf(1.f, exponent);
+    const uint32_t faint = faint_below(exponent);
     Magnitudes all;
     if (s.vec) split_tiles<true, AGAIN>(s, scale, faint, cols, all);
     else split_tiles<false, AGAIN>(s, scale, faint, cols, all);
     if (AGAIN || !s.look) continue;
     all = over_block(all, red);
-    if (threadIdx.x == 0) a.stats[s.source * gridDim.x + blockIdx.x] = all;
+    if (threadIdx.x == 0) a.verdicts[s.source * gridDim.x + blockIdx.x] = verdict(all, exponent);
   }
 }
 
@@ -190,15 +199,15 @@ struct Splitting {
   explicit Splitting(rt_ctx* ctx) : work(ctx) {}
   rt_status prepare(rt_ctx* ctx, Split* const* s, int count, int sources) {
     const int sample_blocks = ctx->sm_count, blocks = 4 * ctx->sm_count;
-    rt_status st = work.alloc(sizeof(Magnitudes) * (size_t)(sample_blocks + blocks) * kMaxSources + sizeof(Decision));
+    rt_status st = work.alloc((sizeof(uint2) * (size_t)sample_blocks + sizeof(uint32_t) * (size_t)blocks) * kMaxSources + sizeof(Decision));
     if (st != RT_OK) return st;
-    Magnitudes* samples = work.as<Magnitudes>();
+    uint2* samples = work.as<uint2>();
     sample.count = split.sources = sources;
     split.count = count;
     split.sample_blocks = sample_blocks;
     split.samples = samples;
-    split.stats = samples + (size_t)sample_blocks * kMaxSources;
-    split.decision = reinterpret_cast<Decision*>(split.stats + (size_t)blocks * kMaxSources);
+    split.verdicts = reinterpret_cast<uint32_t*>(samples + (size_t)sample_blocks * kMaxSources);
+    split.decision = reinterpret_cast<Decision*>(split.verdicts + (size_t)blocks * kMaxSources);
     for (int q = 0; q < count; ++q) {
       if ((st = s[q]->alloc()) != RT_OK) return st;
       const Sample m = sample_of(ctx, s[q]->p, s[q]->ld, s[q]->rows, s[q]->cols, false);
@@ -212,7 +221,7 @@ struct Splitting {
     return RT_OK;
   }
   rt_status run(rt_ctx* ctx) {
-    rt_launch(ctx, sample_kernel, split.sample_blocks, 256, 0, sample, work.as<Magnitudes>());
+    rt_launch(ctx, sample_kernel, split.sample_blocks, 256, 0, sample, work.as<uint2>());
     RT_LAUNCHED(ctx);
     rt_launch(ctx, split_kernel<false>, 4 * ctx->sm_count, 256, 0, split);
     RT_LAUNCHED(ctx);

@@ -42,9 +42,11 @@ struct Decision {
 
 // ---- magnitudes: the largest, and the smallest of the non-zero segments' largest, as the bits of floats (which order as they do; NaN
 // above infinity), and in how many pieces (of eight or sixteen elements) there is a faint one ------------------------------------------
-struct alignas(16) Magnitudes {
-  uint32_t most = 0, least = 0xffffffffu, faint = 0, unused = 0;
+struct Magnitudes {
+  uint32_t most = 0, least = 0xffffffffu, faint = 0;
 };
+// What a block makes of its own, in a word: whether two parts are out of the question, whether there are infinities or NaN, the faint pieces.
+constexpr uint32_t kOutOfRange = 1u << 31, kSpecial = 1u << 30, kFaintOfBlock = 1u << 20;
 struct Sample {
   const float* p;
   int64_t ld;
@@ -78,29 +80,79 @@ __device__ __forceinline__ Magnitudes over_block(Magnitudes m, uint32_t (*red)[8
   m.faint = __reduce_add_sync(0xffffffffu, lane < 8 ? red[2][lane] : 0u);
   return m;
 }
-__device__ __forceinline__ Magnitudes over_blocks(const Magnitudes* stats, int n, uint32_t (*red)[8]) {
-  Magnitudes m;
-  for (int i = threadIdx.x; i < n; i += 256) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(stats + i));
-    m.most = max(m.most, v.x);
-    m.least = min(m.least, v.y);
-    m.faint += v.z;
+// Most and least over all blocks' samples, [source][block].  red: 6 x 8 words.
+__device__ __forceinline__ void over_samples(const uint2* samples, int sources, int blocks, uint32_t (*red)[8], uint2 (&v)[kMaxSources]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < kMaxSources; ++q) v[q] = make_uint2(0u, 0xffffffffu);
+  for (int i = threadIdx.x; i < blocks; i += 256)
+#pragma unroll
+    for (int q = 0; q < kMaxSources; ++q)
+      if (q < sources) {
+        const uint2 w = __ldg(samples + q * blocks + i);
+        v[q] = make_uint2(max(v[q].x, w.x), min(v[q].y, w.y));
+      }
+#pragma unroll
+  for (int q = 0; q < kMaxSources; ++q) {
+    const uint32_t most = __reduce_max_sync(0xffffffffu, v[q].x), least = __reduce_min_sync(0xffffffffu, v[q].y);
+    if (lane == 0) {
+      red[2 * q][warp] = most;
+      red[2 * q + 1][warp] = least;
+    }
   }
-  return over_block(m, red);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kMaxSources; ++q)
+    v[q] = make_uint2(__reduce_max_sync(0xffffffffu, red[2 * q][lane & 7]), __reduce_min_sync(0xffffffffu, red[2 * q + 1][lane & 7]));
+  __syncthreads();
 }
-// The exponent that a sample asks for; more than 100 either way is refused by out_of_range.
+// The exponent that a sample asks for; more than 100 either way is refused by verdict().
 __device__ __forceinline__ int exponent_for(uint32_t most) { return most == 0 || most >= 0x7f800000u ? 0 : kSampleExponent + 127 - (int)(most >> 23); }
 // An element of magnitude m (its bits) is faint if m - 1 is below this: zero is not.
 __device__ __forceinline__ uint32_t faint_below(int exponent) { return max(__float_as_uint(ldexpf(1.f, kFaintExponent - exponent)), 1u) - 1u; }
 // The least of m - 1 over a piece, an element more.
 __device__ __forceinline__ uint32_t lower(uint32_t least, uint32_t m) { return __viaddmin_u32(m, 0xffffffffu, least); }
-__device__ __forceinline__ bool out_of_range(const Magnitudes& v, int exponent, uint32_t most_faint) {
-  if (v.most == 0) return false;
-  return v.most >= 0x7f800000u || exponent > 100 || exponent < -100 || (int)(v.most >> 23) - 127 + exponent > kLargestExponent ||
-         (int)(v.least >> 23) - 127 + exponent < kSmallestExponent || v.faint > most_faint;
+__device__ __forceinline__ uint32_t verdict(const Magnitudes& v, int exponent) {
+  uint32_t w = min(v.faint, kFaintOfBlock);
+  if (v.most >= 0x7f800000u) w |= kSpecial | kOutOfRange;
+  else if (v.most && (exponent > 100 || exponent < -100 || (int)(v.most >> 23) - 127 + exponent > kLargestExponent ||
+                      (int)(v.least >> 23) - 127 + exponent < kSmallestExponent))
+    w |= kOutOfRange;
+  return w;
+}
+// All blocks' verdicts, [source][block].  red: 4 x 8 words.
+__device__ __forceinline__ Decision decide(const uint32_t* verdicts, int sources, int blocks, const uint32_t (&most_faint)[kMaxSources], uint32_t (*red)[8]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t flags = 0, faint[kMaxSources] = {};
+#pragma unroll 4
+  for (int i = threadIdx.x; i < blocks; i += 256)
+#pragma unroll
+    for (int q = 0; q < kMaxSources; ++q)
+      if (q < sources) {
+        const uint32_t w = __ldg(verdicts + q * blocks + i);
+        flags |= w;
+        faint[q] += w & (kSpecial - 1);
+      }
+  flags = __reduce_or_sync(0xffffffffu, flags);
+#pragma unroll
+  for (int q = 0; q < kMaxSources; ++q) faint[q] = __reduce_add_sync(0xffffffffu, faint[q]);
+  if (lane == 0) {
+    red[kMaxSources][warp] = flags;
+#pragma unroll
+    for (int q = 0; q < kMaxSources; ++q) red[q][warp] = faint[q];
+  }
+  __syncthreads();
+  flags = __reduce_or_sync(0xffffffffu, red[kMaxSources][lane & 7]);
+  Decision d{};
+  d.wide = (flags & kOutOfRange) != 0;
+  d.special = (flags & kSpecial) != 0;
+#pragma unroll
+  for (int q = 0; q < kMaxSources; ++q)
+    if (q < sources && __reduce_add_sync(0xffffffffu, lane < 8 ? red[q][lane] : 0u) > most_faint[q]) d.wide = 1;
+  return d;
 }
 // A warp has eight rows of a tile of 64 x 128, eight 128-bit loads in flight.
-static __global__ void __launch_bounds__(256) sample_kernel(const SampleArgs a, Magnitudes* __restrict__ out) {
+static __global__ void __launch_bounds__(256) sample_kernel(const SampleArgs a, uint2* __restrict__ out) {
   RT_PDL_ENTRY();
   __shared__ uint32_t cols[2][8][kTileCols];
   __shared__ uint32_t red[3][8];
@@ -153,7 +205,7 @@ static __global__ void __launch_bounds__(256) sample_kernel(const SampleArgs a, 
       }
     }
     all = over_block(all, red);
-    if (threadIdx.x == 0) out[q * gridDim.x + blockIdx.x] = all;
+    if (threadIdx.x == 0) out[q * gridDim.x + blockIdx.x] = make_uint2(all.most, all.least);
     __syncthreads();
   }
 }

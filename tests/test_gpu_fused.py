@@ -149,13 +149,14 @@ def program_counts(capi):
 # the step is a handful of launches, however many timesteps it has.
 @pytest.mark.parametrize("config,dims,interpreted,launches", [(1, [64, 784, 128, 10], 0, 9), (101, [7, 13, 5, 3], 0, 10), (2, [33, 57], 0, 4),
                                                               (2, [1100, 1000], 0, 4), (3, [16, 28, 32, 64, 128, 10], 0, 21),
-                                                              (103, [5, 8, 3, 4, 7, 3], 0, 23), (4, [2, 3, 6, 5], 0, 22), (104, [8, 64, 56, 128], 0, 26),
+                                                              (103, [5, 8, 3, 4, 7, 3], 0, 23), (4, [2, 3, 6, 5], 0, 22), (104, [8, 64, 56, 128], 0, 27),
                                                               (5, [50, 200, 60, 30], 0, 15), (105, [50, 200, 60, 30], 1, 14), (5, [50, 200, 120, 30], 0, 15),
                                                               (105, [50, 200, 120, 30], 1, 16)])
 def test_the_workloads_find_their_compiled_programs(capi, config, dims, interpreted, launches):
     import rusttensor_b200
 
     tr = rusttensor_b200.DataParallelTrainer(config, dims)
+    rusttensor_b200.engine()._call("sync")  # what others have left unevaluated is none of the step's
     before = program_counts(capi)
     tr.capture()
     found, missed, launched = (b - a for a, b in zip(before, program_counts(capi)))
