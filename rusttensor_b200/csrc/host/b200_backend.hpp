@@ -850,7 +850,7 @@ struct B200Backend {
   static Storage min_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_MIN, o, g, "min"); }
   static Storage prod_backward(const OpB& o, const Storage& g) { return reduce_bwd(RT_RED_PROD, o, g, "prod"); }
   static Storage logsumexp_backward(const OpB& o, const Storage& g) {
-    // g exp(x - logsumexp(x)): elementwise, with the forward result, unless it or x may have been changed since
+    // g exp(x - logsumexp(x)): elementwise, with the forward result, unless it or x may have been changed since (Tag::RowGrad)
     if (o.inputs.size() == 1 && o.cached_outputs && o.cached_outputs->buf) {
       const Storage &x = o.inputs[0].data(), &lse = *o.cached_outputs;
       const Axis3 a = split(x.shape, o.op_type.axis);
@@ -858,7 +858,18 @@ struct B200Backend {
           (int64_t)g.numel() == a.outer && lse.numel() == g.numel() && ((!x.buf->escaped && !lse.buf->escaped) || lazy::capturing())) {
         Shape rows = x.shape;
         rows.back() = 1;
-        return lz_binary(RT_F_MUL, reshaped(g, rows), lz_unary(RT_F_EXP, lz_binary(RT_F_SUB, x, reshaped(lse, rows), x.shape)), x.shape);
+        lazy::Node n{lazy::Kind::Binary};
+        n.op = RT_F_MUL;
+        n.tag = lazy::Tag::RowGrad;
+        n.weight = lazy::op_weight(RT_F_MUL);
+        n.in = {input(reshaped(g, rows)), input(lz_unary(RT_F_EXP, lz_binary(RT_F_SUB, x, reshaped(lse, rows), x.shape))), input(x)};
+        n.run = [a](lazy::Node& nd, DeviceBuffer* b) {
+          const float *px = nd.in[2].buf->data(), *pg = nd.in[0].buf->data();
+          lazy::Block out(b->ctx, b->numel);
+          check(rt_reduce_backward(ctx(), RT_RED_LOGSUMEXP, px, pg, a.outer, a.len, a.inner, out.ptr));
+          b->ptr = out.release();
+        };
+        return defer(std::move(n), x.shape);
       }
     }
     return reduce_bwd(RT_RED_LOGSUMEXP, o, g, "logsumexp");

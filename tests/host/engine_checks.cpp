@@ -18,6 +18,8 @@ int mallocs;
 bool kernels_fail = false;
 int masked_pool_gradients;     // launches of the pooling gradient that masks by the relu in front
 int forward_sequences, backward_sequences;
+int row_gradients, programs;   // launches of the gradient of a logsumexp by its own kernel, of elementwise programs
+bool reductions_known = false; // kernels for programs with a reduction
 bool recording = false;
 int unrecorded;                // kernels while nothing is recorded
 rt_status kernel() {
@@ -106,11 +108,17 @@ rt_status rt_sum_rows_accumulate_list(rt_ctx*, int count, const float* const* xs
 rt_status rt_gemm_bias_act_list(rt_ctx*, int, const float* const*, float* const*, int64_t, int64_t, int64_t, const float*, const float*, int) {
   return kernel();
 }
-rt_status rt_fused_reduction_known(rt_ctx*, const rt_fused_program*, int) { return RT_ERR_UNIMPLEMENTED; }
-rt_status rt_fused_column_sums(rt_ctx*, const rt_fused_program*, int, float*) { return RT_ERR_UNIMPLEMENTED; }
-rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return RT_ERR_UNIMPLEMENTED; }
+rt_status rt_fused_reduction_known(rt_ctx*, const rt_fused_program*, int) { return reductions_known ? RT_OK : RT_ERR_UNIMPLEMENTED; }
+rt_status rt_fused_column_sums(rt_ctx*, const rt_fused_program*, int, float*) { return kernel(); }
+rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return kernel(); }
+rt_status rt_reduce_backward(rt_ctx*, int, const float* x, const float*, int64_t outer, int64_t len, int64_t, float* dx) {
+  ++row_gradients;
+  for (int64_t i = 0; i < outer * len; ++i) dx[i] = x[i];  // to tell which values it has read
+  return kernel();
+}
 rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of windows; results of other programs stay zero
   if (kernel() != RT_OK) return RT_ERR_CUDA;
+  ++programs;
   if (p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_OK;
   const int rows = p->nd == 2 ? p->shape[0] : 1, cols = p->shape[p->nd - 1];
   const rt_fused_operand& o = p->operand[0];
@@ -545,10 +553,41 @@ void refused_programs_take_no_memory() {
   EXPECT(live.empty());
 }
 
+// The gradient of a logsumexp is part of a program that carries a reduction, where there is one; elsewhere it has a kernel of its own, which the
+// program around it reads.
+void gradients_of_rows() {
+  for (bool known : {false, true}) {
+    B::Storage x = make({4, 8}, 0.f), b = make({8}, 0.f);
+    const B::Storage y = B::tanh(B::add(x, b)), lse = B::logsumexp(y, 1);
+    Op<B> o(OpType::with_axis(OpType::LogSumExp, 1), {Tensor<B>(y, true)}, nullptr);
+    o.cached_outputs = lse;
+    reductions_known = known;
+    row_gradients = programs = 0;
+    const B::Storage d = B::logsumexp_backward(o, make({4}, 1.f)), dx = B::lz_mul(d, B::lz_unary(RT_F_ONE_MINUS_SQUARE, y));
+    const B::Storage db = B::unbroadcast(B::lz_mul(dx, x), {8});
+    EXPECT(d.buf->node && row_gradients == 0);
+    dx.ptr();
+    EXPECT(row_gradients == (known ? 0 : 1) && programs == (known ? 0 : 1));
+    db.ptr();
+    reductions_known = false;
+  }
+  {  // what it reads changes in place: it is computed before
+    B::Storage x = make({4, 8}, 3.f);
+    const B::Storage lse = B::logsumexp(x, 1);
+    Op<B> o(OpType::with_axis(OpType::LogSumExp, 1), {Tensor<B>(x, true)}, nullptr);
+    o.cached_outputs = lse;
+    const B::Storage d = B::logsumexp_backward(o, make({4}, 1.f));
+    EXPECT(d.buf->node != nullptr);
+    scribble(B::escape(x), 32);
+    EXPECT(!d.buf->node && holds(d, 3.f));
+  }
+  EXPECT(live.empty() && DeviceBuffer::row_gradients() == 0);
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"refused_programs_take_no_memory", refused_programs_take_no_memory}, {"a_capture_in_two_parts", a_capture_in_two_parts},
+} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"gradients_of_rows", gradients_of_rows}, {"refused_programs_take_no_memory", refused_programs_take_no_memory}, {"a_capture_in_two_parts", a_capture_in_two_parts},
                {"kept_results_stay_where_they_are_written", kept_results_stay_where_they_are_written},
                {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},
