@@ -267,7 +267,10 @@ rt_status rt_fused_elementwise(rt_ctx* ctx, const rt_fused_program* program);
 /* The same for a program over [rows, columns] (nd = 2), with a reduction of one of its outputs in the same launch, where a kernel has been
  * compiled for that (otherwise RT_ERR_UNIMPLEMENTED, and nothing has been done): the column sums of output `which`, which itself is not
  * written (its pointer only has to be valid); the logsumexp of the rows of output 0, which is.  rt_fused_reduction_known asks beforehand, when
- * the outputs need not have memory yet: RT_OK if there is a kernel for the column sums of output `which` (-1: for the logsumexp). */
+ * the outputs need not have memory yet: RT_OK if there is a kernel for the column sums of output `which` (-1: for the logsumexp).
+ * rt_fused_reduction_possible asks before there is a program: whether there is a kernel whose program has just these ops (bit RT_F_ADD for
+ * an addition, and so on; loads, outputs, registers and selections aside), for column sums or, with which = -1, for a logsumexp. */
+rt_status rt_fused_reduction_possible(rt_ctx* ctx, int which, uint64_t ops);
 rt_status rt_fused_reduction_known(rt_ctx* ctx, const rt_fused_program* program, int which);
 rt_status rt_fused_column_sums(rt_ctx* ctx, const rt_fused_program* program, int which, float* sums);
 rt_status rt_fused_logsumexp(rt_ctx* ctx, const rt_fused_program* program, float* out);

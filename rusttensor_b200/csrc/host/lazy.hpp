@@ -1394,9 +1394,28 @@ inline bool evaluate_reduced(DeviceBuffer* b, Compiler& c, float* lse) {
   for (size_t k = 0; k < outs.size(); ++k) blocks[k].to(outs[k]);
   return true;
 }
+// Whether a program of the expression b can be one of those: building it to be told otherwise costs as much as building the one that is launched
+// (3 us of a small model's training step on the host).
+inline bool may_be_reduced(DeviceBuffer* b, int which) {
+  uint64_t ops = 0;
+  std::vector<const DeviceBuffer*> open{b}, seen{b};
+  while (!open.empty()) {
+    const Node& n = *open.back()->node;
+    open.pop_back();
+    if (n.kind == Kind::Unary || n.kind == Kind::BinaryImm || n.kind == Kind::Binary) ops |= uint64_t(1) << n.op;
+    for (const Input& i : n.in) {
+      const DeviceBuffer* x = i.buf.get();
+      if (!x->node || x->node->kind == Kind::Opaque || std::find(seen.begin(), seen.end(), x) != seen.end()) continue;
+      if (seen.size() == RT_FUSED_MAX_CODE) return false;  // no program is as long
+      seen.push_back(x);
+      open.push_back(x);
+    }
+  }
+  return rt_fused_reduction_possible(b->ctx, which, ops) == RT_OK;
+}
 // An expression over [rows, columns] together with the pending column sums of a term that it shares values with.
 inline bool evaluate_with_sums(DeviceBuffer* b) {
-  if (Walk::depth() > 1 || b->node->shape.size() != 2 || b->numel == 0 || !column_sum_waits(b)) return false;
+  if (Walk::depth() > 1 || b->node->shape.size() != 2 || b->numel == 0 || !column_sum_waits(b) || !may_be_reduced(b, 0)) return false;
   Compiler c;
   c.keep_rows();
   return evaluate_reduced(b, c, nullptr);
@@ -1424,6 +1443,7 @@ inline void settle_row_gradients(DeviceBuffer* b) {
 // The rows of an expression and their logsumexp.
 inline bool evaluate_with_logsumexp(DeviceBuffer* b, float* out) {
   if (Walk::depth() > 0 || !b->node || b->node->kind == Kind::Opaque || b->node->kind == Kind::Const || b->node->shape.size() != 2 || b->numel == 0) return false;
+  if (!may_be_reduced(b, -1)) return false;
   std::shared_ptr<DeviceBuffer> guard = b->shared_from_this();
   Compiler c;
   c.keep_rows();

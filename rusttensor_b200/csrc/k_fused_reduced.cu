@@ -9,6 +9,9 @@
 // Measured on [4096, 4096], mean of the logsumexp of exp(-x^2) + tanh(x b) + sin(x) / (1 + x^2) and its gradients to x and b in a captured step:
 // 204 us with the programs and the reductions apart, 148 us here (201 MB, 31 us at the copy bandwidth): the rows with their logsumexp
 // 58 us, the gradient with the column sums 88 us, both bound by instruction issue (125 and 190 slots a warp and element).
+#include <algorithm>
+#include <vector>
+
 #include "fused_known.cuh"
 
 rt_status rt_sum_axis_internal(rt_ctx* ctx, const float* x, int64_t outer, int64_t len, int64_t inner, float* out, float scale);
@@ -172,9 +175,42 @@ const Reduced* find(const Reduced (&list)[N], const FusedParams& p) {
   return find(list, p.n_code, p.n_preload, [&](int i) { return p.code[i].x; });
 }
 
+// The ops of a program as a set; of an op and its reversed form, and of opposite comparisons, the one.
+static_assert(RT_F_COUNT <= 64, "a bit an op");
+uint64_t one_form(uint64_t ops) {
+  auto fold = [&](int from, int to) {
+    if (ops >> from & 1) ops = (ops & ~(uint64_t(1) << from)) | uint64_t(1) << to;
+  };
+  fold(RT_F_LT, RT_F_GT);
+  fold(RT_F_LE, RT_F_GE);
+  return ops;
+}
+template <int N>
+bool has_ops(const Reduced (&list)[N], uint64_t ops) {
+  static const std::vector<uint64_t> sets = [&list] {
+    std::vector<uint64_t> v;
+    for (const Reduced& k : list) {
+      uint64_t set = 0;
+      for (int i = 0; i < k.n_code; ++i) {
+        const int op = (int)(k.code[i] & 255);
+        if (op == RT_F_LOAD || op == RT_F_OUT || op == RT_F_REG || op == RT_F_SELECT) continue;
+        set |= uint64_t(1) << (op == kReverseSub ? RT_F_SUB : (op == kReverseDiv ? RT_F_DIV : (op == kReversePow ? RT_F_POWF : op)));
+      }
+      v.push_back(one_form(set));
+    }
+    return v;
+  }();
+  return std::find(sets.begin(), sets.end(), one_form(ops)) != sets.end();
+}
+
 }  // namespace
 
 extern "C" {
+
+rt_status rt_fused_reduction_possible(rt_ctx* ctx, int which, uint64_t ops) {
+  RT_CHECK_CTX(ctx);
+  return (which < 0 ? has_ops(kWithLogsumexp, ops) : has_ops(kWithSums, ops)) ? RT_OK : RT_ERR_UNIMPLEMENTED;
+}
 
 rt_status rt_fused_reduction_known(rt_ctx* ctx, const rt_fused_program* f, int which) {
   RT_CHECK_CTX(ctx);

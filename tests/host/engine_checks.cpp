@@ -19,6 +19,7 @@ bool kernels_fail = false;
 int masked_pool_gradients;     // launches of the pooling gradient that masks by the relu in front
 int forward_sequences, backward_sequences;
 int row_gradients, programs;   // launches of the gradient of a logsumexp by its own kernel, of elementwise programs
+int asked_of_programs;         // programs built for a kernel with a reduction
 bool reductions_known = false; // kernels for programs with a reduction
 bool recording = false;
 int unrecorded;                // kernels while nothing is recorded
@@ -108,7 +109,9 @@ rt_status rt_sum_rows_accumulate_list(rt_ctx*, int count, const float* const* xs
 rt_status rt_gemm_bias_act_list(rt_ctx*, int, const float* const*, float* const*, int64_t, int64_t, int64_t, const float*, const float*, int) {
   return kernel();
 }
-rt_status rt_fused_reduction_known(rt_ctx*, const rt_fused_program*, int) { return reductions_known ? RT_OK : RT_ERR_UNIMPLEMENTED; }
+uint64_t possible_ops = ~uint64_t(0);  // of kernels with a reduction; all ones: any
+rt_status rt_fused_reduction_possible(rt_ctx*, int, uint64_t ops) { return possible_ops == ~uint64_t(0) || ops == possible_ops ? RT_OK : RT_ERR_UNIMPLEMENTED; }
+rt_status rt_fused_reduction_known(rt_ctx*, const rt_fused_program*, int) { return ++asked_of_programs, reductions_known ? RT_OK : RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_column_sums(rt_ctx*, const rt_fused_program*, int, float*) { return kernel(); }
 rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return kernel(); }
 rt_status rt_reduce_backward(rt_ctx*, int, const float* x, const float*, int64_t outer, int64_t len, int64_t, float* dx) {
@@ -549,6 +552,16 @@ void refused_programs_take_no_memory() {
     v.ptr();
     EXPECT(!v.buf->node && mallocs <= 2);  // v, and u beside it, which somebody holds
     sums.ptr();
+  }
+  {  // nor is one built whose ops are not those of any
+    const B::Storage x = make({4, 8}, 0.f), b = make({8}, 0.f);
+    for (bool other : {false, true}) {
+      possible_ops = uint64_t(1) << RT_F_TANH | uint64_t(1) << RT_F_ADD | uint64_t(1) << RT_F_MUL;
+      asked_of_programs = 0;
+      B::logsumexp(B::add(B::tanh(B::mul(x, b)), other ? B::exp(x) : x), 1).ptr();
+      EXPECT(asked_of_programs == (other ? 0 : 1));
+      possible_ops = ~uint64_t(0);
+    }
   }
   EXPECT(live.empty());
 }
