@@ -16,8 +16,8 @@
 // A K-block in memory is four slots of 16 along the reduction: hi hi lo lo of 32 elements, or the three bf16 parts of 16 and the first once
 // more, with zeros for infinities and NaN: the cross terms take that one, so that an infinity meets no zero which is none.  A row of it is
 // 128 bytes (reduction contiguous) or the block is 64 rows (rows contiguous); TMA fetches it in boxes of 8 KB with the 128-byte swizzle and
-// tcgen05.mma reads it as it lies, either way round, so that nothing is transposed and a matrix that is an operand twice (the upstream
-// gradient of a product) is split once.
+// tcgen05.mma reads it as it lies, either way round, so that nothing is transposed.  A matrix that is an operand with its rows and with its columns as
+// the reduction (the upstream gradient of a product) is looked at once and split both ways.
 //
 // Roles of a CTA (one per SM, walking over tiles of 128 x up to 256): a TMA warp up to four K-blocks ahead, an MMA warp, eight warps that
 // empty the accumulator into registers and write the result.  The tensor core adds into its accumulator with truncation, an error that
@@ -131,7 +131,8 @@ __device__ __forceinline__ void split_tiles(const SplitSource& s, float scale, u
     }
   }
 }
-// Bound by memory: 4 bytes read and 4 written an element.  AGAIN: into three parts, if the first pass has found that two will not do.
+// Bound by memory: 4 bytes read and 4 written an element.  AGAIN: into three parts, if the first pass has found that two will not do; otherwise over
+// in 4 us, of which most is the launch and the verdicts of 592 blocks.
 template <bool AGAIN>
 __global__ void __launch_bounds__(256, 4) split_kernel(const SplitArgs a) {
   RT_PDL_ENTRY();

@@ -18,7 +18,7 @@
 // expires records a code in the status word and goes on without waiting.
 //
 // Bound by latency; at H 512 forward two of the 5.3 us are multiply-adds.  Measured, a timestep: batch 30, H 200: 2.3 us forward, 3.0
-// backward (2.4 and 3.9 before the pairs and the shorter mail); batch 64, H 512: 5.3 and 6.5 (5.4 and 7.9).  As kernels of their own the
+// backward (2.4 and 3.9 before the pairs and the shorter mail); batch 64, H 512: 5.3 and 6.6 (5.4 and 7.9).  As kernels of their own the
 // product, the cell and the concatenation took 9.7 forward, 12.3 backward at the first size.  Sizes whose blocks do not fit beside one
 // another, or whose slice of the weights does not fit into a block, run timestep by timestep.
 #include "packed_fma.cuh"
