@@ -10,7 +10,7 @@
 // at once, splits again into three bf16 parts (8 + 8 + 8 bits, exact, the exponents of fp32) and the same kernel runs six MMAs where it otherwise
 // runs three.  Within these lines an element keeps its 22 bits or is off by less than 2^-36 after scaling, which is 2^-27 of its segment's largest
 // and 2^-14 of itself.  Where the terms of a result all weigh the same, what the parts drop is 1.1e-7 of |A| |B| with magnitudes spread evenly over
-// 2^31, 3.3e-7 with 3xTF32; over 2^33, where the line is crossed, 8e-7 and 5e-7, over 2^40 6e-5.
+// 2^31, 3.3e-7 with 3xTF32.  Over 2^33, which goes to three parts, it would be 8e-7 and 5e-7, over 2^40 6e-5 and 5e-7.
 // The decision is made on the device; nothing waits for it on the host.
 //
 // A K-block in memory is four slots of 16 along the reduction: hi hi lo lo of 32 elements, or the three bf16 parts of 16 and the first once

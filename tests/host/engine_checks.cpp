@@ -78,10 +78,13 @@ rt_status rt_memcpy_d2d(rt_ctx*, void* d, const void* s, size_t n) {
 }
 rt_status rt_unary(rt_ctx*, int op, const float* x, float* y, int64_t n, float, float) {
   if (kernel() != RT_OK) return RT_ERR_CUDA;
-  for (int64_t i = 0; i < n && op == RT_SQUARE; ++i) y[i] = x[i] * x[i];
+  for (int64_t i = 0; i < n; ++i) y[i] = op == RT_SQUARE ? x[i] * x[i] : (op == RT_TANH ? std::tanh(x[i]) : (op == RT_SIGMOID ? 1.f / (1.f + std::exp(-x[i])) : x[i]));
   return RT_OK;
 }
-rt_status rt_binary(rt_ctx*, int, const float*, const int64_t*, int, const float*, const int64_t*, int, float*) {
+rt_status rt_binary(rt_ctx*, int op, const float* a, const int64_t* as, int na, const float* b, const int64_t*, int, float* out) {
+  int64_t n = 1;
+  for (int d = 0; d < na; ++d) n *= as[d];
+  for (int64_t i = 0; i < n && (op == RT_ADD || op == RT_MUL); ++i) out[i] = op == RT_ADD ? a[i] + b[i] : a[i] * b[i];  // of one shape
   return kernel();
 }
 rt_status rt_relu_max_pool2d(rt_ctx*, const float*, int64_t, int64_t, int64_t, int64_t, int, int, int, int, int, int, float*, float*) {
@@ -106,7 +109,9 @@ rt_status rt_sum_rows_accumulate_list(rt_ctx*, int count, const float* const* xs
     for (int64_t i = 0; i < rows * cols; ++i) out[i % cols] += xs[k][i];
   return RT_OK;
 }
-rt_status rt_gemm_bias_act_list(rt_ctx*, int, const float* const*, float* const*, int64_t, int64_t, int64_t, const float*, const float*, int) {
+rt_status rt_gemm_bias_act_list(rt_ctx* ctx, int count, const float* const* as, float* const* outs, int64_t m, int64_t n, int64_t k, const float* b,
+                                const float* bias, int act) {
+  for (int i = 0; i < count; ++i) rt_gemm_bias_act(ctx, m, n, k, as[i], k, b, n, bias, act, outs[i], n);
   return kernel();
 }
 uint64_t possible_ops = ~uint64_t(0);  // of kernels with a reduction; all ones: any
@@ -119,22 +124,89 @@ rt_status rt_reduce_backward(rt_ctx*, int, const float* x, const float*, int64_t
   for (int64_t i = 0; i < outer * len; ++i) dx[i] = x[i];  // to tell which values it has read
   return kernel();
 }
-rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // copies of windows; results of other programs stay zero
+rt_status rt_fused_elementwise(rt_ctx*, const rt_fused_program* p) {  // the ops that the checks use; others pass the accumulator on
   if (kernel() != RT_OK) return RT_ERR_CUDA;
   ++programs;
-  if (p->n_operands != 1 || p->n_outputs != 1 || p->nd > 2) return RT_OK;
-  const int rows = p->nd == 2 ? p->shape[0] : 1, cols = p->shape[p->nd - 1];
-  const rt_fused_operand& o = p->operand[0];
-  for (int i = 0; i < rows; ++i)
-    for (int j = 0; j < cols; ++j) p->out[0][i * cols + j] = o.ptr[(p->nd == 2 ? i * o.stride[0] : 0) + j * o.stride[p->nd - 1]];
+  int64_t n = 1;
+  for (int d = 0; d < p->nd; ++d) n *= p->shape[d];
+  for (int64_t e = 0; e < n; ++e) {
+    int64_t c[RT_FUSED_MAX_DIMS], rest = e;
+    for (int d = p->nd; d-- > 0; rest /= p->shape[d]) c[d] = rest % p->shape[d];
+    auto inside = [&](int r) {
+      bool in = true;
+      for (int d = 0; d < p->nd && r != RT_FUSED_NONE; ++d) in = in && c[d] >= p->region[r].lo[d] && c[d] < p->region[r].hi[d];
+      return in;
+    };
+    auto load = [&](int k) {
+      const float* q = p->operand[k].ptr;
+      for (int d = 0; d < p->nd; ++d) q += c[d] * p->operand[k].stride[d];
+      return inside(p->operand[k].region) ? *q : 0.f;
+    };
+    float reg[RT_FUSED_REGS] = {}, acc = 0.f;
+    for (int k = 0; k < p->n_preload; ++k) reg[k] = load(k);
+    for (int i = 0; i < p->n_code; ++i) {
+      const rt_fused_instr& in = p->code[i];
+      const float other = in.src == RT_FUSED_IMM ? in.imm : (in.src < RT_FUSED_REGS ? reg[in.src] : 0.f);
+      const float x = in.swap ? other : acc, y = in.swap ? acc : other;
+      switch (in.op) {
+        case RT_F_LOAD: acc = load(in.src); break;
+        case RT_F_REG: acc = other; break;
+        case RT_F_OUT: p->out[in.src][e] = acc; break;
+        case RT_F_SELECT: acc = inside(in.swap) ? acc : other; break;
+        case RT_F_ADD: acc = x + y; break;
+        case RT_F_SUB: acc = x - y; break;
+        case RT_F_MUL: acc = x * y; break;
+        case RT_F_SQUARE: acc = acc * acc; break;
+        case RT_F_TANH: acc = std::tanh(acc); break;
+        case RT_F_EXP: acc = std::exp(acc); break;
+        case RT_F_SIGMOID: acc = 1.f / (1.f + std::exp(-acc)); break;
+        default: break;
+      }
+      if (in.dst != RT_FUSED_NONE) reg[in.dst] = acc;
+    }
+  }
   return RT_OK;
+}
+// products and the recurrence, as far as the forward pass goes
+rt_status rt_gemm_bias_act(rt_ctx*, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb, const float* bias, int, float* c,
+                           int64_t ldc) {
+  for (int64_t i = 0; i < m; ++i)
+    for (int64_t j = 0; j < n; ++j) {
+      float sum = bias ? bias[j] : 0.f;
+      for (int64_t l = 0; l < k; ++l) sum += a[i * lda + l] * b[l * ldb + j];
+      c[i * ldc + j] = sum;
+    }
+  return kernel();
+}
+rt_status rt_gemm(rt_ctx* ctx, int ta, int tb, int64_t m, int64_t n, int64_t k, const float* a, int64_t lda, const float* b, int64_t ldb, float* c, int64_t ldc,
+                  int acc) {
+  return ta || tb || acc ? kernel() : rt_gemm_bias_act(ctx, m, n, k, a, lda, b, ldb, nullptr, 0, c, ldc);
+}
+rt_status rt_lstm_sequence(rt_ctx*, const float* pre, const float* w, int64_t ldw, const float* h0, const float* c0, int64_t steps, int64_t batch, int64_t hidden,
+                           float* saved, float* h) {
+  ++forward_sequences;
+  const int64_t n = batch * hidden, plane = steps * n;
+  for (int64_t t = 0; t < steps; ++t)
+    for (int64_t e = 0; e < n; ++e) {
+      const int64_t row = e / hidden, u = e % hidden, o = t * n + e;
+      float z[4];
+      for (int g = 0; g < 4; ++g) {
+        z[g] = pre[(t * batch + row) * 4 * hidden + g * hidden + u];
+        const float* before = t ? h + (t - 1) * n + row * hidden : (h0 ? h0 + row * hidden : nullptr);
+        for (int64_t l = 0; before && l < hidden; ++l) z[g] += before[l] * w[l * ldw + g * hidden + u];
+        z[g] = g == 2 ? std::tanh(z[g]) : 1.f / (1.f + std::exp(-z[g]));
+      }
+      const float c = z[1] * (t ? saved[4 * plane + o - n] : (c0 ? c0[e] : 0.f)) + z[0] * z[2];
+      const float kept[6] = {z[0], z[1], z[2], z[3], c, std::tanh(c)};
+      for (int k = 0; k < 6; ++k) saved[k * plane + o] = kept[k];
+      h[o] = z[3] * kept[5];
+    }
+  return kernel();
 }
 // their results stay zero
 rt_status rt_graph_begin(rt_ctx*) { return recording = true, RT_OK; }
 rt_status rt_graph_end(rt_ctx*, rt_graph**) { return recording = false, RT_OK; }
 rt_status rt_fill(rt_ctx*, float*, float, int64_t) { return kernel(); }
-rt_status rt_gemm(rt_ctx*, int, int, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, float*, int64_t, int) { return kernel(); }
-rt_status rt_gemm_bias_act(rt_ctx*, int64_t, int64_t, int64_t, const float*, int64_t, const float*, int64_t, const float*, int, float*, int64_t) { return kernel(); }
 rt_status rt_softmax_nll_list(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, float, float, int, const float* const*, float*) {
   return kernel();
 }
@@ -146,10 +218,6 @@ rt_status rt_reduce(rt_ctx*, int, const float*, int64_t, int64_t, int64_t, float
 rt_status rt_unbroadcast(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return kernel(); }
 rt_status rt_broadcast_to(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return kernel(); }
 rt_status rt_slice_assign(rt_ctx*, float*, const int64_t*, int, const int64_t*, const float*, const int64_t*) { return kernel(); }
-rt_status rt_lstm_sequence(rt_ctx*, const float*, const float*, int64_t, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) {
-  ++forward_sequences;
-  return kernel();
-}
 rt_status rt_lstm_sequence_backward(rt_ctx*, const float*, const float*, int64_t, const float*, const float*, int64_t, int64_t, int64_t, float*, float*,
                                     float*) {
   ++backward_sequences;
@@ -401,6 +469,70 @@ void cells_become_a_sequence() {
   }
 }
 
+// In a capture every state has the values of the recurrence, whatever is asked for first: the last state, a state, a gate, a cell state, a timestep's
+// inputs, what a product takes.
+void recurrences_have_their_values() {
+  using Tn = Tensor<B>;
+  const size_t T = 7, Bn = 3, V = 4, H = 2;
+  std::vector<float> xs(T * Bn * V), ws((V + H) * 4 * H), bs(4 * H), want_h, want_c;
+  for (size_t i = 0; i < xs.size(); ++i) xs[i] = std::sin(1.f + (float)i);
+  for (size_t i = 0; i < ws.size(); ++i) ws[i] = .7f * std::cos(2.f + (float)i);
+  for (size_t i = 0; i < bs.size(); ++i) bs[i] = .3f * std::sin(3.f * (float)i);
+  for (size_t t = 0; t < T; ++t)
+    for (size_t r = 0; r < Bn; ++r)
+      for (size_t u = 0; u < H; ++u) {
+        float z[4];
+        for (size_t g = 0; g < 4; ++g) {
+          z[g] = bs[g * H + u];
+          for (size_t v = 0; v < V; ++v) z[g] += xs[(t * Bn + r) * V + v] * ws[v * 4 * H + g * H + u];
+          for (size_t l = 0; l < H && t; ++l) z[g] += want_h[((t - 1) * Bn + r) * H + l] * ws[(V + l) * 4 * H + g * H + u];
+          z[g] = g == 2 ? std::tanh(z[g]) : 1.f / (1.f + std::exp(-z[g]));
+        }
+        const float c = z[1] * (t ? want_c[((t - 1) * Bn + r) * H + u] : 0.f) + z[0] * z[2];
+        want_c.push_back(c);
+        want_h.push_back(z[3] * std::tanh(c));
+      }
+  auto filled = [](const Shape& shape, const std::vector<float>& v) {
+    B::Storage x = B::alloc(shape);
+    std::copy(v.begin(), v.end(), x.buf->ptr);
+    return x;
+  };
+  enum { kLast, kState, kGate, kCellState, kInputs, kFirstInputs, kOperand, kSum, kWays };
+  for (int way = 0; way < kWays; ++way)
+    for (size_t at : {size_t(0), size_t(3), T - 1}) {
+      {
+        const Tn x(filled({T * Bn, V}, xs), false), w(filled({V + H, 4 * H}, ws), true), b(filled({4 * H}, bs), true);
+        std::vector<Tn> hs, cs;
+        B::begin_capture();
+        {
+          Tn h = Tn::zeros({Bn, H}, false), c = Tn::zeros({Bn, H}, false), asked;
+          for (size_t t = 0; t < T; ++t) {
+            const Tn xt = ops::slice(x, {{t * Bn, (t + 1) * Bn}, {0, V}}), xh = ops::concat<B>({xt, h}, 1);
+            const Tn z = ops::add(ops::matmul(xh, w), b.broadcast_to({Bn, 4 * H}));
+            auto gate = [&](size_t k) { return ops::slice(z, {{0, Bn}, {k * H, (k + 1) * H}}); };
+            const Tn i = ops::sigmoid(gate(0)), f = ops::sigmoid(gate(1));
+            c = ops::add(ops::mul(f, c), ops::mul(i, ops::tanh(gate(2))));
+            h = ops::mul(ops::sigmoid(gate(3)), ops::tanh(c));
+            hs.push_back(h);
+            cs.push_back(c);
+            if (t == at) asked = way == kState ? h : way == kGate ? f : way == kCellState ? c : way == kOperand ? xh : way == kSum ? ops::add(h, c) : xt;
+            if (t == 0 && way == kFirstInputs) xt.data().ptr();  // while the recurrence is being written
+          }
+          if (way != kLast && way != kFirstInputs) asked.data().ptr();
+          hs.back().data().ptr();
+        }
+        rt_graph* graph = nullptr;
+        for (size_t t = 0; t < T; ++t)
+          for (size_t e = 0; e < Bn * H; ++e) {
+            EXPECT(std::abs(hs[t].data().ptr()[e] - want_h[t * Bn * H + e]) < 1e-5f);
+            EXPECT(std::abs(cs[t].data().ptr()[e] - want_c[t * Bn * H + e]) < 1e-5f);
+          }
+        B::end_capture(&graph);
+      }
+      EXPECT(live.empty() && DeviceBuffer::waiting() == 0);
+    }
+}
+
 // What a captured step computes as rows of one matrix (the states of a sequence, the output layer's results, the gradients of the losses) and
 // somebody keeps stays where every replay writes it when its address is asked for; a slice of it goes elsewhere.
 void kept_results_stay_where_they_are_written() {
@@ -600,7 +732,7 @@ void gradients_of_rows() {
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"gradients_of_rows", gradients_of_rows}, {"refused_programs_take_no_memory", refused_programs_take_no_memory}, {"a_capture_in_two_parts", a_capture_in_two_parts},
+} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"recurrences_have_their_values", recurrences_have_their_values}, {"gradients_of_rows", gradients_of_rows}, {"refused_programs_take_no_memory", refused_programs_take_no_memory}, {"a_capture_in_two_parts", a_capture_in_two_parts},
                {"kept_results_stay_where_they_are_written", kept_results_stay_where_they_are_written},
                {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},
