@@ -267,7 +267,7 @@ class Compiler {
     if (r < 0) return false;
     outputs_.push_back({r, root});
     std::pair<int, DeviceBuffer*> sum{-1, nullptr};
-    if (keep_rows_ && nd_ == 2) sum = waiting_sum();
+    if (look_for_sums_ && nd_ == 2) sum = waiting_sum();
     if (!root->node) return false;
     for (auto& c : stored_) {
       if ((int)outputs_.size() + (sum.second ? 1 : 0) == RT_FUSED_MAX_OUTPUTS) break;
@@ -286,8 +286,11 @@ class Compiler {
     return false;
   }
   const std::vector<std::pair<int, DeviceBuffer*>>& outputs() const { return outputs_; }
-  // The dimensions stay those of the root (two), for a reduction over one of them.
-  void keep_rows() { keep_rows_ = true; }
+  // The dimensions stay those of the root (two), for a reduction over one of them; with_sums: for pending column sums, if there are any.
+  void keep_rows(bool with_sums) {
+    keep_rows_ = true;
+    look_for_sums_ = with_sums;
+  }
   // Among the outputs, the pending column sums of a term that shares values with the root (its buffer in the outputs is the sums'); -1: none.
   int sums() const { return sums_; }
 
@@ -326,7 +329,7 @@ class Compiler {
   std::vector<Memo> memo_;
   std::vector<std::pair<int, DeviceBuffer*>> stored_, outputs_;
 
-  bool keep_rows_ = false;
+  bool keep_rows_ = false, look_for_sums_ = false;
   int sums_ = -1;
   // A bias that is broadcast over the rows gets the column sums of a product of something that is computed here anyway: the term's value
   // and the buffer of the sums.
@@ -1373,13 +1376,12 @@ inline bool column_sum_waits(DeviceBuffer* b) {
       return true;
   return false;
 }
-// A program with a reduction of one of its outputs: column sums of output c.sums(), or with `lse` the logsumexp of the rows.  False: not a form that
-// there is a kernel for, and no memory has been taken for it.
+// A program with a reduction of one of its outputs: column sums of output c.sums(), or with `lse` the logsumexp of the rows.  False: it has not been
+// launched (there is no kernel for such a one, or b has been evaluated while it was built), and no memory has been taken for it.
 inline bool evaluate_reduced(DeviceBuffer* b, Compiler& c, float* lse) {
   rt_fused_program p;
   std::vector<DeviceBuffer*> outs;
-  if (!c.build(b, &p, &outs)) return !b->node;  // evaluated on the way
-  if ((c.sums() < 0) != (lse != nullptr)) return false;
+  if (!c.build(b, &p, &outs) || (c.sums() < 0) != (lse != nullptr)) return false;
   const rt_status known = rt_fused_reduction_known(b->ctx, &p, c.sums());
   if (known == RT_ERR_UNIMPLEMENTED) return false;
   check(b->ctx, known);
@@ -1413,12 +1415,12 @@ inline bool may_be_reduced(DeviceBuffer* b, int which) {
   }
   return rt_fused_reduction_possible(b->ctx, which, ops) == RT_OK;
 }
-// An expression over [rows, columns] together with the pending column sums of a term that it shares values with.
+// An expression over [rows, columns] together with the pending column sums of a term that it shares values with.  True: b is evaluated.
 inline bool evaluate_with_sums(DeviceBuffer* b) {
   if (Walk::depth() > 1 || b->node->shape.size() != 2 || b->numel == 0 || !column_sum_waits(b) || !may_be_reduced(b, 0)) return false;
   Compiler c;
-  c.keep_rows();
-  return evaluate_reduced(b, c, nullptr);
+  c.keep_rows(true);
+  return evaluate_reduced(b, c, nullptr) || !b->node;
 }
 // The gradients of rows that the expression b reads, each by its own kernel: no compiled program without a reduction has one.  (Interpreted within
 // the rest, tanh(x + b) of [4096, 4096] with its logsumexp and gradients 194 us, 164 this way; the same with the sine and exponential of the
@@ -1440,13 +1442,13 @@ inline void settle_row_gradients(DeviceBuffer* b) {
   }
   for (auto& f : found) lazy_evaluate(f.get());
 }
-// The rows of an expression and their logsumexp.
+// The rows of an expression and their logsumexp.  True only if `out` has been computed; b may have been evaluated without it.
 inline bool evaluate_with_logsumexp(DeviceBuffer* b, float* out) {
   if (Walk::depth() > 0 || !b->node || b->node->kind == Kind::Opaque || b->node->kind == Kind::Const || b->node->shape.size() != 2 || b->numel == 0) return false;
   if (!may_be_reduced(b, -1)) return false;
   std::shared_ptr<DeviceBuffer> guard = b->shared_from_this();
   Compiler c;
-  c.keep_rows();
+  c.keep_rows(false);
   return evaluate_reduced(b, c, out);
 }
 

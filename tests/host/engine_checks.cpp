@@ -19,6 +19,7 @@ bool kernels_fail = false;
 int masked_pool_gradients;     // launches of the pooling gradient that masks by the relu in front
 int forward_sequences, backward_sequences;
 int row_gradients, programs;   // launches of the gradient of a logsumexp by its own kernel, of elementwise programs
+int logsumexps;                // launches of a logsumexp, by its own kernel or within a program
 int asked_of_programs;         // programs built for a kernel with a reduction
 bool reductions_known = false; // kernels for programs with a reduction
 bool recording = false;
@@ -118,7 +119,7 @@ uint64_t possible_ops = ~uint64_t(0);  // of kernels with a reduction; all ones:
 rt_status rt_fused_reduction_possible(rt_ctx*, int, uint64_t ops) { return possible_ops == ~uint64_t(0) || ops == possible_ops ? RT_OK : RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_reduction_known(rt_ctx*, const rt_fused_program*, int) { return ++asked_of_programs, reductions_known ? RT_OK : RT_ERR_UNIMPLEMENTED; }
 rt_status rt_fused_column_sums(rt_ctx*, const rt_fused_program*, int, float*) { return kernel(); }
-rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return kernel(); }
+rt_status rt_fused_logsumexp(rt_ctx*, const rt_fused_program*, float*) { return ++logsumexps, kernel(); }
 rt_status rt_reduce_backward(rt_ctx*, int, const float* x, const float*, int64_t outer, int64_t len, int64_t, float* dx) {
   ++row_gradients;
   for (int64_t i = 0; i < outer * len; ++i) dx[i] = x[i];  // to tell which values it has read
@@ -214,7 +215,7 @@ rt_status rt_softmax_nll_with_grad(rt_ctx*, const float*, const float*, int64_t,
 rt_status rt_softmax_nll_scaled_backward(rt_ctx*, const float*, const float*, int64_t, int64_t, float, float*) { return kernel(); }
 rt_status rt_matmul_backward(rt_ctx*, const float*, const float*, const float*, int64_t, int64_t, int64_t, float*, float*) { return kernel(); }
 rt_status rt_gemm_sum_products(rt_ctx*, int, const float* const*, const float* const*, int64_t, int64_t, int64_t, float*) { return kernel(); }
-rt_status rt_reduce(rt_ctx*, int, const float*, int64_t, int64_t, int64_t, float*) { return kernel(); }
+rt_status rt_reduce(rt_ctx*, int op, const float*, int64_t, int64_t, int64_t, float*) { return logsumexps += op == RT_RED_LOGSUMEXP, kernel(); }
 rt_status rt_unbroadcast(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return kernel(); }
 rt_status rt_broadcast_to(rt_ctx*, const float*, const int64_t*, int, const int64_t*, int, float*) { return kernel(); }
 rt_status rt_slice_assign(rt_ctx*, float*, const int64_t*, int, const int64_t*, const float*, const int64_t*) { return kernel(); }
@@ -698,6 +699,25 @@ void refused_programs_take_no_memory() {
   EXPECT(live.empty());
 }
 
+// A logsumexp is computed whatever else waits for what its rows are made of: the rows may be evaluated by looking at that.
+void logsumexps_are_computed() {
+  for (bool known : {false, true})
+    for (bool whole : {false, true}) {
+      reductions_known = known;
+      const B::Storage x = make({4, 8}, 0.f), b = make({8}, 0.f);
+      const B::Storage h = B::tanh(x), y = B::add(h, B::broadcast_to(b, {4, 8}));
+      const B::Storage s = B::reduce(RT_RED_SUM, y, whole ? std::optional<size_t>() : std::optional<size_t>(0));
+      const B::Storage sums = B::unbroadcast(B::mul(h, B::broadcast_to(s, {4, 8})), {8});
+      EXPECT(sums.buf->node != nullptr);
+      logsumexps = 0;
+      const B::Storage lse = B::logsumexp(y, 1);
+      EXPECT(logsumexps == 1 && !y.buf->node);
+      sums.ptr();
+      reductions_known = false;
+    }
+  EXPECT(live.empty());
+}
+
 // The gradient of a logsumexp is part of a program that carries a reduction, where there is one; elsewhere it has a kernel of its own, which the
 // program around it reads.
 void gradients_of_rows() {
@@ -732,7 +752,7 @@ void gradients_of_rows() {
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"recurrences_have_their_values", recurrences_have_their_values}, {"gradients_of_rows", gradients_of_rows}, {"refused_programs_take_no_memory", refused_programs_take_no_memory}, {"a_capture_in_two_parts", a_capture_in_two_parts},
+} kChecks[] = {{"cells_become_a_sequence", cells_become_a_sequence}, {"long_recurrences", long_recurrences}, {"recurrences_have_their_values", recurrences_have_their_values}, {"gradients_of_rows", gradients_of_rows}, {"logsumexps_are_computed", logsumexps_are_computed}, {"refused_programs_take_no_memory", refused_programs_take_no_memory}, {"a_capture_in_two_parts", a_capture_in_two_parts},
                {"kept_results_stay_where_they_are_written", kept_results_stay_where_they_are_written},
                {"rows_do_not_alias", rows_do_not_alias}, {"rows_in_a_capture", rows_in_a_capture},
                {"broadcast_does_not_alias", broadcast_does_not_alias},

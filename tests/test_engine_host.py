@@ -17,7 +17,7 @@ def checks(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("name", ["cells_become_a_sequence", "long_recurrences", "recurrences_have_their_values", "gradients_of_rows", "refused_programs_take_no_memory", "a_capture_in_two_parts", "kept_results_stay_where_they_are_written", "rows_do_not_alias", "rows_in_a_capture", "broadcast_does_not_alias", "pooling_knows_its_relu", "errors_lose_nothing", "written_from_outside", "a_product_of_a_matrix_with_itself"])
+@pytest.mark.parametrize("name", ["cells_become_a_sequence", "long_recurrences", "recurrences_have_their_values", "gradients_of_rows", "logsumexps_are_computed", "refused_programs_take_no_memory", "a_capture_in_two_parts", "kept_results_stay_where_they_are_written", "rows_do_not_alias", "rows_in_a_capture", "broadcast_does_not_alias", "pooling_knows_its_relu", "errors_lose_nothing", "written_from_outside", "a_product_of_a_matrix_with_itself"])
 def test_engine(checks, name):
     r = subprocess.run([checks, name], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, f"exit code {r.returncode}\n{r.stdout}{r.stderr}"
