@@ -43,7 +43,7 @@ struct ConvSplitArgs {
   Decision* decision;
 };
 // Bound by memory: 4 bytes read and 4 written an element.  A block turns 32 channels x 128 pixels at a time through shared memory; what is
-// looked at is 128 pixels of a channel.  AGAIN: into three parts, if the first pass has found that two will not do.
+// looked at is 128 pixels of a channel, and all channels of a pixel.  AGAIN: into three parts, if the first pass has found that two will not do.
 template <bool AGAIN>
 __global__ void __launch_bounds__(256, 4) conv_split_kernel(const ConvSplitArgs a) {
   RT_PDL_ENTRY();
@@ -77,12 +77,13 @@ __global__ void __launch_bounds__(256, 4) conv_split_kernel(const ConvSplitArgs 
     const ImageSplit& s = a.image[q];
     const int exponent = q == 0 ? d.exponent[0] : d.exponent[1];
     const float scale = AGAIN ? 1.f : ldexpf(1.f, exponent);
-    const uint32_t faint = faint_below(exponent);
+    const uint32_t faint = faint_below(exponent), faint_pixel = faint_below(exponent, kFaintPixelExponent);
     Magnitudes all;
     for (int i0 = blockIdx.x; i0 < s.tiles; i0 += gridDim.x) {
       uint32_t im, t;
       s.d_tiles.divmod((uint32_t)i0, im, t);
       const int p0 = (int)t * kSplitPixels, left = s.HW - p0;
+      uint32_t pixel[2] = {};  // largest of this thread's channels of its two pixels
       for (int c0 = 0; c0 < s.C; c0 += 32) {
         const float* src = s.p + ((int64_t)im * s.C + c0) * s.HW + p0;
         float v[4][4];
@@ -123,7 +124,10 @@ __global__ void __launch_bounds__(256, 4) conv_split_kernel(const ConvSplitArgs 
           const int item = i * 256 + threadIdx.x, px = item >> 2, c = (item & 3) * 8;
           float x[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) x[j] = tile[c + j][px];
+          for (int j = 0; j < 8; ++j) {
+            x[j] = tile[c + j][px];
+            if (!AGAIN) pixel[i] = max(pixel[i], __float_as_uint(x[j]) & 0x7fffffffu);
+          }
           // the K-blocks that hold channels are written to their end
           if (px < left && c0 + c < (s.C + depth - 1) / depth * depth) {
             uint4 part[4];
@@ -137,6 +141,14 @@ __global__ void __launch_bounds__(256, 4) conv_split_kernel(const ConvSplitArgs 
             }
           }
         }
+      }
+      if (AGAIN) continue;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {  // four lanes have a pixel
+        uint32_t m = pixel[i];
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        if (m - 1 < faint_pixel) all.least = min(all.least, m);  // which is below what a segment's may be
       }
     }
     if (!AGAIN) {

@@ -32,6 +32,8 @@ constexpr int kLargestExponent = 14, kSmallestExponent = -9;  // of any element,
 // Two parts will do while there are next to none.  Of 2^24 numbers from a normal distribution 0.03 are, of the gate gradients of a recurrent network
 // 4; of magnitudes spread evenly over 2^31 none, over 2^33 one in 20.
 constexpr int kFaintExponent = -22;
+// An image's pixel is multiplied as a whole, all channels: its largest element stays above this, where two parts keep 20 bits at least.
+constexpr int kFaintPixelExponent = -16;
 inline uint32_t most_faint(int64_t elements) { return 4 + (uint32_t)(elements >> 20); }
 
 struct Decision {
@@ -109,7 +111,7 @@ __device__ __forceinline__ void over_samples(const uint2* samples, int sources, 
 // The exponent that a sample asks for; more than 100 either way is refused by verdict().
 __device__ __forceinline__ int exponent_for(uint32_t most) { return most == 0 || most >= 0x7f800000u ? 0 : kSampleExponent + 127 - (int)(most >> 23); }
 // An element of magnitude m (its bits) is faint if m - 1 is below this: zero is not.
-__device__ __forceinline__ uint32_t faint_below(int exponent) { return max(__float_as_uint(ldexpf(1.f, kFaintExponent - exponent)), 1u) - 1u; }
+__device__ __forceinline__ uint32_t faint_below(int exponent, int power = kFaintExponent) { return max(__float_as_uint(ldexpf(1.f, power - exponent)), 1u) - 1u; }
 // The least of m - 1 over a piece, an element more.
 __device__ __forceinline__ uint32_t lower(uint32_t least, uint32_t m) { return __viaddmin_u32(m, 0xffffffffu, least); }
 __device__ __forceinline__ uint32_t verdict(const Magnitudes& v, int exponent) {

@@ -106,6 +106,28 @@ def test_convolution_of_parts_of_wide_ranges(api, octaves):
         assert abs(got - terms.sum()) <= (32 * 2.0**-23 + 2.0**-21) * np.abs(terms).sum()
 
 
+@pytest.mark.parametrize("power", [-34, -30, -26, -18])
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("h,w", [(64, 64), (61, 67)])
+def test_pixels_far_below_the_rest(api, h, w, transposed, power):
+    """Of which the outputs at the same places are made, all channels of them: too few to be counted."""
+    n, cin, cout = 128, 32, 128
+    at = (3, 10, 11), (n - 1, h - 1, w - 1)
+    r = np.random.default_rng(h - power)
+    x = r.standard_normal((n, cin, h, w)).astype(np.float32)
+    wt = r.standard_normal((cin, cout, 1, 1) if transposed else (cout, cin, 1, 1)).astype(np.float32)
+    for i, v, u in at:
+        x[i, :, v, u] *= np.float32(2.0**power)
+    y = api.empty((n, cout, h, w))
+    dev = [api.to_device(v) for v in (x, wt, np.zeros(cout, np.float32))]
+    api.call("conv2d_transpose" if transposed else "conv2d", *[d.ptr for d in dev], i64(n), i64(cin), i64(h), i64(w), i64(cout), 1, 1, 1, 1, 0, 0, y.ptr)
+    got, m = y.numpy(), wt[:, :, 0, 0].astype(np.float64).T if transposed else wt[:, :, 0, 0].astype(np.float64)
+    for i, v, u in at:
+        p = x[i, :, v, u].astype(np.float64)
+        # the parts' own 2^-21, four additions with truncation
+        assert np.all(np.abs(got[i, :, v, u] - m @ p) <= (2.0**-21 + 4 * 2.0**-23) * (np.abs(m) @ np.abs(p)))
+
+
 @pytest.mark.parametrize("transposed", [False, True])
 @pytest.mark.parametrize("n,cin,h,w,cout,k,s,p", [(65, 70, 29, 31, 66, 3, 1, 1), (96, 33, 37, 35, 97, 4, 2, 1), (70, 66, 33, 30, 68, 5, 2, 2)])
 def test_infinities_and_nan_stay_where_they_belong(api, n, cin, h, w, cout, k, s, p, transposed):
